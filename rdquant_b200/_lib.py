@@ -1,19 +1,26 @@
-"""Build and load ``librdq_b200.so`` -- the C-ABI library holding the sm_100a kernels.
+"""Build and load ``librdq_b200.so`` -- the C-ABI library holding the sm_100a kernels -- and
+``_rdq_torch.so``, the CPython extension with the native per-call host path over it.
 
-The library is built in-tree with ``nvcc`` (``build()``) and bound with ``ctypes``;
-signatures follow ``include/rdq_b200.h``.  There is no fallback: if the library is
-missing or a call fails, a ``RuntimeError`` is raised.
+Both are built in-tree (``build()``); the library is bound with ``ctypes``, signatures follow
+``include/rdq_b200.h``.  There is no fallback: if one is missing or a call fails, a
+``RuntimeError`` is raised.
 """
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 import subprocess
+import sysconfig
+import tempfile
 import threading
+from concurrent.futures import ThreadPoolExecutor
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(_HERE, "csrc")
 LIB_PATH = os.path.join(CSRC, "librdq_b200.so")
+TORCH_EXT_PATH = os.path.join(CSRC, "_rdq_torch.so")
 SOURCES = [
     "rdq_api.cu",
     "rdq_dequant.cu",
@@ -23,13 +30,15 @@ SOURCES = [
     "rdq_quantize.cu",
     "rdq_stage.cu",
     "rdq_glue.cu",
+    "rdq_linear.cu",
 ]
+TORCH_EXT_SOURCE = "rdq_torch.cpp"
 HEADERS = ["rdq_common.cuh", "rdq_kernels.cuh", "rdq_gemv_tiled_kernel.inl", "rdq_gemm_kernel.inl",
            os.path.join("..", "..", "include", "rdq_b200.h")]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-lineinfo", "-O3", "-std=c++17",
-    "--shared", "-Xcompiler", "-fPIC",
+    "-Xcompiler", "-fPIC",
 ]
 
 RDQ_GEMV_AUTO = 0
@@ -43,31 +52,43 @@ _lock = threading.Lock()
 _lib = None
 
 
-def _stale() -> bool:
-    if not os.path.exists(LIB_PATH):
+def _older(target: str, files: list) -> bool:
+    if not os.path.exists(target):
         return True
-    t = os.path.getmtime(LIB_PATH)
-    for f in SOURCES + HEADERS:
-        p = os.path.join(CSRC, f)
-        if os.path.exists(p) and os.path.getmtime(p) > t:
-            return True
-    return False
+    t = os.path.getmtime(target)
+    return any(os.path.exists(p) and os.path.getmtime(p) > t for p in (os.path.join(CSRC, f) for f in files))
+
+
+def _stale() -> bool:
+    return _older(LIB_PATH, SOURCES + HEADERS)
+
+
+def _run(cmd: list) -> str:
+    res = subprocess.run(cmd, cwd=CSRC, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"{os.path.basename(cmd[0])} failed:\n" + res.stdout + res.stderr)
+    return res.stderr
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile the kernels for sm_100a into ``csrc/librdq_b200.so`` (needs nvcc, no GPU)."""
-    if not force and not _stale():
-        return LIB_PATH
-    nvcc = os.environ.get("NVCC", "nvcc")
-    cmd = [nvcc, *NVCC_FLAGS, "-o", LIB_PATH, *SOURCES, "-lcuda"]
-    if verbose:
-        cmd.insert(1, "-Xptxas")
-        cmd.insert(2, "-v")
-    res = subprocess.run(cmd, cwd=CSRC, capture_output=True, text=True)
-    if res.returncode != 0:
-        raise RuntimeError("nvcc failed:\n" + res.stdout + res.stderr)
-    if verbose:
-        print(res.stderr)
+    """Compile the kernels for sm_100a into ``csrc/librdq_b200.so`` and the host path into
+    ``csrc/_rdq_torch.so`` (needs nvcc and a C++ compiler, no GPU)."""
+    if force or _stale():
+        nvcc = os.environ.get("NVCC", "nvcc")
+        extra = ["-Xptxas", "-v"] if verbose else []
+        with tempfile.TemporaryDirectory() as tmp, ThreadPoolExecutor() as pool:
+            objs = [os.path.join(tmp, src + ".o") for src in SOURCES]
+            for text in pool.map(lambda so: _run([nvcc, *NVCC_FLAGS, *extra, "-c", so[0], "-o", so[1]]), zip(SOURCES, objs)):
+                if verbose:
+                    print(text)
+            _run([nvcc, "--shared", "-o", LIB_PATH, *objs, "-lcuda"])
+    if force or _older(TORCH_EXT_PATH, [TORCH_EXT_SOURCE, HEADERS[-1]]):
+        from torch.utils.cpp_extension import include_paths, library_paths
+
+        dirs = include_paths("cuda") + [sysconfig.get_paths()["include"]]
+        _run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", TORCH_EXT_SOURCE, "-o", TORCH_EXT_PATH,
+              *("-I" + d for d in dirs), *("-L" + d for d in library_paths("cuda")), "-L" + CSRC, "-l:librdq_b200.so",
+              "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-Wl,-rpath,$ORIGIN"])
     return LIB_PATH
 
 
@@ -132,6 +153,10 @@ def _bind(lib: ctypes.CDLL) -> None:
     lib.rdq_rope_attn_decode.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, f32, f32, i32, vp]
     lib.rdq_silu_mul.restype = i32
     lib.rdq_silu_mul.argtypes = [vp, vp, i32, i32, i32, vp]
+    lib.rdq_linear_workspace_size.restype = i32
+    lib.rdq_linear_workspace_size.argtypes = [vp, i32, i32, ctypes.POINTER(ctypes.c_size_t)]
+    lib.rdq_linear.restype = i32
+    lib.rdq_linear.argtypes = [vp, vp, i32, i32, vp, vp, vp, ctypes.c_size_t, i32, vp]
     lib.rdq_stage_copy.restype = i32
     lib.rdq_stage_copy.argtypes = [vp, vp, ctypes.c_size_t, vp]
     lib.rdq_stage_copy_signal.restype = i32
@@ -161,6 +186,8 @@ EXPORTS = [
     "rdq_gemm_workspace_size",
     "rdq_quantize_nvfp4",
     "rdq_quantize_fp8",
+    "rdq_linear",
+    "rdq_linear_workspace_size",
     "rdq_stage_copy",
     "rdq_stage_copy_signal",
     "rdq_add_rmsnorm",
@@ -174,7 +201,7 @@ EXPORTS = [
 
 
 def available() -> bool:
-    return os.path.exists(LIB_PATH)
+    return os.path.exists(LIB_PATH) and os.path.exists(TORCH_EXT_PATH)
 
 
 def lib() -> ctypes.CDLL:
@@ -193,6 +220,26 @@ def lib() -> ctypes.CDLL:
             _bind(handle)
             _lib = handle
     return _lib
+
+
+_torch_ext = None
+
+
+def torch_ext():
+    """The native host path (module ``_rdq_torch``); raise ``RuntimeError`` if it has not been built."""
+    global _torch_ext
+    if _torch_ext is None:
+        lib()
+        with _lock:
+            if _torch_ext is None:
+                if not os.path.exists(TORCH_EXT_PATH):
+                    raise RuntimeError(f"{TORCH_EXT_PATH} is missing: run rdquant_b200._lib.build()")
+                loader = importlib.machinery.ExtensionFileLoader("_rdq_torch", TORCH_EXT_PATH)
+                spec = importlib.util.spec_from_file_location("_rdq_torch", TORCH_EXT_PATH, loader=loader)
+                module = importlib.util.module_from_spec(spec)
+                loader.exec_module(module)
+                _torch_ext = module
+    return _torch_ext
 
 
 def check(rc: int, what: str) -> None:

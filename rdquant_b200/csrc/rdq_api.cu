@@ -107,13 +107,13 @@ int rdq_gemv_mixed(const void *x, int M, const void *w_fp4, const void *w_fp4_sc
   a.w16 = static_cast<const __half *>(w_fp16);
   a.perm = perm;
   a.bias = static_cast<const __half *>(bias);
-  a.y = static_cast<__half *>(y);
+  a.y = y;
   a.n4 = n_fp4;
   a.n8 = n_fp8;
   a.n16 = n_fp16;
   a.K = K;
-  a.workspace = static_cast<float *>(workspace);
-  a.counters = counters;
+  (void)workspace;
+  (void)counters;
   (void)flags;
   return launch_gemv_generic(a, static_cast<cudaStream_t>(stream));
 }
@@ -150,14 +150,14 @@ int rdq_gemv_tiled(const void *x, int M, const void *w_tiled, const float *w_fp8
   RDQ_REQUIRE(aligned16(x) && aligned16(w_tiled), RDQ_E_INVALID, "x and w_tiled must be 16-byte aligned");
   RDQ_REQUIRE(n_fp8 == 0 || w_fp8_scales != nullptr, RDQ_E_INVALID, "w_fp8_scales must not be null when n_fp8 > 0");
   GemvTiledArgs a;
-  a.x = static_cast<const __half *>(x);
+  a.x = x;
   a.M = M;
   a.tiled = static_cast<const uint8_t *>(w_tiled);
   a.s8 = w_fp8_scales;
   a.global4 = w_fp4_global_scale;
   a.perm = perm;
   a.bias = static_cast<const __half *>(bias);
-  a.y = static_cast<__half *>(y);
+  a.y = y;
   a.n4 = n_fp4;
   a.n8 = n_fp8;
   a.n16 = n_fp16;
@@ -189,14 +189,14 @@ int rdq_gemv_tiled_xop(int op, const void *x, const void *x_aux, const void *x_w
               "x_out must not alias x or x_aux: every CTA reads them");
   RDQ_REQUIRE(n_fp8 == 0 || w_fp8_scales != nullptr, RDQ_E_INVALID, "w_fp8_scales must not be null when n_fp8 > 0");
   GemvTiledArgs a;
-  a.x = static_cast<const __half *>(x);
+  a.x = x;
   a.M = M;
   a.tiled = static_cast<const uint8_t *>(w_tiled);
   a.s8 = w_fp8_scales;
   a.global4 = w_fp4_global_scale;
   a.perm = perm;
   a.bias = static_cast<const __half *>(bias);
-  a.y = static_cast<__half *>(y);
+  a.y = y;
   a.n4 = n_fp4;
   a.n8 = n_fp8;
   a.n16 = n_fp16;
@@ -227,7 +227,7 @@ int rdq_gemv_tiled_peer(const void *x, int M, const void *w_tiled, const float *
   RDQ_REQUIRE(aligned16(x) && aligned16(w_tiled), RDQ_E_INVALID, "x and w_tiled must be 16-byte aligned");
   RDQ_REQUIRE(n_fp8 == 0 || w_fp8_scales != nullptr, RDQ_E_INVALID, "w_fp8_scales must not be null when n_fp8 > 0");
   GemvTiledArgs a;
-  a.x = static_cast<const __half *>(x);
+  a.x = x;
   a.M = M;
   a.tiled = static_cast<const uint8_t *>(w_tiled);
   a.s8 = w_fp8_scales;
@@ -273,14 +273,14 @@ int rdq_gemv_tiled_noalloc(const void *x, int M, const void *w_tiled, const floa
   RDQ_REQUIRE(aligned16(x) && aligned16(w_tiled), RDQ_E_INVALID, "x and w_tiled must be 16-byte aligned");
   RDQ_REQUIRE(n_fp8 == 0 || w_fp8_scales != nullptr, RDQ_E_INVALID, "w_fp8_scales must not be null when n_fp8 > 0");
   GemvTiledArgs a;
-  a.x = static_cast<const __half *>(x);
+  a.x = x;
   a.M = M;
   a.tiled = static_cast<const uint8_t *>(w_tiled);
   a.s8 = w_fp8_scales;
   a.global4 = w_fp4_global_scale;
   a.perm = perm;
   a.bias = static_cast<const __half *>(bias);
-  a.y = static_cast<__half *>(y);
+  a.y = y;
   a.n4 = n_fp4;
   a.n8 = n_fp8;
   a.n16 = n_fp16;
@@ -329,7 +329,7 @@ int rdq_gemm_mixed_ws(const void *x, int M, const void *w_fp4, const void *w_fp4
   a.w16 = static_cast<const __half *>(w_fp16);
   a.inv_perm = inv_perm;
   a.bias = static_cast<const __half *>(bias);
-  a.y = static_cast<__half *>(y);
+  a.y = y;
   a.n4 = n_fp4;
   a.n8 = n_fp8;
   a.n16 = n_fp16;

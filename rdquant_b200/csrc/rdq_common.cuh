@@ -212,6 +212,26 @@ __device__ __forceinline__ void linger(unsigned int ns) {
   }
 }
 
+// one output value: f16, or bf16 for callers whose activations are bf16
+__device__ __forceinline__ void store_y(void *y, long long i, float v, int bf16) {
+  if (bf16) static_cast<__nv_bfloat16 *>(y)[i] = __float2bfloat16_rn(v);
+  else static_cast<__half *>(y)[i] = __float2half_rn(v);
+}
+// two adjacent output values packed into a word
+__device__ __forceinline__ uint32_t pack_y2(float a, float b, int bf16) {
+  if (bf16) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t *>(&h);
+  }
+  const __half2 h = __floats2half2_rn(a, b);
+  return *reinterpret_cast<const uint32_t *>(&h);
+}
+// two packed bf16 values -> two packed f16 values (round to nearest even)
+__device__ __forceinline__ uint32_t bf16x2_to_f16x2(uint32_t v) {
+  const __half2 h = __floats2half2_rn(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
+  return *reinterpret_cast<const uint32_t *>(&h);
+}
+
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));

@@ -321,18 +321,17 @@ gemm_mixed_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
                 const int c = cc * 32 + v * 8 + e * 2;
                 const float f0 = fmaf(__uint_as_float(r[v * 8 + e * 2]), S.colscale[c], S.colbias[c]);
                 const float f1 = fmaf(__uint_as_float(r[v * 8 + e * 2 + 1]), S.colscale[c + 1], S.colbias[c + 1]);
-                const __half2 h = __floats2half2_rn(f0, f1);
-                o[e] = *reinterpret_cast<const uint32_t *>(&h);
+                o[e] = pack_y2(f0, f1, a.y_bf16);
               }
               asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(stg + lane * kEpiPitch + hh * 64 + v * 16), "r"(o[0]),
                            "r"(o[1]), "r"(o[2]), "r"(o[3])
                            : "memory");
             }
           } else if (m < a.M) {
-            __half *dst = a.y + 1ll * m * N + n0 + cc * 32;
             for (int e = 0; e < 32; ++e) {
               const int c = cc * 32 + e;
-              if (n0 + c < N) dst[e] = __float2half_rn(fmaf(__uint_as_float(r[e]), S.colscale[c], S.colbias[c]));
+              if (n0 + c < N)
+                store_y(a.y, 1ll * m * N + n0 + c, fmaf(__uint_as_float(r[e]), S.colscale[c], S.colbias[c]), a.y_bf16);
             }
           }
           }  // hh
@@ -348,7 +347,7 @@ gemm_mixed_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
                            : "=r"(val.x), "=r"(val.y), "=r"(val.z), "=r"(val.w)
                            : "r"(stg + row * kEpiPitch + piece * 16)
                            : "memory");
-              if (m_base + row < a.M) *reinterpret_cast<uint4 *>(a.y + 1ll * (m_base + row) * N + n0 + c0 + piece * 8) = val;
+              if (m_base + row < a.M) *reinterpret_cast<uint4 *>(static_cast<__half *>(a.y) + 1ll * (m_base + row) * N + n0 + c0 + piece * 8) = val;
             }
             __syncwarp();
           }
@@ -385,7 +384,7 @@ __global__ void __launch_bounds__(256) gemm_reduce_kernel(const GemmArgs a, int 
     const int r = a.inv_perm ? a.inv_perm[n] : n;
     const float scl = (r < a.n4) ? a.global4 : (r < a.n4 + a.n8 ? a.s8[r - a.n4] : 1.f);
     const float bia = a.bias ? __half2float(a.bias[n]) : 0.f;
-    a.y[i] = __float2half_rn(fmaf(v, scl, bia));
+    store_y(a.y, i, fmaf(v, scl, bia), a.y_bf16);
   }
 }
 

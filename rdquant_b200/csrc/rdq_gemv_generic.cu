@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(256) gemv_generic_kernel(GemvArgs a) {
 #pragma unroll
   for (int m = 0; m < MP; ++m) {
     const float s = warp_sum(acc[m]);
-    if (m < M && lane == 0) a.y[1ll * m * N + col] = __float2half_rn(fmaf(s, out_scale, b));
+    if (m < M && lane == 0) store_y(a.y, 1ll * m * N + col, fmaf(s, out_scale, b), a.y_bf16);
   }
 }
 

@@ -70,14 +70,15 @@ __device__ __forceinline__ uint4 ldg_cg16(const void *p) {
 }
 
 struct TiledArgs {
-  const __half *x;
+  const __half *x;  // bf16 rows with xop == 3
   int M;
   const uint8_t *tiled;
   const float *s8;
   float global4;
   const int32_t *perm;
   const __half *bias;
-  __half *y;
+  void *y;
+  int y_bf16;
   int n4, n8, n16, K;
   float *workspace;
   int32_t *flags;  // one per CTA, then the status word at index status_idx
@@ -98,6 +99,7 @@ struct TiledArgs {
   // Activation prologue (0: x is used as it is).  1: x_in = x (+ x_aux); the CTA's activation rows
   // are f16(x_in * rsqrt(mean(x_in^2) + eps)) * x_weight, and CTA 0 writes x_in to x_out (the
   // updated residual stream).  2: x is [M, 2 K] and the rows are silu(x[:, :K]) * x[:, K:].
+  // 3: x is bf16 and the rows are its f16 rounding.
   int xop;
   const __half *x_aux;
   const __half *x_weight;
@@ -643,8 +645,10 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
           *pw = __uint_as_float(0xffffffffu);  // slot idle again
         }
         const __half h = __float2half_rn(fmaf(v, scl, bia));
-        if (!EXTRA || a.n_dst == 0) {
-          a.y[1ll * m * N + col] = h;
+        if (!EXTRA) {
+          static_cast<__half *>(a.y)[1ll * m * N + col] = h;
+        } else if (a.n_dst == 0) {
+          store_y(a.y, 1ll * m * N + col, fmaf(v, scl, bia), a.y_bf16);
         } else {
           // the 16 rows of a tile are consecutive columns of the slice: the stores of the lanes
           // of one activation row fall into one 32-byte sector per destination
@@ -777,6 +781,25 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
             hv[j] = __hmul2(__floats2half2_rn(f.x * rs, f.y * rs), wh[j]);
           }
           *reinterpret_cast<uint4 *>(xsm + m * xpitch + 16 * i) = v;
+        }
+      }
+    } else if (a.xop == 3) {
+      for (int u = warp; u < M * cpr; u += kMmaWarps) {
+        const int m = u / cpr, c = u - m * cpr;
+        const int hi = min(nvec, (c + 1) * per);
+        const __half *xr = a.x + 1ll * m * K;
+        for (int i0 = c * per + lane; i0 < hi; i0 += 128) {
+          uint4 v[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (i0 + 32 * q < hi) v[q] = ldg_cg16(xr + 8 * (i0 + 32 * q));
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int i = i0 + 32 * q;
+            if (i >= hi) break;
+            *reinterpret_cast<uint4 *>(xsm + m * xpitch + 16 * i) =
+                make_uint4(bf16x2_to_f16x2(v[q].x), bf16x2_to_f16x2(v[q].y), bf16x2_to_f16x2(v[q].z), bf16x2_to_f16x2(v[q].w));
+          }
         }
       }
     } else {
@@ -959,7 +982,7 @@ int launch_gemv_tiled(const GemvTiledArgs &h, bool pdl, cudaStream_t stream) {
   sc.img8 = img_bytes(1, ck);
 
   TiledArgs a;
-  a.x = h.x; a.M = h.M; a.tiled = h.tiled; a.s8 = h.s8; a.global4 = h.global4; a.perm = h.perm;
+  a.x = static_cast<const __half *>(h.x); a.y_bf16 = h.y_bf16; a.M = h.M; a.tiled = h.tiled; a.s8 = h.s8; a.global4 = h.global4; a.perm = h.perm;
   a.bias = h.bias; a.y = h.y; a.n4 = h.n4; a.n8 = h.n8; a.n16 = h.n16; a.K = h.K;
   a.workspace = h.workspace; a.flags = h.flags;
   a.test_timeout = h.test_timeout;
@@ -969,7 +992,7 @@ int launch_gemv_tiled(const GemvTiledArgs &h, bool pdl, cudaStream_t stream) {
     a.peer_flag[d] = d < h.n_dst ? h.peer_flag[d] : nullptr;
   }
   a.peer_state = h.peer_state;
-  a.xop = h.xop; a.x_aux = h.x_aux; a.x_weight = h.x_weight; a.x_out = h.x_out; a.x_eps = h.x_eps;
+  a.xop = h.x_bf16 ? 3 : h.xop; a.x_aux = h.x_aux; a.x_weight = h.x_weight; a.x_out = h.x_out; a.x_eps = h.x_eps;
   a.status_idx = sm_count();
   a.slot_bytes = (img_bytes(0, ck) + 127) & ~127;
   const int nt = h.M <= 8 ? 1 : 2;
@@ -979,7 +1002,7 @@ int launch_gemv_tiled(const GemvTiledArgs &h, bool pdl, cudaStream_t stream) {
   a.nstages = pl.nst;
   const bool xs = pl.xs;
   const int nst = pl.nst;
-  RDQ_REQUIRE(h.xop == 0 || xs, RDQ_E_UNSUPPORTED,
+  RDQ_REQUIRE(a.xop == 0 || xs, RDQ_E_UNSUPPORTED,
               "activation prologue needs the activation rows in shared memory (M=%d, K=%d)", h.M, h.K);
   RDQ_REQUIRE(h.xop == 0 || (h.xop == 1 && h.x_weight) || h.xop == 2, RDQ_E_INVALID, "bad activation prologue");
   const int smem = pl.smem;
@@ -1040,7 +1063,7 @@ int launch_gemv_tiled(const GemvTiledArgs &h, bool pdl, cudaStream_t stream) {
   int dev = 0;
   RDQ_CUDA(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> smem_lock(smem_mutex);
-  const bool extra = h.xop != 0 || h.n_dst > 0;
+  const bool extra = a.xop != 0 || h.n_dst > 0 || h.y_bf16;
   const int variant = (extra ? 4 : 0) + (nt - 1) * 2 + (xs ? 1 : 0);
   static const void *const fns[8] = {
       reinterpret_cast<const void *>(gemv_tiled_kernel<1, false, false>),

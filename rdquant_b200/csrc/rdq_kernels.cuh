@@ -25,10 +25,9 @@ struct GemvArgs {
   const __half *w16;
   const int32_t *perm;
   const __half *bias;
-  __half *y;
+  void *y;
   int n4, n8, n16, K;
-  float *workspace;   // unused by the any-shape kernel
-  int32_t *counters;
+  int y_bf16 = 0;  // y is bf16 instead of f16
 };
 
 struct GemmArgs {
@@ -42,8 +41,9 @@ struct GemmArgs {
   const __half *w16;
   const int32_t *inv_perm;
   const __half *bias;
-  __half *y;
+  void *y;
   int n4, n8, n16, K;
+  int y_bf16 = 0;  // y is bf16 instead of f16
   int ksplit;      // CTAs that share the k range of a tile (blockIdx.z); 1 = no split
   float *partial;  // ksplit > 1: raw FP32 sums [ksplit][M][N], reduced by a second kernel
   int test_timeout = 0;  // self-test: CTA (0,0,0) ends with a wait that runs out
@@ -54,18 +54,23 @@ int launch_dequant(const void *w_fp4, const void *w_fp4_scales, float global4, c
                    const int32_t *inv_perm, void *w_out, int out_is_f32, int n4, int n8, int n16,
                    int K, cudaStream_t stream);
 
+// bf16 -> f16, count % 8 == 0, both 16-byte aligned
+int launch_cast_rows(const void *x_bf16, void *x_f16, long long count, bool pdl, cudaStream_t stream);
+
 int launch_gemv_generic(const GemvArgs &a, cudaStream_t stream);
 
 // ---- tiled layout (rdq_gemv_tiled.cu)
 struct GemvTiledArgs {
-  const __half *x;
+  const void *x;
+  int x_bf16 = 0;  // x is bf16: the kernel rounds the rows to f16 as it stages them in shared memory
+  int y_bf16 = 0;  // y is bf16 instead of f16
   int M;
   const uint8_t *tiled;
   const float *s8;
   float global4;
   const int32_t *perm;
   const __half *bias;
-  __half *y;
+  void *y;
   int n4, n8, n16, K;
   float *workspace;
   int32_t *flags;

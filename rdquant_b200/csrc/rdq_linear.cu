@@ -1,0 +1,219 @@
+// The operator behind one call: picks the kernel by the number of activation rows and by the
+// layouts the layer carries, and converts bf16 activations where the kernel does not do it itself.
+//
+// Reference behaviour replaced: the dispatch of FusedMixedLinear.forward
+// (rdquant/inference.py:689-708) with its x.half() / y.to(x.dtype) conversions (:696, :707).
+#include "rdq_kernels.cuh"
+
+namespace rdq {
+
+namespace {
+
+// HBM-bound: reads and writes 2 bytes per element.
+__global__ void __launch_bounds__(256) cast_rows_kernel(const uint4 *__restrict__ x, uint4 *__restrict__ out, long long nvec) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const long long stride = 1ll * gridDim.x * blockDim.x;
+  for (long long i = 1ll * blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += 4 * stride) {
+    uint4 v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (i + q * stride < nvec) v[q] = x[i + q * stride];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (i + q * stride < nvec)
+        out[i + q * stride] =
+            make_uint4(bf16x2_to_f16x2(v[q].x), bf16x2_to_f16x2(v[q].y), bf16x2_to_f16x2(v[q].z), bf16x2_to_f16x2(v[q].w));
+  }
+}
+__global__ void __launch_bounds__(256) cast_elems_kernel(const __nv_bfloat16 *__restrict__ x, __half *__restrict__ out,
+                                                         long long count) {
+  pdl_launch_dependents();
+  pdl_wait();
+  for (long long i = 1ll * blockIdx.x * blockDim.x + threadIdx.x; i < count; i += 1ll * gridDim.x * blockDim.x)
+    out[i] = __float2half_rn(__bfloat162float(x[i]));
+}
+
+enum class Path { kGemvTiled, kGemvGeneric, kGemm, kPanelsTiled, kPanelsGeneric };
+
+bool has_row_major(const rdq_layer &l) {
+  return (l.n_fp4 == 0 || l.w_fp4) && (l.n_fp8 == 0 || l.w_fp8) && (l.n_fp16 == 0 || l.w_fp16);
+}
+
+// Up to 16 rows: the decode GEMV (tiled layout, else the any-shape kernel).  More rows: the
+// tensor-core GEMM, which tiles K in blocks of 64 and reads the row-major tensors; what it cannot
+// take runs as 16-row panels of the decode kernel.
+Path path_of(const rdq_layer &l, int M) {
+  if (M <= RDQ_MAX_GEMV_M) return l.w_tiled ? Path::kGemvTiled : Path::kGemvGeneric;
+  if (l.K % 64 == 0 && has_row_major(l)) return Path::kGemm;
+  return l.w_tiled ? Path::kPanelsTiled : Path::kPanelsGeneric;
+}
+
+// true when the kernel of this path rounds bf16 rows itself
+bool takes_bf16(const rdq_layer &l, Path p, int M) { return p == Path::kGemvTiled && tiled_stages_x(M, l.K); }
+
+size_t align256(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
+
+struct Need {
+  size_t cast = 0, gemm = 0;
+};
+Need need_of(const rdq_layer &l, Path p, int M, int x_type) {
+  Need n;
+  if (x_type == RDQ_BF16 && !takes_bf16(l, p, M)) n.cast = align256(2ull * M * l.K);
+  if (p == Path::kGemm) n.gemm = gemm_workspace_bytes(M, l.n_fp4 + l.n_fp8 + l.n_fp16, l.K);
+  return n;
+}
+
+int run_gemv(const rdq_layer &l, bool tiled, const void *x, int x_bf16, int M, const void *bias, void *y, int y_bf16, bool pdl,
+             cudaStream_t stream) {
+  if (tiled) {
+    GemvTiledArgs a;
+    a.x = x;
+    a.x_bf16 = x_bf16;
+    a.y_bf16 = y_bf16;
+    a.M = M;
+    a.tiled = static_cast<const uint8_t *>(l.w_tiled);
+    a.s8 = l.w_fp8_scales;
+    a.global4 = l.w_fp4_global_scale;
+    a.perm = l.perm;
+    a.bias = static_cast<const __half *>(bias);
+    a.y = y;
+    a.n4 = l.n_fp4;
+    a.n8 = l.n_fp8;
+    a.n16 = l.n_fp16;
+    a.K = l.K;
+    a.workspace = static_cast<float *>(l.gemv_ws);
+    a.flags = l.gemv_counters;
+    return launch_gemv_tiled(a, pdl, stream);
+  }
+  GemvArgs a;
+  a.x = static_cast<const __half *>(x);
+  a.M = M;
+  a.w4 = static_cast<const uint8_t *>(l.w_fp4);
+  a.s4 = static_cast<const uint8_t *>(l.w_fp4_scales);
+  a.global4 = l.w_fp4_global_scale;
+  a.w8 = static_cast<const uint8_t *>(l.w_fp8);
+  a.s8 = l.w_fp8_scales;
+  a.w16 = static_cast<const __half *>(l.w_fp16);
+  a.perm = l.perm;
+  a.bias = static_cast<const __half *>(bias);
+  a.y = y;
+  a.n4 = l.n_fp4;
+  a.n8 = l.n_fp8;
+  a.n16 = l.n_fp16;
+  a.K = l.K;
+  a.y_bf16 = y_bf16;
+  return launch_gemv_generic(a, stream);
+}
+
+}  // namespace
+
+int launch_cast_rows(const void *x_bf16, void *x_f16, long long count, bool pdl, cudaStream_t stream) {
+  if (count == 0) return RDQ_OK;
+  const bool vec = count % 8 == 0 && aligned16(x_bf16) && aligned16(x_f16);
+  const long long per = vec ? 8 * 256 : 256;
+  long long blocks = (count + per - 1) / per;
+  const long long cap = 8ll * sm_count();
+  if (blocks > cap) blocks = cap;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(blocks));
+  cfg.blockDim = dim3(256);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (vec) {
+    RDQ_CUDA(cudaLaunchKernelEx(&cfg, cast_rows_kernel, static_cast<const uint4 *>(x_bf16), static_cast<uint4 *>(x_f16),
+                                count / 8));
+  } else {
+    RDQ_CUDA(cudaLaunchKernelEx(&cfg, cast_elems_kernel, static_cast<const __nv_bfloat16 *>(x_bf16),
+                                static_cast<__half *>(x_f16), count));
+  }
+  return RDQ_OK;
+}
+
+}  // namespace rdq
+
+using namespace rdq;
+
+extern "C" {
+
+int rdq_linear_workspace_size(const rdq_layer *layer, int M, int x_type, size_t *bytes) {
+  RDQ_REQUIRE(layer && bytes && M >= 0, RDQ_E_INVALID, "bad arguments to rdq_linear_workspace_size");
+  const Need n = need_of(*layer, path_of(*layer, M), M, x_type);
+  *bytes = n.cast + n.gemm;
+  return RDQ_OK;
+}
+
+int rdq_linear(const rdq_layer *layer, const void *x, int x_type, int M, const void *bias, void *y, void *workspace,
+               size_t workspace_bytes, int flags, void *stream_) {
+  RDQ_REQUIRE(layer != nullptr && M >= 0 && (x_type == RDQ_F16 || x_type == RDQ_BF16), RDQ_E_INVALID, "bad arguments to rdq_linear");
+  const rdq_layer &l = *layer;
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  const int N = l.n_fp4 + l.n_fp8 + l.n_fp16;
+  if (M == 0 || N == 0) return RDQ_OK;
+  const Path p = path_of(l, M);
+  RDQ_REQUIRE(l.w_tiled || has_row_major(l), RDQ_E_INVALID, "the layer has neither the tiled nor the row-major tensors");
+  RDQ_REQUIRE(x && y, RDQ_E_INVALID, "x and y must not be null");
+  const Need need = need_of(l, p, M, x_type);
+  RDQ_REQUIRE(need.cast + need.gemm <= workspace_bytes && (need.cast + need.gemm == 0 || (workspace && aligned16(workspace))),
+              RDQ_E_INVALID, "rdq_linear needs %zu bytes of 16-byte aligned workspace for this shape", need.cast + need.gemm);
+  const int bf16 = x_type == RDQ_BF16 ? 1 : 0;
+  bool pdl = (flags & RDQ_GEMV_PDL) != 0;
+  const void *xh = x;
+  int x_bf16 = bf16;
+  if (need.cast) {
+    const int rc = launch_cast_rows(x, workspace, 1ll * M * l.K, pdl, stream);
+    if (rc != RDQ_OK) return rc;
+    xh = workspace;
+    x_bf16 = 0;
+    pdl = true;  // the kernel before is ours and waits for its own predecessor
+  }
+  void *rest = static_cast<char *>(workspace) + need.cast;
+  switch (p) {
+    case Path::kGemvTiled:
+    case Path::kGemvGeneric:
+    case Path::kPanelsTiled:
+    case Path::kPanelsGeneric: {
+      const bool tiled = p == Path::kGemvTiled || p == Path::kPanelsTiled;
+      RDQ_REQUIRE(!tiled || (l.gemv_ws && l.gemv_counters), RDQ_E_INVALID, "the tiled GEMV needs its scratch pair");
+      RDQ_REQUIRE(aligned16(xh) || (!tiled && l.K % 16 != 0), RDQ_E_INVALID, "x must be 16-byte aligned");
+      for (int r0 = 0; r0 < M; r0 += RDQ_MAX_GEMV_M) {
+        const int m = M - r0 < RDQ_MAX_GEMV_M ? M - r0 : RDQ_MAX_GEMV_M;
+        const int rc = run_gemv(l, tiled, static_cast<const char *>(xh) + 2ll * r0 * l.K, x_bf16, m, bias,
+                                static_cast<char *>(y) + 2ll * r0 * N, bf16, pdl, stream);
+        if (rc != RDQ_OK) return rc;
+      }
+      return RDQ_OK;
+    }
+    case Path::kGemm:
+      break;
+  }
+  RDQ_REQUIRE(aligned16(xh) && aligned16(y), RDQ_E_INVALID, "x and y must be 16-byte aligned");
+  RDQ_REQUIRE(1ll * l.n_fp4 * (l.K / 2) < (1ll << 32) && 1ll * l.n_fp8 * l.K < (1ll << 32) && 2ll * l.n_fp16 * l.K < (1ll << 32),
+              RDQ_E_UNSUPPORTED, "a format group of this layer exceeds 4 GB");
+  GemmArgs a;
+  a.x = static_cast<const __half *>(xh);
+  a.M = M;
+  a.w4 = static_cast<const uint8_t *>(l.w_fp4);
+  a.s4 = static_cast<const uint8_t *>(l.w_fp4_scales);
+  a.global4 = l.w_fp4_global_scale;
+  a.w8 = static_cast<const uint8_t *>(l.w_fp8);
+  a.s8 = l.w_fp8_scales;
+  a.w16 = static_cast<const __half *>(l.w_fp16);
+  a.inv_perm = l.inv_perm;
+  a.bias = static_cast<const __half *>(bias);
+  a.y = y;
+  a.n4 = l.n_fp4;
+  a.n8 = l.n_fp8;
+  a.n16 = l.n_fp16;
+  a.K = l.K;
+  a.y_bf16 = bf16;
+  a.ksplit = 1;
+  a.partial = nullptr;
+  return launch_gemm(a, rest, need.gemm, stream);
+}
+
+}  // extern "C"

@@ -1,0 +1,216 @@
+// CPython extension `_rdq_torch`: the per-call host path of a packed layer in native code.
+//
+// A `Layer` object is made once per packed layer from its dict of device tensors and keeps what a
+// call needs (pointers, sizes, references that keep the tensors alive).  Its `linear(x, bias,
+// flags)` checks the input, allocates the output with torch's CUDA allocator, takes torch's current
+// stream and calls rdq_linear (include/rdq_b200.h).  What the fast path does not take -- another
+// dtype, a non-contiguous or host tensor, a wrong last dimension -- returns None, and the caller's
+// Python path handles or refuses it.
+//
+// Why native: a decode step calls dozens of linears whose kernels take 5-10 us, and the same
+// checks, allocation and ctypes call written in Python took 25-33 us per call.
+//
+// Reference counterpart: the pybind wrappers of rdquant/csrc/bindings.cpp:156-201.
+#include <Python.h>
+
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <new>
+#include <vector>
+
+#include "../../include/rdq_b200.h"
+
+namespace {
+
+struct LayerObject {
+  PyObject_HEAD
+  rdq_layer layer;
+  int64_t n_out;
+  c10::DeviceIndex device;
+  std::vector<at::Tensor> *keep;
+};
+
+// makes `device` current while it lives
+struct OnDevice {
+  c10::DeviceIndex prev;
+  bool changed;
+  explicit OnDevice(c10::DeviceIndex device) : prev(c10::cuda::current_device()), changed(prev != device) {
+    if (changed) c10::cuda::set_device(device);
+  }
+  ~OnDevice() {
+    if (changed) c10::cuda::set_device(prev);
+  }
+};
+
+bool take(LayerObject *self, PyObject *dict, const char *key, const void **out) {
+  *out = nullptr;
+  PyObject *v = PyDict_GetItemString(dict, key);  // borrowed
+  if (v == nullptr || v == Py_None) return true;
+  if (!THPVariable_Check(v)) {
+    PyErr_Format(PyExc_TypeError, "%s must be a tensor or None", key);
+    return false;
+  }
+  const at::Tensor &t = THPVariable_Unpack(v);
+  if (!t.is_cuda() || !t.is_contiguous()) {
+    PyErr_Format(PyExc_RuntimeError, "%s must be a contiguous CUDA tensor", key);
+    return false;
+  }
+  if (self->device < 0) self->device = t.get_device();
+  if (t.get_device() != self->device) {
+    PyErr_Format(PyExc_RuntimeError, "%s is on another device than the rest of the layer", key);
+    return false;
+  }
+  *out = t.data_ptr();
+  self->keep->push_back(t);
+  return true;
+}
+
+bool take_int(PyObject *dict, const char *key, int *out) {
+  PyObject *v = PyDict_GetItemString(dict, key);
+  if (v == nullptr) {
+    PyErr_Format(PyExc_KeyError, "%s", key);
+    return false;
+  }
+  *out = static_cast<int>(PyLong_AsLong(v));
+  return !(PyErr_Occurred());
+}
+
+PyObject *layer_new(PyTypeObject *type, PyObject *args, PyObject *) {
+  PyObject *dict = nullptr;
+  if (!PyArg_ParseTuple(args, "O!", &PyDict_Type, &dict)) return nullptr;
+  LayerObject *self = reinterpret_cast<LayerObject *>(type->tp_alloc(type, 0));
+  if (self == nullptr) return nullptr;
+  self->keep = new (std::nothrow) std::vector<at::Tensor>();
+  self->device = -1;
+  rdq_layer &l = self->layer;
+  l = rdq_layer{};
+  const void *s8 = nullptr, *perm = nullptr, *inv = nullptr, *ws = nullptr, *cnt = nullptr;
+  bool ok = self->keep != nullptr && take_int(dict, "n_fp4", &l.n_fp4) && take_int(dict, "n_fp8", &l.n_fp8) &&
+            take_int(dict, "n_fp16", &l.n_fp16) && take_int(dict, "k", &l.K) && take(self, dict, "w_fp4_q", &l.w_fp4) &&
+            take(self, dict, "w_fp4_scales", &l.w_fp4_scales) && take(self, dict, "w_fp8_q", &l.w_fp8) &&
+            take(self, dict, "w_fp8_scales", &s8) && take(self, dict, "w_fp16", &l.w_fp16) &&
+            take(self, dict, "w_tiled", &l.w_tiled) && take(self, dict, "perm", &perm) && take(self, dict, "inv_perm", &inv) &&
+            take(self, dict, "workspace", &ws) && take(self, dict, "tile_counters", &cnt);
+  l.w_fp4_global_scale = 1.0f;
+  if (ok) {
+    if (PyObject *gs = PyDict_GetItemString(dict, "w_fp4_global_scale")) {
+      l.w_fp4_global_scale = static_cast<float>(PyFloat_AsDouble(gs));
+      ok = !PyErr_Occurred();
+    }
+  }
+  if (!ok) {
+    if (!PyErr_Occurred()) PyErr_NoMemory();
+    Py_DECREF(self);
+    return nullptr;
+  }
+  l.w_fp8_scales = static_cast<const float *>(s8);
+  l.perm = static_cast<const int32_t *>(perm);
+  l.inv_perm = static_cast<const int32_t *>(inv);
+  l.gemv_ws = const_cast<void *>(ws);
+  l.gemv_counters = static_cast<int32_t *>(const_cast<void *>(cnt));
+  self->n_out = static_cast<int64_t>(l.n_fp4) + l.n_fp8 + l.n_fp16;
+  return reinterpret_cast<PyObject *>(self);
+}
+
+void layer_dealloc(PyObject *obj) {
+  delete reinterpret_cast<LayerObject *>(obj)->keep;
+  Py_TYPE(obj)->tp_free(obj);
+}
+
+// linear(x, bias or None, flags) -> y, or None when the fast path does not take this input
+PyObject *layer_linear(PyObject *obj, PyObject *const *args, Py_ssize_t nargs) {
+  LayerObject *self = reinterpret_cast<LayerObject *>(obj);
+  if (nargs != 3 || !THPVariable_Check(args[0])) {
+    PyErr_SetString(PyExc_TypeError, "linear(x, bias, flags)");
+    return nullptr;
+  }
+  const rdq_layer &l = self->layer;
+  const at::Tensor &x = THPVariable_Unpack(args[0]);
+  const int64_t dims = x.dim();
+  const auto type = x.scalar_type();
+  if (!x.is_cuda() || x.get_device() != self->device || dims < 1 || x.size(dims - 1) != l.K || !x.is_contiguous() ||
+      (type != at::kHalf && type != at::kBFloat16) || l.K == 0)
+    Py_RETURN_NONE;
+  const int64_t m = x.numel() / l.K;
+  const void *xp = x.data_ptr();
+  if (m == 0 || m > 0x7fffffff || (reinterpret_cast<uintptr_t>(xp) & 15)) Py_RETURN_NONE;
+  const void *bias = nullptr;
+  if (args[1] != Py_None) {
+    if (!THPVariable_Check(args[1])) Py_RETURN_NONE;
+    const at::Tensor &b = THPVariable_Unpack(args[1]);
+    if (!b.is_cuda() || b.get_device() != self->device || b.scalar_type() != at::kHalf || !b.is_contiguous() ||
+        b.numel() != self->n_out)
+      Py_RETURN_NONE;
+    bias = b.data_ptr();
+  }
+  const long flags = PyLong_AsLong(args[2]);
+  if (flags == -1 && PyErr_Occurred()) return nullptr;
+  try {
+    OnDevice guard(self->device);
+    const c10::Device device(c10::kCUDA, self->device);
+    at::Tensor y;
+    if (dims == 2) {
+      const int64_t sizes[2] = {m, self->n_out};
+      y = at::detail::empty_cuda(at::IntArrayRef(sizes, 2), type, device, std::nullopt);
+    } else {
+      std::vector<int64_t> sizes(x.sizes().begin(), x.sizes().end());
+      sizes.back() = self->n_out;
+      y = at::detail::empty_cuda(sizes, type, device, std::nullopt);
+    }
+    const int xt = type == at::kBFloat16 ? RDQ_BF16 : RDQ_F16;
+    size_t need = 0;
+    int rc = rdq_linear_workspace_size(&l, static_cast<int>(m), xt, &need);
+    if (rc == RDQ_OK) {
+      // scratch of this call alone: the allocator orders its reuse behind the work queued here
+      at::Tensor ws;
+      if (need) {
+        const int64_t sizes[1] = {static_cast<int64_t>(need)};
+        ws = at::detail::empty_cuda(at::IntArrayRef(sizes, 1), at::kByte, device, std::nullopt);
+      }
+      rc = rdq_linear(&l, xp, xt, static_cast<int>(m), bias, y.data_ptr(), need ? ws.data_ptr() : nullptr, need,
+                      static_cast<int>(flags), c10::cuda::getCurrentCUDAStream(self->device).stream());
+    }
+    if (rc != RDQ_OK) {
+      PyErr_Format(PyExc_RuntimeError, "rdq_linear failed (code %d): %s", rc, rdq_last_error());
+      return nullptr;
+    }
+    return THPVariable_Wrap(std::move(y));
+  } catch (const std::exception &e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+    return nullptr;
+  }
+}
+
+PyMethodDef layer_methods[] = {
+    {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(layer_linear)), METH_FASTCALL,
+     "linear(x, bias, flags): y = x @ W.T (+ bias), or None when the input needs the checked path"},
+    {nullptr, nullptr, 0, nullptr}};
+
+PyTypeObject layer_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
+
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_rdq_torch", "native host path of the packed layers", -1, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__rdq_torch(void) {
+  layer_type.tp_name = "_rdq_torch.Layer";
+  layer_type.tp_basicsize = sizeof(LayerObject);
+  layer_type.tp_flags = Py_TPFLAGS_DEFAULT;
+  layer_type.tp_new = layer_new;
+  layer_type.tp_dealloc = layer_dealloc;
+  layer_type.tp_methods = layer_methods;
+  layer_type.tp_doc = "Layer(fd): a packed layer ready to be called";
+  if (PyType_Ready(&layer_type) < 0) return nullptr;
+  PyObject *m = PyModule_Create(&module_def);
+  if (m == nullptr) return nullptr;
+  Py_INCREF(&layer_type);
+  if (PyModule_AddObject(m, "Layer", reinterpret_cast<PyObject *>(&layer_type)) < 0) {
+    Py_DECREF(&layer_type);
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
+}

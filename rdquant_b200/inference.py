@@ -15,7 +15,7 @@ from typing import Optional
 import torch
 import torch.nn as nn
 
-from rdquant_b200 import _lib
+from rdquant_b200 import _lib, rdquant_cuda
 from rdquant_b200.fused_gemv_pack import (
     build_marlin_data,
     fused_gemv_available,
@@ -90,11 +90,18 @@ class FusedMixedLinear(nn.Module):
             self._fd_scalars = {kk: v for kk, v in fused_data.items() if kk not in _FD_TENSORS}
         self._fd_cache = None
         self._bias_h = None
+        self._native = None
 
     def _apply(self, fn, recurse=True):
         self._fd_cache = None
         self._bias_h = None
+        self._native = None
         return super()._apply(fn, recurse)
+
+    def __getstate__(self):
+        state = dict(self.__dict__)
+        state["_native"] = state["_fd_cache"] = None  # rebuilt on the next call
+        return state
 
     def _fd(self) -> dict:
         if self._fd_cache is None:
@@ -107,7 +114,24 @@ class FusedMixedLinear(nn.Module):
     def _can_use_fused(self, x_2d: torch.Tensor) -> bool:
         return self._has_fused and x_2d.is_cuda
 
+    def _make_native(self, device) -> None:
+        fd = self._fd()
+        if self.bias is not None:
+            self._bias_h = self.bias.detach().to(device=device, dtype=torch.float16).contiguous()
+        self._native = _lib.torch_ext().Layer(fd)
+
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        # the native path takes contiguous float16 / bfloat16 CUDA rows and answers None otherwise
+        if not rdquant_cuda.VALIDATE:
+            if self._native is None and self._has_fused and x.is_cuda:
+                self._make_native(x.device)
+            if self._native is not None:
+                y = self._native.linear(x, self._bias_h, _lib.RDQ_GEMV_PDL if self.use_pdl else 0)
+                if y is not None:
+                    return y
+        return self._forward_checked(x)
+
+    def _forward_checked(self, x: torch.Tensor) -> torch.Tensor:
         orig_shape = x.shape
         x_2d = x.reshape(-1, self.K)
         if not self._can_use_fused(x_2d):

@@ -12,14 +12,16 @@ from typing import Optional
 
 import torch
 
+from rdquant_b200 import _lib, rdquant_cuda
 from rdquant_b200.core.formats import QuantizedTensor
 
 _PACK_CACHE: "OrderedDict[int, tuple]" = OrderedDict()
 _PACK_CACHE_MAX = 128  # packed layers kept alive for reuse (each entry also pins its qtensors dict)
 
 
-def _packed_for(qtensors: dict, splits: dict, inv_perm: torch.Tensor, device: torch.device) -> dict:
-    """Pack ``qtensors`` once per (dict object, device); later calls reuse the device buffers."""
+def _packed_for(qtensors: dict, splits: dict, inv_perm: torch.Tensor, device: torch.device) -> tuple:
+    """Pack ``qtensors`` once per (dict object, device); later calls reuse the device buffers.
+    Returns (packed dict, native layer)."""
     from rdquant_b200.core.formats import qtensor_to_packed
     from rdquant_b200.fused_gemv_pack import pack_for_fused_gemv
 
@@ -27,7 +29,7 @@ def _packed_for(qtensors: dict, splits: dict, inv_perm: torch.Tensor, device: to
     hit = _PACK_CACHE.get(key)
     if hit is not None and hit[0] is qtensors and hit[1] is inv_perm:
         _PACK_CACHE.move_to_end(key)
-        return hit[2]
+        return hit[2], hit[3]
     layer_data = {"inv_permutation": inv_perm}
     k = None
     for fmt, qt in qtensors.items():
@@ -40,10 +42,11 @@ def _packed_for(qtensors: dict, splits: dict, inv_perm: torch.Tensor, device: to
     fd = pack_for_fused_gemv(layer_data, splits, k, device)
     if fd is None:
         raise RuntimeError("rdquant_b200 kernels unavailable: build librdq_b200.so and run on a CUDA device")
-    _PACK_CACHE[key] = (qtensors, inv_perm, fd)
+    native = _lib.torch_ext().Layer(fd)
+    _PACK_CACHE[key] = (qtensors, inv_perm, fd, native)
     while len(_PACK_CACHE) > _PACK_CACHE_MAX:
         _PACK_CACHE.popitem(last=False)
-    return fd
+    return fd, native
 
 
 def mixed_precision_linear(
@@ -59,11 +62,14 @@ def mixed_precision_linear(
     float16 and the result cast back, as ``FusedMixedLinear`` does,
     rdquant/inference.py:696, :707).
     """
-    from rdquant_b200 import rdquant_cuda
-
     if not x.is_cuda:
         raise RuntimeError("rdquant_b200.ops.mixed_precision_linear runs on CUDA tensors only (no host path)")
-    fd = _packed_for(qtensors, splits, inv_perm, x.device)
+    fd, native = _packed_for(qtensors, splits, inv_perm, x.device)
+    if not rdquant_cuda.VALIDATE:
+        # None: the input needs the conversions and checks below
+        y = native.linear(x, bias, 0)
+        if y is not None:
+            return y
     lead = x.shape[:-1]
     x2 = x.reshape(-1, x.shape[-1])
     xh = x2 if x2.dtype == torch.float16 else x2.to(torch.float16)
