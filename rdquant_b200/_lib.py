@@ -27,13 +27,15 @@ SOURCES = [
     "rdq_gemv_generic.cu",
     "rdq_gemv_tiled.cu",
     "rdq_gemm.cu",
+    "rdq_gemm_dense.cu",
+    "rdq_gemm_stream.cu",
     "rdq_quantize.cu",
     "rdq_stage.cu",
     "rdq_glue.cu",
     "rdq_linear.cu",
 ]
 TORCH_EXT_SOURCE = "rdq_torch.cpp"
-HEADERS = ["rdq_common.cuh", "rdq_kernels.cuh", "rdq_gemv_tiled_kernel.inl", "rdq_gemm_kernel.inl",
+HEADERS = ["rdq_common.cuh", "rdq_gemm_common.cuh", "rdq_kernels.cuh", "rdq_gemv_tiled_kernel.inl", "rdq_gemm_kernel.inl",
            os.path.join("..", "..", "include", "rdq_b200.h")]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

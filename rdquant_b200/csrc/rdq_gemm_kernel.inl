@@ -370,10 +370,6 @@ gemm_mixed_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
   }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
 // y = f16(sum over parts * channel scale + bias) for a split launch
 __global__ void __launch_bounds__(256) gemm_reduce_kernel(const GemmArgs a, int N) {
   const long long total = 1ll * a.M * N;
@@ -456,6 +452,7 @@ namespace {
 std::atomic<int> g_gemm_test_timeout{0};
 }
 
+int gemm_test_timeout() { return g_gemm_test_timeout.load(); }
 void gemm_set_test_timeout(bool on) { g_gemm_test_timeout.store(on ? 1 : 0); }
 
 int gemm_status(bool reset, cudaStream_t stream) {
@@ -472,7 +469,14 @@ int gemm_status(bool reset, cudaStream_t stream) {
   return RDQ_OK;
 }
 
-int launch_gemm(const GemmArgs &a, void *workspace, size_t workspace_bytes, cudaStream_t stream) {
+namespace {
+typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+}
+
+int encode_2d(CUtensorMap *map, CUtensorMapDataType type, int elem_bytes, const void *base, int cols, int rows, int box_cols,
+              int box_rows) {
   static std::atomic<EncodeTiledFn> encode_cached{nullptr};
   EncodeTiledFn encode = encode_cached.load();
   if (!encode) {
@@ -483,34 +487,51 @@ int launch_gemm(const GemmArgs &a, void *workspace, size_t workspace_bytes, cuda
     encode = reinterpret_cast<EncodeTiledFn>(fn);
     encode_cached.store(encode);
   }
-  const int N = a.n4 + a.n8 + a.n16;
-  CUtensorMap xmap;
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(a.K), static_cast<cuuint64_t>(a.M)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(a.K) * 2};
-  const cuuint32_t box[2] = {BK, BM};
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * elem_bytes};
+  const cuuint32_t box[2] = {static_cast<cuuint32_t>(box_cols), static_cast<cuuint32_t>(box_rows)};
   const cuuint32_t estr[2] = {1, 1};
-  const CUresult rc = encode(&xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half *>(a.x), dims, strides, box, estr,
-                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+  const CUresult rc = encode(map, type, 2, const_cast<void *>(base), dims, strides, box, estr,
+                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   RDQ_REQUIRE(rc == CUDA_SUCCESS, RDQ_E_CUDA, "cuTensorMapEncodeTiled failed with code %d", static_cast<int>(rc));
-  // the largest tile that still gives every SM a CTA: 256 tokens x 256 channels, 256 x 128, 128 x 128
+  return RDQ_OK;
+}
+
+// device address of the status word on the current device
+int gemm_status_ptr(int **out) {
+  static std::atomic<int *> cached[64];
+  int dev = 0;
+  RDQ_CUDA(cudaGetDevice(&dev));
+  int *p = dev >= 0 && dev < 64 ? cached[dev].load() : nullptr;
+  if (!p) {
+    void *v = nullptr;
+    RDQ_CUDA(cudaGetSymbolAddress(&v, g_gemm_status));
+    p = static_cast<int *>(v);
+    if (dev >= 0 && dev < 64) cached[dev].store(p);
+  }
+  *out = p;
+  return RDQ_OK;
+}
+
+size_t gemm_workspace_bytes(int M, int N, int K) { return gemm_dense_takes(K) ? gemm_dense_workspace(M, N, K) : 0; }
+
+int launch_gemm(const GemmArgs &a, void *workspace, size_t workspace_bytes, cudaStream_t stream) {
+  const int N = a.n4 + a.n8 + a.n16;
   GemmArgs b = a;
+  b.test_timeout = gemm_test_timeout();
+  if (workspace != nullptr && gemm_dense_takes(a.K) && workspace_bytes >= gemm_dense_workspace(a.M, N, a.K))
+    return launch_gemm_dense(b, workspace, workspace_bytes, stream);
+  RDQ_REQUIRE(a.K % 64 == 0, RDQ_E_UNSUPPORTED, "the GEMM without a workspace needs K to be a multiple of 64, got K=%d", a.K);
+  CUtensorMap xmap;
+  const int rc = encode_f16_2d(&xmap, a.x, a.K, a.M, BK, BM);
+  if (rc != RDQ_OK) return rc;
   const GemmPlan plan = gemm_plan(a.M, N, a.K);
   b.ksplit = 1;
   b.partial = nullptr;
-  b.test_timeout = g_gemm_test_timeout.load();
-  if (plan.ksplit > 1 && workspace != nullptr && workspace_bytes >= sizeof(float) * plan.ksplit * a.M * N) {
-    b.ksplit = plan.ksplit;
-    b.partial = static_cast<float *>(workspace);
-  }
   if (plan.cfg == 2) return launch_cfg<2, 256>(xmap, b, N, stream);
   if (plan.cfg == 1) return launch_cfg<2, 128>(xmap, b, N, stream);
   return launch_cfg<1, 128>(xmap, b, N, stream);
-}
-
-size_t gemm_workspace_bytes(int M, int N, int K) {
-  const GemmPlan plan = gemm_plan(M, N, K);
-  return plan.ksplit > 1 ? sizeof(float) * plan.ksplit * M * N : 0;
 }
 
 }  // namespace rdq

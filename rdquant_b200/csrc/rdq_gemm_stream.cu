@@ -1,0 +1,755 @@
+// Weight-streaming GEMM for a few dozen to a few hundred activation rows: packed weights go from
+// shared memory through the format converters straight into TENSOR MEMORY, where tcgen05.mma takes
+// them as its first operand.
+//
+//   y[M, N] = x[M, K] . W[N, K]^T * scale (+ bias)
+//
+// Bound: HBM (packed weight bytes) up to about a hundred rows, the tensor pipe and the activation
+// traffic above.  Weights are the rows of the MMA (128 permuted rows of ONE format per tile) and
+// tokens its columns (a multiple of 16 up to 128), so few rows cost few tensor cycles, and the
+// converted weights never pass through shared memory: a converter thread owns one weight row, reads
+// its packed bytes with conflict-free 16-byte loads and writes them as tensor-memory columns.
+//
+// Work: every tile is a run of 16 KB chunks (128 rows x 128 packed bytes = 256 / 128 / 64 k of
+// NVFP4 / FP8 / FP16), all chunks of the layer are numbered in tile order and each CTA takes a
+// contiguous range of equal cost (make_plan).  A tile inside one range is finished by its CTA.  The
+// CTAs that share a tile cut by range borders leave FP32 partial sums in the workspace, wait
+// (bounded) until all parts of the tile are there, and each adds and stores a share of its tokens,
+// parts in CTA order: the result does not depend on timing.  A second kernel for these sums cost
+// 4-7 us per layer, and one CTA per tile adding them up to 13 us.
+//
+// A stage of the pipeline is 128 k: 64 tensor-memory columns of weights and two 64-k activation
+// boxes, on one barrier.  The issuing warp spends about 190 cycles per barrier wait and 40 per MMA
+// whatever the number of tokens, so with 64-k stages and a barrier per operand it took 640 cycles per
+// 64 k; a CTA's share of the HBM rate asks for 64 k every 250.
+//
+// Roles of a CTA's warps:
+//   0        TMA of weight chunks (128 x 128 B boxes out of the row-major tensors, 128B swizzle)
+//   1        TMA of activation boxes (tokens x 64 k); executes griddepcontrol.wait
+//   2        MMA issue; tensor-memory allocation
+//   3        block scales of NVFP4 chunks by cp.async, on the chunk's barrier
+//   4-7      epilogue: tcgen05.ld, channel scale + bias, stores to y[token, perm[row]]
+//   8-15     converters, two groups of four warps (a warp per 32 tensor-memory lanes) taking chunks in
+//            turn (four groups are no faster)
+// Every launch is programmatic: it overlaps the end of the kernel before.  With RDQ_GEMV_PDL the
+// weight and scale loads start before the grid-dependency wait, so that the rings fill meanwhile.  The variant for up to 32 tokens takes half an SM
+// (256 tensor-memory columns, 64 registers, about 110 KB), so that the next layer's CTA fits beside it.
+//
+// Reference behaviour replaced: 2 x marlin_gemm + F.linear + cat + index_select
+// (rdquant/inference.py:620-677).
+#include <cuda.h>
+
+#include <algorithm>
+#include <unordered_map>
+
+#include "rdq_gemm_common.cuh"
+#include "rdq_kernels.cuh"
+
+namespace rdq {
+
+namespace {
+
+constexpr int kGroups = 2;  // converter groups
+constexpr int kThreads = (8 + 4 * kGroups) * 32;
+constexpr int kChunkBytes = 128 * 128;
+constexpr int kScaleBytes = 128 * 16;
+constexpr int kMaxRing = 16;
+constexpr int kMaxTokens = 128;   // per token tile
+constexpr int kMaxCtas = 160;
+
+// Chunks of the layer in processing order: NVFP4 tiles, FP8 tiles, FP16 tiles; inside a channel tile
+// its token tiles one after another.
+struct StreamSched {
+  int mt, nt, M;            // token tiles, tokens per tile
+  int S[3];                 // chunks per tile
+  int E[3];                 // end of each format's chunk range
+  int nkb;                  // k blocks of 64
+  int G;                    // CTAs
+  int bnd[kMaxCtas + 1];    // first chunk of each CTA
+};
+struct Segment {
+  int fmt, row_tile, m_tile;  // 128-row tile inside the format group, token tile
+  int c0, c1;                 // chunks of the tile
+  int start;                  // global index of the tile's first chunk
+};
+__device__ __forceinline__ Segment segment_at(const StreamSched &s, int chunk, int end) {
+  Segment g;
+  g.fmt = chunk < s.E[0] ? 0 : (chunk < s.E[1] ? 1 : 2);
+  const int base = g.fmt == 0 ? 0 : s.E[g.fmt - 1];
+  const int S = s.S[g.fmt];
+  const int t = (chunk - base) / S;
+  g.start = base + t * S;
+  g.row_tile = t / s.mt;
+  g.m_tile = t - g.row_tile * s.mt;
+  g.c0 = chunk - g.start;
+  g.c1 = min(S, end - g.start);
+  return g;
+}
+
+struct StreamArgs {
+  const uint8_t *s4;
+  const float *s8;
+  float global4;
+  const int32_t *perm;
+  const __half *bias;
+  void *y;
+  int y_bf16;
+  int n4, n8, n16, K, N;
+  float *partial;    // [2 * CTA + (0 first, 1 last segment)][token][128 rows]
+  uint32_t *arrived;  // [CTA in which a cut tile starts]: epilogue warps done (low half), CTAs past the wait (high half)
+  int nw;             // weight chunks in flight
+  int early;          // weights may be read before the kernel before this one has finished
+  int scale16;     // block-scale rows can be copied 16 bytes at a time
+  int test_timeout;
+};
+
+struct StreamSmem {
+  uint64_t w_full[kMaxRing], w_empty[kMaxRing];
+  uint64_t full[4], empty[4];
+  uint64_t d_full[2], d_empty[2];
+  uint64_t never;
+  uint32_t tmem_base;
+  int abort_flag;
+};
+
+// position in a ring
+// the CTAs that hold a cut tile: `from` holds its start
+__device__ __forceinline__ int first_cta(const StreamSched &s, int b, int tile_start) {
+  while (s.bnd[b] > tile_start) --b;
+  return b;
+}
+__device__ __forceinline__ int last_cta(const StreamSched &s, int b, int tile_end) {
+  while (s.bnd[b + 1] < tile_end) ++b;
+  return b;
+}
+// workspace slot of CTA c's part of the tile that starts in CTA `from`: a range's first segment goes
+// to the even slot, its last to the odd one
+__device__ __forceinline__ long long part_slot(const StreamSched &s, int c, int from, int tile_start) {
+  return 2ll * c + (c == from && s.bnd[c] < tile_start ? 1 : 0);
+}
+
+struct Cursor {
+  int i = 0;
+  uint32_t ph = 0;
+  __device__ __forceinline__ void next(int n) {
+    if (++i == n) {
+      i = 0;
+      ph ^= 1;
+    }
+  }
+};
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ uint4 lds16(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+// 16 tensor-memory columns (32 k) of this warp's 32 lanes
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+// D (+)= A(tensor memory) . B(smem)^T
+__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// half a k block (32 k) of one weight row -> 16 tensor-memory columns
+__device__ __forceinline__ void convert_fp4(const uint4 &q, uint32_t scales, uint32_t (&o)[16]) {
+  const uint32_t s2 = cvt_e4m3x2(scales);
+  const uint32_t s0 = __byte_perm(s2, 0u, 0x1010u), s1 = __byte_perm(s2, 0u, 0x3232u);
+  cvt_e2m1x8(q.x, o[0], o[1], o[2], o[3]);
+  cvt_e2m1x8(q.y, o[4], o[5], o[6], o[7]);
+  cvt_e2m1x8(q.z, o[8], o[9], o[10], o[11]);
+  cvt_e2m1x8(q.w, o[12], o[13], o[14], o[15]);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    o[i] = hmul2_u32(o[i], s0);
+    o[8 + i] = hmul2_u32(o[8 + i], s1);
+  }
+}
+__device__ __forceinline__ void convert_fp8(const uint4 &a, const uint4 &b, uint32_t (&o)[16]) {
+  cvt_e4m3x4(a.x, o[0], o[1]);
+  cvt_e4m3x4(a.y, o[2], o[3]);
+  cvt_e4m3x4(a.z, o[4], o[5]);
+  cvt_e4m3x4(a.w, o[6], o[7]);
+  cvt_e4m3x4(b.x, o[8], o[9]);
+  cvt_e4m3x4(b.y, o[10], o[11]);
+  cvt_e4m3x4(b.z, o[12], o[13]);
+  cvt_e4m3x4(b.w, o[14], o[15]);
+}
+
+// output column, scale and bias of row r of a segment's tile
+struct Row {
+  bool live;
+  int col;
+  float scl, bia;
+};
+__device__ __forceinline__ Row row_of(const StreamArgs &a, const Segment &g, int r, bool wanted) {
+  Row w;
+  const int row = g.row_tile * 128 + r;  // row inside the format group
+  const int rows = g.fmt == 0 ? a.n4 : (g.fmt == 1 ? a.n8 : a.n16);
+  const int prow = row + (g.fmt == 0 ? 0 : (g.fmt == 1 ? a.n4 : a.n4 + a.n8));
+  w.live = row < rows;
+  w.col = 0;
+  w.scl = 0.f;
+  w.bia = 0.f;
+  if (w.live && wanted) {
+    w.col = a.perm ? a.perm[prow] : prow;
+    w.scl = g.fmt == 0 ? a.global4 : (g.fmt == 1 ? a.s8[row] : 1.f);
+    w.bia = a.bias ? __half2float(a.bias[w.col]) : 0.f;
+  }
+  return w;
+}
+
+// Half of the CTA's threads: waits until all parts of the segment's tile are in the workspace, then
+// adds and stores this CTA's share of its tokens.  `sub` (0, 1) and r (row) identify the thread.
+// With `dry` nothing is read, awaited or stored.
+__device__ __forceinline__ void finish_shared(const StreamArgs &a, const StreamSched &sc, const Segment &g, int r, int sub,
+                                              int bar_id, bool dry, volatile int *abort_flag) {
+  const int b0 = first_cta(sc, blockIdx.x, g.start), b1 = last_cta(sc, blockIdx.x, g.start + sc.S[g.fmt]);
+  const int parts = b1 - b0 + 1;
+  const Row row = row_of(a, g, r, true);
+  const int tok0 = g.m_tile * sc.nt;
+  const int ntok = min(sc.nt, sc.M - tok0);
+  const int lo = ntok * (static_cast<int>(blockIdx.x) - b0) / parts;
+  const int hi = dry ? lo : ntok * (static_cast<int>(blockIdx.x) + 1 - b0) / parts;
+  if (r == 0 && sub == 0 && !dry && !wait_arrivals(a.arrived + b0, 4u * parts, parts)) *abort_flag = 1;
+  if (!dry) {
+    asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "n"(kThreads / 2) : "memory");
+    if (*abort_flag) return;
+  }
+  constexpr int kTok = 8, kSub = 2;
+#pragma unroll 1
+  for (int t0 = lo + sub; t0 < hi || (dry && t0 == lo + sub); t0 += kTok * kSub) {
+    float v[kTok];
+#pragma unroll
+    for (int e = 0; e < kTok; ++e) v[e] = 0.f;
+#pragma unroll 1
+    for (int b = b0; b <= b1; b += 2) {
+      // two parts' loads in flight
+      const float *s0 = a.partial + (part_slot(sc, b, b0, g.start) * sc.nt + t0) * 128 + r;
+      const float *s1 = a.partial + (part_slot(sc, min(b + 1, b1), b0, g.start) * sc.nt + t0) * 128 + r;
+      float p0[kTok], p1[kTok];
+#pragma unroll
+      for (int e = 0; e < kTok; ++e) {
+        p0[e] = t0 + e * kSub < hi ? __ldcg(s0 + e * kSub * 128) : 0.f;
+        p1[e] = t0 + e * kSub < hi && b < b1 ? __ldcg(s1 + e * kSub * 128) : 0.f;
+      }
+#pragma unroll
+      for (int e = 0; e < kTok; ++e) v[e] = (v[e] + p0[e]) + p1[e];
+    }
+    if (row.live) {
+#pragma unroll
+      for (int e = 0; e < kTok; ++e)
+        if (t0 + e * kSub < hi)
+          store_y(a.y, 1ll * (tok0 + t0 + e * kSub) * a.N + row.col, fmaf(v[e], row.scl, row.bia), a.y_bf16);
+    }
+  }
+}
+
+// COLS: tensor-memory columns of the CTA.  512: two accumulators of 128 columns and four weight
+// stages of 64; 256: two of 32 and three, for two CTAs per SM.
+template <int COLS>
+__global__ void __launch_bounds__(kThreads, COLS == 256 ? 2 : 1)
+gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_constant__ CUtensorMap w8map,
+                   const __grid_constant__ CUtensorMap w16map, const __grid_constant__ CUtensorMap xmap,
+                   const __grid_constant__ StreamArgs a, const __grid_constant__ StreamSched sc, int *status) {
+  constexpr int NS = COLS == 256 ? 3 : 4;       // stages
+  constexpr int kAcc = COLS == 256 ? 32 : 128;  // columns of an accumulator
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ StreamSmem S;
+  const uint32_t w_ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t x_ring = w_ring + a.nw * kChunkBytes;
+  const uint32_t x_bytes = static_cast<uint32_t>(sc.nt) * 128;  // one 64-k box
+  const uint32_t s_ring = x_ring + NS * 2 * x_bytes;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int begin = sc.bnd[blockIdx.x], end = sc.bnd[blockIdx.x + 1];
+  auto load_chunk = [&](const Segment &g, int c, int slot) {
+    const uint32_t bar = smem_u32(&S.w_full[slot]);
+    mbar_arrive_expect_tx(bar, kChunkBytes);
+    tma_load_2d(w_ring + slot * kChunkBytes, g.fmt == 0 ? &w4map : (g.fmt == 1 ? &w8map : &w16map),
+                c * (g.fmt == 2 ? 64 : 128), g.row_tile * 128, bar);
+  };
+  // Without leave to read weights early every thread waits for the kernel before this one here; the
+  // launch itself and the instruction fetch still overlap it.
+  if (!a.early) pdl_wait();
+  // The first weight chunks are on their way before anything else is set up.
+  const int early = min(a.nw, end - begin);
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < a.nw; ++i) {
+      mbar_init(smem_u32(&S.w_full[i]), 1 + 32);  // the TMA thread and the scale warp's lanes
+      mbar_init(smem_u32(&S.w_empty[i]), 4);  // the group that converts the chunk
+    }
+    mbar_init_fence();
+    Segment g = segment_at(sc, begin, end);
+    for (int i = 0; i < early; ++i) {
+      if (begin + i == g.start + g.c1) g = segment_at(sc, begin + i, end);
+      load_chunk(g, begin + i - g.start, i);
+    }
+  }
+  // Kernel parameters are read through the constant cache, whose misses would otherwise follow one
+  // another in every role: each warp touches another part of them first.
+  {
+    constexpr int kWords = (sizeof(StreamSched) - kMaxCtas * 4) / 4;
+    const int w0 = reinterpret_cast<const int *>(&sc)[min(warp * 16, kWords)];
+    const int w1 = reinterpret_cast<const int *>(&a)[min(warp * 16, static_cast<int>(sizeof(StreamArgs) / 4) - 1)];
+    asm volatile("" ::"r"(w0), "r"(w1));
+  }
+  if (threadIdx.x == 32) {
+    for (int i = 0; i < NS; ++i) {
+      mbar_init(smem_u32(&S.full[i]), 1 + 4);  // the activation loads and four converter warps
+      mbar_init(smem_u32(&S.empty[i]), 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(smem_u32(&S.d_full[i]), 1);
+      mbar_init(smem_u32(&S.d_empty[i]), 4);
+    }
+    mbar_init(smem_u32(&S.never), 1);
+    S.abort_flag = 0;
+    mbar_init_fence();
+  }
+  if (warp == 2) tmem_alloc(smem_u32(&S.tmem_base), COLS);
+  if (warp == 3 && lane < 4) prefetch_tensormap(lane == 0 ? &w4map : (lane == 1 ? &w8map : (lane == 2 ? &w16map : &xmap)));
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = S.tmem_base;
+  const uint32_t tmem_a = tmem + 2 * kAcc;
+  pdl_launch_dependents();
+
+  // Code that runs once per launch runs out of a cold instruction cache (about 45 ns per instruction
+  // measured): the epilogue warps, which have nothing to do at first, go through the code that ends
+  // the kernel once without effect while the others stream.
+  bool dry = warp >= 4 && warp < 8;
+#pragma unroll 1
+  for (int pass = dry ? 0 : 1; pass < 2; ++pass, dry = false) {
+  if (dry) {
+  } else if (warp == 0) {
+    // ---------------------------------------------------------------- weight chunks
+    const bool leader = elect_one();
+    Cursor w;
+    if (early == a.nw) w.ph ^= 1;
+    else w.i = early;
+    bool alive = true;
+    for (int ck = begin + early; ck < end && alive;) {
+      const Segment g = segment_at(sc, ck, end);
+      for (int c = g.c0; c < g.c1; ++c) {
+        alive = gemm_wait(&S.w_empty[w.i], w.ph ^ 1, &S.abort_flag);
+        if (!alive) break;
+        if (leader) load_chunk(g, c, w.i);
+        w.next(a.nw);
+      }
+      ck = g.start + g.c1;
+    }
+  } else if (warp == 1) {
+    // ---------------------------------------------------------------- activation boxes
+    const bool leader = elect_one();
+    pdl_wait();
+    Cursor x;
+    bool alive = true;
+    for (int ck = begin; ck < end && alive;) {
+      const Segment g = segment_at(sc, ck, end);
+      const int per = 4 >> g.fmt;  // k blocks of 64 per chunk
+      const int kb1 = min(g.c1 * per, sc.nkb), step = min(per, 2);
+      for (int kb = g.c0 * per; kb < kb1; kb += step) {
+        alive = gemm_wait(&S.empty[x.i], x.ph ^ 1, &S.abort_flag);
+        if (!alive) break;
+        if (leader) {
+          const uint32_t bar = smem_u32(&S.full[x.i]);
+          const uint32_t dst = x_ring + x.i * 2 * x_bytes;
+          const bool two = step == 2 && kb + 1 < kb1;
+          mbar_arrive_expect_tx(bar, two ? 2 * x_bytes : x_bytes);
+          tma_load_2d(dst, &xmap, kb * 64, g.m_tile * sc.nt, bar);
+          if (two) tma_load_2d(dst + x_bytes, &xmap, (kb + 1) * 64, g.m_tile * sc.nt, bar);
+        }
+        x.next(NS);
+      }
+      ck = g.start + g.c1;
+    }
+  } else if (warp == 2) {
+    // ---------------------------------------------------------------- MMA issue
+    const bool leader = elect_one();
+    const uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(sc.nt >> 3) << 17) | (8u << 24);
+    Cursor x, d;
+    bool alive = true;
+    for (int ck = begin; ck < end && alive;) {
+      const Segment g = segment_at(sc, ck, end);
+      const int per = 4 >> g.fmt;
+      const int kb0 = g.c0 * per, kb1 = min(g.c1 * per, sc.nkb), step = min(per, 2);
+      alive = gemm_wait(&S.d_empty[d.i], d.ph ^ 1, &S.abort_flag);
+      if (!alive) break;
+      tc_fence_after();
+      const uint32_t acc = tmem + d.i * kAcc;
+      for (int kb = kb0; kb < kb1; kb += step) {
+        alive = gemm_wait(&S.full[x.i], x.ph, &S.abort_flag);
+        if (!alive) break;
+        tc_fence_after();
+        const uint64_t dx = make_desc_sw128(x_ring + x.i * 2 * x_bytes);
+        const uint32_t wa = tmem_a + x.i * 64;
+        if (leader) {
+#pragma unroll
+          for (int k4 = 0; k4 < 4; ++k4) umma_f16_ts(acc, wa + 8 * k4, dx + 2 * k4, idesc, (kb != kb0 || k4 != 0) ? 1u : 0u);
+          if (step == 2 && kb + 1 < kb1) {
+            const uint64_t dx2 = dx + (x_bytes >> 4);
+#pragma unroll
+            for (int k4 = 0; k4 < 4; ++k4) umma_f16_ts(acc, wa + 32 + 8 * k4, dx2 + 2 * k4, idesc, 1u);
+          }
+          umma_commit(smem_u32(&S.empty[x.i]));
+        }
+        x.next(NS);
+      }
+      if (alive && leader) umma_commit(smem_u32(&S.d_full[d.i]));
+      d.next(2);
+      ck = g.start + g.c1;
+    }
+    __syncwarp();
+  } else if (warp == 3) {
+    // ------------------------------------------------------------------ block scales
+    Cursor w;
+    bool alive = true;
+    const int pitch = a.K >> 4;
+    for (int ck = begin; ck < end && alive;) {
+      const Segment g = segment_at(sc, ck, end);
+      for (int c = g.c0; c < g.c1; ++c) {
+        alive = gemm_wait(&S.w_empty[w.i], w.ph ^ 1, &S.abort_flag);
+        if (!alive) break;
+        if (g.fmt == 0) {
+          const uint32_t dst = s_ring + w.i * kScaleBytes;
+          const int words = min(4, sc.nkb - 4 * c);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int r = i * 32 + lane;
+            const uint8_t *src = a.s4 + 1ll * min(g.row_tile * 128 + r, a.n4 - 1) * pitch + c * 16;
+            if (a.scale16) {
+              cp_async16(dst + r * 16, src);
+            } else {
+              for (int j = 0; j < words; ++j) cp_async4(dst + r * 16 + 4 * j, src + 4 * j);
+            }
+          }
+        }
+        cp_async_arrive(smem_u32(&S.w_full[w.i]));
+        w.next(a.nw);
+      }
+      ck = g.start + g.c1;
+    }
+  } else if (warp < 8) {
+    // ------------------------------------------------------------------ epilogue
+    const int q = warp & 3;
+    const uint32_t lanes = static_cast<uint32_t>(q * 32) << 16;
+    Cursor d;
+    bool first = true;
+    for (int ck = begin; ck < end;) {
+      const Segment g = segment_at(sc, ck, end);
+      const bool whole = g.c0 == 0 && g.c1 == sc.S[g.fmt];
+      const Row row = row_of(a, g, q * 32 + lane, whole);
+      const int tok0 = g.m_tile * sc.nt;
+      const int ntok = min(sc.nt, sc.M - tok0);
+      if (!gemm_wait(&S.d_full[d.i], d.ph, &S.abort_flag)) break;
+      tc_fence_after();
+      const uint32_t acc = tmem + d.i * kAcc + lanes;
+      float *part = a.partial + (2ll * blockIdx.x + (first ? 0 : 1)) * sc.nt * 128 + q * 32 + lane;
+      for (int c = 0; c < ntok; c += 16) {
+        uint32_t v[16];
+        tmem_ld16(acc + c, v);
+        tmem_wait_ld();
+        if (c + 16 >= ntok) {  // the accumulator is free once its last columns are read
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&S.d_empty[d.i]));
+        }
+        if (!whole) {
+#pragma unroll
+          for (int e = 0; e < 16; ++e)
+            if (c + e < ntok) part[(c + e) * 128] = __uint_as_float(v[e]);
+        } else if (row.live) {
+#pragma unroll
+          for (int e = 0; e < 16; ++e)
+            if (c + e < ntok)
+              store_y(a.y, 1ll * (tok0 + c + e) * a.N + row.col, fmaf(__uint_as_float(v[e]), row.scl, row.bia), a.y_bf16);
+        }
+      }
+      if (!whole) {
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) arrive_global(a.arrived + first_cta(sc, blockIdx.x, g.start));
+      }
+      first = false;
+      d.next(2);
+      ck = g.start + g.c1;
+    }
+  } else {
+    // ------------------------------------------------------------------ converters
+    const int q = warp & 3, grp = (warp - 8) >> 2;
+    const int row = q * 32 + lane;
+    const uint32_t lanes = static_cast<uint32_t>(q * 32) << 16;
+    const uint32_t rbase = row * 128, sw = row & 7;
+    auto piece = [&](uint32_t base, int p) { return base + rbase + ((p ^ sw) << 4); };
+    Cursor w, s;
+    // A group takes every second chunk: its own stage before was at most three stages back, so when it
+    // waits for the release of stage i - NS it has seen that of stage i - 3 - NS, and with NS >= 3 the
+    // parity it tests cannot be two rounds old.  Likewise for the chunk barriers: what it converted
+    // last lies behind every chunk whose slot it could confuse, as long as nw >= 3.
+    static_assert(kGroups == 2 && NS >= 3, "a stage barrier could be tested two rounds late");
+    int turn = 0;
+    bool alive = true;
+    for (int ck = begin; ck < end && alive;) {
+      const Segment g = segment_at(sc, ck, end);
+      const int per = 4 >> g.fmt;
+      for (int c = g.c0; c < g.c1; ++c, turn ^= 1, w.next(a.nw)) {
+        const int nb = min(per, sc.nkb - c * per);
+        if (turn != grp) {
+          for (int b = 0; b < nb; b += 2) s.next(NS);
+          continue;
+        }
+        alive = gemm_wait(&S.w_full[w.i], w.ph, &S.abort_flag);
+        if (!alive) break;
+        const uint32_t base = w_ring + w.i * kChunkBytes;
+        for (int b = 0; b < nb; b += 2) {
+          alive = gemm_wait(&S.empty[s.i], s.ph ^ 1, &S.abort_flag);
+          if (!alive) break;
+          tc_fence_after();
+          const uint32_t dst = tmem_a + s.i * 64 + lanes;
+          uint32_t o[16];
+          if (g.fmt == 0) {
+            // (a trailing odd block converts the zero fill of the box; the MMAs do not read it)
+            uint32_t s0, s1;
+            asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(s0), "=r"(s1) : "r"(s_ring + w.i * kScaleBytes + row * 16 + b * 4) : "memory");
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+              convert_fp4(lds16(piece(base, 2 * b + h)), (h < 2 ? s0 : s1) >> (16 * (h & 1)), o);
+              tmem_st16(dst + 16 * h, o);
+            }
+          } else if (g.fmt == 1) {
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+              convert_fp8(lds16(piece(base, 2 * h)), lds16(piece(base, 2 * h + 1)), o);
+              tmem_st16(dst + 16 * h, o);
+            }
+          } else {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+#pragma unroll
+              for (int p = 0; p < 4; ++p) {
+                const uint4 v = lds16(piece(base, 4 * h + p));
+                o[4 * p] = v.x;
+                o[4 * p + 1] = v.y;
+                o[4 * p + 2] = v.z;
+                o[4 * p + 3] = v.w;
+              }
+              tmem_st16(dst + 16 * h, o);
+            }
+          }
+          tmem_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&S.full[s.i]));
+          s.next(NS);
+        }
+        if (!alive) break;
+        if (lane == 0) mbar_arrive(smem_u32(&S.w_empty[w.i]));
+      }
+      ck = g.start + g.c1;
+    }
+  }
+
+  __syncwarp();
+  if (!dry) {
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 2) tmem_dealloc(tmem, COLS);
+  }
+  // ---- tiles shared with other CTAs: half of the threads take the range's first segment, half its last
+  if ((dry || !S.abort_flag) && begin < end) {
+    const int half = threadIdx.x >> 8;
+    Segment g = segment_at(sc, begin, end);
+    bool mine = half == 0;
+    if (half == 1 && g.start + g.c1 < end) {
+      mine = true;
+      g = segment_at(sc, end - 1, end);
+      g = segment_at(sc, max(g.start, begin), end);
+    }
+    if (dry || (mine && !(g.c0 == 0 && g.c1 == sc.S[g.fmt])))
+      finish_shared(a, sc, g, threadIdx.x & 127, (threadIdx.x >> 7) & 1, 1 + half, dry, &S.abort_flag);
+  }
+  }  // pass
+  __syncthreads();
+  if (S.abort_flag) {
+    linger(16000);  // let copies that are still in flight land before the shared memory is given up
+    __syncthreads();
+    if (threadIdx.x == 0) atomicExch(status, 1);
+  }
+  if (a.test_timeout && threadIdx.x == 0 && blockIdx.x == 0) {
+    if (!mbar_wait(smem_u32(&S.never), 0, 3u)) atomicExch(status, 2);
+  }
+}
+
+struct StreamPlan {
+  StreamSched sc;
+  int cols, nw, smem;
+};
+
+// Token tiles of equal width; a chunk costs what bounds it: its bytes at the SM's share of the HBM
+// rate (23 B/clk), the conversion of its k blocks, or their tensor time.
+StreamPlan make_plan(int n4, int n8, int n16, int M, int K) {
+  StreamPlan p;
+  StreamSched &s = p.sc;
+  s.M = M;
+  s.mt = (M + kMaxTokens - 1) / kMaxTokens;
+  s.nt = ((M + s.mt - 1) / s.mt + 15) / 16 * 16;
+  s.nkb = (K + 63) / 64;
+  const int n[3] = {n4, n8, n16};
+  const double bytes[3] = {kChunkBytes + kScaleBytes, kChunkBytes, kChunkBytes};
+  int e = 0, u[3];
+  long long w = 0, W[3];
+  for (int f = 0; f < 3; ++f) {
+    const int per = 4 >> f;
+    s.S[f] = (s.nkb + per - 1) / per;
+    const double conv = f == 0 ? 170 : (f == 1 ? 150 : 90);
+    u[f] = static_cast<int>(std::max(bytes[f] / 23.0, per * std::max(conv, 2.0 * s.nt)));
+    const int chunks = (n[f] + 127) / 128 * s.mt * s.S[f];
+    e += chunks;
+    w += 1ll * chunks * u[f];
+    s.E[f] = e;
+    W[f] = w;
+  }
+  // every CTA gets at least one chunk: its share is not below the most expensive one
+  s.G = static_cast<int>(std::min<long long>(std::min(sm_count(), kMaxCtas), std::max(1ll, w / std::max({u[0], u[1], u[2]}))));
+  for (int b = 0; b < s.G; ++b) {
+    const long long pos = w * b / s.G;
+    s.bnd[b] = static_cast<int>(pos < W[0] ? pos / u[0]
+                                           : (pos < W[1] ? s.E[0] + (pos - W[0]) / u[1] : s.E[1] + (pos - W[1]) / u[2]));
+  }
+  s.bnd[s.G] = e;
+  p.cols = s.nt <= 32 ? 256 : 512;
+  const int xb = (p.cols == 256 ? 3 : 4) * 2 * s.nt * 128;
+  p.nw = std::min(8, ((p.cols == 256 ? 108 : 220) * 1024 - 1024 - xb) / (kChunkBytes + kScaleBytes));
+  p.smem = 1024 + xb + p.nw * (kChunkBytes + kScaleBytes);
+  return p;
+}
+
+// the plans of the last few thousand (layer shape, rows) pairs of this thread
+const StreamPlan &stream_plan(int n4, int n8, int n16, int M, int K) {
+  struct Key {
+    int v[6];
+    bool operator==(const Key &o) const { return std::equal(v, v + 6, o.v); }
+  };
+  struct Hash {
+    size_t operator()(const Key &k) const {
+      size_t h = 1469598103934665603ull;
+      for (int x : k.v) h = (h ^ static_cast<size_t>(x)) * 1099511628211ull;
+      return h;
+    }
+  };
+  static thread_local std::unordered_map<Key, StreamPlan, Hash> plans;
+  const Key key{{n4, n8, n16, M, K, sm_count()}};
+  auto it = plans.find(key);
+  if (it == plans.end()) {
+    if (plans.size() >= 4096) plans.clear();
+    it = plans.emplace(key, make_plan(n4, n8, n16, M, K)).first;
+  }
+  return it->second;
+}
+
+int encode_u8_2d(CUtensorMap *map, const void *base, int cols, int rows) {
+  return encode_2d(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, base, cols, rows, 128, 128);
+}
+
+}  // namespace
+
+// 16-byte row pitches for TMA, whole 4-byte groups of block scales
+bool gemm_stream_takes(int K) { return K % 64 == 0; }
+
+size_t gemm_stream_workspace(int M, int K) {
+  (void)K;
+  const int mt = (M + kMaxTokens - 1) / kMaxTokens, nt = ((M + mt - 1) / mt + 15) / 16 * 16;
+  return 2ull * std::min(sm_count(), kMaxCtas) * nt * 128 * sizeof(float);
+}
+
+int launch_gemm_stream(const GemmArgs &g, void *workspace, size_t workspace_bytes, bool pdl, cudaStream_t stream) {
+  const StreamPlan &p = stream_plan(g.n4, g.n8, g.n16, g.M, g.K);
+  RDQ_REQUIRE(workspace && workspace_bytes >= 2ull * p.sc.G * p.sc.nt * 128 * sizeof(float), RDQ_E_INVALID,
+              "GEMM workspace too small");
+  int *status = nullptr;
+  int rc = gemm_status_ptr(&status);
+  if (rc != RDQ_OK) return rc;
+  CUtensorMap w4map, w8map, w16map, xmap;
+  rc = encode_f16_2d(&xmap, g.x, g.K, g.M, 64, p.sc.nt);
+  if (rc != RDQ_OK) return rc;
+  w4map = w8map = w16map = xmap;  // maps of absent groups are never used
+  if (g.n4 && (rc = encode_u8_2d(&w4map, g.w4, g.K / 2, g.n4)) != RDQ_OK) return rc;
+  if (g.n8 && (rc = encode_u8_2d(&w8map, g.w8, g.K, g.n8)) != RDQ_OK) return rc;
+  if (g.n16 && (rc = encode_f16_2d(&w16map, g.w16, g.K, g.n16, 64, 128)) != RDQ_OK) return rc;
+  StreamArgs a;
+  a.s4 = g.s4;
+  a.s8 = g.s8;
+  a.global4 = g.global4;
+  a.perm = g.perm;
+  a.bias = g.bias;
+  a.y = g.y;
+  a.y_bf16 = g.y_bf16;
+  a.n4 = g.n4;
+  a.n8 = g.n8;
+  a.n16 = g.n16;
+  a.K = g.K;
+  a.N = g.n4 + g.n8 + g.n16;
+  a.partial = static_cast<float *>(workspace);
+  a.arrived = reinterpret_cast<uint32_t *>(g.counters);
+  a.nw = p.nw;
+  a.early = pdl;
+  a.scale16 = g.K % 256 == 0 && aligned16(g.s4);
+  a.test_timeout = gemm_test_timeout();
+  const StreamSched &sc = p.sc;
+
+  const void *fn = p.cols == 256 ? reinterpret_cast<const void *>(gemm_stream_kernel<256>)
+                                 : reinterpret_cast<const void *>(gemm_stream_kernel<512>);
+  static std::atomic<int> smem_set[2][64];
+  int dev = 0;
+  RDQ_CUDA(cudaGetDevice(&dev));
+  std::atomic<int> *set = dev >= 0 && dev < 64 ? &smem_set[p.cols == 256][dev] : nullptr;
+  if (!set || set->load() < p.smem) {
+    RDQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, p.cols == 256 ? 110 * 1024 : 222 * 1024));
+    RDQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    if (set) set->store(1 << 30);
+  }
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(sc.G));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = p.smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  void *params[7] = {&w4map, &w8map, &w16map, &xmap, &a, const_cast<StreamSched *>(&sc), &status};
+  RDQ_CUDA(cudaLaunchKernelExC(&cfg, fn, params));
+  return RDQ_OK;
+}
+
+}  // namespace rdq

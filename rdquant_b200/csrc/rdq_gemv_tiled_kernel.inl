@@ -87,6 +87,7 @@ struct TiledArgs {
   int slot_bytes;
   int nepi;    // epilogue warps in use
   int fdepth;  // slots per hand-over ring
+  int early;         // weights may be read before the kernel before this one has finished
   int test_timeout;  // self-test: CTA 0 ends with a wait that runs out
   // Peer mode (column-parallel layers): the outputs go to n_dst destinations -- one slice of a
   // gather buffer on every GPU of the node, this one included, written with plain stores over
@@ -381,6 +382,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
       __syncwarp();
     }
     if (lane != 0) return;
+    if (!a.early) pdl_wait();
     // The ring is filled with weights first (they do not depend on the preceding kernel);
     // only then wait for that kernel and fetch the activations it produced.
     bool x_sent = false;
@@ -427,6 +429,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
     const int ej = warp - kMmaWarps - 1;
     if (ej >= nepi) return;
     float *vst = vstage + ej * kTileRows * vp;
+    if (!a.early) pdl_wait();
     // output column, scale and bias of every row this CTA finishes: constants of the
     // layer, fetched up front so that finishing a tile needs no global round trip.  With
     // more than one epilogue warp the first builds the segment table and the others do this.
@@ -985,6 +988,7 @@ int launch_gemv_tiled(const GemvTiledArgs &h, bool pdl, cudaStream_t stream) {
   a.x = static_cast<const __half *>(h.x); a.y_bf16 = h.y_bf16; a.M = h.M; a.tiled = h.tiled; a.s8 = h.s8; a.global4 = h.global4; a.perm = h.perm;
   a.bias = h.bias; a.y = h.y; a.n4 = h.n4; a.n8 = h.n8; a.n16 = h.n16; a.K = h.K;
   a.workspace = h.workspace; a.flags = h.flags;
+  a.early = pdl;
   a.test_timeout = h.test_timeout;
   a.n_dst = h.n_dst;
   for (int d = 0; d < kMaxPeers; ++d) {
@@ -1091,7 +1095,7 @@ int launch_gemv_tiled(const GemvTiledArgs &h, bool pdl, cudaStream_t stream) {
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   void *params[2] = {&a, &sc};

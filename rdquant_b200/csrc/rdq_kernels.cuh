@@ -40,6 +40,8 @@ struct GemmArgs {
   const float *s8;
   const __half *w16;
   const int32_t *inv_perm;
+  const int32_t *perm = nullptr;  // inverse of inv_perm
+  int32_t *counters = nullptr;    // one zero word per SM, zero again when the launch ends
   const __half *bias;
   void *y;
   int n4, n8, n16, K;
@@ -108,9 +110,19 @@ int launch_peer_gather(const __half *buffer, const long long *index, __half *y, 
 int launch_gemm(const GemmArgs &a, void *workspace, size_t workspace_bytes, cudaStream_t stream);
 // synchronise `stream`, report (and optionally clear) the GEMM's per-device status word
 int gemm_status(bool reset, cudaStream_t stream);
+int gemm_status_ptr(int **out);
+int gemm_test_timeout();
 // self-test switch: launches made while it is on end with a wait that runs out
 void gemm_set_test_timeout(bool on);
 size_t gemm_workspace_bytes(int M, int N, int K);
+// weight-streaming GEMM (rdq_gemm_stream.cu)
+bool gemm_stream_takes(int K);
+size_t gemm_stream_workspace(int M, int K);
+int launch_gemm_stream(const GemmArgs &a, void *workspace, size_t workspace_bytes, bool pdl, cudaStream_t stream);
+// GEMM over weights decoded once per call (rdq_gemm_dense.cu)
+bool gemm_dense_takes(int K);
+size_t gemm_dense_workspace(int M, int N, int K);
+int launch_gemm_dense(const GemmArgs &a, void *workspace, size_t workspace_bytes, cudaStream_t stream);
 
 // staging copy by kernel (rdq_stage.cu)
 int launch_stage_copy(void *dst, const void *src, size_t bytes, int *state, int *flag, cudaStream_t stream);

@@ -34,18 +34,21 @@ __global__ void __launch_bounds__(256) cast_elems_kernel(const __nv_bfloat16 *__
     out[i] = __float2half_rn(__bfloat162float(x[i]));
 }
 
-enum class Path { kGemvTiled, kGemvGeneric, kGemm, kPanelsTiled, kPanelsGeneric };
+enum class Path { kGemvTiled, kGemvGeneric, kStream, kGemm, kPanelsTiled, kPanelsGeneric };
 
 bool has_row_major(const rdq_layer &l) {
   return (l.n_fp4 == 0 || l.w_fp4) && (l.n_fp8 == 0 || l.w_fp8) && (l.n_fp16 == 0 || l.w_fp16);
 }
 
 // Up to 16 rows: the decode GEMV (tiled layout, else the any-shape kernel).  More rows: the
-// tensor-core GEMM, which tiles K in blocks of 64 and reads the row-major tensors; what it cannot
+// tensor-core GEMM, which reads the row-major tensors by TMA (K a multiple of 16); what it cannot
 // take runs as 16-row panels of the decode kernel.
 Path path_of(const rdq_layer &l, int M) {
+  static const int lo = getenv("RDQ_STREAM_LO") ? atoi(getenv("RDQ_STREAM_LO")) : 17;
+  static const int hi = getenv("RDQ_STREAM_HI") ? atoi(getenv("RDQ_STREAM_HI")) : 256;
+  if (M >= lo && M <= hi && gemm_stream_takes(l.K) && has_row_major(l) && l.gemv_counters && (l.perm || !l.inv_perm)) return Path::kStream;
   if (M <= RDQ_MAX_GEMV_M) return l.w_tiled ? Path::kGemvTiled : Path::kGemvGeneric;
-  if (l.K % 64 == 0 && has_row_major(l)) return Path::kGemm;
+  if (gemm_dense_takes(l.K) && has_row_major(l)) return Path::kGemm;
   return l.w_tiled ? Path::kPanelsTiled : Path::kPanelsGeneric;
 }
 
@@ -60,6 +63,7 @@ struct Need {
 Need need_of(const rdq_layer &l, Path p, int M, int x_type) {
   Need n;
   if (x_type == RDQ_BF16 && !takes_bf16(l, p, M)) n.cast = align256(2ull * M * l.K);
+  if (p == Path::kStream) n.gemm = gemm_stream_workspace(M, l.K);
   if (p == Path::kGemm) n.gemm = gemm_workspace_bytes(M, l.n_fp4 + l.n_fp8 + l.n_fp16, l.K);
   return n;
 }
@@ -188,6 +192,7 @@ int rdq_linear(const rdq_layer *layer, const void *x, int x_type, int M, const v
       }
       return RDQ_OK;
     }
+    case Path::kStream:
     case Path::kGemm:
       break;
   }
@@ -204,6 +209,8 @@ int rdq_linear(const rdq_layer *layer, const void *x, int x_type, int M, const v
   a.s8 = l.w_fp8_scales;
   a.w16 = static_cast<const __half *>(l.w_fp16);
   a.inv_perm = l.inv_perm;
+  a.perm = l.perm;
+  a.counters = l.gemv_counters;
   a.bias = static_cast<const __half *>(bias);
   a.y = y;
   a.n4 = l.n_fp4;
@@ -213,6 +220,7 @@ int rdq_linear(const rdq_layer *layer, const void *x, int x_type, int M, const v
   a.y_bf16 = bf16;
   a.ksplit = 1;
   a.partial = nullptr;
+  if (p == Path::kStream) return launch_gemm_stream(a, rest, need.gemm, pdl, stream);
   return launch_gemm(a, rest, need.gemm, stream);
 }
 

@@ -276,9 +276,6 @@ def mixed_gemv_silu(gate_up: torch.Tensor, fd: dict, bias: Optional[torch.Tensor
     return _gemv_xop(XOP_SILU_MUL, gate_up, None, None, None, 0.0, m, k2 // 2, fd, bias, flags, out)
 
 
-_gemm_ws: dict = {}  # device -> scratch tensor of the split-k GEMM
-
-
 def mixed_gemm(x: torch.Tensor, fd: dict, bias: Optional[torch.Tensor] = None,
                out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Prefill GEMM ``y[M, N] = x[M, K] @ W.T (+ bias)`` on the tcgen05 path."""
@@ -300,16 +297,11 @@ def mixed_gemm(x: torch.Tensor, fd: dict, bias: Optional[torch.Tensor] = None,
     if not fd.get("row_major", True):
         raise RuntimeError("this layer was packed without its row-major tensors: the prefill GEMM cannot run it")
     with _on_device(x.device):
-        # scratch for problems with few tiles (the library then splits the k range); the
-        # per-device buffer only grows and is reused by later calls on the same stream order
+        # scratch of this call alone (decoded weights, partial sums): torch's allocator orders its
+        # reuse behind the work queued on the current stream
         need = ctypes.c_size_t(0)
         _lib.check(_lib.lib().rdq_gemm_workspace_size(m, n, k, ctypes.byref(need)), "rdq_gemm_workspace_size")
-        ws = None
-        if need.value:
-            ws = _gemm_ws.get(x.device)
-            if ws is None or ws.numel() < need.value:
-                ws = torch.empty(need.value, dtype=torch.uint8, device=x.device)
-                _gemm_ws[x.device] = ws
+        ws = torch.empty(need.value, dtype=torch.uint8, device=x.device) if need.value else None
         rc = _lib.lib().rdq_gemm_mixed_ws(
             _ptr(x), m, _ptr(fd.get("w_fp4_q")), _ptr(fd.get("w_fp4_scales")), float(fd.get("w_fp4_global_scale", 1.0)),
             _ptr(fd.get("w_fp8_q")), _ptr(fd.get("w_fp8_scales")), _ptr(fd.get("w_fp16")), _ptr(fd.get("inv_perm")),
@@ -325,9 +317,9 @@ def mixed_linear(x: torch.Tensor, fd: dict, bias: Optional[torch.Tensor] = None,
     """GEMV for M <= 16, GEMM above."""
     if x.shape[0] <= MAX_GEMV_M:
         return mixed_gemv(x, fd, bias, flags, out=out)
-    if fd["k"] % 64 == 0 and fd.get("row_major", True):
+    if fd["k"] % 16 == 0 and fd.get("row_major", True):
         return mixed_gemm(x, fd, bias, out=out)
-    # the tensor-core GEMM tiles K in blocks of 64 and reads the row-major tensors; other K, and
+    # the tensor-core GEMM reads the row-major tensors by TMA (K a multiple of 16); other K, and
     # layers packed without them, run the decode kernel over 16-row panels (the reference's
     # dense prefill takes any K, rdquant/inference.py:679-687)
     n = fd["n_fp4"] + fd["n_fp8"] + fd["n_fp16"]
