@@ -141,6 +141,8 @@ def _bind(lib: ctypes.CDLL) -> None:
     lib.rdq_quantize_nvfp4.argtypes = [vp, i32, i32, i32, vp, vp, vp, vp, vp]
     lib.rdq_quantize_fp8.restype = i32
     lib.rdq_quantize_fp8.argtypes = [vp, i32, i32, i32, vp, vp, vp, vp, vp]
+    lib.rdq_quantize_layer.restype = i32
+    lib.rdq_quantize_layer.argtypes = [vp, i32, vp, i32, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, vp]
     lib.rdq_add_rmsnorm.restype = i32
     lib.rdq_add_rmsnorm.argtypes = [vp, vp, vp, vp, i32, i32, f32, i32, vp]
     lib.rdq_qk_rope_cache.restype = i32
@@ -188,6 +190,7 @@ EXPORTS = [
     "rdq_gemm_workspace_size",
     "rdq_quantize_nvfp4",
     "rdq_quantize_fp8",
+    "rdq_quantize_layer",
     "rdq_linear",
     "rdq_linear_workspace_size",
     "rdq_stage_copy",

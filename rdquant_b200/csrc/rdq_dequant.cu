@@ -1,10 +1,13 @@
-// Bit-exact dequantisation of a packed mixed-precision layer to FP16 [N, K] in
-// original channel order.  HBM-bound elementwise kernel: reads the packed
-// bytes once, writes 2*N*K bytes once; each thread owns one 16-element run
-// (one NVFP4 scale block) of one output row.
+// Bit-exact dequantisation of a packed mixed-precision layer to FP16 or FP32 [N, K] in original
+// channel order.  HBM-bound: reads the packed bytes once, writes 2 (or 4) N K bytes once.
+//
+// A warp per output row, a lane per 8 consecutive k: a warp instruction reads 128 / 256 / 512
+// contiguous bytes of an NVFP4 / FP8 / FP16 row and stores 512 (f16), four of them in flight.
+// (16-element runs per thread, with 32-byte store strides and one run in flight, reached 1.9 TB/s.)
 //
 // Arithmetic follows the reference oracle exactly:
 //   NVFP4  f16( f32(LUT[code]) * f32(e4m3 scale) )        rdquant/core/formats.py:145-159
+//          (with a global scale of 1 every product is an f16 value: multiplied in f16)
 //   FP8    f16( f32(e4m3 byte) * scale[channel] )          rdquant/inference.py:104-109
 //   FP16   bf16 -> f32 -> f16 (or a plain copy of f16)     rdquant/inference.py:111-113
 // and the row gather is QuantizedWeight.dequantize's cat()[inv_perm]
@@ -25,98 +28,122 @@ struct DequantArgs {
   int w16_is_bf16;
   const int32_t *inv_perm;
   void *out;
-  int out_is_f32;
   int n4, n8, n16, K;
 };
 
-// `vec` says the row pitch keeps every 16-element run 32 / 64-byte aligned (K % 16 == 0);
-// otherwise the run is stored element by element, full runs included.
-__device__ __forceinline__ void store16(__half *dst, const float (&v)[16], int valid, bool vec) {
-  if (vec) {
-    __half2 o[8];
+constexpr int kUnroll = 4;
+
+__device__ __forceinline__ void store8(__half *row, int v, const float (&f)[8]) {
+  uint4 o;
+  uint32_t *w = reinterpret_cast<uint32_t *>(&o);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) o[i] = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
-    uint4 *d4 = reinterpret_cast<uint4 *>(dst);
-    d4[0] = *reinterpret_cast<uint4 *>(&o[0]);
-    d4[1] = *reinterpret_cast<uint4 *>(&o[4]);
-  } else {
-    for (int i = 0; i < valid; ++i) dst[i] = __float2half_rn(v[i]);
-  }
+  for (int i = 0; i < 4; ++i) w[i] = pack_y2(f[2 * i], f[2 * i + 1], 0);
+  reinterpret_cast<uint4 *>(row)[v] = o;
 }
-__device__ __forceinline__ void store16(float *dst, const float (&v)[16], int valid, bool vec) {
-  if (vec) {
-    float4 *d4 = reinterpret_cast<float4 *>(dst);
+__device__ __forceinline__ void store8(float *row, int v, const float (&f)[8]) {
+  reinterpret_cast<float4 *>(row)[2 * v] = make_float4(f[0], f[1], f[2], f[3]);
+  reinterpret_cast<float4 *>(row)[2 * v + 1] = make_float4(f[4], f[5], f[6], f[7]);
+}
+__device__ __forceinline__ void halves_to_floats(const uint32_t (&h)[4], float (&f)[8]) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) d4[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-  } else {
-    for (int i = 0; i < valid; ++i) dst[i] = v[i];
+  for (int i = 0; i < 4; ++i) {
+    const float2 t = h2_to_f2(h[i]);
+    f[2 * i] = t.x;
+    f[2 * i + 1] = t.y;
   }
 }
 
 // OutT = __half: the operator's weight (products rounded to f16, round to nearest even).
 // OutT = float : the unrounded FP32 product, what formats.dequantize returns.
-template <typename OutT>
+// VEC: K % 8 == 0, so rows are whole runs of 8 with 16-byte (packed: 4-byte) alignment.
+template <typename OutT, bool VEC>
 __global__ void __launch_bounds__(256) dequant_kernel(DequantArgs a) {
-  const int K = a.K;
-  const int chunks = (K + 15) >> 4;
-  const bool vec = (K & 15) == 0;
-  const long long total = 1ll * (a.n4 + a.n8 + a.n16) * chunks;
-  OutT *out = reinterpret_cast<OutT *>(a.out);
-  for (long long item = 1ll * blockIdx.x * blockDim.x + threadIdx.x; item < total;
-       item += 1ll * gridDim.x * blockDim.x) {
-    const int n = static_cast<int>(item / chunks);
-    const int c = static_cast<int>(item - 1ll * n * chunks);
+  const int lane = threadIdx.x & 31;
+  const int K = a.K, N = a.n4 + a.n8 + a.n16;
+  const int nvec = K >> 3;
+  for (int n = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; n < N; n += (gridDim.x * blockDim.x) >> 5) {
     const int r = a.inv_perm ? a.inv_perm[n] : n;
-    const int k0 = c << 4;
-    const int valid = min(16, K - k0);
-    float v[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = 0.f;
+    OutT *row = static_cast<OutT *>(a.out) + 1ll * n * K;
     if (r < a.n4) {
-      // K % 16 == 0 is a precondition of the NVFP4 layout.
-      const uint8_t *src = a.w4 + 1ll * r * (K >> 1) + (k0 >> 1);
-      const float sc = e4m3_to_float(a.s4[1ll * r * (K >> 4) + c]) * a.global4;
-      const uint2 q = *reinterpret_cast<const uint2 *>(src);
-      uint32_t h[8];
-      cvt_e2m1x8(q.x, h[0], h[1], h[2], h[3]);
-      cvt_e2m1x8(q.y, h[4], h[5], h[6], h[7]);
+      // K % 16 == 0 is a precondition of the NVFP4 layout
+      const uint32_t *src = reinterpret_cast<const uint32_t *>(a.w4 + 1ll * r * (K >> 1));
+      const uint8_t *ssrc = a.s4 + 1ll * r * (K >> 4);
+      const bool plain = sizeof(OutT) == 2 && a.global4 == 1.f;
+      for (int v0 = lane; v0 < nvec; v0 += 32 * kUnroll) {
+        uint32_t q[kUnroll], s[kUnroll];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float2 f = h2_to_f2(h[i]);
-        v[2 * i] = f.x * sc;
-        v[2 * i + 1] = f.y * sc;
+        for (int u = 0; u < kUnroll; ++u)
+          if (v0 + 32 * u < nvec) {
+            q[u] = __ldg(src + v0 + 32 * u);
+            s[u] = __ldg(ssrc + ((v0 + 32 * u) >> 1));
+          }
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) {
+          if (v0 + 32 * u >= nvec) break;
+          uint32_t h[4];
+          cvt_e2m1x8(q[u], h[0], h[1], h[2], h[3]);
+          if (plain) {
+            const uint32_t sc = __byte_perm(cvt_e4m3x2(s[u]), 0u, 0x1010u);
+            reinterpret_cast<uint4 *>(row)[v0 + 32 * u] =
+                make_uint4(hmul2_u32(h[0], sc), hmul2_u32(h[1], sc), hmul2_u32(h[2], sc), hmul2_u32(h[3], sc));
+          } else {
+            const float sc = e4m3_to_float(s[u]) * a.global4;
+            float f[8];
+            halves_to_floats(h, f);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) f[i] *= sc;
+            store8(row, v0 + 32 * u, f);
+          }
+        }
       }
     } else if (r < a.n4 + a.n8) {
       const int rr = r - a.n4;
       const float sc = a.s8[rr];
-      const uint8_t *src = a.w8 + 1ll * rr * K + k0;
-      if (vec) {
-        const uint4 q = *reinterpret_cast<const uint4 *>(src);
-        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+      const uint8_t *src = a.w8 + 1ll * rr * K;
+      if (VEC) {
+        for (int v0 = lane; v0 < nvec; v0 += 32 * kUnroll) {
+          uint2 q[kUnroll];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          uint32_t h01, h23;
-          cvt_e4m3x4(w[i], h01, h23);
-          const float2 f0 = h2_to_f2(h01), f1 = h2_to_f2(h23);
-          v[4 * i] = f0.x * sc;
-          v[4 * i + 1] = f0.y * sc;
-          v[4 * i + 2] = f1.x * sc;
-          v[4 * i + 3] = f1.y * sc;
+          for (int u = 0; u < kUnroll; ++u)
+            if (v0 + 32 * u < nvec) q[u] = __ldg(reinterpret_cast<const uint2 *>(src) + v0 + 32 * u);
+#pragma unroll
+          for (int u = 0; u < kUnroll; ++u) {
+            if (v0 + 32 * u >= nvec) break;
+            uint32_t h[4];
+            cvt_e4m3x4(q[u].x, h[0], h[1]);
+            cvt_e4m3x4(q[u].y, h[2], h[3]);
+            float f[8];
+            halves_to_floats(h, f);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) f[i] *= sc;
+            store8(row, v0 + 32 * u, f);
+          }
         }
       } else {
-        for (int i = 0; i < valid; ++i) v[i] = e4m3_to_float(src[i]) * sc;
+        for (int k = lane; k < K; k += 32) row[k] = static_cast<OutT>(e4m3_to_float(src[k]) * sc);
       }
     } else {
-      const int rr = r - a.n4 - a.n8;
-      if (a.w16_is_bf16) {
-        const __nv_bfloat16 *src = reinterpret_cast<const __nv_bfloat16 *>(a.w16) + 1ll * rr * K + k0;
-        for (int i = 0; i < valid; ++i) v[i] = __half2float(__float2half_rn(__bfloat162float(src[i])));
+      const long long off = 1ll * (r - a.n4 - a.n8) * K;
+      const uint16_t *src = static_cast<const uint16_t *>(a.w16) + off;
+      if (VEC) {
+        for (int v = lane; v < nvec; v += 32) {
+          const uint4 q = __ldg(reinterpret_cast<const uint4 *>(src) + v);
+          uint32_t h[4] = {q.x, q.y, q.z, q.w};
+          if (a.w16_is_bf16) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) h[i] = bf16x2_to_f16x2(h[i]);
+          }
+          float f[8];
+          halves_to_floats(h, f);
+          store8(row, v, f);
+        }
       } else {
-        const __half *src = reinterpret_cast<const __half *>(a.w16) + 1ll * rr * K + k0;
-        for (int i = 0; i < valid; ++i) v[i] = __half2float(src[i]);
+        for (int k = lane; k < K; k += 32) {
+          const __half h = a.w16_is_bf16 ? __float2half_rn(__bfloat162float(__ushort_as_bfloat16(src[k]))) : __ushort_as_half(src[k]);
+          row[k] = static_cast<OutT>(__half2float(h));
+        }
       }
     }
-    store16(out + 1ll * n * K + k0, v, valid, vec);
   }
 }
 
@@ -136,20 +163,20 @@ int launch_dequant(const void *w_fp4, const void *w_fp4_scales, float global4, c
   a.w16_is_bf16 = fp16_is_bf16;
   a.inv_perm = inv_perm;
   a.out = w_out;
-  a.out_is_f32 = out_is_f32;
   a.n4 = n4;
   a.n8 = n8;
   a.n16 = n16;
   a.K = K;
-  const long long total = 1ll * (n4 + n8 + n16) * ((K + 15) / 16);
-  if (total == 0) return RDQ_OK;
-  long long blocks = (total + 255) / 256;
-  const long long cap = 1ll * sm_count() * 32;
-  if (blocks > cap) blocks = cap;
+  const long long rows = 1ll * n4 + n8 + n16;
+  if (rows == 0) return RDQ_OK;
+  const unsigned blocks = static_cast<unsigned>(std::min<long long>((rows + 7) / 8, 8ll * sm_count()));
+  const bool vec = K % 8 == 0;
   if (out_is_f32) {
-    dequant_kernel<float><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(a);
+    if (vec) dequant_kernel<float, true><<<blocks, 256, 0, stream>>>(a);
+    else dequant_kernel<float, false><<<blocks, 256, 0, stream>>>(a);
   } else {
-    dequant_kernel<__half><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(a);
+    if (vec) dequant_kernel<__half, true><<<blocks, 256, 0, stream>>>(a);
+    else dequant_kernel<__half, false><<<blocks, 256, 0, stream>>>(a);
   }
   RDQ_CUDA(cudaGetLastError());
   return RDQ_OK;

@@ -3,17 +3,28 @@
 // (rdquant/core/formats.py:84-142 nvfp4_quantize, :166-193 fp8_quantize; byte layout
 // rdquant/integrations/hf_export.py:81-102), plus the per-row sum of squared reconstruction
 // errors that the per-channel MSE of the format search needs
-// (rdquant/core/formats.py:414-436 compute_mse_2d: mean over the row of (w - dequant)^2).
+// (rdquant/core/formats.py:414-436 compute_mse_2d: mean over the row of (w - dequant)^2); and a whole
+// layer at once, its rows gathered by the channel permutation on the way in (rdq_quantize_layer).
 //
-// One warp per row, a lane per block of 16 consecutive k (K % 16 == 0, so the reference's
-// blocks over the flattened group coincide with blocks inside rows).  Arithmetic follows
-// the reference operation by operation in IEEE float32: block scale =
-// e4m3(clamp(absmax / 6)), ratio = v / scale (scale 0 -> 1), code = number of grid midpoints
-// strictly below |ratio| (ties go to the smaller magnitude) + 8 if ratio < 0; FP8 scale =
-// absmax(group) / 448 (0 -> 1), byte = e4m3(clamp(v / scale)).  The E4M3 rounding is the
-// hardware converter's round-to-nearest-even, the same as torch.float8_e4m3fn's.
+// One warp per row, a lane per 8 consecutive k: loads of 512 (f16) contiguous bytes per warp
+// instruction, four in flight; a pair of lanes shares a block of 16 (K % 16 == 0, so the reference's
+// blocks over the flattened group coincide with blocks inside rows).
 //
-// HBM-bound elementwise work: reads 4 (f32) or 2 (f16) bytes per element, writes 0.56 / 1.
+// Bound: HBM (reads 2 or 4 bytes per element, writes 0.56 / 1).  The reference divides every element
+// by its scale; here
+//   NVFP4  no division per element: the code counts the grid midpoints t with fl(v / s) > t, and for a
+//          scale s with a 4-bit mantissa that is v > t s (t s is exact; fl(v / s) > t needs v / s to
+//          exceed t by half an ulp, and a float v above t s exceeds it by more: the relative step of v
+//          is above 2^-24 there, half an ulp of t at most 2^-24).  The sign of a quotient that
+//          underflows to zero is the one exception: denormal inputs take the division.
+//          An f16 v that is not t s itself differs from it by more than 2^-12 of it, so v (1 - 2^-14) / s
+//          lies on the right side of every midpoint and below one that v / s hits: the hardware's
+//          round-to-nearest E2M1 converter then gives the code (adding +0 turns -0 into +0, whose code
+//          is 0).  Counting thresholds instead took 32 us for a 2560 x 9728 layer.
+//   FP8    v is multiplied by 1 / scale; only where the product lies within a few ulp of a rounding
+//          boundary of E4M3 (or in its subnormal range) does the division decide.
+// The E4M3 rounding is the hardware converter's round-to-nearest-even, the same as
+// torch.float8_e4m3fn's.
 #include <cuda_fp8.h>
 
 #include "rdq_kernels.cuh"
@@ -22,31 +33,36 @@ namespace rdq {
 
 namespace {
 
-__device__ __forceinline__ float load_elem(const float *p, long long i) { return p[i]; }
-__device__ __forceinline__ float load_elem(const __half *p, long long i) { return __half2float(p[i]); }
-// 16 consecutive elements starting at a multiple of 16 (the tensor is 16-byte aligned)
-__device__ __forceinline__ void load16(const float *p, long long i, float (&v)[16]) {
-  const float4 *q = reinterpret_cast<const float4 *>(p + i);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float4 t = __ldg(q + j);
-    v[4 * j] = t.x; v[4 * j + 1] = t.y; v[4 * j + 2] = t.z; v[4 * j + 3] = t.w;
-  }
-}
-__device__ __forceinline__ void load16(const __half *p, long long i, float (&v)[16]) {
-  const uint4 *q = reinterpret_cast<const uint4 *>(p + i);
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    const uint4 t = __ldg(q + j);
-    const uint32_t u[4] = {t.x, t.y, t.z, t.w};
+constexpr int kUnroll = 4;  // vectors of 8 elements in flight per lane
+
+template <typename T>
+struct Vec8;
+template <>
+struct Vec8<__half> {
+  uint4 q;
+  __device__ __forceinline__ void load(const __half *p) { q = __ldg(reinterpret_cast<const uint4 *>(p)); }
+  __device__ __forceinline__ void get(float (&v)[8]) const {
+    const uint32_t u[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&u[e]));
-      v[8 * j + 2 * e] = f.x;
-      v[8 * j + 2 * e + 1] = f.y;
+      const float2 f = h2_to_f2(u[e]);
+      v[2 * e] = f.x;
+      v[2 * e + 1] = f.y;
     }
   }
-}
+};
+template <>
+struct Vec8<float> {
+  float4 a, b;
+  __device__ __forceinline__ void load(const float *p) {
+    a = __ldg(reinterpret_cast<const float4 *>(p));
+    b = __ldg(reinterpret_cast<const float4 *>(p) + 1);
+  }
+  __device__ __forceinline__ void get(float (&v)[8]) const {
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+  }
+};
 
 __device__ __forceinline__ uint8_t to_e4m3(float v) {
   return static_cast<uint8_t>(__nv_cvt_float_to_fp8(v, __NV_SATFINITE, __NV_E4M3));
@@ -61,96 +77,282 @@ __device__ __forceinline__ float clamp448(float v) { return fminf(fmaxf(v, -448.
 __device__ __forceinline__ void atomic_max_nonneg(float *addr, float v) {
   atomicMax(reinterpret_cast<unsigned int *>(addr), __float_as_uint(v));
 }
+__device__ __forceinline__ float max8(const float (&v)[8]) {
+  float m = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) m = fmaxf(m, fabsf(v[i]));
+  return m;
+}
+
+// two values -> a byte of E2M1 codes, `lo` in the low nibble
+__device__ __forceinline__ uint32_t cvt_to_e2m1x2(float lo, float hi) {
+  uint32_t r;
+  asm("{\n.reg .b8 b;\ncvt.rn.satfinite.e2m1x2.f32 b, %2, %1;\nmov.b32 %0, {b, b, b, b};\n}\n" : "=r"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+// Half a block of 16: codes of eight values (a nibble each, low nibble first).  F16: the values are
+// finite f16 values.
+template <bool SQERR, bool F16>
+__device__ __forceinline__ uint32_t encode_fp4(const float (&v)[8], float scale, float &err) {
+  const float s = scale == 0.f ? 1.f : scale;
+  if (F16 && !SQERR) {
+    const float c = __fdividef(1.f, s) * (1.f - 6.103515625e-5f);
+    uint32_t b[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) b[i] = cvt_to_e2m1x2(fmaf(v[2 * i], c, 0.f), fmaf(v[2 * i + 1], c, 0.f));
+    return __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
+  }
+  const float t0 = 0.25f * s, t1 = 0.75f * s, t2 = 1.25f * s, t3 = 1.75f * s, t4 = 2.5f * s, t5 = 3.5f * s, t6 = 5.0f * s;
+  uint32_t packed = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float mag = fabsf(v[i]);
+    const int m = (mag > t0) + (mag > t1) + (mag > t2) + (mag > t3) + (mag > t4) + (mag > t5) + (mag > t6);
+    const bool neg = v[i] < 0.f && (mag >= 1.17549435e-38f || __fdiv_rn(v[i], s) < 0.f);
+    packed |= static_cast<uint32_t>(m + (neg ? 8 : 0)) << (4 * i);
+    if (SQERR) {
+      // grid value: 0, .5, 1, 1.5 (m / 2) then 2, 3, 4, 6
+      const float g = (m < 4) ? 0.5f * m : (m == 7 ? 6.f : static_cast<float>(m - 2));
+      const float d = v[i] - __fmul_rn(neg ? -g : g, scale);
+      err = fmaf(d, d, err);
+    }
+  }
+  return packed;
+}
+
+// A row of K values -> codes u8 [K / 2], scales u8 [K / 16]; the largest block scale joins `top`.
+template <typename T, bool SQERR>
+__device__ __forceinline__ void encode_row_fp4(const T *w, int K, uint8_t *codes, uint8_t *scales, int lane, float &top, float &err) {
+  const int nvec = K >> 3;
+  for (int v0 = lane; v0 - lane < nvec; v0 += 32 * kUnroll) {
+    Vec8<T> q[kUnroll];
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u)
+      if (v0 + 32 * u < nvec) q[u].load(w + 8ll * (v0 + 32 * u));
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      if (v0 - lane + 32 * u >= nvec) break;  // the whole warp is past the row
+      const int i = v0 + 32 * u;
+      float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      if (i < nvec) q[u].get(v);
+      // bit patterns order magnitudes and put NaN above infinity; the scale ignores NaN
+      uint32_t bits = 0;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) bits = max(bits, __float_as_uint(v[e]) & 0x7fffffffu);
+      bits = max(bits, __shfl_xor_sync(0xffffffffu, bits, 1));
+      const bool finite = bits < 0x7f800000u;
+      float amax = __uint_as_float(bits);
+      if (__any_sync(0xffffffffu, !finite)) {
+        amax = max8(v);
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+      }
+      const uint8_t sbits = to_e4m3(clamp448(__fdiv_rn(amax, 6.f)));
+      const float scale = from_e4m3(sbits);
+      top = fmaxf(top, scale);
+      if (i < nvec) {
+        reinterpret_cast<uint32_t *>(codes)[i] = sizeof(T) == 2 && finite ? encode_fp4<SQERR, true>(v, scale, err)
+                                                                          : encode_fp4<SQERR, false>(v, scale, err);
+        if (!(i & 1)) scales[i >> 1] = sbits;
+      }
+    }
+  }
+}
+
+// fl(v / scale) rounded to E4M3 for eight values; inv = fl(1 / scale)
+__device__ __forceinline__ uint2 quotients_e4m3(const float (&v)[8], float scale, float inv) {
+  float r[8];
+  bool sure = true;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    r[i] = v[i] * inv;  // within 2 ulp of the quotient
+    const uint32_t low = (__float_as_uint(r[i]) & 0xfffffu) - 0x80000u + 8u;  // distance to a rounding boundary of a normal result
+    sure = sure && low > 16u && fabsf(r[i]) >= 0.015625f && fabsf(r[i]) < 1e30f;
+  }
+  if (!sure) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) r[i] = clamp448(__fdiv_rn(v[i], scale));
+  }
+  uint32_t h[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    h[i] = __nv_cvt_float2_to_fp8x2(make_float2(r[2 * i], r[2 * i + 1]), __NV_SATFINITE, __NV_E4M3);
+  return make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
+}
+
+template <typename T, bool SQERR>
+__device__ __forceinline__ void encode_row_fp8(const T *w, int K, float scale, uint8_t *out, int lane, float &err) {
+  const float inv = __fdiv_rn(1.f, scale);
+  const bool plain = inv > 1e-30f && inv < 1e30f;  // else the product may lose bits the quotient has
+  const int nvec = K >> 3;
+  for (int v0 = lane; v0 < nvec; v0 += 32 * kUnroll) {
+    Vec8<T> q[kUnroll];
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u)
+      if (v0 + 32 * u < nvec) q[u].load(w + 8ll * (v0 + 32 * u));
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      const int i = v0 + 32 * u;
+      if (i >= nvec) break;
+      float v[8];
+      q[u].get(v);
+      const uint2 o = quotients_e4m3(v, scale, plain ? inv : 0.f);
+      if (SQERR) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const float d = v[e] - __fmul_rn(from_e4m3(static_cast<uint8_t>((e < 4 ? o.x : o.y) >> (8 * (e & 3)))), scale);
+          err = fmaf(d, d, err);
+        }
+      }
+      reinterpret_cast<uint2 *>(out)[i] = o;
+    }
+  }
+}
 
 template <typename T>
+__device__ __forceinline__ float absmax_row(const T *w, int K, int lane) {
+  const int nvec = K >> 3;
+  float m = 0.f;
+  for (int v0 = lane; v0 < nvec; v0 += 32 * kUnroll) {
+    Vec8<T> q[kUnroll];
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u)
+      if (v0 + 32 * u < nvec) q[u].load(w + 8ll * (v0 + 32 * u));
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      if (v0 + 32 * u >= nvec) break;
+      float v[8];
+      q[u].get(v);
+      m = fmaxf(m, max8(v));
+    }
+  }
+  return m;
+}
+
+__device__ __forceinline__ float fp8_scale(float absmax) {
+  const float s = __fdiv_rn(absmax, 448.f);
+  return s == 0.f ? 1.f : s;
+}
+
+template <typename T, bool SQERR>
 __global__ void __launch_bounds__(256) quantize_nvfp4_kernel(const T *__restrict__ w, int n, int K, uint8_t *__restrict__ codes,
                                                              uint8_t *__restrict__ scales, float *__restrict__ row_sqerr,
                                                              float *__restrict__ max_scale) {
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
-  const int nblk = K >> 4;
   float top = 0.f;
   for (int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < n; row += warps) {
     float err = 0.f;
-    for (int b = lane; b < nblk; b += 32) {
-      const long long base = 1ll * row * K + 16 * b;
-      float v[16];
-      load16(w, base, v);
-      float amax = 0.f;
-#pragma unroll
-      for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(v[i]));
-      const uint8_t sbits = to_e4m3(clamp448(__fdiv_rn(amax, 6.f)));
-      const float scale = from_e4m3(sbits);
-      const float divisor = (scale == 0.f) ? 1.f : scale;
-      top = fmaxf(top, scale);
-      uint32_t packed[2] = {0u, 0u};
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const float ratio = __fdiv_rn(v[i], divisor);
-        const float mag = fabsf(ratio);
-        const int m = (mag > 0.25f) + (mag > 0.75f) + (mag > 1.25f) + (mag > 1.75f) + (mag > 2.5f) + (mag > 3.5f) + (mag > 5.0f);
-        const int code = m + ((ratio < 0.f) ? 8 : 0);
-        packed[i >> 3] |= static_cast<uint32_t>(code) << (4 * (i & 7));
-        // grid value: 0, .5, 1, 1.5 (m / 2) then 2, 3, 4, 6
-        const float g = (m < 4) ? 0.5f * m : (m == 7 ? 6.f : static_cast<float>(m - 2));
-        const float rec = __fmul_rn((ratio < 0.f) ? -g : g, scale);
-        const float d = v[i] - rec;
-        err = fmaf(d, d, err);
-      }
-      *reinterpret_cast<uint2 *>(codes + 1ll * row * (K >> 1) + 8 * b) = make_uint2(packed[0], packed[1]);
-      scales[1ll * row * nblk + b] = sbits;
-    }
-    if (row_sqerr) {
+    encode_row_fp4<T, SQERR>(w + 1ll * row * K, K, codes + 1ll * row * (K >> 1), scales + 1ll * row * (K >> 4), lane, top, err);
+    if (SQERR) {
       err = warp_sum(err);
       if (lane == 0) row_sqerr[row] = err;
     }
   }
   if (max_scale) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    top = warp_max(top);
     if (lane == 0 && top > 0.f) atomic_max_nonneg(max_scale, top);
   }
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) absmax_kernel(const T *__restrict__ w, long long count, float *__restrict__ out) {
+__global__ void __launch_bounds__(256) absmax_kernel(const T *__restrict__ w, int n, int K, float *__restrict__ out) {
+  const int lane = threadIdx.x & 31;
   float m = 0.f;
-  for (long long i = 1ll * blockIdx.x * blockDim.x + threadIdx.x; i < count; i += 1ll * gridDim.x * blockDim.x)
-    m = fmaxf(m, fabsf(load_elem(w, i)));
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0 && m > 0.f) atomic_max_nonneg(out, m);
+  for (int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < n; row += (gridDim.x * blockDim.x) >> 5)
+    m = fmaxf(m, absmax_row(w + 1ll * row * K, K, lane));
+  m = warp_max(m);
+  if (lane == 0 && m > 0.f) atomic_max_nonneg(out, m);
 }
 
-template <typename T>
+template <typename T, bool SQERR>
 __global__ void __launch_bounds__(256) quantize_fp8_kernel(const T *__restrict__ w, int n, int K, const float *__restrict__ absmax,
                                                            uint8_t *__restrict__ out, float *__restrict__ scale_out,
                                                            float *__restrict__ row_sqerr) {
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
-  float scale = __fdiv_rn(*absmax, 448.f);
-  if (scale == 0.f) scale = 1.f;
+  const float scale = fp8_scale(*absmax);
   for (int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < n; row += warps) {
     float err = 0.f;
-    for (int b = lane; b < (K >> 4); b += 32) {
-      const long long base = 1ll * row * K + 16 * b;
-      uint32_t o[4] = {0u, 0u, 0u, 0u};
-      float v[16];
-      load16(w, base, v);
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const uint8_t q = to_e4m3(clamp448(__fdiv_rn(v[i], scale)));
-        o[i >> 2] |= static_cast<uint32_t>(q) << (8 * (i & 3));
-        const float d = v[i] - __fmul_rn(from_e4m3(q), scale);
-        err = fmaf(d, d, err);
-      }
-      *reinterpret_cast<uint4 *>(out + base) = make_uint4(o[0], o[1], o[2], o[3]);
-    }
+    encode_row_fp8<T, SQERR>(w + 1ll * row * K, K, scale, out + 1ll * row * K, lane, err);
     if (lane == 0 && scale_out) scale_out[row] = scale;
-    if (row_sqerr) {
+    if (SQERR) {
       err = warp_sum(err);
       if (lane == 0) row_sqerr[row] = err;
     }
+  }
+}
+
+// ---- a whole layer: permuted row r is channel perm[r] of w
+struct LayerEncodeArgs {
+  const void *w;
+  const long long *perm;
+  int n4, n8, n16, K;
+  uint8_t *codes, *scales, *fp8;
+  float *fp8_scale;
+  __nv_bfloat16 *fp16;
+  float *tops;  // [0] largest NVFP4 block scale, [1] largest magnitude of the FP8 group; zero at first
+  float *global_scale;
+  int32_t *inv_perm;
+};
+__device__ __forceinline__ long long source_row(const LayerEncodeArgs &a, int r) {
+  const int n = a.n4 + a.n8 + a.n16;
+  long long s = a.perm[r];
+  if (s < 0) s += n;  // indices from the end, as in tensor indexing
+  return s < 0 || s >= n ? 0 : s;
+}
+
+// First pass over all rows: NVFP4 codes, the FP8 group's magnitude, FP16 rows, inverse permutation.
+template <typename T>
+__global__ void __launch_bounds__(256) encode_layer_kernel(LayerEncodeArgs a) {
+  pdl_launch_dependents();
+  const int lane = threadIdx.x & 31;
+  const int n = a.n4 + a.n8 + a.n16, K = a.K;
+  const T *w = static_cast<const T *>(a.w);
+  float top = 0.f, amax = 0.f, none = 0.f;
+  for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += (gridDim.x * blockDim.x) >> 5) {
+    const long long src = source_row(a, r);
+    const T *row = w + src * K;
+    if (lane == 0) a.inv_perm[src] = r;
+    if (r < a.n4) {
+      encode_row_fp4<T, false>(row, K, a.codes + 1ll * r * (K >> 1), a.scales + 1ll * r * (K >> 4), lane, top, none);
+    } else if (r < a.n4 + a.n8) {
+      amax = fmaxf(amax, absmax_row(row, K, lane));
+    } else {
+      // stored as the bf16 rounding of the f16 value
+      __nv_bfloat16 *dst = a.fp16 + 1ll * (r - a.n4 - a.n8) * K;
+      for (int i = lane; i < (K >> 3); i += 32) {
+        Vec8<T> q;
+        float v[8];
+        q.load(row + 8ll * i);
+        q.get(v);
+        uint4 o;
+        uint32_t *ow = reinterpret_cast<uint32_t *>(&o);
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          ow[e] = pack_y2(__half2float(__float2half_rn(v[2 * e])), __half2float(__float2half_rn(v[2 * e + 1])), 1);
+        reinterpret_cast<uint4 *>(dst)[i] = o;
+      }
+    }
+  }
+  top = warp_max(top);
+  amax = warp_max(amax);
+  if (lane == 0 && top > 0.f) atomic_max_nonneg(a.tops, top);
+  if (lane == 0 && amax > 0.f) atomic_max_nonneg(a.tops + 1, amax);
+}
+
+// Second pass: the FP8 rows (their scale is known now; they mostly come out of L2)
+template <typename T>
+__global__ void __launch_bounds__(256) encode_layer_fp8_kernel(LayerEncodeArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int lane = threadIdx.x & 31;
+  const T *w = static_cast<const T *>(a.w);
+  if (blockIdx.x == 0 && threadIdx.x == 0 && a.n4) a.global_scale[0] = a.tops[0] == 0.f ? 1.f : a.tops[0];
+  const float scale = fp8_scale(a.tops[1]);
+  float none = 0.f;
+  for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < a.n8; r += (gridDim.x * blockDim.x) >> 5) {
+    encode_row_fp8<T, false>(w + source_row(a, a.n4 + r) * a.K, a.K, scale, a.fp8 + 1ll * r * a.K, lane, none);
+    if (lane == 0) a.fp8_scale[r] = scale;
   }
 }
 
@@ -160,17 +362,46 @@ int grid_for_rows(int n) {
   return static_cast<int>(want < cap ? (want > 0 ? want : 1) : cap);
 }
 
+template <typename T>
+int run_layer(const LayerEncodeArgs &a, cudaStream_t stream) {
+  encode_layer_kernel<T><<<grid_for_rows(a.n4 + a.n8 + a.n16), 256, 0, stream>>>(a);
+  RDQ_CUDA(cudaGetLastError());
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid_for_rows(a.n8)));
+  cfg.blockDim = dim3(256);
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  RDQ_CUDA(cudaLaunchKernelEx(&cfg, encode_layer_fp8_kernel<T>, a));
+  return RDQ_OK;
+}
+
+template <typename T>
+void run_nvfp4(const void *w, int n, int K, uint8_t *codes, uint8_t *scales, float *row_sqerr, float *max_scale, cudaStream_t stream) {
+  const T *p = static_cast<const T *>(w);
+  const int grid = grid_for_rows(n);
+  if (row_sqerr) quantize_nvfp4_kernel<T, true><<<grid, 256, 0, stream>>>(p, n, K, codes, scales, row_sqerr, max_scale);
+  else quantize_nvfp4_kernel<T, false><<<grid, 256, 0, stream>>>(p, n, K, codes, scales, nullptr, max_scale);
+}
+template <typename T>
+void run_fp8(const void *w, int n, int K, uint8_t *out, float *scale_out, float *row_sqerr, float *absmax, cudaStream_t stream) {
+  const T *p = static_cast<const T *>(w);
+  const int grid = grid_for_rows(n);
+  absmax_kernel<T><<<grid, 256, 0, stream>>>(p, n, K, absmax);
+  if (row_sqerr) quantize_fp8_kernel<T, true><<<grid, 256, 0, stream>>>(p, n, K, absmax, out, scale_out, row_sqerr);
+  else quantize_fp8_kernel<T, false><<<grid, 256, 0, stream>>>(p, n, K, absmax, out, scale_out, nullptr);
+}
+
 }  // namespace
 
 int launch_quantize_nvfp4(const void *w, bool w_is_f32, int n, int K, uint8_t *codes, uint8_t *scales, float *row_sqerr,
                           float *max_scale, cudaStream_t stream) {
   if (max_scale) RDQ_CUDA(cudaMemsetAsync(max_scale, 0, sizeof(float), stream));
-  const int grid = grid_for_rows(n);
-  if (w_is_f32)
-    quantize_nvfp4_kernel<float><<<grid, 256, 0, stream>>>(static_cast<const float *>(w), n, K, codes, scales, row_sqerr, max_scale);
-  else
-    quantize_nvfp4_kernel<__half><<<grid, 256, 0, stream>>>(static_cast<const __half *>(w), n, K, codes, scales, row_sqerr,
-                                                           max_scale);
+  if (w_is_f32) run_nvfp4<float>(w, n, K, codes, scales, row_sqerr, max_scale, stream);
+  else run_nvfp4<__half>(w, n, K, codes, scales, row_sqerr, max_scale, stream);
   RDQ_CUDA(cudaGetLastError());
   return RDQ_OK;
 }
@@ -178,23 +409,43 @@ int launch_quantize_nvfp4(const void *w, bool w_is_f32, int n, int K, uint8_t *c
 int launch_quantize_fp8(const void *w, bool w_is_f32, int n, int K, uint8_t *out, float *scale_out, float *row_sqerr,
                         float *absmax_scratch, cudaStream_t stream) {
   RDQ_CUDA(cudaMemsetAsync(absmax_scratch, 0, sizeof(float), stream));
-  const long long count = 1ll * n * K;
-  long long blocks = (count + 256 * 16 - 1) / (256 * 16);
-  const long long cap = 1ll * sm_count() * 8;
-  if (blocks > cap) blocks = cap;
-  if (blocks < 1) blocks = 1;
-  const int grid = grid_for_rows(n);
-  if (w_is_f32) {
-    absmax_kernel<float><<<static_cast<int>(blocks), 256, 0, stream>>>(static_cast<const float *>(w), count, absmax_scratch);
-    quantize_fp8_kernel<float><<<grid, 256, 0, stream>>>(static_cast<const float *>(w), n, K, absmax_scratch, out, scale_out,
-                                                        row_sqerr);
-  } else {
-    absmax_kernel<__half><<<static_cast<int>(blocks), 256, 0, stream>>>(static_cast<const __half *>(w), count, absmax_scratch);
-    quantize_fp8_kernel<__half><<<grid, 256, 0, stream>>>(static_cast<const __half *>(w), n, K, absmax_scratch, out, scale_out,
-                                                         row_sqerr);
-  }
+  if (w_is_f32) run_fp8<float>(w, n, K, out, scale_out, row_sqerr, absmax_scratch, stream);
+  else run_fp8<__half>(w, n, K, out, scale_out, row_sqerr, absmax_scratch, stream);
   RDQ_CUDA(cudaGetLastError());
   return RDQ_OK;
 }
 
 }  // namespace rdq
+
+using namespace rdq;
+
+extern "C" int rdq_quantize_layer(const void *w, int w_is_f32, const long long *perm, int n_fp4, int n_fp8, int n_fp16, int K,
+                                  void *codes, void *scales, float *global_scale, void *fp8, float *fp8_scale, void *fp16_bf16,
+                                  int32_t *inv_perm, float *scratch, void *stream_) {
+  RDQ_REQUIRE(n_fp4 >= 0 && n_fp8 >= 0 && n_fp16 >= 0 && K > 0 && K % 16 == 0, RDQ_E_INVALID,
+              "rdq_quantize_layer needs K a positive multiple of 16 (n=%d/%d/%d K=%d)", n_fp4, n_fp8, n_fp16, K);
+  if (n_fp4 + n_fp8 + n_fp16 == 0) return RDQ_OK;
+  RDQ_REQUIRE(w && perm && inv_perm && scratch && (!n_fp4 || (codes && scales && global_scale)) && (!n_fp8 || (fp8 && fp8_scale)) &&
+                  (!n_fp16 || fp16_bf16),
+              RDQ_E_INVALID, "null pointer");
+  RDQ_REQUIRE(aligned16(w) && aligned16(codes) && aligned16(fp8) && aligned16(fp16_bf16), RDQ_E_INVALID,
+              "w and the outputs must be 16-byte aligned");
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  RDQ_CUDA(cudaMemsetAsync(scratch, 0, 2 * sizeof(float), stream));
+  LayerEncodeArgs a;
+  a.w = w;
+  a.perm = perm;
+  a.n4 = n_fp4;
+  a.n8 = n_fp8;
+  a.n16 = n_fp16;
+  a.K = K;
+  a.codes = static_cast<uint8_t *>(codes);
+  a.scales = static_cast<uint8_t *>(scales);
+  a.fp8 = static_cast<uint8_t *>(fp8);
+  a.fp8_scale = fp8_scale;
+  a.fp16 = static_cast<__nv_bfloat16 *>(fp16_bf16);
+  a.tops = scratch;
+  a.global_scale = global_scale;
+  a.inv_perm = inv_perm;
+  return w_is_f32 ? run_layer<float>(a, stream) : run_layer<__half>(a, stream);
+}

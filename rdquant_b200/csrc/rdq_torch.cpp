@@ -13,11 +13,13 @@
 // Reference counterpart: the pybind wrappers of rdquant/csrc/bindings.cpp:156-201.
 #include <Python.h>
 
+#include <ATen/EmptyTensor.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <initializer_list>
 #include <new>
 #include <vector>
 
@@ -184,6 +186,134 @@ PyObject *layer_linear(PyObject *obj, PyObject *const *args, Py_ssize_t nargs) {
   }
 }
 
+at::Tensor cuda_empty(at::IntArrayRef sizes, at::ScalarType type, c10::DeviceIndex device) {
+  return at::detail::empty_cuda(sizes, type, c10::Device(c10::kCUDA, device), std::nullopt);
+}
+PyObject *wrap_or_none(at::Tensor t) {
+  if (!t.defined()) Py_RETURN_NONE;
+  return THPVariable_Wrap(std::move(t));
+}
+// a contiguous CUDA tensor of one of the given types on `device` (any device if < 0), or null
+const at::Tensor *cuda_arg(PyObject *o, c10::DeviceIndex device, std::initializer_list<at::ScalarType> types) {
+  if (!THPVariable_Check(o)) return nullptr;
+  const at::Tensor &t = THPVariable_Unpack(o);
+  if (!t.is_cuda() || !t.is_contiguous() || (device >= 0 && t.get_device() != device)) return nullptr;
+  for (auto type : types)
+    if (t.scalar_type() == type) return &t;
+  return nullptr;
+}
+bool int_args(PyObject *const *args, int n, long *out) {
+  for (int i = 0; i < n; ++i) {
+    out[i] = PyLong_AsLong(args[i]);
+    if (out[i] == -1 && PyErr_Occurred()) return false;
+  }
+  return true;
+}
+
+// quantize_layer(weight [N, K], perm int64 [N], n4, n8, n16) -> (codes, scales, global_scale, fp8, fp8_scale,
+// fp16, inv_perm, splits int32 [3] on the host), absent groups None; None when the input needs conversions first
+PyObject *quantize_layer(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
+  long n[3];
+  if (nargs != 5) {
+    PyErr_SetString(PyExc_TypeError, "quantize_layer(weight, perm, n4, n8, n16)");
+    return nullptr;
+  }
+  const at::Tensor *w = cuda_arg(args[0], -1, {at::kHalf, at::kFloat});
+  if (w == nullptr || w->dim() != 2) Py_RETURN_NONE;
+  const c10::DeviceIndex dev = w->get_device();
+  const at::Tensor *perm = cuda_arg(args[1], dev, {at::kLong});
+  if (!int_args(args + 2, 3, n)) return nullptr;
+  const int64_t N = w->size(0), K = w->size(1);
+  if (perm == nullptr || perm->numel() != N || n[0] < 0 || n[1] < 0 || n[2] < 0 || n[0] + n[1] + n[2] != N || K % 16 || K == 0 ||
+      N == 0 || N > 0x7fffffff || K > 0x7fffffff || (reinterpret_cast<uintptr_t>(w->data_ptr()) & 15))
+    Py_RETURN_NONE;
+  try {
+    OnDevice guard(dev);
+    at::Tensor codes, scales, top, fp8, fp8_scale, fp16;
+    if (n[0]) {
+      codes = cuda_empty({n[0], K / 2}, at::kByte, dev);
+      scales = cuda_empty({n[0], K / 16}, at::kByte, dev);
+      top = cuda_empty({1}, at::kFloat, dev);
+    }
+    if (n[1]) {
+      fp8 = cuda_empty({n[1], K}, at::kByte, dev);
+      fp8_scale = cuda_empty({n[1]}, at::kFloat, dev);
+    }
+    if (n[2]) fp16 = cuda_empty({n[2], K}, at::kBFloat16, dev);
+    at::Tensor inv = cuda_empty({N}, at::kInt, dev), scratch = cuda_empty({2}, at::kFloat, dev);
+    auto ptr = [](const at::Tensor &t) { return t.defined() ? t.data_ptr() : nullptr; };
+    const int rc = rdq_quantize_layer(w->data_ptr(), w->scalar_type() == at::kFloat, static_cast<const long long *>(perm->data_ptr()),
+                                      static_cast<int>(n[0]), static_cast<int>(n[1]), static_cast<int>(n[2]), static_cast<int>(K),
+                                      ptr(codes), ptr(scales), static_cast<float *>(ptr(top)), ptr(fp8),
+                                      static_cast<float *>(ptr(fp8_scale)), ptr(fp16), static_cast<int32_t *>(inv.data_ptr()),
+                                      static_cast<float *>(scratch.data_ptr()), c10::cuda::getCurrentCUDAStream(dev).stream());
+    if (rc != RDQ_OK) {
+      PyErr_Format(PyExc_RuntimeError, "rdq_quantize_layer failed (code %d): %s", rc, rdq_last_error());
+      return nullptr;
+    }
+    at::Tensor splits = at::detail::empty_cpu({3}, at::kInt);
+    for (int i = 0; i < 3; ++i) static_cast<int32_t *>(splits.data_ptr())[i] = static_cast<int32_t>(n[i]);
+    return Py_BuildValue("NNNNNNNN", wrap_or_none(std::move(codes)), wrap_or_none(std::move(scales)), wrap_or_none(std::move(top)),
+                         wrap_or_none(std::move(fp8)), wrap_or_none(std::move(fp8_scale)), wrap_or_none(std::move(fp16)),
+                         wrap_or_none(std::move(inv)), wrap_or_none(std::move(splits)));
+  } catch (const std::exception &e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+    return nullptr;
+  }
+}
+
+// dequantize(w4, s4, w8, s8, w16, inv_perm or None, n4, n8, n16, k) -> f16 [N, K], or None when an argument needs the
+// checked path.  Groups of size 0 are not looked at.
+PyObject *dequantize(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
+  long n[4];
+  if (nargs != 10) {
+    PyErr_SetString(PyExc_TypeError, "dequantize(w4, s4, w8, s8, w16, inv_perm, n4, n8, n16, k)");
+    return nullptr;
+  }
+  if (!int_args(args + 6, 4, n)) return nullptr;
+  const int64_t K = n[3], N = n[0] + n[1] + n[2];
+  if (n[0] < 0 || n[1] < 0 || n[2] < 0 || N <= 0 || K <= 0) Py_RETURN_NONE;
+  c10::DeviceIndex dev = -1;
+  const void *p[6] = {};
+  bool bf16 = false;
+  auto take_arg = [&](int i, std::initializer_list<at::ScalarType> types, int64_t numel) {
+    const at::Tensor *t = cuda_arg(args[i], dev, types);
+    if (t == nullptr || t->numel() != numel) return false;
+    if (i != 3 && i != 5 && (t->dim() != 2 || t->size(0) != (i == 4 ? n[2] : n[i / 2]))) return false;
+    dev = t->get_device();
+    p[i] = t->data_ptr();
+    if (i == 4) bf16 = t->scalar_type() == at::kBFloat16;
+    return true;
+  };
+  if (n[0] && !(take_arg(0, {at::kByte}, n[0] * (K / 2)) && take_arg(1, {at::kByte}, n[0] * (K / 16)))) Py_RETURN_NONE;
+  if (n[1] && !(take_arg(2, {at::kByte}, n[1] * K) && take_arg(3, {at::kFloat}, n[1]))) Py_RETURN_NONE;
+  if (n[2] && !take_arg(4, {at::kHalf, at::kBFloat16}, n[2] * K)) Py_RETURN_NONE;
+  if (args[5] != Py_None && !take_arg(5, {at::kInt}, N)) Py_RETURN_NONE;
+  try {
+    OnDevice guard(dev);
+    at::Tensor out = cuda_empty({N, K}, at::kHalf, dev);
+    const int rc = rdq_dequant_packed(p[0], p[1], 1.0f, p[2], static_cast<const float *>(p[3]), p[4], bf16,
+                                      static_cast<const int32_t *>(p[5]), out.data_ptr(), 0, static_cast<int>(n[0]),
+                                      static_cast<int>(n[1]), static_cast<int>(n[2]), static_cast<int>(K),
+                                      c10::cuda::getCurrentCUDAStream(dev).stream());
+    if (rc != RDQ_OK) {
+      PyErr_Format(PyExc_RuntimeError, "rdq_dequant_packed failed (code %d): %s", rc, rdq_last_error());
+      return nullptr;
+    }
+    return THPVariable_Wrap(std::move(out));
+  } catch (const std::exception &e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+    return nullptr;
+  }
+}
+
+PyMethodDef module_methods[] = {
+    {"quantize_layer", reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(quantize_layer)), METH_FASTCALL,
+     "packed tensors of a layer, or None when the input needs conversions first"},
+    {"dequantize", reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(dequantize)), METH_FASTCALL,
+     "f16 weight of a packed layer, or None when an argument needs the checked path"},
+    {nullptr, nullptr, 0, nullptr}};
+
 PyMethodDef layer_methods[] = {
     {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(layer_linear)), METH_FASTCALL,
      "linear(x, bias, flags): y = x @ W.T (+ bias), or None when the input needs the checked path"},
@@ -191,7 +321,7 @@ PyMethodDef layer_methods[] = {
 
 PyTypeObject layer_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
-PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_rdq_torch", "native host path of the packed layers", -1, nullptr};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_rdq_torch", "native host path of the packed layers", -1, module_methods};
 
 }  // namespace
 

@@ -16,6 +16,7 @@ from typing import Optional
 import torch
 import torch.nn as nn
 
+from rdquant_b200 import _lib
 from rdquant_b200.core.formats import QuantizedTensor, get_bits_per_element, quantize
 
 FORMAT_ORDER = ("NVFP4", "FP8", "FP16")
@@ -116,9 +117,18 @@ def quantize_weight_packed(weight: torch.Tensor, permutation: torch.Tensor, spli
     perm = permutation.to(device=weight.device, dtype=torch.long)
     if sum(splits.get(f, 0) for f in FORMAT_ORDER) != n_out:
         raise ValueError("splits must sum to the number of output channels")
-    grouped = weight[perm]
-    if grouped.dtype not in (torch.float16, torch.float32):
-        grouped = grouped.float()
+    sizes = [int(splits.get(f, 0)) for f in FORMAT_ORDER]
+    w = weight if weight.dtype in (torch.float16, torch.float32) else weight.float()
+    # two launches that gather the rows as they encode them; None: a shape or layout it does not take
+    packed = _lib.torch_ext().quantize_layer(w.contiguous(), perm.contiguous(), *sizes)
+    if packed is not None:
+        out = {"splits": packed[7], "inv_permutation": packed[6]}
+        names = ("weight_nvfp4", "weight_nvfp4_scale", "nvfp4_global_scale", "weight_fp8", "weight_fp8_scale", "weight_fp16")
+        out.update((name, t) for name, t in zip(names, packed) if t is not None)
+        if bias is not None:
+            out["bias"] = bias.detach().clone()
+        return out
+    grouped = w[perm]
     out = {
         "splits": torch.tensor([int(splits.get(f, 0)) for f in FORMAT_ORDER], dtype=torch.int32),
         "inv_permutation": inverse_permutation(perm).to(torch.int32),

@@ -125,6 +125,13 @@ def dequantize_packed(layer_data: dict, splits: dict, k: int, inv_perm: Optional
     float32 the unrounded products of ``formats.dequantize``.
     """
     n4, n8, n16 = (int(splits.get(f, 0)) for f in ("NVFP4", "FP8", "FP16"))
+    if out_dtype is torch.float16 and global_scale == 1.0:
+        # native call; None: an argument that needs the conversions and messages below
+        get = layer_data.get
+        out = _lib.torch_ext().dequantize(get("weight_nvfp4"), get("weight_nvfp4_scale"), get("weight_fp8"),
+                                          get("weight_fp8_scale"), get("weight_fp16"), inv_perm, n4, n8, n16, int(k))
+        if out is not None:
+            return out
     w4 = layer_data.get("weight_nvfp4") if n4 else None
     s4 = layer_data.get("weight_nvfp4_scale") if n4 else None
     w8 = layer_data.get("weight_fp8") if n8 else None
@@ -317,9 +324,9 @@ def mixed_linear(x: torch.Tensor, fd: dict, bias: Optional[torch.Tensor] = None,
     """GEMV for M <= 16, GEMM above."""
     if x.shape[0] <= MAX_GEMV_M:
         return mixed_gemv(x, fd, bias, flags, out=out)
-    if fd["k"] % 16 == 0 and fd.get("row_major", True):
+    if fd["k"] % 64 == 0 and fd.get("row_major", True):
         return mixed_gemm(x, fd, bias, out=out)
-    # the tensor-core GEMM reads the row-major tensors by TMA (K a multiple of 16); other K, and
+    # this entry point's tensor-core GEMM tiles K in blocks of 64 and reads the row-major tensors; other K, and
     # layers packed without them, run the decode kernel over 16-row panels (the reference's
     # dense prefill takes any K, rdquant/inference.py:679-687)
     n = fd["n_fp4"] + fd["n_fp8"] + fd["n_fp16"]
