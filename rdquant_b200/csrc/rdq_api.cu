@@ -314,8 +314,7 @@ int rdq_gemm_mixed_ws(const void *x, int M, const void *w_fp4, const void *w_fp4
   if (M == 0 || n_fp4 + n_fp8 + n_fp16 == 0) return RDQ_OK;
   RDQ_REQUIRE(x != nullptr && y != nullptr, RDQ_E_INVALID, "x and y must not be null");
   RDQ_REQUIRE(aligned16(x) && aligned16(y), RDQ_E_INVALID, "x and y must be 16-byte aligned");
-  RDQ_REQUIRE(K % 64 == 0 || (workspace && gemm_dense_takes(K)), RDQ_E_UNSUPPORTED,
-              "rdq_gemm_mixed needs K to be a multiple of 64 (of 16 with a workspace), got K=%d", K);
+  RDQ_REQUIRE(K % 64 == 0, RDQ_E_UNSUPPORTED, "rdq_gemm_mixed needs K to be a multiple of 64, got K=%d", K);
   // the kernel addresses each weight tensor with 32-bit byte offsets
   RDQ_REQUIRE(1ll * n_fp4 * (K / 2) < (1ll << 32) && 1ll * n_fp8 * K < (1ll << 32) && 2ll * n_fp16 * K < (1ll << 32),
               RDQ_E_UNSUPPORTED, "rdq_gemm_mixed: a format group of this layer exceeds 4 GB");
@@ -351,7 +350,7 @@ int rdq_gemm_mixed(const void *x, int M, const void *w_fp4, const void *w_fp4_sc
 
 int rdq_gemm_workspace_size(int M, int N, int K, size_t *bytes) {
   RDQ_REQUIRE(bytes != nullptr, RDQ_E_INVALID, "bytes must not be null");
-  RDQ_REQUIRE(M >= 0 && N >= 0 && K > 0 && (K % 64 == 0 || gemm_dense_takes(K)), RDQ_E_INVALID, "rdq_gemm_workspace_size: bad shape M=%d N=%d K=%d", M, N, K);
+  RDQ_REQUIRE(M >= 0 && N >= 0 && K > 0 && K % 64 == 0, RDQ_E_INVALID, "rdq_gemm_workspace_size: bad shape M=%d N=%d K=%d", M, N, K);
   *bytes = (M == 0 || N == 0) ? 0 : gemm_workspace_bytes(M, N, K);
   return RDQ_OK;
 }

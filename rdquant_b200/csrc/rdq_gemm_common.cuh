@@ -97,6 +97,25 @@ __device__ __forceinline__ bool gemm_wait_cluster(uint64_t *bar, uint32_t parity
   *abort_flag = 1;
   return false;
 }
+// The bounded wait as one asm block without branches that the compiler could see: 0 when it ran out
+// (20000 tries of up to 50 us).
+__device__ __forceinline__ uint32_t wait_bounded(uint32_t bar, uint32_t parity) {
+  uint32_t left;
+  asm volatile(
+      "{\n.reg .pred p, q;\n"
+      "mov.u32 %0, 20000;\n"
+      "WAIT_%=:\n"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
+      "@p bra DONE_%=;\n"
+      "sub.u32 %0, %0, 1;\n"
+      "setp.ne.u32 q, %0, 0;\n"
+      "@q bra WAIT_%=;\n"
+      "DONE_%=:\n}\n"
+      : "=&r"(left)
+      : "r"(bar), "r"(parity), "r"(50000u)
+      : "memory");
+  return left;
+}
 // Wait (bounded, about 0.4 s) until the low half of a global word reaches `count`; the thread that is
 // the last of `parts` to pass puts the word back to zero.
 __device__ __forceinline__ bool wait_arrivals(uint32_t *word, uint32_t count, uint32_t parts) {

@@ -188,15 +188,17 @@ __device__ __forceinline__ WorkItem work_item(const PairArgs &a, int item) {
   return w;
 }
 
-// The four epilogue warps: wait for all parts of a split tile, add and store this part's tokens.
+// The four epilogue warps: wait for all parts of a split tile, add and store this part's tokens.  A
+// warp takes every fourth token, a lane four channels, with the loads of four tokens in flight.
 template <bool BF16>
 __device__ __forceinline__ void finish_shared(const PairArgs &a, const WorkItem &w, uint32_t rank, int q, int lane,
                                               volatile int *abort_flag) {
-  const int ch = w.n * 256 + static_cast<int>(rank) * 128 + q * 32 + lane;
-  float scl = 0.f, bia = 0.f;
-  if (ch < a.N) {
-    scl = a.scale[ch];
-    bia = a.bias ? __half2float(a.bias[ch]) : 0.f;
+  const int ch = w.n * 256 + static_cast<int>(rank) * 128 + lane * 4;
+  float scl[4], bia[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    scl[e] = ch + e < a.N ? a.scale[ch + e] : 0.f;
+    bia[e] = ch + e < a.N && a.bias ? __half2float(a.bias[ch + e]) : 0.f;
   }
   if (q == 0 && lane == 0 && !wait_arrivals(a.counters + w.rem * 2 + rank, 4u * a.parts, a.parts)) *abort_flag = 1;
   asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -204,21 +206,42 @@ __device__ __forceinline__ void finish_shared(const PairArgs &a, const WorkItem 
   const int tok0 = w.m * a.nt, ntok = min(a.nt, a.M - tok0);
   const int lo = ntok * w.part / a.parts, hi = ntok * (w.part + 1) / a.parts;
   const long long part_stride = 2ll * a.nt * 128;
-  const float *src = a.partial + (1ll * w.rem * a.parts * 2 + rank) * a.nt * 128 + q * 32 + lane;
-  constexpr int kTok = 16;
+  const float *src = a.partial + (1ll * w.rem * a.parts * 2 + rank) * a.nt * 128 + lane * 4;
+  const bool vec = (a.N & 3) == 0 && ch + 4 <= a.N;
+  constexpr int kTok = 4;
 #pragma unroll 1
-  for (int t0 = lo; t0 < hi; t0 += kTok) {
-    float p[kMaxParts][kTok];  // all loads in flight together
+  for (int t0 = lo + q; t0 < hi; t0 += 4 * kTok) {
+    float4 p[kMaxParts][kTok];
 #pragma unroll
     for (int b = 0; b < kMaxParts; ++b)
 #pragma unroll
-      for (int e = 0; e < kTok; ++e) p[b][e] = b < a.parts && t0 + e < hi ? __ldcg(src + b * part_stride + (t0 + e) * 128) : 0.f;
+      for (int e = 0; e < kTok; ++e)
+        p[b][e] = b < a.parts && t0 + 4 * e < hi
+                      ? __ldcg(reinterpret_cast<const float4 *>(src + b * part_stride + (t0 + 4 * e) * 128))
+                      : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int e = 0; e < kTok; ++e) {
-      float v = p[0][e];
+      if (t0 + 4 * e >= hi) break;
+      float4 v = p[0][e];
 #pragma unroll
-      for (int b = 1; b < kMaxParts; ++b) v += p[b][e];
-      if (t0 + e < hi && ch < a.N) store_y(a.y, 1ll * (tok0 + t0 + e) * a.N + ch, fmaf(v, scl, bia), BF16);
+      for (int b = 1; b < kMaxParts; ++b) {
+        v.x += p[b][e].x;
+        v.y += p[b][e].y;
+        v.z += p[b][e].z;
+        v.w += p[b][e].w;
+      }
+      const uint32_t h0 = pack_y2(fmaf(v.x, scl[0], bia[0]), fmaf(v.y, scl[1], bia[1]), BF16);
+      const uint32_t h1 = pack_y2(fmaf(v.z, scl[2], bia[2]), fmaf(v.w, scl[3], bia[3]), BF16);
+      uint16_t *dst = static_cast<uint16_t *>(a.y) + 1ll * (tok0 + t0 + 4 * e) * a.N + ch;
+      if (vec) {
+        *reinterpret_cast<uint2 *>(dst) = make_uint2(h0, h1);
+      } else {
+        const uint16_t h[4] = {static_cast<uint16_t>(h0), static_cast<uint16_t>(h0 >> 16), static_cast<uint16_t>(h1),
+                               static_cast<uint16_t>(h1 >> 16)};
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (ch + u < a.N) dst[u] = h[u];
+      }
     }
   }
 }
@@ -431,29 +454,55 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
 }
 
 struct PairPlan {
+  double cycles;  // estimate
   int nt, m_tiles, n_tiles, clusters, full, parts;
 };
-// Token tiles of equal width (a multiple of 32); whole tiles while they fill all SM pairs, the
-// rest split along k into as many parts as there are pairs for it -- at most four, because every
-// part's sums are written and read once more, and only while a part keeps 12 k blocks.
-PairPlan pair_plan(int M, int N, int K) {
-  PairPlan p;
-  p.m_tiles = (M + 255) / 256;
-  p.nt = ((M + p.m_tiles - 1) / p.m_tiles + 31) / 32 * 32;
-  p.m_tiles = (M + p.nt - 1) / p.nt;
-  p.n_tiles = (N + 255) / 256;
-  p.clusters = sm_count() / 2;
-  const int tiles = p.m_tiles * p.n_tiles, kblocks = (K + 63) / 64;
-  p.full = tiles / p.clusters * p.clusters;
-  const int rem = tiles - p.full;
-  p.parts = rem ? std::min({p.clusters / rem, kMaxParts, std::max(1, kblocks / 12)}) : 1;
-  if (p.parts < 2) {
-    p.parts = 1;
-    p.full = tiles;
+// Chosen by estimated cycles among token tiles of equal width (a multiple of 32 up to 256).  A k block
+// costs its MMAs or its loads (64 B/clk of L2 bandwidth per SM); whole tiles run in waves over all SM
+// pairs; the tiles after the last full wave may be split along k into 2 .. 4 parts, whose FP32 sums
+// are written and read once more: about 60 cycles per token of the tile and 4000 for the exchange
+// (measured on tiles of 256 tokens: a split that leaves every part 20 k blocks gains nothing).
+PairPlan make_pair_plan(int M, int N, int K) {
+  PairPlan best{};
+  double best_t = 0;
+  const int pairs = std::max(1, sm_count() / 2), kblocks = (K + 63) / 64;
+  const int lo = (M + 255) / 256, hi = std::max(lo, std::min((M + 95) / 96, lo + 12));
+  for (int mt = lo; mt <= hi; ++mt) {
+    PairPlan p;
+    p.nt = ((M + mt - 1) / mt + 31) / 32 * 32;
+    p.m_tiles = (M + p.nt - 1) / p.nt;
+    p.n_tiles = (N + 255) / 256;
+    const int tiles = p.m_tiles * p.n_tiles;
+    const int waves = tiles / pairs, rem = tiles - waves * pairs;
+    const double kb = std::max(2.0 * p.nt, 256.0 + p.nt);
+    for (int parts = 1; parts <= kMaxParts; ++parts) {
+      if (parts > 1 && (rem == 0 || rem * parts > pairs || kblocks / parts < 4)) break;
+      const double t = waves * kblocks * kb + (rem ? (kblocks + parts - 1) / parts * kb + (parts > 1 ? 4000.0 + 60.0 * p.nt : 0.0) : 0.0);
+      if (best_t == 0 || t < best_t) {
+        best_t = t;
+        p.cycles = t;
+        p.parts = parts;
+        p.full = parts > 1 ? waves * pairs : tiles;
+        p.clusters = std::min(pairs, p.full + (tiles - p.full) * parts);
+        best = p;
+      }
+    }
   }
-  const int items = p.full + (tiles - p.full) * p.parts;
-  if (items < p.clusters) p.clusters = items;
-  return p;
+  return best;
+}
+// (a call asks for its plan three times)
+const PairPlan &pair_plan(int M, int N, int K) {
+  static thread_local PairPlan plan;
+  static thread_local int key[4] = {-1, -1, -1, -1};
+  const int sms = sm_count();
+  if (key[0] != M || key[1] != N || key[2] != K || key[3] != sms) {
+    plan = make_pair_plan(M, N, K);
+    key[0] = M;
+    key[1] = N;
+    key[2] = K;
+    key[3] = sms;
+  }
+  return plan;
 }
 
 size_t up256(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
@@ -475,6 +524,8 @@ DenseLayout dense_layout(const PairPlan &p, int N, int K) {
 }  // namespace
 
 bool gemm_dense_takes(int K) { return K % 16 == 0; }  // 16-byte row pitch for TMA, whole runs of 8 k
+
+double gemm_dense_cycles(int M, int N, int K) { return pair_plan(M, N, K).cycles; }
 
 size_t gemm_dense_workspace(int M, int N, int K) { return dense_layout(pair_plan(M, N, K), N, K).total; }
 

@@ -522,7 +522,6 @@ int launch_gemm(const GemmArgs &a, void *workspace, size_t workspace_bytes, cuda
   b.test_timeout = gemm_test_timeout();
   if (workspace != nullptr && gemm_dense_takes(a.K) && workspace_bytes >= gemm_dense_workspace(a.M, N, a.K))
     return launch_gemm_dense(b, workspace, workspace_bytes, stream);
-  RDQ_REQUIRE(a.K % 64 == 0, RDQ_E_UNSUPPORTED, "the GEMM without a workspace needs K to be a multiple of 64, got K=%d", a.K);
   CUtensorMap xmap;
   const int rc = encode_f16_2d(&xmap, a.x, a.K, a.M, BK, BM);
   if (rc != RDQ_OK) return rc;

@@ -18,28 +18,29 @@
 // parts in CTA order: the result does not depend on timing.  A second kernel for these sums cost
 // 4-7 us per layer, and one CTA per tile adding them up to 13 us.
 //
-// A stage of the pipeline is 128 k: 64 tensor-memory columns of weights and two 64-k activation
-// boxes, on one barrier.  The issuing warp spends about 190 cycles per barrier wait and 40 per MMA
-// whatever the number of tokens, so with 64-k stages and a barrier per operand it took 640 cycles per
-// 64 k; a CTA's share of the HBM rate asks for 64 k every 250.
+// A stage of the pipeline is one chunk: up to 128 tensor-memory columns of weights and up to four
+// 64-k activation boxes, on one barrier.  Every barrier wait of the issuing warp costs about 190 cycles
+// and every hand-over of a converter group 300 to 1000, whatever the number of tokens: with 64-k
+// stages the issuing warp needed 640 cycles per 64 k, with 128-k stages the converters 300, and a
+// CTA's share of the HBM rate asks for 64 k every 250.
 //
 // Roles of a CTA's warps:
 //   0        TMA of weight chunks (128 x 128 B boxes out of the row-major tensors, 128B swizzle)
-//   1        TMA of activation boxes (tokens x 64 k); executes griddepcontrol.wait
+//   1        TMA of activation boxes (tokens x 64 k)
 //   2        MMA issue; tensor-memory allocation
 //   3        block scales of NVFP4 chunks by cp.async, on the chunk's barrier
 //   4-7      epilogue: tcgen05.ld, channel scale + bias, stores to y[token, perm[row]]
-//   8-15     converters, two groups of four warps (a warp per 32 tensor-memory lanes) taking chunks in
-//            turn (four groups are no faster)
+//   8-       converters, a group of four warps (a warp per 32 tensor-memory lanes) per stage: three
+//            groups for up to 64 tokens, two above (the accumulators take more tensor memory)
 // Every launch is programmatic: it overlaps the end of the kernel before.  With RDQ_GEMV_PDL the
-// weight and scale loads start before the grid-dependency wait, so that the rings fill meanwhile.  The variant for up to 32 tokens takes half an SM
-// (256 tensor-memory columns, 64 registers, about 110 KB), so that the next layer's CTA fits beside it.
+// weight and scale loads start before the grid-dependency wait.
 //
 // Reference behaviour replaced: 2 x marlin_gemm + F.linear + cat + index_select
 // (rdquant/inference.py:620-677).
 #include <cuda.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <unordered_map>
 
 #include "rdq_gemm_common.cuh"
@@ -49,11 +50,17 @@ namespace rdq {
 
 namespace {
 
-constexpr int kGroups = 2;  // converter groups
-constexpr int kThreads = (8 + 4 * kGroups) * 32;
+// tokens per tile -> pipeline stages = converter groups: two accumulators of that many columns and
+// 128 columns per stage share the 512 columns
+template <int NT>
+constexpr int kStages = (512 - 2 * NT) / 128;
+template <int NT>
+constexpr int kThreads = (8 + 4 * kStages<NT>) * 32;
+constexpr int kFinishThreads = 512;
 constexpr int kChunkBytes = 128 * 128;
 constexpr int kScaleBytes = 128 * 16;
-constexpr int kMaxRing = 16;
+constexpr int kMaxRing = 8;
+constexpr int kSmemMax = 222 * 1024;
 constexpr int kMaxTokens = 128;   // per token tile
 constexpr int kMaxCtas = 160;
 
@@ -93,7 +100,6 @@ struct StreamArgs {
   const int32_t *perm;
   const __half *bias;
   void *y;
-  int y_bf16;
   int n4, n8, n16, K, N;
   float *partial;    // [2 * CTA + (0 first, 1 last segment)][token][128 rows]
   uint32_t *arrived;  // [CTA in which a cut tile starts]: epilogue warps done (low half), CTAs past the wait (high half)
@@ -105,7 +111,7 @@ struct StreamArgs {
 
 struct StreamSmem {
   uint64_t w_full[kMaxRing], w_empty[kMaxRing];
-  uint64_t full[4], empty[4];
+  uint64_t full[3], empty[3];
   uint64_t d_full[2], d_empty[2];
   uint64_t never;
   uint32_t tmem_base;
@@ -170,13 +176,27 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
       : "r"(taddr)
       : "memory");
 }
-// D (+)= A(tensor memory) . B(smem)^T
-__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+// D (+)= A(tensor memory) . B(smem)^T.  The descriptor comes in halves: only the low one changes from
+// MMA to MMA, and every operand that changes costs the issuing warp a register move.
+__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t db_lo, uint32_t db_hi, uint32_t idesc,
+                                            uint32_t accumulate) {
   asm volatile(
-      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(tmem_d),
-      "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate)
+      "{\n.reg .pred p;\n.reg .b64 db;\nsetp.ne.b32 p, %5, 0;\nmov.b64 db, {%2, %3};\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n}\n" ::"r"(tmem_d),
+      "r"(tmem_a), "r"(db_lo), "r"(db_hi), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+// the MMAs of B k blocks of 64
+template <int B>
+__device__ __forceinline__ void issue_blocks(uint32_t acc, uint32_t wa, uint32_t dx, uint32_t dx_hi, uint32_t box, uint32_t idesc,
+                                             uint32_t accumulate) {
+#pragma unroll
+  for (int b = 0; b < B; ++b) {
+#pragma unroll
+    for (int k4 = 0; k4 < 4; ++k4)
+      umma_f16_ts(acc, wa + 32 * b + 8 * k4, dx + 2 * k4, dx_hi, idesc, b == 0 && k4 == 0 ? accumulate : 1u);
+    dx += box;
+  }
 }
 
 // half a k block (32 k) of one weight row -> 16 tensor-memory columns
@@ -227,26 +247,29 @@ __device__ __forceinline__ Row row_of(const StreamArgs &a, const Segment &g, int
   return w;
 }
 
-// Half of the CTA's threads: waits until all parts of the segment's tile are in the workspace, then
-// adds and stores this CTA's share of its tokens.  `sub` (0, 1) and r (row) identify the thread.
-// With `dry` nothing is read, awaited or stored.
+template <bool BF16>
+__device__ __forceinline__ void store_row(void *y, long long i, float v) {
+  if (BF16) static_cast<__nv_bfloat16 *>(y)[i] = __float2bfloat16_rn(v);
+  else static_cast<__half *>(y)[i] = __float2half_rn(v);
+}
+
+// Half of the first 512 threads: waits until all parts of the segment's tile are in the workspace,
+// then adds and stores this CTA's share of its tokens.  `sub` (0, 1) and r (row) identify the thread.
+template <bool BF16>
 __device__ __forceinline__ void finish_shared(const StreamArgs &a, const StreamSched &sc, const Segment &g, int r, int sub,
-                                              int bar_id, bool dry, volatile int *abort_flag) {
+                                              int bar_id, volatile int *abort_flag) {
   const int b0 = first_cta(sc, blockIdx.x, g.start), b1 = last_cta(sc, blockIdx.x, g.start + sc.S[g.fmt]);
   const int parts = b1 - b0 + 1;
   const Row row = row_of(a, g, r, true);
   const int tok0 = g.m_tile * sc.nt;
   const int ntok = min(sc.nt, sc.M - tok0);
-  const int lo = ntok * (static_cast<int>(blockIdx.x) - b0) / parts;
-  const int hi = dry ? lo : ntok * (static_cast<int>(blockIdx.x) + 1 - b0) / parts;
-  if (r == 0 && sub == 0 && !dry && !wait_arrivals(a.arrived + b0, 4u * parts, parts)) *abort_flag = 1;
-  if (!dry) {
-    asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "n"(kThreads / 2) : "memory");
-    if (*abort_flag) return;
-  }
+  const int lo = ntok * (static_cast<int>(blockIdx.x) - b0) / parts, hi = ntok * (static_cast<int>(blockIdx.x) + 1 - b0) / parts;
+  if (r == 0 && sub == 0 && !wait_arrivals(a.arrived + b0, 4u * parts, parts)) *abort_flag = 1;
+  asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "n"(kFinishThreads / 2) : "memory");
+  if (*abort_flag) return;
   constexpr int kTok = 8, kSub = 2;
 #pragma unroll 1
-  for (int t0 = lo + sub; t0 < hi || (dry && t0 == lo + sub); t0 += kTok * kSub) {
+  for (int t0 = lo + sub; t0 < hi; t0 += kTok * kSub) {
     float v[kTok];
 #pragma unroll
     for (int e = 0; e < kTok; ++e) v[e] = 0.f;
@@ -268,26 +291,24 @@ __device__ __forceinline__ void finish_shared(const StreamArgs &a, const StreamS
 #pragma unroll
       for (int e = 0; e < kTok; ++e)
         if (t0 + e * kSub < hi)
-          store_y(a.y, 1ll * (tok0 + t0 + e * kSub) * a.N + row.col, fmaf(v[e], row.scl, row.bia), a.y_bf16);
+          store_row<BF16>(a.y, 1ll * (tok0 + t0 + e * kSub) * a.N + row.col, fmaf(v[e], row.scl, row.bia));
     }
   }
 }
 
-// COLS: tensor-memory columns of the CTA.  512: two accumulators of 128 columns and four weight
-// stages of 64; 256: two of 32 and three, for two CTAs per SM.
-template <int COLS>
-__global__ void __launch_bounds__(kThreads, COLS == 256 ? 2 : 1)
+// NT: most tokens per tile (64 or 128)
+template <int NT, bool BF16>
+__global__ void __launch_bounds__(kThreads<NT>, 1)
 gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_constant__ CUtensorMap w8map,
                    const __grid_constant__ CUtensorMap w16map, const __grid_constant__ CUtensorMap xmap,
                    const __grid_constant__ StreamArgs a, const __grid_constant__ StreamSched sc, int *status) {
-  constexpr int NS = COLS == 256 ? 3 : 4;       // stages
-  constexpr int kAcc = COLS == 256 ? 32 : 128;  // columns of an accumulator
+  constexpr int NS = kStages<NT>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ StreamSmem S;
   const uint32_t w_ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t x_ring = w_ring + a.nw * kChunkBytes;
   const uint32_t x_bytes = static_cast<uint32_t>(sc.nt) * 128;  // one 64-k box
-  const uint32_t s_ring = x_ring + NS * 2 * x_bytes;
+  const uint32_t s_ring = x_ring + NS * 4 * x_bytes;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int begin = sc.bnd[blockIdx.x], end = sc.bnd[blockIdx.x + 1];
   auto load_chunk = [&](const Segment &g, int c, int slot) {
@@ -297,14 +318,14 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
                 c * (g.fmt == 2 ? 64 : 128), g.row_tile * 128, bar);
   };
   // Without leave to read weights early every thread waits for the kernel before this one here; the
-  // launch itself and the instruction fetch still overlap it.
+  // launch itself still overlaps it.
   if (!a.early) pdl_wait();
   // The first weight chunks are on their way before anything else is set up.
   const int early = min(a.nw, end - begin);
   if (threadIdx.x == 0) {
     for (int i = 0; i < a.nw; ++i) {
       mbar_init(smem_u32(&S.w_full[i]), 1 + 32);  // the TMA thread and the scale warp's lanes
-      mbar_init(smem_u32(&S.w_empty[i]), 4);  // the group that converts the chunk
+      mbar_init(smem_u32(&S.w_empty[i]), 4);      // the group that converts the chunk
     }
     mbar_init_fence();
     Segment g = segment_at(sc, begin, end);
@@ -313,17 +334,9 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
       load_chunk(g, begin + i - g.start, i);
     }
   }
-  // Kernel parameters are read through the constant cache, whose misses would otherwise follow one
-  // another in every role: each warp touches another part of them first.
-  {
-    constexpr int kWords = (sizeof(StreamSched) - kMaxCtas * 4) / 4;
-    const int w0 = reinterpret_cast<const int *>(&sc)[min(warp * 16, kWords)];
-    const int w1 = reinterpret_cast<const int *>(&a)[min(warp * 16, static_cast<int>(sizeof(StreamArgs) / 4) - 1)];
-    asm volatile("" ::"r"(w0), "r"(w1));
-  }
   if (threadIdx.x == 32) {
     for (int i = 0; i < NS; ++i) {
-      mbar_init(smem_u32(&S.full[i]), 1 + 4);  // the activation loads and four converter warps
+      mbar_init(smem_u32(&S.full[i]), 1 + 4);  // the activation loads and the group's warps
       mbar_init(smem_u32(&S.empty[i]), 1);
     }
     for (int i = 0; i < 2; ++i) {
@@ -334,129 +347,121 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
     S.abort_flag = 0;
     mbar_init_fence();
   }
-  if (warp == 2) tmem_alloc(smem_u32(&S.tmem_base), COLS);
-  if (warp == 3 && lane < 4) prefetch_tensormap(lane == 0 ? &w4map : (lane == 1 ? &w8map : (lane == 2 ? &w16map : &xmap)));
+  if (warp == 2) tmem_alloc(smem_u32(&S.tmem_base), 512);
+  if (warp == 3 && lane == 0) prefetch_tensormap(&xmap);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = S.tmem_base;
-  const uint32_t tmem_a = tmem + 2 * kAcc;
+  const uint32_t tmem_a = tmem + 2 * NT;
   pdl_launch_dependents();
 
-  // Code that runs once per launch runs out of a cold instruction cache (about 45 ns per instruction
-  // measured): the epilogue warps, which have nothing to do at first, go through the code that ends
-  // the kernel once without effect while the others stream.
-  bool dry = warp >= 4 && warp < 8;
-#pragma unroll 1
-  for (int pass = dry ? 0 : 1; pass < 2; ++pass, dry = false) {
-  if (dry) {
-  } else if (warp == 0) {
+  if (warp == 0) {
     // ---------------------------------------------------------------- weight chunks
     const bool leader = elect_one();
     Cursor w;
     if (early == a.nw) w.ph ^= 1;
     else w.i = early;
-    bool alive = true;
-    for (int ck = begin + early; ck < end && alive;) {
-      const Segment g = segment_at(sc, ck, end);
-      for (int c = g.c0; c < g.c1; ++c) {
-        alive = gemm_wait(&S.w_empty[w.i], w.ph ^ 1, &S.abort_flag);
-        if (!alive) break;
-        if (leader) load_chunk(g, c, w.i);
-        w.next(a.nw);
-      }
-      ck = g.start + g.c1;
+    Segment g = segment_at(sc, begin, end);
+    for (int i = begin + early; i < end; ++i) {
+      if (i >= g.start + g.c1) g = segment_at(sc, i, end);
+      if (!gemm_wait(&S.w_empty[w.i], w.ph ^ 1, &S.abort_flag)) break;
+      if (leader) load_chunk(g, i - g.start, w.i);
+      w.next(a.nw);
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- activation boxes
     const bool leader = elect_one();
     pdl_wait();
     Cursor x;
-    bool alive = true;
-    for (int ck = begin; ck < end && alive;) {
-      const Segment g = segment_at(sc, ck, end);
+    Segment g = segment_at(sc, begin, end);
+    for (int i = begin; i < end; ++i) {
+      if (i >= g.start + g.c1) g = segment_at(sc, i, end);
       const int per = 4 >> g.fmt;  // k blocks of 64 per chunk
-      const int kb1 = min(g.c1 * per, sc.nkb), step = min(per, 2);
-      for (int kb = g.c0 * per; kb < kb1; kb += step) {
-        alive = gemm_wait(&S.empty[x.i], x.ph ^ 1, &S.abort_flag);
-        if (!alive) break;
-        if (leader) {
-          const uint32_t bar = smem_u32(&S.full[x.i]);
-          const uint32_t dst = x_ring + x.i * 2 * x_bytes;
-          const bool two = step == 2 && kb + 1 < kb1;
-          mbar_arrive_expect_tx(bar, two ? 2 * x_bytes : x_bytes);
-          tma_load_2d(dst, &xmap, kb * 64, g.m_tile * sc.nt, bar);
-          if (two) tma_load_2d(dst + x_bytes, &xmap, (kb + 1) * 64, g.m_tile * sc.nt, bar);
-        }
-        x.next(NS);
+      const int kb0 = (i - g.start) * per, nb = min(per, sc.nkb - kb0);
+      if (!gemm_wait(&S.empty[x.i], x.ph ^ 1, &S.abort_flag)) break;
+      if (leader) {
+        const uint32_t bar = smem_u32(&S.full[x.i]);
+        const uint32_t dst = x_ring + x.i * 4 * x_bytes;
+        mbar_arrive_expect_tx(bar, nb * x_bytes);
+        for (int b = 0; b < nb; ++b) tma_load_2d(dst + b * x_bytes, &xmap, (kb0 + b) * 64, g.m_tile * sc.nt, bar);
       }
-      ck = g.start + g.c1;
+      x.next(NS);
     }
   } else if (warp == 2) {
     // ---------------------------------------------------------------- MMA issue
+    // The inner loop is kept to a wait in one asm block, the MMAs and a commit: with anything that can
+    // diverge in it, every MMA's operands are moved to uniform registers again and an MMA takes 60
+    // cycles to issue instead of 20.
     const bool leader = elect_one();
     const uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(sc.nt >> 3) << 17) | (8u << 24);
-    Cursor x, d;
-    bool alive = true;
-    for (int ck = begin; ck < end && alive;) {
+    const uint64_t desc0 = make_desc_sw128(x_ring);
+    const uint32_t dx0 = static_cast<uint32_t>(desc0), dx_hi = static_cast<uint32_t>(desc0 >> 32), box = x_bytes >> 4;
+    const uint32_t full0 = smem_u32(&S.full[0]), empty0 = smem_u32(&S.empty[0]);
+    uint32_t stage = 0, ph = 0;
+    Cursor d;
+    uint32_t ok = 1;
+    for (int ck = begin; ck < end && ok;) {
       const Segment g = segment_at(sc, ck, end);
       const int per = 4 >> g.fmt;
-      const int kb0 = g.c0 * per, kb1 = min(g.c1 * per, sc.nkb), step = min(per, 2);
-      alive = gemm_wait(&S.d_empty[d.i], d.ph ^ 1, &S.abort_flag);
-      if (!alive) break;
+      if (!gemm_wait(&S.d_empty[d.i], d.ph ^ 1, &S.abort_flag)) break;
       tc_fence_after();
-      const uint32_t acc = tmem + d.i * kAcc;
-      for (int kb = kb0; kb < kb1; kb += step) {
-        alive = gemm_wait(&S.full[x.i], x.ph, &S.abort_flag);
-        if (!alive) break;
-        tc_fence_after();
-        const uint64_t dx = make_desc_sw128(x_ring + x.i * 2 * x_bytes);
-        const uint32_t wa = tmem_a + x.i * 64;
-        if (leader) {
-#pragma unroll
-          for (int k4 = 0; k4 < 4; ++k4) umma_f16_ts(acc, wa + 8 * k4, dx + 2 * k4, idesc, (kb != kb0 || k4 != 0) ? 1u : 0u);
-          if (step == 2 && kb + 1 < kb1) {
-            const uint64_t dx2 = dx + (x_bytes >> 4);
-#pragma unroll
-            for (int k4 = 0; k4 < 4; ++k4) umma_f16_ts(acc, wa + 32 + 8 * k4, dx2 + 2 * k4, idesc, 1u);
+      const uint32_t acc = tmem + d.i * NT;
+      const int whole = min(g.c1, sc.nkb / per) - g.c0;  // chunks with all their k blocks
+      const int rest = whole < g.c1 - g.c0 ? sc.nkb - (g.c1 - 1) * per : 0;
+      uint32_t accumulate = 0;
+      auto run = [&](auto blocks, int count) {
+#pragma unroll 1
+        for (int i = 0; i < count; ++i) {
+          ok = wait_bounded(full0 + stage * 8, ph);
+          if (!ok) break;
+          tc_fence_after();
+          if (leader) {
+            issue_blocks<decltype(blocks)::value>(acc, tmem_a + stage * 128, dx0 + stage * 4 * box, dx_hi, box, idesc, accumulate);
+            umma_commit(empty0 + stage * 8);
           }
-          umma_commit(smem_u32(&S.empty[x.i]));
+          accumulate = 1;
+          stage = stage + 1 == NS ? 0 : stage + 1;
+          ph ^= stage == 0;
         }
-        x.next(NS);
-      }
-      if (alive && leader) umma_commit(smem_u32(&S.d_full[d.i]));
+      };
+      if (per == 4) run(std::integral_constant<int, 4>(), whole);
+      else if (per == 2) run(std::integral_constant<int, 2>(), whole);
+      else run(std::integral_constant<int, 1>(), whole);
+      if (rest == 3) run(std::integral_constant<int, 3>(), 1);
+      else if (rest == 2) run(std::integral_constant<int, 2>(), 1);
+      else if (rest == 1) run(std::integral_constant<int, 1>(), 1);
+      if (ok && leader) umma_commit(smem_u32(&S.d_full[d.i]));
       d.next(2);
       ck = g.start + g.c1;
     }
+    if (!ok) S.abort_flag = 1;
     __syncwarp();
   } else if (warp == 3) {
     // ------------------------------------------------------------------ block scales
     Cursor w;
-    bool alive = true;
     const int pitch = a.K >> 4;
-    for (int ck = begin; ck < end && alive;) {
-      const Segment g = segment_at(sc, ck, end);
-      for (int c = g.c0; c < g.c1; ++c) {
-        alive = gemm_wait(&S.w_empty[w.i], w.ph ^ 1, &S.abort_flag);
-        if (!alive) break;
-        if (g.fmt == 0) {
-          const uint32_t dst = s_ring + w.i * kScaleBytes;
-          const int words = min(4, sc.nkb - 4 * c);
+    Segment g = segment_at(sc, begin, end);
+    for (int i = begin; i < end; ++i) {
+      if (i >= g.start + g.c1) g = segment_at(sc, i, end);
+      if (!gemm_wait(&S.w_empty[w.i], w.ph ^ 1, &S.abort_flag)) break;
+      if (g.fmt == 0) {
+        const int c = i - g.start;
+        const uint32_t dst = s_ring + w.i * kScaleBytes;
+        const int words = min(4, sc.nkb - 4 * c);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int r = i * 32 + lane;
-            const uint8_t *src = a.s4 + 1ll * min(g.row_tile * 128 + r, a.n4 - 1) * pitch + c * 16;
-            if (a.scale16) {
-              cp_async16(dst + r * 16, src);
-            } else {
-              for (int j = 0; j < words; ++j) cp_async4(dst + r * 16 + 4 * j, src + 4 * j);
-            }
+        for (int u = 0; u < 4; ++u) {
+          const int r = u * 32 + lane;
+          const uint8_t *src = a.s4 + 1ll * min(g.row_tile * 128 + r, a.n4 - 1) * pitch + c * 16;
+          if (a.scale16) {
+            cp_async16(dst + r * 16, src);
+          } else {
+            for (int j = 0; j < words; ++j) cp_async4(dst + r * 16 + 4 * j, src + 4 * j);
           }
         }
-        cp_async_arrive(smem_u32(&S.w_full[w.i]));
-        w.next(a.nw);
       }
-      ck = g.start + g.c1;
+      cp_async_arrive(smem_u32(&S.w_full[w.i]));
+      w.next(a.nw);
     }
   } else if (warp < 8) {
     // ------------------------------------------------------------------ epilogue
@@ -472,27 +477,47 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
       const int ntok = min(sc.nt, sc.M - tok0);
       if (!gemm_wait(&S.d_full[d.i], d.ph, &S.abort_flag)) break;
       tc_fence_after();
-      const uint32_t acc = tmem + d.i * kAcc + lanes;
+      const uint32_t acc = tmem + d.i * NT + lanes;
       float *part = a.partial + (2ll * blockIdx.x + (first ? 0 : 1)) * sc.nt * 128 + q * 32 + lane;
-      for (int c = 0; c < ntok; c += 16) {
-        uint32_t v[16];
-        tmem_ld16(acc + c, v);
+      uint16_t *yp = static_cast<uint16_t *>(a.y) + 1ll * tok0 * a.N + row.col;
+      // sixteen tokens at a time; the stores of one batch overlap the load of the next
+      uint32_t v[2][16];
+      tmem_ld16(acc, v[0]);
+      auto batch = [&](uint32_t (&cur)[16], uint32_t (&nxt)[16], int c) {
         tmem_wait_ld();
-        if (c + 16 >= ntok) {  // the accumulator is free once its last columns are read
+        if (c + 16 < ntok) {
+          tmem_ld16(acc + c + 16, nxt);
+        } else {  // the accumulator is free once its last columns are read
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(&S.d_empty[d.i]));
         }
+        const int n = min(16, ntok - c);
         if (!whole) {
+          if (n == 16) {
 #pragma unroll
-          for (int e = 0; e < 16; ++e)
-            if (c + e < ntok) part[(c + e) * 128] = __uint_as_float(v[e]);
+            for (int e = 0; e < 16; ++e) part[(c + e) * 128] = __uint_as_float(cur[e]);
+          } else {
+#pragma unroll
+            for (int e = 0; e < 16; ++e)
+              if (e < n) part[(c + e) * 128] = __uint_as_float(cur[e]);
+          }
         } else if (row.live) {
+          uint16_t *p = yp;
 #pragma unroll
-          for (int e = 0; e < 16; ++e)
-            if (c + e < ntok)
-              store_y(a.y, 1ll * (tok0 + c + e) * a.N + row.col, fmaf(__uint_as_float(v[e]), row.scl, row.bia), a.y_bf16);
+          for (int e = 0; e < 16; e += 2) {
+            const uint32_t h = pack_y2(fmaf(__uint_as_float(cur[e]), row.scl, row.bia),
+                                       fmaf(__uint_as_float(cur[e + 1]), row.scl, row.bia), BF16);
+            if (e < n) p[0] = static_cast<uint16_t>(h);
+            if (e + 1 < n) p[a.N] = static_cast<uint16_t>(h >> 16);
+            p += 2 * a.N;
+          }
+          yp += 16ll * a.N;
         }
+      };
+      for (int c = 0; c < ntok; c += 32) {
+        batch(v[0], v[1], c);
+        if (c + 16 < ntok) batch(v[1], v[0], c + 16);
       }
       if (!whole) {
         __threadfence();
@@ -505,87 +530,76 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
     }
   } else {
     // ------------------------------------------------------------------ converters
+    // Group `grp` owns stage `grp` and takes every NS-th chunk.  It waits for the release of its stage
+    // first: the MMAs have then consumed every chunk up to NS before this one, so the parity it tests
+    // on the chunk's barrier (used by chunk i - nw before, nw >= NS) cannot be a round old.
     const int q = warp & 3, grp = (warp - 8) >> 2;
     const int row = q * 32 + lane;
-    const uint32_t lanes = static_cast<uint32_t>(q * 32) << 16;
     const uint32_t rbase = row * 128, sw = row & 7;
-    auto piece = [&](uint32_t base, int p) { return base + rbase + ((p ^ sw) << 4); };
-    Cursor w, s;
-    // A group takes every second chunk: its own stage before was at most three stages back, so when it
-    // waits for the release of stage i - NS it has seen that of stage i - 3 - NS, and with NS >= 3 the
-    // parity it tests cannot be two rounds old.  Likewise for the chunk barriers: what it converted
-    // last lies behind every chunk whose slot it could confuse, as long as nw >= 3.
-    static_assert(kGroups == 2 && NS >= 3, "a stage barrier could be tested two rounds late");
-    int turn = 0;
-    bool alive = true;
-    for (int ck = begin; ck < end && alive;) {
-      const Segment g = segment_at(sc, ck, end);
-      const int per = 4 >> g.fmt;
-      for (int c = g.c0; c < g.c1; ++c, turn ^= 1, w.next(a.nw)) {
-        const int nb = min(per, sc.nkb - c * per);
-        if (turn != grp) {
-          for (int b = 0; b < nb; b += 2) s.next(NS);
-          continue;
+    const uint32_t dst = tmem_a + grp * 128 + (static_cast<uint32_t>(q * 32) << 16);
+    int slot = grp;
+    uint32_t w_ph = 0, ph = 0;
+    Segment g;
+    g.start = g.c1 = 0;
+    for (int i = begin + grp; i < end; i += NS) {
+      if (i == begin + grp || i >= g.start + g.c1) g = segment_at(sc, i, end);
+      if (!gemm_wait(&S.empty[grp], ph ^ 1, &S.abort_flag)) break;
+      if (!gemm_wait(&S.w_full[slot], w_ph, &S.abort_flag)) break;
+      tc_fence_after();
+      const uint32_t base = w_ring + slot * kChunkBytes + rbase;
+      auto piece = [&](int p) { return lds16(base + ((p ^ sw) << 4)); };
+      uint32_t o[16];
+      if (g.fmt == 0) {
+        // (k blocks beyond K convert the zero fill of the box; the MMAs do not read them)
+        const uint4 s4 = lds16(s_ring + slot * kScaleBytes + row * 16);
+        const uint32_t sc4[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+        for (int h = 0; h < 8; ++h) {
+          convert_fp4(piece(h), sc4[h >> 1] >> (16 * (h & 1)), o);
+          tmem_st16(dst + 16 * h, o);
         }
-        alive = gemm_wait(&S.w_full[w.i], w.ph, &S.abort_flag);
-        if (!alive) break;
-        const uint32_t base = w_ring + w.i * kChunkBytes;
-        for (int b = 0; b < nb; b += 2) {
-          alive = gemm_wait(&S.empty[s.i], s.ph ^ 1, &S.abort_flag);
-          if (!alive) break;
-          tc_fence_after();
-          const uint32_t dst = tmem_a + s.i * 64 + lanes;
-          uint32_t o[16];
-          if (g.fmt == 0) {
-            // (a trailing odd block converts the zero fill of the box; the MMAs do not read it)
-            uint32_t s0, s1;
-            asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(s0), "=r"(s1) : "r"(s_ring + w.i * kScaleBytes + row * 16 + b * 4) : "memory");
+      } else if (g.fmt == 1) {
 #pragma unroll
-            for (int h = 0; h < 4; ++h) {
-              convert_fp4(lds16(piece(base, 2 * b + h)), (h < 2 ? s0 : s1) >> (16 * (h & 1)), o);
-              tmem_st16(dst + 16 * h, o);
-            }
-          } else if (g.fmt == 1) {
+        for (int h = 0; h < 4; ++h) {
+          convert_fp8(piece(2 * h), piece(2 * h + 1), o);
+          tmem_st16(dst + 16 * h, o);
+        }
+      } else {
 #pragma unroll
-            for (int h = 0; h < 4; ++h) {
-              convert_fp8(lds16(piece(base, 2 * h)), lds16(piece(base, 2 * h + 1)), o);
-              tmem_st16(dst + 16 * h, o);
-            }
-          } else {
+        for (int h = 0; h < 2; ++h) {
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-#pragma unroll
-              for (int p = 0; p < 4; ++p) {
-                const uint4 v = lds16(piece(base, 4 * h + p));
-                o[4 * p] = v.x;
-                o[4 * p + 1] = v.y;
-                o[4 * p + 2] = v.z;
-                o[4 * p + 3] = v.w;
-              }
-              tmem_st16(dst + 16 * h, o);
-            }
+          for (int p = 0; p < 4; ++p) {
+            const uint4 v = piece(4 * h + p);
+            o[4 * p] = v.x;
+            o[4 * p + 1] = v.y;
+            o[4 * p + 2] = v.z;
+            o[4 * p + 3] = v.w;
           }
-          tmem_wait_st();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&S.full[s.i]));
-          s.next(NS);
+          tmem_st16(dst + 16 * h, o);
         }
-        if (!alive) break;
-        if (lane == 0) mbar_arrive(smem_u32(&S.w_empty[w.i]));
       }
-      ck = g.start + g.c1;
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(smem_u32(&S.full[grp]));
+        mbar_arrive(smem_u32(&S.w_empty[slot]));
+      }
+      ph ^= 1;
+      slot += NS;
+      if (slot >= a.nw) {
+        slot -= a.nw;
+        w_ph ^= 1;
+      }
     }
   }
 
   __syncwarp();
-  if (!dry) {
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 2) tmem_dealloc(tmem, COLS);
-  }
-  // ---- tiles shared with other CTAs: half of the threads take the range's first segment, half its last
-  if ((dry || !S.abort_flag) && begin < end) {
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 2) tmem_dealloc(tmem, 512);
+  // ---- tiles shared with other CTAs: half of 512 threads take the range's first segment, half its last
+  if (!S.abort_flag && begin < end && threadIdx.x < kFinishThreads) {
     const int half = threadIdx.x >> 8;
     Segment g = segment_at(sc, begin, end);
     bool mine = half == 0;
@@ -594,10 +608,9 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
       g = segment_at(sc, end - 1, end);
       g = segment_at(sc, max(g.start, begin), end);
     }
-    if (dry || (mine && !(g.c0 == 0 && g.c1 == sc.S[g.fmt])))
-      finish_shared(a, sc, g, threadIdx.x & 127, (threadIdx.x >> 7) & 1, 1 + half, dry, &S.abort_flag);
+    if (mine && !(g.c0 == 0 && g.c1 == sc.S[g.fmt]))
+      finish_shared<BF16>(a, sc, g, threadIdx.x & 127, (threadIdx.x >> 7) & 1, 1 + half, &S.abort_flag);
   }
-  }  // pass
   __syncthreads();
   if (S.abort_flag) {
     linger(16000);  // let copies that are still in flight land before the shared memory is given up
@@ -611,7 +624,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
 
 struct StreamPlan {
   StreamSched sc;
-  int cols, nw, smem;
+  int wide, nw, smem;  // wide: the variant for more than 64 tokens per tile
 };
 
 // Token tiles of equal width; a chunk costs what bounds it: its bytes at the SM's share of the HBM
@@ -646,9 +659,9 @@ StreamPlan make_plan(int n4, int n8, int n16, int M, int K) {
                                            : (pos < W[1] ? s.E[0] + (pos - W[0]) / u[1] : s.E[1] + (pos - W[1]) / u[2]));
   }
   s.bnd[s.G] = e;
-  p.cols = s.nt <= 32 ? 256 : 512;
-  const int xb = (p.cols == 256 ? 3 : 4) * 2 * s.nt * 128;
-  p.nw = std::min(8, ((p.cols == 256 ? 108 : 220) * 1024 - 1024 - xb) / (kChunkBytes + kScaleBytes));
+  p.wide = s.nt > 64;
+  const int xb = (p.wide ? kStages<128> : kStages<64>) * 4 * s.nt * 128;
+  p.nw = std::min(kMaxRing, (kSmemMax - 1024 - xb) / (kChunkBytes + kScaleBytes));
   p.smem = 1024 + xb + p.nw * (kChunkBytes + kScaleBytes);
   return p;
 }
@@ -712,7 +725,6 @@ int launch_gemm_stream(const GemmArgs &g, void *workspace, size_t workspace_byte
   a.perm = g.perm;
   a.bias = g.bias;
   a.y = g.y;
-  a.y_bf16 = g.y_bf16;
   a.n4 = g.n4;
   a.n8 = g.n8;
   a.n16 = g.n16;
@@ -726,23 +738,25 @@ int launch_gemm_stream(const GemmArgs &g, void *workspace, size_t workspace_byte
   a.test_timeout = gemm_test_timeout();
   const StreamSched &sc = p.sc;
 
-  const void *fn = p.cols == 256 ? reinterpret_cast<const void *>(gemm_stream_kernel<256>)
-                                 : reinterpret_cast<const void *>(gemm_stream_kernel<512>);
-  static std::atomic<int> smem_set[2][64];
+  static const void *const fns[4] = {
+      reinterpret_cast<const void *>(gemm_stream_kernel<64, false>), reinterpret_cast<const void *>(gemm_stream_kernel<64, true>),
+      reinterpret_cast<const void *>(gemm_stream_kernel<128, false>), reinterpret_cast<const void *>(gemm_stream_kernel<128, true>)};
+  const int variant = p.wide * 2 + (g.y_bf16 ? 1 : 0);
+  const void *fn = fns[variant];
+  static std::atomic<bool> attr_done[4][64];
   int dev = 0;
   RDQ_CUDA(cudaGetDevice(&dev));
-  std::atomic<int> *set = dev >= 0 && dev < 64 ? &smem_set[p.cols == 256][dev] : nullptr;
-  if (!set || set->load() < p.smem) {
-    RDQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, p.cols == 256 ? 110 * 1024 : 222 * 1024));
-    RDQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-    if (set) set->store(1 << 30);
+  std::atomic<bool> *done = dev >= 0 && dev < 64 ? &attr_done[variant][dev] : nullptr;
+  if (!done || !done->load()) {
+    RDQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
+    if (done) done->store(true);
   }
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(sc.G));
-  cfg.blockDim = dim3(kThreads);
+  cfg.blockDim = dim3(p.wide ? kThreads<128> : kThreads<64>);
   cfg.dynamicSmemBytes = p.smem;
   cfg.stream = stream;
   cfg.attrs = attr;

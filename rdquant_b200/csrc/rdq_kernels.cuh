@@ -122,6 +122,7 @@ int launch_gemm_stream(const GemmArgs &a, void *workspace, size_t workspace_byte
 // GEMM over weights decoded once per call (rdq_gemm_dense.cu)
 bool gemm_dense_takes(int K);
 size_t gemm_dense_workspace(int M, int N, int K);
+double gemm_dense_cycles(int M, int N, int K);  // estimate of the product alone
 int launch_gemm_dense(const GemmArgs &a, void *workspace, size_t workspace_bytes, cudaStream_t stream);
 
 // staging copy by kernel (rdq_stage.cu)

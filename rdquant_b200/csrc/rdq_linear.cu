@@ -40,13 +40,35 @@ bool has_row_major(const rdq_layer &l) {
   return (l.n_fp4 == 0 || l.w_fp4) && (l.n_fp8 == 0 || l.w_fp8) && (l.n_fp16 == 0 || l.w_fp16);
 }
 
-// Up to 16 rows: the decode GEMV (tiled layout, else the any-shape kernel).  More rows: the
-// tensor-core GEMM, which reads the row-major tensors by TMA (K a multiple of 16); what it cannot
-// take runs as 16-row panels of the decode kernel.
+// Fewest rows for which the streaming GEMM beats the decode GEMV.  Measured times are about
+// a + bytes / rate with a = 4.5 us and 4.2 (1, 2 rows) or 2.9 TB/s (up to 8) for the GEMV, whose
+// converter work and activation reads grow with the rows, against 9.5 us and 5.8 TB/s whatever the
+// rows: equal at 75 and 29 MB of packed weights (40 measured); above 8 rows the GEMV halves its rate.
+int stream_from(const rdq_layer &l) {
+  if (!l.w_tiled) return 1;
+  const double bytes = l.n_fp4 * (l.K * 0.5625) + l.n_fp8 * (l.K + 4.0) + l.n_fp16 * (l.K * 2.0);
+  return bytes > 80e6 ? 1 : (bytes > 40e6 ? 3 : 9);
+}
+
+// Few rows: the decode GEMV (tiled layout, else the any-shape kernel), or the streaming GEMM from
+// stream_from() on.  More: the streaming GEMM or the one over decoded weights, which read the
+// row-major tensors by TMA (K a multiple of 64 / 16); what they cannot take runs as 16-row panels of
+// the decode kernel.
+//
+// Above 256 rows the streaming GEMM converts the weights once more per 128 rows, the other GEMM decodes
+// them once: estimates in microseconds that agree with measurements between 256 and 1536 rows on five
+// layer shapes within 15 %.
+bool stream_beats_dense(const rdq_layer &l, int M) {
+  if (M <= 256) return true;
+  if (M > 2048) return false;
+  const int N = l.n_fp4 + l.n_fp8 + l.n_fp16;
+  const double weights = 1e-6 * N * l.K;
+  return 14.0 + 1.62e-3 * M * weights < 8.0 + 0.5 * weights + gemm_dense_cycles(M, N, l.K) / 1750.0;
+}
+
 Path path_of(const rdq_layer &l, int M) {
-  static const int lo = getenv("RDQ_STREAM_LO") ? atoi(getenv("RDQ_STREAM_LO")) : 17;
-  static const int hi = getenv("RDQ_STREAM_HI") ? atoi(getenv("RDQ_STREAM_HI")) : 256;
-  if (M >= lo && M <= hi && gemm_stream_takes(l.K) && has_row_major(l) && l.gemv_counters && (l.perm || !l.inv_perm)) return Path::kStream;
+  const bool can_stream = gemm_stream_takes(l.K) && has_row_major(l) && l.gemv_counters && (l.perm || !l.inv_perm);
+  if (can_stream && M >= stream_from(l) && (!gemm_dense_takes(l.K) || stream_beats_dense(l, M))) return Path::kStream;
   if (M <= RDQ_MAX_GEMV_M) return l.w_tiled ? Path::kGemvTiled : Path::kGemvGeneric;
   if (gemm_dense_takes(l.K) && has_row_major(l)) return Path::kGemm;
   return l.w_tiled ? Path::kPanelsTiled : Path::kPanelsGeneric;
