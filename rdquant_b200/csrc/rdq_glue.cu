@@ -239,81 +239,94 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const __half *gu, __half 
 
 // ---- q/k RMSNorm + rotary embedding + KV-cache write + attention of the new token over the
 // cache + merge of the splits, in one launch.
-// One CTA per SM, 128 threads: CTA c is (sequence, KV head) c / nsplit and split c % nsplit, with
-// nsplit = SMs / (sequences x KV heads) (at most 16); it serves the `group` query heads of its KV
-// head over the cache rows [split * chunk, (split + 1) * chunk) with chunk = the n = *pos + 1
-// rows divided by nsplit, rounded up to 32; warp w takes the heads w, w + 4, ...
-//   1. every CTA normalises and rotates its query heads into shared memory (FP16-rounded like the
-//      stored q of the separate kernel, times `scale`); the CTA whose rows include *pos does the
-//      same for the new key, copies the new value, and writes both to the cache and to its tile.
-//   2. K and V rows go to shared memory in tiles of TP rows by cp.async, two tiles in flight, so a
-//      CTA pays one memory round trip, not one per row.
-//   3. scores with one lane per row (K rows padded by 16 bytes against bank conflicts), online
-//      softmax per 32 rows, then P x V with one lane per DH / 32 dimensions.
-//   4. partial (max, sum, values) per split go to scratch; the last CTA of a (b, kvh) to arrive
-//      (counter in scratch, left at zero again) merges them and writes out [B, nq * dh].
-constexpr int kFusedAttnThreads = 256;
-constexpr int kFusedAttnWarps = kFusedAttnThreads / 32;
+// CTA c is (sequence, KV head) c / nsplit and split c % nsplit, with nsplit = SMs / (sequences x KV
+// heads) (at most 16, at least 1); it serves the `group` query heads of its KV head over the cache
+// rows [split * chunk, (split + 1) * chunk), chunk = the n = *pos + 1 rows divided by nsplit.
+//   1. the four warps normalise and rotate the query heads into shared memory (FP16-rounded, like the
+//      stored q of the separate kernel); the warp whose rows include *pos does the same for the new
+//      key, takes the new value, and writes both to the cache.
+//   2. every warp takes every fourth block of 16 rows through a ring of two blocks of its own
+//      (cp.async, rows outside the split zero-filled), so that warps do not wait for one another and
+//      a CTA keeps up to eight blocks (70 KB at head_dim 128) in flight.
+//   3. tensor-core products (mma.sync m16n8k16, FP32 sums) with cache rows as the row operand and up to
+//      eight query heads as columns: S^T = K Q^T, online softmax per block, O^T += V^T P^T.  P goes in
+//      as the sum of two FP16 values, so that its rounding (2^-22) stays below FP32 products' sums.
+//   4. the warps' (max, sum, values) are merged in shared memory; with one split that is the result,
+//      else the partial goes to scratch and the last CTA of a (sequence, KV head) to arrive (counter
+//      in scratch, left at zero again) merges the splits and writes out [B, nq * dh].
+// Bound: HBM (K and V rows once) for many sequences, latency for one.  The scalar kernel before (a
+// lane per row, every query head converting the K rows again) took 44 us for 32 sequences of 700 rows
+// (92 MB).
+constexpr int kFusedAttnWarps = 4;
+constexpr int kFusedAttnThreads = kFusedAttnWarps * 32;
 constexpr int kFusedAttnMaxSplit = 16;  // one batch of merge loads at head_dim <= 128
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+// 16 bytes, or zeros
+__device__ __forceinline__ void cp_async16_if(uint32_t dst, const void *src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t &r0, uint32_t &r1, uint32_t &r2, uint32_t &r3) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
+               : "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t v) {
+  uint32_t r;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+  return r;
+}
 
-template <int DH>
+// NB: blocks of eight query heads per KV head
+template <int DH, int NB>
 __global__ void __launch_bounds__(kFusedAttnThreads, 2) rope_attn_kernel(
     const __half *qkv, const __half *qn, const __half *kn, const __half *cos_t, const __half *sin_t, const long long *pos,
     __half *k_cache, __half *v_cache, float *part, int *counters, __half *out, int nq, int nkv, int S, float scale,
     float eps, int nsplit, int npair) {
-  constexpr int TP = 8192 / DH;        // rows per tile: 16 KB of V, a little more of K
-  constexpr int KP = 2 * DH + 16;      // K row pitch in shared memory (bytes)
-  constexpr int VP = 2 * DH;
-  constexpr int HALF = DH / 2;
-  constexpr int DPL = DH / 32;         // dimensions per lane in P x V
-  constexpr int VPR = DH / 8;          // 16-byte vectors per row
-  extern __shared__ __align__(16) uint8_t smem[];
-  uint8_t *ks = smem;                           // [2][TP][KP]
-  uint8_t *vs = smem + 2 * TP * KP;             // [2][TP][VP]
-  float *qs = reinterpret_cast<float *>(vs + 2 * TP * VP);  // [group][DH]
   constexpr int W = kFusedAttnWarps;
+  constexpr int PITCH = 2 * DH + 16;   // row pitch in shared memory (bytes): an odd multiple of 16
+  constexpr int BLK = 16 * PITCH;      // 16 rows of K or of V
+  constexpr int QP = DH + 8;           // query row pitch (halves)
+  constexpr int HALF = DH / 2;
+  constexpr int DPL = DH / 32;         // dimensions per lane in the merge
+  constexpr int VPR = DH / 8;          // 16-byte vectors per row
+  constexpr int KS = DH / 16;          // k steps of S, row blocks of O
   constexpr int PR = DH + 4;  // a partial: max, sum, two unused, then the DH weighted values (16-byte aligned)
+  extern __shared__ __align__(16) uint8_t smem[];
+  __half *qs = reinterpret_cast<__half *>(smem + W * 4 * BLK);  // [8 NB][QP]
+  float *mrg = reinterpret_cast<float *>(smem);                 // [W][8 NB][PR], over the rings once they are done
   __shared__ int s_last;
 
   pdl_launch_dependents();
   pdl_wait();
-  // CTA -> (sequence, KV head, split).  The grid has one CTA per SM (or one per (sequence, KV
-  // head) when those outnumber the SMs); CTAs beyond the work linger (see below).
+  // The grid has one CTA per SM (or one per (sequence, KV head) when those outnumber the SMs); CTAs
+  // beyond the work linger.
   const int pair = static_cast<int>(blockIdx.x) / nsplit, split = static_cast<int>(blockIdx.x) - pair * nsplit;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int g = lane >> 2, t = lane & 3;
   if (pair >= npair) {
     linger(4000);
     return;
   }
   const int kvh = pair % nkv, b = pair / nkv;
   const int group = nq / nkv;
-  // Warp -> (query head, slice of the rows): hp heads are served at a time, by nsl warps each;
-  // the warps of a head take every nsl-th block of 32 rows and are merged in shared memory.
-  const int hp = min(group, W), nsl = max(1, W / hp);
-  const int slice = warp / hp, head0 = warp - slice * hp;
-  const bool active = slice < nsl;
-  float *mrg = qs + group * DH;  // [W][2][PR]: partials of the slices above 0
-  // Loads that do not depend on the position go first, so that they share a round trip with it:
-  // the raw values of this warp's first query head and the norm weights.
+  // Loads that do not depend on the position go first, so that they share a round trip with it: the
+  // raw values of this warp's first query head and the norm weights.
   const __half *row = qkv + 1ll * b * (nq + 2 * nkv) * DH;
   float qx0[HALF / 32], qx1[HALF / 32], qw0[HALF / 32], qw1[HALF / 32];
   auto load_row = [&](const __half *src, float (&x0)[HALF / 32], float (&x1)[HALF / 32]) {
 #pragma unroll
-    for (int t = 0; t < HALF / 32; ++t) {
-      x0[t] = __half2float(src[lane + 32 * t]);
-      x1[t] = __half2float(src[lane + 32 * t + HALF]);
+    for (int u = 0; u < HALF / 32; ++u) {
+      x0[u] = __half2float(src[lane + 32 * u]);
+      x1[u] = __half2float(src[lane + 32 * u + HALF]);
     }
   };
-  if (slice == 0) load_row(row + 1ll * (kvh * group + head0) * DH, qx0, qx1);
+  if (warp < group) load_row(row + 1ll * (kvh * group + warp) * DH, qx0, qx1);
   if (qn) load_row(qn, qw0, qw1);
   const long long p_new = *pos;
   const int n = static_cast<int>(p_new) + 1;
@@ -324,218 +337,243 @@ __global__ void __launch_bounds__(kFusedAttnThreads, 2) rope_attn_kernel(
     return;
   }
   const int p0 = split * chunk, p1 = min(n, p0 + chunk);
-  const int ntile = (p1 - p0 + TP - 1) / TP;
+  const int nblk = (p1 - p0 + 15) >> 4;
   const __half *kb = k_cache + (1ll * b * nkv + kvh) * S * DH;
   const __half *vb = v_cache + (1ll * b * nkv + kvh) * S * DH;
-  const bool owns_new = p_new >= p0 && p_new < p1;
+  const uint32_t ring = smem_u32(smem) + warp * 4 * BLK;  // [2 stages][K, V][16][PITCH]
 
-  auto load_tile = [&](int t) {
-    const int r0 = p0 + t * TP, rows = min(TP, p1 - r0), st = t & 1;
-    for (int i = tid; i < rows * VPR; i += kFusedAttnThreads) {
-      const int r = i / VPR, c = i - r * VPR;
-      if (r0 + r == p_new) continue;  // the new row is not in the cache yet: step 1 puts it here
-      cp_async16(smem_u32(ks + (st * TP + r) * KP + 16 * c), kb + 1ll * (r0 + r) * DH + 8 * c);
-      cp_async16(smem_u32(vs + (st * TP + r) * VP + 16 * c), vb + 1ll * (r0 + r) * DH + 8 * c);
+  auto load_block = [&](int i, int st) {
+    const int r0 = p0 + 16 * i;
+    const uint32_t dst = ring + st * 2 * BLK;
+#pragma unroll
+    for (int u = 0; u < 16 * VPR / 32; ++u) {
+      const int e = u * 32 + lane, r = e / VPR, c = e - r * VPR;
+      const bool valid = r0 + r < p1 && r0 + r != p_new;  // the new row is not in the cache yet
+      const long long off = valid ? 1ll * (r0 + r) * DH + 8 * c : 0;
+      cp_async16_if(dst + r * PITCH + 16 * c, kb + off, valid);
+      cp_async16_if(dst + BLK + r * PITCH + 16 * c, vb + off, valid);
     }
-    cp_async_commit();
   };
-  load_tile(0);
-  if (ntile > 1) load_tile(1);
+  if (warp < nblk) load_block(warp, 0);
+  cp_async_commit();
+  if (warp + W < nblk) load_block(warp + W, 1);
+  cp_async_commit();
 
   // ---- 1. query heads, new key and value
   const __half *cs = cos_t + p_new * DH, *sn = sin_t + p_new * DH;
   float c0[HALF / 32], s0[HALF / 32], c1[HALF / 32], s1[HALF / 32];
-#pragma unroll
-  for (int t = 0; t < HALF / 32; ++t) {
-    const int i = lane + 32 * t;
-    c0[t] = __half2float(cs[i]);
-    s0[t] = __half2float(sn[i]);
-    c1[t] = __half2float(cs[i + HALF]);
-    s1[t] = __half2float(sn[i + HALF]);
-  }
-  // RMSNorm over the head (when nw), rotary embedding; FP16-rounded results as floats
+  load_row(cs, c0, c1);
+  load_row(sn, s0, s1);
+  // RMSNorm over the head (when nw), rotary embedding
   auto norm_rope = [&](const float (&x0)[HALF / 32], const float (&x1)[HALF / 32], bool nw, const float (&w0)[HALF / 32],
-                       const float (&w1)[HALF / 32], float (&o0)[HALF / 32], float (&o1)[HALF / 32]) {
+                       const float (&w1)[HALF / 32], __half (&o0)[HALF / 32], __half (&o1)[HALF / 32]) {
     float ss = 0.f;
 #pragma unroll
-    for (int t = 0; t < HALF / 32; ++t) ss += x0[t] * x0[t] + x1[t] * x1[t];
+    for (int u = 0; u < HALF / 32; ++u) ss += x0[u] * x0[u] + x1[u] * x1[u];
     float rs = 1.f;
     if (nw) rs = rsqrtf(warp_sum(ss) / DH + eps);
 #pragma unroll
-    for (int t = 0; t < HALF / 32; ++t) {
-      float y0 = x0[t], y1 = x1[t];
+    for (int u = 0; u < HALF / 32; ++u) {
+      float y0 = x0[u], y1 = x1[u];
       if (nw) {
-        y0 = __half2float(__hmul(__float2half_rn(x0[t] * rs), __float2half_rn(w0[t])));
-        y1 = __half2float(__hmul(__float2half_rn(x1[t] * rs), __float2half_rn(w1[t])));
+        y0 = __half2float(__hmul(__float2half_rn(x0[u] * rs), __float2half_rn(w0[u])));
+        y1 = __half2float(__hmul(__float2half_rn(x1[u] * rs), __float2half_rn(w1[u])));
       }
-      o0[t] = __half2float(__float2half_rn(y0 * c0[t] - y1 * s0[t]));
-      o1[t] = __half2float(__float2half_rn(y1 * c1[t] + y0 * s1[t]));
+      o0[u] = __float2half_rn(y0 * c0[u] - y1 * s0[u]);
+      o1[u] = __float2half_rn(y1 * c1[u] + y0 * s1[u]);
     }
   };
-  for (int hq = head0; slice == 0 && hq < group; hq += hp) {
-    float o0[HALF / 32], o1[HALF / 32];
-    if (hq != head0) load_row(row + 1ll * (kvh * group + hq) * DH, qx0, qx1);
-    norm_rope(qx0, qx1, qn != nullptr, qw0, qw1, o0, o1);
+  for (int hq = warp; hq < 8 * NB; hq += W) {
+    __half o0[HALF / 32], o1[HALF / 32];
+    if (hq < group) {
+      if (hq != warp) load_row(row + 1ll * (kvh * group + hq) * DH, qx0, qx1);
+      norm_rope(qx0, qx1, qn != nullptr, qw0, qw1, o0, o1);
+    } else {
 #pragma unroll
-    for (int t = 0; t < HALF / 32; ++t) {
-      qs[hq * DH + lane + 32 * t] = o0[t] * scale;
-      qs[hq * DH + lane + 32 * t + HALF] = o1[t] * scale;
+      for (int u = 0; u < HALF / 32; ++u) o0[u] = o1[u] = __float2half_rn(0.f);
+    }
+#pragma unroll
+    for (int u = 0; u < HALF / 32; ++u) {
+      qs[hq * QP + lane + 32 * u] = o0[u];
+      qs[hq * QP + lane + 32 * u + HALF] = o1[u];
     }
   }
-  // The new row is the last row of the last tile of its CTA.  The last warp (key) and the one
-  // before it (value) keep it in registers, write it to the cache now and into the tile when that tile is current.
-  float knew0[HALF / 32], knew1[HALF / 32];
-  __half vnew[DPL];
-  if (owns_new && warp == W - 1) {
+  // the warp whose block holds the new row: key and value to the cache now, into the block when it is current
+  const int new_blk = p_new >= p0 && p_new < p1 ? static_cast<int>(p_new - p0) >> 4 : -1;
+  const bool owns_new = new_blk >= 0 && new_blk % W == warp;
+  __half knew0[HALF / 32], knew1[HALF / 32], vnew[DPL];
+  if (owns_new) {
     float kx0[HALF / 32], kx1[HALF / 32], kw0[HALF / 32], kw1[HALF / 32];
+    const __half *vsrc = row + 1ll * (nq + nkv + kvh) * DH;
     load_row(row + 1ll * (nq + kvh) * DH, kx0, kx1);
     if (kn) load_row(kn, kw0, kw1);
+#pragma unroll
+    for (int j = 0; j < DPL; ++j) vnew[j] = vsrc[lane + 32 * j];
     norm_rope(kx0, kx1, kn != nullptr, kw0, kw1, knew0, knew1);
     __half *kd = k_cache + ((1ll * b * nkv + kvh) * S + p_new) * DH;
-#pragma unroll
-    for (int t = 0; t < HALF / 32; ++t) {
-      kd[lane + 32 * t] = __float2half_rn(knew0[t]);
-      kd[lane + 32 * t + HALF] = __float2half_rn(knew1[t]);
-    }
-  }
-  if (owns_new && warp == W - 2) {
-    const __half *src = row + 1ll * (nq + nkv + kvh) * DH;
     __half *vd = v_cache + ((1ll * b * nkv + kvh) * S + p_new) * DH;
 #pragma unroll
-    for (int j = 0; j < DPL; ++j) {
-      vnew[j] = src[lane + 32 * j];
-      vd[lane + 32 * j] = vnew[j];
+    for (int u = 0; u < HALF / 32; ++u) {
+      kd[lane + 32 * u] = knew0[u];
+      kd[lane + 32 * u + HALF] = knew1[u];
     }
+#pragma unroll
+    for (int j = 0; j < DPL; ++j) vd[lane + 32 * j] = vnew[j];
   }
+  __syncthreads();  // qs complete
 
-  // ---- 2./3. tiles
-  float m_run[2], l_run[2], acc[2][DPL];  // up to 2 heads per warp (group <= 16)
+  // ---- 2./3. blocks of 16 rows
+  uint32_t qf[NB][KS][2];  // query fragments: head g of the block, dimensions 16 k + 2 t (+ 8)
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    m_run[h] = -INFINITY;
-    l_run[h] = 0.f;
+  for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
-    for (int j = 0; j < DPL; ++j) acc[h][j] = 0.f;
+    for (int k = 0; k < KS; ++k) {
+      const __half *src = qs + (nb * 8 + g) * QP + 16 * k + 2 * t;
+      qf[nb][k][0] = *reinterpret_cast<const uint32_t *>(src);
+      qf[nb][k][1] = *reinterpret_cast<const uint32_t *>(src + 8);
+    }
+  float m_run[NB][2], l_run[NB][2], acc[NB][KS][4];  // heads 2 t, 2 t + 1; acc: dimensions 16 k + g, + 8
+#pragma unroll
+  for (int nb = 0; nb < NB; ++nb) {
+    m_run[nb][0] = m_run[nb][1] = -INFINITY;
+    l_run[nb][0] = l_run[nb][1] = 0.f;
+#pragma unroll
+    for (int k = 0; k < KS; ++k)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[nb][k][j] = 0.f;
   }
-  for (int t = 0; t < ntile; ++t) {
-    if (t + 1 < ntile) cp_async_wait<1>(); else cp_async_wait<0>();
-    const int r0 = p0 + t * TP, rows = min(TP, p1 - r0), st = t & 1;
-    if (owns_new && t == ntile - 1) {
-      const int rr = static_cast<int>(p_new) - r0;
-      if (warp == W - 1) {
-        __half *sd = reinterpret_cast<__half *>(ks + (st * TP + rr) * KP);
+  const uint32_t k_lane = ((lane & 7) + ((lane >> 3) & 1) * 8) * PITCH + (lane >> 4) * 16;
+  const uint32_t v_lane = BLK + ((lane & 7) + (lane >> 4) * 8) * PITCH + ((lane >> 3) & 1) * 16;
+  int st = 0;
+  for (int i = warp; i < nblk; i += W, st ^= 1) {
+    cp_async_wait<1>();
+    const uint32_t blk = ring + st * 2 * BLK;
+    if (owns_new && i == new_blk) {
+      const int rr = static_cast<int>(p_new - p0) & 15;
+      __half *sk = reinterpret_cast<__half *>(smem + warp * 4 * BLK + st * 2 * BLK + rr * PITCH);
+      __half *sv = reinterpret_cast<__half *>(smem + warp * 4 * BLK + st * 2 * BLK + BLK + rr * PITCH);
+      __syncwarp();  // other lanes' zero fill of this row has landed
 #pragma unroll
-        for (int u = 0; u < HALF / 32; ++u) {
-          sd[lane + 32 * u] = __float2half_rn(knew0[u]);
-          sd[lane + 32 * u + HALF] = __float2half_rn(knew1[u]);
-        }
+      for (int u = 0; u < HALF / 32; ++u) {
+        sk[lane + 32 * u] = knew0[u];
+        sk[lane + 32 * u + HALF] = knew1[u];
       }
-      if (warp == W - 2) {
-        __half *sd = reinterpret_cast<__half *>(vs + (st * TP + rr) * VP);
 #pragma unroll
-        for (int j = 0; j < DPL; ++j) sd[lane + 32 * j] = vnew[j];
+      for (int j = 0; j < DPL; ++j) sv[lane + 32 * j] = vnew[j];
+    }
+    __syncwarp();
+    float s[NB][4];
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb) s[nb][0] = s[nb][1] = s[nb][2] = s[nb][3] = 0.f;
+#pragma unroll
+    for (int k = 0; k < KS; ++k) {
+      uint32_t a0, a1, a2, a3;
+      ldmatrix_x4(blk + k_lane + 32 * k, a0, a1, a2, a3);
+#pragma unroll
+      for (int nb = 0; nb < NB; ++nb) mma_16816(s[nb], a0, a1, a2, a3, qf[nb][k][0], qf[nb][k][1]);
+    }
+    const int rows = p1 - p0 - 16 * i;  // valid rows of the block
+    uint32_t ph[NB][2], pl[NB][2];
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb) {
+      float corr[2], p[4];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float x0 = g < rows ? s[nb][h] * scale : -INFINITY, x1 = g + 8 < rows ? s[nb][2 + h] * scale : -INFINITY;
+        float mx = fmaxf(x0, x1);
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        const float mn = fmaxf(m_run[nb][h], mx);
+        corr[h] = __expf(m_run[nb][h] - mn);  // 0 the first time (m_run = -inf, mn finite)
+        m_run[nb][h] = mn;
+        p[h] = __expf(x0 - mn);
+        p[2 + h] = __expf(x1 - mn);
+        l_run[nb][h] = l_run[nb][h] * corr[h] + p[h] + p[2 + h];  // per-lane partial sum, reduced at the end
+      }
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const __half2 hi = __floats2half2_rn(p[2 * half], p[2 * half + 1]);
+        const float2 hf = __half22float2(hi);
+        const __half2 lo = __floats2half2_rn(p[2 * half] - hf.x, p[2 * half + 1] - hf.y);
+        ph[nb][half] = movmatrix_trans(*reinterpret_cast<const uint32_t *>(&hi));
+        pl[nb][half] = movmatrix_trans(*reinterpret_cast<const uint32_t *>(&lo));
+      }
+#pragma unroll
+      for (int k = 0; k < KS; ++k) {
+        acc[nb][k][0] *= corr[0];
+        acc[nb][k][1] *= corr[1];
+        acc[nb][k][2] *= corr[0];
+        acc[nb][k][3] *= corr[1];
       }
     }
-    __syncthreads();  // tile t (and, the first time, qs; the last time, the new row) visible to all warps
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int hq = head0 + hp * h;
-      if (!active || hq >= group) break;
-      const float4 *q4 = reinterpret_cast<const float4 *>(qs + hq * DH);
-      for (int rb = 32 * slice; rb < rows; rb += 32 * nsl) {
-        const int r = rb + lane;
-        float s = -INFINITY;
-        if (r < rows) {
-          const uint4 *kr = reinterpret_cast<const uint4 *>(ks + (st * TP + r) * KP);
-          float d0 = 0.f, d1 = 0.f;
+    for (int k = 0; k < KS; ++k) {
+      uint32_t a0, a1, a2, a3;
+      ldmatrix_x4_trans(blk + v_lane + 32 * k, a0, a1, a2, a3);
 #pragma unroll
-          for (int c = 0; c < VPR; ++c) {
-            const uint4 kv = kr[c];
-            const float4 qa = q4[2 * c], qb = q4[2 * c + 1];
-            const float2 k0 = __half22float2(*reinterpret_cast<const __half2 *>(&kv.x));
-            const float2 k1 = __half22float2(*reinterpret_cast<const __half2 *>(&kv.y));
-            const float2 k2 = __half22float2(*reinterpret_cast<const __half2 *>(&kv.z));
-            const float2 k3 = __half22float2(*reinterpret_cast<const __half2 *>(&kv.w));
-            d0 += qa.x * k0.x + qa.y * k0.y + qa.z * k1.x + qa.w * k1.y;
-            d1 += qb.x * k2.x + qb.y * k2.y + qb.z * k3.x + qb.w * k3.y;
-          }
-          s = d0 + d1;
-        }
-        const float mn = fmaxf(m_run[h], warp_max(s));
-        const float corr = __expf(m_run[h] - mn);  // 0 the first time (m_run = -inf, mn finite)
-        const float w = (r < rows) ? __expf(s - mn) : 0.f;
-        l_run[h] = l_run[h] * corr + w;            // per-lane partial sum, reduced at the end
-        m_run[h] = mn;
-#pragma unroll
-        for (int j = 0; j < DPL; ++j) acc[h][j] *= corr;
-        const int cnt = min(32, rows - rb);
-        const uint8_t *vrow = vs + (st * TP + rb) * VP + lane * DPL * 2;
-#pragma unroll 8
-        for (int j = 0; j < cnt; ++j) {
-          const float wj = __shfl_sync(0xffffffffu, w, j);
-          if (DPL == 4) {
-            const uint2 v = *reinterpret_cast<const uint2 *>(vrow + j * VP);
-            const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&v.x));
-            const float2 c = __half22float2(*reinterpret_cast<const __half2 *>(&v.y));
-            acc[h][0] += wj * a.x; acc[h][1] += wj * a.y; acc[h][2] += wj * c.x; acc[h][3] += wj * c.y;
-          } else {
-            const __half *vh = reinterpret_cast<const __half *>(vrow + j * VP);
-#pragma unroll
-            for (int d = 0; d < DPL; ++d) acc[h][d] += wj * __half2float(vh[d]);
-          }
-        }
+      for (int nb = 0; nb < NB; ++nb) {
+        mma_16816(acc[nb][k], a0, a1, a2, a3, pl[nb][0], pl[nb][1]);
+        mma_16816(acc[nb][k], a0, a1, a2, a3, ph[nb][0], ph[nb][1]);
       }
     }
-    __syncthreads();  // all warps done with stage st
-    if (t + 2 < ntile) load_tile(t + 2);
+    __syncwarp();  // every lane is done with the block before it is refilled
+    if (i + 2 * W < nblk) load_block(i + 2 * W, st);
+    cp_async_commit();
   }
+  cp_async_wait<0>();
 
-  // ---- 4. partials: slices above 0 hand theirs to slice 0 through shared memory, slice 0 writes
-  // the CTA's partial; merge by the last CTA of this (b, kvh)
-#pragma unroll
-  for (int h = 0; h < 2; ++h) l_run[h] = warp_sum(l_run[h]);
-  if (active && slice > 0) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      if (head0 + hp * h >= group) break;
-      float *dst = mrg + (warp * 2 + h) * PR;
-      if (lane == 0) {
-        dst[0] = m_run[h];
-        dst[1] = l_run[h];
-      }
-#pragma unroll
-      for (int j = 0; j < DPL; ++j) dst[4 + lane * DPL + j] = acc[h][j];
-    }
-  }
+  // ---- 4. merge of the warps
   __syncthreads();
-  if (slice == 0) {
+#pragma unroll
+  for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const int hq = head0 + hp * h;
-      if (hq >= group) break;
-      float m = m_run[h];
-      for (int sl = 1; sl < nsl; ++sl) m = fmaxf(m, mrg[((sl * hp + head0) * 2 + h) * PR]);
-      // (a slice that saw no row has max -inf and weight 0; slice 0 of a CTA with work always has rows)
-      const float w0 = __expf(m_run[h] - m);
-      float l = l_run[h] * w0;
+      float l = l_run[nb][h];
 #pragma unroll
-      for (int j = 0; j < DPL; ++j) acc[h][j] *= w0;
-      for (int sl = 1; sl < nsl; ++sl) {
-        const float *src = mrg + ((sl * hp + head0) * 2 + h) * PR;
-        const float ws = __expf(src[0] - m);
-        l += src[1] * ws;
-#pragma unroll
-        for (int j = 0; j < DPL; ++j) acc[h][j] += ws * src[4 + lane * DPL + j];
+      for (int o = 4; o < 32; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+      float *dst = mrg + (warp * 8 * NB + nb * 8 + 2 * t + h) * PR;
+      if (g == 0) {
+        dst[0] = m_run[nb][h];
+        dst[1] = l;
       }
-      float *dst = part + ((1ll * b * nq + kvh * group + hq) * nsplit + split) * PR;
+#pragma unroll
+      for (int k = 0; k < KS; ++k) {
+        dst[4 + 16 * k + g] = acc[nb][k][h];
+        dst[4 + 16 * k + g + 8] = acc[nb][k][2 + h];
+      }
+    }
+  __syncthreads();
+  for (int hq = warp; hq < group; hq += W) {
+    float m = -INFINITY, l = 0.f, a[DPL];
+#pragma unroll
+    for (int w = 0; w < W; ++w) m = fmaxf(m, mrg[(w * 8 * NB + hq) * PR]);
+#pragma unroll
+    for (int j = 0; j < DPL; ++j) a[j] = 0.f;
+#pragma unroll
+    for (int w = 0; w < W; ++w) {  // (a warp without rows has max -inf and weight 0; warp 0 always has rows)
+      const float *src = mrg + (w * 8 * NB + hq) * PR;
+      const float ws = __expf(src[0] - m);
+      l += src[1] * ws;
+#pragma unroll
+      for (int j = 0; j < DPL; ++j) a[j] += ws * src[4 + lane * DPL + j];
+    }
+    const int head = kvh * group + hq;
+    if (used == 1) {
+      __half *o = out + (1ll * b * nq + head) * DH + lane * DPL;
+      const float inv = 1.f / l;
+#pragma unroll
+      for (int j = 0; j < DPL; ++j) o[j] = __float2half_rn(a[j] * inv);
+    } else {
+      float *dst = part + ((1ll * b * nq + head) * nsplit + split) * PR;
       if (lane == 0) {
         dst[0] = m;
         dst[1] = l;
       }
 #pragma unroll
-      for (int j = 0; j < DPL; ++j) dst[4 + lane * DPL + j] = acc[h][j];
+      for (int j = 0; j < DPL; ++j) dst[4 + lane * DPL + j] = a[j];
     }
   }
+  if (used == 1) return;
   __threadfence();
   __syncthreads();
   if (tid == 0) {
@@ -686,8 +724,8 @@ int launch_rope_attn(const __half *qkv, const __half *qn, const __half *kn, cons
   int *counters = static_cast<int *>(scratch);
   float *part = reinterpret_cast<float *>(static_cast<uint8_t *>(scratch) + cnt);
   const int group = nq / nkv;
-  const int tp = 8192 / dh;
-  const int smem = 2 * tp * (2 * dh + 16) + 2 * tp * 2 * dh + group * dh * 4 + kFusedAttnWarps * 2 * (dh + 4) * 4;
+  const int nb = group <= 8 ? 1 : 2;
+  const int smem = kFusedAttnWarps * 4 * 16 * (2 * dh + 16) + 8 * nb * (dh + 8) * 2;
   auto launch = [&](auto kernel) -> int {
     cudaLaunchConfig_t cfg = {};
     // one CTA per SM while the (sequence, KV head) pairs fit: like the GEMVs around it
@@ -706,9 +744,9 @@ int launch_rope_attn(const __half *qkv, const __half *qn, const __half *kn, cons
     return RDQ_OK;
   };
   switch (dh) {
-    case 64: return launch(rope_attn_kernel<64>);
-    case 128: return launch(rope_attn_kernel<128>);
-    case 256: return launch(rope_attn_kernel<256>);
+    case 64: return nb == 1 ? launch(rope_attn_kernel<64, 1>) : launch(rope_attn_kernel<64, 2>);
+    case 128: return nb == 1 ? launch(rope_attn_kernel<128, 1>) : launch(rope_attn_kernel<128, 2>);
+    case 256: return nb == 1 ? launch(rope_attn_kernel<256, 1>) : launch(rope_attn_kernel<256, 2>);
   }
   RDQ_REQUIRE(false, RDQ_E_UNSUPPORTED, "head_dim must be 64, 128 or 256, got %d", dh);
   return RDQ_OK;
