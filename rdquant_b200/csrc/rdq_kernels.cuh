@@ -27,6 +27,7 @@ struct GemvArgs {
   const __half *bias;
   void *y;
   int n4, n8, n16, K;
+  int x_bf16 = 0;  // x is bf16: rounded to f16 as it is read
   int y_bf16 = 0;  // y is bf16 instead of f16
 };
 

@@ -75,7 +75,9 @@ Path path_of(const rdq_layer &l, int M) {
 }
 
 // true when the kernel of this path rounds bf16 rows itself
-bool takes_bf16(const rdq_layer &l, Path p, int M) { return p == Path::kGemvTiled && tiled_stages_x(M, l.K); }
+bool takes_bf16(const rdq_layer &l, Path p, int M) {
+  return p == Path::kGemvGeneric || p == Path::kPanelsGeneric || (p == Path::kGemvTiled && tiled_stages_x(M, l.K));
+}
 
 size_t align256(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
 
@@ -128,6 +130,7 @@ int run_gemv(const rdq_layer &l, bool tiled, const void *x, int x_bf16, int M, c
   a.n8 = l.n_fp8;
   a.n16 = l.n_fp16;
   a.K = l.K;
+  a.x_bf16 = x_bf16;
   a.y_bf16 = y_bf16;
   return launch_gemv_generic(a, stream);
 }
