@@ -47,6 +47,8 @@
 //
 // Reference behaviour replaced: the Marlin-repacked split-K family K2-K7 of
 // rdquant/csrc/fused_gemv.cu (:1244-1969; repack rdquant/fused_gemv_pack.py:151-172).
+#include <unordered_map>
+
 #include "rdq_kernels.cuh"
 
 namespace rdq {

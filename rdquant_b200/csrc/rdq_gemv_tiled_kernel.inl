@@ -968,48 +968,29 @@ static SmemPlan smem_plan(int M, int K) {
 }
 bool tiled_stages_x(int M, int K) { return M >= 1 && M <= RDQ_MAX_GEMV_M && smem_plan(M, K).xs; }
 
-int launch_gemv_tiled(const GemvTiledArgs &h, bool pdl, cudaStream_t stream) {
-  const int ck = tiled_chunk_k(h.K);
+// Schedule and shared-memory plan of a (shape, rows) pair.
+struct TiledPlan {
   TSched sc;
+  SmemPlan pl;
+};
+static TiledPlan make_tiled_plan(int n4, int n8, int n16, int K, int M) {
+  TiledPlan p;
+  TSched &sc = p.sc;
+  p.pl = smem_plan(M, K);
+  const int nst = p.pl.nst;
+  const int ck = tiled_chunk_k(K);
   sc.ck = ck;
-  sc.S4 = h.K / ck;
+  sc.S4 = K / ck;
   sc.S8 = sc.S4 * 2;
   sc.S16 = sc.S4 * 4;
-  sc.t4 = h.n4 / kTileRows;
-  sc.t8 = h.n8 / kTileRows;
-  const int t16 = h.n16 / kTileRows;
+  sc.t4 = n4 / kTileRows;
+  sc.t8 = n8 / kTileRows;
+  const int t16 = n16 / kTileRows;
   sc.e4 = sc.t4 * sc.S4;
   sc.e8 = sc.e4 + sc.t8 * sc.S8;
   sc.e16 = sc.e8 + t16 * sc.S16;
   sc.img4 = img_bytes(0, ck);
   sc.img8 = img_bytes(1, ck);
-
-  TiledArgs a;
-  a.x = static_cast<const __half *>(h.x); a.y_bf16 = h.y_bf16; a.M = h.M; a.tiled = h.tiled; a.s8 = h.s8; a.global4 = h.global4; a.perm = h.perm;
-  a.bias = h.bias; a.y = h.y; a.n4 = h.n4; a.n8 = h.n8; a.n16 = h.n16; a.K = h.K;
-  a.workspace = h.workspace; a.flags = h.flags;
-  a.early = pdl;
-  a.test_timeout = h.test_timeout;
-  a.n_dst = h.n_dst;
-  for (int d = 0; d < kMaxPeers; ++d) {
-    a.dst[d] = d < h.n_dst ? h.dst[d] : nullptr;
-    a.peer_flag[d] = d < h.n_dst ? h.peer_flag[d] : nullptr;
-  }
-  a.peer_state = h.peer_state;
-  a.xop = h.x_bf16 ? 3 : h.xop; a.x_aux = h.x_aux; a.x_weight = h.x_weight; a.x_out = h.x_out; a.x_eps = h.x_eps;
-  a.status_idx = sm_count();
-  a.slot_bytes = (img_bytes(0, ck) + 127) & ~127;
-  const int nt = h.M <= 8 ? 1 : 2;
-  const SmemPlan pl = smem_plan(h.M, h.K);
-  a.nepi = pl.nepi;
-  a.fdepth = pl.fdep;
-  a.nstages = pl.nst;
-  const bool xs = pl.xs;
-  const int nst = pl.nst;
-  RDQ_REQUIRE(a.xop == 0 || xs, RDQ_E_UNSUPPORTED,
-              "activation prologue needs the activation rows in shared memory (M=%d, K=%d)", h.M, h.K);
-  RDQ_REQUIRE(h.xop == 0 || (h.xop == 1 && h.x_weight) || h.xop == 2, RDQ_E_INVALID, "bad activation prologue");
-  const int smem = pl.smem;
 
   // Images are balanced by what they cost a CTA in time, not by their bytes: an NVFP4 image
   // (conversion + block scaling) takes more instructions than an FP8 or FP16 image of the
@@ -1059,6 +1040,62 @@ int launch_gemv_tiled(const GemvTiledArgs &h, bool pdl, cudaStream_t stream) {
   if (maxg < G) G = static_cast<int>(maxg);
   if (G < 1) G = 1;
   sc.G = G;
+  return p;
+}
+// The plans this thread has used (a decode step calls the same few layers again and again; the time
+// model above costs about as much host time as the launch itself).
+static const TiledPlan &tiled_plan(int n4, int n8, int n16, int K, int M) {
+  struct Key {
+    int v[6];
+    bool operator==(const Key &o) const { return std::equal(v, v + 6, o.v); }
+  };
+  struct Hash {
+    size_t operator()(const Key &k) const {
+      size_t h = 1469598103934665603ull;
+      for (int x : k.v) h = (h ^ static_cast<size_t>(x)) * 1099511628211ull;
+      return h;
+    }
+  };
+  static thread_local std::unordered_map<Key, TiledPlan, Hash> plans;
+  const Key key{{n4, n8, n16, K, M, sm_count()}};
+  auto it = plans.find(key);
+  if (it == plans.end()) {
+    if (plans.size() >= 4096) plans.clear();
+    it = plans.emplace(key, make_tiled_plan(n4, n8, n16, K, M)).first;
+  }
+  return it->second;
+}
+
+int launch_gemv_tiled(const GemvTiledArgs &h, bool pdl, cudaStream_t stream) {
+  const TiledPlan &plan = tiled_plan(h.n4, h.n8, h.n16, h.K, h.M);
+  const TSched &sc = plan.sc;
+  const SmemPlan &pl = plan.pl;
+  const int G = sc.G;
+  TiledArgs a;
+  a.x = static_cast<const __half *>(h.x); a.y_bf16 = h.y_bf16; a.M = h.M; a.tiled = h.tiled; a.s8 = h.s8; a.global4 = h.global4; a.perm = h.perm;
+  a.bias = h.bias; a.y = h.y; a.n4 = h.n4; a.n8 = h.n8; a.n16 = h.n16; a.K = h.K;
+  a.workspace = h.workspace; a.flags = h.flags;
+  a.early = pdl;
+  a.test_timeout = h.test_timeout;
+  a.n_dst = h.n_dst;
+  for (int d = 0; d < kMaxPeers; ++d) {
+    a.dst[d] = d < h.n_dst ? h.dst[d] : nullptr;
+    a.peer_flag[d] = d < h.n_dst ? h.peer_flag[d] : nullptr;
+  }
+  a.peer_state = h.peer_state;
+  a.xop = h.x_bf16 ? 3 : h.xop; a.x_aux = h.x_aux; a.x_weight = h.x_weight; a.x_out = h.x_out; a.x_eps = h.x_eps;
+  a.status_idx = sm_count();
+  a.slot_bytes = (img_bytes(0, sc.ck) + 127) & ~127;
+  const int nt = h.M <= 8 ? 1 : 2;
+  a.nepi = pl.nepi;
+  a.fdepth = pl.fdep;
+  a.nstages = pl.nst;
+  const bool xs = pl.xs;
+  RDQ_REQUIRE(a.xop == 0 || xs, RDQ_E_UNSUPPORTED,
+              "activation prologue needs the activation rows in shared memory (M=%d, K=%d)", h.M, h.K);
+  RDQ_REQUIRE(h.xop == 0 || (h.xop == 1 && h.x_weight) || h.xop == 2, RDQ_E_INVALID, "bad activation prologue");
+  const int smem = pl.smem;
+
   RDQ_REQUIRE(sc.W / G / sc.u16 + 2 <= kMaxList, RDQ_E_UNSUPPORTED,
               "layer too large for the tiled GEMV: more than %d images per CTA", kMaxList);
 
@@ -1098,7 +1135,7 @@ int launch_gemv_tiled(const GemvTiledArgs &h, bool pdl, cudaStream_t stream) {
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  void *params[2] = {&a, &sc};
+  void *params[2] = {&a, const_cast<TSched *>(&sc)};
   RDQ_CUDA(cudaLaunchKernelExC(&cfg, fn, params));
   return RDQ_OK;
 }
