@@ -9,21 +9,11 @@ struct TSched {
   int S4, S8, S16;   // images per tile in each group
   int t4, t8;        // tiles in the NVFP4 / FP8 groups
   int e4, e8, e16;   // end of each group's image range
-  int u4, u8, u16;   // scheduling cost of one NVFP4 / FP8 / FP16 image
   int img4, img8;    // image bytes (FP8 and FP16 images have the same size)
-  long long w4, w8, W;
-  int G;
+  int G;             // CTAs with images
+  int bound[kMaxCtas + 1];  // first image of every CTA (computed by the launcher: three 64-bit divisions)
 
-  __device__ __forceinline__ int image_of_pos(long long p) const {
-    if (p < w4) return static_cast<int>(p / u4);
-    if (p < w8) return e4 + static_cast<int>((p - w4) / u8);
-    if (p < W) return e8 + static_cast<int>((p - w8) / u16);
-    return e16;
-  }
-  __device__ __forceinline__ int boundary(int b) const {
-    if (b >= G) return e16;
-    return image_of_pos(W * b / G);
-  }
+  __device__ __forceinline__ int boundary(int b) const { return bound[b < G ? b : G]; }
   __device__ __forceinline__ int tile_of_image(int s) const {
     if (s < e4) return s / S4;
     if (s < e8) return t4 + (s - e4) / S8;
@@ -35,15 +25,6 @@ struct TSched {
     return 1ll * e4 * img4 + 1ll * (s - e4) * img8;
   }
 };
-
-// processing order of a CTA's tile segments: the (possibly split) first tile, whose
-// partial another CTA is waiting for, then the (possibly split) last tile, which this
-// CTA finishes, then the whole tiles in between
-__device__ __forceinline__ int tseg_order(int q, int nseg) {
-  if (q == 0) return 0;
-  if (q == 1) return nseg - 1;
-  return q - 1;
-}
 
 // x is written by the preceding kernel: coherent loads, issued only after the PDL wait
 __device__ __forceinline__ uint4 t_ldx16(const __half *p) {
@@ -63,11 +44,25 @@ __device__ __forceinline__ uint32_t t_ldx4(const __half *p) {
   return v;
 }
 
+__device__ __forceinline__ uint4 ldg_nc16(const void *p) {
+  uint4 v;
+  asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
 __device__ __forceinline__ uint4 ldg_cg16(const void *p) {
   uint4 v;
   asm volatile("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
   return v;
 }
+
+constexpr uint32_t kIdle = 0xffffffffu;  // a workspace word that holds no partial sum
+__device__ __forceinline__ uint4 ld_relaxed16(const float *p) {
+  uint4 v;
+  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+
+constexpr int kStageUnroll = 2;  // pair-loop unrolling of the NVFP4 / FP8 stages
 
 struct TiledArgs {
   const __half *x;  // bf16 rows with xop == 3
@@ -85,7 +80,6 @@ struct TiledArgs {
   int status_idx;
   int nstages;
   int slot_bytes;
-  int nepi;    // epilogue warps in use
   int fdepth;  // slots per hand-over ring
   int early;         // weights may be read before the kernel before this one has finished
   int test_timeout;  // self-test: CTA 0 ends with a wait that runs out
@@ -108,7 +102,6 @@ struct TiledArgs {
   float x_eps;
 };
 
-constexpr int kStageUnroll = 2;  // pair-loop unrolling of the NVFP4 / FP8 stages
 
 // Activation fragment loads: from the shared-memory copy (XS) or from global memory.
 // `base` is a shared-memory byte address (XS) or a generic pointer value.
@@ -150,13 +143,15 @@ __device__ __forceinline__ uint32_t lds_u32(uint32_t addr) {
   return v;
 }
 
-// multiply-accumulate one NVFP4 piece (16 rows x 32 k): raw words of rows g / g+8, the
-// E4M3 scale pair of the piece for each row (low 16 bits), the lane's 8 activations
+// multiply-accumulate one NVFP4 piece (16 rows x 32 k): raw words of rows g / g+8, the lane's block
+// scales of the two rows (low and high half: the multiplies take either half of a register at no
+// cost), the lane's 8 activations
 template <int NT>
-__device__ __forceinline__ void fp4_piece(float (&acc)[NT][2][4], uint32_t wg, uint32_t wg8, uint32_t sraw_g,
-                                          uint32_t sraw_g8, uint32_t sel, const uint4 (&xv)[NT]) {
-  const uint32_t sg = __byte_perm(cvt_e4m3x2(sraw_g), 0u, sel);
-  const uint32_t sg8 = __byte_perm(cvt_e4m3x2(sraw_g8), 0u, sel);
+__device__ __forceinline__ void fp4_piece(float (&acc)[NT][2][4], uint32_t wg, uint32_t wg8, uint32_t scales,
+                                          const uint4 (&xv)[NT]) {
+  const __half2 sc = *reinterpret_cast<const __half2 *>(&scales);
+  const __half2 lo = __low2half2(sc), hi = __high2half2(sc);
+  const uint32_t sg = *reinterpret_cast<const uint32_t *>(&lo), sg8 = *reinterpret_cast<const uint32_t *>(&hi);
   uint32_t a0, a1, a2, a3, b0, b1, b2, b3;
   cvt_e2m1x8(wg, a0, a1, a2, a3);
   cvt_e2m1x8(wg8, b0, b1, b2, b3);
@@ -190,8 +185,10 @@ __device__ __forceinline__ void stage_fp4(float (&acc)[NT][2][4], uint32_t lm_ad
       x0[n] = ldx16<XS>(xb[n], xoff);
       x1[n] = ldx16<XS>(xb[n], xoff + 64);
     }
-    fp4_piece<NT>(acc, w[0], w[1], s_g, s_g8, sel, x0);
-    fp4_piece<NT>(acc, w[2], w[3], s_g >> 16, s_g8 >> 16, sel, x1);
+    uint32_t sc0, sc1;  // (row g, row g + 8) of pieces p and p + 1
+    cvt_e4m3x4(__byte_perm(s_g, s_g8, sel), sc0, sc1);
+    fp4_piece<NT>(acc, w[0], w[1], sc0, x0);
+    fp4_piece<NT>(acc, w[2], w[3], sc1, x1);
     lm_addr += 32;
     sc_addr += 4;
     sc8_addr += 4;
@@ -253,12 +250,6 @@ __device__ __forceinline__ void stage_fp16(float (&acc)[NT][2][4], uint32_t lm_a
   if (i < npairs) one(0);
 }
 
-// Stage list entry (one 32-bit word per image this CTA streams, in processing order):
-//   bits 1:0 format, bit 2 "hand over after this stage", bits 10:3 chunk index inside the
-//   tile, bits 12:11 the epilogue warp that finishes the tile, bits 31:13 image index relative
-//   to the CTA's first image.
-constexpr uint32_t kEntFlush = 4u;
-
 // first image, image count and format of tile gtile
 __device__ __forceinline__ void tile_geom(const TSched &sc, int gtile, int &first_img, int &S, int &fmt) {
   if (gtile < sc.t4) {
@@ -273,14 +264,21 @@ __device__ __forceinline__ void tile_geom(const TSched &sc, int gtile, int &firs
 // NT = number of 8-row activation groups (1: M <= 8, 2: M <= 16)
 // EXTRA: the launch has an activation prologue or peer destinations (compiled apart so that the
 // plain launch carries none of that code)
+//
+// Warp group g takes the g-th third of the CTA's images, in order, through ring slots g, g + 3, ... of
+// its own; epilogue warp g finishes the tiles whose first image (in this CTA) lies in that third.  A
+// group therefore hands sums over once per tile -- images dealt out in turn would end every stage of a
+// two-image tile with a hand-over, which measured a third of the MMA warps' time -- and everybody
+// derives his images from the range alone, without a list.
 template <int NT, bool XS, bool EXTRA>
 __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_constant__ TiledArgs a,
                                                   const __grid_constant__ TSched sc) {
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ __align__(8) uint64_t bar_full[kMaxStages];
   __shared__ __align__(8) uint64_t bar_empty[kMaxStages];
-  __shared__ __align__(8) uint64_t fl_full[kGroups][kEpiWarps][kFlushRing];
-  __shared__ __align__(8) uint64_t fl_empty[kGroups][kEpiWarps][kFlushRing];
+  __shared__ __align__(8) uint64_t fl_full[kGroups][kFlushRing];   // a group's hand-over ring
+  __shared__ __align__(8) uint64_t fl_empty[kGroups][kFlushRing];
+  __shared__ __align__(8) uint64_t fl_cross[kGroups];  // its sums of a tile that an earlier group started
   __shared__ __align__(8) uint64_t bar_x;
   __shared__ __align__(8) uint64_t bar_never;  // nothing ever arrives here (time-out self-test)
   __shared__ float xred[EXTRA ? RDQ_MAX_GEMV_M : 1][kMmaWarps];  // activation prologue: per-warp sums of squares
@@ -291,255 +289,148 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
   const int K = a.K, M = a.M;
   const int N = a.n4 + a.n8 + a.n16;
   const int nst = a.nstages;
-  // hand-over rings, one per (warp group, epilogue warp): kFlushRing slots of
-  // [4 warps][16 rows][mp] partial sums; each ring has one writer group and one reader warp,
-  // which both follow its barriers phase by phase
-  const int mp = (M <= 3) ? M : ((M + 3) & ~3);  // M > 3: rows of four floats, read 16 B at a time
-  const int vp = (M <= 4) ? 4 : 16;               // row pitch of an epilogue warp's staging tile
-  const int nepi = a.nepi;      // epilogue warps in use (1..kEpiWarps)
+  // hand-over slots of [4 warps][16 rows][mp] partial sums: fdep per group, then one per later group
+  // for the tile it shares with an earlier one
+  const int mp = (M + 3) & ~3;
   const int fdep = a.fdepth;    // slots per hand-over ring (1 or 2)
   const int gslot_floats = kWarpsPerGroup * kTileRows * mp;
   float *flush = reinterpret_cast<float *>(smem + nst * a.slot_bytes);
-  int *meta_col = reinterpret_cast<int *>(flush + kGroups * nepi * fdep * gslot_floats);
-  float *meta_scl = reinterpret_cast<float *>(meta_col + kMetaSegs * kTileRows);
-  float *meta_bia = meta_scl + kMetaSegs * kTileRows;
-  uint32_t *list = reinterpret_cast<uint32_t *>(meta_bia + kMetaSegs * kTileRows);
-  uint32_t *segtab = list + kMaxList;
-  float *vstage = reinterpret_cast<float *>(segtab + kMaxList);  // per epilogue warp: [16 rows][16] finished sums of a tile
-  uint8_t *xsm = reinterpret_cast<uint8_t *>(vstage + kEpiWarps * kTileRows * vp);
+  uint8_t *xsm = reinterpret_cast<uint8_t *>(flush + (kGroups * fdep + kGroups - 1) * gslot_floats);
   const int xpitch = 2 * a.K + 16;  // activation row pitch in shared memory: skewed against bank conflicts
 
-  // lane L holds the first image of CTA bx + L (one call site for the 64-bit divisions)
-  const int bnd = sc.boundary(static_cast<int>(blockIdx.x) + lane);
-  const int s_begin = __shfl_sync(0xffffffffu, bnd, 0);
-  const int s_end = __shfl_sync(0xffffffffu, bnd, 1);
+  const int s_begin = sc.boundary(blockIdx.x), s_end = sc.boundary(blockIdx.x + 1);
   const int nimg = s_end - s_begin;
-  const int first_tile = (nimg > 0) ? sc.tile_of_image(s_begin) : 0;
-  const int nseg = (nimg > 0) ? (sc.tile_of_image(s_end - 1) - first_tile + 1) : 0;
+  auto third = [&](int g) { return s_begin + nimg * g / kGroups; };
   int32_t *status = a.flags + a.status_idx;
   const int ck = sc.ck;
   const int pitch = (ck >> 1) + 16;
 
-  if (tid == 0) {
-    for (int i = 0; i < nst; ++i) {
-      mbar_init(smem_u32(&bar_full[i]), 1);
-      mbar_init(smem_u32(&bar_empty[i]), kWarpsPerGroup);
-    }
-    for (int g = 0; g < kGroups; ++g)
-      for (int j = 0; j < kEpiWarps; ++j)
-        for (int i = 0; i < kFlushRing; ++i) {
-          mbar_init(smem_u32(&fl_full[g][j][i]), kWarpsPerGroup);
-          mbar_init(smem_u32(&fl_empty[g][j][i]), 1);
-        }
-    mbar_init(smem_u32(&bar_x), 1);
-    mbar_init(smem_u32(&bar_never), 1);
-    mbar_init_fence();
-  }
-  __syncthreads();
   // Let the next kernel in the stream become resident as early as possible; until this
   // grid completes it only fills its own shared-memory ring with weights.
   pdl_launch_dependents();
-  if (nimg > kMaxList) {  // the launcher refuses such shapes; never reached
-    if (tid == 0) atomicExch(status, 8);
+  if (static_cast<int>(blockIdx.x) >= sc.G) {
+    // The grid has a CTA for every SM: one without images holds its place until the kernel before is
+    // done, so that the next launch finds one free place per SM, not two on some.
+    if (tid == 0) pdl_wait();
     return;
   }
 
   const uint32_t smem_base = smem_u32(smem);
+  if (warp != kMmaWarps) __syncthreads();  // the barriers are set up (the producer warp's part of this is below)
 
   if (warp == kMmaWarps) {
     // ==================================================================== producer
-    // The whole warp first writes the stage list: the CTA's images in processing order --
-    // the (possibly split) first tile, whose partial sums another CTA waits for, then the
-    // (possibly split) last tile, which this CTA finishes, then the whole tiles in between.
-    {
-      int f0, S0, fmt0;
-      tile_geom(sc, first_tile, f0, S0, fmt0);
-      const int n0 = min(s_end, f0 + S0) - s_begin;  // images of the first tile
-      int nl = 0;                                    // images of the last tile
-      if (nseg >= 2) {
-        int fl, Sl, fmtl;
-        tile_geom(sc, first_tile + nseg - 1, fl, Sl, fmtl);
-        nl = s_end - max(s_begin, fl);
-      }
-      auto rel_of = [&](int it) { return it < n0 ? it : (it < n0 + nl ? nimg - nl + (it - n0) : it - nl); };
-      for (int it = lane; it < nimg; it += 32) {
-        const int rel = rel_of(it);
-        const int gt = sc.tile_of_image(s_begin + rel);
-        int f, S, fmt;
-        tile_geom(sc, gt, f, S, fmt);
-        // position of the tile in processing order, and the epilogue warp that takes it
-        const int idx = gt - first_tile;
-        const int q = (idx == 0) ? 0 : (idx == nseg - 1 ? 1 : idx + 1);
-        uint32_t e = static_cast<uint32_t>(fmt) | (static_cast<uint32_t>(s_begin + rel - f) << 3) |
-                     (static_cast<uint32_t>(q % nepi) << 11) | (static_cast<uint32_t>(rel) << 13);
-        // the group that takes this stage hands its sums over after its last stage of the tile;
-        // its next stage sits three slots further, or in its first slot of the next round
-        const int sl = it % nst;
-        const int nxt = (sl + kGroups < nst) ? it + kGroups : it + (nst - sl) + sl % kGroups;
-        if (nxt >= nimg || sc.tile_of_image(s_begin + rel_of(nxt)) != gt) e |= kEntFlush;
-        list[it] = e;
-      }
-      __syncwarp();
-    }
-    if (lane != 0) return;
-    if (!a.early) pdl_wait();
+    const int most = (nimg + kGroups - 1) / kGroups;  // images of the longest third
+    auto copy_in = [&](int img, int slot) {
+      const uint32_t bytes = static_cast<uint32_t>(img < sc.e4 ? sc.img4 : sc.img8);
+      const uint32_t full = smem_u32(&bar_full[slot]);
+      mbar_arrive_expect_tx(full, bytes);
+      bulk_g2s(smem_base + slot * a.slot_bytes, a.tiled + sc.image_offset(img), bytes, full);
+    };
     // The ring is filled with weights first (they do not depend on the preceding kernel);
     // only then wait for that kernel and fetch the activations it produced.
-    bool x_sent = false;
-    auto send_x = [&]() {
-      if (x_sent) return;
-      x_sent = true;
-      // Only this thread executes the grid-dependency wait; every other warp of the CTA
-      // sleeps on bar_x, which completes after it (and after the activation copies).
-      pdl_wait();
-      const uint32_t bx = smem_u32(&bar_x);
-      if (XS && (!EXTRA || a.xop == 0)) {
-        mbar_arrive_expect_tx(bx, static_cast<uint32_t>(M) * 2u * K);
-        for (int m = 0; m < M; ++m) bulk_g2s(smem_u32(xsm) + m * xpitch, a.x + 1ll * m * K, 2u * K, bx);
-      } else {  // the MMA warps fetch (and transform) the activations themselves
-        mbar_arrive(bx);
-      }
+    auto fill = [&]() {
+      int slot = 0;
+      for (int j = 0; j < most && slot < nst; ++j)
+        for (int g = 0; g < kGroups && slot < nst; ++g, ++slot)
+          if (third(g) + j < third(g + 1)) copy_in(third(g) + j, slot);
     };
-    int slot = 0, round = 0;
+    if (lane == 0) {
+      for (int i = 0; i < nst; ++i) {
+        mbar_init(smem_u32(&bar_full[i]), 1);
+        mbar_init(smem_u32(&bar_empty[i]), kWarpsPerGroup);
+      }
+      for (int g = 0; g < kGroups; ++g) {
+        for (int i = 0; i < kFlushRing; ++i) {
+          mbar_init(smem_u32(&fl_full[g][i]), kWarpsPerGroup);
+          mbar_init(smem_u32(&fl_empty[g][i]), 1);
+        }
+        mbar_init(smem_u32(&fl_cross[g]), kWarpsPerGroup);
+      }
+      mbar_init(smem_u32(&bar_x), 1);
+      mbar_init(smem_u32(&bar_never), 1);
+      mbar_init_fence();
+      if (a.early) fill();
+    }
+    __syncwarp();
+    __syncthreads();
+    if (lane != 0) return;
+    // Only this thread executes the grid-dependency wait; every other warp of the CTA
+    // sleeps on bar_x, which completes after it (and after the activation copies).
+    pdl_wait();
+    const uint32_t bx = smem_u32(&bar_x);
+    if (XS && (!EXTRA || a.xop == 0)) {
+      mbar_arrive_expect_tx(bx, static_cast<uint32_t>(M) * 2u * K);
+      for (int m = 0; m < M; ++m) bulk_g2s(smem_u32(xsm) + m * xpitch, a.x + 1ll * m * K, 2u * K, bx);
+    } else {  // the MMA warps fetch (and transform) the activations themselves
+      mbar_arrive(bx);
+    }
+    if (!a.early) fill();
+    // Refills.  Image j of a third sits in the (j mod slots)-th slot of its group; at[g], par: the slot
+    // that is next for group g and the parity of the phase in which it was last given back.
+    int at[kGroups], par = 0;
+#pragma unroll
+    for (int g = 0; g < kGroups; ++g) at[g] = g;
 #pragma unroll 1
-    for (int it = 0; it < nimg; ++it) {
-      const uint32_t e = list[it];
-      const uint32_t bytes = static_cast<uint32_t>((e & 3u) == 0 ? sc.img4 : sc.img8);
-      if (round > 0) {
-        send_x();
-        if (!mbar_wait(smem_u32(&bar_empty[slot]), (round - 1) & 1)) {
+    for (int j = nst / kGroups; j < most; ++j) {
+#pragma unroll
+      for (int g = 0; g < kGroups; ++g) {
+        const int img = third(g) + j;
+        if (g + kGroups * j < nst || img >= third(g + 1)) continue;  // in the first fill, or none left
+        if (!mbar_wait(smem_u32(&bar_empty[at[g]]), (par >> g) & 1)) {
           atomicExch(status, 1);
           return;
         }
+        copy_in(img, at[g]);
+        at[g] += kGroups;
+        if (at[g] >= nst) {
+          at[g] = g;
+          par ^= 1 << g;
+        }
       }
-      const uint32_t full = smem_u32(&bar_full[slot]);
-      mbar_arrive_expect_tx(full, bytes);
-      bulk_g2s(smem_base + slot * a.slot_bytes, a.tiled + sc.image_offset(s_begin + static_cast<int>(e >> 13)), bytes,
-               full);
-      if (++slot == nst) { slot = 0; ++round; }
     }
-    send_x();
     return;
   }
 
   if (warp > kMmaWarps) {
     // =============================================================== epilogue warps
-    // The first nepi of them take the tile segments in turn: segment q (in processing
-    // order) belongs to warp q % nepi.
     const int ej = warp - kMmaWarps - 1;
-    if (ej >= nepi) return;
-    float *vst = vstage + ej * kTileRows * vp;
     if (!a.early) pdl_wait();
-    // output column, scale and bias of every row this CTA finishes: constants of the
-    // layer, fetched up front so that finishing a tile needs no global round trip.  With
-    // more than one epilogue warp the first builds the segment table and the others do this.
-    if (ej > 0 || nepi == 1) {
-      const int nmeta = min(nseg, kMetaSegs) * kTileRows;
-      const int nload = (nepi == 1) ? 1 : nepi - 1;
-      for (int base = (nepi == 1 ? 0 : ej - 1) * 128; base < nmeta; base += 128 * nload) {
-        int col[4];
-        float scl[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int item = base + u * 32 + lane;
-          col[u] = 0;
-          scl[u] = 1.f;
-          if (item < nmeta) {
-            const int gt = first_tile + (item >> 4);
-            const int prow = gt * kTileRows + (item & 15);
-            col[u] = a.perm ? a.perm[prow] : prow;
-            scl[u] = (gt < sc.t4) ? a.global4 : (gt < sc.t4 + sc.t8 ? a.s8[prow - a.n4] : 1.f);
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int item = base + u * 32 + lane;
-          if (item < nmeta) {
-            meta_col[item] = col[u];
-            meta_scl[item] = scl[u];
-            meta_bia[item] = a.bias ? __half2float(a.bias[col[u]]) : 0.f;
-          }
-        }
+    const int g_begin = third(ej), g_end = third(ej + 1);
+    // the first tile to finish: the one of the group's first image, unless an earlier group has an image of it
+    int gt = 0, f = 0, S = 1, fmt = 0;
+    bool mine = g_begin < g_end;
+    if (mine) {
+      gt = sc.tile_of_image(g_begin);
+      tile_geom(sc, gt, f, S, fmt);
+      if (f < g_begin && g_begin > s_begin) {
+        ++gt;
+        mine = f + S < g_end;
+        if (mine) tile_geom(sc, gt, f, S, fmt);
       }
     }
-    // Segment table: one word per tile segment, in processing order --
-    //   bits 8:0 tile index inside the CTA, bit 9 "tile starts here", bit 10 "tile ends here",
-    //   bits 13:11 warp groups that hold partial sums of it, bits 15:14 / 17:16 / 19:18 for
-    //   each group the number (modulo 4) of hand-overs it made to this segment's epilogue
-    //   warp before: ring slot = bit 0, barrier parity = bit 1.
-    // Built by one whole warp: a prefix sum over lanes q, q - nepi, q - 2 nepi, ...
-    if (ej == 0) {
-      int f0, S0, fmt0;
-      tile_geom(sc, first_tile, f0, S0, fmt0);
-      const int n0 = min(s_end, f0 + S0) - s_begin;  // images of the first tile
-      int nl = 0;                                    // images of the last tile
-      if (nseg >= 2) {
-        int fl, Sl, fmtl;
-        tile_geom(sc, first_tile + nseg - 1, fl, Sl, fmtl);
-        nl = s_end - max(s_begin, fl);
-      }
-      int carry[kEpiWarps];  // hand-over counts so far per epilogue warp: 10 bits per group
-#pragma unroll
-      for (int j = 0; j < kEpiWarps; ++j) carry[j] = 0;
-      for (int base = 0; base < nseg; base += 32) {
-        const int q = base + lane;
-        const int qe = q % nepi;
-        int inc = 0;
-        uint32_t e = 0;
-        if (q < nseg) {
-          const int idx = tseg_order(q, nseg);
-          int f, S, fmt;
-          tile_geom(sc, first_tile + idx, f, S, fmt);
-          const int ia = max(s_begin, f), ib = min(s_end, f + S);
-          const int nstage = ib - ia;
-          const int it0 = (q == 0) ? 0 : (q == 1 ? n0 : n0 + nl + (f - (s_begin + n0)));
-          e = static_cast<uint32_t>(idx) | (ia == f ? 1u << 9 : 0u) | (ib == f + S ? 1u << 10 : 0u);
-          // groups that take a stage of this tile: stage i sits in slot i % nst, group slot % 3
-          int mask = 0;
-          for (int i = 0; i < nstage && mask != (1 << kGroups) - 1; ++i) mask |= 1 << (((it0 + i) % nst) % kGroups);
-#pragma unroll
-          for (int g = 0; g < kGroups; ++g) {
-            if ((mask >> g) & 1) {
-              inc |= 1 << (10 * g);
-              e |= 1u << (11 + g);
-            }
-          }
-        }
-        int x = inc;
-        for (int off = nepi; off < 32; off <<= 1) {
-          const int y = __shfl_up_sync(0xffffffffu, x, off);
-          if (lane >= off) x += y;
-        }
-        int mycarry = carry[0];
-#pragma unroll
-        for (int j = 1; j < kEpiWarps; ++j)
-          if (qe == j) mycarry = carry[j];
-        const int before = x - inc + mycarry;
-#pragma unroll
-        for (int g = 0; g < kGroups; ++g) e |= static_cast<uint32_t>((before >> (10 * g)) & 3) << (14 + 2 * g);
-        if (q < nseg) segtab[q] = e;
-        // totals of this chunk per epilogue warp: held by the last lane of each residue class
-#pragma unroll
-        for (int j = 0; j < kEpiWarps; ++j) {
-          if (j < nepi) {
-            int last = 31 - (((base + 31) % nepi) - j + nepi) % nepi;
-            carry[j] += __shfl_sync(0xffffffffu, x, last);
-          }
-        }
-      }
-    }
+    // output column, scale and bias of a tile's rows are constants of the layer: those of the next
+    // tile are fetched while this one is computed
+    const int row = lane & 15;
+    int col = 0;
+    float scl = 1.f, bia = 0.f;
+    auto fetch = [&](int tile) {
+      const int prow = tile * kTileRows + row;
+      col = a.perm ? a.perm[prow] : prow;
+      scl = (tile < sc.t4) ? a.global4 : (tile < sc.t4 + sc.t8 ? a.s8[prow - a.n4] : 1.f);
+      bia = a.bias ? __half2float(a.bias[col]) : 0.f;
+    };
+    if (mine) fetch(gt);
     // a split tile whose first image this CTA holds (only its last tile can be one): the
     // other parts come from the CTAs bx + 1 .. b_last, in that order
     int b_last = blockIdx.x;
-    {
-      int f, S, fmt;
-      tile_geom(sc, first_tile + nseg - 1, f, S, fmt);
-      const int s_last = f + S - 1;
-      b_last += __popc(__ballot_sync(0xffffffffu, lane >= 1 && bnd <= s_last && bnd < sc.e16));
+    if (nimg > 0) {
+      int fl, Sl, fmtl;
+      tile_geom(sc, sc.tile_of_image(s_end - 1), fl, Sl, fmtl);
+      const int bnd = sc.boundary(static_cast<int>(blockIdx.x) + lane);  // first image of CTA bx + lane
+      b_last += __popc(__ballot_sync(0xffffffffu, lane >= 1 && bnd <= fl + Sl - 1 && bnd < sc.e16));
       if (lane == 0 && b_last >= static_cast<int>(blockIdx.x) + 31) atomicExch(status, 7);
     }
-    // metadata and segment table are complete for all epilogue warps in use
-    asm volatile("bar.sync 1, %0;" ::"r"(nepi * 32) : "memory");
     // y, workspace and flags belong to this launch only once the preceding grid is done
     if (!mbar_wait(smem_u32(&bar_x), 0)) {
       if (lane == 0) atomicExch(status, 6);
@@ -547,122 +438,121 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
     }
     // work item = (row, quad of four activation rows): lane L takes item L, and item L + 32
     // when M > 8
-    const int row = lane & 15;
-    const int nitem = (M > 8) ? 2 : 1;
+    constexpr int kItems = NT;
     float *ws_row = a.workspace + 1ll * blockIdx.x * 256 + row * 16;
+    int fslot = 0, fpar = 0;
 #pragma unroll 1
-    for (int q = ej; q < nseg; q += nepi) {
-      const uint32_t e = segtab[q];
-      const int idx = e & 511;
-      const bool starts = (e >> 9) & 1, ends = (e >> 10) & 1;
-#pragma unroll
-      for (int g = 0; g < kGroups; ++g) {
-        const int code = (e >> (14 + 2 * g)) & 3;  // hand-overs before, modulo 4
-        const int fsl = (fdep == 2) ? (code & 1) : 0, fpar = (fdep == 2) ? (code >> 1) : (code & 1);
-        if (((e >> (11 + g)) & 1) && !mbar_wait(smem_u32(&fl_full[g][ej][fsl]), fpar)) {
-          if (lane == 0) atomicExch(status, 2);
-          return;
-        }
-      }
-      int col;
-      float scl, bia;
-      if (idx < kMetaSegs) {
-        col = meta_col[idx * kTileRows + row];
-        scl = meta_scl[idx * kTileRows + row];
-        bia = meta_bia[idx * kTileRows + row];
-      } else {
-        const int gt = first_tile + idx;
-        const int prow = gt * kTileRows + row;
-        col = a.perm ? a.perm[prow] : prow;
-        scl = (gt < sc.t4) ? a.global4 : (gt < sc.t4 + sc.t8 ? a.s8[prow - a.n4] : 1.f);
-        bia = a.bias ? __half2float(a.bias[col]) : 0.f;
-      }
-      // Sum first and give the ring slots back at once: the barrier arrival is a release,
+    while (mine) {
+      const int ia = max(f, s_begin), ib = min(f + S, s_end);
+      const bool starts = ia == f, ends = ib == f + S;
+      const int cur_col = col;
+      const float cur_scl = scl, cur_bia = bia;
+      // the next tile of this third
+      const bool more = f + S < g_end;
+      if (more) fetch(gt + 1);
+      // Sum first and give the ring slot back at once: the barrier arrival is a release,
       // and behind a global store it would wait for that store to be acknowledged.
-      if (M <= 3) {
-        // up to three activation rows: scalar reads, lane = (row, m parity)
-#pragma unroll 1
-        for (int m = lane >> 4; m < M; m += 2) {
-          float v = 0.f;
+      float4 v[kItems];
 #pragma unroll
-          for (int g = 0; g < kGroups; ++g) {
-            if ((e >> (11 + g)) & 1) {
-              const float *ring = flush + ((g * nepi + ej) * fdep + (fdep == 2 ? ((e >> (14 + 2 * g)) & 1) : 0)) * gslot_floats;
+      for (int j = 0; j < kItems; ++j) v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+      auto add = [&](const float *ring) {
 #pragma unroll
-              for (int w = 0; w < kWarpsPerGroup; ++w) v += ring[(w * kTileRows + row) * mp + m];
-            }
-          }
-          vst[row * vp + m] = v;
-        }
-      } else {
-#pragma unroll 1
-        for (int j = 0; j < nitem; ++j) {
+        for (int j = 0; j < kItems; ++j) {
           const int m0 = ((lane >> 4) + 2 * j) * 4;
-          if (m0 < M) {
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (m0 >= M) continue;
 #pragma unroll
-            for (int g = 0; g < kGroups; ++g) {
-              if ((e >> (11 + g)) & 1) {
-                const float *ring = flush + ((g * nepi + ej) * fdep + (fdep == 2 ? ((e >> (14 + 2 * g)) & 1) : 0)) * gslot_floats;
-#pragma unroll
-                for (int w = 0; w < kWarpsPerGroup; ++w) {
-                  const float4 p = *reinterpret_cast<const float4 *>(ring + (w * kTileRows + row) * mp + m0);
-                  v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
-                }
-              }
-            }
-            *reinterpret_cast<float4 *>(vst + row * vp + m0) = v;
+          for (int w = 0; w < kWarpsPerGroup; ++w) {
+            const float4 q = *reinterpret_cast<const float4 *>(ring + (w * kTileRows + row) * mp + m0);
+            v[j].x += q.x; v[j].y += q.y; v[j].z += q.z; v[j].w += q.w;
           }
         }
-      }
+      };
+      bool ok = mbar_wait(smem_u32(&fl_full[ej][fslot]), fpar);
+      if (ok) add(flush + (ej * fdep + fslot) * gslot_floats);
       __syncwarp();
-      if (lane == 0) {
-#pragma unroll
-        for (int g = 0; g < kGroups; ++g)
-          if ((e >> (11 + g)) & 1) mbar_arrive(smem_u32(&fl_empty[g][ej][fdep == 2 ? ((e >> (14 + 2 * g)) & 1) : 0]));
+      if (lane == 0) mbar_arrive(smem_u32(&fl_empty[ej][fslot]));
+      if (++fslot == fdep) {
+        fslot = 0;
+        fpar ^= 1;
+      }
+      for (int g = ej + 1; g < kGroups; ++g) {  // groups that continue the tile
+        if (third(g) >= ib || third(g) == third(g + 1)) continue;
+        ok = ok && mbar_wait(smem_u32(&fl_cross[g]), 0);
+        if (ok) add(flush + (kGroups * fdep + g - 1) * gslot_floats);
+      }
+      if (!ok) {
+        if (lane == 0) atomicExch(status, 2);
+        return;
       }
       const int b_hi = (starts && !ends) ? b_last : static_cast<int>(blockIdx.x);
-      bool ok = true;
-#pragma unroll 1
-      for (int m = lane >> 4; m < M; m += 2) {
-        float v = vst[row * vp + m];
+#pragma unroll
+      for (int j = 0; j < kItems; ++j) {
+        const int m0 = ((lane >> 4) + 2 * j) * 4;
+        if (m0 >= M) continue;
+        const int nm = min(4, M - m0);
         if (!starts) {
           // continuation of a tile another CTA started: store the partial sums into this
           // CTA's workspace slot (idle words read 0xffffffff); the owner polls them
           // strong store: performed at L2 at once (a plain store may linger in this SM while
           // other warps of this CTA poll for another CTA's sums)
-          asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(ws_row + m), "f"(v) : "memory");
+          if (nm == 4) {
+            asm volatile("st.relaxed.gpu.global.v4.f32 [%0], {%1,%2,%3,%4};" ::"l"(ws_row + m0), "f"(v[j].x), "f"(v[j].y), "f"(v[j].z), "f"(v[j].w) : "memory");
+          } else {
+            asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(ws_row + m0), "f"(v[j].x) : "memory");
+            if (nm > 1) asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(ws_row + m0 + 1), "f"(v[j].y) : "memory");
+            if (nm > 2) asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(ws_row + m0 + 2), "f"(v[j].z) : "memory");
+          }
           continue;
         }
+        // The other CTAs' sums, four activation rows to a load and the next CTA's load in flight
+        // behind the present one: each is a round trip to L2, and for M = 8 one row after the other
+        // they took 4 us of a 10 us launch.
+        const float *pw = a.workspace + 256ll * (blockIdx.x + 1) + row * 16 + m0;
+        uint4 nxt = make_uint4(0u, 0u, 0u, 0u);
+        if (static_cast<int>(blockIdx.x) < b_hi) nxt = ld_relaxed16(pw);
 #pragma unroll 1
-        for (int b = blockIdx.x + 1; b <= b_hi; ++b) {
-          float *pw = a.workspace + 1ll * b * 256 + row * 16 + m;
-          uint32_t bits = 0xffffffffu;
-#pragma unroll 1
-          for (int spin = 0; spin < 2000000 && bits == 0xffffffffu; ++spin) {
-            asm volatile("ld.volatile.global.u32 %0, [%1];" : "=r"(bits) : "l"(pw) : "memory");
-            if (bits == 0xffffffffu) __nanosleep(200);
+        for (int b = blockIdx.x + 1; b <= b_hi; ++b, pw += 256) {
+          uint4 w = nxt;
+          if (b < b_hi) nxt = ld_relaxed16(pw + 256);
+          int spin = 0;
+          while (w.x == kIdle || (nm > 1 && w.y == kIdle) || (nm > 2 && w.z == kIdle) || (nm > 3 && w.w == kIdle)) {
+            if (++spin > 2000000) {
+              ok = false;
+              break;
+            }
+            __nanosleep(100);
+            w = ld_relaxed16(pw);
           }
-          if (bits == 0xffffffffu) ok = false;
-          v += __uint_as_float(bits);
-          *pw = __uint_as_float(0xffffffffu);  // slot idle again
+          v[j].x += __uint_as_float(w.x);
+          v[j].y += __uint_as_float(w.y);
+          v[j].z += __uint_as_float(w.z);
+          v[j].w += __uint_as_float(w.w);
+          *reinterpret_cast<uint4 *>(const_cast<float *>(pw)) = make_uint4(kIdle, kIdle, kIdle, kIdle);  // slot idle again
         }
-        const __half h = __float2half_rn(fmaf(v, scl, bia));
-        if (!EXTRA) {
-          static_cast<__half *>(a.y)[1ll * m * N + col] = h;
-        } else if (a.n_dst == 0) {
-          store_y(a.y, 1ll * m * N + col, fmaf(v, scl, bia), a.y_bf16);
-        } else {
-          // the 16 rows of a tile are consecutive columns of the slice: the stores of the lanes
-          // of one activation row fall into one 32-byte sector per destination
-          for (int d = 0; d < a.n_dst; ++d) a.dst[d][1ll * m * N + col] = h;
+        const float o[4] = {fmaf(v[j].x, cur_scl, cur_bia), fmaf(v[j].y, cur_scl, cur_bia), fmaf(v[j].z, cur_scl, cur_bia),
+                            fmaf(v[j].w, cur_scl, cur_bia)};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (i >= nm) break;
+          const long long at = 1ll * (m0 + i) * N + cur_col;
+          if (!EXTRA) {
+            static_cast<__half *>(a.y)[at] = __float2half_rn(o[i]);
+          } else if (a.n_dst == 0) {
+            store_y(a.y, at, o[i], a.y_bf16);
+          } else {
+            // the 16 rows of a tile are consecutive columns of the slice: the stores of the lanes
+            // of one activation row fall into one 32-byte sector per destination
+            for (int d = 0; d < a.n_dst; ++d) a.dst[d][at] = __float2half_rn(o[i]);
+          }
         }
       }
-      __syncwarp();  // vst is rewritten for the next tile
       if (__any_sync(0xffffffffu, !ok)) {
         if (lane == 0) atomicExch(status, 3);
         return;
       }
+      if (!more) break;
+      ++gt;
+      tile_geom(sc, gt, f, S, fmt);
     }
     if (EXTRA && a.n_dst > 0) {
       // This warp's stores to the other GPUs are complete system-wide before it counts itself
@@ -671,7 +561,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
       __threadfence_system();
       __syncwarp();
       if (lane == 0) {
-        const int expected = static_cast<int>(gridDim.x) * nepi;
+        const int expected = sc.G * kEpiWarps;
         if (atomicAdd(a.peer_state, 1) == expected - 1) {
           __threadfence_system();
           const int launch = a.peer_state[1] + 1;
@@ -699,7 +589,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
   const uint32_t lm_lane = ((lane & 7) + ((lane >> 3) & 1) * 8) * pitch + (lane >> 4) * 16;
   const int spitch = scale_pitch(ck);
   const uint32_t sc_lane = kTileRows * pitch + g * spitch;  // block scales of row g
-  const uint32_t sel = (t & 2) ? 0x3232u : 0x1010u;          // this lane's 8 codes sit in block t >> 1
+  const uint32_t sel = (t & 2) ? 0x7351u : 0x6240u;          // this lane's 8 codes sit in block t >> 1
   const int npair = ck >> 6;                                 // pairs of 16-byte pieces per row
   const int grp = warp / kWarpsPerGroup, wq = warp % kWarpsPerGroup;
 
@@ -711,9 +601,28 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
 #pragma unroll
       for (int i = 0; i < 4; ++i) acc[n][c][i] = 0.f;
 
+  // Split of an activation prologue: a row is cut into `cpr` chunks (a divisor of the twelve warps) of
+  // `per` 16-byte vectors; a warp takes chunk warp % cpr of the rows warp / cpr, + 12 / cpr, ...  Chunks
+  // of up to four vectors per lane, and no more rows at a time than there are.
+  const int nvec = K >> 3;
+  int cpr = 1, per = nvec;
+  if (EXTRA && XS && a.xop != 0) {
+    while (cpr < kMmaWarps && (per > 128 || kMmaWarps / cpr > M)) {
+      cpr = cpr == 4 ? 6 : (cpr == 6 ? 12 : cpr + 1);
+      per = (nvec + cpr - 1) / cpr;
+    }
+  }
+  const int vlo = (warp % cpr) * per, vhi = min(nvec, vlo + per), rows_at_once = kMmaWarps / cpr;
+  if (EXTRA && XS && a.xop == 1 && a.early) {
+    // the norm's weights are constants: into L1 while the kernel before this one still runs
+    for (int i = vlo + lane; i < vhi; i += 32) {
+      const uint4 v = ldg_nc16(a.x_weight + 8 * i);
+      asm volatile("" ::"r"(v.x));
+    }
+  }
+
   // x is produced by the preceding kernel: do not touch it before the producer thread has
   // seen that kernel complete (and, with XS, has copied the rows into shared memory).
-  // The stage list is complete by then, too.
   if (!mbar_wait(smem_u32(&bar_x), 0)) {
     if (lane == 0) atomicExch(status, 6);
     return;
@@ -723,31 +632,26 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
     // memory from what the preceding kernels left in global memory (every CTA does the same work:
     // a few KB out of L2).  A row is cut into `cpr` chunks, one warp per chunk, and a lane has
     // four vectors (eight with x_aux) in flight: the cost is a few L2 round trips.
-    const int nvec = K >> 3;  // 16-byte vectors per row
-    const int cpr = M >= kMmaWarps ? 1 : kMmaWarps / M;
-    const int per = (nvec + cpr - 1) / cpr;
     if (a.xop == 1) {
-      for (int u = warp; u < M * cpr; u += kMmaWarps) {
-        const int m = u / cpr, c = u - m * cpr;
-        const int hi = min(nvec, (c + 1) * per);
+      for (int m = warp / cpr; m < M; m += rows_at_once) {
         const __half *xr = a.x + 1ll * m * K;
         const __half *dr = a.x_aux ? a.x_aux + 1ll * m * K : nullptr;
         __half *orow = (a.x_out && blockIdx.x == 0) ? a.x_out + 1ll * m * K : nullptr;
         float ss = 0.f;
-        for (int i0 = c * per + lane; i0 < hi; i0 += 128) {
+        for (int i0 = vlo + lane; i0 < vhi; i0 += 128) {
           uint4 v[4], d[4];
 #pragma unroll
           for (int q = 0; q < 4; ++q)
-            if (i0 + 32 * q < hi) v[q] = ldg_cg16(xr + 8 * (i0 + 32 * q));
+            if (i0 + 32 * q < vhi) v[q] = ldg_cg16(xr + 8 * (i0 + 32 * q));
           if (dr) {
 #pragma unroll
             for (int q = 0; q < 4; ++q)
-              if (i0 + 32 * q < hi) d[q] = ldg_cg16(dr + 8 * (i0 + 32 * q));
+              if (i0 + 32 * q < vhi) d[q] = ldg_cg16(dr + 8 * (i0 + 32 * q));
           }
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             const int i = i0 + 32 * q;
-            if (i >= hi) break;
+            if (i >= vhi) break;
             __half2 *hv = reinterpret_cast<__half2 *>(&v[q]);
             if (dr) {
               const __half2 *dh = reinterpret_cast<const __half2 *>(&d[q]);
@@ -764,64 +668,68 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
           }
         }
         ss = warp_sum(ss);
-        if (lane == 0) xred[m][c] = ss;
+        if (lane == 0) xred[m][warp % cpr] = ss;
       }
       asm volatile("bar.sync 2, %0;" ::"r"(kMmaWarps * 32) : "memory");
-      for (int u = warp; u < M * cpr; u += kMmaWarps) {
-        const int m = u / cpr, c = u - m * cpr;
-        const int hi = min(nvec, (c + 1) * per);
+      for (int m = warp / cpr; m < M; m += rows_at_once) {
         float ss = 0.f;
         for (int w = 0; w < cpr; ++w) ss += xred[m][w];
         const float rs = rsqrtf(ss / K + a.x_eps);
-        for (int i = c * per + lane; i < hi; i += 32) {
-          uint4 v = *reinterpret_cast<uint4 *>(xsm + m * xpitch + 16 * i);
-          const uint4 wv = *reinterpret_cast<const uint4 *>(a.x_weight + 8 * i);
-          __half2 *hv = reinterpret_cast<__half2 *>(&v);
-          const __half2 *wh = reinterpret_cast<const __half2 *>(&wv);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float2 f = __half22float2(hv[j]);
-            hv[j] = __hmul2(__floats2half2_rn(f.x * rs, f.y * rs), wh[j]);
-          }
-          *reinterpret_cast<uint4 *>(xsm + m * xpitch + 16 * i) = v;
-        }
-      }
-    } else if (a.xop == 3) {
-      for (int u = warp; u < M * cpr; u += kMmaWarps) {
-        const int m = u / cpr, c = u - m * cpr;
-        const int hi = min(nvec, (c + 1) * per);
-        const __half *xr = a.x + 1ll * m * K;
-        for (int i0 = c * per + lane; i0 < hi; i0 += 128) {
-          uint4 v[4];
+        for (int i0 = vlo + lane; i0 < vhi; i0 += 128) {
+          uint4 v[4], wv[4];
 #pragma unroll
           for (int q = 0; q < 4; ++q)
-            if (i0 + 32 * q < hi) v[q] = ldg_cg16(xr + 8 * (i0 + 32 * q));
+            if (i0 + 32 * q < vhi) {
+              wv[q] = ldg_nc16(a.x_weight + 8 * (i0 + 32 * q));
+              v[q] = *reinterpret_cast<uint4 *>(xsm + m * xpitch + 16 * (i0 + 32 * q));
+            }
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             const int i = i0 + 32 * q;
-            if (i >= hi) break;
+            if (i >= vhi) break;
+            __half2 *hv = reinterpret_cast<__half2 *>(&v[q]);
+            const __half2 *wh = reinterpret_cast<const __half2 *>(&wv[q]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float2 f = __half22float2(hv[j]);
+              hv[j] = __hmul2(__floats2half2_rn(f.x * rs, f.y * rs), wh[j]);
+            }
+            *reinterpret_cast<uint4 *>(xsm + m * xpitch + 16 * i) = v[q];
+          }
+        }
+      }
+    } else if (a.xop == 3) {
+      for (int m = warp / cpr; m < M; m += rows_at_once) {
+        const __half *xr = a.x + 1ll * m * K;
+        for (int i0 = vlo + lane; i0 < vhi; i0 += 128) {
+          uint4 v[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (i0 + 32 * q < vhi) v[q] = ldg_cg16(xr + 8 * (i0 + 32 * q));
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int i = i0 + 32 * q;
+            if (i >= vhi) break;
             *reinterpret_cast<uint4 *>(xsm + m * xpitch + 16 * i) =
                 make_uint4(bf16x2_to_f16x2(v[q].x), bf16x2_to_f16x2(v[q].y), bf16x2_to_f16x2(v[q].z), bf16x2_to_f16x2(v[q].w));
           }
         }
       }
     } else {
-      for (int u = warp; u < M * cpr; u += kMmaWarps) {
-        const int m = u / cpr, c = u - m * cpr;
-        const int hi = min(nvec, (c + 1) * per);
+      for (int m = warp / cpr; m < M; m += rows_at_once) {
         const __half *gr = a.x + 2ll * m * K;
-        for (int i0 = c * per + lane; i0 < hi; i0 += 128) {
+        for (int i0 = vlo + lane; i0 < vhi; i0 += 128) {
           uint4 gv[4], uv[4];
 #pragma unroll
           for (int q = 0; q < 4; ++q)
-            if (i0 + 32 * q < hi) {
+            if (i0 + 32 * q < vhi) {
               gv[q] = ldg_cg16(gr + 8 * (i0 + 32 * q));
               uv[q] = ldg_cg16(gr + K + 8 * (i0 + 32 * q));
             }
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             const int i = i0 + 32 * q;
-            if (i >= hi) break;
+            if (i >= vhi) break;
             const __half2 *gh = reinterpret_cast<const __half2 *>(&gv[q]);
             const __half2 *uh = reinterpret_cast<const __half2 *>(&uv[q]);
             uint4 o;
@@ -829,8 +737,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               const float2 g2 = __half22float2(gh[j]);
-              const __half2 sl = __floats2half2_rn(g2.x / (1.f + __expf(-g2.x)), g2.y / (1.f + __expf(-g2.y)));
-              oh[j] = __hmul2(sl, uh[j]);
+              oh[j] = __hmul2(__floats2half2_rn(silu(g2.x), silu(g2.y)), uh[j]);
             }
             *reinterpret_cast<uint4 *>(xsm + m * xpitch + 16 * i) = o;
           }
@@ -848,26 +755,26 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
                : reinterpret_cast<uint64_t>(a.x + 1ll * (m < M ? m : 0) * K);
   }
 
-  // Stage it sits in ring slot it % nst and goes to warp group slot % kGroups: a slot always
-  // belongs to the same group, which therefore follows its barriers phase by phase whatever the
-  // ring depth (a group that tested a barrier it had not followed could see a stale phase
-  // parity, read the slot early and arrive twice on its empty barrier).
-  float *fl_base = flush + grp * nepi * fdep * gslot_floats + wq * kTileRows * mp;
-  int slot = grp, round = 0;
-  int fcnt = 0;  // hand-overs made so far to each epilogue warp: 10 bits each
-  int turn = 0;  // stages this group has taken: rotates the pair ranges among its warps
+  const int g_begin = third(grp), g_end = third(grp + 1);
+  if (g_begin == g_end) return;
+  int gt = sc.tile_of_image(g_begin), f, S, fmt;
+  tile_geom(sc, gt, f, S, fmt);
+  int c = g_begin - f;  // image of its tile
+  // sums of a tile that an earlier group started go to that group's epilogue warp
+  bool cross = f < g_begin && g_begin > s_begin;
+  float *fl_own = flush + grp * fdep * gslot_floats + wq * kTileRows * mp;
+  int slot = grp, par = 0;        // ring slot and parity of its phase
+  int fslot = 0, fpar = 1;        // hand-over slot and parity of the phase in which it was given back
+  int turn = wq;
 #pragma unroll 1
-  for (int it = grp; it < nimg; ++turn) {
-    const uint32_t e = list[it];
-    if (!mbar_wait(smem_u32(&bar_full[slot]), round & 1)) {
+  for (int left = g_end - g_begin; left > 0; --left) {
+    if (!mbar_wait(smem_u32(&bar_full[slot]), par)) {
       if (lane == 0) atomicExch(status, 4);
       return;
     }
     const uint32_t sbase = smem_base + slot * a.slot_bytes;
-    const int c = (e >> 3) & 255;
-    const int fmt = e & 3;
     // inside a group the warps take turns on the pair ranges, so uneven splits average out
-    const int lw = (wq + turn) & (kWarpsPerGroup - 1);
+    const int lw = turn++ & (kWarpsPerGroup - 1);
     const int lo = lw * npair / kWarpsPerGroup, hi = (lw + 1) * npair / kWarpsPerGroup;
     if (fmt == 0) {
       stage_fp4<NT, XS>(acc, sbase + lm_lane + lo * 32, sbase + sc_lane + lo * 4, sbase + sc_lane + 8 * spitch + lo * 4,
@@ -879,40 +786,43 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(&bar_empty[slot]));
-    if (slot + kGroups < nst) {
-      slot += kGroups;
-      it += kGroups;
-    } else {  // on to the group's first slot, one round later
-      it += nst - slot + grp;
+    slot += kGroups;
+    if (slot >= nst) {
       slot = grp;
-      ++round;
+      par ^= 1;
     }
+    if (++c < S && left > 1) continue;
 
-    if (e & kEntFlush) {
-      // ---- the group's last stage of this tile: hand the partial sums to the tile's epilogue
-      // warp, through the ring the two share
-      const int ej = (e >> 11) & 3;
-      const int cnt = (fcnt >> (10 * ej)) & 1023;
-      fcnt += 1 << (10 * ej);
-      const int fslot = (fdep == 2) ? (cnt & 1) : 0, fround = (fdep == 2) ? (cnt >> 1) : cnt;
-      if (fround > 0 && !mbar_wait(smem_u32(&fl_empty[grp][ej][fslot]), (fround - 1) & 1)) {
-        if (lane == 0) atomicExch(status, 5);
-        return;
-      }
-      float *buf = fl_base + (ej * fdep + fslot) * gslot_floats;
+    // ---- the group's last image of this tile: hand the partial sums to the epilogue warp
+    float *buf = cross ? flush + (kGroups * fdep + grp - 1) * gslot_floats + wq * kTileRows * mp
+                       : fl_own + fslot * gslot_floats;
+    // (a fresh barrier passes for the parity of the phase before its first)
+    if (!cross && !mbar_wait(smem_u32(&fl_empty[grp][fslot]), fpar)) {
+      if (lane == 0) atomicExch(status, 5);
+      return;
+    }
 #pragma unroll
-      for (int n = 0; n < NT; ++n) {
+    for (int n = 0; n < NT; ++n) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int r = g + (i >> 1) * 8;
-          const int m = n * 8 + 2 * t + (i & 1);
-          if (m < M) buf[r * mp + m] = acc[n][0][i] + acc[n][1][i];
-          acc[n][0][i] = 0.f;
-          acc[n][1][i] = 0.f;
-        }
+      for (int i = 0; i < 4; ++i) {
+        const int r = g + (i >> 1) * 8;
+        const int m = n * 8 + 2 * t + (i & 1);
+        if (m < M) buf[r * mp + m] = acc[n][0][i] + acc[n][1][i];
+        acc[n][0][i] = 0.f;
+        acc[n][1][i] = 0.f;
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&fl_full[grp][ej][fslot]));
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_u32(cross ? &fl_cross[grp] : &fl_full[grp][fslot]));
+    if (!cross && ++fslot == fdep) {
+      fslot = 0;
+      fpar ^= 1;
+    }
+    cross = false;
+    if (c == S && left > 1) {
+      ++gt;
+      tile_geom(sc, gt, f, S, fmt);
+      c = 0;
     }
   }
 }
@@ -929,22 +839,21 @@ void gemv_tiled_scratch(size_t *workspace_bytes, size_t *flag_bytes) {
 // Shared-memory plan of one launch: weight ring | flush ring | output metadata | activations (if
 // they fit).
 struct SmemPlan {
-  int nepi, fdep, nst, smem;
+  int fdep, nst, smem;
   bool xs;
 };
-static SmemPlan smem_plan(int M, int K) {
+static SmemPlan smem_plan(int M, int K, bool shared) {
   SmemPlan p;
   const int slot_bytes = (img_bytes(0, tiled_chunk_k(K)) + 127) & ~127;
-  // hand-over rings: (3 groups x nepi epilogue warps) x kFlushRing slots of 4 warps x 16 rows x
-  // (M rounded up to 4) partial sums; fewer epilogue warps for large M keep this at 18-24 KB
-  // up to four activation rows: 3 epilogue warps, 2-slot rings (18 KB at most); up to eight:
-  // 3 warps, 1-slot rings (18 KB); beyond: 2 warps, 1-slot rings (24 KB)
-  p.nepi = M <= 8 ? kEpiWarps : 2;
-  p.fdep = M <= 4 ? kFlushRing : 1;
-  const int mp = (M <= 3) ? M : ((M + 3) & ~3);
-  const int fl_bytes = kGroups * p.nepi * p.fdep * kWarpsPerGroup * kTileRows * mp * 4;
-  const int fixed = fl_bytes + kMetaSegs * kTileRows * 12 + kMaxList * 8 + kEpiWarps * kTileRows * (M <= 4 ? 4 : 16) * 4;
-  const int total_budget = 112 * 1024;  // two CTAs (this layer's and the next one's) share an SM's 228 KB
+  // hand-over slots of 4 warps x 16 rows x (M rounded up to 4) partial sums (1 - 4 KB): two per group
+  // up to eight activation rows, then one, and one for each later group's part of a shared tile
+  p.fdep = M <= 8 ? kFlushRing : 1;
+  const int fixed = (kGroups * p.fdep + kGroups - 1) * kWarpsPerGroup * kTileRows * ((M + 3) & ~3) * 4;
+  // Where weights may be read early, two CTAs (this layer's and the next one's) share an SM's 228 KB:
+  // 1 KB each is reserved, static 1.3 KB.  Where they may not, the next one could do nothing before
+  // this one ends, and a launch that comes while this one drains would get two places on the SMs
+  // that are empty already: seven projections of a block called one by one, 62.0 -> 53.8 us.
+  const int total_budget = (shared ? 228 * 1024 / 2 : 228 * 1024) - 1024 - 1408;
   int xbytes = M * (2 * K + 16);
   p.xs = true;
   // Ring depth: slot s belongs to warp group s % 3, so depths 3k and 3k + 2 split the slots
@@ -963,21 +872,21 @@ static SmemPlan smem_plan(int M, int K) {
   }
   p.nst = depth(xbytes);
   if (p.nst < kGroups) p.nst = kGroups;  // 3 x 19 KB always fits beside the fixed part
-  p.smem = p.nst * slot_bytes + fixed + xbytes;
+  p.smem = max(p.nst * slot_bytes + fixed + xbytes, shared ? kSlotSmem : kAloneSmem);
   return p;
 }
-bool tiled_stages_x(int M, int K) { return M >= 1 && M <= RDQ_MAX_GEMV_M && smem_plan(M, K).xs; }
+bool tiled_stages_x(int M, int K) { return M >= 1 && M <= RDQ_MAX_GEMV_M && smem_plan(M, K, true).xs; }
 
 // Schedule and shared-memory plan of a (shape, rows) pair.
 struct TiledPlan {
   TSched sc;
   SmemPlan pl;
 };
-static TiledPlan make_tiled_plan(int n4, int n8, int n16, int K, int M) {
+static TiledPlan make_tiled_plan(int n4, int n8, int n16, int K, int M, bool shared) {
   TiledPlan p;
   TSched &sc = p.sc;
-  p.pl = smem_plan(M, K);
-  const int nst = p.pl.nst;
+  p.pl = smem_plan(M, K, shared);
+  const int nst = smem_plan(M, K, true).nst;  // in either case: results do not depend on the flag
   const int ck = tiled_chunk_k(K);
   sc.ck = ck;
   sc.S4 = K / ck;
@@ -995,6 +904,7 @@ static TiledPlan make_tiled_plan(int n4, int n8, int n16, int K, int M) {
   // Images are balanced by what they cost a CTA in time, not by their bytes: an NVFP4 image
   // (conversion + block scaling) takes more instructions than an FP8 or FP16 image of the
   // same size, but images beyond the ring's depth mostly cost the wait for their copy.
+  int u4, u8, u16;  // scheduling cost of one NVFP4 / FP8 / FP16 image
   {
     // Time model of a CTA that streams n images of one format (cycles, three warp groups):
     // the first nst images are in the ring when the kernel may start and cost their compute
@@ -1021,33 +931,38 @@ static TiledPlan make_tiled_plan(int n4, int n8, int n16, int K, int M) {
       if (ctas > sm_count()) lo = T; else hi = T;
     }
     const double n4 = n_of(0, hi), n8 = n_of(1, hi), n16 = n_of(2, hi);
-    sc.u4 = 1000;
-    sc.u8 = max(1, min(1000, static_cast<int>(1000.0 * n4 / n8 + 0.5)));
-    sc.u16 = max(1, min(sc.u8, static_cast<int>(1000.0 * n4 / n16 + 0.5)));
+    u4 = 1000;
+    u8 = max(1, min(1000, static_cast<int>(1000.0 * n4 / n8 + 0.5)));
+    u16 = max(1, min(u8, static_cast<int>(1000.0 * n4 / n16 + 0.5)));
   }
-  sc.w4 = 1ll * sc.e4 * sc.u4;
-  sc.w8 = sc.w4 + 1ll * (sc.e8 - sc.e4) * sc.u8;
-  sc.W = sc.w8 + 1ll * (sc.e16 - sc.e8) * sc.u16;
+  const long long w4 = 1ll * sc.e4 * u4, w8 = w4 + 1ll * (sc.e8 - sc.e4) * u8, W = w8 + 1ll * (sc.e16 - sc.e8) * u16;
   // every CTA must own at least one image: its share may not be shorter than the
   // heaviest image
-  int G = sm_count();
+  int G = min(sm_count(), kMaxCtas);
   // ... and a tile may spread over at most 31 CTAs (the owner finds them with one ballot)
-  long long minshare = sc.u4;  // u4 is the largest cost
-  const long long tile_cost[3] = {1ll * sc.S4 * sc.u4, 1ll * sc.S8 * sc.u8, 1ll * sc.S16 * sc.u16};
+  long long minshare = u4;  // u4 is the largest cost
+  const long long tile_cost[3] = {1ll * sc.S4 * u4, 1ll * sc.S8 * u8, 1ll * sc.S16 * u16};
   for (int f = 0; f < 3; ++f)
     if ((tile_cost[f] + 29) / 30 > minshare) minshare = (tile_cost[f] + 29) / 30;
-  const long long maxg = sc.W / minshare;
+  const long long maxg = W / minshare;
   if (maxg < G) G = static_cast<int>(maxg);
   if (G < 1) G = 1;
   sc.G = G;
+  for (int b = 0; b <= G; ++b) {
+    const long long pos = W * b / G;
+    sc.bound[b] = b == G ? sc.e16
+                  : pos < w4 ? static_cast<int>(pos / u4)
+                  : pos < w8 ? sc.e4 + static_cast<int>((pos - w4) / u8)
+                             : sc.e8 + static_cast<int>((pos - w8) / u16);
+  }
   return p;
 }
 // The plans this thread has used (a decode step calls the same few layers again and again; the time
 // model above costs about as much host time as the launch itself).
-static const TiledPlan &tiled_plan(int n4, int n8, int n16, int K, int M) {
+static const TiledPlan &tiled_plan(int n4, int n8, int n16, int K, int M, bool shared) {
   struct Key {
-    int v[6];
-    bool operator==(const Key &o) const { return std::equal(v, v + 6, o.v); }
+    int v[7];
+    bool operator==(const Key &o) const { return std::equal(v, v + 7, o.v); }
   };
   struct Hash {
     size_t operator()(const Key &k) const {
@@ -1057,20 +972,19 @@ static const TiledPlan &tiled_plan(int n4, int n8, int n16, int K, int M) {
     }
   };
   static thread_local std::unordered_map<Key, TiledPlan, Hash> plans;
-  const Key key{{n4, n8, n16, K, M, sm_count()}};
+  const Key key{{n4, n8, n16, K, M, shared, sm_count()}};
   auto it = plans.find(key);
   if (it == plans.end()) {
     if (plans.size() >= 4096) plans.clear();
-    it = plans.emplace(key, make_tiled_plan(n4, n8, n16, K, M)).first;
+    it = plans.emplace(key, make_tiled_plan(n4, n8, n16, K, M, shared)).first;
   }
   return it->second;
 }
 
 int launch_gemv_tiled(const GemvTiledArgs &h, bool pdl, cudaStream_t stream) {
-  const TiledPlan &plan = tiled_plan(h.n4, h.n8, h.n16, h.K, h.M);
+  const TiledPlan &plan = tiled_plan(h.n4, h.n8, h.n16, h.K, h.M, pdl);
   const TSched &sc = plan.sc;
   const SmemPlan &pl = plan.pl;
-  const int G = sc.G;
   TiledArgs a;
   a.x = static_cast<const __half *>(h.x); a.y_bf16 = h.y_bf16; a.M = h.M; a.tiled = h.tiled; a.s8 = h.s8; a.global4 = h.global4; a.perm = h.perm;
   a.bias = h.bias; a.y = h.y; a.n4 = h.n4; a.n8 = h.n8; a.n16 = h.n16; a.K = h.K;
@@ -1087,17 +1001,15 @@ int launch_gemv_tiled(const GemvTiledArgs &h, bool pdl, cudaStream_t stream) {
   a.status_idx = sm_count();
   a.slot_bytes = (img_bytes(0, sc.ck) + 127) & ~127;
   const int nt = h.M <= 8 ? 1 : 2;
-  a.nepi = pl.nepi;
   a.fdepth = pl.fdep;
   a.nstages = pl.nst;
   const bool xs = pl.xs;
+  RDQ_REQUIRE((reinterpret_cast<uintptr_t>(h.workspace) & 15) == 0, RDQ_E_INVALID, "GEMV workspace must be 16-byte aligned");
   RDQ_REQUIRE(a.xop == 0 || xs, RDQ_E_UNSUPPORTED,
               "activation prologue needs the activation rows in shared memory (M=%d, K=%d)", h.M, h.K);
   RDQ_REQUIRE(h.xop == 0 || (h.xop == 1 && h.x_weight) || h.xop == 2, RDQ_E_INVALID, "bad activation prologue");
   const int smem = pl.smem;
 
-  RDQ_REQUIRE(sc.W / G / sc.u16 + 2 <= kMaxList, RDQ_E_UNSUPPORTED,
-              "layer too large for the tiled GEMV: more than %d images per CTA", kMaxList);
 
   static int smem_set[64][8] = {};
   static std::mutex smem_mutex;
@@ -1126,7 +1038,7 @@ int launch_gemv_tiled(const GemvTiledArgs &h, bool pdl, cudaStream_t stream) {
   }
 
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(G));
+  cfg.gridDim = dim3(static_cast<unsigned>(sm_count()));
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;

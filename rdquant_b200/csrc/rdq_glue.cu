@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const __half *gu, __half 
     for (int t = 0; t < 4; ++t) {
       const float2 a = __half22float2(gh[t]), c = __half22float2(uh[t]);
       // silu in FP32, rounded to FP16 before the product like the framework's two kernels
-      const __half2 s = __floats2half2_rn(a.x / (1.f + __expf(-a.x)), a.y / (1.f + __expf(-a.y)));
+      const __half2 s = __floats2half2_rn(silu(a.x), silu(a.y));
       oh[t] = __hmul2(s, __floats2half2_rn(c.x, c.y));
     }
     reinterpret_cast<uint4 *>(out + 1ll * b * F)[j] = o;

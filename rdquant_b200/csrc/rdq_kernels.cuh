@@ -135,10 +135,11 @@ int launch_add_rmsnorm(__half *x, const __half *delta, const __half *w, __half *
 int launch_qk_rope_cache(const __half *qkv, const __half *qn, const __half *kn, const __half *cos_t, const __half *sin_t,
                          const long long *pos, __half *q_out, __half *k_cache, __half *v_cache, int B, int nq, int nkv,
                          int dh, int S, float eps, bool pdl, cudaStream_t stream);
-// Kernels that sit between two GEMVs of a decode step are launched with one CTA per SM and this
-// much (unused) dynamic shared memory: next to a GEMV's CTA (<= 112 KB + static) an SM then has
-// room for one of their CTAs, not two.
-constexpr int kSlotSmem = 60 * 1024;
+// The GEMVs of a decode step and the kernels between them are launched with one CTA per SM and at
+// least this much dynamic shared memory, so that an SM has room for two of their CTAs whichever they
+// are.  With a third place on some SMs (kernels of 60 KB, GEMVs of 93 KB) two CTAs of a launch landed
+// there, a later GEMV found 107 of 148 SMs and its doubled CTAs took 6 us longer than the others.
+constexpr int kSlotSmem = 100 * 1024;
 cudaError_t pin_slot(const void *fn, int smem);
 int attn_chunk();
 // q/k norm + rotary + cache write + attention + merge of the splits in one launch
