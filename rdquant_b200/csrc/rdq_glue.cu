@@ -251,15 +251,20 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const __half *gu, __half 
 //   3. tensor-core products (mma.sync m16n8k16, FP32 sums) with cache rows as the row operand and up to
 //      eight query heads as columns: S^T = K Q^T, online softmax per block, O^T += V^T P^T.  P goes in
 //      as the sum of two FP16 values, so that its rounding (2^-22) stays below FP32 products' sums.
-//   4. the warps' (max, sum, values) are merged in shared memory; with one split that is the result,
-//      else the partial goes to scratch and the last CTA of a (sequence, KV head) to arrive (counter
-//      in scratch, left at zero again) merges the splits and writes out [B, nq * dh].
+//   4. the warps' (max, sum, values) are merged in shared memory; with one split that is the result.
+//      Else every CTA stores its partial sums in scratch, and CTA `split` of a (sequence, KV head) merges
+//      the query heads split, split + splits, ...: it polls the words it needs until they differ from
+//      zero (a sum that is zero is stored as -0), adds them in split order and puts zeros back, so that
+//      the scratch is idle again when the launch ends.  The last CTA to arrive merging all heads, behind
+//      a fence and a counter, took 4 us of a 9.5 us launch (one sequence of 512 rows).
+// Under programmatic launch the norm weights, the rotary rows and the cache rows are asked into L2 while
+// the kernel before this one runs (a position that is out of date costs no more than the hint).
 // Bound: HBM (K and V rows once) for many sequences, latency for one.  The scalar kernel before (a
 // lane per row, every query head converting the K rows again) took 44 us for 32 sequences of 700 rows
 // (92 MB).
 constexpr int kFusedAttnWarps = 4;
 constexpr int kFusedAttnThreads = kFusedAttnWarps * 32;
-constexpr int kFusedAttnMaxSplit = 16;  // one batch of merge loads at head_dim <= 128
+constexpr int kFusedAttnMaxSplit = 16;  // values a thread of the merge has in flight
 
 // 16 bytes, or zeros
 __device__ __forceinline__ void cp_async16_if(uint32_t dst, const void *src, bool valid) {
@@ -282,33 +287,63 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t v) {
   return r;
 }
 
+// a partial sum as a word that differs from an idle word
+__device__ __forceinline__ float not_idle(float v) { return __float_as_uint(v) == 0u ? -0.f : v; }
+__device__ __forceinline__ float ld_relaxed(const float *p) {
+  float v;
+  asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_relaxed(float *p, float v) {
+  asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
+}
+__device__ __forceinline__ bool is_idle(float v) { return __float_as_uint(v) == 0u; }
+__device__ __forceinline__ void prefetch_l2(const void *p, int bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
 // NB: blocks of eight query heads per KV head
 template <int DH, int NB>
 __global__ void __launch_bounds__(kFusedAttnThreads, 2) rope_attn_kernel(
     const __half *qkv, const __half *qn, const __half *kn, const __half *cos_t, const __half *sin_t, const long long *pos,
-    __half *k_cache, __half *v_cache, float *part, int *counters, __half *out, int nq, int nkv, int S, float scale,
-    float eps, int nsplit, int npair) {
+    __half *k_cache, __half *v_cache, float *part, __half *out, int nq, int nkv, int S, float scale, float eps, int nsplit,
+    int npair) {
   constexpr int W = kFusedAttnWarps;
   constexpr int PITCH = 2 * DH + 16;   // row pitch in shared memory (bytes): an odd multiple of 16
   constexpr int BLK = 16 * PITCH;      // 16 rows of K or of V
   constexpr int QP = DH + 8;           // query row pitch (halves)
   constexpr int HALF = DH / 2;
-  constexpr int DPL = DH / 32;         // dimensions per lane in the merge
+  constexpr int DPL = DH / 32;         // dimensions per lane in the merge of the warps
   constexpr int VPR = DH / 8;          // 16-byte vectors per row
   constexpr int KS = DH / 16;          // k steps of S, row blocks of O
   constexpr int PR = DH + 4;  // a partial: max, sum, two unused, then the DH weighted values (16-byte aligned)
   extern __shared__ __align__(16) uint8_t smem[];
   __half *qs = reinterpret_cast<__half *>(smem + W * 4 * BLK);  // [8 NB][QP]
   float *mrg = reinterpret_cast<float *>(smem);                 // [W][8 NB][PR], over the rings once they are done
-  __shared__ int s_last;
 
   pdl_launch_dependents();
-  pdl_wait();
   // The grid has one CTA per SM (or one per (sequence, KV head) when those outnumber the SMs); CTAs
   // beyond the work linger.
   const int pair = static_cast<int>(blockIdx.x) / nsplit, split = static_cast<int>(blockIdx.x) - pair * nsplit;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
+  if (tid == 0 && pair < npair) {
+    const long long p = *static_cast<const volatile long long *>(pos);
+    // (more rows than a quarter of L2 would only displace one another and the next layers' weights)
+    if (p >= 0 && p < S && 4ll * npair * p * DH <= (32ll << 20)) {
+      const int rows = static_cast<int>(p) / nsplit + 1, r0 = split * rows, r1 = min(static_cast<int>(p), r0 + rows);
+      const long long off = (1ll * pair * S + r0) * DH;  // pair = sequence x KV heads + KV head
+      if (r0 < r1) {
+        prefetch_l2(k_cache + off, (r1 - r0) * DH * 2);
+        prefetch_l2(v_cache + off, (r1 - r0) * DH * 2);
+      }
+      prefetch_l2(cos_t + p * DH, DH * 2);
+      prefetch_l2(sin_t + p * DH, DH * 2);
+    }
+    if (qn) prefetch_l2(qn, DH * 2);
+    if (kn) prefetch_l2(kn, DH * 2);
+  }
+  pdl_wait();
   if (pair >= npair) {
     linger(4000);
     return;
@@ -566,73 +601,54 @@ __global__ void __launch_bounds__(kFusedAttnThreads, 2) rope_attn_kernel(
     } else {
       float *dst = part + ((1ll * b * nq + head) * nsplit + split) * PR;
       if (lane == 0) {
-        dst[0] = m;
-        dst[1] = l;
+        st_relaxed(dst, not_idle(m));
+        st_relaxed(dst + 1, not_idle(l));
       }
 #pragma unroll
-      for (int j = 0; j < DPL; ++j) dst[4 + lane * DPL + j] = a[j];
+      for (int j = 0; j < DPL; ++j) st_relaxed(dst + 4 + lane * DPL + j, not_idle(a[j]));
     }
   }
   if (used == 1) return;
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) {
-    const int old = atomicAdd(&counters[b * nkv + kvh], 1);
-    s_last = (old == used - 1);
-    if (s_last) counters[b * nkv + kvh] = 0;  // ready for the next launch
-  }
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  // The merging CTA reads `used` partials per head out of L2.  All loads of a batch of splits are
-  // issued before any is used (the first batch together with the (max, sum) pairs): two or three
-  // round trips per head instead of one per split.
-  constexpr int BATCH = 64 / DPL;  // splits per batch: 64 value registers per lane
-  for (int hq = warp; hq < group; hq += W) {
+  for (int hq = split; hq < group; hq += used) {
     const int head = kvh * group + hq;
-    const float *src = part + (1ll * b * nq + head) * nsplit * PR;
-    float a[DPL];
+    float *src = part + (1ll * b * nq + head) * nsplit * PR;
+    // lane s: the (max, sum) of split s; thread: dimension tid (+ 128) of every split.  All loads first.
+    float ms = lane < used ? 0.f : -INFINITY, ls = 0.f;
+    for (int d = tid; d < ((DH + 127) & ~127); d += kFusedAttnThreads) {
+      const float *pv = src + 4 + d;
+      float v[kFusedAttnMaxSplit];
 #pragma unroll
-    for (int j = 0; j < DPL; ++j) a[j] = 0.f;
-    float m = 0.f, l = 0.f, w = 0.f;
-    for (int s0 = 0; s0 < used; s0 += BATCH) {
-      float v[BATCH][DPL];
+      for (int q = 0; q < kFusedAttnMaxSplit; ++q) v[q] = 0.f;
+      for (int spin = 0; spin < 1000000; ++spin) {  // (a word that does not come makes the result NaN)
+        if (lane < used && is_idle(ms)) ms = ld_relaxed(src + lane * PR);
+        if (lane < used && is_idle(ls)) ls = ld_relaxed(src + lane * PR + 1);
 #pragma unroll
-      for (int q = 0; q < BATCH; ++q) {
-        if (s0 + q < used) {
-          const float *pv = src + (s0 + q) * PR + 4 + lane * DPL;
-          if (DPL == 4) {
-            const float4 t = __ldcg(reinterpret_cast<const float4 *>(pv));
-            v[q][0] = t.x; v[q][1] = t.y; v[q][2] = t.z; v[q][3] = t.w;
-          } else {
+        for (int q = 0; q < kFusedAttnMaxSplit; ++q)
+          if (q < used && d < DH && is_idle(v[q])) v[q] = ld_relaxed(pv + q * PR);
+        bool idle = lane < used && (is_idle(ms) || is_idle(ls));
 #pragma unroll
-            for (int j = 0; j < DPL; j += 2) {
-              const float2 t = __ldcg(reinterpret_cast<const float2 *>(pv + j));
-              v[q][j] = t.x; v[q][j + 1] = t.y;
-            }
+        for (int q = 0; q < kFusedAttnMaxSplit; ++q) idle = idle || (q < used && d < DH && is_idle(v[q]));
+        if (!__any_sync(0xffffffffu, idle)) break;
+        __nanosleep(20);
+      }
+      const float m = warp_max(ms);
+      const float w = lane < used ? __expf(ms - m) : 0.f;
+      const float l = warp_sum(ls * w);
+      float a = 0.f;
+#pragma unroll
+      for (int q = 0; q < kFusedAttnMaxSplit; ++q) {
+        if (q < used) {
+          const float ws = __shfl_sync(0xffffffffu, w, q);
+          if (d < DH) {
+            a += is_idle(v[q]) ? NAN : ws * v[q];
+            src[q * PR + 4 + d] = 0.f;
           }
         }
       }
-      if (s0 == 0) {  // lane s holds split s's (max, sum); nsplit <= 32
-        const float ms = lane < used ? __ldcg(src + lane * PR) : -INFINITY;
-        const float ls = lane < used ? __ldcg(src + lane * PR + 1) : 0.f;
-        m = warp_max(ms);
-        w = lane < used ? __expf(ms - m) : 0.f;
-        l = warp_sum(ls * w);
-      }
-#pragma unroll
-      for (int q = 0; q < BATCH; ++q) {
-        if (s0 + q < used) {
-          const float ws = __shfl_sync(0xffffffffu, w, s0 + q);
-#pragma unroll
-          for (int j = 0; j < DPL; ++j) a[j] += ws * v[q][j];
-        }
-      }
+      if (d < DH) out[(1ll * b * nq + head) * DH + d] = __float2half_rn(a * (1.f / l));
     }
-    __half *o = out + (1ll * b * nq + head) * DH + lane * DPL;
-    const float inv = 1.f / l;
-#pragma unroll
-    for (int j = 0; j < DPL; ++j) o[j] = __float2half_rn(a[j] * inv);
+    __syncthreads();  // every warp has read the (max, sum) pairs
+    if (tid < used) src[tid * PR] = src[tid * PR + 1] = 0.f;
   }
 }
 
@@ -708,24 +724,22 @@ int rope_attn_splits(int B, int nkv, int S) {
 }
 
 size_t rope_attn_scratch_bytes(int B, int nq, int nkv, int dh, int S) {
-  // counters first (4-byte ints, rounded up to 256 bytes), then the partials.  Sized for every
-  // batch up to B (fewer sequences get more splits each), so one buffer serves smaller batches.
-  const size_t cnt = (static_cast<size_t>(B) * nkv * sizeof(int) + 255) & ~static_cast<size_t>(255);
+  // Sized for every batch up to B (fewer sequences get more splits each), so one buffer serves smaller
+  // batches.
   size_t rows = 0;
   for (int b = 1; b <= B; ++b) rows = std::max(rows, static_cast<size_t>(b) * rope_attn_splits(b, nkv, S));
-  return cnt + sizeof(float) * rows * nq * (dh + 4);
+  return sizeof(float) * rows * nq * (dh + 4);
 }
 
 int launch_rope_attn(const __half *qkv, const __half *qn, const __half *kn, const __half *cos_t, const __half *sin_t,
                      const long long *pos, __half *k_cache, __half *v_cache, void *scratch, __half *out, int B, int nq,
                      int nkv, int dh, int S, float scale, float eps, bool pdl, cudaStream_t stream) {
   const int nsplit = rope_attn_splits(B, nkv, S);
-  const size_t cnt = (static_cast<size_t>(B) * nkv * sizeof(int) + 255) & ~static_cast<size_t>(255);
-  int *counters = static_cast<int *>(scratch);
-  float *part = reinterpret_cast<float *>(static_cast<uint8_t *>(scratch) + cnt);
+  float *part = static_cast<float *>(scratch);
   const int group = nq / nkv;
   const int nb = group <= 8 ? 1 : 2;
-  const int smem = kFusedAttnWarps * 4 * 16 * (2 * dh + 16) + 8 * nb * (dh + 8) * 2;
+  int smem = kFusedAttnWarps * 4 * 16 * (2 * dh + 16) + 8 * nb * (dh + 8) * 2;
+  if (nsplit * nkv * B <= sm_count()) smem = std::max(smem, kSlotSmem);
   auto launch = [&](auto kernel) -> int {
     cudaLaunchConfig_t cfg = {};
     // one CTA per SM while the (sequence, KV head) pairs fit: like the GEMVs around it
@@ -739,8 +753,8 @@ int launch_rope_attn(const __half *qkv, const __half *qn, const __half *kn, cons
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     RDQ_CUDA(pin_slot(reinterpret_cast<const void *>(kernel), smem));
-    RDQ_CUDA(cudaLaunchKernelEx(&cfg, kernel, qkv, qn, kn, cos_t, sin_t, pos, k_cache, v_cache, part, counters, out, nq, nkv, S,
-                                scale, eps, nsplit, nkv * B));
+    RDQ_CUDA(cudaLaunchKernelEx(&cfg, kernel, qkv, qn, kn, cos_t, sin_t, pos, k_cache, v_cache, part, out, nq, nkv, S, scale, eps,
+                                nsplit, nkv * B));
     return RDQ_OK;
   };
   switch (dh) {
