@@ -389,16 +389,29 @@ __global__ void __launch_bounds__(kFusedAttnThreads, 2) rope_attn_kernel(
       cp_async16_if(dst + BLK + r * PITCH + 16 * c, vb + off, valid);
     }
   };
+  // Small loads first: behind 64 KB of cache rows they would wait for those.
+  const __half *cs = cos_t + p_new * DH, *sn = sin_t + p_new * DH;
+  float c0[HALF / 32], s0[HALF / 32], c1[HALF / 32], s1[HALF / 32];
+  load_row(cs, c0, c1);
+  load_row(sn, s0, s1);
+  // the warp whose block holds the new row: key and value to the cache now, into the block when it is current
+  const int new_blk = p_new >= p0 && p_new < p1 ? static_cast<int>(p_new - p0) >> 4 : -1;
+  const bool owns_new = new_blk >= 0 && new_blk % W == warp;
+  __half knew0[HALF / 32], knew1[HALF / 32], vnew[DPL];
+  float kx0[HALF / 32], kx1[HALF / 32], kw0[HALF / 32], kw1[HALF / 32];
+  if (owns_new) {
+    const __half *vsrc = row + 1ll * (nq + nkv + kvh) * DH;
+    load_row(row + 1ll * (nq + kvh) * DH, kx0, kx1);
+    if (kn) load_row(kn, kw0, kw1);
+#pragma unroll
+    for (int j = 0; j < DPL; ++j) vnew[j] = vsrc[lane + 32 * j];
+  }
   if (warp < nblk) load_block(warp, 0);
   cp_async_commit();
   if (warp + W < nblk) load_block(warp + W, 1);
   cp_async_commit();
 
   // ---- 1. query heads, new key and value
-  const __half *cs = cos_t + p_new * DH, *sn = sin_t + p_new * DH;
-  float c0[HALF / 32], s0[HALF / 32], c1[HALF / 32], s1[HALF / 32];
-  load_row(cs, c0, c1);
-  load_row(sn, s0, s1);
   // RMSNorm over the head (when nw), rotary embedding
   auto norm_rope = [&](const float (&x0)[HALF / 32], const float (&x1)[HALF / 32], bool nw, const float (&w0)[HALF / 32],
                        const float (&w1)[HALF / 32], __half (&o0)[HALF / 32], __half (&o1)[HALF / 32]) {
@@ -433,17 +446,7 @@ __global__ void __launch_bounds__(kFusedAttnThreads, 2) rope_attn_kernel(
       qs[hq * QP + lane + 32 * u + HALF] = o1[u];
     }
   }
-  // the warp whose block holds the new row: key and value to the cache now, into the block when it is current
-  const int new_blk = p_new >= p0 && p_new < p1 ? static_cast<int>(p_new - p0) >> 4 : -1;
-  const bool owns_new = new_blk >= 0 && new_blk % W == warp;
-  __half knew0[HALF / 32], knew1[HALF / 32], vnew[DPL];
   if (owns_new) {
-    float kx0[HALF / 32], kx1[HALF / 32], kw0[HALF / 32], kw1[HALF / 32];
-    const __half *vsrc = row + 1ll * (nq + nkv + kvh) * DH;
-    load_row(row + 1ll * (nq + kvh) * DH, kx0, kx1);
-    if (kn) load_row(kn, kw0, kw1);
-#pragma unroll
-    for (int j = 0; j < DPL; ++j) vnew[j] = vsrc[lane + 32 * j];
     norm_rope(kx0, kx1, kn != nullptr, kw0, kw1, knew0, knew1);
     __half *kd = k_cache + ((1ll * b * nkv + kvh) * S + p_new) * DH;
     __half *vd = v_cache + ((1ll * b * nkv + kvh) * S + p_new) * DH;
@@ -497,16 +500,22 @@ __global__ void __launch_bounds__(kFusedAttnThreads, 2) rope_attn_kernel(
       for (int j = 0; j < DPL; ++j) sv[lane + 32 * j] = vnew[j];
     }
     __syncwarp();
-    float s[NB][4];
+    float s[NB][4], s_odd[NB][4];  // two chains: a product waits for the one before the last
 #pragma unroll
-    for (int nb = 0; nb < NB; ++nb) s[nb][0] = s[nb][1] = s[nb][2] = s[nb][3] = 0.f;
+    for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[nb][j] = s_odd[nb][j] = 0.f;
 #pragma unroll
     for (int k = 0; k < KS; ++k) {
       uint32_t a0, a1, a2, a3;
       ldmatrix_x4(blk + k_lane + 32 * k, a0, a1, a2, a3);
 #pragma unroll
-      for (int nb = 0; nb < NB; ++nb) mma_16816(s[nb], a0, a1, a2, a3, qf[nb][k][0], qf[nb][k][1]);
+      for (int nb = 0; nb < NB; ++nb) mma_16816(k & 1 ? s_odd[nb] : s[nb], a0, a1, a2, a3, qf[nb][k][0], qf[nb][k][1]);
     }
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[nb][j] += s_odd[nb][j];
     const int rows = p1 - p0 - 16 * i;  // valid rows of the block
     uint32_t ph[NB][2], pl[NB][2];
 #pragma unroll
@@ -739,7 +748,8 @@ int launch_rope_attn(const __half *qkv, const __half *qn, const __half *kn, cons
   const int group = nq / nkv;
   const int nb = group <= 8 ? 1 : 2;
   int smem = kFusedAttnWarps * 4 * 16 * (2 * dh + 16) + 8 * nb * (dh + 8) * 2;
-  if (nsplit * nkv * B <= sm_count()) smem = std::max(smem, kSlotSmem);
+  // two CTAs per SM while that is enough for the grid: with three, 256 CTAs were placed on 86 SMs
+  if (nsplit * nkv * B <= 2 * sm_count()) smem = std::max(smem, kSlotSmem);
   auto launch = [&](auto kernel) -> int {
     cudaLaunchConfig_t cfg = {};
     // one CTA per SM while the (sequence, KV head) pairs fit: like the GEMVs around it
