@@ -116,18 +116,21 @@ __device__ __forceinline__ uint32_t wait_bounded(uint32_t bar, uint32_t parity) 
       : "memory");
   return left;
 }
-// Wait (bounded, about 0.4 s) until the low half of a global word reaches `count`; the thread that is
-// the last of `parts` to pass puts the word back to zero.
-__device__ __forceinline__ bool wait_arrivals(uint32_t *word, uint32_t count, uint32_t parts) {
+// Wait (bounded, about 0.4 s) until the low half of a global word reaches `count`.  Afterwards each of
+// the `parts` waiting threads counts itself in the high half (pass_arrivals) and later, when the answer
+// has come, puts the word back to zero if it was the last (leave_arrivals).
+__device__ __forceinline__ bool wait_arrivals(uint32_t *word, uint32_t count) {
   uint32_t v = 0;
   for (int i = 0; i < 4000000; ++i) {
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
     if ((v & 0xffffu) == count) break;
     if (i > 64) __nanosleep(100);
   }
-  if ((v & 0xffffu) != count) return false;
-  if (atomicAdd(word, 0x10000u) >> 16 == parts - 1) atomicExch(word, 0u);
-  return true;
+  return (v & 0xffffu) == count;
+}
+__device__ __forceinline__ uint32_t pass_arrivals(uint32_t *word) { return atomicAdd(word, 0x10000u) >> 16; }
+__device__ __forceinline__ void leave_arrivals(uint32_t *word, uint32_t passed, uint32_t parts) {
+  if (passed == parts - 1) asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(word), "r"(0u) : "memory");
 }
 __device__ __forceinline__ void arrive_global(uint32_t *word) {
   asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(word) : "memory");

@@ -200,9 +200,11 @@ __device__ __forceinline__ void finish_shared(const PairArgs &a, const WorkItem 
     scl[e] = ch + e < a.N ? a.scale[ch + e] : 0.f;
     bia[e] = ch + e < a.N && a.bias ? __half2float(a.bias[ch + e]) : 0.f;
   }
-  if (q == 0 && lane == 0 && !wait_arrivals(a.counters + w.rem * 2 + rank, 4u * a.parts, a.parts)) *abort_flag = 1;
+  if (q == 0 && lane == 0 && !wait_arrivals(a.counters + w.rem * 2 + rank, 4u * a.parts)) *abort_flag = 1;
   asm volatile("bar.sync 1, 128;" ::: "memory");
   if (*abort_flag) return;
+  uint32_t *const word = a.counters + w.rem * 2 + rank;
+  const uint32_t passed = q == 0 && lane == 0 ? pass_arrivals(word) : 0u;
   const int tok0 = w.m * a.nt, ntok = min(a.nt, a.M - tok0);
   const int lo = ntok * w.part / a.parts, hi = ntok * (w.part + 1) / a.parts;
   const long long part_stride = 2ll * a.nt * 128;
@@ -244,6 +246,7 @@ __device__ __forceinline__ void finish_shared(const PairArgs &a, const WorkItem 
       }
     }
   }
+  if (q == 0 && lane == 0) leave_arrivals(word, passed, a.parts);
 }
 
 template <bool BF16>

@@ -56,6 +56,9 @@ template <int NT>
 constexpr int kStages = (512 - 2 * NT) / 128;
 template <int NT>
 constexpr int kThreads = (8 + 4 * kStages<NT>) * 32;
+// (bounds for the compiler: 88 registers, so that 256 threads of a kernel with 32 fit beside the CTA)
+template <int NT>
+constexpr int kThreadBound = NT == 64 ? 736 : kThreads<NT>;
 constexpr int kFinishThreads = 512;
 constexpr int kChunkBytes = 128 * 128;
 constexpr int kScaleBytes = 128 * 16;
@@ -109,7 +112,14 @@ struct StreamArgs {
   int test_timeout;
 };
 
+// output column, scale and bias of a row
+struct Row {
+  bool live;
+  int col;
+  float scl, bia;
+};
 struct StreamSmem {
+  Row cut[2][128];  // rows of the range's first and last tile, for finish_shared
   uint64_t w_full[kMaxRing], w_empty[kMaxRing];
   uint64_t full[3], empty[3];
   uint64_t d_full[2], d_empty[2];
@@ -224,12 +234,7 @@ __device__ __forceinline__ void convert_fp8(const uint4 &a, const uint4 &b, uint
   cvt_e4m3x4(b.w, o[14], o[15]);
 }
 
-// output column, scale and bias of row r of a segment's tile
-struct Row {
-  bool live;
-  int col;
-  float scl, bia;
-};
+// row r of a segment's tile
 __device__ __forceinline__ Row row_of(const StreamArgs &a, const Segment &g, int r, bool wanted) {
   Row w;
   const int row = g.row_tile * 128 + r;  // row inside the format group
@@ -255,37 +260,40 @@ __device__ __forceinline__ void store_row(void *y, long long i, float v) {
 
 // Half of the first 512 threads: waits until all parts of the segment's tile are in the workspace,
 // then adds and stores this CTA's share of its tokens.  `sub` (0, 1) and r (row) identify the thread.
-template <bool BF16>
-__device__ __forceinline__ void finish_shared(const StreamArgs &a, const StreamSched &sc, const Segment &g, int r, int sub,
-                                              int bar_id, volatile int *abort_flag) {
+// kPart parts of kTok tokens are read at a time: four of eight for narrow token tiles (a small layer's
+// tile has three or four parts), two of sixteen for wide ones.
+template <bool BF16, int kPart, int kTok>
+__device__ __forceinline__ void finish_shared(const StreamArgs &a, const StreamSched &sc, const Segment &g, const Row &row, int r,
+                                              int sub, int bar_id, volatile int *abort_flag) {
   const int b0 = first_cta(sc, blockIdx.x, g.start), b1 = last_cta(sc, blockIdx.x, g.start + sc.S[g.fmt]);
   const int parts = b1 - b0 + 1;
-  const Row row = row_of(a, g, r, true);
   const int tok0 = g.m_tile * sc.nt;
   const int ntok = min(sc.nt, sc.M - tok0);
   const int lo = ntok * (static_cast<int>(blockIdx.x) - b0) / parts, hi = ntok * (static_cast<int>(blockIdx.x) + 1 - b0) / parts;
-  if (r == 0 && sub == 0 && !wait_arrivals(a.arrived + b0, 4u * parts, parts)) *abort_flag = 1;
+  if (r == 0 && sub == 0 && !wait_arrivals(a.arrived + b0, 4u * parts)) *abort_flag = 1;
   asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "n"(kFinishThreads / 2) : "memory");
   if (*abort_flag) return;
-  constexpr int kTok = 8, kSub = 2;
+  const uint32_t passed = r == 0 && sub == 0 ? pass_arrivals(a.arrived + b0) : 0u;
+  constexpr int kSub = 2;
 #pragma unroll 1
   for (int t0 = lo + sub; t0 < hi; t0 += kTok * kSub) {
     float v[kTok];
 #pragma unroll
     for (int e = 0; e < kTok; ++e) v[e] = 0.f;
 #pragma unroll 1
-    for (int b = b0; b <= b1; b += 2) {
-      // two parts' loads in flight
-      const float *s0 = a.partial + (part_slot(sc, b, b0, g.start) * sc.nt + t0) * 128 + r;
-      const float *s1 = a.partial + (part_slot(sc, min(b + 1, b1), b0, g.start) * sc.nt + t0) * 128 + r;
-      float p0[kTok], p1[kTok];
+    for (int b = b0; b <= b1; b += kPart) {
+      // the loads of kPart parts in flight
+      float p[kPart][kTok];
 #pragma unroll
-      for (int e = 0; e < kTok; ++e) {
-        p0[e] = t0 + e * kSub < hi ? __ldcg(s0 + e * kSub * 128) : 0.f;
-        p1[e] = t0 + e * kSub < hi && b < b1 ? __ldcg(s1 + e * kSub * 128) : 0.f;
+      for (int i = 0; i < kPart; ++i) {
+        const float *src = a.partial + (part_slot(sc, min(b + i, b1), b0, g.start) * sc.nt + t0) * 128 + r;
+#pragma unroll
+        for (int e = 0; e < kTok; ++e) p[i][e] = t0 + e * kSub < hi && b + i <= b1 ? __ldcg(src + e * kSub * 128) : 0.f;
       }
 #pragma unroll
-      for (int e = 0; e < kTok; ++e) v[e] = (v[e] + p0[e]) + p1[e];
+      for (int i = 0; i < kPart; ++i)
+#pragma unroll
+        for (int e = 0; e < kTok; ++e) v[e] += p[i][e];
     }
     if (row.live) {
 #pragma unroll
@@ -294,11 +302,12 @@ __device__ __forceinline__ void finish_shared(const StreamArgs &a, const StreamS
           store_row<BF16>(a.y, 1ll * (tok0 + t0 + e * kSub) * a.N + row.col, fmaf(v[e], row.scl, row.bia));
     }
   }
+  if (r == 0 && sub == 0) leave_arrivals(a.arrived + b0, passed, parts);
 }
 
 // NT: most tokens per tile (64 or 128)
 template <int NT, bool BF16>
-__global__ void __launch_bounds__(kThreads<NT>, 1)
+__global__ void __launch_bounds__(kThreadBound<NT>, 1)
 gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_constant__ CUtensorMap w8map,
                    const __grid_constant__ CUtensorMap w16map, const __grid_constant__ CUtensorMap xmap,
                    const __grid_constant__ StreamArgs a, const __grid_constant__ StreamSched sc, int *status) {
@@ -467,6 +476,9 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
     // ------------------------------------------------------------------ epilogue
     const int q = warp & 3;
     const uint32_t lanes = static_cast<uint32_t>(q * 32) << 16;
+    // constants of the rows that are finished together with other CTAs: fetched now, when nobody waits
+    S.cut[0][q * 32 + lane] = row_of(a, segment_at(sc, begin, end), q * 32 + lane, true);
+    S.cut[1][q * 32 + lane] = row_of(a, segment_at(sc, end - 1, end), q * 32 + lane, true);
     Cursor d;
     bool first = true;
     for (int ck = begin; ck < end;) {
@@ -609,7 +621,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
       g = segment_at(sc, max(g.start, begin), end);
     }
     if (mine && !(g.c0 == 0 && g.c1 == sc.S[g.fmt]))
-      finish_shared<BF16>(a, sc, g, threadIdx.x & 127, (threadIdx.x >> 7) & 1, 1 + half, &S.abort_flag);
+      finish_shared<BF16, NT == 64 ? 4 : 2, NT == 64 ? 8 : 16>(a, sc, g, S.cut[half][threadIdx.x & 127], threadIdx.x & 127, (threadIdx.x >> 7) & 1, 1 + half, &S.abort_flag);
   }
   __syncthreads();
   if (S.abort_flag) {

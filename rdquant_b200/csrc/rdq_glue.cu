@@ -701,9 +701,14 @@ cudaError_t pin_slot(const void *fn, int smem) {
   return e;
 }
 
+// Up to eight rows the linears around these kernels are GEMVs, which share an SM by halves (kSlotSmem).
+// Above they are streaming GEMMs, which need most of an SM's shared memory: their CTAs load weights
+// while a kernel without any runs beside them.
+static bool takes_slot(int B) { return B <= 8; }
+
 int launch_add_rmsnorm(__half *x, const __half *delta, const __half *w, __half *out, int B, int H, float eps, bool pdl,
                        cudaStream_t stream) {
-  return launch_pdl(add_rmsnorm_kernel, dim3(std::max(B, sm_count())), dim3(256), true, pdl, stream, x, delta, w, out, B, H, eps);
+  return launch_pdl(add_rmsnorm_kernel, dim3(std::max(B, sm_count())), dim3(256), takes_slot(B), pdl, stream, x, delta, w, out, B, H, eps);
 }
 
 int launch_qk_rope_cache(const __half *qkv, const __half *qn, const __half *kn, const __half *cos_t, const __half *sin_t,
@@ -779,7 +784,7 @@ int launch_rope_attn(const __half *qkv, const __half *qn, const __half *kn, cons
 int launch_silu_mul(const __half *gu, __half *out, int B, int F, bool pdl, cudaStream_t stream) {
   const long long total = 1ll * B * (F / 8);
   (void)total;
-  return launch_pdl(silu_mul_kernel, dim3(sm_count()), dim3(256), true, pdl, stream, gu, out, B, F);
+  return launch_pdl(silu_mul_kernel, dim3(sm_count()), dim3(256), takes_slot(B), pdl, stream, gu, out, B, F);
 }
 
 }  // namespace rdq
