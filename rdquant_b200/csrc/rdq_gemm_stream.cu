@@ -31,7 +31,10 @@
 //   3        block scales of NVFP4 chunks by cp.async, on the chunk's barrier
 //   4-7      epilogue: tcgen05.ld, channel scale + bias, stores to y[token, perm[row]]
 //   8-       converters, a group of four warps (a warp per 32 tensor-memory lanes) per stage: three
-//            groups for up to 64 tokens, two above (the accumulators take more tensor memory)
+//            groups and stages of a chunk for up to 64 tokens; above, where the accumulators take more
+//            tensor memory and a k block's MMAs longer, four groups and stages of half a chunk (two
+//            of a whole one left the MMAs waiting: 1930 cycles per NVFP4 chunk of 128 tokens, whose
+//            MMAs take 1024)
 // Every launch is programmatic: it overlaps the end of the kernel before.  With RDQ_GEMV_PDL the
 // weight and scale loads start before the grid-dependency wait.
 //
@@ -50,10 +53,12 @@ namespace rdq {
 
 namespace {
 
-// tokens per tile -> pipeline stages = converter groups: two accumulators of that many columns and
-// 128 columns per stage share the 512 columns
+// tokens per tile -> k blocks of 64 per stage, pipeline stages = converter groups: two accumulators of
+// that many columns and 32 columns per k block of a stage share the 512 columns
 template <int NT>
-constexpr int kStages = (512 - 2 * NT) / 128;
+constexpr int kBlocks = NT == 64 ? 4 : 2;
+template <int NT>
+constexpr int kStages = (512 - 2 * NT) / (32 * kBlocks<NT>);
 template <int NT>
 constexpr int kThreads = (8 + 4 * kStages<NT>) * 32;
 // (bounds for the compiler: 88 registers, so that 256 threads of a kernel with 32 fit beside the CTA)
@@ -121,7 +126,7 @@ struct Row {
 struct StreamSmem {
   Row cut[2][128];  // rows of the range's first and last tile, for finish_shared
   uint64_t w_full[kMaxRing], w_empty[kMaxRing];
-  uint64_t full[3], empty[3];
+  uint64_t full[4], empty[4];
   uint64_t d_full[2], d_empty[2];
   uint64_t never;
   uint32_t tmem_base;
@@ -196,16 +201,14 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, ui
       "r"(tmem_a), "r"(db_lo), "r"(db_hi), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// the MMAs of B k blocks of 64
-template <int B>
-__device__ __forceinline__ void issue_blocks(uint32_t acc, uint32_t wa, uint32_t dx, uint32_t dx_hi, uint32_t box, uint32_t idesc,
-                                             uint32_t accumulate) {
+// MMAs FROM .. TO - 1 of a stage (four to a k block of 64)
+template <int FROM, int TO>
+__device__ __forceinline__ void issue_mmas(uint32_t acc, uint32_t wa, uint32_t dx, uint32_t dx_hi, uint32_t box, uint32_t idesc,
+                                           uint32_t accumulate) {
 #pragma unroll
-  for (int b = 0; b < B; ++b) {
-#pragma unroll
-    for (int k4 = 0; k4 < 4; ++k4)
-      umma_f16_ts(acc, wa + 32 * b + 8 * k4, dx + 2 * k4, dx_hi, idesc, b == 0 && k4 == 0 ? accumulate : 1u);
-    dx += box;
+  for (int i = 0; i < TO; ++i) {
+    if (i >= FROM) umma_f16_ts(acc, wa + 8 * i, dx + 2 * (i & 3), dx_hi, idesc, i == 0 ? accumulate : 1u);
+    if ((i & 3) == 3) dx += box;
   }
 }
 
@@ -311,13 +314,13 @@ __global__ void __launch_bounds__(kThreadBound<NT>, 1)
 gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_constant__ CUtensorMap w8map,
                    const __grid_constant__ CUtensorMap w16map, const __grid_constant__ CUtensorMap xmap,
                    const __grid_constant__ StreamArgs a, const __grid_constant__ StreamSched sc, int *status) {
-  constexpr int NS = kStages<NT>;
+  constexpr int NS = kStages<NT>, KB = kBlocks<NT>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ StreamSmem S;
   const uint32_t w_ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t x_ring = w_ring + a.nw * kChunkBytes;
   const uint32_t x_bytes = static_cast<uint32_t>(sc.nt) * 128;  // one 64-k box
-  const uint32_t s_ring = x_ring + NS * 4 * x_bytes;
+  const uint32_t s_ring = x_ring + NS * KB * x_bytes;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int begin = sc.bnd[blockIdx.x], end = sc.bnd[blockIdx.x + 1];
   auto load_chunk = [&](const Segment &g, int c, int slot) {
@@ -334,7 +337,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
   if (threadIdx.x == 0) {
     for (int i = 0; i < a.nw; ++i) {
       mbar_init(smem_u32(&S.w_full[i]), 1 + 32);  // the TMA thread and the scale warp's lanes
-      mbar_init(smem_u32(&S.w_empty[i]), 4);      // the group that converts the chunk
+      mbar_init(smem_u32(&S.w_empty[i]), 16 / KB);  // the groups that convert a chunk of four k blocks
     }
     mbar_init_fence();
     Segment g = segment_at(sc, begin, end);
@@ -365,6 +368,11 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
   const uint32_t tmem_a = tmem + 2 * NT;
   pdl_launch_dependents();
 
+  // stages of a range: its NVFP4 chunks (they come first) take several each above 64 tokens
+  constexpr int split = 4 / KB;
+  const int n4 = max(0, min(end, sc.E[0]) - begin);
+  const int stages = split * n4 + (end - begin - n4);
+
   if (warp == 0) {
     // ---------------------------------------------------------------- weight chunks
     const bool leader = elect_one();
@@ -387,15 +395,21 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
     for (int i = begin; i < end; ++i) {
       if (i >= g.start + g.c1) g = segment_at(sc, i, end);
       const int per = 4 >> g.fmt;  // k blocks of 64 per chunk
-      const int kb0 = (i - g.start) * per, nb = min(per, sc.nkb - kb0);
-      if (!gemm_wait(&S.empty[x.i], x.ph ^ 1, &S.abort_flag)) break;
-      if (leader) {
-        const uint32_t bar = smem_u32(&S.full[x.i]);
-        const uint32_t dst = x_ring + x.i * 4 * x_bytes;
-        mbar_arrive_expect_tx(bar, nb * x_bytes);
-        for (int b = 0; b < nb; ++b) tma_load_2d(dst + b * x_bytes, &xmap, (kb0 + b) * 64, g.m_tile * sc.nt, bar);
+      const int kb0 = (i - g.start) * per, blocks = min(per, sc.nkb - kb0);
+      bool ok = true;
+      for (int b = 0; b < per && ok; b += KB) {  // stages of the chunk; past K a stage can be empty
+        ok = gemm_wait(&S.empty[x.i], x.ph ^ 1, &S.abort_flag);
+        if (ok && leader) {
+          const uint32_t bar = smem_u32(&S.full[x.i]);
+          const uint32_t dst = x_ring + x.i * KB * x_bytes;
+          const int nb = min(KB, blocks - b);
+          if (nb > 0) mbar_arrive_expect_tx(bar, nb * x_bytes);
+          else mbar_arrive(bar);
+          for (int j = 0; j < nb; ++j) tma_load_2d(dst + j * x_bytes, &xmap, (kb0 + b + j) * 64, g.m_tile * sc.nt, bar);
+        }
+        x.next(NS);
       }
-      x.next(NS);
+      if (!ok) break;
     }
   } else if (warp == 2) {
     // ---------------------------------------------------------------- MMA issue
@@ -409,37 +423,56 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
     const uint32_t full0 = smem_u32(&S.full[0]), empty0 = smem_u32(&S.empty[0]);
     uint32_t stage = 0, ph = 0;
     Cursor d;
-    uint32_t ok = 1;
+    int left = stages;
+    uint32_t ok = NT > 64 ? wait_bounded(full0, 0) : 1u;
+    tc_fence_after();
     for (int ck = begin; ck < end && ok;) {
       const Segment g = segment_at(sc, ck, end);
       const int per = 4 >> g.fmt;
       if (!gemm_wait(&S.d_empty[d.i], d.ph ^ 1, &S.abort_flag)) break;
       tc_fence_after();
       const uint32_t acc = tmem + d.i * NT;
-      const int whole = min(g.c1, sc.nkb / per) - g.c0;  // chunks with all their k blocks
-      const int rest = whole < g.c1 - g.c0 ? sc.nkb - (g.c1 - 1) * per : 0;
+      const int bps = min(per, KB);                                    // k blocks of a stage
+      const int blocks = min(g.c1 * per, sc.nkb) - g.c0 * per;
+      const int whole = blocks / bps, rest = blocks - whole * bps;     // stages with all of them
+      const int none = (g.c1 - g.c0) * (per / bps) - whole - (rest > 0);  // stages past K
       uint32_t accumulate = 0;
+      // Above 64 tokens the next stage is waited for ahead of the last two MMAs of the present one: the
+      // tensor pipe takes an MMA when the one before last is done, so that a wait between stages is a
+      // gap of 140 cycles in its work (1700 -> 1540 cycles per NVFP4 chunk of 128 tokens).
       auto run = [&](auto blocks, int count) {
+        constexpr int n = 4 * decltype(blocks)::value, head = NT == 64 ? 0 : (n > 2 ? n - 2 : 0);
 #pragma unroll 1
         for (int i = 0; i < count; ++i) {
-          ok = wait_bounded(full0 + stage * 8, ph);
-          if (!ok) break;
-          tc_fence_after();
-          if (leader) {
-            issue_blocks<decltype(blocks)::value>(acc, tmem_a + stage * 128, dx0 + stage * 4 * box, dx_hi, box, idesc, accumulate);
-            umma_commit(empty0 + stage * 8);
+          const uint32_t wa = tmem_a + stage * (32 * KB), dx = dx0 + stage * KB * box, empty = empty0 + stage * 8;
+          if (NT == 64) {  // (with few columns the weights are what a stage waits for, and its release must not)
+            ok = wait_bounded(full0 + stage * 8, ph);
+            if (!ok) break;
+            tc_fence_after();
+          } else if (leader) {
+            issue_mmas<0, head>(acc, wa, dx, dx_hi, box, idesc, accumulate);
           }
-          accumulate = 1;
           stage = stage + 1 == NS ? 0 : stage + 1;
           ph ^= stage == 0;
+          if (NT > 64) {
+            if (--left > 0) ok = wait_bounded(full0 + stage * 8, ph);
+            tc_fence_after();
+          }
+          if (leader) {
+            issue_mmas<head, n>(acc, wa, dx, dx_hi, box, idesc, accumulate);
+            umma_commit(empty);
+          }
+          accumulate = 1;
+          if (!ok) break;
         }
       };
-      if (per == 4) run(std::integral_constant<int, 4>(), whole);
-      else if (per == 2) run(std::integral_constant<int, 2>(), whole);
+      if (bps == 4) run(std::integral_constant<int, 4>(), whole);
+      else if (bps == 2) run(std::integral_constant<int, 2>(), whole);
       else run(std::integral_constant<int, 1>(), whole);
       if (rest == 3) run(std::integral_constant<int, 3>(), 1);
       else if (rest == 2) run(std::integral_constant<int, 2>(), 1);
       else if (rest == 1) run(std::integral_constant<int, 1>(), 1);
+      run(std::integral_constant<int, 0>(), none);
       if (ok && leader) umma_commit(smem_u32(&S.d_full[d.i]));
       d.next(2);
       ck = g.start + g.c1;
@@ -542,19 +575,28 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
     }
   } else {
     // ------------------------------------------------------------------ converters
-    // Group `grp` owns stage `grp` and takes every NS-th chunk.  It waits for the release of its stage
-    // first: the MMAs have then consumed every chunk up to NS before this one, so the parity it tests
-    // on the chunk's barrier (used by chunk i - nw before, nw >= NS) cannot be a round old.
+    // Group `grp` owns stage `grp` and takes every NS-th stage's worth of chunks: a part of an NVFP4
+    // chunk (`split` to a chunk) or a whole chunk of the other formats.  It waits for the release of its
+    // stage first: the MMAs have then consumed every stage up to NS before this one, so the parity it
+    // tests on the chunk's barrier (used by chunk i - nw before, nw >= NS) cannot be a round old.
     const int q = warp & 3, grp = (warp - 8) >> 2;
     const int row = q * 32 + lane;
     const uint32_t rbase = row * 128, sw = row & 7;
-    const uint32_t dst = tmem_a + grp * 128 + (static_cast<uint32_t>(q * 32) << 16);
-    int slot = grp;
+    const uint32_t dst = tmem_a + grp * (32 * KB) + (static_cast<uint32_t>(q * 32) << 16);
+    int slot = 0, last = begin;
     uint32_t w_ph = 0, ph = 0;
     Segment g;
     g.start = g.c1 = 0;
-    for (int i = begin + grp; i < end; i += NS) {
-      if (i == begin + grp || i >= g.start + g.c1) g = segment_at(sc, i, end);
+    for (int j = grp; j < stages; j += NS) {
+      const int i = j < split * n4 ? begin + j / split : begin + n4 + (j - split * n4);
+      const int part = j < split * n4 ? j % split : 0;
+      slot += i - last;  // at most NS further
+      last = i;
+      if (slot >= a.nw) {
+        slot -= a.nw;
+        w_ph ^= 1;
+      }
+      if (j == grp || i >= g.start + g.c1) g = segment_at(sc, i, end);
       if (!gemm_wait(&S.empty[grp], ph ^ 1, &S.abort_flag)) break;
       if (!gemm_wait(&S.w_full[slot], w_ph, &S.abort_flag)) break;
       tc_fence_after();
@@ -564,10 +606,10 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
       if (g.fmt == 0) {
         // (k blocks beyond K convert the zero fill of the box; the MMAs do not read them)
         const uint4 s4 = lds16(s_ring + slot * kScaleBytes + row * 16);
-        const uint32_t sc4[4] = {s4.x, s4.y, s4.z, s4.w};
+        const uint32_t sc4[4] = {part ? s4.z : s4.x, part ? s4.w : s4.y, s4.z, s4.w};
 #pragma unroll
-        for (int h = 0; h < 8; ++h) {
-          convert_fp4(piece(h), sc4[h >> 1] >> (16 * (h & 1)), o);
+        for (int h = 0; h < 2 * KB; ++h) {
+          convert_fp4(piece(2 * KB * part + h), sc4[h >> 1] >> (16 * (h & 1)), o);
           tmem_st16(dst + 16 * h, o);
         }
       } else if (g.fmt == 1) {
@@ -595,14 +637,9 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(smem_u32(&S.full[grp]));
-        mbar_arrive(smem_u32(&S.w_empty[slot]));
+        mbar_arrive(smem_u32(&S.w_empty[slot]), g.fmt == 0 ? 1u : static_cast<uint32_t>(split));
       }
       ph ^= 1;
-      slot += NS;
-      if (slot >= a.nw) {
-        slot -= a.nw;
-        w_ph ^= 1;
-      }
     }
   }
 
@@ -640,7 +677,8 @@ struct StreamPlan {
 };
 
 // Token tiles of equal width; a chunk costs what bounds it: its bytes at the SM's share of the HBM
-// rate (23 B/clk), the conversion of its k blocks, or their tensor time.
+// rate (23 B/clk; the other token tiles find it in L2), the conversion of its k blocks, or its stages
+// in the tensor pipe.
 StreamPlan make_plan(int n4, int n8, int n16, int M, int K) {
   StreamPlan p;
   StreamSched &s = p.sc;
@@ -655,8 +693,14 @@ StreamPlan make_plan(int n4, int n8, int n16, int M, int K) {
   for (int f = 0; f < 3; ++f) {
     const int per = 4 >> f;
     s.S[f] = (s.nkb + per - 1) / per;
+    // (measured on 128 x 128 tiles: 1540 / 825 / 581 cycles per NVFP4 / FP8 / FP16 chunk)
+    const int bps = std::min(per, kBlocks<128>);
     const double conv = f == 0 ? 170 : (f == 1 ? 150 : 90);
-    u[f] = static_cast<int>(std::max(bytes[f] / 23.0, per * std::max(conv, 2.0 * s.nt)));
+    const double work = s.nt > 64 ? per / bps * (300 + 1.85 * bps * s.nt) : per * std::max(conv, 2.0 * s.nt);
+    // the few FP16 channels lie far apart: every value of their tiles is a memory sector of its own,
+    // 52000 cycles of stores for 128 x 128 of them (an FP16 CTA was 10 us late at 512 tokens)
+    const double scattered = f == 2 && s.nt > 64 ? 410.0 * s.nt / s.S[f] : 0.0;
+    u[f] = static_cast<int>(std::max(bytes[f] / (23.0 * s.mt), work) + scattered);
     const int chunks = (n[f] + 127) / 128 * s.mt * s.S[f];
     e += chunks;
     w += 1ll * chunks * u[f];
@@ -672,7 +716,7 @@ StreamPlan make_plan(int n4, int n8, int n16, int M, int K) {
   }
   s.bnd[s.G] = e;
   p.wide = s.nt > 64;
-  const int xb = (p.wide ? kStages<128> : kStages<64>) * 4 * s.nt * 128;
+  const int xb = (p.wide ? kStages<128> * kBlocks<128> : kStages<64> * kBlocks<64>) * s.nt * 128;
   p.nw = std::min(kMaxRing, (kSmemMax - 1024 - xb) / (kChunkBytes + kScaleBytes));
   p.smem = 1024 + xb + p.nw * (kChunkBytes + kScaleBytes);
   return p;
