@@ -55,15 +55,15 @@ int stream_from(const rdq_layer &l) {
 // row-major tensors by TMA (K a multiple of 64 / 16); what they cannot take runs as 16-row panels of
 // the decode kernel.
 //
-// Above 256 rows the streaming GEMM converts the weights once more per 128 rows, the other GEMM decodes
-// them once: estimates in microseconds that agree with measurements between 256 and 1536 rows on five
-// layer shapes within 15 %.
+// The streaming GEMM converts the weights once more per 128 rows, the other GEMM decodes them once:
+// estimates in microseconds that agree with measurements between 65 and 2048 rows on seven layer
+// shapes within 15 %.  (With up to 64 rows the streaming GEMM was faster on all of them.)
 bool stream_beats_dense(const rdq_layer &l, int M) {
-  if (M <= 256) return true;
+  if (M <= 64) return true;
   if (M > 2048) return false;
   const int N = l.n_fp4 + l.n_fp8 + l.n_fp16;
   const double weights = 1e-6 * N * l.K;
-  return 14.0 + 1.62e-3 * M * weights < 8.0 + 0.5 * weights + gemm_dense_cycles(M, N, l.K) / 1750.0;
+  return 15.5 + 1.62e-3 * M * weights < 4.5 + 0.6 * weights + gemm_dense_cycles(M, N, l.K) / 1750.0;
 }
 
 Path path_of(const rdq_layer &l, int M) {
