@@ -261,16 +261,37 @@ __device__ __forceinline__ void tile_geom(const TSched &sc, int gtile, int &firs
   }
 }
 
+// Split of an activation prologue: a row is cut into `cpr` chunks (a divisor of the twelve warps) of
+// `per` 16-byte vectors; a warp takes chunk warp % cpr of the rows warp / cpr, + 12 / cpr, ...  Chunks
+// of up to four vectors per lane, and no more rows at a time than there are.
+__host__ __device__ inline void prologue_split(int M, int nvec, int &cpr, int &per) {
+  cpr = 1;
+  per = nvec;
+  while (cpr < kMmaWarps && (per > 128 || kMmaWarps / cpr > M)) {
+    cpr = cpr == 4 ? 6 : (cpr == 6 ? 12 : cpr + 1);
+    per = (nvec + cpr - 1) / cpr;
+  }
+}
+// All rows at once with up to two vectors per lane: they stay in registers between the two passes of a
+// norm (2560 wide, one row: 2.0 -> 1.5 us).
+inline bool norm_in_registers(int M, int K) {
+  int cpr, per;
+  prologue_split(M, K >> 3, cpr, per);
+  return M <= kMmaWarps / cpr && per <= 64;
+}
+
 // NT = number of 8-row activation groups (1: M <= 8, 2: M <= 16)
-// EXTRA: the launch has an activation prologue or peer destinations (compiled apart so that the
-// plain launch carries none of that code)
+// EXTRA 1: the launch has an activation prologue or peer destinations (compiled apart so that the
+// plain launch carries none of that code).  The usual prologues of up to eight rows are compiled apart
+// once more, for the code and registers of the others cost them 1 to 2 %: 2 norm whose rows stay in
+// registers (norm_in_registers), 3 silu, 4 bf16.
 //
 // Warp group g takes the g-th third of the CTA's images, in order, through ring slots g, g + 3, ... of
 // its own; epilogue warp g finishes the tiles whose first image (in this CTA) lies in that third.  A
 // group therefore hands sums over once per tile -- images dealt out in turn would end every stage of a
 // two-image tile with a hand-over, which measured a third of the MMA warps' time -- and everybody
 // derives his images from the range alone, without a list.
-template <int NT, bool XS, bool EXTRA>
+template <int NT, bool XS, int EXTRA>
 __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_constant__ TiledArgs a,
                                                   const __grid_constant__ TSched sc) {
   extern __shared__ __align__(128) uint8_t smem[];
@@ -283,6 +304,8 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
   __shared__ __align__(8) uint64_t bar_never;  // nothing ever arrives here (time-out self-test)
   __shared__ float xred[EXTRA ? RDQ_MAX_GEMV_M : 1][kMmaWarps];  // activation prologue: per-warp sums of squares
 
+  // the prologue: known at compile time but for EXTRA 1
+  const int xop = EXTRA == 0 ? 0 : EXTRA == 2 ? 1 : EXTRA == 3 ? 2 : EXTRA == 4 ? 3 : a.xop;
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
@@ -359,7 +382,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
     // sleeps on bar_x, which completes after it (and after the activation copies).
     pdl_wait();
     const uint32_t bx = smem_u32(&bar_x);
-    if (XS && (!EXTRA || a.xop == 0)) {
+    if (XS && (!EXTRA || xop == 0)) {
       mbar_arrive_expect_tx(bx, static_cast<uint32_t>(M) * 2u * K);
       for (int m = 0; m < M; ++m) bulk_g2s(smem_u32(xsm) + m * xpitch, a.x + 1ll * m * K, 2u * K, bx);
     } else {  // the MMA warps fetch (and transform) the activations themselves
@@ -535,9 +558,9 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
         for (int i = 0; i < 4; ++i) {
           if (i >= nm) break;
           const long long at = 1ll * (m0 + i) * N + cur_col;
-          if (!EXTRA) {
+          if (EXTRA != 1 && EXTRA != 4) {
             static_cast<__half *>(a.y)[at] = __float2half_rn(o[i]);
-          } else if (a.n_dst == 0) {
+          } else if (EXTRA == 4 || a.n_dst == 0) {
             store_y(a.y, at, o[i], a.y_bf16);
           } else {
             // the 16 rows of a tile are consecutive columns of the slice: the stores of the lanes
@@ -554,7 +577,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
       ++gt;
       tile_geom(sc, gt, f, S, fmt);
     }
-    if (EXTRA && a.n_dst > 0) {
+    if (EXTRA == 1 && a.n_dst > 0) {
       // This warp's stores to the other GPUs are complete system-wide before it counts itself
       // done; the warp that completes the count publishes the launch number in this rank's flag
       // word on every GPU (release: fence, then the flag stores).
@@ -601,23 +624,18 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
 #pragma unroll
       for (int i = 0; i < 4; ++i) acc[n][c][i] = 0.f;
 
-  // Split of an activation prologue: a row is cut into `cpr` chunks (a divisor of the twelve warps) of
-  // `per` 16-byte vectors; a warp takes chunk warp % cpr of the rows warp / cpr, + 12 / cpr, ...  Chunks
-  // of up to four vectors per lane, and no more rows at a time than there are.
   const int nvec = K >> 3;
   int cpr = 1, per = nvec;
-  if (EXTRA && XS && a.xop != 0) {
-    while (cpr < kMmaWarps && (per > 128 || kMmaWarps / cpr > M)) {
-      cpr = cpr == 4 ? 6 : (cpr == 6 ? 12 : cpr + 1);
-      per = (nvec + cpr - 1) / cpr;
-    }
-  }
+  if (EXTRA && XS && xop != 0) prologue_split(M, nvec, cpr, per);
   const int vlo = (warp % cpr) * per, vhi = min(nvec, vlo + per), rows_at_once = kMmaWarps / cpr;
-  if (EXTRA && XS && a.xop == 1 && a.early) {
-    // the norm's weights are constants: into L1 while the kernel before this one still runs
-    for (int i = vlo + lane; i < vhi; i += 32) {
+  uint4 nw[2];  // (EXTRA 2)
+  if (EXTRA && XS && xop == 1 && a.early) {
+    // the norm's weights are constants: into registers, or L1, while the kernel before this one still runs
+    for (int i = vlo + lane, q = 0; i < vhi; i += 32, ++q) {
       const uint4 v = ldg_nc16(a.x_weight + 8 * i);
-      asm volatile("" ::"r"(v.x));
+      if (EXTRA == 2 && q == 0) nw[0] = v;
+      else if (EXTRA == 2) nw[1] = v;
+      else asm volatile("" ::"r"(v.x));
     }
   }
 
@@ -627,12 +645,62 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
     if (lane == 0) atomicExch(status, 6);
     return;
   }
-  if (EXTRA && XS && a.xop != 0) {
+  if (EXTRA && XS && xop != 0) {
     // ---- activation prologue: the twelve MMA warps build the CTA's activation rows in shared
     // memory from what the preceding kernels left in global memory (every CTA does the same work:
     // a few KB out of L2).  A row is cut into `cpr` chunks, one warp per chunk, and a lane has
     // four vectors (eight with x_aux) in flight: the cost is a few L2 round trips.
-    if (a.xop == 1) {
+    if (EXTRA == 2) {
+      const int m = warp / cpr;
+      const __half *xr = a.x + 1ll * m * K;
+      uint4 v[2], d[2];
+      float ss = 0.f;
+      if (m < M) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const int i = vlo + lane + 32 * q;
+          if (i >= vhi) break;
+          v[q] = ldg_cg16(xr + 8 * i);
+          if (a.x_aux) d[q] = ldg_cg16(a.x_aux + 1ll * m * K + 8 * i);
+          if (!a.early) nw[q] = ldg_nc16(a.x_weight + 8 * i);
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const int i = vlo + lane + 32 * q;
+          if (i >= vhi) break;
+          __half2 *hv = reinterpret_cast<__half2 *>(&v[q]);
+          const __half2 *dh = reinterpret_cast<const __half2 *>(&d[q]);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if (a.x_aux) hv[j] = __hadd2(hv[j], dh[j]);
+            const float2 f = __half22float2(hv[j]);
+            ss += f.x * f.x + f.y * f.y;
+          }
+          if (a.x_out && blockIdx.x == 0) *reinterpret_cast<uint4 *>(a.x_out + 1ll * m * K + 8 * i) = v[q];
+        }
+        ss = warp_sum(ss);
+        if (lane == 0) xred[m][warp % cpr] = ss;
+      }
+      asm volatile("bar.sync 2, %0;" ::"r"(kMmaWarps * 32) : "memory");
+      if (m < M) {
+        ss = 0.f;
+        for (int w = 0; w < cpr; ++w) ss += xred[m][w];
+        const float rs = rsqrtf(ss / K + a.x_eps);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const int i = vlo + lane + 32 * q;
+          if (i >= vhi) break;
+          __half2 *hv = reinterpret_cast<__half2 *>(&v[q]);
+          const __half2 *wh = reinterpret_cast<const __half2 *>(&nw[q]);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 f = __half22float2(hv[j]);
+            hv[j] = __hmul2(__floats2half2_rn(f.x * rs, f.y * rs), wh[j]);
+          }
+          *reinterpret_cast<uint4 *>(xsm + m * xpitch + 16 * i) = v[q];
+        }
+      }
+    } else if (xop == 1) {
       for (int m = warp / cpr; m < M; m += rows_at_once) {
         const __half *xr = a.x + 1ll * m * K;
         const __half *dr = a.x_aux ? a.x_aux + 1ll * m * K : nullptr;
@@ -698,7 +766,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
           }
         }
       }
-    } else if (a.xop == 3) {
+    } else if (xop == 3) {
       for (int m = warp / cpr; m < M; m += rows_at_once) {
         const __half *xr = a.x + 1ll * m * K;
         for (int i0 = vlo + lane; i0 < vhi; i0 += 128) {
@@ -1011,22 +1079,30 @@ int launch_gemv_tiled(const GemvTiledArgs &h, bool pdl, cudaStream_t stream) {
   const int smem = pl.smem;
 
 
-  static int smem_set[64][8] = {};
+  static int smem_set[64][11] = {};
   static std::mutex smem_mutex;
   int dev = 0;
   RDQ_CUDA(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> smem_lock(smem_mutex);
   const bool extra = a.xop != 0 || h.n_dst > 0 || h.y_bf16;
-  const int variant = (extra ? 4 : 0) + (nt - 1) * 2 + (xs ? 1 : 0);
-  static const void *const fns[8] = {
-      reinterpret_cast<const void *>(gemv_tiled_kernel<1, false, false>),
-      reinterpret_cast<const void *>(gemv_tiled_kernel<1, true, false>),
-      reinterpret_cast<const void *>(gemv_tiled_kernel<2, false, false>),
-      reinterpret_cast<const void *>(gemv_tiled_kernel<2, true, false>),
-      reinterpret_cast<const void *>(gemv_tiled_kernel<1, false, true>),
-      reinterpret_cast<const void *>(gemv_tiled_kernel<1, true, true>),
-      reinterpret_cast<const void *>(gemv_tiled_kernel<2, false, true>),
-      reinterpret_cast<const void *>(gemv_tiled_kernel<2, true, true>)};
+  const bool in_registers = a.xop == 1 && !h.y_bf16 && norm_in_registers(h.M, h.K);
+  const bool own = extra && h.n_dst == 0 && nt == 1 && xs;  // a variant of its own
+  const int variant = own && in_registers                      ? 8
+                      : own && a.xop == 2 && !h.y_bf16 ? 9
+                      : own && a.xop == 3              ? 10
+                                                       : (extra ? 4 : 0) + (nt - 1) * 2 + (xs ? 1 : 0);
+  static const void *const fns[11] = {
+      reinterpret_cast<const void *>(gemv_tiled_kernel<1, false, 0>),
+      reinterpret_cast<const void *>(gemv_tiled_kernel<1, true, 0>),
+      reinterpret_cast<const void *>(gemv_tiled_kernel<2, false, 0>),
+      reinterpret_cast<const void *>(gemv_tiled_kernel<2, true, 0>),
+      reinterpret_cast<const void *>(gemv_tiled_kernel<1, false, 1>),
+      reinterpret_cast<const void *>(gemv_tiled_kernel<1, true, 1>),
+      reinterpret_cast<const void *>(gemv_tiled_kernel<2, false, 1>),
+      reinterpret_cast<const void *>(gemv_tiled_kernel<2, true, 1>),
+      reinterpret_cast<const void *>(gemv_tiled_kernel<1, true, 2>),
+      reinterpret_cast<const void *>(gemv_tiled_kernel<1, true, 3>),
+      reinterpret_cast<const void *>(gemv_tiled_kernel<1, true, 4>)};
   const void *fn = fns[variant];
   if (dev < 64 && smem_set[dev][variant] < smem) {
     RDQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
