@@ -240,7 +240,7 @@ PyObject *quantize_layer(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
       fp8_scale = cuda_empty({n[1]}, at::kFloat, dev);
     }
     if (n[2]) fp16 = cuda_empty({n[2], K}, at::kBFloat16, dev);
-    at::Tensor inv = cuda_empty({N}, at::kInt, dev), scratch = cuda_empty({2}, at::kFloat, dev);
+    at::Tensor inv = cuda_empty({N}, at::kInt, dev), scratch = cuda_empty({RDQ_QUANTIZE_LAYER_SCRATCH}, at::kFloat, dev);
     auto ptr = [](const at::Tensor &t) { return t.defined() ? t.data_ptr() : nullptr; };
     const int rc = rdq_quantize_layer(w->data_ptr(), w->scalar_type() == at::kFloat, static_cast<const long long *>(perm->data_ptr()),
                                       static_cast<int>(n[0]), static_cast<int>(n[1]), static_cast<int>(n[2]), static_cast<int>(K),
