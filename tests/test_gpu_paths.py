@@ -1,0 +1,153 @@
+"""Packed layers, single-token attention and the layer encoder at the sizes where their kernels and
+dispatch rules begin and end: edges of tiles and stages, remainders, smallest and largest rows."""
+import numpy as np
+import pytest
+import torch
+import torch.nn.functional as F
+
+from conftest import ORDER
+from oracle import oracle_np as onp
+from rdquant_b200 import _lib
+from rdquant_b200 import rdquant_cuda as rc
+from rdquant_b200.inference import FusedMixedLinear
+from rdquant_b200.integrations.hf_export import pack_layer
+from rdquant_b200.quantize import quantize_weight, quantize_weight_packed
+from rdquant_b200.synthetic import random_packed_layer
+from test_gpu_quantize import _special, _weights
+
+pytestmark = pytest.mark.gpu
+
+
+def _check_linear(n4, n8, n16, k, rows, dtype, bias, lead=()):
+    layer = random_packed_layer(n4, n8, n16, k, seed=n4 + n8 + k + rows)
+    splits = dict(zip(ORDER, (n4, n8, n16)))
+    n = n4 + n8 + n16
+    gen = torch.Generator().manual_seed(rows)
+    if bias:
+        layer["bias"] = (torch.randn(n, generator=gen) * 0.5).half()
+    mod = FusedMixedLinear.from_layer_data(layer, splits, k, "cuda")
+    x = torch.randn(rows, k, generator=gen).to(dtype).cuda()
+    y = mod(x.view(*lead, -1, k) if lead else x)
+    assert y.dtype == dtype and y.shape == (*(x.view(*lead, -1, k) if lead else x).shape[:-1], n)
+    assert torch.equal(mod(x), y.view(rows, n)), "two calls differ"
+    w = torch.from_numpy(onp.dequantize_layer_f32(onp.torch_layer_to_np(layer), splits, k)).cuda().double()
+    xd = x.double()
+    ref = xd @ w.t() + (layer["bias"].cuda().double() if bias else 0.0)
+    # a sum of k exact products in FP32: at most k rounding errors of 2^-24 of the sum of magnitudes (and
+    # one per weight for its channel scale); bf16 rows become f16 rows (below 2^-14 a step of 2^-24); then
+    # the rounding of the result
+    mags = xd.abs() @ w.abs().t()
+    bound = (k + 2) * 2.0 ** -24 * mags + (2.0 ** -25 * w.abs().sum(1) if dtype == torch.bfloat16 else 0.0)
+    bound = bound + (2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8) * (ref.abs() + bound) + 2.0 ** -25
+    assert bool(((y.view(rows, n).double() - ref).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("rows", [1, 16, 17, 64, 65, 128, 129, 256, 257])
+@pytest.mark.parametrize("shape", [
+    (256, 128, 128, 320),    # k past the last whole chunk of every format; one CTA's worth of chunks
+    (300, 130, 20, 576),     # ragged groups
+    (0, 130, 0, 128), (64, 0, 0, 64), (0, 0, 200, 192),  # one format, a single stage
+    (1280, 896, 128, 1088),  # tiles cut by ranges
+])
+def test_streaming_gemm_edges(shape, rows):
+    _check_linear(*shape, rows, torch.float16 if rows % 2 else torch.bfloat16, bias=rows in (16, 65, 129))
+
+
+@pytest.mark.parametrize("shape,rows", [
+    ((128, 64, 16, 208), 17),      # k a multiple of 16 only: decoded once from the first GEMM row on
+    ((600, 303, 100, 336), 700),   # odd number of channels, partial tiles of both kinds
+    ((768, 256, 0, 256), 2049),    # beyond the streaming GEMM
+    ((2048, 384, 128, 2560), 1280),  # tiles split along k
+])
+def test_decoded_once_gemm_edges(shape, rows):
+    _check_linear(*shape, rows, torch.float16, bias=True)
+    _check_linear(*shape, rows, torch.bfloat16, bias=False)
+
+
+@pytest.mark.parametrize("rows", [1, 8, 9, 16])
+@pytest.mark.parametrize("shape", [(201, 90, 10, 4112), (17, 0, 0, 16), (0, 33, 0, 48), (5, 3, 1, 1040)])
+def test_row_major_gemv_edges(shape, rows):
+    _check_linear(*shape, rows, torch.float16, bias=rows == 9)
+    _check_linear(*shape, rows, torch.bfloat16, bias=False)
+
+
+@pytest.mark.parametrize("rows,lead", [(1, ()), (3, (3,)), (8, (2, 2)), (5, ())])
+@pytest.mark.parametrize("shape", [(16, 16, 16, 64), (1328, 640, 80, 2560), (320, 160, 32, 9728)])
+def test_tiled_gemv_edges(shape, rows, lead):
+    """Fewer images than warp groups, tiles shared by groups and CTAs, bf16 rows."""
+    _check_linear(*shape, rows, torch.float16, bias=False, lead=lead)
+    _check_linear(*shape, rows, torch.bfloat16, bias=True, lead=lead)
+
+
+@pytest.mark.parametrize("k", [64, 2560, 6144, 12288])
+@pytest.mark.parametrize("rows", [1, 2, 5])
+def test_norm_prologue_edges(k, rows):
+    """The norm inside the GEMV with rows in registers and through shared memory: the same as the
+    separate kernel up to the order of the mean square's sum."""
+    if not rc.gemv_stages_x(rows, k):
+        pytest.skip("rows do not fit")
+    layer = random_packed_layer(64, 32, 16, k, seed=k)
+    mod = FusedMixedLinear.from_layer_data(layer, dict(zip(ORDER, (64, 32, 16))), k, "cuda")
+    gen = torch.Generator().manual_seed(k + rows)
+    x, d = (torch.randn(rows, k, generator=gen).half().cuda() for _ in range(2))
+    w = (1 + 0.1 * torch.randn(k, generator=gen)).half().cuda()
+    res = torch.empty_like(x)
+    y = rc.mixed_gemv_norm(x, d, w, 1e-6, mod._fd(), residual_out=res, flags=_lib.RDQ_GEMV_PDL)
+    assert torch.equal(y, rc.mixed_gemv_norm(x, d, w, 1e-6, mod._fd()))
+    h, r = torch.empty_like(x), x.clone()
+    rc.add_rmsnorm(r, d, w, h, 1e-6, 0)
+    assert torch.equal(res, r)
+    ref = rc.mixed_gemv(h, mod._fd()).float()
+    # a normalised value may move by one f16 step (2^-10 of it), twice (norm, weight)
+    w_abs = torch.from_numpy(np.abs(onp.dequantize_layer_f32(onp.torch_layer_to_np(layer), dict(zip(ORDER, (64, 32, 16))), k))).cuda()
+    assert bool(((y.float() - ref).abs() <= 2.0 ** -9 * (h.float().abs() @ w_abs.t()) + 2.0 ** -10 * ref.abs()).all())
+
+
+@pytest.mark.parametrize("b,nq,nkv,dh,s,pos_v", [
+    (1, 24, 2, 64, 40, 0),       # one row, twelve query heads per KV head
+    (1, 16, 1, 256, 300, 255),   # one KV head: most splits
+    (2, 32, 8, 128, 530, 512),   # the new row opens a block
+    (40, 16, 8, 64, 50, 47),     # more sequences than two CTAs per SM
+    (19, 32, 8, 128, 90, 77),    # one split per KV head, one wave
+])
+def test_single_token_attention_edges(b, nq, nkv, dh, s, pos_v):
+    gen = torch.Generator().manual_seed(b + nq + pos_v)
+    qkv = torch.randn(b, (nq + 2 * nkv) * dh, generator=gen).half().cuda()
+    k_cache, v_cache = (torch.randn(b, nkv, s, dh, generator=gen).half().cuda() for _ in range(2))
+    ang = torch.arange(s).float()[:, None] / 1e4 ** (torch.arange(0, dh, 2).float() / dh)[None, :]
+    cos, sin = (torch.cat([f(ang), f(ang)], -1).half().cuda() for f in (torch.cos, torch.sin))
+    pos = torch.tensor([pos_v], dtype=torch.long, device="cuda")
+    k1, v1 = k_cache.clone(), v_cache.clone()
+    q = torch.empty(b, nq, dh, dtype=torch.float16, device="cuda")
+    rc.qk_rope_cache(qkv, None, None, cos, sin, pos, q, k1, v1, 1e-6, 0)
+    scratch = rc.rope_attn_scratch(b, nq, nkv, dh, s, "cuda")
+    for flags in (0, _lib.RDQ_GEMV_PDL):
+        k2, v2 = k_cache.clone(), v_cache.clone()
+        out = torch.full((b, nq * dh), float("nan"), dtype=torch.float16, device="cuda")
+        rc.rope_attn_decode(qkv, None, None, cos, sin, pos, k2, v2, scratch, out, nq, dh ** -0.5, 1e-6, flags)
+        assert torch.equal(k2, k1) and torch.equal(v2, v1)
+        assert int(scratch.view(torch.int32).abs().sum()) == 0, "scratch not idle"
+        kd, vd = k1[:, :, :pos_v + 1].double(), v1[:, :, :pos_v + 1].double()
+        ref = F.scaled_dot_product_attention(q[:, :, None].double(), kd, vd, enable_gqa=True).reshape(b, nq * dh)
+        # scores are FP32 sums of dh products (and the exponential a few 2^-22): a relative error e of every
+        # weight moves the average by at most 2 e max |v|; the weights' own rounding is 2^-22; then f16
+        mags = (q.double().abs().amax() * kd.abs().amax() * dh * dh ** -0.5).item()
+        e = dh * 2.0 ** -24 * mags + 2.0 ** -20
+        assert bool(((out.double() - ref).abs() <= 2.0 ** -11 * ref.abs() + 2 * e * vd.abs().max()).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("n4,n8,n16,k", [(12, 0, 0, 32), (40, 25, 3, 16), (0, 70, 0, 528), (30, 20, 10, 1040), (600, 500, 0, 512),
+                                         (0, 0, 9, 48)])
+def test_layer_encoder_edges(n4, n8, n16, k, dtype):
+    """The whole layer in two launches: byte for byte the host route."""
+    n = n4 + n8 + n16
+    w = _special(dtype).repeat(2, 1)[:n] if k == 32 else _weights(n, k, n + k, dtype)
+    perm = torch.randperm(n, generator=torch.Generator().manual_seed(n))
+    splits = dict(zip(ORDER, (n4, n8, n16)))
+    host = pack_layer(quantize_weight(w, perm, splits), None)
+    dev = quantize_weight_packed(w.cuda(), perm, splits)
+    assert set(host) == set(dev)
+    for key in host:
+        a, b = host[key], dev[key].cpu()
+        assert a.dtype == b.dtype and torch.equal(a, b), key
