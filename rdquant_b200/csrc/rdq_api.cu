@@ -334,8 +334,6 @@ int rdq_gemm_mixed_ws(const void *x, int M, const void *w_fp4, const void *w_fp4
   a.n8 = n_fp8;
   a.n16 = n_fp16;
   a.K = K;
-  a.ksplit = 1;
-  a.partial = nullptr;
   RDQ_REQUIRE(workspace == nullptr || aligned16(workspace), RDQ_E_INVALID, "workspace must be 16-byte aligned");
   return launch_gemm(a, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
 }

@@ -7,13 +7,6 @@ namespace {
 // time-out self-test).  Read and cleared by gemm_status().
 __device__ int g_gemm_status;
 
-
-__device__ __forceinline__ uint32_t ldg_nc2(const void *p) {
-  uint16_t v;
-  asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p));
-  return v;
-}
-
 // Stage bookkeeping of one producer thread: before writing stage s of round ph it waits until
 // the MMA has released it; afterwards it makes its generic-proxy writes visible to the async
 // proxy and arrives on full[s].
@@ -51,7 +44,7 @@ __device__ __forceinline__ uint2 ldg_nc8(const void *p) {
 
 template <int NS, int SB, int TMAX, int PF>
 __device__ __forceinline__ void produce_rows(GemmSmem &S, const GemmArgs &a, uint32_t b_base, int pwarp, int nwarps,
-                                             int lane, int kb0, int nkb) {
+                                             int lane, int nkb) {
   const int chunk = lane & 7, sub = lane >> 3;
   const int nq = S.nquad;
   // per task: 32-bit byte offset of this lane's chunk from the format's weight tensor (the
@@ -109,9 +102,9 @@ __device__ __forceinline__ void produce_rows(GemmSmem &S, const GemmArgs &a, uin
 #pragma unroll
   for (int p = 0; p < PF; ++p) {
 #pragma unroll
-    for (int t = 0; t < TMAX; ++t) q[p][t] = (kb0 + p < nkb) ? load(t, kb0 + p) : make_uint4(0u, 0u, 0u, 0u);
+    for (int t = 0; t < TMAX; ++t) q[p][t] = (p < nkb) ? load(t, p) : make_uint4(0u, 0u, 0u, 0u);
   }
-  for (int kbase = kb0; kbase < nkb; kbase += PF) {
+  for (int kbase = 0; kbase < nkb; kbase += PF) {
 #pragma unroll
     for (int p = 0; p < PF; ++p) {
       const int kb = kbase + p;
@@ -165,10 +158,7 @@ gemm_mixed_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
   const int m0 = blockIdx.x * BM * MT;
   const int n0 = blockIdx.y * BN;
   const int N = a.n4 + a.n8 + a.n16;
-  // this CTA's k blocks [kb0, nkb): the whole K, or one of ksplit equal parts (blockIdx.z)
-  const int nkb_all = a.K / BK;
-  const int kb0 = static_cast<int>(1ll * blockIdx.z * nkb_all / a.ksplit);
-  const int nkb = static_cast<int>(1ll * (blockIdx.z + 1) * nkb_all / a.ksplit);
+  const int nkb = a.K / BK;
 
   if (tid == 32) {
     // the TMA unit reads the tensor map from memory: start that fetch now
@@ -234,7 +224,7 @@ gemm_mixed_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
     if (lane == 0) {
       bool alive = true;
       int s = 0, ph = 0;
-      for (int kb = kb0; kb < nkb && alive; ++kb) {
+      for (int kb = 0; kb < nkb && alive; ++kb) {
         if (ph > 0) alive = gemm_wait(&S.empty[s], (ph - 1) & 1, &S.abort_flag);
         if (!alive) break;
         const uint32_t full = smem_u32(&S.full[s]);
@@ -251,7 +241,7 @@ gemm_mixed_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
       constexpr uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(BN >> 3) << 17) | (static_cast<uint32_t>(BM >> 4) << 24);
       bool alive = true;
       int s = 0, ph = 0;
-      for (int kb = kb0; kb < nkb && alive; ++kb) {
+      for (int kb = 0; kb < nkb && alive; ++kb) {
         alive = gemm_wait(&S.full[s], ph & 1, &S.abort_flag);
         if (!alive) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -261,7 +251,7 @@ gemm_mixed_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
           const uint64_t da = make_desc_sw128(a_base + s * kStageAll + mt * kStageA);
 #pragma unroll
           for (int k4 = 0; k4 < BK / 16; ++k4)
-            umma_f16(tmem + mt * BN, da + 2 * k4, db + 2 * k4, idesc, (kb != kb0 || k4 != 0) ? 1u : 0u);
+            umma_f16(tmem + mt * BN, da + 2 * k4, db + 2 * k4, idesc, (kb != 0 || k4 != 0) ? 1u : 0u);
         }
         umma_commit(smem_u32(&S.empty[s]));
         if (++s == NS) { s = 0; ++ph; }
@@ -270,7 +260,7 @@ gemm_mixed_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
     }
   } else {
     // ------------------------------------------------------------- weight dequantisation
-    produce_rows<NS, SB, Cfg::kTasks, Cfg::kPrefetch>(S, a, b_base, warp - 2, Cfg::kProducerWarps, lane, kb0, nkb);
+    produce_rows<NS, SB, Cfg::kTasks, Cfg::kPrefetch>(S, a, b_base, warp - 2, Cfg::kProducerWarps, lane, nkb);
 
     // ----------------------------------------------------------------------- epilogue
     // A warp may read the tensor-memory lanes 32 (warp % 4) ...; the producer warps that share a
@@ -288,7 +278,7 @@ gemm_mixed_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
         for (int cp = sub; cp < MT * (BN / 64); cp += kEpiWarps / 4) {
           const int mt = cp / (BN / 64);
           const int m = m0 + mt * BM + q * 32 + lane;
-          const bool wide = a.ksplit == 1 && n0 + (cp % (BN / 64)) * 64 + 64 <= N && (N & 7) == 0;
+          const bool wide = n0 + (cp % (BN / 64)) * 64 + 64 <= N && (N & 7) == 0;
           const uint32_t stg = a_base + static_cast<uint32_t>(warp - 2) * (32 * kEpiPitch);
 #pragma unroll 1
           for (int hh = 0; hh < 2; ++hh) {
@@ -296,19 +286,7 @@ gemm_mixed_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
           uint32_t r[32];
           tmem_ld32(tmem + (static_cast<uint32_t>(q * 32) << 16) + mt * BN + cc * 32, r);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if (m < a.M && a.ksplit > 1) {
-            // split k range: raw FP32 sums go to this part's plane; scale, bias and the f16
-            // conversion happen in the reduction kernel
-            float *dst = a.partial + (1ll * blockIdx.z * a.M + m) * N + n0 + cc * 32;
-            if (n0 + cc * 32 + 32 <= N && (N & 3) == 0) {
-#pragma unroll
-              for (int v = 0; v < 8; ++v)
-                *reinterpret_cast<uint4 *>(dst + 4 * v) = make_uint4(r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]);
-            } else {
-              for (int e = 0; e < 32; ++e)
-                if (n0 + cc * 32 + e < N) dst[e] = __uint_as_float(r[e]);
-            }
-          } else if (wide) {
+          if (wide) {
             // Whole 64-channel pair: the warp turns its 32 rows x 128 B around in shared memory
             // (the stage buffers are free once the accumulators are complete) so that a store
             // instruction writes four rows x 128 contiguous bytes instead of 32 rows x 16 B:
@@ -363,24 +341,10 @@ gemm_mixed_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constan
                  : "memory");
   }
   if (tid == 0 && S.abort_flag) atomicExch(&g_gemm_status, 1);
-  if (a.test_timeout && tid == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {
+  if (a.test_timeout && tid == 0 && blockIdx.x == 0 && blockIdx.y == 0) {
     // Self-test of the time-out path: the tile is finished and nothing of this CTA is in flight;
     // wait (three suspended tries) on a barrier that nothing completes and report it.
     if (!mbar_wait(smem_u32(&S.never), 0, 3u)) atomicExch(&g_gemm_status, 2);
-  }
-}
-
-// y = f16(sum over parts * channel scale + bias) for a split launch
-__global__ void __launch_bounds__(256) gemm_reduce_kernel(const GemmArgs a, int N) {
-  const long long total = 1ll * a.M * N;
-  for (long long i = 1ll * blockIdx.x * blockDim.x + threadIdx.x; i < total; i += 1ll * gridDim.x * blockDim.x) {
-    const int n = static_cast<int>(i % N);
-    float v = 0.f;
-    for (int z = 0; z < a.ksplit; ++z) v += a.partial[z * total + i];
-    const int r = a.inv_perm ? a.inv_perm[n] : n;
-    const float scl = (r < a.n4) ? a.global4 : (r < a.n4 + a.n8 ? a.s8[r - a.n4] : 1.f);
-    const float bia = a.bias ? __half2float(a.bias[n]) : 0.f;
-    store_y(a.y, i, fmaf(v, scl, bia), a.y_bf16);
   }
 }
 
@@ -394,53 +358,33 @@ int launch_cfg(const CUtensorMap &xmap, const GemmArgs &a, int N, cudaStream_t s
     RDQ_CUDA(cudaFuncSetAttribute(gemm_mixed_kernel<MT, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
     if (dev >= 0 && dev < 64) attr_done[dev].store(true);
   }
-  const dim3 grid((a.M + MT * BM - 1) / (MT * BM), (N + BN - 1) / BN, a.ksplit);
+  const dim3 grid((a.M + MT * BM - 1) / (MT * BM), (N + BN - 1) / BN);
   gemm_mixed_kernel<MT, BN><<<grid, Cfg::kThreads, Cfg::kSmem, stream>>>(xmap, a);
   RDQ_CUDA(cudaGetLastError());
-  if (a.ksplit > 1) {
-    long long blocks = (1ll * a.M * N + 255) / 256;
-    if (blocks > 8ll * sm_count()) blocks = 8ll * sm_count();
-    gemm_reduce_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(a, N);
-    RDQ_CUDA(cudaGetLastError());
-  }
   return RDQ_OK;
 }
 
 }  // namespace
 
 namespace {
-// Tile configuration (0: 128 x 128, 1: 256 tokens x 128, 2: 256 x 256) and k split of a problem,
-// chosen by a small time estimate: waves of CTAs x work per CTA / efficiency of the
-// configuration.  Efficiencies are the measured throughputs of the three configurations on
-// large problems (424 / 715 / 921 TFLOP/s): wider tiles convert each weight byte for more
-// tokens.  Few tiles leave SMs idle for the whole launch: then up to four CTAs share a tile's
-// k range (as long as each keeps at least eight k blocks) and a second kernel adds their sums.
-struct GemmPlan {
-  int cfg, ksplit;
-};
-GemmPlan gemm_plan(int M, int N, int K) {
+// Tile configuration (0: 128 x 128, 1: 256 tokens x 128, 2: 256 x 256) of a problem, chosen by a
+// small time estimate: waves of CTAs x work per CTA / efficiency of the configuration.
+// Efficiencies are the measured throughputs of the three configurations on large problems
+// (424 / 715 / 921 TFLOP/s): wider tiles convert each weight byte for more tokens.
+int gemm_config(int M, int N) {
   const int sms = sm_count();
-  const int nkb = K / BK;
   const long long t256 = (M + 255) / 256, t128 = (M + 127) / 128;
   const long long n256 = (N + 255) / 256, n128 = (N + 127) / 128;
   const long long tiles[3] = {t128 * n128, t256 * n128, t256 * n256};
   const double area[3] = {128.0 * 128, 256.0 * 128, 256.0 * 256};
   const double eff[3] = {0.46, 0.78, 1.0};
-  GemmPlan best{0, 1};
+  int best = 0;
   double best_t = 0;
   for (int c = 0; c < 3; ++c) {
-    int split = 1;
-    if (tiles[c] * 2 <= sms) {
-      split = static_cast<int>(sms / tiles[c]);
-      if (split > 4) split = 4;
-      if (split > nkb / 8) split = nkb / 8;
-      if (split < 1) split = 1;
-    }
-    const long long waves = (tiles[c] * split + sms - 1) / sms;
-    const double t = waves * area[c] / eff[c] / split * (split > 1 ? 1.15 : 1.0);
+    const double t = (tiles[c] + sms - 1) / sms * area[c] / eff[c];
     if (c == 0 || t < best_t) {
       best_t = t;
-      best = GemmPlan{c, split};
+      best = c;
     }
   }
   return best;
@@ -525,11 +469,9 @@ int launch_gemm(const GemmArgs &a, void *workspace, size_t workspace_bytes, cuda
   CUtensorMap xmap;
   const int rc = encode_f16_2d(&xmap, a.x, a.K, a.M, BK, BM);
   if (rc != RDQ_OK) return rc;
-  const GemmPlan plan = gemm_plan(a.M, N, a.K);
-  b.ksplit = 1;
-  b.partial = nullptr;
-  if (plan.cfg == 2) return launch_cfg<2, 256>(xmap, b, N, stream);
-  if (plan.cfg == 1) return launch_cfg<2, 128>(xmap, b, N, stream);
+  const int cfg = gemm_config(a.M, N);
+  if (cfg == 2) return launch_cfg<2, 256>(xmap, b, N, stream);
+  if (cfg == 1) return launch_cfg<2, 128>(xmap, b, N, stream);
   return launch_cfg<1, 128>(xmap, b, N, stream);
 }
 

@@ -47,8 +47,6 @@ struct GemmArgs {
   void *y;
   int n4, n8, n16, K;
   int y_bf16 = 0;  // y is bf16 instead of f16
-  int ksplit;      // CTAs that share the k range of a tile (blockIdx.z); 1 = no split
-  float *partial;  // ksplit > 1: raw FP32 sums [ksplit][M][N], reduced by a second kernel
   int test_timeout = 0;  // self-test: CTA (0,0,0) ends with a wait that runs out
 };
 

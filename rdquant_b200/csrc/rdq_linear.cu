@@ -243,8 +243,6 @@ int rdq_linear(const rdq_layer *layer, const void *x, int x_type, int M, const v
   a.n16 = l.n_fp16;
   a.K = l.K;
   a.y_bf16 = bf16;
-  a.ksplit = 1;
-  a.partial = nullptr;
   if (p == Path::kStream) return launch_gemm_stream(a, rest, need.gemm, pdl, stream);
   return launch_gemm(a, rest, need.gemm, stream);
 }
