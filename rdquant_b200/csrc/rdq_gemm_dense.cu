@@ -51,6 +51,9 @@ struct DecodeArgs {
   int *counters;  // zeroed for the GEMM
   int n_counters;
   int n4, n8, N, K;
+  const uint4 *x_bf16;  // bf16 activations to round to f16 on the way (or null), in vectors of eight
+  uint4 *x;
+  long long x_vecs;
 };
 
 constexpr int kDecodeUnroll = 4;
@@ -61,6 +64,20 @@ __global__ void __launch_bounds__(256) decode_rows_kernel(DecodeArgs a) {
   const int lane = threadIdx.x & 31;
   const int gid = blockIdx.x * blockDim.x + threadIdx.x;
   for (int i = gid; i < a.n_counters; i += gridDim.x * blockDim.x) a.counters[i] = 0;
+  if (a.x_bf16) {  // (a launch of its own for these took 3 us)
+    const long long stride = 1ll * gridDim.x * blockDim.x;
+    for (long long i = gid; i < a.x_vecs; i += 4 * stride) {
+      uint4 v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (i + q * stride < a.x_vecs) v[q] = a.x_bf16[i + q * stride];
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (i + q * stride < a.x_vecs)
+          a.x[i + q * stride] =
+              make_uint4(bf16x2_to_f16x2(v[q].x), bf16x2_to_f16x2(v[q].y), bf16x2_to_f16x2(v[q].z), bf16x2_to_f16x2(v[q].w));
+    }
+  }
   const int K = a.K;
   const int nvec = K >> 3;  // runs of 8 k (the launcher requires K % 8 == 0)
   for (int j = gid >> 5; j < a.N; j += (gridDim.x * blockDim.x) >> 5) {
@@ -554,6 +571,9 @@ int launch_gemm_dense(const GemmArgs &g, void *workspace, size_t workspace_bytes
   d.n8 = g.n8;
   d.N = N;
   d.K = g.K;
+  d.x_bf16 = static_cast<const uint4 *>(g.x_bf16);
+  d.x = reinterpret_cast<uint4 *>(const_cast<__half *>(g.x));
+  d.x_vecs = 1ll * g.M * g.K / 8;
 
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -562,8 +582,9 @@ int launch_gemm_dense(const GemmArgs &g, void *workspace, size_t workspace_bytes
   cfg.stream = stream;
   cfg.blockDim = dim3(256);
   cfg.gridDim = dim3(static_cast<unsigned>(std::min(8 * sm_count(), (N + 7) / 8)));
-  decode_rows_kernel<<<cfg.gridDim, cfg.blockDim, 0, stream>>>(d);
-  RDQ_CUDA(cudaGetLastError());
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  RDQ_CUDA(cudaLaunchKernelEx(&cfg, decode_rows_kernel, d));
 
   int *status = nullptr;
   int rc = gemm_status_ptr(&status);
@@ -602,8 +623,6 @@ int launch_gemm_dense(const GemmArgs &g, void *workspace, size_t workspace_bytes
   cfg.gridDim = dim3(static_cast<unsigned>(2 * p.clusters));
   cfg.blockDim = dim3(kPairThreads);
   cfg.dynamicSmemBytes = kPairSmem;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
   void *params[4] = {&xmap, &wmap, &a, &status};
   RDQ_CUDA(cudaLaunchKernelExC(&cfg, fn, params));
   return RDQ_OK;

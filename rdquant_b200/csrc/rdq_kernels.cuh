@@ -32,6 +32,7 @@ struct GemvArgs {
 };
 
 struct GemmArgs {
+  const void *x_bf16 = nullptr;  // bf16 rows to be rounded into x first (launch_gemm with a workspace)
   const __half *x;
   int M;
   const uint8_t *w4;

@@ -193,7 +193,11 @@ int rdq_linear(const rdq_layer *layer, const void *x, int x_type, int M, const v
   bool pdl = (flags & RDQ_GEMV_PDL) != 0;
   const void *xh = x;
   int x_bf16 = bf16;
-  if (need.cast) {
+  // (the decoded-once GEMM's first launch rounds the rows itself)
+  const bool cast_inside = need.cast && p == Path::kGemm && aligned16(x);
+  if (cast_inside) {
+    xh = workspace;
+  } else if (need.cast) {
     const int rc = launch_cast_rows(x, workspace, 1ll * M * l.K, pdl, stream);
     if (rc != RDQ_OK) return rc;
     xh = workspace;
@@ -243,6 +247,7 @@ int rdq_linear(const rdq_layer *layer, const void *x, int x_type, int M, const v
   a.n16 = l.n_fp16;
   a.K = l.K;
   a.y_bf16 = bf16;
+  if (cast_inside) a.x_bf16 = x;
   if (p == Path::kStream) return launch_gemm_stream(a, rest, need.gemm, pdl, stream);
   return launch_gemm(a, rest, need.gemm, stream);
 }
