@@ -58,17 +58,18 @@ int stream_from(const rdq_layer &l) {
 // The streaming GEMM converts the weights once more per 128 rows, the other GEMM decodes them once:
 // estimates in microseconds that agree with measurements between 65 and 2048 rows on seven layer
 // shapes within 15 %.  (With up to 64 rows the streaming GEMM was faster on all of them.)
-bool stream_beats_dense(const rdq_layer &l, int M) {
+bool stream_beats_dense(const rdq_layer &l, int M, int x_type) {
   if (M <= 64) return true;
   if (M > 2048) return false;
   const int N = l.n_fp4 + l.n_fp8 + l.n_fp16;
   const double weights = 1e-6 * N * l.K;
-  return 15.5 + 1.62e-3 * M * weights < 4.5 + 0.6 * weights + gemm_dense_cycles(M, N, l.K) / 1750.0;
+  const double cast = x_type == RDQ_BF16 ? 2.5 : 0.0;  // the other GEMM's decoding launch rounds bf16 rows along the way
+  return cast + 15.5 + 1.62e-3 * M * weights < 4.0 + 0.6 * weights + gemm_dense_cycles(M, N, l.K) / 1750.0;
 }
 
-Path path_of(const rdq_layer &l, int M) {
+Path path_of(const rdq_layer &l, int M, int x_type) {
   const bool can_stream = gemm_stream_takes(l.K) && has_row_major(l) && l.gemv_counters && (l.perm || !l.inv_perm);
-  if (can_stream && M >= stream_from(l) && (!gemm_dense_takes(l.K) || stream_beats_dense(l, M))) return Path::kStream;
+  if (can_stream && M >= stream_from(l) && (!gemm_dense_takes(l.K) || stream_beats_dense(l, M, x_type))) return Path::kStream;
   if (M <= RDQ_MAX_GEMV_M) return l.w_tiled ? Path::kGemvTiled : Path::kGemvGeneric;
   if (gemm_dense_takes(l.K) && has_row_major(l)) return Path::kGemm;
   return l.w_tiled ? Path::kPanelsTiled : Path::kPanelsGeneric;
@@ -137,7 +138,7 @@ int run_gemv(const rdq_layer &l, bool tiled, const void *x, int x_bf16, int M, c
 
 }  // namespace
 
-int launch_cast_rows(const void *x_bf16, void *x_f16, long long count, bool pdl, cudaStream_t stream) {
+int launch_cast_rows(const void *x_bf16, void *x_f16, long long count, cudaStream_t stream) {
   if (count == 0) return RDQ_OK;
   const bool vec = count % 8 == 0 && aligned16(x_bf16) && aligned16(x_f16);
   const long long per = vec ? 8 * 256 : 256;
@@ -150,7 +151,7 @@ int launch_cast_rows(const void *x_bf16, void *x_f16, long long count, bool pdl,
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;  // (the kernels wait before they read)
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   if (vec) {
@@ -171,7 +172,7 @@ extern "C" {
 
 int rdq_linear_workspace_size(const rdq_layer *layer, int M, int x_type, size_t *bytes) {
   RDQ_REQUIRE(layer && bytes && M >= 0, RDQ_E_INVALID, "bad arguments to rdq_linear_workspace_size");
-  const Need n = need_of(*layer, path_of(*layer, M), M, x_type);
+  const Need n = need_of(*layer, path_of(*layer, M, x_type), M, x_type);
   *bytes = n.cast + n.gemm;
   return RDQ_OK;
 }
@@ -183,7 +184,7 @@ int rdq_linear(const rdq_layer *layer, const void *x, int x_type, int M, const v
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   const int N = l.n_fp4 + l.n_fp8 + l.n_fp16;
   if (M == 0 || N == 0) return RDQ_OK;
-  const Path p = path_of(l, M);
+  const Path p = path_of(l, M, x_type);
   RDQ_REQUIRE(l.w_tiled || has_row_major(l), RDQ_E_INVALID, "the layer has neither the tiled nor the row-major tensors");
   RDQ_REQUIRE(x && y, RDQ_E_INVALID, "x and y must not be null");
   const Need need = need_of(l, p, M, x_type);
@@ -198,7 +199,7 @@ int rdq_linear(const rdq_layer *layer, const void *x, int x_type, int M, const v
   if (cast_inside) {
     xh = workspace;
   } else if (need.cast) {
-    const int rc = launch_cast_rows(x, workspace, 1ll * M * l.K, pdl, stream);
+    const int rc = launch_cast_rows(x, workspace, 1ll * M * l.K, stream);
     if (rc != RDQ_OK) return rc;
     xh = workspace;
     x_bf16 = 0;
