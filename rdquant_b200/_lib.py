@@ -46,6 +46,8 @@ NVCC_FLAGS = [
 RDQ_GEMV_AUTO = 0
 RDQ_GEMV_GENERIC = 1
 RDQ_GEMV_PDL = 16
+RDQ_GEMV_OPENS = 32
+RDQ_GEMV_BESIDE = 128
 RDQ_GEMV_TEST_TIMEOUT = 64
 
 RDQ_E_DEVICE = -4

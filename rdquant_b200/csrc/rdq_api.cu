@@ -165,6 +165,8 @@ int rdq_gemv_tiled(const void *x, int M, const void *w_tiled, const float *w_fp8
   a.workspace = static_cast<float *>(workspace);
   a.flags = counters;
   a.test_timeout = (flags & RDQ_GEMV_TEST_TIMEOUT) ? 1 : 0;
+  a.opens = (flags & RDQ_GEMV_PDL) && (flags & RDQ_GEMV_OPENS);
+  a.beside = (flags & RDQ_GEMV_PDL) && (flags & RDQ_GEMV_BESIDE);
   return launch_gemv_tiled(a, (flags & RDQ_GEMV_PDL) != 0, static_cast<cudaStream_t>(stream));
 }
 

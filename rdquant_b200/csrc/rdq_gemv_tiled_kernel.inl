@@ -82,6 +82,8 @@ struct TiledArgs {
   int slot_bytes;
   int fdepth;  // slots per hand-over ring
   int early;         // weights may be read before the kernel before this one has finished
+  int opens;         // let the next kernel start only when that kernel has finished
+  int beside;        // everything may be: wait for it at the end
   int test_timeout;  // self-test: CTA 0 ends with a wait that runs out
   // Peer mode (column-parallel layers): the outputs go to n_dst destinations -- one slice of a
   // gather buffer on every GPU of the node, this one included, written with plain stores over
@@ -330,7 +332,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
 
   // Let the next kernel in the stream become resident as early as possible; until this
   // grid completes it only fills its own shared-memory ring with weights.
-  pdl_launch_dependents();
+  if (!a.opens) pdl_launch_dependents();
   if (static_cast<int>(blockIdx.x) >= sc.G) {
     // The grid has a CTA for every SM: one without images holds its place until the kernel before is
     // done, so that the next launch finds one free place per SM, not two on some.
@@ -380,7 +382,8 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
     if (lane != 0) return;
     // Only this thread executes the grid-dependency wait; every other warp of the CTA
     // sleeps on bar_x, which completes after it (and after the activation copies).
-    pdl_wait();
+    if (!a.beside) pdl_wait();
+    if (a.opens) pdl_launch_dependents();
     const uint32_t bx = smem_u32(&bar_x);
     if (XS && (!EXTRA || xop == 0)) {
       mbar_arrive_expect_tx(bx, static_cast<uint32_t>(M) * 2u * K);
@@ -412,6 +415,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
         }
       }
     }
+    if (a.beside) pdl_wait();  // launches that wait for this one rely on the one before as well
     return;
   }
 
@@ -1058,6 +1062,8 @@ int launch_gemv_tiled(const GemvTiledArgs &h, bool pdl, cudaStream_t stream) {
   a.bias = h.bias; a.y = h.y; a.n4 = h.n4; a.n8 = h.n8; a.n16 = h.n16; a.K = h.K;
   a.workspace = h.workspace; a.flags = h.flags;
   a.early = pdl;
+  a.opens = h.opens;
+  a.beside = h.beside;
   a.test_timeout = h.test_timeout;
   a.n_dst = h.n_dst;
   for (int d = 0; d < kMaxPeers; ++d) {

@@ -77,6 +77,7 @@ struct GemvTiledArgs {
   float *workspace;
   int32_t *flags;
   int test_timeout = 0;  // RDQ_GEMV_TEST_TIMEOUT
+  int opens = 0, beside = 0;  // RDQ_GEMV_OPENS, RDQ_GEMV_BESIDE
   // peer mode (see TiledArgs): destinations, this rank's flag word on every GPU, local state
   int n_dst = 0;
   __half *dst[kMaxPeers] = {};

@@ -9,7 +9,7 @@ from conftest import ORDER
 from oracle import oracle_np as onp
 from rdquant_b200 import _lib
 from rdquant_b200 import rdquant_cuda as rc
-from rdquant_b200.inference import FusedMixedLinear
+from rdquant_b200.inference import FusedMixedLinear, GraphedDecodeStep
 from rdquant_b200.integrations.hf_export import pack_layer
 from rdquant_b200.quantize import quantize_weight, quantize_weight_packed
 from rdquant_b200.synthetic import random_packed_layer
@@ -151,3 +151,22 @@ def test_layer_encoder_edges(n4, n8, n16, k, dtype):
     for key in host:
         a, b = host[key], dev[key].cpu()
         assert a.dtype == b.dtype and torch.equal(a, b), key
+
+
+@pytest.mark.parametrize("m,twice", [(1, False), (8, False), (2, True)])
+def test_graphed_step_layers_beside_each_other(m, twice):
+    """Layers of very different sizes that run beside each other, inputs changing from step to step; with a
+    layer twice in the list (shared scratch) one after another."""
+    shapes = [(16, 16, 0, 64), (2048, 1024, 128, 2560), (64, 32, 16, 9728), (4096, 2048, 0, 1024)]
+    mods = [FusedMixedLinear.from_layer_data(random_packed_layer(*s, seed=s[3]), dict(zip(ORDER, s[:3])), s[3], "cuda") for s in shapes]
+    if twice:
+        mods = mods[:2] + mods[1:2]
+    step = GraphedDecodeStep(mods, m=m)
+    gen = torch.Generator().manual_seed(m)
+    for _ in range(12):
+        xs = [torch.randn(m, mod.K, generator=gen).half() for mod in mods]
+        for buf, x in zip(step.x_host, xs):
+            buf.copy_(x)
+        out = [y.clone() for y in step.run()]
+        for mod, x, y in zip(mods, xs, out):
+            assert torch.equal(y, rc.mixed_gemv(x.cuda(), mod._fd()).cpu())
