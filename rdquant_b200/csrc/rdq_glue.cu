@@ -29,43 +29,72 @@ __device__ __forceinline__ float block_sum(float v, float *smem) {
   return warp_sum(t);
 }
 
+__device__ __forceinline__ void prefetch_l2(const void *p, int bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
 // ---- x (+= delta); out = rmsnorm(x) * w.  One CTA per row.
+// Bound: latency.  The first kNormVecs vectors of a thread (8192 values of a row: more than the models
+// this serves have) stay in registers between the sum and the product, and their norm weights are
+// loaded beside them: one round trip to memory per row instead of one per vector and pass.  With the
+// loads of silu_mul_kernel ahead likewise: 4 blocks of 32 rows x 2560 323.7 -> 318.8 us.
+constexpr int kNormVecs = 4;
+
 __global__ void __launch_bounds__(256) add_rmsnorm_kernel(__half *x, const __half *delta, const __half *w, __half *out,
                                                          int B, int H, float eps) {
   __shared__ float red[32];
   pdl_launch_dependents();
+  if (blockIdx.x == 0 && threadIdx.x == 0) prefetch_l2(w, H * 2);  // a hint while the kernel before runs
   pdl_wait();
   if (static_cast<int>(blockIdx.x) >= B) {  // the grid has a CTA per SM (see linger())
     linger(1500);
     return;
   }
-  __half *xr = x + 1ll * blockIdx.x * H;
-  const __half *dr = delta ? delta + 1ll * blockIdx.x * H : nullptr;
+  const int n8 = H / 8, tail = kNormVecs * static_cast<int>(blockDim.x);
+  uint4 *xr = reinterpret_cast<uint4 *>(x + 1ll * blockIdx.x * H);
+  const uint4 *dr = reinterpret_cast<const uint4 *>(delta ? delta + 1ll * blockIdx.x * H : nullptr);
+  const uint4 *w8 = reinterpret_cast<const uint4 *>(w);
   float ss = 0.f;
-  for (int i = threadIdx.x; i < H / 8; i += blockDim.x) {
-    uint4 v = reinterpret_cast<const uint4 *>(xr)[i];
+  auto add_and_sum = [&](uint4 &v, const uint4 &d, int i) {
     __half2 *h = reinterpret_cast<__half2 *>(&v);
     if (dr) {
-      const uint4 d = reinterpret_cast<const uint4 *>(dr)[i];
       const __half2 *dh = reinterpret_cast<const __half2 *>(&d);
 #pragma unroll
       for (int j = 0; j < 4; ++j) h[j] = __hadd2(h[j], dh[j]);
-      reinterpret_cast<uint4 *>(xr)[i] = v;
+      xr[i] = v;
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const float2 f = __half22float2(h[j]);
       ss += f.x * f.x + f.y * f.y;
     }
+  };
+  uint4 v[kNormVecs], d[kNormVecs], wv[kNormVecs];
+#pragma unroll
+  for (int u = 0; u < kNormVecs; ++u) {
+    const int i = u * blockDim.x + threadIdx.x;
+    if (i < n8) {
+      v[u] = xr[i];
+      if (dr) d[u] = dr[i];
+      wv[u] = w8[i];
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kNormVecs; ++u) {
+    const int i = u * blockDim.x + threadIdx.x;
+    if (i < n8) add_and_sum(v[u], d[u], i);
+  }
+  for (int i = tail + threadIdx.x; i < n8; i += blockDim.x) {
+    uint4 vt = xr[i], dt = make_uint4(0, 0, 0, 0);
+    if (dr) dt = dr[i];
+    add_and_sum(vt, dt, i);
   }
   ss = block_sum(ss, red);
   const float rs = rsqrtf(ss / H + eps);
-  __half *orow = out + 1ll * blockIdx.x * H;
-  for (int i = threadIdx.x; i < H / 8; i += blockDim.x) {
-    const uint4 v = reinterpret_cast<const uint4 *>(xr)[i];
-    const uint4 wv = reinterpret_cast<const uint4 *>(w)[i];
-    const __half2 *h = reinterpret_cast<const __half2 *>(&v);
-    const __half2 *wh = reinterpret_cast<const __half2 *>(&wv);
+  uint4 *orow = reinterpret_cast<uint4 *>(out + 1ll * blockIdx.x * H);
+  auto scaled = [&](const uint4 &vv, const uint4 &ww) {
+    const __half2 *h = reinterpret_cast<const __half2 *>(&vv);
+    const __half2 *wh = reinterpret_cast<const __half2 *>(&ww);
     uint4 o;
     __half2 *oh = reinterpret_cast<__half2 *>(&o);
 #pragma unroll
@@ -73,8 +102,14 @@ __global__ void __launch_bounds__(256) add_rmsnorm_kernel(__half *x, const __hal
       const float2 f = __half22float2(h[j]);
       oh[j] = __hmul2(__floats2half2_rn(f.x * rs, f.y * rs), wh[j]);
     }
-    reinterpret_cast<uint4 *>(orow)[i] = o;
+    return o;
+  };
+#pragma unroll
+  for (int u = 0; u < kNormVecs; ++u) {
+    const int i = u * blockDim.x + threadIdx.x;
+    if (i < n8) orow[i] = scaled(v[u], wv[u]);
   }
+  for (int i = tail + threadIdx.x; i < n8; i += blockDim.x) orow[i] = scaled(xr[i], w8[i]);
 }
 
 // ---- per head: (q, k) RMSNorm over head_dim (optional), rotary embedding, q -> q_out, k / v -> cache
@@ -218,22 +253,40 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const __half *gu, __half 
     linger(1500);
     return;
   }
-  for (long long i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-    const int b = static_cast<int>(i / (F / 8)), j = static_cast<int>(i - 1ll * b * (F / 8));
-    const uint4 g = reinterpret_cast<const uint4 *>(gu + 2ll * b * F)[j];
-    const uint4 u = reinterpret_cast<const uint4 *>(gu + 2ll * b * F + F)[j];
-    const __half2 *gh = reinterpret_cast<const __half2 *>(&g);
-    const __half2 *uh = reinterpret_cast<const __half2 *>(&u);
-    uint4 o;
-    __half2 *oh = reinterpret_cast<__half2 *>(&o);
+  // Two vectors per turn, their loads ahead of the arithmetic: at 32 rows of 9728 a share is 263
+  // vectors for 256 threads.  Rows by a 32-bit division of the distance from the share's first row.
+  const unsigned f8 = static_cast<unsigned>(F / 8), n = static_cast<unsigned>(hi - lo);
+  const long long row0 = lo / f8;
+  const unsigned off0 = static_cast<unsigned>(lo - row0 * f8);
+  for (unsigned i = threadIdx.x; i < n; i += 2 * blockDim.x) {
+    uint4 gv[2], uv[2], *dst[2];
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const float2 a = __half22float2(gh[t]), c = __half22float2(uh[t]);
-      // silu in FP32, rounded to FP16 before the product like the framework's two kernels
-      const __half2 s = __floats2half2_rn(silu(a.x), silu(a.y));
-      oh[t] = __hmul2(s, __floats2half2_rn(c.x, c.y));
+    for (int k = 0; k < 2; ++k) {
+      const unsigned e = i + k * blockDim.x;
+      if (e < n) {
+        const unsigned r = (off0 + e) / f8, j = off0 + e - r * f8;
+        const long long b = row0 + r;
+        gv[k] = reinterpret_cast<const uint4 *>(gu + 2 * b * F)[j];
+        uv[k] = reinterpret_cast<const uint4 *>(gu + 2 * b * F + F)[j];
+        dst[k] = reinterpret_cast<uint4 *>(out + b * F) + j;
+      }
     }
-    reinterpret_cast<uint4 *>(out + 1ll * b * F)[j] = o;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      if (i + k * blockDim.x >= n) break;
+      const __half2 *gh = reinterpret_cast<const __half2 *>(&gv[k]);
+      const __half2 *uh = reinterpret_cast<const __half2 *>(&uv[k]);
+      uint4 o;
+      __half2 *oh = reinterpret_cast<__half2 *>(&o);
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const float2 a = __half22float2(gh[t]), c = __half22float2(uh[t]);
+        // silu in FP32, rounded to FP16 before the product like the framework's two kernels
+        const __half2 s = __floats2half2_rn(silu(a.x), silu(a.y));
+        oh[t] = __hmul2(s, __floats2half2_rn(c.x, c.y));
+      }
+      *dst[k] = o;
+    }
   }
 }
 
@@ -298,9 +351,6 @@ __device__ __forceinline__ void st_relaxed(float *p, float v) {
   asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
 }
 __device__ __forceinline__ bool is_idle(float v) { return __float_as_uint(v) == 0u; }
-__device__ __forceinline__ void prefetch_l2(const void *p, int bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
 
 // NB: blocks of eight query heads per KV head
 template <int DH, int NB>

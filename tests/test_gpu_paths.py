@@ -170,3 +170,32 @@ def test_graphed_step_layers_beside_each_other(m, twice):
         out = [y.clone() for y in step.run()]
         for mod, x, y in zip(mods, xs, out):
             assert torch.equal(y, rc.mixed_gemv(x.cuda(), mod._fd()).cpu())
+
+
+@pytest.mark.parametrize("rows,h", [(1, 8), (33, 2048), (2, 8192), (3, 8200), (200, 16392)])
+@pytest.mark.parametrize("with_delta", [False, True])
+def test_add_rmsnorm_row_lengths(rows, h, with_delta):
+    """Rows shorter than a turn of the block, as long as its registers hold, and longer."""
+    gen = torch.Generator().manual_seed(rows + h)
+    x, d = (torch.randn(rows, h, generator=gen).half().cuda() for _ in range(2))
+    w = (1 + 0.1 * torch.randn(h, generator=gen)).half().cuda()
+    xs = x + d if with_delta else x.clone()
+    xd = xs.double()
+    ref = xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-6) * w.double()
+    out = torch.empty_like(x)
+    rc.add_rmsnorm(x, d if with_delta else None, w, out, 1e-6)
+    assert torch.equal(x, xs)
+    # two roundings to f16 (2^-11 each; 2^-24 where subnormal) and an FP32 sum far below them
+    assert bool(((out.double() - ref).abs() <= 2.1 * 2.0 ** -11 * ref.abs() + 2.0 ** -23).all())
+
+
+@pytest.mark.parametrize("rows,f", [(1, 8), (32, 9728), (148, 2048), (148, 2056), (295, 4104)])
+def test_silu_mul_shares(rows, f):
+    """Shares of a CTA of nothing, of one turn, of a turn and one, and of several with rows that end in them."""
+    gu = torch.randn(rows, 2 * f, generator=torch.Generator().manual_seed(rows + f)).half().cuda()
+    out = torch.empty(rows, f, dtype=torch.float16, device="cuda")
+    rc.silu_mul(gu, out)
+    g, u = gu[:, :f].double(), gu[:, f:].double()
+    ref = g * torch.sigmoid(g) * u
+    # silu and product each rounded to f16; a subnormal silu is off by 2^-25, times u
+    assert bool(((out.double() - ref).abs() <= 2.1 * 2.0 ** -11 * ref.abs() + 2.0 ** -25 * (u.abs() + 1)).all())
