@@ -60,7 +60,6 @@ constexpr int kDecodeUnroll = 4;
 
 __global__ void __launch_bounds__(256) decode_rows_kernel(DecodeArgs a) {
   pdl_launch_dependents();
-  pdl_wait();  // the scratch may be in use by the kernel before
   const int lane = threadIdx.x & 31;
   const int gid = blockIdx.x * blockDim.x + threadIdx.x;
   for (int i = gid; i < a.n_counters; i += gridDim.x * blockDim.x) a.counters[i] = 0;
@@ -582,8 +581,9 @@ int launch_gemm_dense(const GemmArgs &g, void *workspace, size_t workspace_bytes
   cfg.stream = stream;
   cfg.blockDim = dim3(256);
   cfg.gridDim = dim3(static_cast<unsigned>(std::min(8 * sm_count(), (N + 7) / 8)));
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  // In stream order, not overlapping the kernel before: calls that follow one another would chain GEMMs
+  // without an end, and with fewer clusters than SM pairs the next call's clusters start beside this
+  // one's.  Such a chain of 200 rows x 4560 -> 7017 stopped making progress after some hundred calls.
   RDQ_CUDA(cudaLaunchKernelEx(&cfg, decode_rows_kernel, d));
 
   int *status = nullptr;
@@ -623,6 +623,8 @@ int launch_gemm_dense(const GemmArgs &g, void *workspace, size_t workspace_bytes
   cfg.gridDim = dim3(static_cast<unsigned>(2 * p.clusters));
   cfg.blockDim = dim3(kPairThreads);
   cfg.dynamicSmemBytes = kPairSmem;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
   void *params[4] = {&xmap, &wmap, &a, &status};
   RDQ_CUDA(cudaLaunchKernelExC(&cfg, fn, params));
   return RDQ_OK;

@@ -57,7 +57,7 @@ int launch_dequant(const void *w_fp4, const void *w_fp4_scales, float global4, c
                    int K, cudaStream_t stream);
 
 // bf16 -> f16, count % 8 == 0, both 16-byte aligned
-int launch_cast_rows(const void *x_bf16, void *x_f16, long long count, cudaStream_t stream);
+int launch_cast_rows(const void *x_bf16, void *x_f16, long long count, bool pdl, cudaStream_t stream);
 
 int launch_gemv_generic(const GemvArgs &a, cudaStream_t stream);
 

@@ -138,7 +138,7 @@ int run_gemv(const rdq_layer &l, bool tiled, const void *x, int x_bf16, int M, c
 
 }  // namespace
 
-int launch_cast_rows(const void *x_bf16, void *x_f16, long long count, cudaStream_t stream) {
+int launch_cast_rows(const void *x_bf16, void *x_f16, long long count, bool pdl, cudaStream_t stream) {
   if (count == 0) return RDQ_OK;
   const bool vec = count % 8 == 0 && aligned16(x_bf16) && aligned16(x_f16);
   const long long per = vec ? 8 * 256 : 256;
@@ -151,7 +151,7 @@ int launch_cast_rows(const void *x_bf16, void *x_f16, long long count, cudaStrea
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;  // (the kernels wait before they read)
+  attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   if (vec) {
@@ -199,7 +199,7 @@ int rdq_linear(const rdq_layer *layer, const void *x, int x_type, int M, const v
   if (cast_inside) {
     xh = workspace;
   } else if (need.cast) {
-    const int rc = launch_cast_rows(x, workspace, 1ll * M * l.K, stream);
+    const int rc = launch_cast_rows(x, workspace, 1ll * M * l.K, pdl, stream);
     if (rc != RDQ_OK) return rc;
     xh = workspace;
     x_bf16 = 0;
