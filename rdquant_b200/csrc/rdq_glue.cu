@@ -305,11 +305,10 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const __half *gu, __half 
 //      eight query heads as columns: S^T = K Q^T, online softmax per block, O^T += V^T P^T.  P goes in
 //      as the sum of two FP16 values, so that its rounding (2^-22) stays below FP32 products' sums.
 //   4. the warps' (max, sum, values) are merged in shared memory; with one split that is the result.
-//      Else every CTA stores its partial sums in scratch, and CTA `split` of a (sequence, KV head) merges
-//      the query heads split, split + splits, ...: it polls the words it needs until they differ from
-//      zero (a sum that is zero is stored as -0), adds them in split order and puts zeros back, so that
-//      the scratch is idle again when the launch ends.  The last CTA to arrive merging all heads, behind
-//      a fence and a counter, took 4 us of a 9.5 us launch (one sequence of 512 rows).
+//      Else every CTA stores its partial sums in scratch and counts itself, and the CTA that counts last
+//      merges the heads of its (sequence, KV head), a warp per head, the loads of all splits in flight, in
+//      split order.  Nobody waits, so nothing relies on the CTAs of a launch running at the same time.
+//      The words it read and the count go back to zero.
 // Under programmatic launch the norm weights, the rotary rows and the cache rows are asked into L2 while
 // the kernel before this one runs (a position that is out of date costs no more than the hint).
 // Bound: HBM (K and V rows once) for many sequences, latency for one.  The scalar kernel before (a
@@ -317,7 +316,7 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const __half *gu, __half 
 // (92 MB).
 constexpr int kFusedAttnWarps = 4;
 constexpr int kFusedAttnThreads = kFusedAttnWarps * 32;
-constexpr int kFusedAttnMaxSplit = 16;  // values a thread of the merge has in flight
+constexpr int kFusedAttnMaxSplit = 16;  // vectors a lane of the merge has in flight
 
 // 16 bytes, or zeros
 __device__ __forceinline__ void cp_async16_if(uint32_t dst, const void *src, bool valid) {
@@ -340,24 +339,41 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t v) {
   return r;
 }
 
-// a partial sum as a word that differs from an idle word
-__device__ __forceinline__ float not_idle(float v) { return __float_as_uint(v) == 0u ? -0.f : v; }
-__device__ __forceinline__ float ld_relaxed(const float *p) {
-  float v;
-  asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
-  return v;
+// N consecutive floats (2, 4 or 8, aligned to 8 or 16 bytes) past L1
+template <int N>
+__device__ __forceinline__ void ldcg_floats(const float *p, float (&v)[N]) {
+  if (N == 2) {
+    const float2 t = __ldcg(reinterpret_cast<const float2 *>(p));
+    v[0] = t.x;
+    v[1] = t.y;
+  } else {
+#pragma unroll
+    for (int i = 0; i < N / 4; ++i) {
+      const float4 t = __ldcg(reinterpret_cast<const float4 *>(p) + i);
+      v[4 * i] = t.x;
+      v[4 * i + 1] = t.y;
+      v[4 * i + 2] = t.z;
+      v[4 * i + 3] = t.w;
+    }
+  }
 }
-__device__ __forceinline__ void st_relaxed(float *p, float v) {
-  asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
+template <int N>
+__device__ __forceinline__ void stcg_floats(float *p, const float (&v)[N]) {
+  if (N == 2) {
+    __stcg(reinterpret_cast<float2 *>(p), make_float2(v[0], v[1]));
+  } else {
+#pragma unroll
+    for (int i = 0; i < N / 4; ++i)
+      __stcg(reinterpret_cast<float4 *>(p) + i, make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]));
+  }
 }
-__device__ __forceinline__ bool is_idle(float v) { return __float_as_uint(v) == 0u; }
 
 // NB: blocks of eight query heads per KV head
 template <int DH, int NB>
 __global__ void __launch_bounds__(kFusedAttnThreads, 2) rope_attn_kernel(
     const __half *qkv, const __half *qn, const __half *kn, const __half *cos_t, const __half *sin_t, const long long *pos,
-    __half *k_cache, __half *v_cache, float *part, __half *out, int nq, int nkv, int S, float scale, float eps, int nsplit,
-    int npair) {
+    __half *k_cache, __half *v_cache, float *part, int *counters, __half *out, int nq, int nkv, int S, float scale, float eps,
+    int nsplit, int npair) {
   constexpr int W = kFusedAttnWarps;
   constexpr int PITCH = 2 * DH + 16;   // row pitch in shared memory (bytes): an odd multiple of 16
   constexpr int BLK = 16 * PITCH;      // 16 rows of K or of V
@@ -659,55 +675,51 @@ __global__ void __launch_bounds__(kFusedAttnThreads, 2) rope_attn_kernel(
       for (int j = 0; j < DPL; ++j) o[j] = __float2half_rn(a[j] * inv);
     } else {
       float *dst = part + ((1ll * b * nq + head) * nsplit + split) * PR;
-      if (lane == 0) {
-        st_relaxed(dst, not_idle(m));
-        st_relaxed(dst + 1, not_idle(l));
-      }
-#pragma unroll
-      for (int j = 0; j < DPL; ++j) st_relaxed(dst + 4 + lane * DPL + j, not_idle(a[j]));
+      if (lane == 0) __stcg(reinterpret_cast<float2 *>(dst), make_float2(m, l));
+      stcg_floats(dst + 4 + lane * DPL, a);
     }
   }
   if (used == 1) return;
-  for (int hq = split; hq < group; hq += used) {
+  __shared__ int last;
+  __syncthreads();
+  if (tid == 0) {
+    __threadfence();
+    last = atomicAdd(&counters[pair], 1) == used - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last) return;
+  if (tid == 0) counters[pair] = 0;
+  for (int hq = warp; hq < group; hq += W) {
     const int head = kvh * group + hq;
     float *src = part + (1ll * b * nq + head) * nsplit * PR;
-    // lane s: the (max, sum) of split s; thread: dimension tid (+ 128) of every split.  All loads first.
-    float ms = lane < used ? 0.f : -INFINITY, ls = 0.f;
-    for (int d = tid; d < ((DH + 127) & ~127); d += kFusedAttnThreads) {
-      const float *pv = src + 4 + d;
-      float v[kFusedAttnMaxSplit];
+    // lane s: the (max, sum) of split s; every lane: its dimensions of all splits
+    float2 ml = make_float2(-INFINITY, 0.f);
+    if (lane < used) ml = __ldcg(reinterpret_cast<const float2 *>(src + lane * PR));
+    float v[kFusedAttnMaxSplit][DPL];
 #pragma unroll
-      for (int q = 0; q < kFusedAttnMaxSplit; ++q) v[q] = 0.f;
-      for (int spin = 0; spin < 1000000; ++spin) {  // (a word that does not come makes the result NaN)
-        if (lane < used && is_idle(ms)) ms = ld_relaxed(src + lane * PR);
-        if (lane < used && is_idle(ls)) ls = ld_relaxed(src + lane * PR + 1);
+    for (int q = 0; q < kFusedAttnMaxSplit; ++q)
+      if (q < used) ldcg_floats(src + q * PR + 4 + lane * DPL, v[q]);
+    const float m = warp_max(ml.x);
+    const float w = lane < used ? __expf(ml.x - m) : 0.f;
+    const float inv = 1.f / warp_sum(ml.y * w);
+    const float zeros[DPL] = {};
+    float a[DPL];
 #pragma unroll
-        for (int q = 0; q < kFusedAttnMaxSplit; ++q)
-          if (q < used && d < DH && is_idle(v[q])) v[q] = ld_relaxed(pv + q * PR);
-        bool idle = lane < used && (is_idle(ms) || is_idle(ls));
+    for (int j = 0; j < DPL; ++j) a[j] = 0.f;
 #pragma unroll
-        for (int q = 0; q < kFusedAttnMaxSplit; ++q) idle = idle || (q < used && d < DH && is_idle(v[q]));
-        if (!__any_sync(0xffffffffu, idle)) break;
-        __nanosleep(20);
+    for (int q = 0; q < kFusedAttnMaxSplit; ++q) {
+      const float ws = __shfl_sync(0xffffffffu, w, q);
+      if (q < used) {
+#pragma unroll
+        for (int j = 0; j < DPL; ++j) a[j] += ws * v[q][j];
+        stcg_floats(src + q * PR + 4 + lane * DPL, zeros);
       }
-      const float m = warp_max(ms);
-      const float w = lane < used ? __expf(ms - m) : 0.f;
-      const float l = warp_sum(ls * w);
-      float a = 0.f;
-#pragma unroll
-      for (int q = 0; q < kFusedAttnMaxSplit; ++q) {
-        if (q < used) {
-          const float ws = __shfl_sync(0xffffffffu, w, q);
-          if (d < DH) {
-            a += is_idle(v[q]) ? NAN : ws * v[q];
-            src[q * PR + 4 + d] = 0.f;
-          }
-        }
-      }
-      if (d < DH) out[(1ll * b * nq + head) * DH + d] = __float2half_rn(a * (1.f / l));
     }
-    __syncthreads();  // every warp has read the (max, sum) pairs
-    if (tid < used) src[tid * PR] = src[tid * PR + 1] = 0.f;
+    if (lane < used) *reinterpret_cast<float2 *>(src + lane * PR) = make_float2(0.f, 0.f);
+    __half *o = out + (1ll * b * nq + head) * DH + lane * DPL;
+#pragma unroll
+    for (int j = 0; j < DPL; ++j) o[j] = __float2half_rn(a[j] * inv);
   }
 }
 
@@ -787,19 +799,23 @@ int rope_attn_splits(int B, int nkv, int S) {
   return std::min(kFusedAttnMaxSplit, std::max(1, sm_count() / std::max(1, B * nkv)));
 }
 
+// The count of each (sequence, KV head) comes first, then the partial sums.
+static size_t rope_attn_counter_bytes(int B, int nkv) { return (sizeof(int) * static_cast<size_t>(B) * nkv + 255) / 256 * 256; }
+
 size_t rope_attn_scratch_bytes(int B, int nq, int nkv, int dh, int S) {
   // Sized for every batch up to B (fewer sequences get more splits each), so one buffer serves smaller
-  // batches.
+  // batches: all of it is zero between calls.
   size_t rows = 0;
   for (int b = 1; b <= B; ++b) rows = std::max(rows, static_cast<size_t>(b) * rope_attn_splits(b, nkv, S));
-  return sizeof(float) * rows * nq * (dh + 4);
+  return rope_attn_counter_bytes(B, nkv) + sizeof(float) * rows * nq * (dh + 4);
 }
 
 int launch_rope_attn(const __half *qkv, const __half *qn, const __half *kn, const __half *cos_t, const __half *sin_t,
                      const long long *pos, __half *k_cache, __half *v_cache, void *scratch, __half *out, int B, int nq,
                      int nkv, int dh, int S, float scale, float eps, bool pdl, cudaStream_t stream) {
   const int nsplit = rope_attn_splits(B, nkv, S);
-  float *part = static_cast<float *>(scratch);
+  int *counters = static_cast<int *>(scratch);
+  float *part = reinterpret_cast<float *>(static_cast<char *>(scratch) + rope_attn_counter_bytes(B, nkv));
   const int group = nq / nkv;
   const int nb = group <= 8 ? 1 : 2;
   int smem = kFusedAttnWarps * 4 * 16 * (2 * dh + 16) + 8 * nb * (dh + 8) * 2;
@@ -818,8 +834,8 @@ int launch_rope_attn(const __half *qkv, const __half *qn, const __half *kn, cons
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     RDQ_CUDA(pin_slot(reinterpret_cast<const void *>(kernel), smem));
-    RDQ_CUDA(cudaLaunchKernelEx(&cfg, kernel, qkv, qn, kn, cos_t, sin_t, pos, k_cache, v_cache, part, out, nq, nkv, S, scale, eps,
-                                nsplit, nkv * B));
+    RDQ_CUDA(cudaLaunchKernelEx(&cfg, kernel, qkv, qn, kn, cos_t, sin_t, pos, k_cache, v_cache, part, counters, out, nq, nkv, S, scale,
+                                eps, nsplit, nkv * B));
     return RDQ_OK;
   };
   switch (dh) {

@@ -521,7 +521,7 @@ def attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, p
 
 
 def rope_attn_scratch(b: int, nq: int, nkv: int, dh: int, s: int, device) -> torch.Tensor:
-    """Zeroed scratch of :func:`rope_attn_decode` (partial sums per split; idle words are zero)."""
+    """Zeroed scratch of :func:`rope_attn_decode` (a count per KV head, then partial sums per split)."""
     need = ctypes.c_size_t(0)
     _lib.check(_lib.lib().rdq_rope_attn_decode_scratch_size(b, nq, nkv, dh, s, ctypes.byref(need)),
                "rdq_rope_attn_decode_scratch_size")

@@ -159,3 +159,23 @@ def test_rope_attn_decode_refuses_what_it_cannot_run():
         call(34, 2, 64)
     with pytest.raises(RuntimeError):
         call(4, 2, 64, qkv_cols=100)
+
+
+@pytest.mark.parametrize("b,nq,nkv,dh,s,pos_v", [(1, 32, 8, 128, 600, 520), (4, 32, 8, 128, 600, 333), (1, 16, 1, 64, 300, 255),
+                                                  (1, 8, 4, 256, 900, 800)])
+def test_rope_attn_decode_merges_its_own_parts_only(b, nq, nkv, dh, s, pos_v):
+    """Partial sums that something left behind in the scratch are not taken for this launch's: only the
+    counts, which come first, have to be zero."""
+    g = torch.Generator().manual_seed(nq + dh)
+    qkv = torch.randn(b, (nq + 2 * nkv) * dh, generator=g).half().cuda()
+    cos, sin = (torch.rand(s, dh, generator=g).half().cuda() for _ in range(2))
+    k_cache, v_cache = (torch.randn(b, nkv, s, dh, generator=g).half().cuda() for _ in range(2))
+    pos = torch.tensor([pos_v], dtype=torch.long, device="cuda")
+    outs = []
+    for left in (0.0, 3.0):
+        scratch = rc.rope_attn_scratch(b, nq, nkv, dh, s, "cuda")
+        scratch[(b * nkv + 63) // 64 * 64:] = left
+        out = torch.empty(b, nq * dh, dtype=torch.float16, device="cuda")
+        rc.rope_attn_decode(qkv, None, None, cos, sin, pos, k_cache, v_cache, scratch, out, nq, dh ** -0.5, 1e-6)
+        outs.append(out)
+    assert torch.equal(*outs)
