@@ -304,7 +304,7 @@ int rdq_gemv_tiled_noalloc_status(int reset, void *stream) {
 
 int rdq_gemm_status(int reset, void *stream) { return gemm_status(reset != 0, static_cast<cudaStream_t>(stream)); }
 
-void rdq_gemm_test_timeout(int enable) { gemm_set_test_timeout(enable != 0); }
+void rdq_gemm_test_timeout(int enable) { gemm_set_test_timeout(enable == 2 ? 2 : enable != 0); }
 
 int rdq_gemm_mixed_ws(const void *x, int M, const void *w_fp4, const void *w_fp4_scales,
                       float w_fp4_global_scale, const void *w_fp8, const float *w_fp8_scales,

@@ -116,21 +116,33 @@ __device__ __forceinline__ uint32_t wait_bounded(uint32_t bar, uint32_t parity) 
       : "memory");
   return left;
 }
-// Wait (bounded, about 0.4 s) until the low half of a global word reaches `count`.  Afterwards each of
-// the `parts` waiting threads counts itself in the high half (pass_arrivals) and later, when the answer
-// has come, puts the word back to zero if it was the last (leave_arrivals).
-__device__ __forceinline__ bool wait_arrivals(uint32_t *word, uint32_t count) {
-  uint32_t v = 0;
-  for (int i = 0; i < 4000000; ++i) {
+// ---- tiles whose k range several CTAs share
+// Each of the `parts` CTAs leaves FP32 sums in the workspace and its four epilogue warps count themselves
+// in a word of the tile (arrive_global).  When all are there, each CTA adds and stores a share of the
+// tile's tokens.  That must not rely on the CTAs running at the same time -- kernels of another stream
+// may hold the SMs that some of them need until these here give theirs up -- so a CTA that has waited for
+// long leaves without doing anything (await_parts).  Nobody leaves once all have arrived, and the CTA
+// that arrives last need not wait (its own warps have arrived when it asks): at least one is present then, and those present do the WHOLE tile
+// when anyone has left.  The sums and their order are the same, so several doing it changes nothing.
+// The word: warps arrived (bits 0-11), CTAs that left (12-21), CTAs done waiting (22-31).
+constexpr int kPatience = 500;  // about half a millisecond: CTAs of a launch start within a few microseconds
+constexpr uint32_t kMostParts = 1000;
+
+// How many CTAs left, once all parts are there; -1: this CTA is to leave.
+__device__ __forceinline__ int await_parts(uint32_t *word, uint32_t parts, int patience) {
+  for (int i = 0;; ++i) {  // (ends: beyond the patience a failed exchange means that another CTA changed the word)
+    uint32_t v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
-    if ((v & 0xffffu) == count) break;
+    if ((v & 0xfffu) == 4 * parts) return static_cast<int>((v >> 12) & 0x3ffu);
+    if (i >= patience && atomicCAS(word, v, v + (1u << 12)) == v) return -1;
     if (i > 64) __nanosleep(100);
   }
-  return (v & 0xffffu) == count;
 }
-__device__ __forceinline__ uint32_t pass_arrivals(uint32_t *word) { return atomicAdd(word, 0x10000u) >> 16; }
-__device__ __forceinline__ void leave_arrivals(uint32_t *word, uint32_t passed, uint32_t parts) {
-  if (passed == parts - 1) asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(word), "r"(0u) : "memory");
+// The CTAs present count themselves once they are done waiting; the last of them puts the word back to
+// zero (later, when the answer has come).
+__device__ __forceinline__ uint32_t pass_parts(uint32_t *word) { return atomicAdd(word, 1u << 22) >> 22; }
+__device__ __forceinline__ void clear_parts(uint32_t *word, uint32_t passed, int left, uint32_t parts) {
+  if (passed + 1 + left == parts) asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(word), "r"(0u) : "memory");
 }
 __device__ __forceinline__ void arrive_global(uint32_t *word) {
   asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(word) : "memory");

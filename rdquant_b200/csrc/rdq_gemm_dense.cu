@@ -26,8 +26,9 @@
 //               works on one accumulator while the MMAs fill the other.
 // Tiles are walked in groups of eight token tiles so that concurrent tiles share operands in L2.
 // Tiles beyond the last full wave are split along k: every part leaves its FP32 sums in the
-// workspace, waits (bounded) for the others -- they run at the same time, as the last work of their
-// CTAs -- and adds and stores its share of the tile's tokens, in the order of the parts.
+// workspace, waits for a while for the others -- they mostly run at the same time, as the last work of
+// their CTAs -- and adds and stores its share of the tile's tokens, in the order of the parts
+// (await_parts: those that leave, and who does their share).
 //
 // Reference behaviour replaced: F.linear over a materialised FP16 weight copy
 // (rdquant/inference.py:679-687).
@@ -161,7 +162,8 @@ struct PairArgs {
   const __half *bias;
   void *y;
   float *partial;  // [tile - full][part][CTA][token][128 channels]
-  uint32_t *counters;  // [tile - full][CTA]: epilogue warps done (low half), parts past the wait (high half)
+  uint32_t *counters;  // [tile - full][CTA]: the tile's word (await_parts)
+  int patience;
   int test_timeout;
 };
 
@@ -173,6 +175,7 @@ struct PairSmem {
   uint64_t never;
   uint32_t tmem_base;
   int abort_flag;
+  int left;  // finish_shared: what await_parts answered
 };
 
 struct WorkItem {
@@ -204,11 +207,12 @@ __device__ __forceinline__ WorkItem work_item(const PairArgs &a, int item) {
   return w;
 }
 
-// The four epilogue warps: wait for all parts of a split tile, add and store this part's tokens.  A
+// The four epilogue warps: wait for all parts of a split tile, add and store this part's tokens (all of
+// them when CTAs have left).  A
 // warp takes every fourth token, a lane four channels, with the loads of four tokens in flight.
 template <bool BF16>
 __device__ __forceinline__ void finish_shared(const PairArgs &a, const WorkItem &w, uint32_t rank, int q, int lane,
-                                              volatile int *abort_flag) {
+                                              volatile int *answer) {
   const int ch = w.n * 256 + static_cast<int>(rank) * 128 + lane * 4;
   float scl[4], bia[4];
 #pragma unroll
@@ -216,13 +220,15 @@ __device__ __forceinline__ void finish_shared(const PairArgs &a, const WorkItem 
     scl[e] = ch + e < a.N ? a.scale[ch + e] : 0.f;
     bia[e] = ch + e < a.N && a.bias ? __half2float(a.bias[ch + e]) : 0.f;
   }
-  if (q == 0 && lane == 0 && !wait_arrivals(a.counters + w.rem * 2 + rank, 4u * a.parts)) *abort_flag = 1;
-  asm volatile("bar.sync 1, 128;" ::: "memory");
-  if (*abort_flag) return;
   uint32_t *const word = a.counters + w.rem * 2 + rank;
-  const uint32_t passed = q == 0 && lane == 0 ? pass_arrivals(word) : 0u;
+  asm volatile("bar.sync 1, 128;" ::: "memory");  // this CTA's warps have all arrived: the last CTA to arrive does not leave
+  if (q == 0 && lane == 0) *answer = await_parts(word, a.parts, a.patience);
+  asm volatile("bar.sync 1, 128;" ::: "memory");
+  const int left = *answer;
+  if (left < 0) return;
+  const uint32_t passed = q == 0 && lane == 0 ? pass_parts(word) : 0u;
   const int tok0 = w.m * a.nt, ntok = min(a.nt, a.M - tok0);
-  const int lo = ntok * w.part / a.parts, hi = ntok * (w.part + 1) / a.parts;
+  const int lo = left ? 0 : ntok * w.part / a.parts, hi = left ? ntok : ntok * (w.part + 1) / a.parts;
   const long long part_stride = 2ll * a.nt * 128;
   const float *src = a.partial + (1ll * w.rem * a.parts * 2 + rank) * a.nt * 128 + lane * 4;
   const bool vec = (a.N & 3) == 0 && ch + 4 <= a.N;
@@ -262,7 +268,7 @@ __device__ __forceinline__ void finish_shared(const PairArgs &a, const WorkItem 
       }
     }
   }
-  if (q == 0 && lane == 0) leave_arrivals(word, passed, a.parts);
+  if (q == 0 && lane == 0) clear_parts(word, passed, left, a.parts);
 }
 
 template <bool BF16>
@@ -459,7 +465,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
         __syncwarp();
       }
     }
-    if (shared.rem >= 0 && !S.abort_flag) finish_shared<BF16>(a, shared, rank, q, lane, &S.abort_flag);
+    if (shared.rem >= 0 && !S.abort_flag) finish_shared<BF16>(a, shared, rank, q, lane, &S.left);
   }
 
   tc_fence_before();
@@ -608,7 +614,8 @@ int launch_gemm_dense(const GemmArgs &g, void *workspace, size_t workspace_bytes
   a.y = g.y;
   a.partial = reinterpret_cast<float *>(ws + lay.partial);
   a.counters = reinterpret_cast<uint32_t *>(d.counters);
-  a.test_timeout = gemm_test_timeout();
+  a.test_timeout = gemm_test_timeout() == 1;
+  a.patience = gemm_test_timeout() == 2 ? 0 : kPatience;
 
   const void *fn = g.y_bf16 ? reinterpret_cast<const void *>(gemm_pair_kernel<true>)
                             : reinterpret_cast<const void *>(gemm_pair_kernel<false>);

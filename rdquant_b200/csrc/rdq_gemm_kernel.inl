@@ -397,7 +397,7 @@ std::atomic<int> g_gemm_test_timeout{0};
 }
 
 int gemm_test_timeout() { return g_gemm_test_timeout.load(); }
-void gemm_set_test_timeout(bool on) { g_gemm_test_timeout.store(on ? 1 : 0); }
+void gemm_set_test_timeout(int mode) { g_gemm_test_timeout.store(mode); }
 
 int gemm_status(bool reset, cudaStream_t stream) {
   int code = 0;
@@ -463,7 +463,7 @@ size_t gemm_workspace_bytes(int M, int N, int K) { return gemm_dense_takes(K) ? 
 int launch_gemm(const GemmArgs &a, void *workspace, size_t workspace_bytes, cudaStream_t stream) {
   const int N = a.n4 + a.n8 + a.n16;
   GemmArgs b = a;
-  b.test_timeout = gemm_test_timeout();
+  b.test_timeout = gemm_test_timeout() == 1;
   if (workspace != nullptr && gemm_dense_takes(a.K) && workspace_bytes >= gemm_dense_workspace(a.M, N, a.K))
     return launch_gemm_dense(b, workspace, workspace_bytes, stream);
   CUtensorMap xmap;

@@ -13,9 +13,9 @@
 // Work: every tile is a run of 16 KB chunks (128 rows x 128 packed bytes = 256 / 128 / 64 k of
 // NVFP4 / FP8 / FP16), all chunks of the layer are numbered in tile order and each CTA takes a
 // contiguous range of equal cost (make_plan).  A tile inside one range is finished by its CTA.  The
-// CTAs that share a tile cut by range borders leave FP32 partial sums in the workspace, wait
-// (bounded) until all parts of the tile are there, and each adds and stores a share of its tokens,
-// parts in CTA order: the result does not depend on timing.  A second kernel for these sums cost
+// CTAs that share a tile cut by range borders leave FP32 partial sums in the workspace, wait for a while
+// until all parts of the tile are there, and each adds and stores a share of its tokens, parts in CTA
+// order: the result does not depend on timing (await_parts: those that leave, and who does their share).  A second kernel for these sums cost
 // 4-7 us per layer, and one CTA per tile adding them up to 13 us.
 //
 // A stage of the pipeline is one chunk: up to 128 tensor-memory columns of weights and up to four
@@ -71,6 +71,7 @@ constexpr int kMaxRing = 8;
 constexpr int kSmemMax = 222 * 1024;
 constexpr int kMaxTokens = 128;   // per token tile
 constexpr int kMaxCtas = 160;
+static_assert(kMaxCtas <= kMostParts, "fields of a shared tile's word");
 
 // Chunks of the layer in processing order: NVFP4 tiles, FP8 tiles, FP16 tiles; inside a channel tile
 // its token tiles one after another.
@@ -110,7 +111,8 @@ struct StreamArgs {
   void *y;
   int n4, n8, n16, K, N;
   float *partial;    // [2 * CTA + (0 first, 1 last segment)][token][128 rows]
-  uint32_t *arrived;  // [CTA in which a cut tile starts]: epilogue warps done (low half), CTAs past the wait (high half)
+  uint32_t *arrived;  // [CTA in which a cut tile starts]: its word (await_parts)
+  int patience;
   int nw;             // weight chunks in flight
   int early;          // weights may be read before the kernel before this one has finished
   int scale16;     // block-scale rows can be copied 16 bytes at a time
@@ -131,6 +133,7 @@ struct StreamSmem {
   uint64_t never;
   uint32_t tmem_base;
   int abort_flag;
+  int left[2];  // finish_shared: what await_parts answered
 };
 
 // position in a ring
@@ -262,21 +265,23 @@ __device__ __forceinline__ void store_row(void *y, long long i, float v) {
 }
 
 // Half of the first 512 threads: waits until all parts of the segment's tile are in the workspace,
-// then adds and stores this CTA's share of its tokens.  `sub` (0, 1) and r (row) identify the thread.
+// then adds and stores this CTA's share of its tokens, or all of them when CTAs have left.  `sub` (0, 1) and r (row) identify the thread.
 // kPart parts of kTok tokens are read at a time: four of eight for narrow token tiles (a small layer's
 // tile has three or four parts), two of sixteen for wide ones.
 template <bool BF16, int kPart, int kTok>
 __device__ __forceinline__ void finish_shared(const StreamArgs &a, const StreamSched &sc, const Segment &g, const Row &row, int r,
-                                              int sub, int bar_id, volatile int *abort_flag) {
+                                              int sub, int bar_id, volatile int *answer) {
   const int b0 = first_cta(sc, blockIdx.x, g.start), b1 = last_cta(sc, blockIdx.x, g.start + sc.S[g.fmt]);
   const int parts = b1 - b0 + 1;
   const int tok0 = g.m_tile * sc.nt;
   const int ntok = min(sc.nt, sc.M - tok0);
-  const int lo = ntok * (static_cast<int>(blockIdx.x) - b0) / parts, hi = ntok * (static_cast<int>(blockIdx.x) + 1 - b0) / parts;
-  if (r == 0 && sub == 0 && !wait_arrivals(a.arrived + b0, 4u * parts)) *abort_flag = 1;
+  if (r == 0 && sub == 0) *answer = await_parts(a.arrived + b0, parts, a.patience);
   asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "n"(kFinishThreads / 2) : "memory");
-  if (*abort_flag) return;
-  const uint32_t passed = r == 0 && sub == 0 ? pass_arrivals(a.arrived + b0) : 0u;
+  const int left = *answer;
+  if (left < 0) return;
+  const uint32_t passed = r == 0 && sub == 0 ? pass_parts(a.arrived + b0) : 0u;
+  const int share = static_cast<int>(blockIdx.x) - b0;
+  const int lo = left ? 0 : ntok * share / parts, hi = left ? ntok : ntok * (share + 1) / parts;
   constexpr int kSub = 2;
 #pragma unroll 1
   for (int t0 = lo + sub; t0 < hi; t0 += kTok * kSub) {
@@ -305,7 +310,7 @@ __device__ __forceinline__ void finish_shared(const StreamArgs &a, const StreamS
           store_row<BF16>(a.y, 1ll * (tok0 + t0 + e * kSub) * a.N + row.col, fmaf(v[e], row.scl, row.bia));
     }
   }
-  if (r == 0 && sub == 0) leave_arrivals(a.arrived + b0, passed, parts);
+  if (r == 0 && sub == 0) clear_parts(a.arrived + b0, passed, left, parts);
 }
 
 // NT: most tokens per tile (64 or 128)
@@ -658,7 +663,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
       g = segment_at(sc, max(g.start, begin), end);
     }
     if (mine && !(g.c0 == 0 && g.c1 == sc.S[g.fmt]))
-      finish_shared<BF16, NT == 64 ? 4 : 2, NT == 64 ? 8 : 16>(a, sc, g, S.cut[half][threadIdx.x & 127], threadIdx.x & 127, (threadIdx.x >> 7) & 1, 1 + half, &S.abort_flag);
+      finish_shared<BF16, NT == 64 ? 4 : 2, NT == 64 ? 8 : 16>(a, sc, g, S.cut[half][threadIdx.x & 127], threadIdx.x & 127, (threadIdx.x >> 7) & 1, 1 + half, &S.left[half]);
   }
   __syncthreads();
   if (S.abort_flag) {
@@ -793,7 +798,8 @@ int launch_gemm_stream(const GemmArgs &g, void *workspace, size_t workspace_byte
   a.nw = p.nw;
   a.early = pdl;
   a.scale16 = g.K % 256 == 0 && aligned16(g.s4);
-  a.test_timeout = gemm_test_timeout();
+  a.test_timeout = gemm_test_timeout() == 1;
+  a.patience = gemm_test_timeout() == 2 ? 0 : kPatience;
   const StreamSched &sc = p.sc;
 
   static const void *const fns[4] = {

@@ -113,8 +113,9 @@ int launch_gemm(const GemmArgs &a, void *workspace, size_t workspace_bytes, cuda
 int gemm_status(bool reset, cudaStream_t stream);
 int gemm_status_ptr(int **out);
 int gemm_test_timeout();
-// self-test switch: launches made while it is on end with a wait that runs out
-void gemm_set_test_timeout(bool on);
+// self-test switch: 1: launches made while it is on end with a wait that runs out, 2: CTAs that share a
+// tile leave at once when they would have to wait
+void gemm_set_test_timeout(int mode);
 size_t gemm_workspace_bytes(int M, int N, int K);
 // weight-streaming GEMM (rdq_gemm_stream.cu)
 bool gemm_stream_takes(int K);

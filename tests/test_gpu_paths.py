@@ -199,3 +199,25 @@ def test_silu_mul_shares(rows, f):
     ref = g * torch.sigmoid(g) * u
     # silu and product each rounded to f16; a subnormal silu is off by 2^-25, times u
     assert bool(((out.double() - ref).abs() <= 2.1 * 2.0 ** -11 * ref.abs() + 2.0 ** -25 * (u.abs() + 1)).all())
+
+
+@pytest.mark.parametrize("shape,rows", [
+    ((1280, 896, 128, 1088), 17), ((1280, 896, 128, 1088), 64), ((300, 130, 20, 576), 100), ((0, 640, 128, 4096), 129),
+    ((0, 0, 256, 8192), 40),         # tiles shared by many CTAs
+    ((2048, 384, 128, 2560), 1280), ((600, 303, 100, 336), 700),  # the decoded-once GEMM, tiles split along k
+])
+def test_shared_tiles_do_not_need_their_ctas_at_the_same_time(shape, rows):
+    """CTAs that leave instead of waiting for the others of a tile: the ones that come last do its whole,
+    with the same result bit for bit, and nothing is left behind for the next call."""
+    layer = random_packed_layer(*shape, seed=rows)
+    mod = FusedMixedLinear.from_layer_data(layer, dict(zip(ORDER, shape[:3])), shape[3], "cuda")
+    x = torch.randn(rows, shape[3], generator=torch.Generator().manual_seed(rows)).half().cuda()
+    y = mod(x)
+    _lib.lib().rdq_gemm_test_timeout(2)
+    try:
+        for _ in range(5):
+            assert torch.equal(mod(x), y)
+    finally:
+        _lib.lib().rdq_gemm_test_timeout(0)
+    assert torch.equal(mod(x), y)
+    rc.check_gemm_status("cuda")
