@@ -92,7 +92,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         dirs = include_paths("cuda") + [sysconfig.get_paths()["include"]]
         _run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", TORCH_EXT_SOURCE, "-o", TORCH_EXT_PATH,
               *("-I" + d for d in dirs), *("-L" + d for d in library_paths("cuda")), "-L" + CSRC, "-l:librdq_b200.so",
-              "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-Wl,-rpath,$ORIGIN"])
+              "-lc10", "-lc10_cuda", "-lcudart", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-Wl,-rpath,$ORIGIN"])
     return LIB_PATH
 
 
@@ -163,6 +163,8 @@ def _bind(lib: ctypes.CDLL) -> None:
     lib.rdq_linear_workspace_size.argtypes = [vp, i32, i32, ctypes.POINTER(ctypes.c_size_t)]
     lib.rdq_linear.restype = i32
     lib.rdq_linear.argtypes = [vp, vp, i32, i32, vp, vp, vp, ctypes.c_size_t, i32, vp]
+    lib.rdq_linear_words.restype = i32
+    lib.rdq_linear_words.argtypes = [vp, vp, i32, i32, vp, vp, vp, ctypes.c_size_t, vp, i32, vp]
     lib.rdq_stage_copy.restype = i32
     lib.rdq_stage_copy.argtypes = [vp, vp, ctypes.c_size_t, vp]
     lib.rdq_stage_copy_signal.restype = i32
@@ -194,6 +196,7 @@ EXPORTS = [
     "rdq_quantize_fp8",
     "rdq_quantize_layer",
     "rdq_linear",
+    "rdq_linear_words",
     "rdq_linear_workspace_size",
     "rdq_stage_copy",
     "rdq_stage_copy_signal",

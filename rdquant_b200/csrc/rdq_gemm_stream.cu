@@ -70,7 +70,7 @@ constexpr int kScaleBytes = 128 * 16;
 constexpr int kMaxRing = 8;
 constexpr int kSmemMax = 222 * 1024;
 constexpr int kMaxTokens = 128;   // per token tile
-constexpr int kMaxCtas = 160;
+constexpr int kMaxCtas = RDQ_LINEAR_WORDS;
 static_assert(kMaxCtas <= kMostParts, "fields of a shared tile's word");
 
 // Chunks of the layer in processing order: NVFP4 tiles, FP8 tiles, FP16 tiles; inside a channel tile

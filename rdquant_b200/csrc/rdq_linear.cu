@@ -68,7 +68,7 @@ bool stream_beats_dense(const rdq_layer &l, int M, int x_type) {
 }
 
 Path path_of(const rdq_layer &l, int M, int x_type) {
-  const bool can_stream = gemm_stream_takes(l.K) && has_row_major(l) && l.gemv_counters && (l.perm || !l.inv_perm);
+  const bool can_stream = gemm_stream_takes(l.K) && has_row_major(l) && (l.perm || !l.inv_perm);
   if (can_stream && M >= stream_from(l) && (!gemm_dense_takes(l.K) || stream_beats_dense(l, M, x_type))) return Path::kStream;
   if (M <= RDQ_MAX_GEMV_M) return l.w_tiled ? Path::kGemvTiled : Path::kGemvGeneric;
   if (gemm_dense_takes(l.K) && has_row_major(l)) return Path::kGemm;
@@ -178,7 +178,13 @@ int rdq_linear_workspace_size(const rdq_layer *layer, int M, int x_type, size_t 
 }
 
 int rdq_linear(const rdq_layer *layer, const void *x, int x_type, int M, const void *bias, void *y, void *workspace,
-               size_t workspace_bytes, int flags, void *stream_) {
+               size_t workspace_bytes, int flags, void *stream) {
+  return rdq_linear_words(layer, x, x_type, M, bias, y, workspace, workspace_bytes, layer ? layer->gemv_counters : nullptr,
+                          flags & ~RDQ_LINEAR_FRESH, stream);
+}
+
+int rdq_linear_words(const rdq_layer *layer, const void *x, int x_type, int M, const void *bias, void *y, void *workspace,
+                     size_t workspace_bytes, int32_t *words, int flags, void *stream_) {
   RDQ_REQUIRE(layer != nullptr && M >= 0 && (x_type == RDQ_F16 || x_type == RDQ_BF16), RDQ_E_INVALID, "bad arguments to rdq_linear");
   const rdq_layer &l = *layer;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
@@ -192,6 +198,8 @@ int rdq_linear(const rdq_layer *layer, const void *x, int x_type, int M, const v
               RDQ_E_INVALID, "rdq_linear needs %zu bytes of 16-byte aligned workspace for this shape", need.cast + need.gemm);
   const int bf16 = x_type == RDQ_BF16 ? 1 : 0;
   bool pdl = (flags & RDQ_GEMV_PDL) != 0;
+  if (words && (flags & RDQ_LINEAR_FRESH)) RDQ_CUDA(cudaMemsetAsync(words, 0, RDQ_LINEAR_WORDS * sizeof(int32_t), stream));
+  RDQ_REQUIRE(words || p != Path::kStream, RDQ_E_INVALID, "words must not be null");
   const void *xh = x;
   int x_bf16 = bf16;
   // (the decoded-once GEMM's first launch rounds the rows itself)
@@ -240,7 +248,7 @@ int rdq_linear(const rdq_layer *layer, const void *x, int x_type, int M, const v
   a.w16 = static_cast<const __half *>(l.w_fp16);
   a.inv_perm = l.inv_perm;
   a.perm = l.perm;
-  a.counters = l.gemv_counters;
+  a.counters = words;
   a.bias = static_cast<const __half *>(bias);
   a.y = y;
   a.n4 = l.n_fp4;

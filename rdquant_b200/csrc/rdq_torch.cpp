@@ -19,6 +19,9 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <cuda_runtime_api.h>
+
+#include <algorithm>
 #include <initializer_list>
 #include <new>
 #include <vector>
@@ -46,6 +49,44 @@ struct OnDevice {
     if (changed) c10::cuda::set_device(prev);
   }
 };
+
+// Words of rdq_linear_words.  They are zero between launches, so the calls of a stream share a set; a
+// stream that is being captured has one per capture, which the graph zeroes on every replay.  A set that
+// is dropped goes back to torch's allocator, which gives it to later work of the same stream only.  At
+// most kMostSets are kept, the last used; all are dropped with the last layer.  (Under the GIL.)
+struct Words {
+  c10::DeviceIndex device;
+  c10::StreamId stream;
+  unsigned long long capture;
+  at::Tensor t;
+};
+constexpr size_t kMostSets = 64;
+std::vector<Words> *word_sets = new std::vector<Words>();  // not destroyed at exit: CUDA may be gone by then
+long layers_alive = 0;
+
+// `fresh`: the words have any content
+int32_t *words_of(c10::DeviceIndex device, const c10::cuda::CUDAStream &stream, bool *fresh) {
+  const c10::StreamId id = stream.id();
+  unsigned long long capture = 0;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamGetCaptureInfo(stream.stream(), &status, &capture) != cudaSuccess)
+    cudaGetLastError();  // (a launch on such a stream will say what is wrong with it)
+  if (status != cudaStreamCaptureStatusActive) capture = 0;
+  auto &sets = *word_sets;
+  sets.erase(std::remove_if(sets.begin(), sets.end(), [&](const Words &w) { return w.capture != 0 && w.capture != capture; }), sets.end());
+  auto it = std::find_if(sets.begin(), sets.end(),
+                         [&](const Words &w) { return w.device == device && w.stream == id && w.capture == capture; });
+  *fresh = it == sets.end();
+  if (*fresh) {
+    if (sets.size() >= kMostSets) sets.erase(sets.begin());
+    const int64_t sizes[1] = {RDQ_LINEAR_WORDS};
+    sets.push_back({device, id, capture,
+                    at::detail::empty_cuda(at::IntArrayRef(sizes, 1), at::kInt, c10::Device(c10::kCUDA, device), std::nullopt)});
+  } else if (it + 1 != sets.end()) {
+    std::rotate(it, it + 1, sets.end());
+  }
+  return static_cast<int32_t *>(sets.back().t.data_ptr());
+}
 
 bool take(LayerObject *self, PyObject *dict, const char *key, const void **out) {
   *out = nullptr;
@@ -85,6 +126,7 @@ PyObject *layer_new(PyTypeObject *type, PyObject *args, PyObject *) {
   if (!PyArg_ParseTuple(args, "O!", &PyDict_Type, &dict)) return nullptr;
   LayerObject *self = reinterpret_cast<LayerObject *>(type->tp_alloc(type, 0));
   if (self == nullptr) return nullptr;
+  ++layers_alive;
   self->keep = new (std::nothrow) std::vector<at::Tensor>();
   self->device = -1;
   rdq_layer &l = self->layer;
@@ -119,6 +161,7 @@ PyObject *layer_new(PyTypeObject *type, PyObject *args, PyObject *) {
 
 void layer_dealloc(PyObject *obj) {
   delete reinterpret_cast<LayerObject *>(obj)->keep;
+  if (--layers_alive == 0) word_sets->clear();
   Py_TYPE(obj)->tp_free(obj);
 }
 
@@ -172,8 +215,14 @@ PyObject *layer_linear(PyObject *obj, PyObject *const *args, Py_ssize_t nargs) {
         const int64_t sizes[1] = {static_cast<int64_t>(need)};
         ws = at::detail::empty_cuda(at::IntArrayRef(sizes, 1), at::kByte, device, std::nullopt);
       }
-      rc = rdq_linear(&l, xp, xt, static_cast<int>(m), bias, y.data_ptr(), need ? ws.data_ptr() : nullptr, need,
-                      static_cast<int>(flags), c10::cuda::getCurrentCUDAStream(self->device).stream());
+      const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream(self->device);
+      // (without a workspace it is a decode kernel, which needs no words)
+      int32_t *words = nullptr;
+      bool fresh = false;
+      if (need) words = words_of(self->device, stream, &fresh);
+      rc = rdq_linear_words(&l, xp, xt, static_cast<int>(m), bias, y.data_ptr(), need ? ws.data_ptr() : nullptr, need, words,
+                            static_cast<int>(flags) | (fresh ? RDQ_LINEAR_FRESH : 0), stream.stream());
+      if (fresh && rc != RDQ_OK) word_sets->pop_back();  // perhaps not zeroed
     }
     if (rc != RDQ_OK) {
       PyErr_Format(PyExc_RuntimeError, "rdq_linear failed (code %d): %s", rc, rdq_last_error());

@@ -221,3 +221,30 @@ def test_shared_tiles_do_not_need_their_ctas_at_the_same_time(shape, rows):
         _lib.lib().rdq_gemm_test_timeout(0)
     assert torch.equal(mod(x), y)
     rc.check_gemm_status("cuda")
+
+
+@pytest.mark.parametrize("rows", [40, 120])
+def test_one_layer_on_several_streams(rows):
+    """Calls of one layer that overlap: three streams at once, and a captured call replayed beside them."""
+    layer = random_packed_layer(1280, 896, 128, 1088, seed=21)
+    mod = FusedMixedLinear.from_layer_data(layer, dict(zip(ORDER, (1280, 896, 128))), 1088, "cuda")
+    gen = torch.Generator().manual_seed(rows)
+    xs = [torch.randn(rows, 1088, generator=gen).half().cuda() for _ in range(4)]
+    refs = [mod(x) for x in xs]
+    streams = [torch.cuda.Stream() for _ in xs]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=streams[3]):
+        captured = [mod(xs[3]) for _ in range(3)]
+    torch.cuda.synchronize()
+    outs = []
+    for _ in range(40):
+        with torch.cuda.stream(streams[3]):
+            graph.replay()
+        for s, x in zip(streams[:3], xs):
+            with torch.cuda.stream(s):
+                outs.append(mod(x))
+    torch.cuda.synchronize()
+    for i, y in enumerate(outs):
+        assert torch.equal(y, refs[i % 3])
+    assert all(torch.equal(y, refs[3]) for y in captured)
+    rc.check_gemm_status("cuda")
