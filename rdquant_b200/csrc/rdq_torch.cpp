@@ -356,7 +356,16 @@ PyObject *dequantize(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
   }
 }
 
+// drop_words() -> number of sets dropped: the next calls start with zeroed ones (after a time-out, which
+// leaves counts behind)
+PyObject *drop_words(PyObject *, PyObject *) {
+  const size_t n = word_sets->size();
+  word_sets->clear();
+  return PyLong_FromSize_t(n);
+}
+
 PyMethodDef module_methods[] = {
+    {"drop_words", drop_words, METH_NOARGS, "forget the words of rdq_linear_words, which a time-out leaves in disorder"},
     {"quantize_layer", reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(quantize_layer)), METH_FASTCALL,
      "packed tensors of a layer, or None when the input needs conversions first"},
     {"dequantize", reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(dequantize)), METH_FASTCALL,

@@ -93,10 +93,13 @@ def check_status(fd: dict) -> None:
 
 
 def check_gemm_status(device) -> None:
-    """The same for the prefill GEMM (one status word per device, cleared when it is reported)."""
+    """The same for the GEMMs (one status word per device, cleared when it is reported).  The layers stay
+    usable: the counts that a launch which gave up leaves behind are dropped with the report."""
     device = torch.device(device)
     with _on_device(device):
         rc = _lib.lib().rdq_gemm_status(1, _stream(device))
+    if rc != 0:
+        _lib.torch_ext().drop_words()
     _lib.check(rc, "rdq_gemm_status")
 
 

@@ -10,6 +10,7 @@ from conftest import ORDER
 from oracle import oracle_np as onp
 from rdquant_b200 import _lib, rdquant_cuda
 from rdquant_b200.fused_gemv_pack import pack_for_fused_gemv
+from rdquant_b200.inference import FusedMixedLinear
 from rdquant_b200.synthetic import random_packed_layer
 
 pytestmark = pytest.mark.gpu
@@ -78,3 +79,28 @@ def test_gemm_timeout_is_reported_and_cleared():
     assert torch.equal(y_ok, y_again)
     ref = onp.mixed_precision_linear(x.cpu().numpy(), onp.torch_layer_to_np(layer), splits, k)
     assert onp.rel_err(y_again.cpu().float().numpy(), ref) < 2e-3
+
+
+@pytest.mark.parametrize("rows", [32, 100])
+def test_streaming_gemm_timeout_is_reported_and_cleared(rows):
+    """The GEMM a module call takes for a few rows: its status is reported, and the counts of its launches,
+    which a launch that gave up leaves behind, do not outlive the report."""
+    layer, splits, k, _ = _layer(seed=6)
+    lib = _lib.lib()
+    mod = FusedMixedLinear.from_layer_data(layer, splits, k, "cuda")
+    x = torch.randn(rows, k, generator=torch.Generator().manual_seed(4)).half().cuda()
+    y_ok = mod(x)
+    rdquant_cuda.check_gemm_status(x.device)
+    lib.rdq_gemm_test_timeout(1)
+    try:
+        mod(x)
+    finally:
+        lib.rdq_gemm_test_timeout(0)
+    with pytest.raises(RuntimeError, match="GEMM: a bounded device-side wait"):
+        rdquant_cuda.check_gemm_status(x.device)
+    assert _lib.torch_ext().drop_words() == 0, "the report drops the counts"
+    rdquant_cuda.check_gemm_status(x.device)
+    assert torch.equal(mod(x), y_ok)
+    rdquant_cuda.check_gemm_status(x.device)
+    ref = onp.mixed_precision_linear(x.cpu().numpy(), onp.torch_layer_to_np(layer), splits, k)
+    assert onp.rel_err(y_ok.cpu().float().numpy(), ref) < 2e-3
