@@ -122,13 +122,14 @@ class FusedMixedLinear(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         # the native path takes contiguous float16 / bfloat16 CUDA rows and answers None otherwise
-        if not rdquant_cuda.VALIDATE:
-            if self._native is None and self._has_fused and x.is_cuda:
-                self._make_native(x.device)
-            if self._native is not None:
-                y = self._native.linear(x, self._bias_h, _lib.RDQ_GEMV_PDL if self.use_pdl else 0)
-                if y is not None:
-                    return y
+        if self._native is None and self._has_fused and x.is_cuda:
+            self._make_native(x.device)
+        if self._native is not None:
+            y = self._native.linear(x, self._bias_h, _lib.RDQ_GEMV_PDL if self.use_pdl else 0)
+            if y is not None:
+                if rdquant_cuda.VALIDATE:
+                    rdquant_cuda.check_linear_status(self._fd())
+                return y
         return self._forward_checked(x)
 
     def _forward_checked(self, x: torch.Tensor) -> torch.Tensor:

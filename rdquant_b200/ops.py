@@ -65,11 +65,12 @@ def mixed_precision_linear(
     if not x.is_cuda:
         raise RuntimeError("rdquant_b200.ops.mixed_precision_linear runs on CUDA tensors only (no host path)")
     fd, native = _packed_for(qtensors, splits, inv_perm, x.device)
-    if not rdquant_cuda.VALIDATE:
-        # None: the input needs the conversions and checks below
-        y = native.linear(x, bias, 0)
-        if y is not None:
-            return y
+    # None: the input needs the conversions and checks below
+    y = native.linear(x, bias, 0)
+    if y is not None:
+        if rdquant_cuda.VALIDATE:
+            rdquant_cuda.check_linear_status(fd)
+        return y
     lead = x.shape[:-1]
     x2 = x.reshape(-1, x.shape[-1])
     xh = x2 if x2.dtype == torch.float16 else x2.to(torch.float16)

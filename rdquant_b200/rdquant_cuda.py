@@ -16,8 +16,8 @@ import torch
 from rdquant_b200 import _lib
 
 MAX_GEMV_M = 16
-# RDQ_B200_VALIDATE=1: synchronise after every GEMV / GEMM call and raise if the kernel gave up a
-# bounded device-side wait (debugging aid; costs a device round trip per call)
+# RDQ_B200_VALIDATE=1: synchronise after every GEMV / GEMM call -- the kernels that run without it -- and
+# raise if one gave up a bounded device-side wait (debugging aid; costs a device round trip per call)
 VALIDATE = os.environ.get("RDQ_B200_VALIDATE", "0") not in ("", "0")
 
 
@@ -101,6 +101,12 @@ def check_gemm_status(device) -> None:
     if rc != 0:
         _lib.torch_ext().drop_words()
     _lib.check(rc, "rdq_gemm_status")
+
+
+def check_linear_status(fd: dict) -> None:
+    """Both, for a call that may have run on either kind of kernel."""
+    check_status(fd)
+    check_gemm_status(fd["tile_counters"].device)
 
 
 _scratch_by_device: dict = {}

@@ -11,6 +11,8 @@ from oracle import oracle_np as onp
 from rdquant_b200 import _lib, rdquant_cuda
 from rdquant_b200.fused_gemv_pack import pack_for_fused_gemv
 from rdquant_b200.inference import FusedMixedLinear
+from rdquant_b200.ops import mixed_precision_linear
+from rdquant_b200.quantize import quantize_weight
 from rdquant_b200.synthetic import random_packed_layer
 
 pytestmark = pytest.mark.gpu
@@ -104,3 +106,29 @@ def test_streaming_gemm_timeout_is_reported_and_cleared(rows):
     rdquant_cuda.check_gemm_status(x.device)
     ref = onp.mixed_precision_linear(x.cpu().numpy(), onp.torch_layer_to_np(layer), splits, k)
     assert onp.rel_err(y_ok.cpu().float().numpy(), ref) < 2e-3
+
+
+@pytest.mark.parametrize("rows,dtype", [(32, torch.float16), (32, torch.bfloat16), (700, torch.bfloat16)])
+@pytest.mark.parametrize("functional", [False, True])
+def test_validate_mode_checks_the_kernels_that_run(monkeypatch, rows, dtype, functional):
+    """Modules and the functional operator: the same kernels as without the mode, and their time-outs raise."""
+    layer, splits, k, _ = _layer((256, 128, 0, 1024), seed=7)
+    lib = _lib.lib()
+    x = torch.randn(rows, k, generator=torch.Generator().manual_seed(5)).to(dtype).cuda()
+    if functional:
+        n = sum(splits.values())
+        perm = torch.randperm(n, generator=torch.Generator().manual_seed(6))
+        qw = quantize_weight(torch.randn(n, k, generator=torch.Generator().manual_seed(7)), perm, splits)
+        call = lambda: mixed_precision_linear(x, qw.qtensors, qw.splits, qw.inv_permutation)
+    else:
+        call = lambda mod=FusedMixedLinear.from_layer_data(layer, splits, k, "cuda"): mod(x)
+    y = call()
+    monkeypatch.setattr(rdquant_cuda, "VALIDATE", True)
+    assert torch.equal(call(), y)
+    lib.rdq_gemm_test_timeout(1)
+    try:
+        with pytest.raises(RuntimeError, match="GEMM: a bounded device-side wait"):
+            call()
+    finally:
+        lib.rdq_gemm_test_timeout(0)
+    assert torch.equal(call(), y)
