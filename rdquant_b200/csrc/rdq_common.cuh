@@ -172,6 +172,17 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t
       "l"(src), "r"(bytes), "r"(bar)
       : "memory");
 }
+// ---- which launch may start when
+// A programmatic launch may start once every CTA of the launch before it has called
+// pdl_launch_dependents() or ended.  pdl_wait() returns when the launch before is complete; every kernel
+// here waits before it ends, so that everything before that one is complete too, and writes nothing
+// before.  The rule for the order of the two: wait first, then let the next launch start.  At most two
+// launches of a stream are then on the device, one that works and one that waits.  Only kernels whose
+// grid has a CTA for every SM, each with kSlotSmem or more of shared memory, may let the next one start
+// first (the GEMV with RDQ_GEMV_PDL, the kernels between two of them at up to eight rows, the staging
+// copies): an SM has two places for those, so that a launch finds none before the last but one has left.
+// A chain that broke the rule -- decoding and GEMM launches that both let the next one start before they
+// waited, with grids that left SMs free -- once stopped making progress after some hundred calls.
 __device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }

@@ -60,7 +60,7 @@ struct DecodeArgs {
 constexpr int kDecodeUnroll = 4;
 
 __global__ void __launch_bounds__(256) decode_rows_kernel(DecodeArgs a) {
-  pdl_launch_dependents();
+  pdl_launch_dependents();  // (launched in stream order: everything before it is complete)
   const int lane = threadIdx.x & 31;
   const int gid = blockIdx.x * blockDim.x + threadIdx.x;
   for (int i = gid; i < a.n_counters; i += gridDim.x * blockDim.x) a.counters[i] = 0;
@@ -309,8 +309,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
   cluster_sync();  // the partner's barriers exist
   tc_fence_after();
   const uint32_t tmem = S.tmem_base;
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
 
   if (warp == 0) {
     {

@@ -371,7 +371,6 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
   tc_fence_after();
   const uint32_t tmem = S.tmem_base;
   const uint32_t tmem_a = tmem + 2 * NT;
-  pdl_launch_dependents();
 
   // stages of a range: its NVFP4 chunks (they come first) take several each above 64 tokens
   constexpr int split = 4 / KB;
@@ -395,6 +394,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
     // ---------------------------------------------------------------- activation boxes
     const bool leader = elect_one();
     pdl_wait();
+    pdl_launch_dependents();
     Cursor x;
     Segment g = segment_at(sc, begin, end);
     for (int i = begin; i < end; ++i) {

@@ -138,8 +138,8 @@ __device__ __forceinline__ void run_rows(const GemvArgs &a, int r, int r8, int w
 template <int NT, bool XBF16>
 __global__ void __launch_bounds__(kWarps * 32) gemv_rows_kernel(const __grid_constant__ GemvArgs a) {
   __shared__ float sums[kWarps][16][8 * NT + 1];
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int t4 = (a.n4 + 15) >> 4, t8 = (a.n8 + 15) >> 4;
@@ -196,8 +196,8 @@ __device__ __forceinline__ float elem(const __half *x, long long i, int bf16) {
 }
 // K not a multiple of 16 (no NVFP4 group then)
 __global__ void __launch_bounds__(256) gemv_scalar_kernel(const __grid_constant__ GemvArgs a) {
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int N = a.n4 + a.n8 + a.n16;

@@ -330,9 +330,11 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
   const int ck = sc.ck;
   const int pitch = (ck >> 1) + 16;
 
-  // Let the next kernel in the stream become resident as early as possible; until this
-  // grid completes it only fills its own shared-memory ring with weights.
-  if (!a.opens) pdl_launch_dependents();
+  // In a chain (RDQ_GEMV_PDL) the next kernel may become resident as early as possible: until this grid
+  // completes it only fills its own shared-memory ring with weights.  Otherwise it may once this one has
+  // waited (the rule at pdl_wait()).
+  const bool first = a.early && !a.opens;
+  if (first) pdl_launch_dependents();
   if (static_cast<int>(blockIdx.x) >= sc.G) {
     // The grid has a CTA for every SM: one without images holds its place until the kernel before is
     // done, so that the next launch finds one free place per SM, not two on some.
@@ -383,7 +385,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
     // Only this thread executes the grid-dependency wait; every other warp of the CTA
     // sleeps on bar_x, which completes after it (and after the activation copies).
     if (!a.beside) pdl_wait();
-    if (a.opens) pdl_launch_dependents();
+    if (!first) pdl_launch_dependents();
     const uint32_t bx = smem_u32(&bar_x);
     if (XS && (!EXTRA || xop == 0)) {
       mbar_arrive_expect_tx(bx, static_cast<uint32_t>(M) * 2u * K);

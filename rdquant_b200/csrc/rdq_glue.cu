@@ -6,10 +6,10 @@
 // HBM/latency-bound kernels of their own because, at one token per step, each of the ~20 framework
 // kernels between two linears costs more than the linear itself.
 //
-// Every kernel takes part in programmatic dependent launch the way the decode GEMV does: it lets
-// its successor become resident at once (griddepcontrol.launch_dependents) -- so the next GEMV
-// fills its weight rings while this kernel runs -- and reads its inputs only after
-// griddepcontrol.wait.  All arithmetic is FP32 with one rounding to FP16 per stored value.
+// Every kernel takes part in programmatic dependent launch the way the decode GEMV does: it reads its
+// inputs only after griddepcontrol.wait, and those that keep the one-CTA-per-SM shape (`first`, see
+// pdl_wait()) let their successor become resident at once, so that the next GEMV fills its weight rings
+// while they run.  All arithmetic is FP32 with one rounding to FP16 per stored value.
 #include "rdq_kernels.cuh"
 
 #include <utility>
@@ -41,11 +41,12 @@ __device__ __forceinline__ void prefetch_l2(const void *p, int bytes) {
 constexpr int kNormVecs = 4;
 
 __global__ void __launch_bounds__(256) add_rmsnorm_kernel(__half *x, const __half *delta, const __half *w, __half *out,
-                                                         int B, int H, float eps) {
+                                                         int B, int H, float eps, bool first) {
   __shared__ float red[32];
-  pdl_launch_dependents();
+  if (first) pdl_launch_dependents();
   if (blockIdx.x == 0 && threadIdx.x == 0) prefetch_l2(w, H * 2);  // a hint while the kernel before runs
   pdl_wait();
+  if (!first) pdl_launch_dependents();
   if (static_cast<int>(blockIdx.x) >= B) {  // the grid has a CTA per SM (see linger())
     linger(1500);
     return;
@@ -119,8 +120,8 @@ __global__ void __launch_bounds__(128) qk_rope_cache_kernel(const __half *qkv, c
                                                            __half *q_out, __half *k_cache, __half *v_cache, int nq, int nkv,
                                                            int dh, int S, float eps) {
   __shared__ float red[32];
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   const int head = blockIdx.x, b = blockIdx.y, i = threadIdx.x, half = dh >> 1;
   const long long p = *pos;
   const __half *src = qkv + (1ll * b * (nq + 2 * nkv) + head) * dh;
@@ -159,8 +160,8 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attn_split_kernel(const __hal
                                                                     const __half *v_cache, const long long *pos,
                                                                     float *part, int nq, int nkv, int dh, int S, int chunk,
                                                                     float scale) {
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
   const int nsplit = gridDim.x, group = nq / nkv;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -223,8 +224,8 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attn_split_kernel(const __hal
 
 // grid = (nq, B), one thread per dimension
 __global__ void __launch_bounds__(256) attn_combine_kernel(const float *part, __half *out, int nq, int dh, int nsplit) {
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   const int head = blockIdx.x, b = blockIdx.y, d = threadIdx.x;
   const float *src = part + (1ll * b * nq + head) * nsplit * (dh + 2);
   float m = -INFINITY;
@@ -241,9 +242,10 @@ __global__ void __launch_bounds__(256) attn_combine_kernel(const float *part, __
 }
 
 // ---- out[b, f] = silu(gu[b, f]) * gu[b, F + f]
-__global__ void __launch_bounds__(256) silu_mul_kernel(const __half *gu, __half *out, int B, int F) {
-  pdl_launch_dependents();
+__global__ void __launch_bounds__(256) silu_mul_kernel(const __half *gu, __half *out, int B, int F, bool first) {
+  if (first) pdl_launch_dependents();
   pdl_wait();
+  if (!first) pdl_launch_dependents();
   // every CTA takes an equal, contiguous share of the 16-byte vectors, so that (nearly) all SMs
   // work and leave together
   const long long total = 1ll * B * (F / 8);
@@ -373,7 +375,7 @@ template <int DH, int NB>
 __global__ void __launch_bounds__(kFusedAttnThreads, 2) rope_attn_kernel(
     const __half *qkv, const __half *qn, const __half *kn, const __half *cos_t, const __half *sin_t, const long long *pos,
     __half *k_cache, __half *v_cache, float *part, int *counters, __half *out, int nq, int nkv, int S, float scale, float eps,
-    int nsplit, int npair) {
+    int nsplit, int npair, bool first) {
   constexpr int W = kFusedAttnWarps;
   constexpr int PITCH = 2 * DH + 16;   // row pitch in shared memory (bytes): an odd multiple of 16
   constexpr int BLK = 16 * PITCH;      // 16 rows of K or of V
@@ -387,7 +389,7 @@ __global__ void __launch_bounds__(kFusedAttnThreads, 2) rope_attn_kernel(
   __half *qs = reinterpret_cast<__half *>(smem + W * 4 * BLK);  // [8 NB][QP]
   float *mrg = reinterpret_cast<float *>(smem);                 // [W][8 NB][PR], over the rings once they are done
 
-  pdl_launch_dependents();
+  if (first) pdl_launch_dependents();
   // The grid has one CTA per SM (or one per (sequence, KV head) when those outnumber the SMs); CTAs
   // beyond the work linger.
   const int pair = static_cast<int>(blockIdx.x) / nsplit, split = static_cast<int>(blockIdx.x) - pair * nsplit;
@@ -410,6 +412,7 @@ __global__ void __launch_bounds__(kFusedAttnThreads, 2) rope_attn_kernel(
     if (kn) prefetch_l2(kn, DH * 2);
   }
   pdl_wait();
+  if (!first) pdl_launch_dependents();
   if (pair >= npair) {
     linger(4000);
     return;
@@ -770,7 +773,8 @@ static bool takes_slot(int B) { return B <= 8; }
 
 int launch_add_rmsnorm(__half *x, const __half *delta, const __half *w, __half *out, int B, int H, float eps, bool pdl,
                        cudaStream_t stream) {
-  return launch_pdl(add_rmsnorm_kernel, dim3(std::max(B, sm_count())), dim3(256), takes_slot(B), pdl, stream, x, delta, w, out, B, H, eps);
+  return launch_pdl(add_rmsnorm_kernel, dim3(std::max(B, sm_count())), dim3(256), takes_slot(B), pdl, stream, x, delta, w, out, B, H,
+                    eps, takes_slot(B));
 }
 
 int launch_qk_rope_cache(const __half *qkv, const __half *qn, const __half *kn, const __half *cos_t, const __half *sin_t,
@@ -820,7 +824,8 @@ int launch_rope_attn(const __half *qkv, const __half *qn, const __half *kn, cons
   const int nb = group <= 8 ? 1 : 2;
   int smem = kFusedAttnWarps * 4 * 16 * (2 * dh + 16) + 8 * nb * (dh + 8) * 2;
   // two CTAs per SM while that is enough for the grid: with three, 256 CTAs were placed on 86 SMs
-  if (nsplit * nkv * B <= 2 * sm_count()) smem = std::max(smem, kSlotSmem);
+  const bool slot = nsplit * nkv * B <= 2 * sm_count();
+  if (slot) smem = std::max(smem, kSlotSmem);
   auto launch = [&](auto kernel) -> int {
     cudaLaunchConfig_t cfg = {};
     // one CTA per SM while the (sequence, KV head) pairs fit: like the GEMVs around it
@@ -835,7 +840,7 @@ int launch_rope_attn(const __half *qkv, const __half *qn, const __half *kn, cons
     cfg.numAttrs = 1;
     RDQ_CUDA(pin_slot(reinterpret_cast<const void *>(kernel), smem));
     RDQ_CUDA(cudaLaunchKernelEx(&cfg, kernel, qkv, qn, kn, cos_t, sin_t, pos, k_cache, v_cache, part, counters, out, nq, nkv, S, scale,
-                                eps, nsplit, nkv * B));
+                                eps, nsplit, nkv * B, slot));
     return RDQ_OK;
   };
   switch (dh) {
@@ -850,7 +855,7 @@ int launch_rope_attn(const __half *qkv, const __half *qn, const __half *kn, cons
 int launch_silu_mul(const __half *gu, __half *out, int B, int F, bool pdl, cudaStream_t stream) {
   const long long total = 1ll * B * (F / 8);
   (void)total;
-  return launch_pdl(silu_mul_kernel, dim3(sm_count()), dim3(256), takes_slot(B), pdl, stream, gu, out, B, F);
+  return launch_pdl(silu_mul_kernel, dim3(sm_count()), dim3(256), takes_slot(B), pdl, stream, gu, out, B, F, takes_slot(B));
 }
 
 }  // namespace rdq

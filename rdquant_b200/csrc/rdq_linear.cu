@@ -11,8 +11,8 @@ namespace {
 
 // HBM-bound: reads and writes 2 bytes per element.
 __global__ void __launch_bounds__(256) cast_rows_kernel(const uint4 *__restrict__ x, uint4 *__restrict__ out, long long nvec) {
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   const long long stride = 1ll * gridDim.x * blockDim.x;
   for (long long i = 1ll * blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += 4 * stride) {
     uint4 v[4];
@@ -28,8 +28,8 @@ __global__ void __launch_bounds__(256) cast_rows_kernel(const uint4 *__restrict_
 }
 __global__ void __launch_bounds__(256) cast_elems_kernel(const __nv_bfloat16 *__restrict__ x, __half *__restrict__ out,
                                                          long long count) {
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   for (long long i = 1ll * blockIdx.x * blockDim.x + threadIdx.x; i < count; i += 1ll * gridDim.x * blockDim.x)
     out[i] = __float2half_rn(__bfloat162float(x[i]));
 }

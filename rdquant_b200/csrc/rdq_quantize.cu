@@ -402,7 +402,7 @@ struct Piece {
 // waited three times per row: 20 us for 2560 x 9728, now 18, with the second pass 13.5 -> 10 us.
 template <typename T>
 __global__ void __launch_bounds__(256, 4) encode_layer_kernel(LayerEncodeArgs a) {
-  pdl_launch_dependents();
+  pdl_launch_dependents();  // (launched in stream order: everything before it is complete)
   __shared__ float red[2][8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int K = a.K, nvec = K >> 3, tasks = (a.n4 + a.n8 + a.n16) * a.segs, stride = (gridDim.x * blockDim.x) >> 5;
@@ -454,7 +454,6 @@ __global__ void __launch_bounds__(256, 4) encode_layer_kernel(LayerEncodeArgs a)
 // Second pass: the FP8 rows (their scale is known now; they mostly come out of L2)
 template <typename T>
 __global__ void __launch_bounds__(256, 4) encode_layer_fp8_kernel(LayerEncodeArgs a, int blocks) {
-  pdl_launch_dependents();
   __shared__ float red[2][8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nvec = a.K >> 3, tasks = a.n8 * a.segs, stride = (gridDim.x * blockDim.x) >> 5;
@@ -462,6 +461,7 @@ __global__ void __launch_bounds__(256, 4) encode_layer_fp8_kernel(LayerEncodeArg
   int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (t < tasks) cur.load(a, t, a.n4, lane);  // (inputs of both passes)
   pdl_wait();
+  pdl_launch_dependents();
   float m[2] = {0.f, 0.f};
   for (int i = threadIdx.x; i < blocks; i += blockDim.x) {
     const float2 p = __ldcg(reinterpret_cast<const float2 *>(a.tops) + i);

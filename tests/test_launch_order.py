@@ -1,0 +1,47 @@
+"""The order of programmatic launches, read from the kernels' sources: a kernel waits for the launch before
+it and only then lets the next one start, unless it keeps the shape that bounds how many launches an SM
+has places for (the rule at pdl_wait() in rdq_common.cuh)."""
+import glob
+import os
+import re
+
+from conftest import ROOT
+
+CSRC = os.path.join(ROOT, "rdquant_b200", "csrc")
+# one CTA per SM with the shared memory of a place, in every launch
+ALWAYS_ONE_PER_SM = {"stage_copy_kernel", "peer_gather_kernel"}
+# launched in stream order: nothing to wait for
+STREAM_ORDER = {"decode_rows_kernel", "encode_layer_kernel"}
+
+
+def _kernels():
+    """(name, body) of every __global__ function."""
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.inl"))):
+        text = re.sub(r"//[^\n]*", "", open(path).read())
+        for m in re.finditer(r"__global__", text):
+            start = text.index("{", m.end())
+            name = re.findall(r"(\w+)\s*\(", text[m.end():start])
+            depth, i = 0, start
+            while True:
+                depth += {"{": 1, "}": -1}.get(text[i], 0)
+                i += 1
+                if depth == 0:
+                    break
+            yield next(n for n in name if n.endswith("_kernel")), text[start:i]
+
+
+def test_kernels_wait_before_they_let_the_next_launch_start():
+    seen = set()
+    for name, body in _kernels():
+        if "pdl_launch_dependents()" not in body:
+            continue
+        seen.add(name)
+        wait = body.find("pdl_wait()")
+        if name in STREAM_ORDER:
+            assert wait < 0, name
+            continue
+        assert wait >= 0, name
+        for m in re.finditer(r"([^\n]*)pdl_launch_dependents\(\)", body):
+            early = m.start() < wait
+            assert not early or name in ALWAYS_ONE_PER_SM or "if (first)" in m.group(1), name
+    assert {"gemv_tiled_kernel", "gemm_stream_kernel", "gemm_pair_kernel", "gemv_rows_kernel", "rope_attn_kernel"} <= seen
