@@ -4,8 +4,9 @@
 // call needs (pointers, sizes, references that keep the tensors alive).  Its `linear(x, bias,
 // flags)` checks the input, allocates the output with torch's CUDA allocator, takes torch's current
 // stream and calls rdq_linear (include/rdq_b200.h).  What the fast path does not take -- another
-// dtype, a non-contiguous or host tensor, a wrong last dimension -- returns None, and the caller's
-// Python path handles or refuses it.
+// dtype, a non-contiguous or host tensor, a wrong last dimension, a tensor whose memory cannot be asked
+// for (of tracing or vmap, a sparse layout: the accessors throw or answer null) -- returns None, and the
+// caller's Python path handles or refuses it.  No C++ exception leaves an entry point.
 //
 // Why native: a decode step calls dozens of linears whose kernels take 5-10 us, and the same
 // checks, allocation and ctypes call written in Python took 25-33 us per call.
@@ -88,6 +89,29 @@ int32_t *words_of(c10::DeviceIndex device, const c10::cuda::CUDAStream &stream, 
   return static_cast<int32_t *>(sets.back().t.data_ptr());
 }
 
+// f() with a C++ exception as a RuntimeError (a Python exception behind it stays what it is) and null
+template <typename F>
+PyObject *guarded(F f) {
+  try {
+    return f();
+  } catch (const std::exception &e) {
+    if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, e.what());
+  } catch (...) {
+    if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "unknown C++ exception");
+  }
+  return nullptr;
+}
+// f(), a look at arguments: false also where an accessor throws
+template <typename F>
+bool accepts(F f) {
+  try {
+    return f();
+  } catch (...) {
+    PyErr_Clear();
+    return false;
+  }
+}
+
 bool take(LayerObject *self, PyObject *dict, const char *key, const void **out) {
   *out = nullptr;
   PyObject *v = PyDict_GetItemString(dict, key);  // borrowed
@@ -107,6 +131,10 @@ bool take(LayerObject *self, PyObject *dict, const char *key, const void **out) 
     return false;
   }
   *out = t.data_ptr();
+  if (*out == nullptr && t.numel() != 0) {
+    PyErr_Format(PyExc_RuntimeError, "%s has no memory", key);
+    return false;
+  }
   self->keep->push_back(t);
   return true;
 }
@@ -121,18 +149,11 @@ bool take_int(PyObject *dict, const char *key, int *out) {
   return !(PyErr_Occurred());
 }
 
-PyObject *layer_new(PyTypeObject *type, PyObject *args, PyObject *) {
-  PyObject *dict = nullptr;
-  if (!PyArg_ParseTuple(args, "O!", &PyDict_Type, &dict)) return nullptr;
-  LayerObject *self = reinterpret_cast<LayerObject *>(type->tp_alloc(type, 0));
-  if (self == nullptr) return nullptr;
-  ++layers_alive;
-  self->keep = new (std::nothrow) std::vector<at::Tensor>();
-  self->device = -1;
+// the fields of a new object; false with an exception set
+bool fill_layer(LayerObject *self, PyObject *dict) {
   rdq_layer &l = self->layer;
-  l = rdq_layer{};
   const void *s8 = nullptr, *perm = nullptr, *inv = nullptr, *ws = nullptr, *cnt = nullptr;
-  bool ok = self->keep != nullptr && take_int(dict, "n_fp4", &l.n_fp4) && take_int(dict, "n_fp8", &l.n_fp8) &&
+  bool ok = take_int(dict, "n_fp4", &l.n_fp4) && take_int(dict, "n_fp8", &l.n_fp8) &&
             take_int(dict, "n_fp16", &l.n_fp16) && take_int(dict, "k", &l.K) && take(self, dict, "w_fp4_q", &l.w_fp4) &&
             take(self, dict, "w_fp4_scales", &l.w_fp4_scales) && take(self, dict, "w_fp8_q", &l.w_fp8) &&
             take(self, dict, "w_fp8_scales", &s8) && take(self, dict, "w_fp16", &l.w_fp16) &&
@@ -145,18 +166,31 @@ PyObject *layer_new(PyTypeObject *type, PyObject *args, PyObject *) {
       ok = !PyErr_Occurred();
     }
   }
-  if (!ok) {
-    if (!PyErr_Occurred()) PyErr_NoMemory();
-    Py_DECREF(self);
-    return nullptr;
-  }
+  if (!ok) return false;
   l.w_fp8_scales = static_cast<const float *>(s8);
   l.perm = static_cast<const int32_t *>(perm);
   l.inv_perm = static_cast<const int32_t *>(inv);
   l.gemv_ws = const_cast<void *>(ws);
   l.gemv_counters = static_cast<int32_t *>(const_cast<void *>(cnt));
   self->n_out = static_cast<int64_t>(l.n_fp4) + l.n_fp8 + l.n_fp16;
-  return reinterpret_cast<PyObject *>(self);
+  return true;
+}
+
+PyObject *layer_new(PyTypeObject *type, PyObject *args, PyObject *) {
+  PyObject *dict = nullptr;
+  if (!PyArg_ParseTuple(args, "O!", &PyDict_Type, &dict)) return nullptr;
+  LayerObject *self = reinterpret_cast<LayerObject *>(type->tp_alloc(type, 0));
+  if (self == nullptr) return nullptr;
+  ++layers_alive;
+  self->layer = rdq_layer{};
+  self->device = -1;
+  self->keep = nullptr;
+  PyObject *made = guarded([&]() -> PyObject * {
+    self->keep = new std::vector<at::Tensor>();
+    return fill_layer(self, dict) ? reinterpret_cast<PyObject *>(self) : nullptr;
+  });
+  if (made == nullptr) Py_DECREF(self);
+  return made;
 }
 
 void layer_dealloc(PyObject *obj) {
@@ -172,28 +206,33 @@ PyObject *layer_linear(PyObject *obj, PyObject *const *args, Py_ssize_t nargs) {
     PyErr_SetString(PyExc_TypeError, "linear(x, bias, flags)");
     return nullptr;
   }
+  const long flags = PyLong_AsLong(args[2]);
+  if (flags == -1 && PyErr_Occurred()) return nullptr;
   const rdq_layer &l = self->layer;
   const at::Tensor &x = THPVariable_Unpack(args[0]);
-  const int64_t dims = x.dim();
-  const auto type = x.scalar_type();
-  if (!x.is_cuda() || x.get_device() != self->device || dims < 1 || x.size(dims - 1) != l.K || !x.is_contiguous() ||
-      (type != at::kHalf && type != at::kBFloat16) || l.K == 0)
-    Py_RETURN_NONE;
-  const int64_t m = x.numel() / l.K;
-  const void *xp = x.data_ptr();
-  if (m == 0 || m > 0x7fffffff || (reinterpret_cast<uintptr_t>(xp) & 15)) Py_RETURN_NONE;
-  const void *bias = nullptr;
-  if (args[1] != Py_None) {
-    if (!THPVariable_Check(args[1])) Py_RETURN_NONE;
+  int64_t dims = 0, m = 0;
+  auto type = at::kHalf;
+  const void *xp = nullptr, *bias = nullptr;
+  const bool ok = accepts([&] {
+    dims = x.dim();
+    type = x.scalar_type();
+    if (!x.is_cuda() || x.get_device() != self->device || dims < 1 || x.size(dims - 1) != l.K || !x.is_contiguous() ||
+        (type != at::kHalf && type != at::kBFloat16) || l.K == 0)
+      return false;
+    m = x.numel() / l.K;
+    xp = x.data_ptr();
+    if (m == 0 || m > 0x7fffffff || xp == nullptr || (reinterpret_cast<uintptr_t>(xp) & 15)) return false;
+    if (args[1] == Py_None) return true;
+    if (!THPVariable_Check(args[1])) return false;
     const at::Tensor &b = THPVariable_Unpack(args[1]);
     if (!b.is_cuda() || b.get_device() != self->device || b.scalar_type() != at::kHalf || !b.is_contiguous() ||
         b.numel() != self->n_out)
-      Py_RETURN_NONE;
+      return false;
     bias = b.data_ptr();
-  }
-  const long flags = PyLong_AsLong(args[2]);
-  if (flags == -1 && PyErr_Occurred()) return nullptr;
-  try {
+    return bias != nullptr || self->n_out == 0;
+  });
+  if (!ok) Py_RETURN_NONE;
+  return guarded([&]() -> PyObject * {
     OnDevice guard(self->device);
     const c10::Device device(c10::kCUDA, self->device);
     at::Tensor y;
@@ -229,10 +268,7 @@ PyObject *layer_linear(PyObject *obj, PyObject *const *args, Py_ssize_t nargs) {
       return nullptr;
     }
     return THPVariable_Wrap(std::move(y));
-  } catch (const std::exception &e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
-  }
+  });
 }
 
 at::Tensor cuda_empty(at::IntArrayRef sizes, at::ScalarType type, c10::DeviceIndex device) {
@@ -267,16 +303,28 @@ PyObject *quantize_layer(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     PyErr_SetString(PyExc_TypeError, "quantize_layer(weight, perm, n4, n8, n16)");
     return nullptr;
   }
-  const at::Tensor *w = cuda_arg(args[0], -1, {at::kHalf, at::kFloat});
-  if (w == nullptr || w->dim() != 2) Py_RETURN_NONE;
-  const c10::DeviceIndex dev = w->get_device();
-  const at::Tensor *perm = cuda_arg(args[1], dev, {at::kLong});
   if (!int_args(args + 2, 3, n)) return nullptr;
-  const int64_t N = w->size(0), K = w->size(1);
-  if (perm == nullptr || perm->numel() != N || n[0] < 0 || n[1] < 0 || n[2] < 0 || n[0] + n[1] + n[2] != N || K % 16 || K == 0 ||
-      N == 0 || N > 0x7fffffff || K > 0x7fffffff || (reinterpret_cast<uintptr_t>(w->data_ptr()) & 15))
-    Py_RETURN_NONE;
-  try {
+  const at::Tensor *w = nullptr;
+  const void *wp = nullptr;
+  const long long *pp = nullptr;
+  int64_t N = 0, K = 0;
+  c10::DeviceIndex dev = -1;
+  const bool ok = accepts([&] {
+    w = cuda_arg(args[0], -1, {at::kHalf, at::kFloat});
+    if (w == nullptr || w->dim() != 2) return false;
+    dev = w->get_device();
+    N = w->size(0);
+    K = w->size(1);
+    const at::Tensor *perm = cuda_arg(args[1], dev, {at::kLong});
+    if (perm == nullptr || perm->numel() != N || n[0] < 0 || n[1] < 0 || n[2] < 0 || n[0] + n[1] + n[2] != N || K % 16 || K == 0 ||
+        N == 0 || N > 0x7fffffff || K > 0x7fffffff)
+      return false;
+    wp = w->data_ptr();
+    pp = static_cast<const long long *>(perm->data_ptr());
+    return wp != nullptr && pp != nullptr && (reinterpret_cast<uintptr_t>(wp) & 15) == 0;
+  });
+  if (!ok) Py_RETURN_NONE;
+  return guarded([&]() -> PyObject * {
     OnDevice guard(dev);
     at::Tensor codes, scales, top, fp8, fp8_scale, fp16;
     if (n[0]) {
@@ -291,7 +339,7 @@ PyObject *quantize_layer(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     if (n[2]) fp16 = cuda_empty({n[2], K}, at::kBFloat16, dev);
     at::Tensor inv = cuda_empty({N}, at::kInt, dev), scratch = cuda_empty({RDQ_QUANTIZE_LAYER_SCRATCH}, at::kFloat, dev);
     auto ptr = [](const at::Tensor &t) { return t.defined() ? t.data_ptr() : nullptr; };
-    const int rc = rdq_quantize_layer(w->data_ptr(), w->scalar_type() == at::kFloat, static_cast<const long long *>(perm->data_ptr()),
+    const int rc = rdq_quantize_layer(wp, w->scalar_type() == at::kFloat, pp,
                                       static_cast<int>(n[0]), static_cast<int>(n[1]), static_cast<int>(n[2]), static_cast<int>(K),
                                       ptr(codes), ptr(scales), static_cast<float *>(ptr(top)), ptr(fp8),
                                       static_cast<float *>(ptr(fp8_scale)), ptr(fp16), static_cast<int32_t *>(inv.data_ptr()),
@@ -305,10 +353,7 @@ PyObject *quantize_layer(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     return Py_BuildValue("NNNNNNNN", wrap_or_none(std::move(codes)), wrap_or_none(std::move(scales)), wrap_or_none(std::move(top)),
                          wrap_or_none(std::move(fp8)), wrap_or_none(std::move(fp8_scale)), wrap_or_none(std::move(fp16)),
                          wrap_or_none(std::move(inv)), wrap_or_none(std::move(splits)));
-  } catch (const std::exception &e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
-  }
+  });
 }
 
 // dequantize(w4, s4, w8, s8, w16, inv_perm or None, n4, n8, n16, k) -> f16 [N, K], or None when an argument needs the
@@ -331,14 +376,18 @@ PyObject *dequantize(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     if (i != 3 && i != 5 && (t->dim() != 2 || t->size(0) != (i == 4 ? n[2] : n[i / 2]))) return false;
     dev = t->get_device();
     p[i] = t->data_ptr();
+    if (p[i] == nullptr) return false;
     if (i == 4) bf16 = t->scalar_type() == at::kBFloat16;
     return true;
   };
-  if (n[0] && !(take_arg(0, {at::kByte}, n[0] * (K / 2)) && take_arg(1, {at::kByte}, n[0] * (K / 16)))) Py_RETURN_NONE;
-  if (n[1] && !(take_arg(2, {at::kByte}, n[1] * K) && take_arg(3, {at::kFloat}, n[1]))) Py_RETURN_NONE;
-  if (n[2] && !take_arg(4, {at::kHalf, at::kBFloat16}, n[2] * K)) Py_RETURN_NONE;
-  if (args[5] != Py_None && !take_arg(5, {at::kInt}, N)) Py_RETURN_NONE;
-  try {
+  const bool ok = accepts([&] {
+    if (n[0] && !(take_arg(0, {at::kByte}, n[0] * (K / 2)) && take_arg(1, {at::kByte}, n[0] * (K / 16)))) return false;
+    if (n[1] && !(take_arg(2, {at::kByte}, n[1] * K) && take_arg(3, {at::kFloat}, n[1]))) return false;
+    if (n[2] && !take_arg(4, {at::kHalf, at::kBFloat16}, n[2] * K)) return false;
+    return args[5] == Py_None || take_arg(5, {at::kInt}, N);
+  });
+  if (!ok) Py_RETURN_NONE;
+  return guarded([&]() -> PyObject * {
     OnDevice guard(dev);
     at::Tensor out = cuda_empty({N, K}, at::kHalf, dev);
     const int rc = rdq_dequant_packed(p[0], p[1], 1.0f, p[2], static_cast<const float *>(p[3]), p[4], bf16,
@@ -350,10 +399,7 @@ PyObject *dequantize(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
       return nullptr;
     }
     return THPVariable_Wrap(std::move(out));
-  } catch (const std::exception &e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
-  }
+  });
 }
 
 // drop_words() -> number of sets dropped: the next calls start with zeroed ones (after a time-out, which
