@@ -145,6 +145,8 @@ def _bind(lib: ctypes.CDLL) -> None:
     lib.rdq_quantize_fp8.argtypes = [vp, i32, i32, i32, vp, vp, vp, vp, vp]
     lib.rdq_quantize_layer.restype = i32
     lib.rdq_quantize_layer.argtypes = [vp, i32, vp, i32, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, vp]
+    lib.rdq_quantize_status.restype = i32
+    lib.rdq_quantize_status.argtypes = [vp]
     lib.rdq_add_rmsnorm.restype = i32
     lib.rdq_add_rmsnorm.argtypes = [vp, vp, vp, vp, i32, i32, f32, i32, vp]
     lib.rdq_qk_rope_cache.restype = i32
@@ -195,6 +197,7 @@ EXPORTS = [
     "rdq_quantize_nvfp4",
     "rdq_quantize_fp8",
     "rdq_quantize_layer",
+    "rdq_quantize_status",
     "rdq_linear",
     "rdq_linear_words",
     "rdq_linear_workspace_size",

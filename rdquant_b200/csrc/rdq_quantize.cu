@@ -370,12 +370,14 @@ struct LayerEncodeArgs {
   int segs;     // pieces of a row
   float *global_scale;
   int32_t *inv_perm;
+  int *bad_index;  // pinned host word: 1 once an entry of a permutation was out of range
 };
+// channel of permuted row r, or -1
 __device__ __forceinline__ long long source_row(const LayerEncodeArgs &a, int r) {
   const int n = a.n4 + a.n8 + a.n16;
   long long s = a.perm[r];
   if (s < 0) s += n;  // indices from the end, as in tensor indexing
-  return s < 0 || s >= n ? 0 : s;
+  return s < 0 || s >= n ? -1 : s;
 }
 
 // Pieces of rows as a warp takes them: kPiece vectors per lane, those of the next piece loaded before
@@ -388,7 +390,7 @@ struct Piece {
   __device__ __forceinline__ void load(const LayerEncodeArgs &a, int t, int first_row, int lane) {
     r = t / a.segs;
     v0 = (t - r * a.segs) * 32 * kPiece + lane;
-    const T *row = static_cast<const T *>(a.w) + source_row(a, first_row + r) * a.K;
+    const T *row = static_cast<const T *>(a.w) + max(source_row(a, first_row + r), 0ll) * a.K;
 #pragma unroll
     for (int u = 0; u < kPiece; ++u)
       if (v0 + 32 * u < (a.K >> 3)) q[u].load(row + 8ll * (v0 + 32 * u));
@@ -413,7 +415,11 @@ __global__ void __launch_bounds__(256, 4) encode_layer_kernel(LayerEncodeArgs a)
   for (; t < tasks; t += stride) {
     if (t + stride < tasks) next.load(a, t + stride, 0, lane);
     const int r = cur.r, v0 = cur.v0;
-    if (v0 == 0) a.inv_perm[source_row(a, r)] = r;
+    if (v0 == 0) {
+      const long long s = source_row(a, r);
+      if (s >= 0) a.inv_perm[s] = r;
+      else *static_cast<volatile int *>(a.bad_index) = 1;  // (the row has channel 0's values)
+    }
 #pragma unroll
     for (int u = 0; u < kPiece; ++u) {
       const int i = v0 + 32 * u;
@@ -451,7 +457,8 @@ __global__ void __launch_bounds__(256, 4) encode_layer_kernel(LayerEncodeArgs a)
   }
 }
 
-// Second pass: the FP8 rows (their scale is known now; they mostly come out of L2)
+// Second pass: the FP8 rows (their scale is known now; they mostly come out of L2).  Channels that the
+// permutation does not name get row 0 as their inverse: whoever reads it finds an index in range.
 template <typename T>
 __global__ void __launch_bounds__(256, 4) encode_layer_fp8_kernel(LayerEncodeArgs a, int blocks) {
   __shared__ float red[2][8];
@@ -492,6 +499,11 @@ __global__ void __launch_bounds__(256, 4) encode_layer_fp8_kernel(LayerEncodeArg
     if (cur.v0 == 0) a.fp8_scale[cur.r] = scale;
     cur = next;
   }
+  const int n = a.n4 + a.n8 + a.n16;
+  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+    const int r = __ldcg(a.inv_perm + j);
+    if (r < 0 || r >= n || source_row(a, r) != j) a.inv_perm[j] = 0;
+  }
 }
 
 int grid_for_rows(int n) {
@@ -506,6 +518,32 @@ int one_wave(K kernel) {
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, 0) != cudaSuccess || per_sm < 1) per_sm = 1;
   return std::min(sm_count() * per_sm, RDQ_QUANTIZE_LAYER_SCRATCH / 2);
+}
+
+// The pinned word of LayerEncodeArgs::bad_index, one per process.
+int bad_index_word(int **out) {
+  static std::mutex mu;
+  static int *word = nullptr;
+  std::lock_guard<std::mutex> lock(mu);
+  if (word == nullptr) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // the allocation is no part of a capture
+    RDQ_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    void *p = nullptr;
+    const cudaError_t e = cudaHostAlloc(&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    RDQ_CUDA(e);
+    word = static_cast<int *>(p);
+    *word = 0;
+  }
+  *out = word;
+  return RDQ_OK;
+}
+int report_bad_index(int *word) {
+  if (*static_cast<volatile int *>(word) == 0) return RDQ_OK;
+  *static_cast<volatile int *>(word) = 0;
+  RDQ_REQUIRE(false, RDQ_E_INVALID, "rdq_quantize_layer: a permutation given to an earlier call had an entry out of range; "
+              "its tensors are invalid");
+  return RDQ_OK;
 }
 
 template <typename T>
@@ -580,6 +618,9 @@ extern "C" int rdq_quantize_layer(const void *w, int w_is_f32, const long long *
               "w and the outputs must be 16-byte aligned");
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   LayerEncodeArgs a;
+  int rc = bad_index_word(&a.bad_index);
+  if (rc == RDQ_OK) rc = report_bad_index(a.bad_index);
+  if (rc != RDQ_OK) return rc;
   a.w = w;
   a.perm = perm;
   a.n4 = n_fp4;
@@ -596,4 +637,12 @@ extern "C" int rdq_quantize_layer(const void *w, int w_is_f32, const long long *
   a.global_scale = global_scale;
   a.inv_perm = inv_perm;
   return w_is_f32 ? run_layer<float>(a, stream) : run_layer<__half>(a, stream);
+}
+
+extern "C" int rdq_quantize_status(void *stream) {
+  int *word = nullptr;
+  const int rc = bad_index_word(&word);
+  if (rc != RDQ_OK) return rc;
+  RDQ_CUDA(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)));
+  return report_bad_index(word);
 }

@@ -107,7 +107,9 @@ def quantize_weight_packed(weight: torch.Tensor, permutation: torch.Tensor, spli
     straight from a CUDA weight ``[N, K]`` (K % 16 == 0), encoded by the CUDA encoders.
 
     Byte-identical to the host route (rdquant/quantize.py:233-280 followed by
-    rdquant/integrations/hf_export.py:58-125); tensors stay on the weight's device.
+    rdquant/integrations/hf_export.py:58-125); tensors stay on the weight's device.  An entry of the
+    permutation out of range raises ``IndexError``; in a CUDA permutation it is found on the device and
+    raises at the next call, when the layer is packed, or in ``rdquant_cuda.check_quantize_status``.
     """
     from rdquant_b200 import rdquant_cuda
 
@@ -117,11 +119,17 @@ def quantize_weight_packed(weight: torch.Tensor, permutation: torch.Tensor, spli
     perm = permutation.to(device=weight.device, dtype=torch.long)
     if sum(splits.get(f, 0) for f in FORMAT_ORDER) != n_out:
         raise ValueError("splits must sum to the number of output channels")
+    if not permutation.is_cuda and permutation.numel():
+        low, high = int(permutation.min()), int(permutation.max())
+        if low < -n_out or high >= n_out:
+            raise IndexError(f"permutation entry out of range for {n_out} channels: {low if low < -n_out else high}")
     sizes = [int(splits.get(f, 0)) for f in FORMAT_ORDER]
     w = weight if weight.dtype in (torch.float16, torch.float32) else weight.float()
     # two launches that gather the rows as they encode them; None: a shape or layout it does not take
     packed = _lib.torch_ext().quantize_layer(w.contiguous(), perm.contiguous(), *sizes)
     if packed is not None:
+        if rdquant_cuda.VALIDATE:
+            rdquant_cuda.check_quantize_status(weight.device)
         out = {"splits": packed[7], "inv_permutation": packed[6]}
         names = ("weight_nvfp4", "weight_nvfp4_scale", "nvfp4_global_scale", "weight_fp8", "weight_fp8_scale", "weight_fp16")
         out.update((name, t) for name, t in zip(names, packed) if t is not None)

@@ -103,6 +103,14 @@ def check_gemm_status(device) -> None:
     _lib.check(rc, "rdq_gemm_status")
 
 
+def check_quantize_status(device) -> None:
+    """Wait for the work queued on the current stream and raise ``RuntimeError`` if a permutation given to
+    ``quantize_weight_packed`` as a CUDA tensor had an entry out of range (its tensors are then invalid)."""
+    device = torch.device(device)
+    with _on_device(device):
+        _lib.check(_lib.lib().rdq_quantize_status(_stream(device)), "rdq_quantize_status")
+
+
 def check_linear_status(fd: dict) -> None:
     """Both, for a call that may have run on either kind of kernel."""
     check_status(fd)

@@ -248,3 +248,35 @@ def test_one_layer_on_several_streams(rows):
         assert torch.equal(y, refs[i % 3])
     assert all(torch.equal(y, refs[3]) for y in captured)
     rc.check_gemm_status("cuda")
+
+
+@pytest.mark.parametrize("k", [512, 1040])
+@pytest.mark.parametrize("bad", [120, 1 << 40, -121])
+def test_layer_encoder_refuses_bad_permutations(k, bad):
+    """Entries out of range: refused at once on the host; on the device found without an access out of range,
+    reported once, and the inverse holds valid rows."""
+    splits = dict(zip(ORDER, (60, 40, 20)))
+    w = _weights(120, k, k, torch.float16).cuda()
+    perm = torch.randperm(120, generator=torch.Generator().manual_seed(k))
+    rc.check_quantize_status("cuda")
+    good = quantize_weight_packed(w, perm, splits)
+    wrong = perm.clone()
+    wrong[77] = bad
+    with pytest.raises(IndexError, match="out of range"):
+        quantize_weight_packed(w, wrong, splits)
+    for report in (lambda: rc.check_quantize_status("cuda"), lambda: quantize_weight_packed(w, perm, splits)):
+        inv = quantize_weight_packed(w, wrong.cuda(), splits)["inv_permutation"]
+        assert int(inv.min()) >= 0 and int(inv.max()) < 120
+        inv[perm[77]] = 77
+        assert torch.equal(inv, good["inv_permutation"]), "the other channels are where they belong"
+        with pytest.raises(RuntimeError, match="entry out of range"):
+            report()
+    rc.check_quantize_status("cuda")
+    fromend = quantize_weight_packed(w, (perm - 120).cuda(), splits)
+    for key in good:
+        assert torch.equal(good[key], fromend[key]), key
+    twice = perm.clone()
+    twice[5] = twice[6]  # not a permutation, but indices all the same
+    inv = quantize_weight_packed(w, twice.cuda(), splits)["inv_permutation"]
+    assert int(inv.min()) >= 0 and int(inv.max()) < 120 and int(inv[perm[5]]) == 0
+    rc.check_quantize_status("cuda")
