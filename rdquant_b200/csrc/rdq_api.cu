@@ -27,9 +27,7 @@ int sm_count() {
   return n;
 }
 
-namespace {
-
-// Shape / pointer checks shared by the three operators; mirrors the
+// Shape / pointer checks shared by the operators; mirrors the
 // TORCH_CHECKs of the reference wrapper (rdquant/csrc/bindings.cpp:167-182).
 int check_layer(const void *w_fp4, const void *w_fp4_scales, const void *w_fp8,
                 const float *w_fp8_scales, const void *w_fp16, int n4, int n8, int n16, int K) {
@@ -53,7 +51,6 @@ int check_layer(const void *w_fp4, const void *w_fp4_scales, const void *w_fp8,
   return RDQ_OK;
 }
 
-}  // namespace
 }  // namespace rdq
 
 using namespace rdq;

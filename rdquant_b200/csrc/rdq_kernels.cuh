@@ -51,6 +51,10 @@ struct GemmArgs {
   int test_timeout = 0;  // self-test: CTA (0,0,0) ends with a wait that runs out
 };
 
+// RDQ_OK, or an error when sizes, pointers or alignments are not what the row-major kernels rely on (rdq_api.cu)
+int check_layer(const void *w_fp4, const void *w_fp4_scales, const void *w_fp8, const float *w_fp8_scales, const void *w_fp16,
+                int n4, int n8, int n16, int K);
+
 int launch_dequant(const void *w_fp4, const void *w_fp4_scales, float global4, const void *w_fp8,
                    const float *w_fp8_scales, const void *w_fp16, int fp16_is_bf16,
                    const int32_t *inv_perm, void *w_out, int out_is_f32, int n4, int n8, int n16,

@@ -136,6 +136,24 @@ int run_gemv(const rdq_layer &l, bool tiled, const void *x, int x_bf16, int M, c
   return launch_gemv_generic(a, stream);
 }
 
+// What the kernels rely on, for every layout that the layer carries: the entry points of the single
+// kernels check the same.
+int check_layouts(const rdq_layer &l) {
+  RDQ_REQUIRE(l.n_fp4 >= 0 && l.n_fp8 >= 0 && l.n_fp16 >= 0 && l.K > 0, RDQ_E_INVALID, "bad layer shape");
+  RDQ_REQUIRE(l.w_tiled || has_row_major(l), RDQ_E_INVALID, "the layer has neither the tiled nor the row-major tensors");
+  if (has_row_major(l)) {
+    const int rc = check_layer(l.w_fp4, l.w_fp4_scales, l.w_fp8, l.w_fp8_scales, l.w_fp16, l.n_fp4, l.n_fp8, l.n_fp16, l.K);
+    if (rc != RDQ_OK) return rc;
+  }
+  if (l.w_tiled) {
+    RDQ_REQUIRE(l.n_fp4 + l.n_fp8 + l.n_fp16 == 0 || tiled_supported(l.n_fp4, l.n_fp8, l.n_fp16, l.K), RDQ_E_UNSUPPORTED,
+                "shape has no tiled layout (K=%d, n=%d/%d/%d)", l.K, l.n_fp4, l.n_fp8, l.n_fp16);
+    RDQ_REQUIRE(aligned16(l.w_tiled), RDQ_E_INVALID, "w_tiled must be 16-byte aligned");
+    RDQ_REQUIRE(l.n_fp8 == 0 || l.w_fp8_scales, RDQ_E_INVALID, "w_fp8_scales must not be null when n_fp8 > 0");
+  }
+  return RDQ_OK;
+}
+
 }  // namespace
 
 int launch_cast_rows(const void *x_bf16, void *x_f16, long long count, bool pdl, cudaStream_t stream) {
@@ -171,7 +189,12 @@ using namespace rdq;
 extern "C" {
 
 int rdq_linear_workspace_size(const rdq_layer *layer, int M, int x_type, size_t *bytes) {
-  RDQ_REQUIRE(layer && bytes && M >= 0, RDQ_E_INVALID, "bad arguments to rdq_linear_workspace_size");
+  RDQ_REQUIRE(layer && bytes && M >= 0 && (x_type == RDQ_F16 || x_type == RDQ_BF16), RDQ_E_INVALID,
+              "bad arguments to rdq_linear_workspace_size");
+  const int rc = check_layouts(*layer);
+  if (rc != RDQ_OK) return rc;
+  *bytes = 0;
+  if (M == 0 || layer->n_fp4 + layer->n_fp8 + layer->n_fp16 == 0) return RDQ_OK;
   const Need n = need_of(*layer, path_of(*layer, M, x_type), M, x_type);
   *bytes = n.cast + n.gemm;
   return RDQ_OK;
@@ -188,10 +211,11 @@ int rdq_linear_words(const rdq_layer *layer, const void *x, int x_type, int M, c
   RDQ_REQUIRE(layer != nullptr && M >= 0 && (x_type == RDQ_F16 || x_type == RDQ_BF16), RDQ_E_INVALID, "bad arguments to rdq_linear");
   const rdq_layer &l = *layer;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  int rc = check_layouts(l);
+  if (rc != RDQ_OK) return rc;
   const int N = l.n_fp4 + l.n_fp8 + l.n_fp16;
   if (M == 0 || N == 0) return RDQ_OK;
   const Path p = path_of(l, M, x_type);
-  RDQ_REQUIRE(l.w_tiled || has_row_major(l), RDQ_E_INVALID, "the layer has neither the tiled nor the row-major tensors");
   RDQ_REQUIRE(x && y, RDQ_E_INVALID, "x and y must not be null");
   const Need need = need_of(l, p, M, x_type);
   RDQ_REQUIRE(need.cast + need.gemm <= workspace_bytes && (need.cast + need.gemm == 0 || (workspace && aligned16(workspace))),
@@ -207,7 +231,7 @@ int rdq_linear_words(const rdq_layer *layer, const void *x, int x_type, int M, c
   if (cast_inside) {
     xh = workspace;
   } else if (need.cast) {
-    const int rc = launch_cast_rows(x, workspace, 1ll * M * l.K, pdl, stream);
+    rc = launch_cast_rows(x, workspace, 1ll * M * l.K, pdl, stream);
     if (rc != RDQ_OK) return rc;
     xh = workspace;
     x_bf16 = 0;
@@ -224,7 +248,7 @@ int rdq_linear_words(const rdq_layer *layer, const void *x, int x_type, int M, c
       RDQ_REQUIRE(aligned16(xh) || (!tiled && l.K % 16 != 0), RDQ_E_INVALID, "x must be 16-byte aligned");
       for (int r0 = 0; r0 < M; r0 += RDQ_MAX_GEMV_M) {
         const int m = M - r0 < RDQ_MAX_GEMV_M ? M - r0 : RDQ_MAX_GEMV_M;
-        const int rc = run_gemv(l, tiled, static_cast<const char *>(xh) + 2ll * r0 * l.K, x_bf16, m, bias,
+        rc = run_gemv(l, tiled, static_cast<const char *>(xh) + 2ll * r0 * l.K, x_bf16, m, bias,
                                 static_cast<char *>(y) + 2ll * r0 * N, bf16, pdl, stream);
         if (rc != RDQ_OK) return rc;
       }

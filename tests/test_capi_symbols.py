@@ -4,6 +4,8 @@ import ctypes
 import os
 import re
 
+import pytest
+
 from conftest import ROOT
 from rdquant_b200 import _lib
 
@@ -33,3 +35,41 @@ def test_argument_validation_needs_no_gpu():
     assert rc == -1 and b"multiple of 16" in lib.rdq_last_error()
     rc = lib.rdq_gemv_mixed(None, 17, None, None, 1.0, None, None, None, None, None, None, 0, 16, 0, 32, None, None, 0, None)
     assert rc != 0
+
+
+class _Layer(ctypes.Structure):
+    """rdq_layer"""
+
+    _fields_ = ([(name, ctypes.c_int) for name in ("n_fp4", "n_fp8", "n_fp16", "K")] + [("w_fp4_global_scale", ctypes.c_float)]
+                + [(name, ctypes.c_void_p) for name in ("w_fp4", "w_fp4_scales", "w_fp8", "w_fp8_scales", "w_fp16", "w_tiled",
+                                                        "perm", "inv_perm", "gemv_ws", "gemv_counters")])
+
+
+@pytest.mark.parametrize("change,text", [
+    (dict(K=72), b"multiple of 16"),                        # with an NVFP4 group
+    (dict(K=0), b"shape"),
+    (dict(n_fp8=-16), b"shape"),
+    (dict(w_fp4_scales=None), b"must not be null"),
+    (dict(w_fp8_scales=None), b"w_fp8_scales must not be null"),
+    (dict(w_fp8_scales=None, w_fp4=None, w_tiled=4096), b"w_fp8_scales must not be null"),
+    (dict(w_fp4=4100), b"16-byte aligned"),
+    (dict(w_fp4_scales=4098), b"16-byte aligned"),
+    (dict(w_fp8=4104), b"16-byte aligned"),
+    (dict(w_tiled=4104), b"16-byte aligned"),
+    (dict(n_fp4=24, w_tiled=4096), b"no tiled layout"),
+    (dict(w_fp4=None), b"neither"),
+])
+@pytest.mark.parametrize("rows", [1, 40, 3000])
+def test_linear_checks_what_its_kernels_rely_on(rows, change, text):
+    """Refused before anything touches the device (on a machine without one, and with addresses that are none)."""
+    fields = dict(n_fp4=32, n_fp8=16, n_fp16=0, K=128, w_fp4_global_scale=1.0, w_fp4=4096, w_fp4_scales=4096, w_fp8=4096,
+                  w_fp8_scales=4096, w_fp16=None, w_tiled=None, perm=4096, inv_perm=4096, gemv_ws=4096, gemv_counters=4096)
+    fields.update(change)
+    layer = _Layer(**fields)
+    lib = _lib.lib()
+    need = ctypes.c_size_t(0)
+    assert lib.rdq_linear_workspace_size(ctypes.byref(layer), rows, 0, ctypes.byref(need)) < 0 and text in lib.rdq_last_error()
+    # no rows' memory either: a call that these checks let through would be refused for that
+    for rc in (lib.rdq_linear(ctypes.byref(layer), None, 0, rows, None, None, None, 0, 0, None),
+               lib.rdq_linear(ctypes.byref(layer), None, 1, rows, None, None, None, 0, 0, None)):
+        assert rc < 0 and text in lib.rdq_last_error()
