@@ -558,6 +558,10 @@ def rope_attn_decode(qkv: torch.Tensor, q_norm: Optional[torch.Tensor], k_norm: 
     b, nkv, s, dh = k_cache.shape
     if qkv.shape != (b, (nq + 2 * nkv) * dh) or out.shape != (b, nq * dh):
         raise RuntimeError("rope_attn_decode: qkv must be [B, (nq + 2 nkv) * dh] and out [B, nq * dh]")
+    if min(cos.numel(), sin.numel()) < s * dh:
+        # tables with fewer rows than the cache: started under the kernel before, the kernel would ask for the
+        # rows of a position that is not this call's yet and may lie beyond them
+        flags &= ~_lib.RDQ_GEMV_PDL
     with _on_device(qkv.device):
         rc = _lib.lib().rdq_rope_attn_decode(_ptr(qkv), _ptr(q_norm), _ptr(k_norm), _ptr(cos), _ptr(sin), _ptr(pos),
                                              _ptr(k_cache), _ptr(v_cache), _ptr(scratch), _ptr(out), b, nq, nkv, dh, s,

@@ -179,3 +179,32 @@ def test_rope_attn_decode_merges_its_own_parts_only(b, nq, nkv, dh, s, pos_v):
         rc.rope_attn_decode(qkv, None, None, cos, sin, pos, k_cache, v_cache, scratch, out, nq, dh ** -0.5, 1e-6)
         outs.append(out)
     assert torch.equal(*outs)
+
+
+@pytest.mark.parametrize("offset", [1, 4, 8])
+@pytest.mark.parametrize("flags", [0, _lib.RDQ_GEMV_PDL])
+def test_rope_attn_decode_takes_tables_and_weights_at_any_address(offset, flags):
+    """Norm weights and rotary tables that are slices at odd places, and tables that end at the position."""
+    b, nq, nkv, dh, s, pos_v = 2, 8, 2, 128, 200, 150
+    g = torch.Generator().manual_seed(offset)
+    qkv = torch.randn(b, (nq + 2 * nkv) * dh, generator=g).half().cuda()
+    tables = [torch.rand(s, dh, generator=g).half().cuda() for _ in range(2)]
+    norms = [(1 + 0.1 * torch.randn(dh, generator=g)).half().cuda() for _ in range(2)]
+    k_cache, v_cache = (torch.randn(b, nkv, s, dh, generator=g).half().cuda() for _ in range(2))
+    pos = torch.tensor([pos_v], dtype=torch.long, device="cuda")
+
+    def moved(t):
+        buf = torch.zeros(t.numel() + offset, dtype=torch.float16, device="cuda")
+        buf[offset:] = t.reshape(-1)
+        return buf[offset:].view(t.shape)
+
+    outs = []
+    for cos, sin, qn, kn in ((*tables, *norms), (*map(moved, tables), *map(moved, norms)),
+                             (*(moved(t[:pos_v + 1]) for t in tables), *norms)):
+        kc, vc = k_cache.clone(), v_cache.clone()
+        out = torch.empty(b, nq * dh, dtype=torch.float16, device="cuda")
+        rc.rope_attn_decode(qkv, qn, kn, cos, sin, pos, kc, vc, rc.rope_attn_scratch(b, nq, nkv, dh, s, "cuda"), out, nq,
+                            dh ** -0.5, 1e-6, flags)
+        outs.append((out, kc, vc))
+    for other in outs[1:]:
+        assert all(torch.equal(x, y) for x, y in zip(outs[0], other))
