@@ -259,8 +259,6 @@ int rdq_linear_words(const rdq_layer *layer, const void *x, int x_type, int M, c
       break;
   }
   RDQ_REQUIRE(aligned16(xh) && aligned16(y), RDQ_E_INVALID, "x and y must be 16-byte aligned");
-  RDQ_REQUIRE(1ll * l.n_fp4 * (l.K / 2) < (1ll << 32) && 1ll * l.n_fp8 * l.K < (1ll << 32) && 2ll * l.n_fp16 * l.K < (1ll << 32),
-              RDQ_E_UNSUPPORTED, "a format group of this layer exceeds 4 GB");
   GemmArgs a;
   a.x = static_cast<const __half *>(xh);
   a.M = M;

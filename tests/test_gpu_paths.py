@@ -280,3 +280,25 @@ def test_layer_encoder_refuses_bad_permutations(k, bad):
     inv = quantize_weight_packed(w, twice.cuda(), splits)["inv_permutation"]
     assert int(inv.min()) >= 0 and int(inv.max()) < 120 and int(inv[perm[5]]) == 0
     rc.check_quantize_status("cuda")
+
+
+def test_layers_with_a_format_group_above_4_gb():
+    """Byte offsets beyond 32 bits, decode to prompt: the rows around the border, the first and the last ones."""
+    k, n = 65536, 65536 + 128
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    codes = torch.randint(0, 0x78, (n, k), generator=gen, device="cuda", dtype=torch.uint8)  # up to 2^7
+    scale = (torch.rand(n, generator=gen, device="cuda") + 0.5) / 64  # sums of a few hundred: f16 holds them
+    perm = torch.randperm(n, generator=gen, device="cuda")
+    inv = torch.empty_like(perm)
+    inv[perm] = torch.arange(n, device="cuda")
+    mod = FusedMixedLinear.from_layer_data({"weight_fp8": codes, "weight_fp8_scale": scale, "inv_permutation": inv},
+                                           dict(zip(ORDER, (0, n, 0))), k, "cuda")
+    rows = torch.cat([torch.arange(0, 4), torch.arange(65536 - 4, 65536 + 4), torch.arange(n - 4, n)]).cuda()
+    w = codes[rows].view(torch.float8_e4m3fn).double() * scale[rows].double()[:, None]
+    for m in (1, 40, 300):
+        x = torch.randn(m, k, generator=gen, device="cuda").half()
+        y = mod(x)[:, perm[rows]].double()
+        ref, mags = x.double() @ w.t(), x.double().abs() @ w.abs().t()
+        # as in _check_linear
+        assert bool(((y - ref).abs() <= (k + 2) * 2.0 ** -24 * mags + 2.0 ** -11 * ref.abs() + 2.0 ** -25).all()), m
+    rc.check_linear_status(mod._fd())
