@@ -6,7 +6,8 @@
 // stream and calls rdq_linear (include/rdq_b200.h).  What the fast path does not take -- another
 // dtype, a non-contiguous or host tensor, a wrong last dimension, a tensor whose memory cannot be asked
 // for (of tracing or vmap, a sparse layout: the accessors throw or answer null) -- returns None, and the
-// caller's Python path handles or refuses it.  No C++ exception leaves an entry point.
+// caller's Python path handles or refuses it; so does a call whose scratch does not fit on the device.
+// No C++ exception leaves an entry point.
 //
 // Why native: a decode step calls dozens of linears whose kernels take 5-10 us, and the same
 // checks, allocation and ctypes call written in Python took 25-33 us per call.
@@ -252,7 +253,11 @@ PyObject *layer_linear(PyObject *obj, PyObject *const *args, Py_ssize_t nargs) {
       at::Tensor ws;
       if (need) {
         const int64_t sizes[1] = {static_cast<int64_t>(need)};
-        ws = at::detail::empty_cuda(at::IntArrayRef(sizes, 1), at::kByte, device, std::nullopt);
+        try {
+          ws = at::detail::empty_cuda(at::IntArrayRef(sizes, 1), at::kByte, device, std::nullopt);
+        } catch (const c10::OutOfMemoryError &) {
+          Py_RETURN_NONE;  // the caller's path has kernels that need none
+        }
       }
       const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream(self->device);
       // (without a workspace it is a decode kernel, which needs no words)

@@ -325,7 +325,12 @@ def mixed_gemm(x: torch.Tensor, fd: dict, bias: Optional[torch.Tensor] = None,
         # reuse behind the work queued on the current stream
         need = ctypes.c_size_t(0)
         _lib.check(_lib.lib().rdq_gemm_workspace_size(m, n, k, ctypes.byref(need)), "rdq_gemm_workspace_size")
-        ws = torch.empty(need.value, dtype=torch.uint8, device=x.device) if need.value else None
+        ws = None
+        if need.value:
+            try:
+                ws = torch.empty(need.value, dtype=torch.uint8, device=x.device)
+            except torch.OutOfMemoryError:
+                need.value = 0  # the kernel that converts the weights on the way takes no scratch
         rc = _lib.lib().rdq_gemm_mixed_ws(
             _ptr(x), m, _ptr(fd.get("w_fp4_q")), _ptr(fd.get("w_fp4_scales")), float(fd.get("w_fp4_global_scale", 1.0)),
             _ptr(fd.get("w_fp8_q")), _ptr(fd.get("w_fp8_scales")), _ptr(fd.get("w_fp16")), _ptr(fd.get("inv_perm")),

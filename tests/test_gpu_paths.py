@@ -302,3 +302,27 @@ def test_layers_with_a_format_group_above_4_gb():
         # as in _check_linear
         assert bool(((y - ref).abs() <= (k + 2) * 2.0 ** -24 * mags + 2.0 ** -11 * ref.abs() + 2.0 ** -25).all()), m
     rc.check_linear_status(mod._fd())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_calls_whose_scratch_does_not_fit(dtype):
+    """No room for the decoded weights: the kernel that needs none runs instead."""
+    splits = dict(zip(ORDER, (6528, 3072, 128)))
+    mod = FusedMixedLinear.from_layer_data(random_packed_layer(6528, 3072, 128, 2560, seed=12), splits, 2560, "cuda")
+    x = torch.randn(700, 2560, generator=torch.Generator().manual_seed(12)).to(dtype).cuda()
+    y = mod(x).float()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    # room for the outputs (14 MB each) and converted rows (20 MB), not for 50 MB of scratch
+    limit = torch.cuda.memory_reserved() + (52 << 20)
+    torch.cuda.set_per_process_memory_fraction(limit / torch.cuda.get_device_properties(0).total_memory)
+    try:
+        with pytest.raises(torch.OutOfMemoryError):
+            torch.empty(60 << 20, dtype=torch.uint8, device="cuda")
+        z = mod(x)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert z.dtype == dtype
+    # FP32 sums in another order, then a rounding (bf16: to f16 on the way as well)
+    step = 2.0 ** -10 if dtype == torch.float16 else 2.0 ** -7
+    assert bool(((z.float() - y).abs() <= step * y.abs() + 1e-4 * y.abs().max()).all())
