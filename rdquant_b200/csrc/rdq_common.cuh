@@ -254,7 +254,8 @@ __device__ __forceinline__ float silu(float g) {
   const float r = __fdividef(1.f, d);
   const float q = g * r;
   const float c = fmaf(fmaf(-q, d, g), r, q);
-  return c == c ? c : q;  // infinite g: no residual
+  // zeros (the residual would turn -0 into +0), infinities and NaN as a division gives them
+  return fabsf(c) > 0.f ? c : (c != c && g < 0.f ? g - g : q);
 }
 
 __device__ __forceinline__ float warp_max(float v) {

@@ -326,3 +326,20 @@ def test_calls_whose_scratch_does_not_fit(dtype):
     # FP32 sums in another order, then a rounding (bf16: to f16 on the way as well)
     step = 2.0 ** -10 if dtype == torch.float16 else 2.0 ** -7
     assert bool(((z.float() - y).abs() <= step * y.abs() + 1e-4 * y.abs().max()).all())
+
+
+@pytest.mark.parametrize("rows", [1, 40])
+def test_silu_mul_of_infinities_and_nan(rows):
+    """What a division gives: an infinite gate stays infinite, minus infinity and NaN give NaN, the far ends
+    of the range nearly zero and the gate itself."""
+    inf, nan = float("inf"), float("nan")
+    gate = torch.tensor([inf, -inf, nan, 65504.0, -65504.0, -100.0, -88.0, 88.0, 0.0, -0.0, 1.0, -1.0, 20.0, -20.0, 1e-3, -1e-3])
+    gu = torch.cat([gate, torch.ones(16)]).half().cuda().repeat(rows, 1)
+    out = torch.empty(rows, 16, dtype=torch.float16, device="cuda")
+    rc.silu_mul(gu, out)
+    ref = (gu[:, :16].float() / (1 + torch.exp(-gu[:, :16].float()))).half()
+    assert torch.equal(out.isnan(), ref.isnan()) and torch.equal(out.isinf(), ref.isinf())
+    ok = ~ref.isnan()
+    assert torch.equal(out.signbit()[ok], ref.signbit()[ok])
+    ok &= ~ref.isinf()
+    assert bool(((out - ref)[ok].abs() <= 2.0 ** -10 * ref[ok].abs()).all())
