@@ -306,8 +306,11 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const __half *gu, __half 
 //      (cp.async, rows outside the split zero-filled), so that warps do not wait for one another and
 //      a CTA keeps up to eight blocks (70 KB at head_dim 128) in flight.
 //   3. tensor-core products (mma.sync m16n8k16, FP32 sums) with cache rows as the row operand and up to
-//      eight query heads as columns: S^T = K Q^T, online softmax per block, O^T += V^T P^T.  P goes in
-//      as the sum of two FP16 values, so that its rounding (2^-22) stays below FP32 products' sums.
+//      eight query heads as columns: S^T = K Q^T, online softmax per block, O^T += V^T P^T.  P, at
+//      most 1, goes in as the sum of two FP16 values of 2^15 P: its rounding is 2^-22 of it down to
+//      P = 2^-28 and 2^-40 below, less than FP32 sums lose of terms that small next to 1.  (Without the
+//      factor weights below 2^-25 were lost: 4 % of the result for 4096 rows of weight 2^-26 whose values
+//      are 750 times the others'.)
 //   4. the warps' (max, sum, values) are merged in shared memory; with one split that is the result.
 //      Else every CTA stores its partial sums in scratch and counts itself, and the CTA that counts last
 //      merges the heads of its (sequence, KV head), a warp per head, the loads of all splits in flight, in
@@ -320,6 +323,7 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const __half *gu, __half 
 // (92 MB).
 constexpr int kFusedAttnWarps = 4;
 constexpr int kFusedAttnThreads = kFusedAttnWarps * 32;
+constexpr float kProbScale = 32768.f;
 constexpr int kFusedAttnMaxSplit = 16;  // vectors a lane of the merge has in flight
 
 // 16 bytes, or zeros
@@ -607,9 +611,10 @@ __global__ void __launch_bounds__(kFusedAttnThreads, 2) rope_attn_kernel(
       }
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
-        const __half2 hi = __floats2half2_rn(p[2 * half], p[2 * half + 1]);
+        const float p0 = p[2 * half] * kProbScale, p1 = p[2 * half + 1] * kProbScale;
+        const __half2 hi = __floats2half2_rn(p0, p1);
         const float2 hf = __half22float2(hi);
-        const __half2 lo = __floats2half2_rn(p[2 * half] - hf.x, p[2 * half + 1] - hf.y);
+        const __half2 lo = __floats2half2_rn(p0 - hf.x, p1 - hf.y);
         ph[nb][half] = movmatrix_trans(*reinterpret_cast<const uint32_t *>(&hi));
         pl[nb][half] = movmatrix_trans(*reinterpret_cast<const uint32_t *>(&lo));
       }
@@ -653,8 +658,8 @@ __global__ void __launch_bounds__(kFusedAttnThreads, 2) rope_attn_kernel(
       }
 #pragma unroll
       for (int k = 0; k < KS; ++k) {
-        dst[4 + 16 * k + g] = acc[nb][k][h];
-        dst[4 + 16 * k + g + 8] = acc[nb][k][2 + h];
+        dst[4 + 16 * k + g] = acc[nb][k][h] * (1.f / kProbScale);
+        dst[4 + 16 * k + g + 8] = acc[nb][k][2 + h] * (1.f / kProbScale);
       }
     }
   __syncthreads();

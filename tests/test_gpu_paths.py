@@ -343,3 +343,29 @@ def test_silu_mul_of_infinities_and_nan(rows):
     assert torch.equal(out.signbit()[ok], ref.signbit()[ok])
     ok &= ~ref.isinf()
     assert bool(((out - ref)[ok].abs() <= 2.0 ** -10 * ref[ok].abs()).all())
+
+
+def test_single_token_attention_keeps_small_weights():
+    """One row of weight 1 before thousands of about 2^-26 whose values are 750 times larger."""
+    b, nq, nkv, dh, s = 37, 4, 4, 64, 16384  # as many KV heads as SMs: one split, four warps
+    f16 = dict(dtype=torch.float16, device="cuda")
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    k_cache = torch.full((b, nkv, s, dh), -2.25, **f16)
+    k_cache[:, :, 0] = 0.0
+    v_cache = (500 + 500 * torch.rand(b, nkv, s, dh, generator=gen, device="cuda")).half()
+    v_cache[:, :, 0] = 1.0
+    qkv = torch.ones(b, (nq + 2 * nkv) * dh, **f16)
+    qkv[:, nq * dh:(nq + nkv) * dh] = -2.25
+    qkv[:, (nq + nkv) * dh:] = 750.0
+    cos, sin = torch.ones(s, dh, **f16), torch.zeros(s, dh, **f16)
+    pos = torch.tensor([s - 1], dtype=torch.long, device="cuda")
+    out = torch.empty(b, nq * dh, **f16)
+    rc.rope_attn_decode(qkv, None, None, cos, sin, pos, k_cache, v_cache, rc.rope_attn_scratch(b, nq, nkv, dh, s, "cuda"), out, nq,
+                        0.125, 1e-6)
+    w = torch.full((s,), -18.0, dtype=torch.float64, device="cuda").exp()  # scores 0.125 * 64 * -2.25
+    w[0] = 1.0
+    for i in range(0, b, 9):
+        ref = (w[:, None] * v_cache[i].double()).sum(1) / w.sum()
+        # the scores are exact; an exponential of -18 is off by 2^-19 of it at most, and so is their sum; then f16
+        bound = 2.0 ** -11 * ref + 2.0 ** -18 * (ref - 1.0).abs() + 2.0 ** -20
+        assert bool(((out[i].view(nq, dh).double() - ref).abs() <= bound).all())
