@@ -906,7 +906,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
 
 void gemv_tiled_scratch(size_t *workspace_bytes, size_t *flag_bytes) {
   const int G = sm_count();
-  *workspace_bytes = static_cast<size_t>(G) * 256 * sizeof(float);  // one partial tile per CTA
+  *workspace_bytes = static_cast<size_t>(G) * 256 * sizeof(float) + 16;  // one partial tile per CTA, from a multiple of 16 on
   *flag_bytes = (static_cast<size_t>(G) + 2) * sizeof(int32_t);     // status word at index G
 }
 
@@ -1062,7 +1062,9 @@ int launch_gemv_tiled(const GemvTiledArgs &h, bool pdl, cudaStream_t stream) {
   TiledArgs a;
   a.x = static_cast<const __half *>(h.x); a.y_bf16 = h.y_bf16; a.M = h.M; a.tiled = h.tiled; a.s8 = h.s8; a.global4 = h.global4; a.perm = h.perm;
   a.bias = h.bias; a.y = h.y; a.n4 = h.n4; a.n8 = h.n8; a.n16 = h.n16; a.K = h.K;
-  a.workspace = h.workspace; a.flags = h.flags;
+  // the kernel's loads take four words at a time; a workspace at any word serves, its size leaves room
+  a.workspace = reinterpret_cast<float *>((reinterpret_cast<uintptr_t>(h.workspace) + 15) & ~static_cast<uintptr_t>(15));
+  a.flags = h.flags;
   a.early = pdl;
   a.opens = h.opens;
   a.beside = h.beside;
@@ -1080,7 +1082,6 @@ int launch_gemv_tiled(const GemvTiledArgs &h, bool pdl, cudaStream_t stream) {
   a.fdepth = pl.fdep;
   a.nstages = pl.nst;
   const bool xs = pl.xs;
-  RDQ_REQUIRE((reinterpret_cast<uintptr_t>(h.workspace) & 15) == 0, RDQ_E_INVALID, "GEMV workspace must be 16-byte aligned");
   RDQ_REQUIRE(a.xop == 0 || xs, RDQ_E_UNSUPPORTED,
               "activation prologue needs the activation rows in shared memory (M=%d, K=%d)", h.M, h.K);
   RDQ_REQUIRE(h.xop == 0 || (h.xop == 1 && h.x_weight) || h.xop == 2, RDQ_E_INVALID, "bad activation prologue");

@@ -220,3 +220,21 @@ def test_prologue_refused_when_rows_do_not_fit():
                               "cuda")
     with pytest.raises(RuntimeError, match="alias"):
         rdquant_cuda.mixed_gemv_norm(x, None, x[0], 1e-6, fd2, residual_out=x)
+
+
+@pytest.mark.parametrize("offset", [1, 2, 3])
+def test_tiled_gemv_workspace_at_any_word(offset):
+    """A workspace that starts at a word which is no multiple of 16 bytes."""
+    layer = random_packed_layer(1328, 640, 80, 2560, seed=offset)
+    fd = pack_for_fused_gemv(layer, dict(zip(ORDER, (1328, 640, 80))), 2560, "cuda")
+    x = torch.randn(5, 2560, generator=torch.Generator().manual_seed(offset)).half().cuda()
+    y = rdquant_cuda.mixed_gemv(x, fd)
+    size = fd["workspace"].numel()
+    guard = torch.full((size + 8,), -1, dtype=torch.int32, device="cuda")
+    guard[:offset] = guard[offset + size:] = 77  # not the call's
+    fd["workspace"] = guard[offset:offset + size].view(torch.float32)
+    for _ in range(3):
+        assert torch.equal(rdquant_cuda.mixed_gemv(x, fd), y)
+    rdquant_cuda.check_status(fd)
+    assert bool((guard[:offset] == 77).all()) and bool((guard[offset + size:] == 77).all())
+    assert bool((guard[offset:offset + size] == -1).all())
