@@ -44,9 +44,13 @@ bool has_row_major(const rdq_layer &l) {
 // a + bytes / rate with a = 4.5 us and 4.2 (1, 2 rows) or 2.9 TB/s (up to 8) for the GEMV, whose
 // converter work and activation reads grow with the rows, against 9.5 us and 5.8 TB/s whatever the
 // rows: equal at 75 and 29 MB of packed weights (40 measured); above 8 rows the GEMV halves its rate.
+// The row-major GEMV of layers without a tiled layout starts at 1.9 us where the streaming GEMM takes 6
+// to 9 (300 NVFP4 + 130 FP8 + 20 FP16 rows of 1024: 2.3 against 9.0 us at one row), and is slower from
+// 40 MB (9001 + 4500 + 3 of 4096: 17.2 us each at 8 rows), above 8 rows from 18 MB (6500 + 3100 + 128 of
+// 2560: 13.5 us each at 14 rows).
 int stream_from(const rdq_layer &l) {
-  if (!l.w_tiled) return 1;
   const double bytes = l.n_fp4 * (l.K * 0.5625) + l.n_fp8 * (l.K + 4.0) + l.n_fp16 * (l.K * 2.0);
+  if (!l.w_tiled) return bytes > 40e6 ? 1 : (bytes > 18e6 ? 9 : RDQ_MAX_GEMV_M + 1);
   return bytes > 80e6 ? 1 : (bytes > 40e6 ? 3 : 9);
 }
 

@@ -73,3 +73,15 @@ def test_linear_checks_what_its_kernels_rely_on(rows, change, text):
     for rc in (lib.rdq_linear(ctypes.byref(layer), None, 0, rows, None, None, None, 0, 0, None),
                lib.rdq_linear(ctypes.byref(layer), None, 1, rows, None, None, None, 0, 0, None)):
         assert rc < 0 and text in lib.rdq_last_error()
+
+
+@pytest.mark.parametrize("n4,n8,k,decode_rows", [(300, 130, 1024, 16), (2001, 900, 4096, 16), (5001, 2503, 4096, 8), (9003, 5007, 8192, 0)])
+def test_small_layers_without_tiles_stay_on_the_decode_kernel(n4, n8, k, decode_rows):
+    """Which of its kernels a call takes, told by the scratch it asks for: the decode kernel needs none."""
+    layer = _Layer(n_fp4=n4, n_fp8=n8, n_fp16=0, K=k, w_fp4_global_scale=1.0, w_fp4=4096, w_fp4_scales=4096, w_fp8=4096,
+                   w_fp8_scales=4096, w_fp16=None, w_tiled=None, perm=4096, inv_perm=4096, gemv_ws=4096, gemv_counters=4096)
+    need = ctypes.c_size_t(0)
+    for x_type in (0, 1):
+        for rows in range(1, 20):
+            assert _lib.lib().rdq_linear_workspace_size(ctypes.byref(layer), rows, x_type, ctypes.byref(need)) == 0
+            assert (need.value == 0) == (rows <= decode_rows), (rows, need.value)
