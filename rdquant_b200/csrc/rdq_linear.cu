@@ -59,16 +59,20 @@ int stream_from(const rdq_layer &l) {
 // row-major tensors by TMA (K a multiple of 64 / 16); what they cannot take runs as 16-row panels of
 // the decode kernel.
 //
-// The streaming GEMM converts the weights once more per 128 rows, the other GEMM decodes them once:
-// estimates in microseconds that agree with measurements between 65 and 2048 rows on seven layer
-// shapes within 15 %.  (With up to 64 rows the streaming GEMM was faster on all of them.)
+// The streaming GEMM converts the weights once more per 128 rows, the other GEMM decodes them once.
+// Estimates in microseconds, fitted to both kernels at 16 numbers of rows between 65 and 2048, f16 and
+// bf16, on 13 layers (channels x K: 6144, 19456, 4096, 9728 and 1024 x 2560, 2560 x 4096, 2560 x 9728,
+// 4096 x 3072, 16384 and 8192 x 8192, 1024 x 16384, 1024 and 11392 x 1024): off by 8 and 7 % on average, by
+// up to 40 % on the smallest.  Choosing by them costs 0.4 % on average over the faster kernel, 15 % at
+// worst (34 % once: 2048 bf16 rows x 1024 x 16384); the constants before, fitted to a decoding launch
+// that overlapped its predecessor, 1.6 %.  (With up to 64 rows the streaming GEMM was always faster.)
 bool stream_beats_dense(const rdq_layer &l, int M, int x_type) {
   if (M <= 64) return true;
   if (M > 2048) return false;
   const int N = l.n_fp4 + l.n_fp8 + l.n_fp16;
   const double weights = 1e-6 * N * l.K;
-  const double cast = x_type == RDQ_BF16 ? 2.5 : 0.0;  // the other GEMM's decoding launch rounds bf16 rows along the way
-  return cast + 15.5 + 1.62e-3 * M * weights < 4.0 + 0.6 * weights + gemm_dense_cycles(M, N, l.K) / 1750.0;
+  const double cast = x_type == RDQ_BF16 ? 1.8 : 0.0;  // the other GEMM's decoding launch rounds bf16 rows along the way
+  return cast + 15.6 + 1.57e-3 * M * weights < 5.1 + 0.545 * weights + gemm_dense_cycles(M, N, l.K) / 1500.0;
 }
 
 Path path_of(const rdq_layer &l, int M, int x_type) {
