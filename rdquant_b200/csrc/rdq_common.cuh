@@ -254,8 +254,9 @@ __device__ __forceinline__ float silu(float g) {
   const float r = __fdividef(1.f, d);
   const float q = g * r;
   const float c = fmaf(fmaf(-q, d, g), r, q);
-  // zeros (the residual would turn -0 into +0), infinities and NaN as a division gives them
-  return fabsf(c) > 0.f ? c : (c != c && g < 0.f ? g - g : q);
+  // zeros (the residual would turn -0 into +0), infinities and NaN as a division gives them: c is NaN for
+  // an infinite g, which is right for minus infinity only
+  return c > 0.f || g < 0.f ? c : q;
 }
 
 __device__ __forceinline__ float warp_max(float v) {
