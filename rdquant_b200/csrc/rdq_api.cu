@@ -122,8 +122,9 @@ size_t rdq_gemv_tiled_bytes(int n_fp4, int n_fp8, int n_fp16, int K) {
 
 int rdq_gemv_repack(const void *w_fp4, const void *w_fp4_scales, const void *w_fp8, const void *w_fp16,
                     void *w_tiled, int n_fp4, int n_fp8, int n_fp16, int K, void *stream) {
-  int rc = check_layer(w_fp4, w_fp4_scales, w_fp8, reinterpret_cast<const float *>(w_fp8), w_fp16, n_fp4, n_fp8,
-                       n_fp16, K);
+  int rc = quantize_error();
+  if (rc == RDQ_OK)
+    rc = check_layer(w_fp4, w_fp4_scales, w_fp8, reinterpret_cast<const float *>(w_fp8), w_fp16, n_fp4, n_fp8, n_fp16, K);
   if (rc != RDQ_OK) return rc;
   RDQ_REQUIRE(tiled_supported(n_fp4, n_fp8, n_fp16, K), RDQ_E_UNSUPPORTED,
               "tiled layout needs groups in multiples of 16 rows and K divisible into chunks that are "

@@ -160,6 +160,9 @@ int launch_silu_mul(const __half *gu, __half *out, int B, int F, bool pdl, cudaS
 // encoders (rdq_quantize.cu)
 int launch_quantize_nvfp4(const void *w, bool w_is_f32, int n, int K, uint8_t *codes, uint8_t *scales, float *row_sqerr,
                           float *max_scale, cudaStream_t stream);
+// RDQ_OK, or the error of an encoder launch that found a permutation entry out of range (reported once; looks at
+// a word of host memory)
+int quantize_error();
 int launch_quantize_fp8(const void *w, bool w_is_f32, int n, int K, uint8_t *out, float *scale_out, float *row_sqerr,
                         float *absmax_scratch, cudaStream_t stream);
 

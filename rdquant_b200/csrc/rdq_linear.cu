@@ -219,7 +219,8 @@ int rdq_linear_words(const rdq_layer *layer, const void *x, int x_type, int M, c
   RDQ_REQUIRE(layer != nullptr && M >= 0 && (x_type == RDQ_F16 || x_type == RDQ_BF16), RDQ_E_INVALID, "bad arguments to rdq_linear");
   const rdq_layer &l = *layer;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  int rc = check_layouts(l);
+  int rc = quantize_error();
+  if (rc == RDQ_OK) rc = check_layouts(l);
   if (rc != RDQ_OK) return rc;
   const int N = l.n_fp4 + l.n_fp8 + l.n_fp16;
   if (M == 0 || N == 0) return RDQ_OK;

@@ -521,10 +521,11 @@ int one_wave(K kernel) {
 }
 
 // The pinned word of LayerEncodeArgs::bad_index, one per process.
+std::atomic<int *> bad_index{nullptr};
 int bad_index_word(int **out) {
   static std::mutex mu;
-  static int *word = nullptr;
   std::lock_guard<std::mutex> lock(mu);
+  int *word = bad_index.load();
   if (word == nullptr) {
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // the allocation is no part of a capture
     RDQ_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
@@ -534,15 +535,9 @@ int bad_index_word(int **out) {
     RDQ_CUDA(e);
     word = static_cast<int *>(p);
     *word = 0;
+    bad_index.store(word);
   }
   *out = word;
-  return RDQ_OK;
-}
-int report_bad_index(int *word) {
-  if (*static_cast<volatile int *>(word) == 0) return RDQ_OK;
-  *static_cast<volatile int *>(word) = 0;
-  RDQ_REQUIRE(false, RDQ_E_INVALID, "rdq_quantize_layer: a permutation given to an earlier call had an entry out of range; "
-              "its tensors are invalid");
   return RDQ_OK;
 }
 
@@ -601,6 +596,15 @@ int launch_quantize_fp8(const void *w, bool w_is_f32, int n, int K, uint8_t *out
   return RDQ_OK;
 }
 
+int quantize_error() {
+  volatile int *const word = bad_index.load();
+  if (word == nullptr || *word == 0) return RDQ_OK;
+  *word = 0;
+  RDQ_REQUIRE(false, RDQ_E_INVALID, "rdq_quantize_layer: a permutation given to an earlier call had an entry out of range; "
+              "its tensors are invalid");
+  return RDQ_OK;
+}
+
 }  // namespace rdq
 
 using namespace rdq;
@@ -619,7 +623,7 @@ extern "C" int rdq_quantize_layer(const void *w, int w_is_f32, const long long *
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   LayerEncodeArgs a;
   int rc = bad_index_word(&a.bad_index);
-  if (rc == RDQ_OK) rc = report_bad_index(a.bad_index);
+  if (rc == RDQ_OK) rc = quantize_error();
   if (rc != RDQ_OK) return rc;
   a.w = w;
   a.perm = perm;
@@ -640,9 +644,6 @@ extern "C" int rdq_quantize_layer(const void *w, int w_is_f32, const long long *
 }
 
 extern "C" int rdq_quantize_status(void *stream) {
-  int *word = nullptr;
-  const int rc = bad_index_word(&word);
-  if (rc != RDQ_OK) return rc;
   RDQ_CUDA(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)));
-  return report_bad_index(word);
+  return quantize_error();
 }

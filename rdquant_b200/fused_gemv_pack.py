@@ -99,8 +99,6 @@ def pack_for_fused_gemv(layer_data: dict, splits: dict, k: int, device,
         return t.to(device=device, dtype=dtype).contiguous()
 
     if "inv_permutation" in layer_data:
-        if layer_data["inv_permutation"].is_cuda:  # perhaps from the GPU encoder
-            rdquant_cuda.check_quantize_status(layer_data["inv_permutation"].device)
         inv = dev(layer_data["inv_permutation"], torch.int32)
     else:
         inv = torch.arange(n, dtype=torch.int32, device=device)

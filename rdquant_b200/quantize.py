@@ -109,7 +109,8 @@ def quantize_weight_packed(weight: torch.Tensor, permutation: torch.Tensor, spli
     Byte-identical to the host route (rdquant/quantize.py:233-280 followed by
     rdquant/integrations/hf_export.py:58-125); tensors stay on the weight's device.  An entry of the
     permutation out of range raises ``IndexError``; in a CUDA permutation it is found on the device and
-    raises at the next call, when the layer is packed, or in ``rdquant_cuda.check_quantize_status``.
+    raises ``RuntimeError`` in a later call -- of this function, the packing of a layer or a linear -- or in
+    ``rdquant_cuda.check_quantize_status``.
     """
     from rdquant_b200 import rdquant_cuda
 

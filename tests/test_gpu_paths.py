@@ -264,7 +264,9 @@ def test_layer_encoder_refuses_bad_permutations(k, bad):
     wrong[77] = bad
     with pytest.raises(IndexError, match="out of range"):
         quantize_weight_packed(w, wrong, splits)
-    for report in (lambda: rc.check_quantize_status("cuda"), lambda: quantize_weight_packed(w, perm, splits)):
+    mod = FusedMixedLinear.from_layer_data(good, splits, k, "cuda")
+    for report in (lambda: rc.check_quantize_status("cuda"), lambda: quantize_weight_packed(w, perm, splits),
+                   lambda: mod(w[:1])):
         inv = quantize_weight_packed(w, wrong.cuda(), splits)["inv_permutation"]
         assert int(inv.min()) >= 0 and int(inv.max()) < 120
         inv[perm[77]] = 77
