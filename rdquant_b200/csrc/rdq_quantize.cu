@@ -16,7 +16,7 @@
 //          scale s with a 4-bit mantissa that is v > t s (t s is exact; fl(v / s) > t needs v / s to
 //          exceed t by half an ulp, and a float v above t s exceeds it by more: the relative step of v
 //          is above 2^-24 there, half an ulp of t at most 2^-24).  The sign of a quotient that
-//          underflows to zero is the one exception: denormal inputs take the division.
+//          underflows to zero is the one exception: denormal inputs are compared with s / 2 steps.
 //          An f16 v that is not t s itself differs from it by more than 2^-12 of it, so v (1 - 2^-14) / s
 //          lies on the right side of every midpoint and below one that v / s hits: the hardware's
 //          round-to-nearest E2M1 converter then gives the code (adding +0 turns -0 into +0, whose code
@@ -142,22 +142,27 @@ __device__ __forceinline__ uint32_t cvt_to_e2m1x8(const float (&v)[8]) {
       : "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]));
   return r;
 }
+// value of the code in the low four bits: its sign, two exponent bits and a mantissa bit at a float's places
+// are the value times 2^-126
+__device__ __forceinline__ float grid_value(uint32_t c) {
+  return __uint_as_float(((c & 8u) << 28) | ((c & 7u) << 22)) * 8.50705917e37f;
+}
 // Half a block of 16: codes of eight values (a nibble each, low nibble first), by counting thresholds.
 template <bool SQERR>
 __device__ __forceinline__ uint32_t encode_fp4(const float (&v)[8], float scale, float &err) {
   const float s = scale == 0.f ? 1.f : scale;
   const float t0 = 0.25f * s, t1 = 0.75f * s, t2 = 1.25f * s, t3 = 1.75f * s, t4 = 2.5f * s, t5 = 3.5f * s, t6 = 5.0f * s;
+  // the quotient of a denormal v (its bits count steps of 2^-149) is zero when v is at most s / 2 of them
+  const int vanish = static_cast<int>(0.5f * s);
   uint32_t packed = 0;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const float mag = fabsf(v[i]);
     const int m = (mag > t0) + (mag > t1) + (mag > t2) + (mag > t3) + (mag > t4) + (mag > t5) + (mag > t6);
-    const bool neg = v[i] < 0.f && (mag >= 1.17549435e-38f || __fdiv_rn(v[i], s) < 0.f);
+    const bool neg = v[i] < 0.f && __float_as_int(mag) > vanish;
     packed |= static_cast<uint32_t>(m + (neg ? 8 : 0)) << (4 * i);
     if (SQERR) {
-      // grid value: 0, .5, 1, 1.5 (m / 2) then 2, 3, 4, 6
-      const float g = (m < 4) ? 0.5f * m : (m == 7 ? 6.f : static_cast<float>(m - 2));
-      const float d = v[i] - __fmul_rn(neg ? -g : g, scale);
+      const float d = v[i] - __fmul_rn(grid_value(static_cast<uint32_t>(m + (neg ? 8 : 0))), scale);
       err = fmaf(d, d, err);
     }
   }
@@ -198,9 +203,22 @@ __device__ __forceinline__ void encode_vec_fp4(Vec8<T> &q, bool live, int i, uin
   top = fmaxf(top, scale);
   if (live) {
     uint32_t code;
-    if (SQERR || sizeof(T) == 4) code = encode_fp4<SQERR>(v, scale, err);
-    else if (finite) code = encode_fp4_f16(v, scale);
-    else code = encode_fp4_any(make_float4(v[0], v[1], v[2], v[3]), make_float4(v[4], v[5], v[6], v[7]), scale);
+    if (sizeof(T) == 4) {
+      code = encode_fp4<SQERR>(v, scale, err);
+    } else if (finite) {
+      code = encode_fp4_f16(v, scale);
+      if (SQERR) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const float d = v[e] - __fmul_rn(grid_value(code >> (4 * e)), scale);
+          err = fmaf(d, d, err);
+        }
+      }
+    } else if (SQERR) {
+      code = encode_fp4<SQERR>(v, scale, err);
+    } else {
+      code = encode_fp4_any(make_float4(v[0], v[1], v[2], v[3]), make_float4(v[4], v[5], v[6], v[7]), scale);
+    }
     reinterpret_cast<uint32_t *>(codes)[i] = code;
     if (!(i & 1)) scales[i >> 1] = sbits;
   }

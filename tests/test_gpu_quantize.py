@@ -116,3 +116,20 @@ def test_layer_fast_path_equals_host_route():
     for key in host:
         a, b = host[key], dev[key].cpu()
         assert a.dtype == b.dtype and torch.equal(a, b), key
+
+
+def test_nvfp4_sign_of_denormal_values():
+    """Negative values whose quotient by the block scale is the smallest denormal, half of it (rounds to zero),
+    or less: the sign bit of the code follows the quotient."""
+    step = 2.0 ** -149
+    rows = []
+    for top in (2688.0, 336.0, 6.0, 0.0117):  # block scales 448, 56, 1 and the smallest, 2^-9
+        ks = [1, 2, 27, 28, 29, 223, 224, 225, 448, 2 ** 22, 2 ** 23, 2 ** 23 + 1]
+        rows.append([top] + [-k * step for k in ks] + [224 * step, -0.0, 0.0])
+    w = torch.tensor(rows, dtype=torch.float64).float()
+    assert int((w[:, 1:13] != 0).sum()) == w.shape[0] * 12, "denormals survive"
+    host, _, _ = _host_nvfp4(w)
+    for sq in (False, True):
+        dev = rdquant_cuda.quantize_nvfp4_packed(w.cuda(), sq)
+        assert torch.equal(dev["weight_nvfp4"].cpu(), host["weight_nvfp4"])
+        assert torch.equal(dev["weight_nvfp4_scale"].cpu(), host["weight_nvfp4_scale"])
