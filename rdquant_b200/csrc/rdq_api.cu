@@ -349,7 +349,7 @@ int rdq_gemm_mixed(const void *x, int M, const void *w_fp4, const void *w_fp4_sc
 int rdq_gemm_workspace_size(int M, int N, int K, size_t *bytes) {
   RDQ_REQUIRE(bytes != nullptr, RDQ_E_INVALID, "bytes must not be null");
   RDQ_REQUIRE(M >= 0 && N >= 0 && K > 0 && K % 64 == 0, RDQ_E_INVALID, "rdq_gemm_workspace_size: bad shape M=%d N=%d K=%d", M, N, K);
-  *bytes = (M == 0 || N == 0) ? 0 : gemm_workspace_bytes(M, N, K);
+  *bytes = (M == 0 || N == 0 || gemm_better_without_scratch(M, N, K)) ? 0 : gemm_workspace_bytes(M, N, K);
   return RDQ_OK;
 }
 

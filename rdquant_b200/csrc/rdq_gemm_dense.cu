@@ -550,7 +550,7 @@ DenseLayout dense_layout(const PairPlan &p, int N, int K) {
 
 bool gemm_dense_takes(int K) { return K % 16 == 0; }  // 16-byte row pitch for TMA, whole runs of 8 k
 
-double gemm_dense_cycles(int M, int N, int K) { return pair_plan(M, N, K).cycles; }
+double gemm_dense_estimate(int M, int N, int K) { return 5.1 + 0.545e-6 * N * K + pair_plan(M, N, K).cycles / 1500.0; }
 
 size_t gemm_dense_workspace(int M, int N, int K) { return dense_layout(pair_plan(M, N, K), N, K).total; }
 

@@ -121,6 +121,7 @@ int gemm_test_timeout();
 // tile leave at once when they would have to wait
 void gemm_set_test_timeout(int mode);
 size_t gemm_workspace_bytes(int M, int N, int K);
+bool gemm_better_without_scratch(int M, int N, int K);
 // weight-streaming GEMM (rdq_gemm_stream.cu)
 bool gemm_stream_takes(int K);
 size_t gemm_stream_workspace(int M, int K);
@@ -128,7 +129,7 @@ int launch_gemm_stream(const GemmArgs &a, void *workspace, size_t workspace_byte
 // GEMM over weights decoded once per call (rdq_gemm_dense.cu)
 bool gemm_dense_takes(int K);
 size_t gemm_dense_workspace(int M, int N, int K);
-double gemm_dense_cycles(int M, int N, int K);  // estimate of the product alone
+double gemm_dense_estimate(int M, int N, int K);  // microseconds, decoding and product
 int launch_gemm_dense(const GemmArgs &a, void *workspace, size_t workspace_bytes, cudaStream_t stream);
 
 // staging copy by kernel (rdq_stage.cu)

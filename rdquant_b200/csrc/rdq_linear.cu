@@ -72,7 +72,7 @@ bool stream_beats_dense(const rdq_layer &l, int M, int x_type) {
   const int N = l.n_fp4 + l.n_fp8 + l.n_fp16;
   const double weights = 1e-6 * N * l.K;
   const double cast = x_type == RDQ_BF16 ? 1.8 : 0.0;  // the other GEMM's decoding launch rounds bf16 rows along the way
-  return cast + 15.6 + 1.57e-3 * M * weights < 5.1 + 0.545 * weights + gemm_dense_cycles(M, N, l.K) / 1500.0;
+  return cast + 15.6 + 1.57e-3 * M * weights < gemm_dense_estimate(M, N, l.K);
 }
 
 Path path_of(const rdq_layer &l, int M, int x_type) {

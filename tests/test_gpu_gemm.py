@@ -1,12 +1,14 @@
 """Prefill GEMM (tcgen05) through the C ABI against the oracle: golden layers, random byte
 patterns, the benchmark block shapes, ragged M, bias."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
 
 from conftest import ORDER, golden_layer_torch
 from oracle import oracle_np as onp
-from rdquant_b200 import rdquant_cuda
+from rdquant_b200 import _lib, rdquant_cuda
 from rdquant_b200.fused_gemv_pack import pack_for_fused_gemv
 from rdquant_b200.synthetic import QWEN3_4B_BLOCK, fixed_splits, random_packed_layer
 
@@ -126,3 +128,21 @@ def test_benchmark_launches(group, m):
         ref = x[r0:r0 + 2048].float() @ w.float().T
         worst = max(worst, float((y[r0:r0 + 2048].float() - ref).abs().max() / ref.abs().max()))
     assert worst < TOL
+
+
+@pytest.mark.parametrize("rows,shape,scratch", [(64, (22016, 10624, 128, 1024), False), (250, (22016, 10624, 128, 1024), False),
+                                                (600, (22016, 10624, 128, 1024), True), (64, (2560, 1280, 256, 512), True)])
+def test_wide_layers_of_few_rows_need_no_decoding(rows, shape, scratch):
+    """Which of the two kernels mixed_gemm takes, told by the scratch it asks for; both give the same product."""
+    n4, n8, n16, k = shape
+    need = ctypes.c_size_t(0)
+    assert _lib.lib().rdq_gemm_workspace_size(rows, n4 + n8 + n16, k, ctypes.byref(need)) == 0
+    assert (need.value > 0) == scratch
+    layer = random_packed_layer(n4, n8, n16, k, seed=rows)
+    fd = pack_for_fused_gemv(layer, dict(zip(ORDER, shape[:3])), k, "cuda")
+    x = torch.randn(rows, k, generator=torch.Generator().manual_seed(rows)).half()
+    y = rdquant_cuda.mixed_gemm(x.cuda(), fd)
+    rdquant_cuda.check_gemm_status("cuda")
+    some = torch.arange(0, rows, 7)
+    ref = onp.mixed_precision_linear(x[some].numpy(), onp.torch_layer_to_np(layer), dict(zip(ORDER, shape[:3])), k)
+    assert onp.rel_err(y.cpu()[some].float().numpy(), ref) < TOL
