@@ -326,7 +326,8 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
   const uint32_t x_ring = w_ring + a.nw * kChunkBytes;
   const uint32_t x_bytes = static_cast<uint32_t>(sc.nt) * 128;  // one 64-k box
   const uint32_t s_ring = x_ring + NS * KB * x_bytes;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // (from lane 0, so that the compiler keeps the roles' branches and loops in uniform registers)
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int begin = sc.bnd[blockIdx.x], end = sc.bnd[blockIdx.x + 1];
   auto load_chunk = [&](const Segment &g, int c, int slot) {
     const uint32_t bar = smem_u32(&S.w_full[slot]);
@@ -612,15 +613,23 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
         // (k blocks beyond K convert the zero fill of the box; the MMAs do not read them)
         const uint4 s4 = lds16(s_ring + slot * kScaleBytes + row * 16);
         const uint32_t sc4[4] = {part ? s4.z : s4.x, part ? s4.w : s4.y, s4.z, s4.w};
+        // Four pieces are read ahead of their conversion: one after the other, each waited for its own read.
+        uint4 v[4] = {piece(2 * KB * part), piece(2 * KB * part + 1), piece(2 * KB * part + 2), piece(2 * KB * part + 3)};
 #pragma unroll
         for (int h = 0; h < 2 * KB; ++h) {
-          convert_fp4(piece(2 * KB * part + h), sc4[h >> 1] >> (16 * (h & 1)), o);
+          convert_fp4(v[h & 3], sc4[h >> 1] >> (16 * (h & 1)), o);
+          if (h + 4 < 2 * KB) v[h & 3] = piece(2 * KB * part + h + 4);
           tmem_st16(dst + 16 * h, o);
         }
       } else if (g.fmt == 1) {
+        uint4 v[4] = {piece(0), piece(1), piece(2), piece(3)};
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
-          convert_fp8(piece(2 * h), piece(2 * h + 1), o);
+          convert_fp8(v[2 * (h & 1)], v[2 * (h & 1) + 1], o);
+          if (h < 2) {
+            v[2 * h] = piece(2 * h + 4);
+            v[2 * h + 1] = piece(2 * h + 5);
+          }
           tmem_st16(dst + 16 * h, o);
         }
       } else {
