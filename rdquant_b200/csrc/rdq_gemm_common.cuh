@@ -28,6 +28,11 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
       "l"(map), "r"(x), "r"(y), "r"(bar)
       : "memory");
 }
+// The box into L2 only.  That may run ahead of the grid-dependency wait whatever the kernel before writes:
+// L2 is where its writes go, and the load that follows the wait reads them there.
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap *map, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
+}
 // into this CTA's shared memory, completing on a barrier of either CTA of the pair
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
   asm volatile(

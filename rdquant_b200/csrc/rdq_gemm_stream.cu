@@ -36,7 +36,9 @@
 //            of a whole one left the MMAs waiting: 1930 cycles per NVFP4 chunk of 128 tokens, whose
 //            MMAs take 1024)
 // Every launch is programmatic: it overlaps the end of the kernel before.  With RDQ_GEMV_PDL the
-// weight and scale loads start before the grid-dependency wait.
+// weight and scale loads start before the grid-dependency wait.  Without it the first chunks are asked into
+// L2 ahead of the wait and loaded from there behind it: with every thread waiting before the set-up, the
+// first MMA came 1.7 us later than with the flag (2.6 us after the wait, 2560 -> 6144 at 32 rows).
 //
 // Reference behaviour replaced: 2 x marlin_gemm + F.linear + cat + index_select
 // (rdquant/inference.py:620-677).
@@ -329,17 +331,15 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
   // (from lane 0, so that the compiler keeps the roles' branches and loops in uniform registers)
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int begin = sc.bnd[blockIdx.x], end = sc.bnd[blockIdx.x + 1];
+  auto wmap = [&](int fmt) { return fmt == 0 ? &w4map : (fmt == 1 ? &w8map : &w16map); };
   auto load_chunk = [&](const Segment &g, int c, int slot) {
     const uint32_t bar = smem_u32(&S.w_full[slot]);
     mbar_arrive_expect_tx(bar, kChunkBytes);
-    tma_load_2d(w_ring + slot * kChunkBytes, g.fmt == 0 ? &w4map : (g.fmt == 1 ? &w8map : &w16map),
-                c * (g.fmt == 2 ? 64 : 128), g.row_tile * 128, bar);
+    tma_load_2d(w_ring + slot * kChunkBytes, wmap(g.fmt), c * (g.fmt == 2 ? 64 : 128), g.row_tile * 128, bar);
   };
-  // Without leave to read weights early every thread waits for the kernel before this one here; the
-  // launch itself still overlaps it.
-  if (!a.early) pdl_wait();
-  // The first weight chunks are on their way before anything else is set up.
-  const int early = min(a.nw, end - begin);
+  // The first weight chunks are on their way before anything else is set up; without leave to read weights
+  // early, on their way into L2.
+  const int ahead = min(a.nw, end - begin), early = a.early ? ahead : 0;
   if (threadIdx.x == 0) {
     for (int i = 0; i < a.nw; ++i) {
       mbar_init(smem_u32(&S.w_full[i]), 1 + 32);  // the TMA thread and the scale warp's lanes
@@ -347,9 +347,10 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
     }
     mbar_init_fence();
     Segment g = segment_at(sc, begin, end);
-    for (int i = 0; i < early; ++i) {
+    for (int i = 0; i < ahead; ++i) {
       if (begin + i == g.start + g.c1) g = segment_at(sc, begin + i, end);
-      load_chunk(g, begin + i - g.start, i);
+      if (a.early) load_chunk(g, begin + i - g.start, i);
+      else tma_prefetch_2d(wmap(g.fmt), (begin + i - g.start) * (g.fmt == 2 ? 64 : 128), g.row_tile * 128);
     }
   }
   if (threadIdx.x == 32) {
@@ -381,6 +382,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
   if (warp == 0) {
     // ---------------------------------------------------------------- weight chunks
     const bool leader = elect_one();
+    if (!a.early) pdl_wait();
     Cursor w;
     if (early == a.nw) w.ph ^= 1;
     else w.i = early;
@@ -487,6 +489,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
     __syncwarp();
   } else if (warp == 3) {
     // ------------------------------------------------------------------ block scales
+    if (!a.early) pdl_wait();
     Cursor w;
     const int pitch = a.K >> 4;
     Segment g = segment_at(sc, begin, end);
@@ -515,6 +518,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
     // ------------------------------------------------------------------ epilogue
     const int q = warp & 3;
     const uint32_t lanes = static_cast<uint32_t>(q * 32) << 16;
+    if (!a.early) pdl_wait();
     // constants of the rows that are finished together with other CTAs: fetched now, when nobody waits
     S.cut[0][q * 32 + lane] = row_of(a, segment_at(sc, begin, end), q * 32 + lane, true);
     S.cut[1][q * 32 + lane] = row_of(a, segment_at(sc, end - 1, end), q * 32 + lane, true);

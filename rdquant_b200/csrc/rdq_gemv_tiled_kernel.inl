@@ -356,12 +356,13 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
     };
     // The ring is filled with weights first (they do not depend on the preceding kernel);
     // only then wait for that kernel and fetch the activations it produced.
-    auto fill = [&]() {
+    auto first_images = [&](auto &&take) {
       int slot = 0;
       for (int j = 0; j < most && slot < nst; ++j)
         for (int g = 0; g < kGroups && slot < nst; ++g, ++slot)
-          if (third(g) + j < third(g + 1)) copy_in(third(g) + j, slot);
+          if (third(g) + j < third(g + 1)) take(third(g) + j, slot);
     };
+    auto fill = [&]() { first_images(copy_in); };
     if (lane == 0) {
       for (int i = 0; i < nst; ++i) {
         mbar_init(smem_u32(&bar_full[i]), 1);
@@ -377,7 +378,13 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
       mbar_init(smem_u32(&bar_x), 1);
       mbar_init(smem_u32(&bar_never), 1);
       mbar_init_fence();
-      if (a.early) fill();
+      if (a.early) {
+        fill();
+      } else {  // into L2, whatever the kernel before writes: they are read there, behind the wait
+        first_images([&](int img, int) {
+          l2_prefetch(a.tiled + sc.image_offset(img), static_cast<uint32_t>(img < sc.e4 ? sc.img4 : sc.img8));
+        });
+      }
     }
     __syncwarp();
     __syncthreads();
