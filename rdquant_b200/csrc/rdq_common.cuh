@@ -172,10 +172,6 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t
       "l"(src), "r"(bytes), "r"(bar)
       : "memory");
 }
-// The same stretch into L2 only.
-__device__ __forceinline__ void l2_prefetch(const void *src, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
-}
 // ---- which launch may start when
 // A programmatic launch may start once every CTA of the launch before it has called
 // pdl_launch_dependents() or ended.  pdl_wait() returns when the launch before is complete; every kernel

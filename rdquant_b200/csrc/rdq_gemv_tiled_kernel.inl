@@ -62,6 +62,7 @@ __device__ __forceinline__ uint4 ld_relaxed16(const float *p) {
   return v;
 }
 
+constexpr int kAskAhead = 20 * 1024;  // bytes of weights per warp group that are asked into L2 before they may be read (12 and 40 KB: slower)
 constexpr int kStageUnroll = 2;  // pair-loop unrolling of the NVFP4 / FP8 stages
 
 struct TiledArgs {
@@ -356,13 +357,12 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
     };
     // The ring is filled with weights first (they do not depend on the preceding kernel);
     // only then wait for that kernel and fetch the activations it produced.
-    auto first_images = [&](auto &&take) {
+    auto fill = [&]() {
       int slot = 0;
       for (int j = 0; j < most && slot < nst; ++j)
         for (int g = 0; g < kGroups && slot < nst; ++g, ++slot)
-          if (third(g) + j < third(g + 1)) take(third(g) + j, slot);
+          if (third(g) + j < third(g + 1)) copy_in(third(g) + j, slot);
     };
-    auto fill = [&]() { first_images(copy_in); };
     if (lane == 0) {
       for (int i = 0; i < nst; ++i) {
         mbar_init(smem_u32(&bar_full[i]), 1);
@@ -378,13 +378,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
       mbar_init(smem_u32(&bar_x), 1);
       mbar_init(smem_u32(&bar_never), 1);
       mbar_init_fence();
-      if (a.early) {
-        fill();
-      } else {  // into L2, whatever the kernel before writes: they are read there, behind the wait
-        first_images([&](int img, int) {
-          l2_prefetch(a.tiled + sc.image_offset(img), static_cast<uint32_t>(img < sc.e4 ? sc.img4 : sc.img8));
-        });
-      }
+      if (a.early) fill();
     }
     __syncwarp();
     __syncthreads();
@@ -431,8 +425,18 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
   if (warp > kMmaWarps) {
     // =============================================================== epilogue warps
     const int ej = warp - kMmaWarps - 1;
-    if (!a.early) pdl_wait();
     const int g_begin = third(ej), g_end = third(ej + 1);
+    if (!a.early) {
+      // Without leave to read weights early they are asked into L2 ahead of the wait, which is right whatever
+      // the kernel before writes: the copies behind the wait read them there.  By these warps, for they have
+      // nothing else to do now (the producer, image by image, delayed its own wait by 0.5 us).  Not in the
+      // variants that chains with the flag use: the code alone cost them 0.5 %.
+      if (EXTRA == 0 || EXTRA == 4) {
+        const long long from = sc.image_offset(g_begin), to = min(sc.image_offset(g_end), from + kAskAhead);
+        for (long long at = from + lane * 128; at < to; at += 32 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.tiled + at));
+      }
+      pdl_wait();
+    }
     // the first tile to finish: the one of the group's first image, unless an earlier group has an image of it
     int gt = 0, f = 0, S = 1, fmt = 0;
     bool mine = g_begin < g_end;
