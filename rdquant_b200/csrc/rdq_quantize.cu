@@ -386,6 +386,7 @@ struct LayerEncodeArgs {
   __nv_bfloat16 *fp16;
   float *tops;  // [block of the first pass]: largest NVFP4 block scale, largest magnitude of the FP8 group
   int segs;     // pieces of a row
+  int len;      // of 32 vectors each, in a piece
   float *global_scale;
   int32_t *inv_perm;
   int *bad_index;  // pinned host word: 1 once an entry of a permutation was out of range
@@ -398,36 +399,43 @@ __device__ __forceinline__ long long source_row(const LayerEncodeArgs &a, int r)
   return s < 0 || s >= n ? -1 : s;
 }
 
-// Pieces of rows as a warp takes them: kPiece vectors per lane, those of the next piece loaded before
-// the present one is encoded.
-constexpr int kPiece = 2;
-template <typename T>
+// Pieces of rows as a warp takes them: up to P vectors per lane, those of the next piece loaded before
+// the present one is encoded.  A piece costs about 70 instructions besides its vectors (which row it is,
+// the channel, addresses); with pieces of five vectors of halves instead of two, and the registers for
+// them (three blocks to an SM), a 2560 x 9728 layer takes 23.7 instead of 26.3 us, 13840 x 3884 39.1 instead of
+// 47.3.  Six or more, or four with the registers of four blocks, are slower; floats take twice the
+// registers.  FULL: pieces have P (a row's last one maybe fewer), else a.len: asking costs 1.5 us of the 39.
+constexpr int kShortPiece = 2, kLongPiece = 5;
+template <int P>
+constexpr int kBlocks = P > kShortPiece ? 3 : 4;
+template <typename T, int P, bool FULL>
 struct Piece {
-  Vec8<T> q[kPiece];
+  Vec8<T> q[P];
   int r, v0;  // row inside the pass's rows, first vector of this lane
+  static __device__ __forceinline__ bool has(const LayerEncodeArgs &a, int u) { return FULL || u < a.len; }
   __device__ __forceinline__ void load(const LayerEncodeArgs &a, int t, int first_row, int lane) {
     r = t / a.segs;
-    v0 = (t - r * a.segs) * 32 * kPiece + lane;
+    v0 = (t - r * a.segs) * 32 * a.len + lane;
     const T *row = static_cast<const T *>(a.w) + max(source_row(a, first_row + r), 0ll) * a.K;
 #pragma unroll
-    for (int u = 0; u < kPiece; ++u)
-      if (v0 + 32 * u < (a.K >> 3)) q[u].load(row + 8ll * (v0 + 32 * u));
+    for (int u = 0; u < P; ++u)
+      if (has(a, u) && v0 + 32 * u < (a.K >> 3)) q[u].load(row + 8ll * (v0 + 32 * u));
   }
 };
 
 // First pass over all rows: NVFP4 codes, the FP8 group's magnitude, FP16 rows, inverse permutation.
 // Bound by instruction issue for f16 input (about 130 warp instructions per 256 values, HBM asks for
 // less than 80): magnitudes and block scales come from packed halves and without a division, pieces
-// go round a single wave of blocks.  A warp per row left the last rows to a wave of their own and
-// waited three times per row: 20 us for 2560 x 9728, now 18, with the second pass 13.5 -> 10 us.
-template <typename T>
-__global__ void __launch_bounds__(256, 4) encode_layer_kernel(LayerEncodeArgs a) {
+// go round a single wave of blocks.  (A warp per row left the last rows to a wave of their own and
+// waited three times per row.)
+template <typename T, int P, bool FULL>
+__global__ void __launch_bounds__(256, kBlocks<P>) encode_layer_kernel(LayerEncodeArgs a) {
   pdl_launch_dependents();  // (launched in stream order: everything before it is complete)
   __shared__ float red[2][8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int K = a.K, nvec = K >> 3, tasks = (a.n4 + a.n8 + a.n16) * a.segs, stride = (gridDim.x * blockDim.x) >> 5;
   float top = 0.f, amax = 0.f, none = 0.f;
-  Piece<T> cur, next;
+  Piece<T, P, FULL> cur, next;
   int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (t < tasks) cur.load(a, t, 0, lane);
   for (; t < tasks; t += stride) {
@@ -439,9 +447,9 @@ __global__ void __launch_bounds__(256, 4) encode_layer_kernel(LayerEncodeArgs a)
       else *static_cast<volatile int *>(a.bad_index) = 1;  // (the row has channel 0's values)
     }
 #pragma unroll
-    for (int u = 0; u < kPiece; ++u) {
+    for (int u = 0; u < P; ++u) {
       const int i = v0 + 32 * u;
-      if (i - lane >= nvec) break;  // the whole warp is past the row
+      if (!cur.has(a, u) || i - lane >= nvec) break;  // the whole warp is past the row
       if (r < a.n4) {
         encode_vec_fp4<T, false>(cur.q[u], i < nvec, i, a.codes + 1ll * r * (K >> 1), a.scales + 1ll * r * (K >> 4), top, none);
       } else if (i >= nvec) {
@@ -477,12 +485,12 @@ __global__ void __launch_bounds__(256, 4) encode_layer_kernel(LayerEncodeArgs a)
 
 // Second pass: the FP8 rows (their scale is known now; they mostly come out of L2).  Channels that the
 // permutation does not name get row 0 as their inverse: whoever reads it finds an index in range.
-template <typename T>
-__global__ void __launch_bounds__(256, 4) encode_layer_fp8_kernel(LayerEncodeArgs a, int blocks) {
+template <typename T, int P, bool FULL>
+__global__ void __launch_bounds__(256, kBlocks<P>) encode_layer_fp8_kernel(LayerEncodeArgs a, int blocks) {
   __shared__ float red[2][8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nvec = a.K >> 3, tasks = a.n8 * a.segs, stride = (gridDim.x * blockDim.x) >> 5;
-  Piece<T> cur, next;
+  Piece<T, P, FULL> cur, next;
   int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (t < tasks) cur.load(a, t, a.n4, lane);  // (inputs of both passes)
   pdl_wait();
@@ -507,9 +515,9 @@ __global__ void __launch_bounds__(256, 4) encode_layer_fp8_kernel(LayerEncodeArg
   for (; t < tasks; t += stride) {
     if (t + stride < tasks) next.load(a, t + stride, a.n4, lane);
 #pragma unroll
-    for (int u = 0; u < kPiece; ++u) {
+    for (int u = 0; u < P; ++u) {
       const int i = cur.v0 + 32 * u;
-      if (i >= nvec) break;
+      if (!cur.has(a, u) || i >= nvec) break;
       float v[8];
       cur.q[u].get(v);
       reinterpret_cast<uint2 *>(a.fp8 + 1ll * cur.r * a.K)[i] = quotients_e4m3(v, scale, inv);
@@ -559,11 +567,11 @@ int bad_index_word(int **out) {
   return RDQ_OK;
 }
 
-template <typename T>
-int run_layer(const LayerEncodeArgs &a, cudaStream_t stream) {
-  static const int most1 = one_wave(encode_layer_kernel<T>), most2 = one_wave(encode_layer_fp8_kernel<T>);
+template <typename T, int P, bool FULL>
+int run_pieces(const LayerEncodeArgs &a, cudaStream_t stream) {
+  static const int most1 = one_wave(encode_layer_kernel<T, P, FULL>), most2 = one_wave(encode_layer_fp8_kernel<T, P, FULL>);
   const int blocks = static_cast<int>(std::min<long long>(most1, (1ll * (a.n4 + a.n8 + a.n16) * a.segs + 7) / 8));
-  encode_layer_kernel<T><<<blocks, 256, 0, stream>>>(a);
+  encode_layer_kernel<T, P, FULL><<<blocks, 256, 0, stream>>>(a);
   RDQ_CUDA(cudaGetLastError());
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -574,8 +582,22 @@ int run_layer(const LayerEncodeArgs &a, cudaStream_t stream) {
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  RDQ_CUDA(cudaLaunchKernelEx(&cfg, encode_layer_fp8_kernel<T>, a, blocks));
+  RDQ_CUDA(cudaLaunchKernelEx(&cfg, encode_layer_fp8_kernel<T, P, FULL>, a, blocks));
   return RDQ_OK;
+}
+// Pieces of a row have equal length: the warps take them in turn, so that a short one would always meet the
+// same warps.  Long ones where every warp of the chip gets at least ten vectors: 2560 x 2560 (seven) takes 11.9 us
+// with short pieces and 12.3 with long ones, 4096 x 2560 (twelve) 15.0 and 14.3.
+template <typename T>
+int run_layer(LayerEncodeArgs a, cudaStream_t stream) {
+  const int chunks = ((a.K >> 3) + 31) / 32;
+  const bool lengthy = sizeof(T) == 2 && 1ll * (a.n4 + a.n8 + a.n16) * chunks >= 10ll * sm_count() * kBlocks<kLongPiece> * 8;
+  const int most = lengthy ? kLongPiece : kShortPiece;
+  a.segs = (chunks + most - 1) / most;
+  a.len = (chunks + a.segs - 1) / a.segs;
+  if (!lengthy) return run_pieces<T, kShortPiece, true>(a, stream);  // (of one vector, if there is but one)
+  if constexpr (sizeof(T) == 2)
+    return a.len == kLongPiece ? run_pieces<T, kLongPiece, true>(a, stream) : run_pieces<T, kLongPiece, false>(a, stream);
 }
 
 template <typename T>
@@ -655,7 +677,6 @@ extern "C" int rdq_quantize_layer(const void *w, int w_is_f32, const long long *
   a.fp8_scale = fp8_scale;
   a.fp16 = static_cast<__nv_bfloat16 *>(fp16_bf16);
   a.tops = scratch;
-  a.segs = ((K >> 3) + 32 * kPiece - 1) / (32 * kPiece);
   a.global_scale = global_scale;
   a.inv_perm = inv_perm;
   return w_is_f32 ? run_layer<float>(a, stream) : run_layer<__half>(a, stream);

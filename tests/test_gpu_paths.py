@@ -153,6 +153,21 @@ def test_layer_encoder_edges(n4, n8, n16, k, dtype):
         assert a.dtype == b.dtype and torch.equal(a, b), key
 
 
+@pytest.mark.parametrize("n4,n8,n16,k", [(5000, 2150, 50, 1280), (4000, 2000, 0, 1296), (4000, 1200, 13, 1552), (0, 36000, 0, 16)])
+def test_layer_encoder_long_pieces(n4, n8, n16, k):
+    """Layers large enough for the encoder's long pieces of a row -- five vectors of 256 values, three, four and
+    a ragged rest, a fraction of one: byte for byte the host route."""
+    n = n4 + n8 + n16
+    w = _weights(n, k, n + k, torch.float16)
+    perm = torch.randperm(n, generator=torch.Generator().manual_seed(n))
+    splits = dict(zip(ORDER, (n4, n8, n16)))
+    host = pack_layer(quantize_weight(w, perm, splits), None)
+    dev = quantize_weight_packed(w.cuda(), perm, splits)
+    assert set(host) == set(dev)
+    for key in host:
+        assert torch.equal(host[key], dev[key].cpu()), key
+
+
 @pytest.mark.parametrize("m,twice", [(1, False), (8, False), (2, True)])
 def test_graphed_step_layers_beside_each_other(m, twice):
     """Layers of very different sizes that run beside each other, inputs changing from step to step; with a
