@@ -1,8 +1,11 @@
 // Bit-exact dequantisation of a packed mixed-precision layer to FP16 or FP32 [N, K] in original
 // channel order.  HBM-bound: reads the packed bytes once, writes 2 (or 4) N K bytes once.
 //
-// A warp per output row, a lane per 8 consecutive k: a warp instruction reads 128 / 256 / 512
-// contiguous bytes of an NVFP4 / FP8 / FP16 row and stores 512 (f16), four of them in flight.
+// A warp per piece of an output row, a lane per 8 consecutive k: a warp instruction reads 128 / 256 / 512
+// contiguous bytes of an NVFP4 / FP8 / FP16 row and stores 512 (f16), up to five of them in flight.
+// Pieces, because a warp per row leaves a layer of few long rows with too few warps (3884 rows of
+// 13840: 36.1 us, now 26.8) and one whose rows are a few more than the warps of the chip with a second
+// round for those (9728 rows of 2560: 14.0, now 12.4).
 // (16-element runs per thread, with 32-byte store strides and one run in flight, reached 1.9 TB/s.)
 //
 // Arithmetic follows the reference oracle exactly:
@@ -29,9 +32,10 @@ struct DequantArgs {
   const int32_t *inv_perm;
   void *out;
   int n4, n8, n16, K;
+  int segs, len;  // pieces of a row, vectors of eight in a piece
 };
 
-constexpr int kUnroll = 4;
+constexpr int kUnroll = 5;
 
 __device__ __forceinline__ void store8(__half *row, int v, const float (&f)[8]) {
   uint4 o;
@@ -60,8 +64,10 @@ template <typename OutT, bool VEC>
 __global__ void __launch_bounds__(256) dequant_kernel(DequantArgs a) {
   const int lane = threadIdx.x & 31;
   const int K = a.K, N = a.n4 + a.n8 + a.n16;
-  const int nvec = K >> 3;
-  for (int n = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; n < N; n += (gridDim.x * blockDim.x) >> 5) {
+  const unsigned task = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), segs = a.segs;
+  const int n = static_cast<int>(task / segs), first = static_cast<int>(task - n * segs) * a.len + lane;
+  const int nvec = min(K >> 3, first - lane + a.len);  // end of the piece
+  if (n < N) {
     const int r = a.inv_perm ? a.inv_perm[n] : n;
     OutT *row = static_cast<OutT *>(a.out) + 1ll * n * K;
     if (r < a.n4) {
@@ -69,7 +75,7 @@ __global__ void __launch_bounds__(256) dequant_kernel(DequantArgs a) {
       const uint32_t *src = reinterpret_cast<const uint32_t *>(a.w4 + 1ll * r * (K >> 1));
       const uint8_t *ssrc = a.s4 + 1ll * r * (K >> 4);
       const bool plain = sizeof(OutT) == 2 && a.global4 == 1.f;
-      for (int v0 = lane; v0 < nvec; v0 += 32 * kUnroll) {
+      for (int v0 = first; v0 < nvec; v0 += 32 * kUnroll) {
         uint32_t q[kUnroll], s[kUnroll];
 #pragma unroll
         for (int u = 0; u < kUnroll; ++u)
@@ -101,7 +107,7 @@ __global__ void __launch_bounds__(256) dequant_kernel(DequantArgs a) {
       const float sc = a.s8[rr];
       const uint8_t *src = a.w8 + 1ll * rr * K;
       if (VEC) {
-        for (int v0 = lane; v0 < nvec; v0 += 32 * kUnroll) {
+        for (int v0 = first; v0 < nvec; v0 += 32 * kUnroll) {
           uint2 q[kUnroll];
 #pragma unroll
           for (int u = 0; u < kUnroll; ++u)
@@ -126,7 +132,7 @@ __global__ void __launch_bounds__(256) dequant_kernel(DequantArgs a) {
       const long long off = 1ll * (r - a.n4 - a.n8) * K;
       const uint16_t *src = static_cast<const uint16_t *>(a.w16) + off;
       if (VEC) {
-        for (int v = lane; v < nvec; v += 32) {
+        for (int v = first; v < nvec; v += 32) {
           const uint4 q = __ldg(reinterpret_cast<const uint4 *>(src) + v);
           uint32_t h[4] = {q.x, q.y, q.z, q.w};
           if (a.w16_is_bf16) {
@@ -169,8 +175,11 @@ int launch_dequant(const void *w_fp4, const void *w_fp4_scales, float global4, c
   a.K = K;
   const long long rows = 1ll * n4 + n8 + n16;
   if (rows == 0) return RDQ_OK;
-  const unsigned blocks = static_cast<unsigned>(std::min<long long>((rows + 7) / 8, 8ll * sm_count()));
   const bool vec = K % 8 == 0;
+  const int chunks = (K / 8 + 31) / 32;
+  a.segs = vec ? std::max(1, (chunks + kUnroll - 1) / kUnroll) : 1;
+  a.len = 32 * ((chunks + a.segs - 1) / a.segs);
+  const unsigned blocks = static_cast<unsigned>((rows * a.segs + 7) / 8);
   if (out_is_f32) {
     if (vec) dequant_kernel<float, true><<<blocks, 256, 0, stream>>>(a);
     else dequant_kernel<float, false><<<blocks, 256, 0, stream>>>(a);

@@ -101,3 +101,16 @@ def test_bad_arguments_raise():
         rdquant_cuda.dequantize_packed({"weight_nvfp4": torch.zeros(4, 12, dtype=torch.uint8).cuda(),
                                         "weight_nvfp4_scale": torch.zeros(4, 1, dtype=torch.uint8).cuda()},
                                        {"NVFP4": 4}, 24)
+
+
+@pytest.mark.parametrize("k", [1280, 1296, 2576, 13840])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_rows_decoded_in_pieces(k, dtype):
+    """Rows of one whole piece, a vector more than that, and several with a ragged last one, bit for bit."""
+    n4, n8, n16 = 13, 9, 2
+    layer = random_packed_layer(n4, n8, n16, k, seed=k)
+    splits = dict(zip(ORDER, (n4, n8, n16)))
+    dev = {kk: v.cuda() for kk, v in layer.items()}
+    w = rdquant_cuda.dequantize_packed(dev, splits, k, inv_perm=dev["inv_permutation"], out_dtype=dtype)
+    ref = onp.dequantize_layer(onp.torch_layer_to_np(layer), splits, k)
+    assert np.array_equal(w.cpu().numpy().astype(np.float16).view(np.uint16), ref.view(np.uint16))
