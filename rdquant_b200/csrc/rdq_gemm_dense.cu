@@ -8,9 +8,10 @@
 // scratch costs 2 N K bytes written and read once per call (it mostly stays in the 126 MB L2) and
 // leaves a GEMM whose operands both arrive by TMA.
 //
-// Decoding pass (decode_rows_kernel), HBM-bound: a warp per output channel, a lane per 8 k -- loads
-// of 128 / 256 / 512 contiguous bytes and stores of 512 contiguous bytes per warp instruction, four
-// of them in flight.  NVFP4 is scaled by its block scale (exact in f16), FP8 stays unscaled: channel
+// Decoding pass (decode_rows_kernel), HBM-bound: a warp per piece of an output channel, a lane per 8 k --
+// loads of 128 / 256 / 512 contiguous bytes and stores of 512 contiguous bytes per warp instruction, five
+// of them in flight.  (A warp per channel left layers of few long rows with too few warps: see
+// rdq_dequant.cu.)  NVFP4 is scaled by its block scale (exact in f16), FP8 stays unscaled: channel
 // scale and NVFP4 global scale go into scale[N] and are applied to the FP32 sum.
 //
 // GEMM (gemm_pair_kernel): a cluster of two CTAs computes 256 channels x up to 256 tokens with
@@ -52,18 +53,19 @@ struct DecodeArgs {
   int *counters;  // zeroed for the GEMM
   int n_counters;
   int n4, n8, N, K;
+  int segs, len;        // pieces of a row, vectors of eight in a piece
   const uint4 *x_bf16;  // bf16 activations to round to f16 on the way (or null), in vectors of eight
   uint4 *x;
   long long x_vecs;
 };
 
-constexpr int kDecodeUnroll = 4;
+constexpr int kDecodeUnroll = 5;
 
 __global__ void __launch_bounds__(256) decode_rows_kernel(DecodeArgs a) {
   pdl_launch_dependents();  // (launched in stream order: everything before it is complete)
   const int lane = threadIdx.x & 31;
-  const int gid = blockIdx.x * blockDim.x + threadIdx.x;
-  for (int i = gid; i < a.n_counters; i += gridDim.x * blockDim.x) a.counters[i] = 0;
+  const long long gid = 1ll * blockIdx.x * blockDim.x + threadIdx.x;
+  for (long long i = gid; i < a.n_counters; i += 1ll * gridDim.x * blockDim.x) a.counters[i] = 0;
   if (a.x_bf16) {  // (a launch of its own for these took 3 us)
     const long long stride = 1ll * gridDim.x * blockDim.x;
     for (long long i = gid; i < a.x_vecs; i += 4 * stride) {
@@ -79,15 +81,17 @@ __global__ void __launch_bounds__(256) decode_rows_kernel(DecodeArgs a) {
     }
   }
   const int K = a.K;
-  const int nvec = K >> 3;  // runs of 8 k (the launcher requires K % 8 == 0)
-  for (int j = gid >> 5; j < a.N; j += (gridDim.x * blockDim.x) >> 5) {
+  const unsigned task = static_cast<unsigned>(gid >> 5), segs = a.segs;
+  const int j = static_cast<int>(task / segs), first = static_cast<int>(task - j * segs) * a.len + lane;
+  const int nvec = min(K >> 3, first - lane + a.len);  // end of the piece (the launcher requires K % 8 == 0)
+  if (j < a.N) {
     const int r = a.inv_perm ? a.inv_perm[j] : j;
     __half *orow = a.out + 1ll * j * K;
     if (r < a.n4) {
       const uint8_t *wrow = a.w4 + 1ll * r * (K >> 1);
       const uint8_t *srow = a.s4 + 1ll * r * (K >> 4);
-      if (lane == 0) a.scale[j] = a.global4;
-      for (int v0 = lane; v0 < nvec; v0 += 32 * kDecodeUnroll) {
+      if (first == 0) a.scale[j] = a.global4;
+      for (int v0 = first; v0 < nvec; v0 += 32 * kDecodeUnroll) {
         uint32_t q[kDecodeUnroll], s[kDecodeUnroll];
 #pragma unroll
         for (int u = 0; u < kDecodeUnroll; ++u) {
@@ -115,8 +119,8 @@ __global__ void __launch_bounds__(256) decode_rows_kernel(DecodeArgs a) {
     } else if (r < a.n4 + a.n8) {
       const int rr = r - a.n4;
       const uint8_t *wrow = a.w8 + 1ll * rr * K;
-      if (lane == 0) a.scale[j] = a.s8[rr];
-      for (int v0 = lane; v0 < nvec; v0 += 32 * kDecodeUnroll) {
+      if (first == 0) a.scale[j] = a.s8[rr];
+      for (int v0 = first; v0 < nvec; v0 += 32 * kDecodeUnroll) {
         uint2 q[kDecodeUnroll];
 #pragma unroll
         for (int u = 0; u < kDecodeUnroll; ++u) {
@@ -136,8 +140,8 @@ __global__ void __launch_bounds__(256) decode_rows_kernel(DecodeArgs a) {
       }
     } else {
       const uint4 *wrow = reinterpret_cast<const uint4 *>(a.w16 + 2ll * (r - a.n4 - a.n8) * K);
-      if (lane == 0) a.scale[j] = 1.f;
-      for (int v = lane; v < nvec; v += 32) reinterpret_cast<uint4 *>(orow)[v] = __ldg(wrow + v);
+      if (first == 0) a.scale[j] = 1.f;
+      for (int v = first; v < nvec; v += 32) reinterpret_cast<uint4 *>(orow)[v] = __ldg(wrow + v);
     }
   }
 }
@@ -586,7 +590,10 @@ int launch_gemm_dense(const GemmArgs &g, void *workspace, size_t workspace_bytes
   cudaLaunchConfig_t cfg = {};
   cfg.stream = stream;
   cfg.blockDim = dim3(256);
-  cfg.gridDim = dim3(static_cast<unsigned>(std::min(8 * sm_count(), (N + 7) / 8)));
+  const int chunks = (g.K / 8 + 31) / 32;
+  d.segs = std::max(1, (chunks + kDecodeUnroll - 1) / kDecodeUnroll);
+  d.len = 32 * ((chunks + d.segs - 1) / d.segs);
+  cfg.gridDim = dim3(static_cast<unsigned>((1ll * N * d.segs + 7) / 8));
   // In stream order, not overlapping the kernel before: calls that follow one another would chain GEMMs
   // without an end, and with fewer clusters than SM pairs the next call's clusters start beside this
   // one's.  Such a chain of 200 rows x 4560 -> 7017 stopped making progress after some hundred calls.
