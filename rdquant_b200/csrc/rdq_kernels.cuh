@@ -29,6 +29,7 @@ struct GemvArgs {
   int n4, n8, n16, K;
   int x_bf16 = 0;  // x is bf16: rounded to f16 as it is read
   int y_bf16 = 0;  // y is bf16 instead of f16
+  int ask_ahead = 0;  // (set by the launcher) ask the weights into L2 ahead of the grid-dependency wait
 };
 
 struct GemmArgs {

@@ -63,9 +63,9 @@ int stream_from(const rdq_layer &l) {
 // Estimates in microseconds, fitted to both kernels at 16 numbers of rows between 65 and 2048, f16 and
 // bf16, on 13 layers (channels x K: 6144, 19456, 4096, 9728 and 1024 x 2560, 2560 x 4096, 2560 x 9728,
 // 4096 x 3072, 16384 and 8192 x 8192, 1024 x 16384, 1024 and 11392 x 1024): off by 8 and 7 % on average, by
-// up to 40 % on the smallest.  Choosing by them costs 0.4 % on average over the faster kernel, 15 % at
-// worst (34 % once: 2048 bf16 rows x 1024 x 16384); the constants before, fitted to a decoding launch
-// that overlapped its predecessor, 1.6 %.  (With up to 64 rows the streaming GEMM was always faster.)
+// up to 40 % on the smallest.  With the decoding launch that takes a warp per piece of a channel, choosing by
+// them costs 0.6 % on average over the faster kernel, 13 % at worst, on eleven of these layers; refitted
+// constants would cost 0.2 %.  (With up to 64 rows the streaming GEMM was always faster.)
 bool stream_beats_dense(const rdq_layer &l, int M, int x_type) {
   if (M <= 64) return true;
   if (M > 2048) return false;
