@@ -71,7 +71,9 @@ __device__ __forceinline__ bool mbar_try_cluster(uint32_t bar, uint32_t parity, 
   return ok != 0;
 }
 
-// Wait on a barrier unless the CTA is aborting; raises the abort flag when about a second passed.
+// Wait on a barrier unless the CTA is aborting; raises the abort flag when about a second passed.  That
+// second is for this launch's own work: what waits may wait for the launch before as well, which can take
+// longer, so after a millisecond the wait goes on behind pdl_wait(), which has no limit of its own.
 // The first try carries no time hint: it returns 40 cycles sooner when the phase is complete.
 __device__ __forceinline__ bool mbar_try_now(uint32_t bar, uint32_t parity) {
   uint32_t ok;
@@ -89,6 +91,7 @@ __device__ __forceinline__ bool gemm_wait(uint64_t *bar, uint32_t parity, volati
   for (int i = 0; i < 20000; ++i) {
     if (mbar_try(smem_u32(bar), parity, 50000u)) return true;
     if (*abort_flag) return false;
+    if (i == 20) pdl_wait();
   }
   *abort_flag = 1;
   return false;
@@ -103,7 +106,7 @@ __device__ __forceinline__ bool gemm_wait_cluster(uint64_t *bar, uint32_t parity
   return false;
 }
 // The bounded wait as one asm block without branches that the compiler could see: 0 when it ran out
-// (20000 tries of up to 50 us).
+// (20000 tries of up to 50 us; the launch before has to be complete).
 __device__ __forceinline__ uint32_t wait_bounded(uint32_t bar, uint32_t parity) {
   uint32_t left;
   asm volatile(

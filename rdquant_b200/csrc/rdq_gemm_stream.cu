@@ -425,6 +425,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
     // diverge in it, every MMA's operands are moved to uniform registers again and an MMA takes 60
     // cycles to issue instead of 20.
     const bool leader = elect_one();
+    pdl_wait();  // (it needs the activations in any case, and its bounded waits are for this launch's own work)
     const uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(sc.nt >> 3) << 17) | (8u << 24);
     const uint64_t desc0 = make_desc_sw128(x_ring);
     const uint32_t dx0 = static_cast<uint32_t>(desc0), dx_hi = static_cast<uint32_t>(desc0 >> 32), box = x_bytes >> 4;

@@ -45,3 +45,29 @@ def test_kernels_wait_before_they_let_the_next_launch_start():
             early = m.start() < wait
             assert not early or name in ALWAYS_ONE_PER_SM or "if (first)" in m.group(1), name
     assert {"gemv_tiled_kernel", "gemm_stream_kernel", "gemm_pair_kernel", "gemv_rows_kernel", "rope_attn_kernel"} <= seen
+
+
+def _function(path, name):
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, path)).read())
+    start = text.index("{", re.search(r"__device__ __forceinline__ \w+ " + name + r"\(", text).end())
+    depth, i = 0, start
+    while True:
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        i += 1
+        if depth == 0:
+            return text[start:i]
+
+
+def test_bounded_waits_are_for_the_launch_s_own_work():
+    """What waits with a limit may be waiting for the launch before, however long that takes: the limit counts
+    from the end of that launch on."""
+    for path, name in (("rdq_gemm_common.cuh", "gemm_wait"),):
+        assert re.search(r"for \(.*pdl_wait\(\)", _function(path, name), re.S), name
+    bodies = dict(_kernels())
+    # the streaming GEMM: the MMA warp, whose waits are an asm block, needs the activations first
+    mma = bodies["gemm_stream_kernel"].split("else if (warp == 2) {")[1].split("else if (warp == 3) {")[0]
+    assert 0 <= mma.find("\n    pdl_wait();") < mma.index("wait_bounded(")
+    assert not re.search(r"\bmbar_(try|wait)\w*\((?!smem_u32\(&S\.never\))", bodies["gemm_stream_kernel"])
+    # the decoded-once GEMM waits for it with all threads, ahead of everything
+    pair = bodies["gemm_pair_kernel"]
+    assert 0 <= pair.find("\n  pdl_wait();") < pair.index("gemm_wait_cluster(")
