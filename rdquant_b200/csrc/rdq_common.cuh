@@ -190,6 +190,18 @@ __device__ __forceinline__ void pdl_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// mbar_wait() on what the launch before has a part in: the limit is for this launch's own work, and that
+// launch can take longer -- the gather of a tensor-parallel step lets the next GEMV start and then waits for
+// the other ranks -- so after a millisecond the wait goes on behind pdl_wait(), which has no limit of its own.
+__device__ __forceinline__ bool mbar_wait_launch(uint32_t bar, uint32_t parity) {
+#pragma unroll 1
+  for (uint32_t i = 0; i < 10000u; ++i) {
+    if (mbar_try(bar, parity, 100000u)) return true;
+    if (i == 10u) pdl_wait();
+  }
+  return false;
+}
+
 // ---------------------------------------------------------------------------
 // warp matrix helpers
 // ---------------------------------------------------------------------------

@@ -472,7 +472,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
       if (lane == 0 && b_last >= static_cast<int>(blockIdx.x) + 31) atomicExch(status, 7);
     }
     // y, workspace and flags belong to this launch only once the preceding grid is done
-    if (!mbar_wait(smem_u32(&bar_x), 0)) {
+    if (!mbar_wait_launch(smem_u32(&bar_x), 0)) {
       if (lane == 0) atomicExch(status, 6);
       return;
     }
@@ -658,7 +658,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
 
   // x is produced by the preceding kernel: do not touch it before the producer thread has
   // seen that kernel complete (and, with XS, has copied the rows into shared memory).
-  if (!mbar_wait(smem_u32(&bar_x), 0)) {
+  if (!mbar_wait_launch(smem_u32(&bar_x), 0)) {
     if (lane == 0) atomicExch(status, 6);
     return;
   }

@@ -61,13 +61,20 @@ def _function(path, name):
 def test_bounded_waits_are_for_the_launch_s_own_work():
     """What waits with a limit may be waiting for the launch before, however long that takes: the limit counts
     from the end of that launch on."""
-    for path, name in (("rdq_gemm_common.cuh", "gemm_wait"),):
+    for path, name in (("rdq_gemm_common.cuh", "gemm_wait"), ("rdq_common.cuh", "mbar_wait_launch")):
         assert re.search(r"for \(.*pdl_wait\(\)", _function(path, name), re.S), name
     bodies = dict(_kernels())
     # the streaming GEMM: the MMA warp, whose waits are an asm block, needs the activations first
     mma = bodies["gemm_stream_kernel"].split("else if (warp == 2) {")[1].split("else if (warp == 3) {")[0]
     assert 0 <= mma.find("\n    pdl_wait();") < mma.index("wait_bounded(")
     assert not re.search(r"\bmbar_(try|wait)\w*\((?!smem_u32\(&S\.never\))", bodies["gemm_stream_kernel"])
+    # the tiled GEMV: all warps but the producer begin with the barrier that stands for the launch before
+    tiled = bodies["gemv_tiled_kernel"]
+    producer, rest = tiled.split("if (warp > kMmaWarps) {")
+    assert 0 <= producer.find("if (!a.beside) pdl_wait();") < producer.index("mbar_wait(")
+    for part in rest.split("const int grp = warp / kWarpsPerGroup"):
+        waits = re.findall(r"\bmbar_\w*(?:try|wait)\w*\([^,]*", part)
+        assert waits[0] == "mbar_wait_launch(smem_u32(&bar_x)" and "bar_x" not in "".join(waits[1:])
     # the decoded-once GEMM waits for it with all threads, ahead of everything
     pair = bodies["gemm_pair_kernel"]
     assert 0 <= pair.find("\n  pdl_wait();") < pair.index("gemm_wait_cluster(")
