@@ -78,3 +78,24 @@ def test_bounded_waits_are_for_the_launch_s_own_work():
     # the decoded-once GEMM waits for it with all threads, ahead of everything
     pair = bodies["gemm_pair_kernel"]
     assert 0 <= pair.find("\n  pdl_wait();") < pair.index("gemm_wait_cluster(")
+
+
+def test_roles_of_the_streaming_gemm_wait_before_they_read():
+    """Without leave to read weights early, each warp of gemm_stream_kernel that reads memory has waited for the
+    launch before; ahead of that, addresses are only asked into L2."""
+    body = dict(_kernels())["gemm_stream_kernel"]
+    setup, *roles = re.split(r"(?:else )?if \(warp (?:== \d|< 8)\) \{", body[:body.index("finish_shared<")])
+    roles[-1:] = roles[-1].split("} else {", 1)  # the converters
+    assert len(roles) == 6
+    read = re.compile(r"load_chunk\(|tma_load_2d\(|row_of\(|cp_async\d+\(|\ba\.(s4|s8|perm|bias)\b")
+    waits = re.compile(r"(if \(!a\.early\) )?pdl_wait\(\)")
+    reading = 0
+    for role in roles:
+        first = read.search(role)
+        if first:
+            reading += 1
+            wait = waits.search(role)
+            assert wait and wait.start() < first.start(), role[:80]
+    assert reading == 4, "weights, activations, block scales, rows of the epilogue"
+    assert re.findall(r"if \(a\.early\) (\w+)\(|else (\w+)\(", setup[setup.index("Segment g"):])[:2] == [
+        ("load_chunk", ""), ("", "tma_prefetch_2d")]
