@@ -586,12 +586,15 @@ int run_pieces(const LayerEncodeArgs &a, cudaStream_t stream) {
   return RDQ_OK;
 }
 // Pieces of a row have equal length: the warps take them in turn, so that a short one would always meet the
-// same warps.  Long ones where every warp of the chip gets at least ten vectors: 2560 x 2560 (seven) takes 11.9 us
-// with short pieces and 12.3 with long ones, 4096 x 2560 (twelve) 15.0 and 14.3.
+// same warps.  Long ones where every warp of the chip gets at least ten vectors -- 2560 x 2560 (seven) takes 11.9 us
+// with short pieces and 12.3 with long ones, 4096 x 2560 (twelve) 15.0 and 14.3 -- and a row is longer than a
+// short piece: otherwise both have the same pieces, and the short kernel has the fourth block on an SM
+// (512 x 60000 33.1 us, 38.2 with the long one's three; 64 x 200000 70.3, 82.6; but 768 x 40000 36.0, 31.9).
 template <typename T>
 int run_layer(LayerEncodeArgs a, cudaStream_t stream) {
   const int chunks = ((a.K >> 3) + 31) / 32;
-  const bool lengthy = sizeof(T) == 2 && 1ll * (a.n4 + a.n8 + a.n16) * chunks >= 10ll * sm_count() * kBlocks<kLongPiece> * 8;
+  const long long vectors = 1ll * (a.n4 + a.n8 + a.n16) * chunks, warps = 8ll * sm_count() * kBlocks<kLongPiece>;
+  const bool lengthy = sizeof(T) == 2 && chunks > kShortPiece && vectors >= 10 * warps;
   const int most = lengthy ? kLongPiece : kShortPiece;
   a.segs = (chunks + most - 1) / most;
   a.len = (chunks + a.segs - 1) / a.segs;
