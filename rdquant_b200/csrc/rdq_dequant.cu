@@ -35,7 +35,10 @@ struct DequantArgs {
   int segs, len;  // pieces of a row, vectors of eight in a piece
 };
 
-constexpr int kUnroll = 5;
+// Most vectors of a lane in a piece.  Floats take twice the bytes: with five 1280 x 8000 FP16 rows took 15.7 us,
+// with four 14.5, 16384 x 512 NVFP4 rows 13.5 and 12.6; halves are faster with five (1280 x 8000 NVFP4 rows 8.5, 7.5).
+template <typename OutT>
+constexpr int kUnroll = sizeof(OutT) == 2 ? 5 : 4;
 
 __device__ __forceinline__ void store8(__half *row, int v, const float (&f)[8]) {
   uint4 o;
@@ -62,6 +65,7 @@ __device__ __forceinline__ void halves_to_floats(const uint32_t (&h)[4], float (
 // VEC: K % 8 == 0, so rows are whole runs of 8 with 16-byte (packed: 4-byte) alignment.
 template <typename OutT, bool VEC>
 __global__ void __launch_bounds__(256) dequant_kernel(DequantArgs a) {
+  constexpr int U = kUnroll<OutT>;
   const int lane = threadIdx.x & 31;
   const int K = a.K, N = a.n4 + a.n8 + a.n16;
   const unsigned task = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), segs = a.segs;
@@ -75,16 +79,16 @@ __global__ void __launch_bounds__(256) dequant_kernel(DequantArgs a) {
       const uint32_t *src = reinterpret_cast<const uint32_t *>(a.w4 + 1ll * r * (K >> 1));
       const uint8_t *ssrc = a.s4 + 1ll * r * (K >> 4);
       const bool plain = sizeof(OutT) == 2 && a.global4 == 1.f;
-      for (int v0 = first; v0 < nvec; v0 += 32 * kUnroll) {
-        uint32_t q[kUnroll], s[kUnroll];
+      for (int v0 = first; v0 < nvec; v0 += 32 * U) {
+        uint32_t q[U], s[U];
 #pragma unroll
-        for (int u = 0; u < kUnroll; ++u)
+        for (int u = 0; u < U; ++u)
           if (v0 + 32 * u < nvec) {
             q[u] = __ldg(src + v0 + 32 * u);
             s[u] = __ldg(ssrc + ((v0 + 32 * u) >> 1));
           }
 #pragma unroll
-        for (int u = 0; u < kUnroll; ++u) {
+        for (int u = 0; u < U; ++u) {
           if (v0 + 32 * u >= nvec) break;
           uint32_t h[4];
           cvt_e2m1x8(q[u], h[0], h[1], h[2], h[3]);
@@ -107,13 +111,13 @@ __global__ void __launch_bounds__(256) dequant_kernel(DequantArgs a) {
       const float sc = a.s8[rr];
       const uint8_t *src = a.w8 + 1ll * rr * K;
       if (VEC) {
-        for (int v0 = first; v0 < nvec; v0 += 32 * kUnroll) {
-          uint2 q[kUnroll];
+        for (int v0 = first; v0 < nvec; v0 += 32 * U) {
+          uint2 q[U];
 #pragma unroll
-          for (int u = 0; u < kUnroll; ++u)
+          for (int u = 0; u < U; ++u)
             if (v0 + 32 * u < nvec) q[u] = __ldg(reinterpret_cast<const uint2 *>(src) + v0 + 32 * u);
 #pragma unroll
-          for (int u = 0; u < kUnroll; ++u) {
+          for (int u = 0; u < U; ++u) {
             if (v0 + 32 * u >= nvec) break;
             uint32_t h[4];
             cvt_e4m3x4(q[u].x, h[0], h[1]);
@@ -177,7 +181,8 @@ int launch_dequant(const void *w_fp4, const void *w_fp4_scales, float global4, c
   if (rows == 0) return RDQ_OK;
   const bool vec = K % 8 == 0;
   const int chunks = (K / 8 + 31) / 32;
-  a.segs = vec ? std::max(1, (chunks + kUnroll - 1) / kUnroll) : 1;
+  const int most = out_is_f32 ? kUnroll<float> : kUnroll<__half>;
+  a.segs = vec ? std::max(1, (chunks + most - 1) / most) : 1;
   a.len = 32 * ((chunks + a.segs - 1) / a.segs);
   const unsigned blocks = static_cast<unsigned>((rows * a.segs + 7) / 8);
   if (out_is_f32) {
