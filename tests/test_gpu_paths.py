@@ -156,11 +156,36 @@ def test_layer_encoder_edges(n4, n8, n16, k, dtype):
 @pytest.mark.parametrize("n4,n8,n16,k", [(5000, 2150, 50, 1280), (4000, 2000, 0, 1296), (4000, 1200, 13, 1552), (0, 36000, 0, 16)])
 def test_layer_encoder_long_pieces(n4, n8, n16, k):
     """Layers large enough for the encoder's long pieces of a row -- five vectors of 256 values, three, four and
-    a ragged rest, a fraction of one: byte for byte the host route."""
+    a ragged rest -- and as large with rows of a fraction of one: byte for byte the host route."""
     n = n4 + n8 + n16
     w = _weights(n, k, n + k, torch.float16)
     perm = torch.randperm(n, generator=torch.Generator().manual_seed(n))
     splits = dict(zip(ORDER, (n4, n8, n16)))
+    host = pack_layer(quantize_weight(w, perm, splits), None)
+    dev = quantize_weight_packed(w.cuda(), perm, splits)
+    assert set(host) == set(dev)
+    for key in host:
+        assert torch.equal(host[key], dev[key].cpu()), key
+
+
+def _long_piece_rows(k):
+    """Rows from which the encoder takes the long pieces: ten vectors of 256 values for every warp of the chip."""
+    chunks = -(-(k // 8) // 32)
+    return -(-10 * torch.cuda.get_device_properties(0).multi_processor_count * 3 * 8 // chunks)
+
+
+@pytest.mark.parametrize("k", [16, 512, 528, 1280, 1296, 1552, 2560, 3344])
+@pytest.mark.parametrize("share8,share16", [(0.3, 0.01), (1.0, 0.0)])
+@pytest.mark.parametrize("fewer", [0, 1])
+def test_layer_encoder_pieces_by_size(k, share8, share16, fewer):
+    """Layers large enough for the encoder's long pieces of a row, and a row too small for them: rows of up to two
+    vectors of 256 values, which keep the short pieces, then two and a rest, five, three and a rest, four and a
+    rest, twice five, and 5 + 5 + 4; byte for byte the host route."""
+    n = _long_piece_rows(k) - fewer
+    n8, n16 = int(share8 * n), int(share16 * n)
+    w = _weights(n, k, n + k, torch.float16)
+    perm = torch.randperm(n, generator=torch.Generator().manual_seed(n))
+    splits = dict(zip(ORDER, (n - n8 - n16, n8, n16)))
     host = pack_layer(quantize_weight(w, perm, splits), None)
     dev = quantize_weight_packed(w.cuda(), perm, splits)
     assert set(host) == set(dev)
@@ -296,6 +321,40 @@ def test_layer_encoder_refuses_bad_permutations(k, bad):
     twice[5] = twice[6]  # not a permutation, but indices all the same
     inv = quantize_weight_packed(w, twice.cuda(), splits)["inv_permutation"]
     assert int(inv.min()) >= 0 and int(inv.max()) < 120 and int(inv[perm[5]]) == 0
+    rc.check_quantize_status("cuda")
+
+
+@pytest.mark.parametrize("k", [2560, 3344])
+def test_layer_encoder_permutations_with_long_pieces(k):
+    """The same for layers of long pieces: entries out of range at both ends of the formats, indices from the
+    end, an entry twice."""
+    n = _long_piece_rows(k)
+    n4, n8 = int(0.6 * n), int(0.3 * n)
+    splits = dict(zip(ORDER, (n4, n8, n - n4 - n8)))
+    w = _weights(n, k, k, torch.float16).cuda()
+    perm = torch.randperm(n, generator=torch.Generator().manual_seed(k))
+    rc.check_quantize_status("cuda")
+    good = quantize_weight_packed(w, perm, splits)
+    for at, bad in ((0, n), (n4 - 1, -n - 1), (n4, 1 << 40), (n - 1, -(1 << 40))):
+        wrong = perm.clone()
+        wrong[at] = bad
+        made = quantize_weight_packed(w, wrong.cuda(), splits)
+        with pytest.raises(RuntimeError, match="entry out of range"):
+            rc.check_quantize_status("cuda")
+        inv = made["inv_permutation"]
+        assert int(inv.min()) >= 0 and int(inv.max()) < n
+        inv[perm[at]] = at
+        assert torch.equal(inv, good["inv_permutation"]), "the other channels are where they belong"
+        other = torch.arange(n, device="cuda") != at  # the other NVFP4 and FP16 rows are what they were
+        assert torch.equal(made["weight_nvfp4"][other[:n4]], good["weight_nvfp4"][other[:n4]])
+        assert torch.equal(made["weight_fp16"][other[n4 + n8:]], good["weight_fp16"][other[n4 + n8:]])
+    fromend = quantize_weight_packed(w, (perm - n).cuda(), splits)
+    for key in good:
+        assert torch.equal(good[key], fromend[key]), key
+    twice = perm.clone()
+    twice[5] = twice[n - 1]
+    inv = quantize_weight_packed(w, twice.cuda(), splits)["inv_permutation"]
+    assert int(inv.min()) >= 0 and int(inv.max()) < n and int(inv[perm[5]]) == 0
     rc.check_quantize_status("cuda")
 
 
