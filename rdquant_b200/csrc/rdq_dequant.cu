@@ -4,8 +4,9 @@
 // A warp per piece of an output row, a lane per 8 consecutive k: a warp instruction reads 128 / 256 / 512
 // contiguous bytes of an NVFP4 / FP8 / FP16 row and stores 512 (f16), up to five of them in flight.
 // Pieces, because a warp per row leaves a layer of few long rows with too few warps (3884 rows of
-// 13840: 36.1 us, now 26.8) and one whose rows are a few more than the warps of the chip with a second
-// round for those (9728 rows of 2560: 14.0, now 12.4).
+// 13840: 34.4 us, now 25.3) and one whose rows are a few more than the warps of the chip with a second
+// round for those (9728 rows of 2560: 15.2, now 13.4).  A piece is one turn without a loop, whose registers would
+// leave floats six blocks on an SM instead of eight (64 x 300000 66.4 us, now 52.4).
 // (16-element runs per thread, with 32-byte store strides and one run in flight, reached 1.9 TB/s.)
 //
 // Arithmetic follows the reference oracle exactly:
@@ -35,8 +36,9 @@ struct DequantArgs {
   int segs, len;  // pieces of a row, vectors of eight in a piece
 };
 
-// Most vectors of a lane in a piece.  Floats take twice the bytes: with five 1280 x 8000 FP16 rows took 15.7 us,
-// with four 14.5, 16384 x 512 NVFP4 rows 13.5 and 12.6; halves are faster with five (1280 x 8000 NVFP4 rows 8.5, 7.5).
+// Most vectors of a lane in a piece.  Floats take twice the bytes: with five 1280 x 8000 FP16 rows take 17.3 us, with
+// four 14.4, 2560 x 4096 NVFP4 rows 15.7 and 14.0.  Halves: 1280 x 8000 6.8 us with five, 7.3 with four; longer rows
+// are up to 3 % faster with four.
 template <typename OutT>
 constexpr int kUnroll = sizeof(OutT) == 2 ? 5 : 4;
 
@@ -79,31 +81,29 @@ __global__ void __launch_bounds__(256) dequant_kernel(DequantArgs a) {
       const uint32_t *src = reinterpret_cast<const uint32_t *>(a.w4 + 1ll * r * (K >> 1));
       const uint8_t *ssrc = a.s4 + 1ll * r * (K >> 4);
       const bool plain = sizeof(OutT) == 2 && a.global4 == 1.f;
-      for (int v0 = first; v0 < nvec; v0 += 32 * U) {
-        uint32_t q[U], s[U];
+      uint32_t q[U], s[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u)
-          if (v0 + 32 * u < nvec) {
-            q[u] = __ldg(src + v0 + 32 * u);
-            s[u] = __ldg(ssrc + ((v0 + 32 * u) >> 1));
-          }
+      for (int u = 0; u < U; ++u)
+        if (first + 32 * u < nvec) {
+          q[u] = __ldg(src + first + 32 * u);
+          s[u] = __ldg(ssrc + ((first + 32 * u) >> 1));
+        }
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          if (v0 + 32 * u >= nvec) break;
-          uint32_t h[4];
-          cvt_e2m1x8(q[u], h[0], h[1], h[2], h[3]);
-          if (plain) {
-            const uint32_t sc = __byte_perm(cvt_e4m3x2(s[u]), 0u, 0x1010u);
-            reinterpret_cast<uint4 *>(row)[v0 + 32 * u] =
-                make_uint4(hmul2_u32(h[0], sc), hmul2_u32(h[1], sc), hmul2_u32(h[2], sc), hmul2_u32(h[3], sc));
-          } else {
-            const float sc = e4m3_to_float(s[u]) * a.global4;
-            float f[8];
-            halves_to_floats(h, f);
+      for (int u = 0; u < U; ++u) {
+        if (first + 32 * u >= nvec) break;
+        uint32_t h[4];
+        cvt_e2m1x8(q[u], h[0], h[1], h[2], h[3]);
+        if (plain) {
+          const uint32_t sc = __byte_perm(cvt_e4m3x2(s[u]), 0u, 0x1010u);
+          reinterpret_cast<uint4 *>(row)[first + 32 * u] =
+              make_uint4(hmul2_u32(h[0], sc), hmul2_u32(h[1], sc), hmul2_u32(h[2], sc), hmul2_u32(h[3], sc));
+        } else {
+          const float sc = e4m3_to_float(s[u]) * a.global4;
+          float f[8];
+          halves_to_floats(h, f);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) f[i] *= sc;
-            store8(row, v0 + 32 * u, f);
-          }
+          for (int i = 0; i < 8; ++i) f[i] *= sc;
+          store8(row, first + 32 * u, f);
         }
       }
     } else if (r < a.n4 + a.n8) {
@@ -111,23 +111,21 @@ __global__ void __launch_bounds__(256) dequant_kernel(DequantArgs a) {
       const float sc = a.s8[rr];
       const uint8_t *src = a.w8 + 1ll * rr * K;
       if (VEC) {
-        for (int v0 = first; v0 < nvec; v0 += 32 * U) {
-          uint2 q[U];
+        uint2 q[U];
 #pragma unroll
-          for (int u = 0; u < U; ++u)
-            if (v0 + 32 * u < nvec) q[u] = __ldg(reinterpret_cast<const uint2 *>(src) + v0 + 32 * u);
+        for (int u = 0; u < U; ++u)
+          if (first + 32 * u < nvec) q[u] = __ldg(reinterpret_cast<const uint2 *>(src) + first + 32 * u);
 #pragma unroll
-          for (int u = 0; u < U; ++u) {
-            if (v0 + 32 * u >= nvec) break;
-            uint32_t h[4];
-            cvt_e4m3x4(q[u].x, h[0], h[1]);
-            cvt_e4m3x4(q[u].y, h[2], h[3]);
-            float f[8];
-            halves_to_floats(h, f);
+        for (int u = 0; u < U; ++u) {
+          if (first + 32 * u >= nvec) break;
+          uint32_t h[4];
+          cvt_e4m3x4(q[u].x, h[0], h[1]);
+          cvt_e4m3x4(q[u].y, h[2], h[3]);
+          float f[8];
+          halves_to_floats(h, f);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) f[i] *= sc;
-            store8(row, v0 + 32 * u, f);
-          }
+          for (int i = 0; i < 8; ++i) f[i] *= sc;
+          store8(row, first + 32 * u, f);
         }
       } else {
         for (int k = lane; k < K; k += 32) row[k] = static_cast<OutT>(e4m3_to_float(src[k]) * sc);
@@ -136,16 +134,21 @@ __global__ void __launch_bounds__(256) dequant_kernel(DequantArgs a) {
       const long long off = 1ll * (r - a.n4 - a.n8) * K;
       const uint16_t *src = static_cast<const uint16_t *>(a.w16) + off;
       if (VEC) {
-        for (int v = first; v < nvec; v += 32) {
-          const uint4 q = __ldg(reinterpret_cast<const uint4 *>(src) + v);
-          uint32_t h[4] = {q.x, q.y, q.z, q.w};
+        uint4 q[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (first + 32 * u < nvec) q[u] = __ldg(reinterpret_cast<const uint4 *>(src) + first + 32 * u);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (first + 32 * u >= nvec) break;
+          uint32_t h[4] = {q[u].x, q[u].y, q[u].z, q[u].w};
           if (a.w16_is_bf16) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) h[i] = bf16x2_to_f16x2(h[i]);
           }
           float f[8];
           halves_to_floats(h, f);
-          store8(row, v, f);
+          store8(row, first + 32 * u, f);
         }
       } else {
         for (int k = lane; k < K; k += 32) {
@@ -180,10 +183,9 @@ int launch_dequant(const void *w_fp4, const void *w_fp4_scales, float global4, c
   const long long rows = 1ll * n4 + n8 + n16;
   if (rows == 0) return RDQ_OK;
   const bool vec = K % 8 == 0;
-  const int chunks = (K / 8 + 31) / 32;
-  const int most = out_is_f32 ? kUnroll<float> : kUnroll<__half>;
-  a.segs = vec ? std::max(1, (chunks + most - 1) / most) : 1;
-  a.len = 32 * ((chunks + a.segs - 1) / a.segs);
+  const RowPieces cut = vec ? row_pieces(K, out_is_f32 ? kUnroll<float> : kUnroll<__half>) : RowPieces{1, 0};
+  a.segs = cut.pieces;
+  a.len = 32 * cut.len;
   const unsigned blocks = static_cast<unsigned>((rows * a.segs + 7) / 8);
   if (out_is_f32) {
     if (vec) dequant_kernel<float, true><<<blocks, 256, 0, stream>>>(a);

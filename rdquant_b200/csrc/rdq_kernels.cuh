@@ -159,6 +159,16 @@ int launch_attn_decode(const __half *q, const __half *k_cache, const __half *v_c
                        __half *out, int B, int nq, int nkv, int dh, int S, float scale, bool pdl, cudaStream_t stream);
 int launch_silu_mul(const __half *gu, __half *out, int B, int F, bool pdl, cudaStream_t stream);
 
+// A row of K values cut into `pieces` of equal length -- `len` turns of a warp whose lanes hold eight values each,
+// at most `most` -- of which only the last can be shorter.
+struct RowPieces {
+  int pieces, len;
+};
+inline RowPieces row_pieces(int K, int most) {
+  const int turns = (K / 8 + 31) / 32, pieces = turns > most ? (turns + most - 1) / most : 1;
+  return {pieces, (turns + pieces - 1) / pieces};
+}
+
 // encoders (rdq_quantize.cu)
 int launch_quantize_nvfp4(const void *w, bool w_is_f32, int n, int K, uint8_t *codes, uint8_t *scales, float *row_sqerr,
                           float *max_scale, cudaStream_t stream);
