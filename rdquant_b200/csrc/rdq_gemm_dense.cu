@@ -9,7 +9,7 @@
 // leaves a GEMM whose operands both arrive by TMA.
 //
 // Decoding pass (decode_rows_kernel), HBM-bound: a warp per piece of an output channel, a lane per 8 k --
-// loads of 128 / 256 / 512 contiguous bytes and stores of 512 contiguous bytes per warp instruction, five
+// loads of 128 / 256 / 512 contiguous bytes and stores of 512 contiguous bytes per warp instruction, up to five
 // of them in flight.  (A warp per channel left layers of few long rows with too few warps: see
 // rdq_dequant.cu.)  NVFP4 is scaled by its block scale (exact in f16), FP8 stays unscaled: channel
 // scale and NVFP4 global scale go into scale[N] and are applied to the FP32 sum.
@@ -91,57 +91,59 @@ __global__ void __launch_bounds__(256) decode_rows_kernel(DecodeArgs a) {
       const uint8_t *wrow = a.w4 + 1ll * r * (K >> 1);
       const uint8_t *srow = a.s4 + 1ll * r * (K >> 4);
       if (first == 0) a.scale[j] = a.global4;
-      for (int v0 = first; v0 < nvec; v0 += 32 * kDecodeUnroll) {
-        uint32_t q[kDecodeUnroll], s[kDecodeUnroll];
+      uint32_t q[kDecodeUnroll], s[kDecodeUnroll];
 #pragma unroll
-        for (int u = 0; u < kDecodeUnroll; ++u) {
-          const int v = v0 + 32 * u;
-          if (v < nvec) {
-            q[u] = __ldg(reinterpret_cast<const uint32_t *>(wrow) + v);
-            s[u] = __ldg(srow + (v >> 1));
-          }
+      for (int u = 0; u < kDecodeUnroll; ++u) {
+        const int v = first + 32 * u;
+        if (v < nvec) {
+          q[u] = __ldg(reinterpret_cast<const uint32_t *>(wrow) + v);
+          s[u] = __ldg(srow + (v >> 1));
         }
+      }
 #pragma unroll
-        for (int u = 0; u < kDecodeUnroll; ++u) {
-          const int v = v0 + 32 * u;
-          if (v < nvec) {
-            const uint32_t scl = __byte_perm(cvt_e4m3x2(s[u]), 0u, 0x1010u);
-            uint4 o;
-            cvt_e2m1x8(q[u], o.x, o.y, o.z, o.w);
-            o.x = hmul2_u32(o.x, scl);
-            o.y = hmul2_u32(o.y, scl);
-            o.z = hmul2_u32(o.z, scl);
-            o.w = hmul2_u32(o.w, scl);
-            reinterpret_cast<uint4 *>(orow)[v] = o;
-          }
+      for (int u = 0; u < kDecodeUnroll; ++u) {
+        const int v = first + 32 * u;
+        if (v < nvec) {
+          const uint32_t scl = __byte_perm(cvt_e4m3x2(s[u]), 0u, 0x1010u);
+          uint4 o;
+          cvt_e2m1x8(q[u], o.x, o.y, o.z, o.w);
+          o.x = hmul2_u32(o.x, scl);
+          o.y = hmul2_u32(o.y, scl);
+          o.z = hmul2_u32(o.z, scl);
+          o.w = hmul2_u32(o.w, scl);
+          reinterpret_cast<uint4 *>(orow)[v] = o;
         }
       }
     } else if (r < a.n4 + a.n8) {
       const int rr = r - a.n4;
       const uint8_t *wrow = a.w8 + 1ll * rr * K;
       if (first == 0) a.scale[j] = a.s8[rr];
-      for (int v0 = first; v0 < nvec; v0 += 32 * kDecodeUnroll) {
-        uint2 q[kDecodeUnroll];
+      uint2 q[kDecodeUnroll];
 #pragma unroll
-        for (int u = 0; u < kDecodeUnroll; ++u) {
-          const int v = v0 + 32 * u;
-          if (v < nvec) q[u] = __ldg(reinterpret_cast<const uint2 *>(wrow) + v);
-        }
+      for (int u = 0; u < kDecodeUnroll; ++u) {
+        const int v = first + 32 * u;
+        if (v < nvec) q[u] = __ldg(reinterpret_cast<const uint2 *>(wrow) + v);
+      }
 #pragma unroll
-        for (int u = 0; u < kDecodeUnroll; ++u) {
-          const int v = v0 + 32 * u;
-          if (v < nvec) {
-            uint4 o;
-            cvt_e4m3x4(q[u].x, o.x, o.y);
-            cvt_e4m3x4(q[u].y, o.z, o.w);
-            reinterpret_cast<uint4 *>(orow)[v] = o;
-          }
+      for (int u = 0; u < kDecodeUnroll; ++u) {
+        const int v = first + 32 * u;
+        if (v < nvec) {
+          uint4 o;
+          cvt_e4m3x4(q[u].x, o.x, o.y);
+          cvt_e4m3x4(q[u].y, o.z, o.w);
+          reinterpret_cast<uint4 *>(orow)[v] = o;
         }
       }
     } else {
       const uint4 *wrow = reinterpret_cast<const uint4 *>(a.w16 + 2ll * (r - a.n4 - a.n8) * K);
       if (first == 0) a.scale[j] = 1.f;
-      for (int v = first; v < nvec; v += 32) reinterpret_cast<uint4 *>(orow)[v] = __ldg(wrow + v);
+      uint4 q[kDecodeUnroll];
+#pragma unroll
+      for (int u = 0; u < kDecodeUnroll; ++u)
+        if (first + 32 * u < nvec) q[u] = __ldg(wrow + first + 32 * u);
+#pragma unroll
+      for (int u = 0; u < kDecodeUnroll; ++u)
+        if (first + 32 * u < nvec) reinterpret_cast<uint4 *>(orow)[first + 32 * u] = q[u];
     }
   }
 }
@@ -590,9 +592,9 @@ int launch_gemm_dense(const GemmArgs &g, void *workspace, size_t workspace_bytes
   cudaLaunchConfig_t cfg = {};
   cfg.stream = stream;
   cfg.blockDim = dim3(256);
-  const int chunks = (g.K / 8 + 31) / 32;
-  d.segs = std::max(1, (chunks + kDecodeUnroll - 1) / kDecodeUnroll);
-  d.len = 32 * ((chunks + d.segs - 1) / d.segs);
+  const RowPieces cut = row_pieces(g.K, kDecodeUnroll);
+  d.segs = cut.pieces;
+  d.len = 32 * cut.len;
   cfg.gridDim = dim3(static_cast<unsigned>((1ll * N * d.segs + 7) / 8));
   // In stream order, not overlapping the kernel before: calls that follow one another would chain GEMMs
   // without an end, and with fewer clusters than SM pairs the next call's clusters start beside this
