@@ -383,8 +383,8 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
     __syncwarp();
     __syncthreads();
     if (lane != 0) return;
-    // Only this thread executes the grid-dependency wait; every other warp of the CTA
-    // sleeps on bar_x, which completes after it (and after the activation copies).
+    // This thread executes the grid-dependency wait (without the flag the epilogue warps do as well); the
+    // other warps sleep on bar_x, which completes after it (and after the activation copies).
     if (!a.beside) pdl_wait();
     if (!first) pdl_launch_dependents();
     const uint32_t bx = smem_u32(&bar_x);
@@ -429,8 +429,9 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
     if (!a.early) {
       // Without leave to read weights early they are asked into L2 ahead of the wait, which is right whatever
       // the kernel before writes: the copies behind the wait read them there.  By these warps, for they have
-      // nothing else to do now (the producer, image by image, delayed its own wait by 0.5 us).  Not in the
-      // variants that chains with the flag use: the code alone cost them 0.5 %.
+      // nothing else to do now (the producer, image by image, delayed its own wait by 0.5 us).  In the plain
+      // variant, where chains with the flag carry the code as well (host-to-host step 39.4 and 39.3 us without
+      // and with it), and in that of bf16 rows; the norm and SiLU variants lost 0.5 % to the code alone.
       if (EXTRA == 0 || EXTRA == 4) {
         const long long from = sc.image_offset(g_begin), to = min(sc.image_offset(g_end), from + kAskAhead);
         for (long long at = from + lane * 128; at < to; at += 32 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.tiled + at));

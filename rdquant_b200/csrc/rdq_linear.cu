@@ -40,14 +40,18 @@ bool has_row_major(const rdq_layer &l) {
   return (l.n_fp4 == 0 || l.w_fp4) && (l.n_fp8 == 0 || l.w_fp8) && (l.n_fp16 == 0 || l.w_fp16);
 }
 
-// Fewest rows for which the streaming GEMM beats the decode GEMV.  Measured times are about
-// a + bytes / rate with a = 4.5 us and 4.2 (1, 2 rows) or 2.9 TB/s (up to 8) for the GEMV, whose
-// converter work and activation reads grow with the rows, against 9.5 us and 5.8 TB/s whatever the
-// rows: equal at 75 and 29 MB of packed weights (40 measured); above 8 rows the GEMV halves its rate.
+// Fewest rows for which the streaming GEMM is taken instead of the decode GEMV.  The GEMV slows with the rows
+// (its conversions and activation reads grow with them, above 8 rows it halves its rate), the streaming GEMM hardly
+// does.  Calls one after another, GEMV / streaming GEMM in us, without RDQ_GEMV_PDL and with it:
+//   36 MB (19456 x 2560)  8 rows 11.1 / 14.5, 14.8 / 13.9     9 rows 24.1 / 14.5, 22.2 / 14.0
+//   40 MB (13440 x 4096)  4 rows 10.9 / 14.8, 13.5 / 14.0     8 rows 16.3 / 14.8, 17.4 / 14.2
+//   48 MB (8192 x 8192)   2 rows 11.9 / 15.7, 15.8 / 14.8     4 rows 18.3 / 16.0, 19.9 / 15.0
+//   97 MB (16384 x 8192)  1 row  19.6 / 22.8, 27.8 / 21.7     4 rows 31.5 / 23.2, 36.5 / 22.1
 // The row-major GEMV of layers without a tiled layout starts at 1.9 us where the streaming GEMM takes 6
-// to 9 (300 NVFP4 + 130 FP8 + 20 FP16 rows of 1024: 2.3 against 9.0 us at one row), and is slower from
-// 40 MB (9001 + 4500 + 3 of 4096: 17.2 us each at 8 rows), above 8 rows from 18 MB (6500 + 3100 + 128 of
-// 2560: 13.5 us each at 14 rows).
+// to 9 (300 NVFP4 + 130 FP8 + 20 FP16 rows of 1024: 2.3 against 9.0 us at one row).  Its lines, 40 MB up to 8
+// rows and 18 MB up to 16, date from a streaming GEMM that set up behind its wait; now 19 MB (6500 x 4096) takes
+// 12.2 us on either at 8 rows and 40 MB (13504 x 4096) 18.1 / 14.9, at 16 rows 11 MB (6144 x 2560) 9.1 / 10.9 and 18 MB
+// (2560 x 9728) 14.5 / 12.8.
 int stream_from(const rdq_layer &l) {
   const double bytes = l.n_fp4 * (l.K * 0.5625) + l.n_fp8 * (l.K + 4.0) + l.n_fp16 * (l.K * 2.0);
   if (!l.w_tiled) return bytes > 40e6 ? 1 : (bytes > 18e6 ? 9 : RDQ_MAX_GEMV_M + 1);
@@ -63,9 +67,10 @@ int stream_from(const rdq_layer &l) {
 // Estimates in microseconds, fitted to both kernels at 16 numbers of rows between 65 and 2048, f16 and
 // bf16, on 13 layers (channels x K: 6144, 19456, 4096, 9728 and 1024 x 2560, 2560 x 4096, 2560 x 9728,
 // 4096 x 3072, 16384 and 8192 x 8192, 1024 x 16384, 1024 and 11392 x 1024): off by 8 and 7 % on average, by
-// up to 40 % on the smallest.  With the decoding launch that takes a warp per piece of a channel, choosing by
-// them costs 0.6 % on average over the faster kernel, 13 % at worst, on eleven of these layers; refitted
-// constants would cost 0.2 %.  (With up to 64 rows the streaming GEMM was always faster.)
+// up to 40 % on the smallest.  With the present kernels, choosing by them costs 0.3 % on average over the faster
+// one on these layers (above 512 rows without 16384 x 8192, where the power cap decides), 31 % at worst (1024 x 16384
+// at 2048 f16 rows, 17 % at 1536), elsewhere up to 12 %; on 3584 x 2048, 13824 x 3584, 5120 x 5120, 3072 x 12288
+// and 2048 x 6144 0.2 %, 10 % at worst.  (With up to 64 rows the streaming GEMM was always faster.)
 bool stream_beats_dense(const rdq_layer &l, int M, int x_type) {
   if (M <= 64) return true;
   if (M > 2048) return false;

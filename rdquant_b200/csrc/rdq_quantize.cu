@@ -402,7 +402,7 @@ __device__ __forceinline__ long long source_row(const LayerEncodeArgs &a, int r)
 // Pieces of rows as a warp takes them: up to P vectors per lane, those of the next piece loaded before
 // the present one is encoded.  A piece costs about 70 instructions besides its vectors (which row it is,
 // the channel, addresses); with pieces of five vectors of halves instead of two, and the registers for
-// them (three blocks to an SM), a 2560 x 9728 layer takes 23.7 instead of 26.3 us, 13840 x 3884 39.1 instead of
+// them (three blocks to an SM), a 2560 x 9728 layer takes 23.7 instead of 26.1 us, 13840 x 3884 39.1 instead of
 // 47.3.  Six or more, or four with the registers of four blocks, are slower; floats take twice the
 // registers.  FULL: pieces have P (a row's last one maybe fewer), else a.len: asking costs 1.5 us of the 39.
 constexpr int kShortPiece = 2, kLongPiece = 5;
@@ -424,9 +424,9 @@ struct Piece {
 };
 
 // First pass over all rows: NVFP4 codes, the FP8 group's magnitude, FP16 rows, inverse permutation.
-// Bound by instruction issue for f16 input (about 130 warp instructions per 256 values, HBM asks for
-// less than 80): magnitudes and block scales come from packed halves and without a division, pieces
-// go round a single wave of blocks.  (A warp per row left the last rows to a wave of their own and
+// Bound by instruction issue for f16 input (88 warp instructions per 256 values with long pieces, 113 with short
+// ones; 60 % of the issue slots, 34 % of the DRAM rate): magnitudes and block scales come from packed halves
+// and without a division, pieces go round a single wave of blocks.  (A warp per row left the last rows to a wave of their own and
 // waited three times per row.)
 template <typename T, int P, bool FULL>
 __global__ void __launch_bounds__(256, kBlocks<P>) encode_layer_kernel(LayerEncodeArgs a) {
@@ -595,9 +595,9 @@ int run_layer(LayerEncodeArgs a, cudaStream_t stream) {
   const int chunks = ((a.K >> 3) + 31) / 32;
   const long long vectors = 1ll * (a.n4 + a.n8 + a.n16) * chunks, warps = 8ll * sm_count() * kBlocks<kLongPiece>;
   const bool lengthy = sizeof(T) == 2 && chunks > kShortPiece && vectors >= 10 * warps;
-  const int most = lengthy ? kLongPiece : kShortPiece;
-  a.segs = (chunks + most - 1) / most;
-  a.len = (chunks + a.segs - 1) / a.segs;
+  const RowPieces cut = row_pieces(a.K, lengthy ? kLongPiece : kShortPiece);
+  a.segs = cut.pieces;
+  a.len = cut.len;
   if (!lengthy) return run_pieces<T, kShortPiece, true>(a, stream);  // (of one vector, if there is but one)
   if constexpr (sizeof(T) == 2)
     return a.len == kLongPiece ? run_pieces<T, kLongPiece, true>(a, stream) : run_pieces<T, kLongPiece, false>(a, stream);
