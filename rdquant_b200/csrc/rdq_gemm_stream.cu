@@ -117,7 +117,7 @@ struct StreamArgs {
   int patience;
   int nw;             // weight chunks in flight
   int early;          // weights may be read before the kernel before this one has finished
-  int scale16;     // block-scale rows can be copied 16 bytes at a time
+  int scale_bytes;  // a block-scale row is copied 16, 8 or 4 bytes at a time
   int test_timeout;
 };
 
@@ -167,6 +167,9 @@ struct Cursor {
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async8(uint32_t dst, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async4(uint32_t dst, const void *src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
@@ -490,25 +493,36 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
     __syncwarp();
   } else if (warp == 3) {
     // ------------------------------------------------------------------ block scales
+    // (a row's address once per tile: with it computed per chunk this warp was late at times; 8192 -> 57344 at 16 rows 56.3 us, now 55.3)
     if (!a.early) pdl_wait();
     Cursor w;
     const int pitch = a.K >> 4;
-    Segment g = segment_at(sc, begin, end);
+    Segment g;
+    g.start = g.c1 = 0;
+    const uint8_t *src[4];
+    int rows = 0;
     for (int i = begin; i < end; ++i) {
-      if (i >= g.start + g.c1) g = segment_at(sc, i, end);
-      if (!gemm_wait(&S.w_empty[w.i], w.ph ^ 1, &S.abort_flag)) break;
-      if (g.fmt == 0) {
-        const int c = i - g.start;
-        const uint32_t dst = s_ring + w.i * kScaleBytes;
-        const int words = min(4, sc.nkb - 4 * c);
+      if (i == begin || i >= g.start + g.c1) {
+        g = segment_at(sc, i, end);
+        rows = g.fmt != 0 ? 0 : 4;
 #pragma unroll
+        for (int u = 0; u < 4; ++u) src[u] = a.s4 + 1ll * min(g.row_tile * 128 + u * 32 + lane, a.n4 - 1) * pitch;
+      }
+      if (!gemm_wait(&S.w_empty[w.i], w.ph ^ 1, &S.abort_flag)) break;
+      const int c = i - g.start;
+      const uint32_t dst = s_ring + w.i * kScaleBytes + lane * 16;
+      if (a.scale_bytes == 16) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (u < rows) cp_async16(dst + u * 512, src[u] + c * 16);
+      } else {
+        const int words = min(4, sc.nkb - 4 * c);
         for (int u = 0; u < 4; ++u) {
-          const int r = u * 32 + lane;
-          const uint8_t *src = a.s4 + 1ll * min(g.row_tile * 128 + r, a.n4 - 1) * pitch + c * 16;
-          if (a.scale16) {
-            cp_async16(dst + r * 16, src);
-          } else {
-            for (int j = 0; j < words; ++j) cp_async4(dst + r * 16 + 4 * j, src + 4 * j);
+          if (u >= rows) break;
+          const uint8_t *from = u == 0 ? src[0] : (u == 1 ? src[1] : (u == 2 ? src[2] : src[3]));
+          for (int j = 0; j < words; j += a.scale_bytes >> 2) {
+            if (a.scale_bytes == 8) cp_async8(dst + u * 512 + 4 * j, from + c * 16 + 4 * j);
+            else cp_async4(dst + u * 512 + 4 * j, from + c * 16 + 4 * j);
           }
         }
       }
@@ -811,7 +825,7 @@ int launch_gemm_stream(const GemmArgs &g, void *workspace, size_t workspace_byte
   a.arrived = reinterpret_cast<uint32_t *>(g.counters);
   a.nw = p.nw;
   a.early = pdl;
-  a.scale16 = g.K % 256 == 0 && aligned16(g.s4);
+  a.scale_bytes = !aligned16(g.s4) ? 4 : (g.K % 256 == 0 ? 16 : (g.K % 128 == 0 ? 8 : 4));
   a.test_timeout = gemm_test_timeout() == 1;
   a.patience = gemm_test_timeout() == 2 ? 0 : kPatience;
   const StreamSched &sc = p.sc;

@@ -10,6 +10,7 @@ from conftest import ORDER, golden_layer_torch
 from oracle import oracle_np as onp
 from rdquant_b200 import _lib, rdquant_cuda
 from rdquant_b200.fused_gemv_pack import pack_for_fused_gemv
+from rdquant_b200.inference import FusedMixedLinear
 from rdquant_b200.synthetic import QWEN3_4B_BLOCK, fixed_splits, random_packed_layer
 
 pytestmark = pytest.mark.gpu
@@ -146,3 +147,29 @@ def test_wide_layers_of_few_rows_need_no_decoding(rows, shape, scratch):
     some = torch.arange(0, rows, 7)
     ref = onp.mixed_precision_linear(x[some].numpy(), onp.torch_layer_to_np(layer), dict(zip(ORDER, shape[:3])), k)
     assert onp.rel_err(y.cpu()[some].float().numpy(), ref) < TOL
+
+
+@pytest.mark.parametrize("shape,rows", [
+    # block scales copied 8 bytes at a time
+    ((300, 130, 20, 896), 33), ((1280, 640, 128, 2176), 100), ((1280, 640, 128, 2176), 140),
+])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_streaming_gemm_tiles(shape, rows, dtype):
+    """The streaming GEMM through the module, against 64-bit sums over the dequantised weight (test_gpu_dequant.py: bit-exact)."""
+    n4, n8, n16, k = shape
+    splits = dict(zip(ORDER, shape[:3]))
+    layer = random_packed_layer(n4, n8, n16, k, seed=k + rows)
+    gen = torch.Generator().manual_seed(rows)
+    layer["bias"] = (torch.randn(n4 + n8 + n16, generator=gen) * 0.5).half()
+    mod = FusedMixedLinear.from_layer_data(layer, splits, k, "cuda")
+    x = torch.randn(rows, k, generator=gen).to(dtype).cuda()
+    y = mod(x)
+    assert y.dtype == dtype and all(torch.equal(mod(x), y) for _ in range(3))
+    rdquant_cuda.check_gemm_status(x.device)
+    dev = {key: v.cuda() for key, v in layer.items()}
+    w = rdquant_cuda.dequantize_packed(dev, splits, k, inv_perm=dev["inv_permutation"], out_dtype=torch.float32).double()
+    ref = x.half().double() @ w.T + dev["bias"].double()
+    # the result's rounding is half an ulp of a value (2^-11, 2^-8); FP32 sums of up to 9792 products stay far below
+    err = (y.double() - ref).abs()
+    half = 2.0 ** (-11 if dtype == torch.float16 else -8)
+    assert float((err - 1.01 * half * ref.abs()).max() / ref.abs().max()) < 2e-5
