@@ -165,6 +165,8 @@ def _bind(lib: ctypes.CDLL) -> None:
     lib.rdq_linear_workspace_size.argtypes = [vp, i32, i32, ctypes.POINTER(ctypes.c_size_t)]
     lib.rdq_linear.restype = i32
     lib.rdq_linear.argtypes = [vp, vp, i32, i32, vp, vp, vp, ctypes.c_size_t, i32, vp]
+    lib.rdq_linear_uses_words.restype = i32
+    lib.rdq_linear_uses_words.argtypes = [vp, i32, i32]
     lib.rdq_linear_words.restype = i32
     lib.rdq_linear_words.argtypes = [vp, vp, i32, i32, vp, vp, vp, ctypes.c_size_t, vp, i32, vp]
     lib.rdq_stage_copy.restype = i32
@@ -200,6 +202,7 @@ EXPORTS = [
     "rdq_quantize_status",
     "rdq_linear",
     "rdq_linear_words",
+    "rdq_linear_uses_words",
     "rdq_linear_workspace_size",
     "rdq_stage_copy",
     "rdq_stage_copy_signal",

@@ -18,6 +18,11 @@
 // order: the result does not depend on timing (await_parts: those that leave, and who does their share).  A second kernel for these sums cost
 // 4-7 us per layer, and one CTA per tile adding them up to 13 us.
 //
+// Up to 64 tokens (best_plan) tiles are not cut: a tile has as many rows (8 to 128) as make all tiles cost the same bytes, and belongs
+// to one cluster of one, two or four CTAs that share its k.  A chunk is 256 k of any format then (one, two or four boxes).  The
+// CTAs of a cluster exchange FP32 sums through distributed shared memory (finish_in_cluster): each finishes a share of the tokens.
+// They run at the same time by construction, and no word in global memory is involved.
+//
 // A stage of the pipeline is one chunk: up to 128 tensor-memory columns of weights and up to four
 // 64-k activation boxes, on one barrier.  Every barrier wait of the issuing warp costs about 190 cycles
 // and every hand-over of a converter group 300 to 1000, whatever the number of tokens: with 64-k
@@ -69,7 +74,7 @@ constexpr int kThreadBound = NT == 64 ? 736 : kThreads<NT>;
 constexpr int kFinishThreads = 512;
 constexpr int kChunkBytes = 128 * 128;
 constexpr int kScaleBytes = 128 * 16;
-constexpr int kMaxRing = 8;
+constexpr int kMaxRing = 16;
 constexpr int kSmemMax = 222 * 1024;
 constexpr int kMaxTokens = 128;   // per token tile
 constexpr int kMaxCtas = RDQ_LINEAR_WORDS;
@@ -82,6 +87,8 @@ struct StreamSched {
   int S[3];                 // chunks per tile
   int E[3];                 // end of each format's chunk range
   int nkb;                  // k blocks of 64
+  int R[3];                 // rows per tile
+  int cluster;              // (whole tiles) CTAs that share a tile's k: E and bnd are tiles then, bnd of a cluster
   int G;                    // CTAs
   int bnd[kMaxCtas + 1];    // first chunk of each CTA
 };
@@ -90,6 +97,18 @@ struct Segment {
   int c0, c1;                 // chunks of the tile
   int start;                  // global index of the tile's first chunk
 };
+// the same where `S` chunks of every tile are this CTA's, numbered through
+__device__ __forceinline__ Segment whole_segment_at(const StreamSched &s, int S, int chunk) {
+  Segment g;
+  const int t = chunk / S;
+  g.fmt = t < s.E[0] ? 0 : (t < s.E[1] ? 1 : 2);
+  g.row_tile = t - (g.fmt == 0 ? 0 : s.E[g.fmt - 1]);
+  g.m_tile = 0;
+  g.start = t * S;
+  g.c0 = chunk - g.start;
+  g.c1 = S;
+  return g;
+}
 __device__ __forceinline__ Segment segment_at(const StreamSched &s, int chunk, int end) {
   Segment g;
   g.fmt = chunk < s.E[0] ? 0 : (chunk < s.E[1] ? 1 : 2);
@@ -116,6 +135,7 @@ struct StreamArgs {
   uint32_t *arrived;  // [CTA in which a cut tile starts]: its word (await_parts)
   int patience;
   int nw;             // weight chunks in flight
+  int w_pitch, s_pitch;  // bytes of a ring slot: weights, block scales
   int early;          // weights may be read before the kernel before this one has finished
   int scale_bytes;  // a block-scale row is copied 16, 8 or 4 bytes at a time
   int test_timeout;
@@ -136,6 +156,7 @@ struct StreamSmem {
   uint32_t tmem_base;
   int abort_flag;
   int left[2];  // finish_shared: what await_parts answered
+  uint64_t r_full[2][4], r_empty[2][4];  // sums from the cluster's other CTAs: [buffer][epilogue warp]
 };
 
 // position in a ring
@@ -199,6 +220,20 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
       : "r"(taddr)
       : "memory");
 }
+// ... and waits for it: the values pass through, so that no use of one moves ahead of the wait
+__device__ __forceinline__ void tmem_wait_ld16(uint32_t (&r)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
+                 "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+               :
+               : "memory");
+}
+// 16 bytes to shared memory of another CTA of the cluster, counted on a barrier there: no fence on this side
+__device__ __forceinline__ void st_async16(uint32_t addr, uint32_t bar, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%2,%3,%4,%5}, [%1];" ::"r"(addr), "r"(bar), "r"(a),
+               "r"(b), "r"(c), "r"(d)
+               : "memory");
+}
 // D (+)= A(tensor memory) . B(smem)^T.  The descriptor comes in halves: only the low one changes from
 // MMA to MMA, and every operand that changes costs the issuing warp a register move.
 __device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t db_lo, uint32_t db_hi, uint32_t idesc,
@@ -246,12 +281,13 @@ __device__ __forceinline__ void convert_fp8(const uint4 &a, const uint4 &b, uint
 }
 
 // row r of a segment's tile
-__device__ __forceinline__ Row row_of(const StreamArgs &a, const Segment &g, int r, bool wanted) {
+// (of `height` rows)
+__device__ __forceinline__ Row row_of(const StreamArgs &a, const Segment &g, int height, int r, bool wanted) {
   Row w;
-  const int row = g.row_tile * 128 + r;  // row inside the format group
+  const int row = g.row_tile * height + r;  // row inside the format group
   const int rows = g.fmt == 0 ? a.n4 : (g.fmt == 1 ? a.n8 : a.n16);
   const int prow = row + (g.fmt == 0 ? 0 : (g.fmt == 1 ? a.n4 : a.n4 + a.n8));
-  w.live = row < rows;
+  w.live = r < height && row < rows;
   w.col = 0;
   w.scl = 0.f;
   w.bia = 0.f;
@@ -318,8 +354,95 @@ __device__ __forceinline__ void finish_shared(const StreamArgs &a, const StreamS
   if (r == 0 && sub == 0) clear_parts(a.arrived + b0, passed, left, parts);
 }
 
-// NT: most tokens per tile (64 or 128)
-template <int NT, bool BF16>
+// a row's sums of up to 16 tokens from `tok` on
+template <bool BF16>
+__device__ __forceinline__ void store_tokens(const StreamSched &sc, const StreamArgs &a, const Row &row, const float (&v)[16], int tok,
+                                             int count) {
+  const int n = row.live ? min(count, sc.M - tok) : 0;
+  uint16_t *y = static_cast<uint16_t *>(a.y) + 1ll * tok * a.N + row.col;
+#pragma unroll
+  for (int e = 0; e < 16; e += 2) {
+    const uint32_t h = pack_y2(fmaf(v[e], row.scl, row.bia), fmaf(v[e + 1], row.scl, row.bia), BF16);
+    if (e < n) y[0] = static_cast<uint16_t>(h);
+    if (e + 1 < n) y[a.N] = static_cast<uint16_t>(h >> 16);
+    y += 2 * a.N;
+  }
+}
+// a tile that this CTA has alone
+template <bool BF16>
+__device__ __forceinline__ void finish_alone(const StreamSched &sc, const StreamArgs &a, const Row &row, uint32_t acc, bool dry) {
+#pragma unroll 1
+  for (int t = 0; t < sc.M; t += 16) {
+    uint32_t v[16];
+    tmem_ld16(acc + t, v);
+    tmem_wait_ld16(v);
+    float o[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) o[e] = __uint_as_float(v[e]);
+    store_tokens<BF16>(sc, a, row, o, t, dry ? 0 : 16);
+    if (dry) break;
+  }
+}
+
+// Tiles whose k the CTAs of a cluster share: epilogue warp q sends its 32 rows' sums of the tokens that another CTA
+// finishes to that CTA's warp q, waits for those of its own tokens and adds, in the order of the ranks.  `turn` counts the
+// tiles; two buffers take turns.  Layout of a buffer: [rank][four tokens][128 rows][4].
+template <bool BF16>
+__device__ __forceinline__ void finish_in_cluster(StreamSmem &S, const StreamSched &sc, const StreamArgs &a, const Row &row, uint32_t acc,
+                                                  uint32_t r_ring, int rank, int q, int lane, int turn, bool more, bool dry) {
+  const int C = sc.cluster, share = sc.nt / C;  // a multiple of four
+  const uint32_t part = share * 512;            // bytes of a rank's sums
+  const uint32_t buf = r_ring + (turn & 1) * C * part, at = (q * 32 + lane) * 16;
+  const int parity = (turn >> 1) & 1;
+  uint64_t *full = &S.r_full[turn & 1][q], *empty = &S.r_empty[turn & 1][q];
+  if (!dry && turn >= 2 && !gemm_wait_cluster(empty, parity ^ 1, &S.abort_flag)) return;
+  uint32_t v[16];
+#pragma unroll 1
+  for (int p = 1; p < C; ++p) {
+    const int to = rank + p < C ? rank + p : rank + p - C;
+    const uint32_t dst = mapa_u32(buf + rank * part + at, to), bar = mapa_u32(smem_u32(full), to);
+#pragma unroll 1
+    for (int t = 0; t < share; t += 16) {
+      tmem_ld16(acc + to * share + t, v);
+      tmem_wait_ld16(v);
+#pragma unroll
+      for (int e = 0; e < 16; e += 4)
+        if (!dry && t + e < share) st_async16(dst + (t + e) * 512, bar, v[e], v[e + 1], v[e + 2], v[e + 3]);
+    }
+  }
+  if (!dry && lane == 0) mbar_arrive_expect_tx(smem_u32(full), (C - 1) * share * 128);
+#pragma unroll 1
+  for (int t = 0; t < share; t += 16) {
+    const int tok = rank * share + t;
+    tmem_ld16(acc + tok, v);
+    tmem_wait_ld16(v);
+    if (!dry && t == 0 && !gemm_wait_cluster(full, parity, &S.abort_flag)) return;
+    float o[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) o[e] = 0.f;
+#pragma unroll 1
+    for (int p = 0; p < C; ++p) {
+#pragma unroll
+      for (int e = 0; e < 16; e += 4) {
+        uint4 w = make_uint4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+        if (p != rank && t + e < share) w = lds16(buf + p * part + (t + e) * 512 + at);
+        o[e] += __uint_as_float(w.x);
+        o[e + 1] += __uint_as_float(w.y);
+        o[e + 2] += __uint_as_float(w.z);
+        o[e + 3] += __uint_as_float(w.w);
+      }
+    }
+    // This buffer of theirs is read; ahead of the stores, whose end the release would wait for.
+    if (t + 16 >= share && more && !dry) {
+      __syncwarp();
+      if (lane < C) mbar_arrive_cluster(mapa_u32(smem_u32(empty), lane));
+    }
+    store_tokens<BF16>(sc, a, row, o, tok, dry ? 0 : min(16, share - t));
+  }
+}
+
+// NT: most tokens per tile (64 or 128).  WHOLE: every tile belongs to one CTA, a chunk has 256 k of any format (make_whole_plan)
+template <int NT, bool BF16, bool WHOLE>
 __global__ void __launch_bounds__(kThreadBound<NT>, 1)
 gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_constant__ CUtensorMap w8map,
                    const __grid_constant__ CUtensorMap w16map, const __grid_constant__ CUtensorMap xmap,
@@ -328,18 +451,35 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
   extern __shared__ uint8_t smem_raw[];
   __shared__ StreamSmem S;
   const uint32_t w_ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t x_ring = w_ring + a.nw * kChunkBytes;
+  // (tiles of 128 rows: constants)
+  const uint32_t w_pitch = WHOLE ? a.w_pitch : kChunkBytes, s_pitch = WHOLE ? a.s_pitch : kScaleBytes;
+  const uint32_t x_ring = w_ring + a.nw * w_pitch;
   const uint32_t x_bytes = static_cast<uint32_t>(sc.nt) * 128;  // one 64-k box
   const uint32_t s_ring = x_ring + NS * KB * x_bytes;
+  const uint32_t r_ring = x_ring + NS * KB * x_bytes + a.nw * s_pitch + 512;
   // (from lane 0, so that the compiler keeps the roles' branches and loops in uniform registers)
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  const int begin = sc.bnd[blockIdx.x], end = sc.bnd[blockIdx.x + 1];
+  // WHOLE: this CTA has the chunks lo .. lo + own - 1 of its cluster's tiles
+  const uint32_t rank = WHOLE && sc.cluster > 1 ? cluster_ctarank() : 0u;
+  const int worker = WHOLE ? static_cast<int>(blockIdx.x) / sc.cluster : static_cast<int>(blockIdx.x);
+  const int lo = WHOLE ? sc.S[0] * static_cast<int>(rank) / sc.cluster : 0;
+  const int own = WHOLE ? sc.S[0] * static_cast<int>(rank + 1) / sc.cluster - lo : 0;
+  const int begin = sc.bnd[worker] * (WHOLE ? own : 1), end = sc.bnd[worker + 1] * (WHOLE ? own : 1);
+  auto seg_at = [&](int chunk, int to) { return WHOLE ? whole_segment_at(sc, own, chunk) : segment_at(sc, chunk, to); };
   auto wmap = [&](int fmt) { return fmt == 0 ? &w4map : (fmt == 1 ? &w8map : &w16map); };
+  // the boxes of a chunk: one of 128 rows, or as many as 256 k take (those past K are left out)
+  auto height_of = [&](int fmt) { return WHOLE ? sc.R[fmt] : 128; };
+  auto boxes_of = [&](const Segment &g, int c) { return WHOLE ? min(1 << g.fmt, (sc.nkb - 4 * (lo + c) + (3 >> g.fmt)) >> (2 - g.fmt)) : 1; };
+  auto box_x = [&](const Segment &g, int c, int j) { return ((WHOLE ? (lo + c) << g.fmt : c) + j) * (g.fmt == 2 ? 64 : 128); };
   auto load_chunk = [&](const Segment &g, int c, int slot) {
     const uint32_t bar = smem_u32(&S.w_full[slot]);
-    mbar_arrive_expect_tx(bar, kChunkBytes);
-    tma_load_2d(w_ring + slot * kChunkBytes, wmap(g.fmt), c * (g.fmt == 2 ? 64 : 128), g.row_tile * 128, bar);
+    const uint32_t box = height_of(g.fmt) * 128;
+    const int boxes = boxes_of(g, c);
+    mbar_arrive_expect_tx(bar, boxes * box);
+    for (int j = 0; j < boxes; ++j)
+      tma_load_2d(w_ring + slot * w_pitch + j * box, wmap(g.fmt), box_x(g, c, j), g.row_tile * height_of(g.fmt), bar);
   };
+  auto blocks_of = [](int fmt) { return WHOLE ? 4 : 4 >> fmt; };  // k blocks of a chunk
   // The first weight chunks are on their way before anything else is set up; without leave to read weights
   // early, on their way into L2.
   const int ahead = min(a.nw, end - begin), early = a.early ? ahead : 0;
@@ -349,11 +489,14 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
       mbar_init(smem_u32(&S.w_empty[i]), 16 / KB);  // the groups that convert a chunk of four k blocks
     }
     mbar_init_fence();
-    Segment g = segment_at(sc, begin, end);
+    Segment g = seg_at(begin, end);
     for (int i = 0; i < ahead; ++i) {
-      if (begin + i == g.start + g.c1) g = segment_at(sc, begin + i, end);
-      if (a.early) load_chunk(g, begin + i - g.start, i);
-      else tma_prefetch_2d(wmap(g.fmt), (begin + i - g.start) * (g.fmt == 2 ? 64 : 128), g.row_tile * 128);
+      if (begin + i == g.start + g.c1) g = seg_at(begin + i, end);
+      const int c = begin + i - g.start;
+      if (a.early) load_chunk(g, c, i);
+      else tma_prefetch_2d(wmap(g.fmt), box_x(g, c, 0), g.row_tile * height_of(g.fmt));
+      for (int j = 1; WHOLE && !a.early && j < boxes_of(g, c); ++j)
+        tma_prefetch_2d(wmap(g.fmt), box_x(g, c, j), g.row_tile * height_of(g.fmt));
     }
   }
   if (threadIdx.x == 32) {
@@ -365,6 +508,12 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
       mbar_init(smem_u32(&S.d_full[i]), 1);
       mbar_init(smem_u32(&S.d_empty[i]), 4);
     }
+    if (WHOLE) {
+      for (int i = 0; i < 8; ++i) {
+        mbar_init(smem_u32(&S.r_full[i >> 2][i & 3]), 1);
+        mbar_init(smem_u32(&S.r_empty[i >> 2][i & 3]), sc.cluster);
+      }
+    }
     mbar_init(smem_u32(&S.never), 1);
     S.abort_flag = 0;
     mbar_init_fence();
@@ -373,13 +522,14 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
   if (warp == 3 && lane == 0) prefetch_tensormap(&xmap);
   tc_fence_before();
   __syncthreads();
+  if (WHOLE && sc.cluster > 1) cluster_arrive();  // (waited for ahead of the first word to another CTA)
   tc_fence_after();
   const uint32_t tmem = S.tmem_base;
   const uint32_t tmem_a = tmem + 2 * NT;
 
   // stages of a range: its NVFP4 chunks (they come first) take several each above 64 tokens
   constexpr int split = 4 / KB;
-  const int n4 = max(0, min(end, sc.E[0]) - begin);
+  const int n4 = WHOLE ? 0 : max(0, min(end, sc.E[0]) - begin);
   const int stages = split * n4 + (end - begin - n4);
 
   if (warp == 0) {
@@ -389,9 +539,9 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
     Cursor w;
     if (early == a.nw) w.ph ^= 1;
     else w.i = early;
-    Segment g = segment_at(sc, begin, end);
+    Segment g = seg_at(begin, end);
     for (int i = begin + early; i < end; ++i) {
-      if (i >= g.start + g.c1) g = segment_at(sc, i, end);
+      if (i >= g.start + g.c1) g = seg_at(i, end);
       if (!gemm_wait(&S.w_empty[w.i], w.ph ^ 1, &S.abort_flag)) break;
       if (leader) load_chunk(g, i - g.start, w.i);
       w.next(a.nw);
@@ -402,11 +552,11 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
     pdl_wait();
     pdl_launch_dependents();
     Cursor x;
-    Segment g = segment_at(sc, begin, end);
+    Segment g = seg_at(begin, end);
     for (int i = begin; i < end; ++i) {
-      if (i >= g.start + g.c1) g = segment_at(sc, i, end);
-      const int per = 4 >> g.fmt;  // k blocks of 64 per chunk
-      const int kb0 = (i - g.start) * per, blocks = min(per, sc.nkb - kb0);
+      if (i >= g.start + g.c1) g = seg_at(i, end);
+      const int per = blocks_of(g.fmt);  // k blocks of 64 per chunk
+      const int kb0 = (lo + i - g.start) * per, blocks = min(per, sc.nkb - kb0);
       bool ok = true;
       for (int b = 0; b < per && ok; b += KB) {  // stages of the chunk; past K a stage can be empty
         ok = gemm_wait(&S.empty[x.i], x.ph ^ 1, &S.abort_flag);
@@ -439,13 +589,13 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
     uint32_t ok = NT > 64 ? wait_bounded(full0, 0) : 1u;
     tc_fence_after();
     for (int ck = begin; ck < end && ok;) {
-      const Segment g = segment_at(sc, ck, end);
-      const int per = 4 >> g.fmt;
+      const Segment g = seg_at(ck, end);
+      const int per = blocks_of(g.fmt);
       if (!gemm_wait(&S.d_empty[d.i], d.ph ^ 1, &S.abort_flag)) break;
       tc_fence_after();
       const uint32_t acc = tmem + d.i * NT;
       const int bps = min(per, KB);                                    // k blocks of a stage
-      const int blocks = min(g.c1 * per, sc.nkb) - g.c0 * per;
+      const int blocks = min((lo + g.c1) * per, sc.nkb) - (lo + g.c0) * per;
       const int whole = blocks / bps, rest = blocks - whole * bps;     // stages with all of them
       const int none = (g.c1 - g.c0) * (per / bps) - whole - (rest > 0);  // stages past K
       uint32_t accumulate = 0;
@@ -500,17 +650,18 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
     Segment g;
     g.start = g.c1 = 0;
     const uint8_t *src[4];
-    int rows = 0;
+    int rows = 0;  // of this lane
     for (int i = begin; i < end; ++i) {
       if (i == begin || i >= g.start + g.c1) {
-        g = segment_at(sc, i, end);
-        rows = g.fmt != 0 ? 0 : 4;
+        g = seg_at(i, end);
+        const int height = height_of(0);
+        rows = g.fmt != 0 ? 0 : (height - lane + 31) / 32;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) src[u] = a.s4 + 1ll * min(g.row_tile * 128 + u * 32 + lane, a.n4 - 1) * pitch;
+        for (int u = 0; u < 4; ++u) src[u] = a.s4 + 1ll * min(g.row_tile * height + u * 32 + lane, a.n4 - 1) * pitch;
       }
       if (!gemm_wait(&S.w_empty[w.i], w.ph ^ 1, &S.abort_flag)) break;
-      const int c = i - g.start;
-      const uint32_t dst = s_ring + w.i * kScaleBytes + lane * 16;
+      const int c = lo + i - g.start;
+      const uint32_t dst = s_ring + w.i * s_pitch + lane * 16;
       if (a.scale_bytes == 16) {
 #pragma unroll
         for (int u = 0; u < 4; ++u)
@@ -535,23 +686,47 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
     const uint32_t lanes = static_cast<uint32_t>(q * 32) << 16;
     if (!a.early) pdl_wait();
     // constants of the rows that are finished together with other CTAs: fetched now, when nobody waits
-    S.cut[0][q * 32 + lane] = row_of(a, segment_at(sc, begin, end), q * 32 + lane, true);
-    S.cut[1][q * 32 + lane] = row_of(a, segment_at(sc, end - 1, end), q * 32 + lane, true);
+    if (!WHOLE) S.cut[0][q * 32 + lane] = row_of(a, seg_at(begin, end), 128, q * 32 + lane, true);
+    if (!WHOLE) S.cut[1][q * 32 + lane] = row_of(a, seg_at(end - 1, end), 128, q * 32 + lane, true);
     Cursor d;
     bool first = true;
+    int turn = 0;
+    if (WHOLE && sc.cluster > 1) cluster_wait();
+    // (whole tiles) The first turn of the loop, while nothing is there to be stored, runs through without a wait, a store or
+    // an arrival: it brings the code into the instruction caches, 2000 cycles that would be spent behind the last MMA.
+    bool dry = WHOLE;
     for (int ck = begin; ck < end;) {
-      const Segment g = segment_at(sc, ck, end);
-      const bool whole = g.c0 == 0 && g.c1 == sc.S[g.fmt];
-      const Row row = row_of(a, g, q * 32 + lane, whole);
+      const Segment g = seg_at(ck, end);
+      const bool whole = WHOLE || (g.c0 == 0 && g.c1 == sc.S[g.fmt]);
+      const Row row = row_of(a, g, height_of(g.fmt), q * 32 + lane, whole);
       const int tok0 = g.m_tile * sc.nt;
       const int ntok = min(sc.nt, sc.M - tok0);
-      if (!gemm_wait(&S.d_full[d.i], d.ph, &S.abort_flag)) break;
-      tc_fence_after();
+      if (!(WHOLE && dry)) {
+        if (!gemm_wait(&S.d_full[d.i], d.ph, &S.abort_flag)) break;
+        tc_fence_after();
+      }
       const uint32_t acc = tmem + d.i * NT + lanes;
       float *part = a.partial + (2ll * blockIdx.x + (first ? 0 : 1)) * sc.nt * 128 + q * 32 + lane;
       uint16_t *yp = static_cast<uint16_t *>(a.y) + 1ll * tok0 * a.N + row.col;
       // sixteen tokens at a time; the stores of one batch overlap the load of the next
       uint32_t v[2][16];
+      if (WHOLE) {
+        if (q * 32 < sc.R[g.fmt]) {  // (else no rows)
+          if (sc.cluster > 1) finish_in_cluster<BF16>(S, sc, a, row, acc, r_ring, static_cast<int>(rank), q, lane, turn, ck + 2 * own < end, dry);
+          else finish_alone<BF16>(sc, a, row, acc, dry);
+        }
+        if (dry) {
+          dry = false;
+          continue;
+        }
+        ++turn;
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&S.d_empty[d.i]));
+        d.next(2);
+        ck = g.start + g.c1;
+        continue;
+      }
       tmem_ld16(acc, v[0]);
       auto batch = [&](uint32_t (&cur)[16], uint32_t (&nxt)[16], int c) {
         tmem_wait_ld();
@@ -621,16 +796,40 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
         slot -= a.nw;
         w_ph ^= 1;
       }
-      if (j == grp || i >= g.start + g.c1) g = segment_at(sc, i, end);
+      if (j == grp || i >= g.start + g.c1) g = seg_at(i, end);
       if (!gemm_wait(&S.empty[grp], ph ^ 1, &S.abort_flag)) break;
       if (!gemm_wait(&S.w_full[slot], w_ph, &S.abort_flag)) break;
       tc_fence_after();
-      const uint32_t base = w_ring + slot * kChunkBytes + rbase;
+      const uint32_t base = w_ring + slot * w_pitch + rbase;
       auto piece = [&](int p) { return lds16(base + ((p ^ sw) << 4)); };
       uint32_t o[16];
-      if (g.fmt == 0) {
+      if (WHOLE && q * 32 >= sc.R[g.fmt]) {
+        // no rows: the MMAs read whatever these lanes hold, for sums that nobody reads
+      } else if (WHOLE && g.fmt > 0) {
+        const uint32_t box = sc.R[g.fmt] * 128;
+        const int halves = 2 * min(4, sc.nkb - 4 * (lo + i - g.start));
+#pragma unroll
+        for (int h = 0; h < 8; ++h) {  // 32 k at a time: of a box of 128 or 64 k
+          if (h >= halves) break;
+          const uint32_t at = base + (g.fmt == 1 ? h >> 2 : h >> 1) * box;
+          auto part = [&](int p) { return lds16(at + ((p ^ sw) << 4)); };
+          if (g.fmt == 1) {
+            convert_fp8(part(2 * (h & 3)), part(2 * (h & 3) + 1), o);
+          } else {
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+              const uint4 v = part(4 * (h & 1) + p);
+              o[4 * p] = v.x;
+              o[4 * p + 1] = v.y;
+              o[4 * p + 2] = v.z;
+              o[4 * p + 3] = v.w;
+            }
+          }
+          tmem_st16(dst + 16 * h, o);
+        }
+      } else if (g.fmt == 0) {
         // (k blocks beyond K convert the zero fill of the box; the MMAs do not read them)
-        const uint4 s4 = lds16(s_ring + slot * kScaleBytes + row * 16);
+        const uint4 s4 = lds16(s_ring + slot * s_pitch + row * 16);
         const uint32_t sc4[4] = {part ? s4.z : s4.x, part ? s4.w : s4.y, s4.z, s4.w};
         // Four pieces are read ahead of their conversion: one after the other, each waited for its own read.
         uint4 v[4] = {piece(2 * KB * part), piece(2 * KB * part + 1), piece(2 * KB * part + 2), piece(2 * KB * part + 3)};
@@ -677,23 +876,26 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
   }
 
   __syncwarp();
+  if (WHOLE && sc.cluster > 1 && (warp < 4 || warp >= 8)) cluster_wait();  // (the epilogue's warps have)
   tc_fence_before();
   __syncthreads();
+  if (WHOLE && sc.cluster > 1) cluster_arrive_relaxed();  // nobody leaves while another CTA may write to it
   if (warp == 2) tmem_dealloc(tmem, 512);
   // ---- tiles shared with other CTAs: half of 512 threads take the range's first segment, half its last
-  if (!S.abort_flag && begin < end && threadIdx.x < kFinishThreads) {
+  if (!WHOLE && !S.abort_flag && begin < end && threadIdx.x < kFinishThreads) {
     const int half = threadIdx.x >> 8;
-    Segment g = segment_at(sc, begin, end);
+    Segment g = seg_at(begin, end);
     bool mine = half == 0;
     if (half == 1 && g.start + g.c1 < end) {
       mine = true;
-      g = segment_at(sc, end - 1, end);
-      g = segment_at(sc, max(g.start, begin), end);
+      g = seg_at(end - 1, end);
+      g = seg_at(max(g.start, begin), end);
     }
-    if (mine && !(g.c0 == 0 && g.c1 == sc.S[g.fmt]))
+    if (!WHOLE && mine && !(g.c0 == 0 && g.c1 == sc.S[g.fmt]))
       finish_shared<BF16, NT == 64 ? 4 : 2, NT == 64 ? 8 : 16>(a, sc, g, S.cut[half][threadIdx.x & 127], threadIdx.x & 127, (threadIdx.x >> 7) & 1, 1 + half, &S.left[half]);
   }
-  __syncthreads();
+  if (!WHOLE) __syncthreads();
+  if (WHOLE && sc.cluster > 1) cluster_wait();
   if (S.abort_flag) {
     linger(16000);  // let copies that are still in flight land before the shared memory is given up
     __syncthreads();
@@ -707,6 +909,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
 struct StreamPlan {
   StreamSched sc;
   int wide, nw, smem;  // wide: the variant for more than 64 tokens per tile
+  int whole, w_pitch, s_pitch;
 };
 
 // Token tiles of equal width; a chunk costs what bounds it: its bytes at the SM's share of the HBM
@@ -726,6 +929,7 @@ StreamPlan make_plan(int n4, int n8, int n16, int M, int K) {
   for (int f = 0; f < 3; ++f) {
     const int per = 4 >> f;
     s.S[f] = (s.nkb + per - 1) / per;
+    s.R[f] = 128;
     // (measured on 128 x 128 tiles: 1540 / 825 / 581 cycles per NVFP4 / FP8 / FP16 chunk)
     const int bps = std::min(per, kBlocks<128>);
     const double conv = f == 0 ? 170 : (f == 1 ? 150 : 90);
@@ -753,8 +957,122 @@ StreamPlan make_plan(int n4, int n8, int n16, int M, int K) {
   p.wide = s.nt > 64;
   const int xb = (p.wide ? kStages<128> * kBlocks<128> : kStages<64> * kBlocks<64>) * s.nt * 128;
   p.nw = std::min(kMaxRing, (kSmemMax - 1024 - xb) / (kChunkBytes + kScaleBytes));
+  p.nw = std::min(p.nw, 8);
   p.smem = 1024 + xb + p.nw * (kChunkBytes + kScaleBytes);
+  p.whole = 0;
+  s.cluster = 1;
+  p.w_pitch = kChunkBytes;
+  p.s_pitch = kScaleBytes;
   return p;
+}
+
+// clusters of that many CTAs (1, 2, 4) that run at the same time: fewer than the SMs would make where an SM of a group
+// is left over; 0 when the device cannot say
+int clusters_at_once(int size) {
+  const int sms = std::min(sm_count(), kMaxCtas);
+  if (size == 1) return sms;
+  static std::atomic<int> cached[64][2];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  std::atomic<int> &known = cached[dev][size / 4];
+  if (known.load() == 0) {
+    const void *fn = reinterpret_cast<const void *>(gemm_stream_kernel<64, false, true>);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = static_cast<unsigned>(size);
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(sms / size * size));
+    cfg.blockDim = dim3(kThreads<64>);
+    cfg.dynamicSmemBytes = kSmemMax;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, fn, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    known.store(n > 0 ? std::min(n, sms / size) : -1);
+  }
+  return std::max(0, known.load());
+}
+
+// Whole tiles: each belongs to one cluster alone, whose CTAs share its k, so that nothing is put together through global
+// memory.  Rows per tile by the bytes of a row, so that all tiles cost the same; `us`: an estimate of the launch's time.
+bool make_whole_plan(int n4, int n8, int n16, int M, int K, int cluster, StreamPlan *out, double *us) {
+  const int workers = clusters_at_once(cluster);
+  if (M > 64 || workers == 0 || (K + 255) / 256 < cluster) return false;
+  StreamPlan p;
+  StreamSched &s = p.sc;
+  s.M = M;
+  s.mt = 1;
+  s.nt = (M + 15) / 16 * 16;
+  s.nkb = (K + 63) / 64;
+  s.cluster = cluster;
+  const int n[3] = {n4, n8, n16};
+  const double bytes[3] = {0.5625, 1.0, 2.0};
+  int least = 0;
+  for (int f = 0; f < 3; ++f) least += (n[f] + 127) / 128;
+  const int most = std::max(1, (least + workers - 1) / workers);  // tiles of a cluster
+  int tiles = 0;
+  for (double t = 4.5;; t += 0.5) {
+    tiles = 0;
+    for (int f = 0; f < 3; ++f) {
+      s.R[f] = std::max(8, std::min(128, static_cast<int>(t / bytes[f] / 8) * 8));
+      tiles += (n[f] + s.R[f] - 1) / s.R[f];
+    }
+    if (tiles <= most * workers) break;  // (holds at the latest where all tiles have 128 rows)
+  }
+  int e = 0;
+  double heaviest = 0;
+  for (int f = 0; f < 3; ++f) {
+    s.S[f] = (s.nkb + 3) / 4;
+    e += (n[f] + s.R[f] - 1) / s.R[f];
+    s.E[f] = e;
+    if (n[f]) heaviest = std::max(heaviest, s.R[f] * bytes[f]);
+  }
+  s.G = std::min(workers, tiles);
+  for (int b = 0; b <= s.G; ++b) s.bnd[b] = static_cast<int>(1ll * tiles * b / s.G);
+  const int each = (tiles + s.G - 1) / s.G;
+  p.wide = 0;
+  p.whole = 1;
+  p.w_pitch = std::max({n4 ? s.R[0] : 0, n8 ? 2 * s.R[1] : 0, n16 ? 4 * s.R[2] : 0}) * 128;
+  p.s_pitch = s.R[0] * 16;
+  const int xb = kStages<64> * kBlocks<64> * s.nt * 128 + (cluster > 1 ? std::min(2, each) * s.nt * 512 : 0);
+  // (a warp reads the rows of all its lanes: 512 bytes behind the last slot's block scales)
+  p.nw = std::min(kMaxRing, (kSmemMax - 1024 - 512 - xb) / (p.w_pitch + p.s_pitch));
+  if (p.nw < (each > 1 ? kStages<64> + 1 : kStages<64>)) return false;
+  p.smem = 1024 + 512 + xb + p.nw * (p.w_pitch + p.s_pitch);
+  // Fitted to calls one after another on 40 layers (0.4 to 350 MB, K 1024 to 16384, 9 to 64 rows): the faster of the
+  // clusters is picked but for 0.5 % on average, 9 % at worst.
+  const double steps = each * ((s.S[0] + cluster - 1) / cluster) * (0.181 + 0.0035 * s.nt);
+  const double memory = heaviest * K / cluster * each / 43e3 * 0.484;
+  *us = 4.9 + std::max(steps, memory) + 1.35 * std::min(steps, memory) + (cluster > 1 ? 1.2 : 0.0) + (cluster > 2 ? 0.25 : 0.0);
+  *out = p;
+  return true;
+}
+
+// Up to 64 tokens tiles are whole: the CTAs that share a cut one spend 7000 cycles behind the last MMA (partial sums, fence,
+// arrival, sums, each a round trip to L2 by code that is run once), a cluster 1700 and a CTA alone 1000.  32 rows, calls
+// one after another, us before and now: 2560 -> 6144 10.6, 8.3; 4096 -> 2560 10.6, 7.7; 9728 -> 2560 12.5, 10.6; 1024 -> 1024 8.0,
+// 6.0; 8192 -> 8192 15.5, 13.7.  Above 200 MB the tail is short beside the rest and cut tiles use the MMA's 128 rows better (8192 ->
+// 57344 at 48 rows 73.6, 76.2) unless there are few tokens (9 rows 61.1, 58.4).
+StreamPlan best_plan(int n4, int n8, int n16, int M, int K) {
+  StreamPlan best = {};
+  bool found = false;
+  if (M <= 64 && (n4 * 0.5625 + n8 + 2.0 * n16) * K < 150e6) {
+    double least = 0;
+    for (int cluster = 1; cluster <= 4; cluster *= 2) {
+      StreamPlan p;
+      double us = 0;
+      if (!make_whole_plan(n4, n8, n16, M, K, cluster, &p, &us) || (found && us >= least)) continue;
+      best = p;
+      least = us;
+      found = true;
+    }
+  }
+  return found ? best : make_plan(n4, n8, n16, M, K);
 }
 
 // the plans of the last few thousand (layer shape, rows) pairs of this thread
@@ -775,13 +1093,13 @@ const StreamPlan &stream_plan(int n4, int n8, int n16, int M, int K) {
   auto it = plans.find(key);
   if (it == plans.end()) {
     if (plans.size() >= 4096) plans.clear();
-    it = plans.emplace(key, make_plan(n4, n8, n16, M, K)).first;
+    it = plans.emplace(key, best_plan(n4, n8, n16, M, K)).first;
   }
   return it->second;
 }
 
-int encode_u8_2d(CUtensorMap *map, const void *base, int cols, int rows) {
-  return encode_2d(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, base, cols, rows, 128, 128);
+int encode_u8_2d(CUtensorMap *map, const void *base, int cols, int rows, int box_rows) {
+  return encode_2d(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, base, cols, rows, 128, box_rows);
 }
 
 }  // namespace
@@ -789,15 +1107,16 @@ int encode_u8_2d(CUtensorMap *map, const void *base, int cols, int rows) {
 // 16-byte row pitches for TMA, whole 4-byte groups of block scales
 bool gemm_stream_takes(int K) { return K % 64 == 0; }
 
-size_t gemm_stream_workspace(int M, int K) {
-  (void)K;
-  const int mt = (M + kMaxTokens - 1) / kMaxTokens, nt = ((M + mt - 1) / mt + 15) / 16 * 16;
-  return 2ull * std::min(sm_count(), kMaxCtas) * nt * 128 * sizeof(float);
+// Partial sums of cut tiles.  Whole tiles have none; not 0 all the same, by which callers tell a decode kernel.
+size_t gemm_stream_workspace(int n4, int n8, int n16, int M, int K) {
+  const StreamPlan &p = stream_plan(n4, n8, n16, M, K);
+  return p.whole ? 256 : 2ull * p.sc.G * p.sc.nt * 128 * sizeof(float);
 }
+bool gemm_stream_uses_words(int n4, int n8, int n16, int M, int K) { return !stream_plan(n4, n8, n16, M, K).whole; }
 
 int launch_gemm_stream(const GemmArgs &g, void *workspace, size_t workspace_bytes, bool pdl, cudaStream_t stream) {
   const StreamPlan &p = stream_plan(g.n4, g.n8, g.n16, g.M, g.K);
-  RDQ_REQUIRE(workspace && workspace_bytes >= 2ull * p.sc.G * p.sc.nt * 128 * sizeof(float), RDQ_E_INVALID,
+  RDQ_REQUIRE(p.whole || (workspace && g.counters && workspace_bytes >= 2ull * p.sc.G * p.sc.nt * 128 * sizeof(float)), RDQ_E_INVALID,
               "GEMM workspace too small");
   int *status = nullptr;
   int rc = gemm_status_ptr(&status);
@@ -806,9 +1125,9 @@ int launch_gemm_stream(const GemmArgs &g, void *workspace, size_t workspace_byte
   rc = encode_f16_2d(&xmap, g.x, g.K, g.M, 64, p.sc.nt);
   if (rc != RDQ_OK) return rc;
   w4map = w8map = w16map = xmap;  // maps of absent groups are never used
-  if (g.n4 && (rc = encode_u8_2d(&w4map, g.w4, g.K / 2, g.n4)) != RDQ_OK) return rc;
-  if (g.n8 && (rc = encode_u8_2d(&w8map, g.w8, g.K, g.n8)) != RDQ_OK) return rc;
-  if (g.n16 && (rc = encode_f16_2d(&w16map, g.w16, g.K, g.n16, 64, 128)) != RDQ_OK) return rc;
+  if (g.n4 && (rc = encode_u8_2d(&w4map, g.w4, g.K / 2, g.n4, p.sc.R[0])) != RDQ_OK) return rc;
+  if (g.n8 && (rc = encode_u8_2d(&w8map, g.w8, g.K, g.n8, p.sc.R[1])) != RDQ_OK) return rc;
+  if (g.n16 && (rc = encode_f16_2d(&w16map, g.w16, g.K, g.n16, 64, p.sc.R[2])) != RDQ_OK) return rc;
   StreamArgs a;
   a.s4 = g.s4;
   a.s8 = g.s8;
@@ -824,18 +1143,21 @@ int launch_gemm_stream(const GemmArgs &g, void *workspace, size_t workspace_byte
   a.partial = static_cast<float *>(workspace);
   a.arrived = reinterpret_cast<uint32_t *>(g.counters);
   a.nw = p.nw;
+  a.w_pitch = p.w_pitch;
+  a.s_pitch = p.s_pitch;
   a.early = pdl;
   a.scale_bytes = !aligned16(g.s4) ? 4 : (g.K % 256 == 0 ? 16 : (g.K % 128 == 0 ? 8 : 4));
   a.test_timeout = gemm_test_timeout() == 1;
   a.patience = gemm_test_timeout() == 2 ? 0 : kPatience;
   const StreamSched &sc = p.sc;
 
-  static const void *const fns[4] = {
-      reinterpret_cast<const void *>(gemm_stream_kernel<64, false>), reinterpret_cast<const void *>(gemm_stream_kernel<64, true>),
-      reinterpret_cast<const void *>(gemm_stream_kernel<128, false>), reinterpret_cast<const void *>(gemm_stream_kernel<128, true>)};
-  const int variant = p.wide * 2 + (g.y_bf16 ? 1 : 0);
+  static const void *const fns[6] = {
+      reinterpret_cast<const void *>(gemm_stream_kernel<64, false, false>), reinterpret_cast<const void *>(gemm_stream_kernel<64, true, false>),
+      reinterpret_cast<const void *>(gemm_stream_kernel<128, false, false>), reinterpret_cast<const void *>(gemm_stream_kernel<128, true, false>),
+      reinterpret_cast<const void *>(gemm_stream_kernel<64, false, true>), reinterpret_cast<const void *>(gemm_stream_kernel<64, true, true>)};
+  const int variant = (p.whole ? 4 : p.wide * 2) + (g.y_bf16 ? 1 : 0);
   const void *fn = fns[variant];
-  static std::atomic<bool> attr_done[4][64];
+  static std::atomic<bool> attr_done[6][64];
   int dev = 0;
   RDQ_CUDA(cudaGetDevice(&dev));
   std::atomic<bool> *done = dev >= 0 && dev < 64 ? &attr_done[variant][dev] : nullptr;
@@ -843,16 +1165,19 @@ int launch_gemm_stream(const GemmArgs &g, void *workspace, size_t workspace_byte
     RDQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
     if (done) done->store(true);
   }
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(sc.cluster);
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(sc.G));
+  cfg.gridDim = dim3(static_cast<unsigned>(sc.G * sc.cluster));
   cfg.blockDim = dim3(p.wide ? kThreads<128> : kThreads<64>);
   cfg.dynamicSmemBytes = p.smem;
   cfg.stream = stream;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = sc.cluster > 1 ? 2 : 1;
   void *params[7] = {&w4map, &w8map, &w16map, &xmap, &a, const_cast<StreamSched *>(&sc), &status};
   RDQ_CUDA(cudaLaunchKernelExC(&cfg, fn, params));
   return RDQ_OK;

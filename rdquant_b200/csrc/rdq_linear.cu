@@ -101,9 +101,13 @@ struct Need {
 Need need_of(const rdq_layer &l, Path p, int M, int x_type) {
   Need n;
   if (x_type == RDQ_BF16 && !takes_bf16(l, p, M)) n.cast = align256(2ull * M * l.K);
-  if (p == Path::kStream) n.gemm = gemm_stream_workspace(M, l.K);
+  if (p == Path::kStream) n.gemm = gemm_stream_workspace(l.n_fp4, l.n_fp8, l.n_fp16, M, l.K);
   if (p == Path::kGemm) n.gemm = gemm_workspace_bytes(M, l.n_fp4 + l.n_fp8 + l.n_fp16, l.K);
   return n;
+}
+
+bool uses_words(const rdq_layer &l, Path p, int M) {
+  return p == Path::kStream && gemm_stream_uses_words(l.n_fp4, l.n_fp8, l.n_fp16, M, l.K);
 }
 
 int run_gemv(const rdq_layer &l, bool tiled, const void *x, int x_bf16, int M, const void *bias, void *y, int y_bf16, bool pdl,
@@ -213,6 +217,13 @@ int rdq_linear_workspace_size(const rdq_layer *layer, int M, int x_type, size_t 
   return RDQ_OK;
 }
 
+int rdq_linear_uses_words(const rdq_layer *layer, int M, int x_type) {
+  if (!layer || M <= 0 || (x_type != RDQ_F16 && x_type != RDQ_BF16) || check_layouts(*layer) != RDQ_OK ||
+      layer->n_fp4 + layer->n_fp8 + layer->n_fp16 == 0)
+    return 0;
+  return uses_words(*layer, path_of(*layer, M, x_type), M) ? 1 : 0;
+}
+
 int rdq_linear(const rdq_layer *layer, const void *x, int x_type, int M, const void *bias, void *y, void *workspace,
                size_t workspace_bytes, int flags, void *stream) {
   return rdq_linear_words(layer, x, x_type, M, bias, y, workspace, workspace_bytes, layer ? layer->gemv_counters : nullptr,
@@ -237,7 +248,7 @@ int rdq_linear_words(const rdq_layer *layer, const void *x, int x_type, int M, c
   const int bf16 = x_type == RDQ_BF16 ? 1 : 0;
   bool pdl = (flags & RDQ_GEMV_PDL) != 0;
   if (words && (flags & RDQ_LINEAR_FRESH)) RDQ_CUDA(cudaMemsetAsync(words, 0, RDQ_LINEAR_WORDS * sizeof(int32_t), stream));
-  RDQ_REQUIRE(words || p != Path::kStream, RDQ_E_INVALID, "words must not be null");
+  RDQ_REQUIRE(words || !uses_words(l, p, M), RDQ_E_INVALID, "words must not be null");
   const void *xh = x;
   int x_bf16 = bf16;
   // (the decoded-once GEMM's first launch rounds the rows itself)

@@ -260,10 +260,10 @@ PyObject *layer_linear(PyObject *obj, PyObject *const *args, Py_ssize_t nargs) {
         }
       }
       const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream(self->device);
-      // (without a workspace it is a decode kernel, which needs no words)
+      // (without a workspace it is a decode kernel, and a GEMM of whole tiles counts nothing either)
       int32_t *words = nullptr;
       bool fresh = false;
-      if (need) words = words_of(self->device, stream, &fresh);
+      if (need && rdq_linear_uses_words(&l, static_cast<int>(m), xt)) words = words_of(self->device, stream, &fresh);
       rc = rdq_linear_words(&l, xp, xt, static_cast<int>(m), bias, y.data_ptr(), need ? ws.data_ptr() : nullptr, need, words,
                             static_cast<int>(flags) | (fresh ? RDQ_LINEAR_FRESH : 0), stream.stream());
       if (fresh && rc != RDQ_OK) word_sets->pop_back();  // perhaps not zeroed

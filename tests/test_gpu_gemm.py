@@ -150,7 +150,14 @@ def test_wide_layers_of_few_rows_need_no_decoding(rows, shape, scratch):
 
 
 @pytest.mark.parametrize("shape,rows", [
-    # block scales copied 8 bytes at a time
+    # whole tiles, a CTA each: K of less than a chunk, of no whole chunk, groups that end inside a tile
+    ((64, 32, 16, 64), 17), ((0, 0, 128, 192), 9), ((300, 130, 20, 576), 33), ((37, 0, 5, 1344), 24),
+    ((60800, 20480, 5120, 256), 20),     # five tiles each
+    # clusters of two and four: chunks of k dealt out unevenly, several tiles each (buffers used again)
+    ((4096, 2048, 0, 4096), 64), ((13056, 6144, 256, 2560), 20), ((13056, 6144, 256, 2624), 64),
+    ((2048, 384, 128, 2560), 20), ((640, 384, 0, 9792), 31), ((0, 0, 256, 8192), 40), ((0, 700, 0, 3008), 48),
+    ((30000, 4000, 0, 8192), 33),        # 170 MB: cut tiles
+    # block scales copied 8 bytes at a time: whole tiles, cut ones, two tiles of tokens
     ((300, 130, 20, 896), 33), ((1280, 640, 128, 2176), 100), ((1280, 640, 128, 2176), 140),
 ])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
