@@ -275,6 +275,10 @@ __host__ __device__ inline void prologue_split(int M, int nvec, int &cpr, int &p
     per = (nvec + cpr - 1) / cpr;
   }
 }
+// Up to six rows of 2048 to 3072: a warp takes a twelfth of every row, a vector per lane.  Decode step of four blocks, before and now,
+// us: 2560 wide, 3 rows 205.3, 199.0; 4 rows 211.2, 202.1; 6 rows 236.4, 228.2; 3072 wide, 6 rows 272.4, 263.7.  But 8 rows of 2560
+// 242.7, 242.9, and 6 rows of 2048 196.8, 200.5.
+inline bool norm_by_columns(int M, int K) { return M > 1 && M <= 6 && K > 2048 && (K >> 3) <= kMmaWarps * 32; }
 // All rows at once with up to two vectors per lane: they stay in registers between the two passes of a
 // norm (2560 wide, one row: 2.0 -> 1.5 us).
 inline bool norm_in_registers(int M, int K) {
@@ -287,7 +291,7 @@ inline bool norm_in_registers(int M, int K) {
 // EXTRA 1: the launch has an activation prologue or peer destinations (compiled apart so that the
 // plain launch carries none of that code).  The usual prologues of up to eight rows are compiled apart
 // once more, for the code and registers of the others cost them 1 to 2 %: 2 norm whose rows stay in
-// registers (norm_in_registers), 3 silu, 4 bf16.
+// registers (norm_in_registers), 3 silu, 4 bf16, 5 norm of several rows (norm_by_columns).
 //
 // Warp group g takes the g-th third of the CTA's images, in order, through ring slots g, g + 3, ... of
 // its own; epilogue warp g finishes the tiles whose first image (in this CTA) lies in that third.  A
@@ -308,7 +312,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
   __shared__ float xred[EXTRA ? RDQ_MAX_GEMV_M : 1][kMmaWarps];  // activation prologue: per-warp sums of squares
 
   // the prologue: known at compile time but for EXTRA 1
-  const int xop = EXTRA == 0 ? 0 : EXTRA == 2 ? 1 : EXTRA == 3 ? 2 : EXTRA == 4 ? 3 : a.xop;
+  const int xop = EXTRA == 0 ? 0 : EXTRA == 2 ? 1 : EXTRA == 3 ? 2 : EXTRA == 4 ? 3 : EXTRA == 5 ? 1 : a.xop;
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
@@ -644,14 +648,19 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
 
   const int nvec = K >> 3;
   int cpr = 1, per = nvec;
-  if (EXTRA && XS && xop != 0) prologue_split(M, nvec, cpr, per);
+  if (EXTRA == 5) {
+    cpr = kMmaWarps;
+    per = (nvec + kMmaWarps - 1) / kMmaWarps;
+  } else if (EXTRA && XS && xop != 0) {
+    prologue_split(M, nvec, cpr, per);
+  }
   const int vlo = (warp % cpr) * per, vhi = min(nvec, vlo + per), rows_at_once = kMmaWarps / cpr;
-  uint4 nw[2];  // (EXTRA 2)
+  uint4 nw[2];  // (EXTRA 2, 5)
   if (EXTRA && XS && xop == 1 && a.early) {
     // the norm's weights are constants: into registers, or L1, while the kernel before this one still runs
     for (int i = vlo + lane, q = 0; i < vhi; i += 32, ++q) {
       const uint4 v = ldg_nc16(a.x_weight + 8 * i);
-      if (EXTRA == 2 && q == 0) nw[0] = v;
+      if (EXTRA == 5 || (EXTRA == 2 && q == 0)) nw[0] = v;
       else if (EXTRA == 2) nw[1] = v;
       else asm volatile("" ::"r"(v.x));
     }
@@ -717,6 +726,64 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
           }
           *reinterpret_cast<uint4 *>(xsm + m * xpitch + 16 * i) = v[q];
         }
+      }
+    } else if (EXTRA == 5) {
+      // Two rows' loads in flight at a time, the weights there before the wait, and little code: what is run once a launch is
+      // fetched while the launch waits (all rows unrolled and kept in registers: slower than the general form).
+      constexpr int kRows = 2;
+      const int i = vlo + lane;
+      const bool in = i < vhi;
+      if (!a.early && in) nw[0] = ldg_nc16(a.x_weight + 8 * i);
+#pragma unroll 1
+      for (int m0 = 0; m0 < M; m0 += kRows) {
+        uint4 v[kRows], d[kRows];
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+          v[r] = d[r] = make_uint4(0u, 0u, 0u, 0u);
+          if (!in || m0 + r >= M) continue;
+          v[r] = ldg_cg16(a.x + 1ll * (m0 + r) * K + 8 * i);
+          if (a.x_aux) d[r] = ldg_cg16(a.x_aux + 1ll * (m0 + r) * K + 8 * i);
+        }
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+          __half2 *hv = reinterpret_cast<__half2 *>(&v[r]);
+          const __half2 *dh = reinterpret_cast<const __half2 *>(&d[r]);
+          float ss = 0.f;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if (a.x_aux) hv[j] = __hadd2(hv[j], dh[j]);
+            const float2 f = __half22float2(hv[j]);
+            ss += f.x * f.x + f.y * f.y;
+          }
+          if (in && m0 + r < M) {
+            if (a.x_out && blockIdx.x == 0) *reinterpret_cast<uint4 *>(a.x_out + 1ll * (m0 + r) * K + 8 * i) = v[r];
+            *reinterpret_cast<uint4 *>(xsm + (m0 + r) * xpitch + 16 * i) = v[r];
+          }
+          ss = warp_sum(ss);
+          if (lane == 0 && m0 + r < M) xred[m0 + r][warp] = ss;
+        }
+      }
+      asm volatile("bar.sync 2, %0;" ::"r"(kMmaWarps * 32) : "memory");
+      float rs = 0.f;  // of row `lane`
+      if (lane < M) {
+        float sum = 0.f;
+#pragma unroll
+        for (int w = 0; w < kMmaWarps; ++w) sum += xred[lane][w];
+        rs = rsqrtf(sum / K + a.x_eps);
+      }
+#pragma unroll 1
+      for (int m = 0; m < M; ++m) {
+        const float rm = __shfl_sync(0xffffffffu, rs, m);
+        if (!in) continue;
+        uint4 v = *reinterpret_cast<uint4 *>(xsm + m * xpitch + 16 * i);
+        __half2 *hv = reinterpret_cast<__half2 *>(&v);
+        const __half2 *wh = reinterpret_cast<const __half2 *>(&nw[0]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 f = __half22float2(hv[j]);
+          hv[j] = __hmul2(__floats2half2_rn(f.x * rm, f.y * rm), wh[j]);
+        }
+        *reinterpret_cast<uint4 *>(xsm + m * xpitch + 16 * i) = v;
       }
     } else if (xop == 1) {
       for (int m = warp / cpr; m < M; m += rows_at_once) {
@@ -1100,7 +1167,7 @@ int launch_gemv_tiled(const GemvTiledArgs &h, bool pdl, cudaStream_t stream) {
   const int smem = pl.smem;
 
 
-  static int smem_set[64][11] = {};
+  static int smem_set[64][12] = {};
   static std::mutex smem_mutex;
   int dev = 0;
   RDQ_CUDA(cudaGetDevice(&dev));
@@ -1108,11 +1175,13 @@ int launch_gemv_tiled(const GemvTiledArgs &h, bool pdl, cudaStream_t stream) {
   const bool extra = a.xop != 0 || h.n_dst > 0 || h.y_bf16;
   const bool in_registers = a.xop == 1 && !h.y_bf16 && norm_in_registers(h.M, h.K);
   const bool own = extra && h.n_dst == 0 && nt == 1 && xs;  // a variant of its own
+  const bool by_columns = a.xop == 1 && !h.y_bf16 && norm_by_columns(h.M, h.K);
   const int variant = own && in_registers                      ? 8
+                      : own && by_columns              ? 11
                       : own && a.xop == 2 && !h.y_bf16 ? 9
                       : own && a.xop == 3              ? 10
                                                        : (extra ? 4 : 0) + (nt - 1) * 2 + (xs ? 1 : 0);
-  static const void *const fns[11] = {
+  static const void *const fns[12] = {
       reinterpret_cast<const void *>(gemv_tiled_kernel<1, false, 0>),
       reinterpret_cast<const void *>(gemv_tiled_kernel<1, true, 0>),
       reinterpret_cast<const void *>(gemv_tiled_kernel<2, false, 0>),
@@ -1123,7 +1192,8 @@ int launch_gemv_tiled(const GemvTiledArgs &h, bool pdl, cudaStream_t stream) {
       reinterpret_cast<const void *>(gemv_tiled_kernel<2, true, 1>),
       reinterpret_cast<const void *>(gemv_tiled_kernel<1, true, 2>),
       reinterpret_cast<const void *>(gemv_tiled_kernel<1, true, 3>),
-      reinterpret_cast<const void *>(gemv_tiled_kernel<1, true, 4>)};
+      reinterpret_cast<const void *>(gemv_tiled_kernel<1, true, 4>),
+      reinterpret_cast<const void *>(gemv_tiled_kernel<1, true, 5>)};
   const void *fn = fns[variant];
   if (dev < 64 && smem_set[dev][variant] < smem) {
     RDQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
