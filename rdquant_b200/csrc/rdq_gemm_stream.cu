@@ -18,7 +18,7 @@
 // order: the result does not depend on timing (await_parts: those that leave, and who does their share).  A second kernel for these sums cost
 // 4-7 us per layer, and one CTA per tile adding them up to 13 us.
 //
-// Up to 64 tokens (best_plan) tiles are not cut: a tile has as many rows (8 to 128) as make all tiles cost the same bytes, and belongs
+// Up to 64 tokens, or 256 where that is faster (best_plan), tiles are not cut: a tile has as many rows (8 to 128) as make all tiles cost the same bytes, and belongs
 // to one cluster of one, two or four CTAs that share its k.  A chunk is 256 k of any format then (one, two or four boxes).  The
 // CTAs of a cluster exchange FP32 sums through distributed shared memory (finish_in_cluster): each finishes a share of the tokens.
 // They run at the same time by construction, and no word in global memory is involved.
@@ -50,6 +50,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 #include <unordered_map>
 
@@ -88,7 +89,7 @@ struct StreamSched {
   int E[3];                 // end of each format's chunk range
   int nkb;                  // k blocks of 64
   int R[3];                 // rows per tile
-  int cluster;              // (whole tiles) CTAs that share a tile's k: E and bnd are tiles then, bnd of a cluster
+  int cluster;              // (whole tiles) CTAs that share a tile's k: E are tiles of rows then, bnd a cluster's first (tile, token tile)
   int G;                    // CTAs
   int bnd[kMaxCtas + 1];    // first chunk of each CTA
 };
@@ -100,10 +101,10 @@ struct Segment {
 // the same where `S` chunks of every tile are this CTA's, numbered through
 __device__ __forceinline__ Segment whole_segment_at(const StreamSched &s, int S, int chunk) {
   Segment g;
-  const int t = chunk / S;
-  g.fmt = t < s.E[0] ? 0 : (t < s.E[1] ? 1 : 2);
-  g.row_tile = t - (g.fmt == 0 ? 0 : s.E[g.fmt - 1]);
-  g.m_tile = 0;
+  const int t = chunk / S, rt = t / s.mt;
+  g.m_tile = t - rt * s.mt;
+  g.fmt = rt < s.E[0] ? 0 : (rt < s.E[1] ? 1 : 2);
+  g.row_tile = rt - (g.fmt == 0 ? 0 : s.E[g.fmt - 1]);
   g.start = t * S;
   g.c0 = chunk - g.start;
   g.c1 = S;
@@ -370,16 +371,17 @@ __device__ __forceinline__ void store_tokens(const StreamSched &sc, const Stream
 }
 // a tile that this CTA has alone
 template <bool BF16>
-__device__ __forceinline__ void finish_alone(const StreamSched &sc, const StreamArgs &a, const Row &row, uint32_t acc, bool dry) {
+__device__ __forceinline__ void finish_alone(const StreamSched &sc, const StreamArgs &a, const Row &row, uint32_t acc, int tok0, int ntok,
+                                             bool dry) {
 #pragma unroll 1
-  for (int t = 0; t < sc.M; t += 16) {
+  for (int t = 0; t < ntok; t += 16) {
     uint32_t v[16];
     tmem_ld16(acc + t, v);
     tmem_wait_ld16(v);
     float o[16];
 #pragma unroll
     for (int e = 0; e < 16; ++e) o[e] = __uint_as_float(v[e]);
-    store_tokens<BF16>(sc, a, row, o, t, dry ? 0 : 16);
+    store_tokens<BF16>(sc, a, row, o, tok0 + t, dry ? 0 : min(16, ntok - t));
     if (dry) break;
   }
 }
@@ -389,7 +391,7 @@ __device__ __forceinline__ void finish_alone(const StreamSched &sc, const Stream
 // tiles; two buffers take turns.  Layout of a buffer: [rank][four tokens][128 rows][4].
 template <bool BF16>
 __device__ __forceinline__ void finish_in_cluster(StreamSmem &S, const StreamSched &sc, const StreamArgs &a, const Row &row, uint32_t acc,
-                                                  uint32_t r_ring, int rank, int q, int lane, int turn, bool more, bool dry) {
+                                                  uint32_t r_ring, int tok0, int rank, int q, int lane, int turn, bool more, bool dry) {
   const int C = sc.cluster, share = sc.nt / C;  // a multiple of four
   const uint32_t part = share * 512;            // bytes of a rank's sums
   const uint32_t buf = r_ring + (turn & 1) * C * part, at = (q * 32 + lane) * 16;
@@ -437,7 +439,7 @@ __device__ __forceinline__ void finish_in_cluster(StreamSmem &S, const StreamSch
       __syncwarp();
       if (lane < C) mbar_arrive_cluster(mapa_u32(smem_u32(empty), lane));
     }
-    store_tokens<BF16>(sc, a, row, o, tok, dry ? 0 : min(16, share - t));
+    store_tokens<BF16>(sc, a, row, o, tok0 + tok, dry ? 0 : min(16, share - t));
   }
 }
 
@@ -712,8 +714,8 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
       uint32_t v[2][16];
       if (WHOLE) {
         if (q * 32 < sc.R[g.fmt]) {  // (else no rows)
-          if (sc.cluster > 1) finish_in_cluster<BF16>(S, sc, a, row, acc, r_ring, static_cast<int>(rank), q, lane, turn, ck + 2 * own < end, dry);
-          else finish_alone<BF16>(sc, a, row, acc, dry);
+          if (sc.cluster > 1) finish_in_cluster<BF16>(S, sc, a, row, acc, r_ring, tok0, static_cast<int>(rank), q, lane, turn, ck + 2 * own < end, dry);
+          else finish_alone<BF16>(sc, a, row, acc, tok0, ntok, dry);
         }
         if (dry) {
           dry = false;
@@ -910,6 +912,7 @@ struct StreamPlan {
   StreamSched sc;
   int wide, nw, smem;  // wide: the variant for more than 64 tokens per tile
   int whole, w_pitch, s_pitch;
+  double us;  // estimated time
 };
 
 // Token tiles of equal width; a chunk costs what bounds it: its bytes at the SM's share of the HBM
@@ -957,6 +960,13 @@ StreamPlan make_plan(int n4, int n8, int n16, int M, int K) {
   p.wide = s.nt > 64;
   const int xb = (p.wide ? kStages<128> * kBlocks<128> : kStages<64> * kBlocks<64>) * s.nt * 128;
   p.nw = std::min(kMaxRing, (kSmemMax - 1024 - xb) / (kChunkBytes + kScaleBytes));
+  // Fitted to 40 layers at 72 to 512 rows (6 % off on average, 49 % at worst): a CTA's share and the parts that the most
+  // divided tile is put together from.
+  const double share = static_cast<double>(w) / s.G;
+  double parts = 0;
+  for (int f = 0; f < 3; ++f)
+    if (n[f]) parts = std::max(parts, std::ceil(s.S[f] * u[f] / share));
+  p.us = 7.6 + 0.672e-3 * share + 0.22 * parts + 0.32 * M / 128;
   p.nw = std::min(p.nw, 8);
   p.smem = 1024 + xb + p.nw * (kChunkBytes + kScaleBytes);
   p.whole = 0;
@@ -999,22 +1009,22 @@ int clusters_at_once(int size) {
 }
 
 // Whole tiles: each belongs to one cluster alone, whose CTAs share its k, so that nothing is put together through global
-// memory.  Rows per tile by the bytes of a row, so that all tiles cost the same; `us`: an estimate of the launch's time.
-bool make_whole_plan(int n4, int n8, int n16, int M, int K, int cluster, StreamPlan *out, double *us) {
+// memory.  Rows per tile by the bytes of a row, so that all tiles cost the same.
+bool make_whole_plan(int n4, int n8, int n16, int M, int K, int cluster, StreamPlan *out) {
   const int workers = clusters_at_once(cluster);
-  if (M > 64 || workers == 0 || (K + 255) / 256 < cluster) return false;
+  if (workers == 0 || (K + 255) / 256 < cluster) return false;
   StreamPlan p;
   StreamSched &s = p.sc;
   s.M = M;
-  s.mt = 1;
-  s.nt = (M + 15) / 16 * 16;
+  s.mt = (M + 63) / 64;
+  s.nt = ((M + s.mt - 1) / s.mt + 15) / 16 * 16;
   s.nkb = (K + 63) / 64;
   s.cluster = cluster;
   const int n[3] = {n4, n8, n16};
   const double bytes[3] = {0.5625, 1.0, 2.0};
   int least = 0;
   for (int f = 0; f < 3; ++f) least += (n[f] + 127) / 128;
-  const int most = std::max(1, (least + workers - 1) / workers);  // tiles of a cluster
+  const int most = std::max(1, (least * s.mt + workers - 1) / workers);  // tiles of a cluster
   int tiles = 0;
   for (double t = 4.5;; t += 0.5) {
     tiles = 0;
@@ -1022,7 +1032,7 @@ bool make_whole_plan(int n4, int n8, int n16, int M, int K, int cluster, StreamP
       s.R[f] = std::max(8, std::min(128, static_cast<int>(t / bytes[f] / 8) * 8));
       tiles += (n[f] + s.R[f] - 1) / s.R[f];
     }
-    if (tiles <= most * workers) break;  // (holds at the latest where all tiles have 128 rows)
+    if (tiles * s.mt <= most * workers) break;  // (holds at the latest where all tiles have 128 rows)
   }
   int e = 0;
   double heaviest = 0;
@@ -1032,9 +1042,10 @@ bool make_whole_plan(int n4, int n8, int n16, int M, int K, int cluster, StreamP
     s.E[f] = e;
     if (n[f]) heaviest = std::max(heaviest, s.R[f] * bytes[f]);
   }
-  s.G = std::min(workers, tiles);
-  for (int b = 0; b <= s.G; ++b) s.bnd[b] = static_cast<int>(1ll * tiles * b / s.G);
-  const int each = (tiles + s.G - 1) / s.G;
+  const int items = tiles * s.mt;
+  s.G = std::min(workers, items);
+  for (int b = 0; b <= s.G; ++b) s.bnd[b] = static_cast<int>(1ll * items * b / s.G);
+  const int each = (items + s.G - 1) / s.G;
   p.wide = 0;
   p.whole = 1;
   p.w_pitch = std::max({n4 ? s.R[0] : 0, n8 ? 2 * s.R[1] : 0, n16 ? 4 * s.R[2] : 0}) * 128;
@@ -1048,7 +1059,7 @@ bool make_whole_plan(int n4, int n8, int n16, int M, int K, int cluster, StreamP
   // clusters is picked but for 0.5 % on average, 9 % at worst.
   const double steps = each * ((s.S[0] + cluster - 1) / cluster) * (0.181 + 0.0035 * s.nt);
   const double memory = heaviest * K / cluster * each / 43e3 * 0.484;
-  *us = 4.9 + std::max(steps, memory) + 1.35 * std::min(steps, memory) + (cluster > 1 ? 1.2 : 0.0) + (cluster > 2 ? 0.25 : 0.0);
+  p.us = 4.9 + std::max(steps, memory) + 1.35 * std::min(steps, memory) + (cluster > 1 ? 1.2 : 0.0) + (cluster > 2 ? 0.25 : 0.0);
   *out = p;
   return true;
 }
@@ -1058,21 +1069,25 @@ bool make_whole_plan(int n4, int n8, int n16, int M, int K, int cluster, StreamP
 // one after another, us before and now: 2560 -> 6144 10.6, 8.3; 4096 -> 2560 10.6, 7.7; 9728 -> 2560 12.5, 10.6; 1024 -> 1024 8.0,
 // 6.0; 8192 -> 8192 15.5, 13.7.  Above 200 MB the tail is short beside the rest and cut tiles use the MMA's 128 rows better (8192 ->
 // 57344 at 48 rows 73.6, 76.2) unless there are few tokens (9 rows 61.1, 58.4).
+//
+// More tokens come in tiles of 64, each work of its own: the weights are converted for each, where cut tiles convert them for 128
+// at a time, so that it pays where a CTA's share is small beside the tail.  The estimates decide; the margin covers theirs
+// (12416 -> 896 at 192 rows, 0.89 by them, is 20.8 us whole and 17.1 cut).  Over 40 layers, against
+// cut tiles and the GEMM over decoded weights, 20 % less time at 72 to 128 rows and 12 % at 160 to 256 (2560 -> 1024 at 128
+// rows 11.2 us, now 7.6; 2560 -> 6144 16.5, 11.4; 4096 -> 2560 at 192 rows 14.6, 11.6).  Beyond, 7 % would be left.
 StreamPlan best_plan(int n4, int n8, int n16, int M, int K) {
-  StreamPlan best = {};
-  bool found = false;
-  if (M <= 64 && (n4 * 0.5625 + n8 + 2.0 * n16) * K < 150e6) {
-    double least = 0;
+  const bool fits = (n4 * 0.5625 + n8 + 2.0 * n16) * K < 150e6, few = M <= 64 && fits;
+  StreamPlan best = make_plan(n4, n8, n16, M, K);
+  double least = few ? 1e30 : 0.88 * best.us;
+  if (fits && M <= 256) {
     for (int cluster = 1; cluster <= 4; cluster *= 2) {
       StreamPlan p;
-      double us = 0;
-      if (!make_whole_plan(n4, n8, n16, M, K, cluster, &p, &us) || (found && us >= least)) continue;
+      if (!make_whole_plan(n4, n8, n16, M, K, cluster, &p) || p.us >= least) continue;
       best = p;
-      least = us;
-      found = true;
+      least = p.us;
     }
   }
-  return found ? best : make_plan(n4, n8, n16, M, K);
+  return best;
 }
 
 // the plans of the last few thousand (layer shape, rows) pairs of this thread
@@ -1111,6 +1126,10 @@ bool gemm_stream_takes(int K) { return K % 64 == 0; }
 size_t gemm_stream_workspace(int n4, int n8, int n16, int M, int K) {
   const StreamPlan &p = stream_plan(n4, n8, n16, M, K);
   return p.whole ? 256 : 2ull * p.sc.G * p.sc.nt * 128 * sizeof(float);
+}
+double gemm_stream_estimate(int n4, int n8, int n16, int M, int K) {
+  const StreamPlan &p = stream_plan(n4, n8, n16, M, K);
+  return p.whole ? p.us : 0.0;
 }
 bool gemm_stream_uses_words(int n4, int n8, int n16, int M, int K) { return !stream_plan(n4, n8, n16, M, K).whole; }
 

@@ -126,6 +126,7 @@ bool gemm_better_without_scratch(int M, int N, int K);
 // weight-streaming GEMM (rdq_gemm_stream.cu)
 bool gemm_stream_takes(int K);
 size_t gemm_stream_workspace(int n4, int n8, int n16, int M, int K);
+double gemm_stream_estimate(int n4, int n8, int n16, int M, int K);  // microseconds where its tiles are whole, else 0
 bool gemm_stream_uses_words(int n4, int n8, int n16, int M, int K);  // GemmArgs::counters
 int launch_gemm_stream(const GemmArgs &a, void *workspace, size_t workspace_bytes, bool pdl, cudaStream_t stream);
 // GEMM over weights decoded once per call (rdq_gemm_dense.cu)

@@ -159,6 +159,9 @@ def test_wide_layers_of_few_rows_need_no_decoding(rows, shape, scratch):
     ((30000, 4000, 0, 8192), 33),        # 170 MB: cut tiles
     # block scales copied 8 bytes at a time: whole tiles, cut ones, two tiles of tokens
     ((300, 130, 20, 896), 33), ((1280, 640, 128, 2176), 100), ((1280, 640, 128, 2176), 140),
+    # whole tiles of more than 64 tokens: clusters of one, two and four; tiles of tokens that are hardly filled; several tiles a CTA
+    ((1280, 640, 128, 640), 65), ((3072, 896, 128, 4096), 128), ((640, 384, 0, 2560), 129), ((300, 130, 20, 2624), 200),
+    ((4096, 1920, 128, 2560), 193), ((0, 0, 256, 8192), 256), ((13056, 6144, 256, 2560), 66), ((640, 384, 0, 2560), 257),
 ])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_streaming_gemm_tiles(shape, rows, dtype):
