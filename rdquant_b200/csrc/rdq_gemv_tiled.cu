@@ -14,7 +14,7 @@
 // time-balanced range of them (a small model of ring-resident and streamed images per format,
 // see launch_gemv_tiled).  Inside a CTA
 //   producer warp   one thread sets up the barriers and issues one cp.async.bulk (TMA) copy per
-//                   image (10-19 KB) into a shared-memory ring, mbarrier tracked.  It starts BEFORE
+//                   image (10-19 KB; a run of smaller ones) into a shared-memory ring, mbarrier tracked.  It starts BEFORE
 //                   griddepcontrol.wait where the caller allows it: the ring of this layer fills
 //                   while the preceding kernel runs.  It is also the only thread that executes
 //                   that wait; the other warps sleep on an mbarrier it completes once the

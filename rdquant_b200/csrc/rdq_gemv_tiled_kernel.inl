@@ -4,8 +4,12 @@ namespace rdq {
 namespace {
 
 // Image schedule, identical on every CTA.  Images are numbered in storage order.
+//
+// Where K has only short chunks (images_per_run) the numbered images are runs of up to `run` stored ones of a tile: one copy,
+// one ring slot and one turn of a warp group each, everything else below counts in them.
 struct TSched {
   int ck;            // chunk length in NVFP4 elements
+  int run, chunks;   // stored images per numbered one, of an NVFP4 tile
   int S4, S8, S16;   // images per tile in each group
   int t4, t8;        // tiles in the NVFP4 / FP8 groups
   int e4, e8, e16;   // end of each group's image range
@@ -23,6 +27,17 @@ struct TSched {
   __device__ __forceinline__ long long image_offset(int s) const {
     if (s < e4) return 1ll * s * img4;
     return 1ll * e4 * img4 + 1ll * (s - e4) * img8;
+  }
+  // the stored images of run s: their number, size and place
+  __device__ __forceinline__ int run_at(int s, int &img, long long &offset) const {
+    const int fmt = s < e4 ? 0 : (s < e8 ? 1 : 2);
+    const int i = s - (fmt == 0 ? 0 : (fmt == 1 ? e4 : e8)), S = fmt == 0 ? S4 : (fmt == 1 ? S8 : S16);
+    const int tile = i / S, first = (i - tile * S) * run, all = chunks << fmt;
+    img = fmt == 0 ? img4 : img8;
+    offset = (1ll * tile * all + first) * img;
+    if (fmt > 0) offset += 1ll * chunks * t4 * img4;
+    if (fmt > 1) offset += 2ll * chunks * t8 * img8;
+    return min(run, all - first);
   }
 };
 
@@ -62,6 +77,8 @@ __device__ __forceinline__ uint4 ld_relaxed16(const float *p) {
   return v;
 }
 
+constexpr int kRunBytes = 15872;  // NVFP4 bytes of a run: three slots fit beside 44 KB of activations and the hand-over slots of 16 rows
+constexpr int kRunChunk = 512;   // longest chunk whose images travel in runs
 constexpr int kAskAhead = 20 * 1024;  // bytes of weights per warp group that are asked into L2 before they may be read (12 and 40 KB: slower)
 constexpr int kStageUnroll = 2;  // pair-loop unrolling of the NVFP4 / FP8 stages
 
@@ -298,7 +315,9 @@ inline bool norm_in_registers(int M, int K) {
 // group therefore hands sums over once per tile -- images dealt out in turn would end every stage of a
 // two-image tile with a hand-over, which measured a third of the MMA warps' time -- and everybody
 // derives his images from the range alone, without a list.
-template <int NT, bool XS, int EXTRA>
+//
+// RUNS: a numbered image is a run of stored ones (TSched), whose pieces the warps of a group share as if they were one.
+template <int NT, bool XS, int EXTRA, bool RUNS = false>
 __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_constant__ TiledArgs a,
                                                   const __grid_constant__ TSched sc) {
   extern __shared__ __align__(128) uint8_t smem[];
@@ -354,10 +373,18 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
     // ==================================================================== producer
     const int most = (nimg + kGroups - 1) / kGroups;  // images of the longest third
     auto copy_in = [&](int img, int slot) {
-      const uint32_t bytes = static_cast<uint32_t>(img < sc.e4 ? sc.img4 : sc.img8);
+      uint32_t bytes = static_cast<uint32_t>(img < sc.e4 ? sc.img4 : sc.img8);
+      long long from;
+      if (RUNS) {
+        int one;
+        bytes = sc.run_at(img, one, from);
+        bytes *= one;
+      } else {
+        from = sc.image_offset(img);
+      }
       const uint32_t full = smem_u32(&bar_full[slot]);
       mbar_arrive_expect_tx(full, bytes);
-      bulk_g2s(smem_base + slot * a.slot_bytes, a.tiled + sc.image_offset(img), bytes, full);
+      bulk_g2s(smem_base + slot * a.slot_bytes, a.tiled + from, bytes, full);
     };
     // The ring is filled with weights first (they do not depend on the preceding kernel);
     // only then wait for that kernel and fetch the activations it produced.
@@ -437,7 +464,16 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
       // variant, where chains with the flag carry the code as well (host-to-host step 39.4 and 39.3 us without
       // and with it), and in that of bf16 rows; the norm and SiLU variants lost 0.5 % to the code alone.
       if (EXTRA == 0 || EXTRA == 4) {
-        const long long from = sc.image_offset(g_begin), to = min(sc.image_offset(g_end), from + kAskAhead);
+        long long from = 0, to = 0;
+        if (RUNS) {
+          int one;
+          sc.run_at(g_begin, one, from);
+          sc.run_at(g_end, one, to);
+        } else {
+          from = sc.image_offset(g_begin);
+          to = sc.image_offset(g_end);
+        }
+        to = min(to, from + kAskAhead);
         for (long long at = from + lane * 128; at < to; at += 32 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.tiled + at));
       }
       pdl_wait();
@@ -929,7 +965,27 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_tiled_kernel(const __grid_co
     // inside a group the warps take turns on the pair ranges, so uneven splits average out
     const int lw = turn++ & (kWarpsPerGroup - 1);
     const int lo = lw * npair / kWarpsPerGroup, hi = (lw + 1) * npair / kWarpsPerGroup;
-    if (fmt == 0) {
+    if (RUNS) {
+      const int first = c * sc.run, pairs = min(sc.run, (sc.chunks << fmt) - first) * npair;
+      const int end = (lw + 1) * pairs / kWarpsPerGroup, img = fmt == 0 ? sc.img4 : sc.img8;
+      int p = lw * pairs / kWarpsPerGroup, i = p / npair, q = p - i * npair;
+#pragma unroll 1
+      while (p < end) {
+        const int n = min(npair - q, end - p);
+        const uint32_t ibase = sbase + i * img;
+        if (fmt == 0) {
+          stage_fp4<NT, XS>(acc, ibase + lm_lane + q * 32, ibase + sc_lane + q * 4, ibase + sc_lane + 8 * spitch + q * 4, xb,
+                            2 * ((first + i) * ck + q * 64 + t * 8), n, sel);
+        } else if (fmt == 1) {
+          stage_fp8<NT, XS>(acc, ibase + lm_lane + q * 32, xb, 2 * ((first + i) * (ck >> 1) + q * 32 + t * 4), n);
+        } else {
+          stage_fp16<NT, XS>(acc, ibase + lm_lane + q * 32, xb, 2 * ((first + i) * (ck >> 2) + q * 16 + t * 2), n);
+        }
+        p += n;
+        ++i;
+        q = 0;
+      }
+    } else if (fmt == 0) {
       stage_fp4<NT, XS>(acc, sbase + lm_lane + lo * 32, sbase + sc_lane + lo * 4, sbase + sc_lane + 8 * spitch + lo * 4,
                         xb, 2 * (c * ck + lo * 64 + t * 8), hi - lo, sel);
     } else if (fmt == 1) {
@@ -989,6 +1045,19 @@ void gemv_tiled_scratch(size_t *workspace_bytes, size_t *flag_bytes) {
   *flag_bytes = (static_cast<size_t>(G) + 2) * sizeof(int32_t);     // status word at index G
 }
 
+// Stored images per copy: one, unless the chunks are short (K / 64 with a large prime factor: 64 * 2 * 67 has chunks of 128 and
+// images of 1.5 KB, eighteen of which were all that an SM had on its way).  As many as leave a slot to every warp group beside the
+// most activations that go to shared memory, all runs of a tile about equal: runs of 10, 8 and 5 KB took 8, 17 and 37 % longer over
+// fourteen layers.  Calls one after another, image by image and in runs, us, one row / eight: 2368 -> 8192 38.7 / 38.8, 9.5 / 9.6;
+// 4736 -> 2048 12.0 / 11.1, 6.4 / 7.8; 11008 -> 4096 25.1 / 22.4, 11.7 / 15.5; 18944 -> 3584 20.5 / 16.0, 15.0 / 15.0, but with leave
+// to read weights early 21.1, 21.5 for one.  From chunks of 704 on (26048 -> 1536) runs cost up to 2.5 %.
+inline int images_per_run(int K) {
+  const int ck = tiled_chunk_k(K), chunks = K / ck, most = kRunBytes / img_bytes(0, ck);
+  if (ck > kRunChunk || most < 2) return 1;
+  const int runs = (chunks + most - 1) / most;
+  return (chunks + runs - 1) / runs;
+}
+
 // Shared-memory plan of one launch: weight ring | flush ring | output metadata | activations (if
 // they fit).
 struct SmemPlan {
@@ -997,7 +1066,7 @@ struct SmemPlan {
 };
 static SmemPlan smem_plan(int M, int K, bool shared) {
   SmemPlan p;
-  const int slot_bytes = (img_bytes(0, tiled_chunk_k(K)) + 127) & ~127;
+  const int slot_bytes = (images_per_run(K) * img_bytes(0, tiled_chunk_k(K)) + 127) & ~127;
   // hand-over slots of 4 warps x 16 rows x (M rounded up to 4) partial sums (1 - 4 KB): two per group
   // up to eight activation rows, then one, and one for each later group's part of a shared tile
   p.fdep = M <= 8 ? kFlushRing : 1;
@@ -1042,9 +1111,11 @@ static TiledPlan make_tiled_plan(int n4, int n8, int n16, int K, int M, bool sha
   const int nst = smem_plan(M, K, true).nst;  // in either case: results do not depend on the flag
   const int ck = tiled_chunk_k(K);
   sc.ck = ck;
-  sc.S4 = K / ck;
-  sc.S8 = sc.S4 * 2;
-  sc.S16 = sc.S4 * 4;
+  sc.chunks = K / ck;
+  sc.run = images_per_run(K);
+  sc.S4 = (sc.chunks + sc.run - 1) / sc.run;
+  sc.S8 = (sc.chunks * 2 + sc.run - 1) / sc.run;
+  sc.S16 = (sc.chunks * 4 + sc.run - 1) / sc.run;
   sc.t4 = n4 / kTileRows;
   sc.t8 = n8 / kTileRows;
   const int t16 = n16 / kTileRows;
@@ -1068,7 +1139,7 @@ static TiledPlan make_tiled_plan(int n4, int n8, int n16, int K, int M, bool sha
     // block (landing time: 2500 .. 7000 give the same step time within 2 %, 1200 is 8 % slower).
     const double kappa[3] = {0.123, 0.0715, 0.038};  // compute cycles per image byte and group
     const double land = 4500.0;                      // cycles from copy issue to landing under load
-    const double img[3] = {double(sc.img4), double(sc.img8), double(sc.img8)};
+    const double img[3] = {double(sc.img4) * sc.run, double(sc.img8) * sc.run, double(sc.img8) * sc.run};
     const double cnt[3] = {double(sc.e4), double(sc.e8 - sc.e4), double(sc.e16 - sc.e8)};
     const double spg = double(nst) / kGroups;
     auto n_of = [&](int f, double T) {
@@ -1156,7 +1227,7 @@ int launch_gemv_tiled(const GemvTiledArgs &h, bool pdl, cudaStream_t stream) {
   a.peer_state = h.peer_state;
   a.xop = h.x_bf16 ? 3 : h.xop; a.x_aux = h.x_aux; a.x_weight = h.x_weight; a.x_out = h.x_out; a.x_eps = h.x_eps;
   a.status_idx = sm_count();
-  a.slot_bytes = (img_bytes(0, sc.ck) + 127) & ~127;
+  a.slot_bytes = (sc.run * img_bytes(0, sc.ck) + 127) & ~127;
   const int nt = h.M <= 8 ? 1 : 2;
   a.fdepth = pl.fdep;
   a.nstages = pl.nst;
@@ -1167,21 +1238,22 @@ int launch_gemv_tiled(const GemvTiledArgs &h, bool pdl, cudaStream_t stream) {
   const int smem = pl.smem;
 
 
-  static int smem_set[64][12] = {};
+  static int smem_set[64][20] = {};
   static std::mutex smem_mutex;
   int dev = 0;
   RDQ_CUDA(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> smem_lock(smem_mutex);
   const bool extra = a.xop != 0 || h.n_dst > 0 || h.y_bf16;
   const bool in_registers = a.xop == 1 && !h.y_bf16 && norm_in_registers(h.M, h.K);
-  const bool own = extra && h.n_dst == 0 && nt == 1 && xs;  // a variant of its own
+  const bool runs = sc.run > 1;
+  const bool own = extra && h.n_dst == 0 && nt == 1 && xs && !runs;  // a variant of its own
   const bool by_columns = a.xop == 1 && !h.y_bf16 && norm_by_columns(h.M, h.K);
   const int variant = own && in_registers                      ? 8
                       : own && by_columns              ? 11
                       : own && a.xop == 2 && !h.y_bf16 ? 9
                       : own && a.xop == 3              ? 10
-                                                       : (extra ? 4 : 0) + (nt - 1) * 2 + (xs ? 1 : 0);
-  static const void *const fns[12] = {
+                                                       : (runs ? 12 : 0) + (extra ? 4 : 0) + (nt - 1) * 2 + (xs ? 1 : 0);
+  static const void *const fns[20] = {
       reinterpret_cast<const void *>(gemv_tiled_kernel<1, false, 0>),
       reinterpret_cast<const void *>(gemv_tiled_kernel<1, true, 0>),
       reinterpret_cast<const void *>(gemv_tiled_kernel<2, false, 0>),
@@ -1193,7 +1265,15 @@ int launch_gemv_tiled(const GemvTiledArgs &h, bool pdl, cudaStream_t stream) {
       reinterpret_cast<const void *>(gemv_tiled_kernel<1, true, 2>),
       reinterpret_cast<const void *>(gemv_tiled_kernel<1, true, 3>),
       reinterpret_cast<const void *>(gemv_tiled_kernel<1, true, 4>),
-      reinterpret_cast<const void *>(gemv_tiled_kernel<1, true, 5>)};
+      reinterpret_cast<const void *>(gemv_tiled_kernel<1, true, 5>),
+      reinterpret_cast<const void *>(gemv_tiled_kernel<1, false, 0, true>),
+      reinterpret_cast<const void *>(gemv_tiled_kernel<1, true, 0, true>),
+      reinterpret_cast<const void *>(gemv_tiled_kernel<2, false, 0, true>),
+      reinterpret_cast<const void *>(gemv_tiled_kernel<2, true, 0, true>),
+      reinterpret_cast<const void *>(gemv_tiled_kernel<1, false, 1, true>),
+      reinterpret_cast<const void *>(gemv_tiled_kernel<1, true, 1, true>),
+      reinterpret_cast<const void *>(gemv_tiled_kernel<2, false, 1, true>),
+      reinterpret_cast<const void *>(gemv_tiled_kernel<2, true, 1, true>)};
   const void *fn = fns[variant];
   if (dev < 64 && smem_set[dev][variant] < smem) {
     RDQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));

@@ -52,6 +52,36 @@ def test_random_bytes(shape, m, flags):
     assert onp.rel_err(y, y_ref) < TOL
 
 
+@pytest.mark.parametrize("m", [1, 3, 8, 16])
+@pytest.mark.parametrize("shape", [(128, 64, 32, 2368), (384, 0, 0, 4736), (0, 48, 0, 8576), (0, 0, 32, 13568), (2048, 896, 128, 4736),
+                                   (3072, 1024, 128, 11008), (48, 32, 16, 18944), (8192, 2048, 128, 4672)])
+def test_short_chunks(shape, m):
+    """K / 64 with a large prime factor: chunks of 64 to 512 whose images travel in runs, the last of a tile a shorter one;
+    tiles shared by groups and CTAs, and several tiles a group.  The activation prologues take the same rows."""
+    n4, n8, n16, k = shape
+    layer = random_packed_layer(n4, n8, n16, k, seed=k + m)
+    splits = dict(zip(ORDER, shape[:3]))
+    y, y_ref, fd = _run(layer, splits, k, m, _lib.RDQ_GEMV_AUTO, bias=True, seed=m)
+    assert onp.rel_err(y, y_ref) < TOL
+    if k % 128 or not rdquant_cuda.gemv_stages_x(m, k):
+        return
+    gen = torch.Generator().manual_seed(k)
+    gu = torch.randn(m, 2 * k, generator=gen).half().cuda()
+    w = (1 + 0.1 * torch.randn(k, generator=gen)).half().cuda()
+    act, res = torch.empty(m, k, dtype=torch.float16, device="cuda"), torch.empty(m, k, dtype=torch.float16, device="cuda")
+    rdquant_cuda.silu_mul(gu, act, 0)
+    plain = rdquant_cuda.mixed_gemv(act, fd)
+    for flags in (0, _lib.RDQ_GEMV_PDL):
+        assert torch.equal(rdquant_cuda.mixed_gemv_silu(gu, fd, flags=flags), plain)
+    x = gu[:, :k].contiguous()
+    y = rdquant_cuda.mixed_gemv_norm(x, act, w, 1e-6, fd, residual_out=res, flags=_lib.RDQ_GEMV_PDL)
+    assert torch.equal(res, x + act)
+    hn = (res.float() * torch.rsqrt(res.float().pow(2).mean(-1, keepdim=True) + 1e-6)).half() * w
+    ref = onp.mixed_precision_linear(hn.cpu().numpy(), onp.torch_layer_to_np(layer), splits, k, None)
+    assert onp.rel_err(y.cpu().float().numpy(), ref) < TOL
+    assert int(fd["tile_counters"].abs().sum()) == 0
+
+
 @pytest.mark.parametrize("m", [1, 5, 16])
 def test_many_tiles_per_cta(m):
     """Short rows, many channels: every warp group finishes several whole tiles and its ring
