@@ -52,10 +52,16 @@ bool has_row_major(const rdq_layer &l) {
 // rows and 18 MB up to 16, date from a streaming GEMM that set up behind its wait; now 19 MB (6500 x 4096) takes
 // 12.2 us on either at 8 rows and 40 MB (13504 x 4096) 18.1 / 14.9, at 16 rows 11 MB (6144 x 2560) 9.1 / 10.9 and 18 MB
 // (2560 x 9728) 14.5 / 12.8.
+// Seven and eight rows that the GEMV does not keep in shared memory go to the streaming GEMM from 28 MB on: 37 MB
+// (3584 x 14336) 15.5 / 13.3 us, 30 MB (12672 x 3328) 0.83 of the time, 26 MB (5120 x 7168) 1.1; decode steps of eight
+// sequences and four blocks, 3328 wide 295 / 272, 3584 wide 313 / 283, but 25 MB (3072 x 11648) cost 2 % there.  Not
+// fewer rows: a step whose norms still run inside the GEMV lost 5 % to a streaming down projection in between (3584
+// wide, 6 sequences 320 / 337).
 int stream_from(const rdq_layer &l) {
   const double bytes = l.n_fp4 * (l.K * 0.5625) + l.n_fp8 * (l.K + 4.0) + l.n_fp16 * (l.K * 2.0);
   if (!l.w_tiled) return bytes > 40e6 ? 1 : (bytes > 18e6 ? 9 : RDQ_MAX_GEMV_M + 1);
-  return bytes > 80e6 ? 1 : (bytes > 40e6 ? 3 : 9);
+  if (bytes > 40e6) return bytes > 80e6 ? 1 : 3;
+  return bytes > 28e6 && !tiled_stages_x(8, l.K) ? (tiled_stages_x(7, l.K) ? 8 : 7) : 9;
 }
 
 // Few rows: the decode GEMV (tiled layout, else the any-shape kernel), or the streaming GEMM from
