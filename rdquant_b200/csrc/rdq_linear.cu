@@ -47,11 +47,14 @@ bool has_row_major(const rdq_layer &l) {
 //   40 MB (13440 x 4096)  4 rows 10.9 / 14.8, 13.5 / 14.0     8 rows 16.3 / 14.8, 17.4 / 14.2
 //   48 MB (8192 x 8192)   2 rows 11.9 / 15.7, 15.8 / 14.8     4 rows 18.3 / 16.0, 19.9 / 15.0
 //   97 MB (16384 x 8192)  1 row  19.6 / 22.8, 27.8 / 21.7     4 rows 31.5 / 23.2, 36.5 / 22.1
-// The row-major GEMV of layers without a tiled layout starts at 1.9 us where the streaming GEMM takes 6
-// to 9 (300 NVFP4 + 130 FP8 + 20 FP16 rows of 1024: 2.3 against 9.0 us at one row).  Its lines, 40 MB up to 8
-// rows and 18 MB up to 16, date from a streaming GEMM that set up behind its wait; now 19 MB (6500 x 4096) takes
-// 12.2 us on either at 8 rows and 40 MB (13504 x 4096) 18.1 / 14.9, at 16 rows 11 MB (6144 x 2560) 9.1 / 10.9 and 18 MB
-// (2560 x 9728) 14.5 / 12.8.
+// The row-major GEMV of layers without a tiled layout starts at 1.9 us where the streaming GEMM takes 6 to 8 (2 MB,
+// 3001 x 1024: 2.6 / 6.3 us at one row).  With leave to read weights early or without:
+//   12 MB (2001 x 8192)   1 row 10.0 / 10.8    8 rows 10.2 / 10.8    16 rows 11.2 / 10.8
+//   15 MB (5001 x 4096)   1 row 10.6 / 10.5    8 rows 11.4 / 10.5    16 rows 12.7 / 10.5
+//   19 MB (3072 x 8576)   1 row 11.5 / 12.1    8 rows 12.0 / 12.1    16 rows 13.0 / 12.2
+//   22 MB (12001 x 2560)  1 row 11.9 / 10.2    8 rows 12.7 / 10.2    16 rows 14.3 / 10.3
+// It keeps up to eight rows up to 22 MB, more of them up to 12; of 22 layers 9001 x 3008 (19 MB) fares worst, 10.6 / 12.0
+// at nine rows.
 // Seven and eight rows that the GEMV does not keep in shared memory go to the streaming GEMM from 28 MB on: 37 MB
 // (3584 x 14336) 15.5 / 13.3 us, 30 MB (12672 x 3328) 0.83 of the time, 26 MB (5120 x 7168) 1.1; decode steps of eight
 // sequences and four blocks, 3328 wide 295 / 272, 3584 wide 313 / 283, but 25 MB (3072 x 11648) cost 2 % there.  Not
@@ -59,7 +62,7 @@ bool has_row_major(const rdq_layer &l) {
 // wide, 6 sequences 320 / 337).
 int stream_from(const rdq_layer &l) {
   const double bytes = l.n_fp4 * (l.K * 0.5625) + l.n_fp8 * (l.K + 4.0) + l.n_fp16 * (l.K * 2.0);
-  if (!l.w_tiled) return bytes > 40e6 ? 1 : (bytes > 18e6 ? 9 : RDQ_MAX_GEMV_M + 1);
+  if (!l.w_tiled) return bytes > 22e6 ? 1 : (bytes > 12e6 ? 9 : RDQ_MAX_GEMV_M + 1);
   if (bytes > 40e6) return bytes > 80e6 ? 1 : 3;
   return bytes > 28e6 && !tiled_stages_x(8, l.K) ? (tiled_stages_x(7, l.K) ? 8 : 7) : 9;
 }
