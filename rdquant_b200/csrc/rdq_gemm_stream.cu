@@ -1077,12 +1077,17 @@ bool make_whole_plan(int n4, int n8, int n16, int M, int K, int cluster, StreamP
 // rows 11.2 us, now 7.6; 2560 -> 6144 16.5, 11.4; 4096 -> 2560 at 192 rows 14.6, 11.6).  Beyond, 7 % would be left.
 StreamPlan best_plan(int n4, int n8, int n16, int M, int K) {
   const bool fits = (n4 * 0.5625 + n8 + 2.0 * n16) * K < 150e6, few = M <= 64 && fits;
+  const int tiles = (n4 + 127) / 128 + (n8 + 127) / 128 + (n16 + 127) / 128;
   StreamPlan best = make_plan(n4, n8, n16, M, K);
   double least = few ? 1e30 : 0.88 * best.us;
   if (fits && M <= 256) {
-    for (int cluster = 1; cluster <= 4; cluster *= 2) {
+    for (int cluster = 4; cluster >= 1; cluster /= 2) {
       StreamPlan p;
-      if (!make_whole_plan(n4, n8, n16, M, K, cluster, &p) || p.us >= least) continue;
+      const bool can = make_whole_plan(n4, n8, n16, M, K, cluster, &p);
+      // Layers of a tile to every cluster of four whose slots do not fit beside the activations of 49 to 64 tokens: 12288 -> 4096 at
+      // 64 rows 19.0 us by clusters of two, 16.4 cut; 8192 -> 4096 15.6, 13.8; 6144 -> 4096 13.8, 13.4; 4096 -> 4096 12.0, 12.5.
+      if (few && !can && cluster == 4 && (K + 255) / 256 >= 4 && tiles <= clusters_at_once(4)) least = 0.85 * best.us;
+      if (!can || p.us >= least) continue;
       best = p;
       least = p.us;
     }

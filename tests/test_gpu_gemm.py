@@ -157,6 +157,7 @@ def test_wide_layers_of_few_rows_need_no_decoding(rows, shape, scratch):
     ((4096, 2048, 0, 4096), 64), ((13056, 6144, 256, 2560), 20), ((13056, 6144, 256, 2624), 64),
     ((2048, 384, 128, 2560), 20), ((640, 384, 0, 9792), 31), ((0, 0, 256, 8192), 40), ((0, 700, 0, 3008), 48),
     ((30000, 4000, 0, 8192), 33),        # 170 MB: cut tiles
+    ((2688, 1280, 128, 8192), 64), ((2688, 1280, 128, 4096), 64),  # no room for the slots of a cluster of four: cut tiles, clusters of two
     # the line to the decode GEMV: rows that it does not keep in shared memory (eight of 2816, seven it does)
     ((2560, 896, 128, 13568), 7), ((9600, 4864, 128, 2816), 8), ((9600, 4864, 128, 2816), 7),
     # block scales copied 8 bytes at a time: whole tiles, cut ones, two tiles of tokens
