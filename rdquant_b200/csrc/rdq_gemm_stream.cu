@@ -18,8 +18,8 @@
 // order: the result does not depend on timing (await_parts: those that leave, and who does their share).  A second kernel for these sums cost
 // 4-7 us per layer, and one CTA per tile adding them up to 13 us.
 //
-// Up to 64 tokens, or 256 where that is faster (best_plan), tiles are not cut: a tile has as many rows (8 to 128) as make all tiles cost the same bytes, and belongs
-// to one cluster of one, two or four CTAs that share its k.  A chunk is 256 k of any format then (one, two or four boxes).  The
+// Up to 64 tokens, or 256 where that is faster (best_plan), tiles are not cut: a tile has as many rows (8 to 128) as make all
+// tiles cost the same bytes, and belongs to one cluster of one, two or four CTAs that share its k.  A chunk is 256 k of any format then (one, two or four boxes).  The
 // CTAs of a cluster exchange FP32 sums through distributed shared memory (finish_in_cluster): each finishes a share of the tokens.
 // They run at the same time by construction, and no word in global memory is involved.
 //
@@ -89,7 +89,7 @@ struct StreamSched {
   int E[3];                 // end of each format's chunk range
   int nkb;                  // k blocks of 64
   int R[3];                 // rows per tile
-  int cluster;              // (whole tiles) CTAs that share a tile's k: E are tiles of rows then, bnd a cluster's first (tile, token tile)
+  int cluster;              // (whole tiles) CTAs that share a tile's k: E are tiles of rows then, bnd tiles, numbered token tile by token tile
   int G;                    // CTAs
   int bnd[kMaxCtas + 1];    // first chunk of each CTA
 };
@@ -99,10 +99,16 @@ struct Segment {
   int start;                  // global index of the tile's first chunk
 };
 // the same where `S` chunks of every tile are this CTA's, numbered through
+template <bool MANY>
 __device__ __forceinline__ Segment whole_segment_at(const StreamSched &s, int S, int chunk) {
   Segment g;
-  const int t = chunk / S, rt = t / s.mt;
-  g.m_tile = t - rt * s.mt;
+  const int t = chunk / S;
+  int rt = t;
+  g.m_tile = 0;
+  while (MANY && rt >= s.E[2]) {
+    rt -= s.E[2];
+    ++g.m_tile;
+  }
   g.fmt = rt < s.E[0] ? 0 : (rt < s.E[1] ? 1 : 2);
   g.row_tile = rt - (g.fmt == 0 ? 0 : s.E[g.fmt - 1]);
   g.start = t * S;
@@ -381,7 +387,7 @@ __device__ __forceinline__ void finish_alone(const StreamSched &sc, const Stream
     float o[16];
 #pragma unroll
     for (int e = 0; e < 16; ++e) o[e] = __uint_as_float(v[e]);
-    store_tokens<BF16>(sc, a, row, o, tok0 + t, dry ? 0 : min(16, ntok - t));
+    store_tokens<BF16>(sc, a, row, o, tok0 + t, dry ? 0 : 16);
     if (dry) break;
   }
 }
@@ -443,8 +449,10 @@ __device__ __forceinline__ void finish_in_cluster(StreamSmem &S, const StreamSch
   }
 }
 
-// NT: most tokens per tile (64 or 128).  WHOLE: every tile belongs to one CTA, a chunk has 256 k of any format (make_whole_plan)
-template <int NT, bool BF16, bool WHOLE>
+// NT: most tokens per tile (64 or 128).  WHOLE: every tile belongs to one CTA, a chunk has 256 k of any format (make_whole_plan).
+// MANY: of several token tiles; without it their arithmetic, which every role does ahead of its first chunk, is not there (decode
+// step of 32 rows 284 us with a division by their number, 277 with a loop, 269 without).
+template <int NT, bool BF16, bool WHOLE, bool MANY = false>
 __global__ void __launch_bounds__(kThreadBound<NT>, 1)
 gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_constant__ CUtensorMap w8map,
                    const __grid_constant__ CUtensorMap w16map, const __grid_constant__ CUtensorMap xmap,
@@ -467,7 +475,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
   const int lo = WHOLE ? sc.S[0] * static_cast<int>(rank) / sc.cluster : 0;
   const int own = WHOLE ? sc.S[0] * static_cast<int>(rank + 1) / sc.cluster - lo : 0;
   const int begin = sc.bnd[worker] * (WHOLE ? own : 1), end = sc.bnd[worker + 1] * (WHOLE ? own : 1);
-  auto seg_at = [&](int chunk, int to) { return WHOLE ? whole_segment_at(sc, own, chunk) : segment_at(sc, chunk, to); };
+  auto seg_at = [&](int chunk, int to) { return WHOLE ? whole_segment_at<MANY>(sc, own, chunk) : segment_at(sc, chunk, to); };
   auto wmap = [&](int fmt) { return fmt == 0 ? &w4map : (fmt == 1 ? &w8map : &w16map); };
   // the boxes of a chunk: one of 128 rows, or as many as 256 k take (those past K are left out)
   auto height_of = [&](int fmt) { return WHOLE ? sc.R[fmt] : 128; };
@@ -1175,13 +1183,14 @@ int launch_gemm_stream(const GemmArgs &g, void *workspace, size_t workspace_byte
   a.patience = gemm_test_timeout() == 2 ? 0 : kPatience;
   const StreamSched &sc = p.sc;
 
-  static const void *const fns[6] = {
+  static const void *const fns[8] = {
       reinterpret_cast<const void *>(gemm_stream_kernel<64, false, false>), reinterpret_cast<const void *>(gemm_stream_kernel<64, true, false>),
       reinterpret_cast<const void *>(gemm_stream_kernel<128, false, false>), reinterpret_cast<const void *>(gemm_stream_kernel<128, true, false>),
-      reinterpret_cast<const void *>(gemm_stream_kernel<64, false, true>), reinterpret_cast<const void *>(gemm_stream_kernel<64, true, true>)};
-  const int variant = (p.whole ? 4 : p.wide * 2) + (g.y_bf16 ? 1 : 0);
+      reinterpret_cast<const void *>(gemm_stream_kernel<64, false, true>), reinterpret_cast<const void *>(gemm_stream_kernel<64, true, true>),
+      reinterpret_cast<const void *>(gemm_stream_kernel<64, false, true, true>), reinterpret_cast<const void *>(gemm_stream_kernel<64, true, true, true>)};
+  const int variant = (p.whole ? (sc.mt > 1 ? 6 : 4) : p.wide * 2) + (g.y_bf16 ? 1 : 0);
   const void *fn = fns[variant];
-  static std::atomic<bool> attr_done[6][64];
+  static std::atomic<bool> attr_done[8][64];
   int dev = 0;
   RDQ_CUDA(cudaGetDevice(&dev));
   std::atomic<bool> *done = dev >= 0 && dev < 64 ? &attr_done[variant][dev] : nullptr;
