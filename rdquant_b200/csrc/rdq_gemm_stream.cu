@@ -394,7 +394,8 @@ __device__ __forceinline__ void finish_alone(const StreamSched &sc, const Stream
 
 // Tiles whose k the CTAs of a cluster share: epilogue warp q sends its 32 rows' sums of the tokens that another CTA
 // finishes to that CTA's warp q, waits for those of its own tokens and adds, in the order of the ranks.  `turn` counts the
-// tiles; two buffers take turns.  Layout of a buffer: [rank][four tokens][128 rows][4].
+// tiles in which the warp has rows, for its barriers complete a phase in those alone; two buffers take turns, `more` where
+// the buffer will be used again.  Layout of a buffer: [rank][four tokens][128 rows][4].
 template <bool BF16>
 __device__ __forceinline__ void finish_in_cluster(StreamSmem &S, const StreamSched &sc, const StreamArgs &a, const Row &row, uint32_t acc,
                                                   uint32_t r_ring, int tok0, int rank, int q, int lane, int turn, bool more, bool dry) {
@@ -700,8 +701,19 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
     if (!WHOLE) S.cut[1][q * 32 + lane] = row_of(a, seg_at(end - 1, end), 128, q * 32 + lane, true);
     Cursor d;
     bool first = true;
-    int turn = 0;
-    if (WHOLE && sc.cluster > 1) cluster_wait();
+    // Tiles in which this warp has rows, so far and in all.  Tiles get lower from format to format: the last ones of a token
+    // tile may have none, and the next token tile starts with high ones again.
+    int turn = 0, turns = 0;
+    if (WHOLE && sc.cluster > 1) {
+      const int with = q * 32 < sc.R[2] ? sc.E[2] : (q * 32 < sc.R[1] ? sc.E[1] : (q * 32 < sc.R[0] ? sc.E[0] : 0));
+      auto before = [&](int tile) {
+        int n = 0;
+        for (; MANY && tile >= sc.E[2]; tile -= sc.E[2]) n += with;
+        return n + min(tile, with);
+      };
+      turns = before(sc.bnd[worker + 1]) - before(sc.bnd[worker]);
+      cluster_wait();
+    }
     // (whole tiles) The first turn of the loop, while nothing is there to be stored, runs through without a wait, a store or
     // an arrival: it brings the code into the instruction caches, 2000 cycles that would be spent behind the last MMA.
     bool dry = WHOLE;
@@ -722,14 +734,14 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_const
       uint32_t v[2][16];
       if (WHOLE) {
         if (q * 32 < sc.R[g.fmt]) {  // (else no rows)
-          if (sc.cluster > 1) finish_in_cluster<BF16>(S, sc, a, row, acc, r_ring, tok0, static_cast<int>(rank), q, lane, turn, ck + 2 * own < end, dry);
+          if (sc.cluster > 1) finish_in_cluster<BF16>(S, sc, a, row, acc, r_ring, tok0, static_cast<int>(rank), q, lane, turn, turn + 2 < turns, dry);
           else finish_alone<BF16>(sc, a, row, acc, tok0, ntok, dry);
+          if (!dry) ++turn;
         }
         if (dry) {
           dry = false;
           continue;
         }
-        ++turn;
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&S.d_empty[d.i]));

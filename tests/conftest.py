@@ -68,3 +68,26 @@ def golden_layer_torch(case: dict, device="cpu"):
 @pytest.fixture(scope="session")
 def layers():
     return golden_layers()
+
+
+def streaming_tiles(fd, rows, dtype):
+    """What a linear of so many rows runs on, told by the words and the scratch it asks for: "cut" or "whole" tiles of the
+    streaming GEMM, or None for another kernel."""
+    import ctypes
+
+    import torch
+
+    from rdquant_b200 import _lib
+    from test_capi_symbols import _Layer
+
+    p = lambda key: None if fd.get(key) is None or fd[key].numel() == 0 else fd[key].data_ptr()
+    layer = _Layer(n_fp4=fd["n_fp4"], n_fp8=fd["n_fp8"], n_fp16=fd["n_fp16"], K=fd["k"], w_fp4_global_scale=1.0, w_fp4=p("w_fp4_q"),
+                   w_fp4_scales=p("w_fp4_scales"), w_fp8=p("w_fp8_q"), w_fp8_scales=p("w_fp8_scales"), w_fp16=p("w_fp16"),
+                   w_tiled=p("w_tiled"), perm=p("perm"), inv_perm=p("inv_perm"), gemv_ws=p("workspace"), gemv_counters=p("tile_counters"))
+    bf16 = int(dtype == torch.bfloat16)
+    if _lib.lib().rdq_linear_uses_words(ctypes.byref(layer), rows, bf16):
+        return "cut"
+    need = ctypes.c_size_t(0)
+    assert _lib.lib().rdq_linear_workspace_size(ctypes.byref(layer), rows, bf16, ctypes.byref(need)) == 0
+    rounded = (2 * rows * fd["k"] + 255) // 256 * 256 if bf16 else 0  # bf16 rows as f16
+    return "whole" if need.value == rounded + 256 else None

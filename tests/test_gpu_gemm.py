@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 import torch
 
-from conftest import ORDER, golden_layer_torch
+from conftest import ORDER, golden_layer_torch, streaming_tiles
 from oracle import oracle_np as onp
 from rdquant_b200 import _lib, rdquant_cuda
 from rdquant_b200.fused_gemv_pack import pack_for_fused_gemv
@@ -168,6 +168,10 @@ def test_wide_layers_of_few_rows_need_no_decoding(rows, shape, scratch):
 ])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_streaming_gemm_tiles(shape, rows, dtype):
+    _check_streaming_gemm(shape, rows, dtype)
+
+
+def _check_streaming_gemm(shape, rows, dtype, tiles=None):
     """The streaming GEMM through the module, against 64-bit sums over the dequantised weight (test_gpu_dequant.py: bit-exact)."""
     n4, n8, n16, k = shape
     splits = dict(zip(ORDER, shape[:3]))
@@ -175,6 +179,8 @@ def test_streaming_gemm_tiles(shape, rows, dtype):
     gen = torch.Generator().manual_seed(rows)
     layer["bias"] = (torch.randn(n4 + n8 + n16, generator=gen) * 0.5).half()
     mod = FusedMixedLinear.from_layer_data(layer, splits, k, "cuda")
+    if tiles:
+        assert streaming_tiles(mod._fd(), rows, dtype) == tiles
     x = torch.randn(rows, k, generator=gen).to(dtype).cuda()
     y = mod(x)
     assert y.dtype == dtype and all(torch.equal(mod(x), y) for _ in range(3))
@@ -186,3 +192,16 @@ def test_streaming_gemm_tiles(shape, rows, dtype):
     err = (y.double() - ref).abs()
     half = 2.0 ** (-11 if dtype == torch.float16 else -8)
     assert float((err - 1.01 * half * ref.abs()).max() / ref.abs().max()) < 2e-5
+
+
+@pytest.mark.parametrize("shape,rows", [
+    # clusters of two with tiles FP16, FP16, NVFP4 and FP16, NVFP4, NVFP4 of 32 and 120 rows; FP8 of 48 rows and NVFP4 of 96
+    ((4224, 2176, 128, 1536), 134), ((5376, 896, 128, 1536), 134), ((6784, 128, 0, 1408), 177),
+    # clusters of four, five tiles each
+    ((7936, 1408, 128, 1024), 85), ((8192, 1152, 128, 896), 65),
+])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_streaming_gemm_clusters_across_token_tiles(shape, rows, dtype):
+    """Clusters whose tiles reach from the low ones at the end of a token tile into the high ones of the next: warps without
+    rows in one tile have some two tiles later."""
+    _check_streaming_gemm(shape, rows, dtype, "whole")
