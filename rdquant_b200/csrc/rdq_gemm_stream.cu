@@ -932,7 +932,10 @@ struct StreamPlan {
   StreamSched sc;
   int wide, nw, smem;  // wide: the variant for more than 64 tokens per tile
   int whole, w_pitch, s_pitch;
-  double us;  // estimated time
+  double us;     // estimated time
+  double share;  // (cut tiles) a CTA's cycles
+  int parts;     // (cut tiles) CTAs that share a tile, at most
+  int each;      // (whole tiles) tiles of a cluster, at most
 };
 
 // Token tiles of equal width; a chunk costs what bounds it: its bytes at the SM's share of the HBM
@@ -987,6 +990,9 @@ StreamPlan make_plan(int n4, int n8, int n16, int M, int K) {
   for (int f = 0; f < 3; ++f)
     if (n[f]) parts = std::max(parts, std::ceil(s.S[f] * u[f] / share));
   p.us = 7.6 + 0.672e-3 * share + 0.22 * parts + 0.32 * M / 128;
+  p.share = share;
+  p.parts = static_cast<int>(parts);
+  p.each = 0;
   p.nw = std::min(p.nw, 8);
   p.smem = 1024 + xb + p.nw * (kChunkBytes + kScaleBytes);
   p.whole = 0;
@@ -1068,6 +1074,9 @@ bool make_whole_plan(int n4, int n8, int n16, int M, int K, int cluster, StreamP
   const int each = (items + s.G - 1) / s.G;
   p.wide = 0;
   p.whole = 1;
+  p.each = each;
+  p.share = 0;
+  p.parts = 0;
   p.w_pitch = std::max({n4 ? s.R[0] : 0, n8 ? 2 * s.R[1] : 0, n16 ? 4 * s.R[2] : 0}) * 128;
   p.s_pitch = s.R[0] * 16;
   const int xb = kStages<64> * kBlocks<64> * s.nt * 128 + (cluster > 1 ? std::min(2, each) * s.nt * 512 : 0);
@@ -1084,11 +1093,26 @@ bool make_whole_plan(int n4, int n8, int n16, int M, int K, int cluster, StreamP
   return true;
 }
 
-// Up to 64 tokens tiles are whole: the CTAs that share a cut one spend 7000 cycles behind the last MMA (partial sums, fence,
+// What whole tiles of up to 64 tokens take more than cut ones, in microseconds.  Whole ones cost by their steps of 256 k and
+// by the exchange, cut ones by a CTA's share and by the parts of a tile.  Where a row of block scales is no
+// multiple of 16 bytes the warp that copies them 8 bytes at a time bounds both, whole tiles by their rows of NVFP4.
+// Fitted to the difference of both on 190 layers (1 to 150 MB, K 1024 to 16384, 50 to 90 % NVFP4) at 9 to 64 rows: of 890
+// points the choice is 0.04 % behind the faster on average, 5 % at worst; always whole was 0.8 % behind, 23 % at worst.
+double whole_minus_cut(const StreamPlan &whole, const StreamPlan &cut, int n4, int K) {
+  const StreamSched &s = whole.sc;
+  const bool narrow = n4 > 0 && K % 256 != 0;
+  const int steps = whole.each * ((s.S[0] + s.cluster - 1) / s.cluster);
+  const double exchange = s.cluster == 1 ? 0.0 : (s.cluster == 2 ? 1.5 : 1.5 * whole.each);
+  return steps * (narrow ? 0.143 * ((s.R[0] + 31) / 32) : 0.32) + exchange -
+         (1.2 + (narrow ? 0.74e-3 : 0.4e-3) * cut.share + 0.09 * cut.parts + 0.02 * s.nt);
+}
+
+// Up to 64 tokens: the CTAs that share a cut tile spend 7000 cycles behind the last MMA (partial sums, fence,
 // arrival, sums, each a round trip to L2 by code that is run once), a cluster 1700 and a CTA alone 1000.  32 rows, calls
-// one after another, us before and now: 2560 -> 6144 10.6, 8.3; 4096 -> 2560 10.6, 7.7; 9728 -> 2560 12.5, 10.6; 1024 -> 1024 8.0,
-// 6.0; 8192 -> 8192 15.5, 13.7.  Above 200 MB the tail is short beside the rest and cut tiles use the MMA's 128 rows better (8192 ->
-// 57344 at 48 rows 73.6, 76.2) unless there are few tokens (9 rows 61.1, 58.4).
+// one after another, us of cut tiles and of whole ones: 2560 -> 6144 10.6, 8.3; 4096 -> 2560 10.6, 7.7; 9728 -> 2560 12.5, 10.6;
+// 1024 -> 1024 8.0, 6.0; 8192 -> 8192 15.5, 13.7.  But a tile that no cluster of four has room for, of a long K, takes
+// longer than its shares: 13312 -> 4608 15.4, 17.6; 8192 -> 4224 13.2, 13.7; 12288 -> 4096 at 64 rows 16.0, 18.6.  From 150 MB on
+// tiles are cut: the tail is short beside the rest, and they use the MMA's 128 rows (8192 -> 57344, 292 MB, at 48 rows 73.6, 76.2).
 //
 // More tokens come in tiles of 64, each work of its own: the weights are converted for each, where cut tiles convert them for 128
 // at a time, so that it pays where a CTA's share is small beside the tail.  The estimates decide; the margin covers theirs
@@ -1096,23 +1120,21 @@ bool make_whole_plan(int n4, int n8, int n16, int M, int K, int cluster, StreamP
 // cut tiles and the GEMM over decoded weights, 20 % less time at 72 to 128 rows and 12 % at 160 to 256 (2560 -> 1024 at 128
 // rows 11.2 us, now 7.6; 2560 -> 6144 16.5, 11.4; 4096 -> 2560 at 192 rows 14.6, 11.6).  Beyond, 7 % would be left.
 StreamPlan best_plan(int n4, int n8, int n16, int M, int K) {
-  const bool fits = (n4 * 0.5625 + n8 + 2.0 * n16) * K < 150e6, few = M <= 64 && fits;
-  const int tiles = (n4 + 127) / 128 + (n8 + 127) / 128 + (n16 + 127) / 128;
-  StreamPlan best = make_plan(n4, n8, n16, M, K);
-  double least = few ? 1e30 : 0.88 * best.us;
-  if (fits && M <= 256) {
-    for (int cluster = 4; cluster >= 1; cluster /= 2) {
-      StreamPlan p;
-      const bool can = make_whole_plan(n4, n8, n16, M, K, cluster, &p);
-      // Layers of a tile to every cluster of four whose slots do not fit beside the activations of 49 to 64 tokens: 12288 -> 4096 at
-      // 64 rows 19.0 us by clusters of two, 16.4 cut; 8192 -> 4096 15.6, 13.8; 6144 -> 4096 13.8, 13.4; 4096 -> 4096 12.0, 12.5.
-      if (few && !can && cluster == 4 && (K + 255) / 256 >= 4 && tiles <= clusters_at_once(4)) least = 0.85 * best.us;
-      if (!can || p.us >= least) continue;
-      best = p;
-      least = p.us;
-    }
+  const StreamPlan cut = make_plan(n4, n8, n16, M, K);
+  if (M > 256 || (n4 * 0.5625 + n8 + 2.0 * n16) * K >= 150e6) return cut;
+  StreamPlan best = cut;
+  double least = M <= 64 ? 1e30 : 0.88 * cut.us;
+  for (int cluster = 4; cluster >= 1; cluster /= 2) {
+    StreamPlan p;
+    if (!make_whole_plan(n4, n8, n16, M, K, cluster, &p)) continue;
+    // (up to 64 tokens a further tile costs a cluster of four a microsecond that the estimate does not have: 8064 -> 9984 at
+    // 24 rows, three each, 24.6 us, alone 21.3)
+    const double us = p.us + (M <= 64 && cluster == 4 ? p.each - 1 : 0);
+    if (us >= least) continue;
+    best = p;
+    least = us;
   }
-  return best;
+  return best.whole && M <= 64 && whole_minus_cut(best, cut, n4, K) > 0 ? cut : best;
 }
 
 // the plans of the last few thousand (layer shape, rows) pairs of this thread

@@ -205,3 +205,17 @@ def test_streaming_gemm_clusters_across_token_tiles(shape, rows, dtype):
     """Clusters whose tiles reach from the low ones at the end of a token tile into the high ones of the next: warps without
     rows in one tile have some two tiles later."""
     _check_streaming_gemm(shape, rows, dtype, "whole")
+
+
+@pytest.mark.parametrize("shape,rows,tiles", [
+    # a tile that no cluster of four has room for, of a long K: cut, unless there are more tiles than that
+    ((3072, 1408, 128, 13312), 24, "cut"), ((2816, 1280, 128, 8192), 9, "cut"), ((2688, 1280, 128, 12288), 64, "cut"),
+    ((2688, 1280, 128, 12288), 48, "whole"), ((5504, 2560, 128, 8192), 33, "whole"), ((12672, 6144, 128, 5120), 9, "cut"),
+    # block scales copied 8 bytes at a time, where both cost more, and 4
+    ((2816, 1280, 128, 13184), 24, "cut"), ((3456, 1664, 128, 11904), 33, "whole"), ((6656, 3200, 128, 8064), 24, "whole"),
+    ((4352, 2048, 128, 6464), 24, "whole"),
+])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_streaming_gemm_tiles_of_up_to_64_rows(shape, rows, tiles, dtype):
+    """Whole tiles and cut ones, each where it is the faster."""
+    _check_streaming_gemm(shape, rows, dtype, tiles)
