@@ -48,23 +48,39 @@ bool has_row_major(const rdq_layer &l) {
 //   48 MB (8192 x 8192)   2 rows 11.9 / 15.7, 15.8 / 14.8     4 rows 18.3 / 16.0, 19.9 / 15.0
 //   97 MB (16384 x 8192)  1 row  19.6 / 22.8, 27.8 / 21.7     4 rows 31.5 / 23.2, 36.5 / 22.1
 // The row-major GEMV of layers without a tiled layout starts at 1.9 us where the streaming GEMM takes 6 to 8 (2 MB,
-// 3001 x 1024: 2.6 / 6.3 us at one row).  With leave to read weights early or without:
+// 3001 x 1024: 2.6 / 6.3 us at one row).  With leave to read weights early or without, f16 rows:
 //   12 MB (2001 x 8192)   1 row 10.0 / 10.8    8 rows 10.2 / 10.8    16 rows 11.2 / 10.8
 //   15 MB (5001 x 4096)   1 row 10.6 / 10.5    8 rows 11.4 / 10.5    16 rows 12.7 / 10.5
 //   19 MB (3072 x 8576)   1 row 11.5 / 12.1    8 rows 12.0 / 12.1    16 rows 13.0 / 12.2
 //   22 MB (12001 x 2560)  1 row 11.9 / 10.2    8 rows 12.7 / 10.2    16 rows 14.3 / 10.3
-// It keeps up to eight rows up to 22 MB, more of them up to 12; of 22 layers 9001 x 3008 (19 MB) fares worst, 10.6 / 12.0
-// at nine rows.
-// Seven and eight rows that the GEMV does not keep in shared memory go to the streaming GEMM from 28 MB on: 37 MB
-// (3584 x 14336) 15.5 / 13.3 us, 30 MB (12672 x 3328) 0.83 of the time, 26 MB (5120 x 7168) 1.1; decode steps of eight
+// It keeps up to eight rows up to 22 MB, more of them up to 12.  bf16 rows, which the GEMV rounds itself and the GEMM has
+// rounded by a launch before it, stay up to 24 and 18 MB (3341 x 9216, 22 MB, 8 rows 13.2 / 14.5; 5309 x 3520, 14 MB, 9 rows
+// 12.1 / 13.1).  The streaming GEMM's narrow copies of block scales (8 bytes where K is no multiple of 256, 4 where it is
+// none of 128) keep few rows with the GEMV up to 40 MB, bf16 rows and K of no multiple of 128, unless K is below 2048: time of the GEMM over
+// the GEMV's at four rows, f16 and bf16, 26 MB (3659 x 9664) 1.06, 1.40; 40 MB (4677 x 11712) 1.14, 1.50; 26 MB (12227 x 2944) 0.95,
+// 1.21; but 30 MB (8613 x 4864) 0.75, 0.97 and 36 MB (33535 x 1472) 0.82, 0.96.  Of 56 layers the f16 rows of 4027 x 5504 (16 MB)
+// fare worst, 1.25 at nine.
+// Seven and eight rows that the GEMV does not keep in shared memory go to the streaming GEMM from 28 MB on where its
+// tiles are whole and its copies wide, or K is below 8000: 37 MB (3584 x 14336) 15.5 / 13.3 us, 38 MB (4096 x 12288) 16.5 / 12.1,
+// 30 MB (12672 x 3328) 0.83 of the time, 26 MB (5120 x 7168) 1.1; but 37 MB (3072 x 16000) 14.9 / 16.1, with bf16 rows
+// 17.6 / 22.4, and 35 MB (4224 x 11264, cut tiles) with bf16 rows 16.5 / 18.0.  Of 38 layers between 28 and 40 MB 8 % less time,
+// at worst 10 % more (bf16 rows, 7040 x 5760); decode steps of eight
 // sequences and four blocks, 3328 wide 295 / 272, 3584 wide 313 / 283, but 25 MB (3072 x 11648) cost 2 % there.  Not
 // fewer rows: a step whose norms still run inside the GEMV lost 5 % to a streaming down projection in between (3584
 // wide, 6 sequences 320 / 337).
-int stream_from(const rdq_layer &l) {
+int stream_from(const rdq_layer &l, int x_type) {
   const double bytes = l.n_fp4 * (l.K * 0.5625) + l.n_fp8 * (l.K + 4.0) + l.n_fp16 * (l.K * 2.0);
-  if (!l.w_tiled) return bytes > 22e6 ? 1 : (bytes > 12e6 ? 9 : RDQ_MAX_GEMV_M + 1);
+  const bool wide = l.K % 256 == 0;
+  if (!l.w_tiled) {
+    const bool bf16 = x_type == RDQ_BF16;
+    const double few = wide || l.K < 2048 || (!bf16 && l.K % 128 == 0) ? (bf16 ? 24e6 : 22e6) : 40e6;
+    if (bytes > few) return 1;
+    return bytes > (bf16 ? 18e6 : 12e6) ? 9 : RDQ_MAX_GEMV_M + 1;
+  }
   if (bytes > 40e6) return bytes > 80e6 ? 1 : 3;
-  return bytes > 28e6 && !tiled_stages_x(8, l.K) ? (tiled_stages_x(7, l.K) ? 8 : 7) : 9;
+  if (bytes <= 28e6 || tiled_stages_x(8, l.K)) return 9;
+  if (l.K >= 8000 && (!wide || gemm_stream_uses_words(l.n_fp4, l.n_fp8, l.n_fp16, 8, l.K))) return 9;
+  return tiled_stages_x(7, l.K) ? 8 : 7;
 }
 
 // Few rows: the decode GEMV (tiled layout, else the any-shape kernel), or the streaming GEMM from
@@ -94,7 +110,7 @@ bool stream_beats_dense(const rdq_layer &l, int M, int x_type) {
 
 Path path_of(const rdq_layer &l, int M, int x_type) {
   const bool can_stream = gemm_stream_takes(l.K) && has_row_major(l) && (l.perm || !l.inv_perm);
-  if (can_stream && M >= stream_from(l) && (!gemm_dense_takes(l.K) || stream_beats_dense(l, M, x_type))) return Path::kStream;
+  if (can_stream && M >= stream_from(l, x_type) && (!gemm_dense_takes(l.K) || stream_beats_dense(l, M, x_type))) return Path::kStream;
   if (M <= RDQ_MAX_GEMV_M) return l.w_tiled ? Path::kGemvTiled : Path::kGemvGeneric;
   if (gemm_dense_takes(l.K) && has_row_major(l)) return Path::kGemm;
   return l.w_tiled ? Path::kPanelsTiled : Path::kPanelsGeneric;

@@ -85,3 +85,27 @@ def test_small_layers_without_tiles_stay_on_the_decode_kernel(n4, n8, k, decode_
         for rows in range(1, 20):
             assert _lib.lib().rdq_linear_workspace_size(ctypes.byref(layer), rows, x_type, ctypes.byref(need)) == 0
             assert (need.value == 0) == (rows <= decode_rows), (rows, need.value)
+
+
+@pytest.mark.parametrize("n4,n8,k,tiled,x_type,first", [
+    # row-major layers: f16 and bf16 rows between the lines, K of multiples of 256, 128 and 64, and a short K
+    (5001, 2503, 2560, False, 0, 9), (5001, 2503, 2560, False, 1, 17),          # 14 MB
+    (7001, 3503, 4096, False, 0, 1), (7001, 3503, 4096, False, 1, 1),           # 30 MB
+    (6001, 3003, 4096, False, 0, 1), (6001, 3003, 3968, False, 1, 1 + 8),       # 26, 25 MB
+    (8192, 4035, 2944, False, 0, 1), (8192, 4035, 2944, False, 1, 9),           # 25 MB
+    (2451, 1208, 9664, False, 0, 9), (2451, 1208, 9664, False, 1, 9),           # 25 MB
+    (22468, 11067, 1472, False, 0, 1), (22468, 11067, 1472, False, 1, 1),       # 35 MB
+    # tiled ones whose rows stay out of the decode kernel's shared memory: narrow copies of block scales of a long and a short K
+    (2048, 1024, 16000, True, 0, 9), (2048, 1024, 16000, True, 1, 9),           # 35 MB
+    (10240, 5120, 2944, True, 0, 8), (4864, 2048, 5760, True, 0, 9),            # 32, 28 MB
+])
+def test_first_row_of_the_gemm(n4, n8, k, tiled, x_type, first):
+    """The fewest rows that leave the decode kernel, told by the scratch beyond that for rounded bf16 rows."""
+    layer = _Layer(n_fp4=n4, n_fp8=n8, n_fp16=0, K=k, w_fp4_global_scale=1.0, w_fp4=4096, w_fp4_scales=4096, w_fp8=4096,
+                   w_fp8_scales=4096, w_fp16=None, w_tiled=4096 if tiled else None, perm=4096, inv_perm=4096, gemv_ws=4096,
+                   gemv_counters=4096)
+    need = ctypes.c_size_t(0)
+    for rows in range(1, 20):
+        assert _lib.lib().rdq_linear_workspace_size(ctypes.byref(layer), rows, x_type, ctypes.byref(need)) == 0
+        rounded = (2 * rows * k + 255) // 256 * 256 if x_type else 0
+        assert (need.value not in (0, rounded)) == (rows >= first), (rows, need.value)
