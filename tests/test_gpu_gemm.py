@@ -149,38 +149,41 @@ def test_wide_layers_of_few_rows_need_no_decoding(rows, shape, scratch):
     assert onp.rel_err(y.cpu()[some].float().numpy(), ref) < TOL
 
 
-@pytest.mark.parametrize("shape,rows", [
+@pytest.mark.parametrize("shape,rows,tiles", [
     # whole tiles, a CTA each: K of less than a chunk, of no whole chunk, groups that end inside a tile
-    ((64, 32, 16, 64), 17), ((0, 0, 128, 192), 9), ((300, 130, 20, 576), 33), ((37, 0, 5, 1344), 24),
-    ((60800, 20480, 5120, 256), 20),     # five tiles each
+    ((64, 32, 16, 64), 17, "whole"), ((0, 0, 128, 192), 9, "whole"), ((300, 130, 20, 576), 33, "whole"), ((37, 0, 5, 1344), 24, "whole"),
+    ((60800, 20480, 5120, 256), 20, "whole"),     # five tiles each
     # clusters of two and four: chunks of k dealt out unevenly, several tiles each (buffers used again)
-    ((4096, 2048, 0, 4096), 64), ((13056, 6144, 256, 2560), 20), ((13056, 6144, 256, 2624), 64),
-    ((2048, 384, 128, 2560), 20), ((640, 384, 0, 9792), 31), ((0, 0, 256, 8192), 40), ((0, 700, 0, 3008), 48),
-    ((30000, 4000, 0, 8192), 33),        # 170 MB: cut tiles
-    ((2688, 1280, 128, 8192), 64), ((2688, 1280, 128, 4096), 64),  # no room for the slots of a cluster of four: cut tiles, clusters of two
+    ((4096, 2048, 0, 4096), 64, "whole"), ((13056, 6144, 256, 2560), 20, "whole"), ((13056, 6144, 256, 2624), 64, "whole"),
+    ((2048, 384, 128, 2560), 20, "whole"), ((640, 384, 0, 9792), 31, "whole"), ((0, 0, 256, 8192), 40, "whole"), ((0, 700, 0, 3008), 48, "whole"),
+    ((30000, 4000, 0, 8192), 33, "cut"),          # 170 MB
+    # no room for the slots of a cluster of four: cut tiles, clusters of two
+    ((2688, 1280, 128, 8192), 64, "cut"), ((2688, 1280, 128, 4096), 64, "whole"),
     # the line to the decode GEMV: rows that it does not keep in shared memory (eight of 2816, seven it does)
-    ((2560, 896, 128, 13568), 7), ((9600, 4864, 128, 2816), 8), ((9600, 4864, 128, 2816), 7),
-    # block scales copied 8 bytes at a time: whole tiles, cut ones, two tiles of tokens
-    ((300, 130, 20, 896), 33), ((1280, 640, 128, 2176), 100), ((1280, 640, 128, 2176), 140),
-    # whole tiles of more than 64 tokens: clusters of one, two and four; tiles of tokens that are hardly filled; several tiles a CTA
-    ((1280, 640, 128, 640), 65), ((3072, 896, 128, 4096), 128), ((640, 384, 0, 2560), 129), ((300, 130, 20, 2624), 200),
-    ((4096, 1920, 128, 2560), 193), ((0, 0, 256, 8192), 256), ((13056, 6144, 256, 2560), 66), ((640, 384, 0, 2560), 257),
+    ((2560, 896, 128, 13568), 7, "whole"), ((9600, 4864, 128, 2816), 8, "whole"), ((9600, 4864, 128, 2816), 7, None),
+    # block scales copied 8 bytes at a time: whole tiles, one tile of tokens and several
+    ((300, 130, 20, 896), 33, "whole"), ((1280, 640, 128, 2176), 100, "whole"), ((1280, 640, 128, 2176), 140, "whole"),
+    # whole tiles of more than 64 tokens: clusters of one, two and four; tiles of tokens that are hardly filled
+    ((1280, 640, 128, 640), 65, "whole"), ((3072, 896, 128, 4096), 128, "whole"), ((640, 384, 0, 2560), 129, "whole"),
+    ((300, 130, 20, 2624), 200, "whole"), ((0, 0, 256, 8192), 256, "whole"),
+    # cut ones where those are the faster, and beyond 256 rows; there small layers are decoded first
+    ((4096, 1920, 128, 2560), 193, "cut"), ((13056, 6144, 256, 2560), 66, "cut"), ((1280, 640, 128, 4096), 300, "cut"),
+    ((640, 384, 0, 2560), 257, None),
 ])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-def test_streaming_gemm_tiles(shape, rows, dtype):
-    _check_streaming_gemm(shape, rows, dtype)
+def test_streaming_gemm_tiles(shape, rows, tiles, dtype):
+    _check_streaming_gemm(shape, rows, dtype, tiles)
 
 
-def _check_streaming_gemm(shape, rows, dtype, tiles=None):
-    """The streaming GEMM through the module, against 64-bit sums over the dequantised weight (test_gpu_dequant.py: bit-exact)."""
+def _check_streaming_gemm(shape, rows, dtype, tiles):
+    """The streaming GEMM through the module, with the tiles that are meant, against 64-bit sums over the dequantised weight (test_gpu_dequant.py: bit-exact)."""
     n4, n8, n16, k = shape
     splits = dict(zip(ORDER, shape[:3]))
     layer = random_packed_layer(n4, n8, n16, k, seed=k + rows)
     gen = torch.Generator().manual_seed(rows)
     layer["bias"] = (torch.randn(n4 + n8 + n16, generator=gen) * 0.5).half()
     mod = FusedMixedLinear.from_layer_data(layer, splits, k, "cuda")
-    if tiles:
-        assert streaming_tiles(mod._fd(), rows, dtype) == tiles
+    assert streaming_tiles(mod._fd(), rows, dtype) == tiles
     x = torch.randn(rows, k, generator=gen).to(dtype).cuda()
     y = mod(x)
     assert y.dtype == dtype and all(torch.equal(mod(x), y) for _ in range(3))

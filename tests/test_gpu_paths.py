@@ -5,7 +5,7 @@ import pytest
 import torch
 import torch.nn.functional as F
 
-from conftest import ORDER
+from conftest import ORDER, streaming_tiles
 from oracle import oracle_np as onp
 from rdquant_b200 import _lib
 from rdquant_b200 import rdquant_cuda as rc
@@ -241,16 +241,20 @@ def test_silu_mul_shares(rows, f):
     assert bool(((out.double() - ref).abs() <= 2.1 * 2.0 ** -11 * ref.abs() + 2.0 ** -25 * (u.abs() + 1)).all())
 
 
-@pytest.mark.parametrize("shape,rows", [
-    ((1280, 896, 128, 1088), 17), ((1280, 896, 128, 1088), 64), ((300, 130, 20, 576), 100), ((0, 640, 128, 4096), 129),
-    ((0, 0, 256, 8192), 40),         # tiles shared by many CTAs
-    ((2048, 384, 128, 2560), 1280), ((600, 303, 100, 336), 700),  # the decoded-once GEMM, tiles split along k
+@pytest.mark.parametrize("shape,rows,tiles", [
+    ((1280, 896, 128, 1088), 17, "whole"), ((1280, 896, 128, 1088), 64, "whole"), ((300, 130, 20, 576), 100, "whole"),
+    ((0, 640, 128, 4096), 129, "whole"), ((0, 0, 256, 8192), 40, "whole"),  # (of one cluster: nobody may leave)
+    # cut tiles: up to 64 tokens, shared by up to thirteen CTAs, and more of them, in one and several tiles of tokens
+    ((2816, 1280, 128, 8192), 9, "cut"), ((2688, 1280, 128, 8192), 64, "cut"), ((13056, 6144, 256, 2560), 66, "cut"),
+    ((4096, 1920, 128, 2560), 193, "cut"), ((3000, 700, 70, 2560), 257, "cut"), ((1280, 640, 128, 4096), 300, "cut"),
+    ((2048, 384, 128, 2560), 1280, None), ((600, 303, 100, 336), 700, None),  # the decoded-once GEMM, tiles split along k
 ])
-def test_shared_tiles_do_not_need_their_ctas_at_the_same_time(shape, rows):
+def test_shared_tiles_do_not_need_their_ctas_at_the_same_time(shape, rows, tiles):
     """CTAs that leave instead of waiting for the others of a tile: the ones that come last do its whole,
     with the same result bit for bit, and nothing is left behind for the next call."""
     layer = random_packed_layer(*shape, seed=rows)
     mod = FusedMixedLinear.from_layer_data(layer, dict(zip(ORDER, shape[:3])), shape[3], "cuda")
+    assert streaming_tiles(mod._fd(), rows, torch.float16) == tiles
     x = torch.randn(rows, shape[3], generator=torch.Generator().manual_seed(rows)).half().cuda()
     y = mod(x)
     _lib.lib().rdq_gemm_test_timeout(2)
@@ -263,13 +267,19 @@ def test_shared_tiles_do_not_need_their_ctas_at_the_same_time(shape, rows):
     rc.check_gemm_status("cuda")
 
 
-@pytest.mark.parametrize("rows", [40, 120])
-def test_one_layer_on_several_streams(rows):
+@pytest.mark.parametrize("shape,rows,tiles", [
+    ((1280, 896, 128, 1088), 40, "whole"), ((1280, 896, 128, 1088), 120, "whole"),
+    ((2816, 1280, 128, 8192), 40, "cut"), ((1280, 640, 128, 4096), 300, "cut"),  # with counting words of the stream, or the capture
+])
+def test_one_layer_on_several_streams(shape, rows, tiles):
     """Calls of one layer that overlap: three streams at once, and a captured call replayed beside them."""
-    layer = random_packed_layer(1280, 896, 128, 1088, seed=21)
-    mod = FusedMixedLinear.from_layer_data(layer, dict(zip(ORDER, (1280, 896, 128))), 1088, "cuda")
+    k = shape[3]
+    layer = random_packed_layer(*shape, seed=21)
+    mod = FusedMixedLinear.from_layer_data(layer, dict(zip(ORDER, shape[:3])), k, "cuda")
+    assert streaming_tiles(mod._fd(), rows, torch.float16) == tiles
     gen = torch.Generator().manual_seed(rows)
-    xs = [torch.randn(rows, 1088, generator=gen).half().cuda() for _ in range(4)]
+    xs = [torch.randn(rows, k, generator=gen).half().cuda() for _ in range(4)]
+    _lib.torch_ext().drop_words()
     refs = [mod(x) for x in xs]
     streams = [torch.cuda.Stream() for _ in xs]
     graph = torch.cuda.CUDAGraph()
@@ -288,6 +298,8 @@ def test_one_layer_on_several_streams(rows):
         assert torch.equal(y, refs[i % 3])
     assert all(torch.equal(y, refs[3]) for y in captured)
     rc.check_gemm_status("cuda")
+    # (a set of words for the stream of the first calls, the three streams, and the capture until a later call finds it over)
+    assert _lib.torch_ext().drop_words() == (4 if tiles == "cut" else 0)
 
 
 @pytest.mark.parametrize("k", [512, 1040])

@@ -6,7 +6,7 @@ import ctypes
 import pytest
 import torch
 
-from conftest import ORDER
+from conftest import ORDER, streaming_tiles
 from oracle import oracle_np as onp
 from rdquant_b200 import _lib, rdquant_cuda
 from rdquant_b200.fused_gemv_pack import pack_for_fused_gemv
@@ -83,16 +83,22 @@ def test_gemm_timeout_is_reported_and_cleared():
     assert onp.rel_err(y_again.cpu().float().numpy(), ref) < 2e-3
 
 
-@pytest.mark.parametrize("rows", [32, 100])
-def test_streaming_gemm_timeout_is_reported_and_cleared(rows):
+@pytest.mark.parametrize("shape,rows,tiles", [
+    ((256, 128, 64, 1024), 32, "whole"), ((256, 128, 64, 1024), 100, "whole"),
+    ((2816, 1280, 128, 8192), 9, "cut"), ((1280, 640, 128, 4096), 300, "cut"),  # those count
+])
+def test_streaming_gemm_timeout_is_reported_and_cleared(shape, rows, tiles):
     """The GEMM a module call takes for a few rows: its status is reported, and the counts of its launches,
     which a launch that gave up leaves behind, do not outlive the report."""
-    layer, splits, k, _ = _layer(seed=6)
+    layer, splits, k, _ = _layer(shape, seed=6)
     lib = _lib.lib()
     mod = FusedMixedLinear.from_layer_data(layer, splits, k, "cuda")
+    assert streaming_tiles(mod._fd(), rows, torch.float16) == tiles
+    _lib.torch_ext().drop_words()
     x = torch.randn(rows, k, generator=torch.Generator().manual_seed(4)).half().cuda()
     y_ok = mod(x)
     rdquant_cuda.check_gemm_status(x.device)
+    assert _lib.torch_ext().drop_words() == (tiles == "cut"), "a set of words was handed out where the call counts"
     lib.rdq_gemm_test_timeout(1)
     try:
         mod(x)
