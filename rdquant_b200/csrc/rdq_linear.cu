@@ -96,7 +96,8 @@ int stream_from(const rdq_layer &l, int x_type) {
 // one on these layers (above 512 rows without 16384 x 8192, where the power cap decides), 31 % at worst (1024 x 16384
 // at 2048 f16 rows, 17 % at 1536), elsewhere up to 12 %; on 3584 x 2048, 13824 x 3584, 5120 x 5120, 3072 x 12288
 // and 2048 x 6144 0.2 %, 10 % at worst.  (With up to 64 rows the streaming GEMM was always faster.)
-// Where the streaming GEMM's tiles are whole, up to 256 rows, its own estimate takes the place of this fit.
+// Where the streaming GEMM's tiles are whole, up to 256 rows, its own estimate takes the place of this fit, and the rounding
+// launch of bf16 rows counts what 100 layers lost by it (median 3.0 us; with 1.8 1152 -> 9600 at 230 rows, 18.3 us decoded first, took 20.7).
 bool stream_beats_dense(const rdq_layer &l, int M, int x_type) {
   if (M <= 64) return true;
   if (M > 2048) return false;
@@ -104,7 +105,7 @@ bool stream_beats_dense(const rdq_layer &l, int M, int x_type) {
   const double weights = 1e-6 * N * l.K;
   const double cast = x_type == RDQ_BF16 ? 1.8 : 0.0;  // the other GEMM's decoding launch rounds bf16 rows along the way
   const double whole = M <= 256 ? gemm_stream_estimate(l.n_fp4, l.n_fp8, l.n_fp16, M, l.K) : 0.0;
-  if (whole > 0.0) return cast + whole < gemm_dense_estimate(M, N, l.K);
+  if (whole > 0.0) return (x_type == RDQ_BF16 ? 3.0 : 0.0) + whole < gemm_dense_estimate(M, N, l.K);
   return cast + 15.6 + 1.57e-3 * M * weights < gemm_dense_estimate(M, N, l.K);
 }
 

@@ -164,7 +164,7 @@ def test_wide_layers_of_few_rows_need_no_decoding(rows, shape, scratch):
     # block scales copied 8 bytes at a time: whole tiles, one tile of tokens and several
     ((300, 130, 20, 896), 33, "whole"), ((1280, 640, 128, 2176), 100, "whole"), ((1280, 640, 128, 2176), 140, "whole"),
     # whole tiles of more than 64 tokens: clusters of one, two and four; tiles of tokens that are hardly filled
-    ((1280, 640, 128, 640), 65, "whole"), ((3072, 896, 128, 4096), 128, "whole"), ((640, 384, 0, 2560), 129, "whole"),
+    ((2688, 1280, 128, 1088), 129, "whole"), ((3072, 896, 128, 4096), 128, "whole"), ((640, 384, 0, 2560), 129, "whole"),
     ((300, 130, 20, 2624), 200, "whole"), ((0, 0, 256, 8192), 256, "whole"),
     # cut ones where those are the faster, and beyond 256 rows; there small layers are decoded first
     ((4096, 1920, 128, 2560), 193, "cut"), ((13056, 6144, 256, 2560), 66, "cut"), ((1280, 640, 128, 4096), 300, "cut"),
@@ -222,3 +222,9 @@ def test_streaming_gemm_clusters_across_token_tiles(shape, rows, dtype):
 def test_streaming_gemm_tiles_of_up_to_64_rows(shape, rows, tiles, dtype):
     """Whole tiles and cut ones, each where it is the faster."""
     _check_streaming_gemm(shape, rows, dtype, tiles)
+
+
+@pytest.mark.parametrize("dtype,tiles", [(torch.float16, "whole"), (torch.bfloat16, None)])
+def test_bf16_rows_count_their_rounding(dtype, tiles):
+    """A layer near the line between the GEMMs: bf16 rows are rounded ahead of the streaming one, inside the other's first launch."""
+    _check_streaming_gemm((6400, 3072, 128, 1152), 230, dtype, tiles)
