@@ -18,7 +18,7 @@
 // order: the result does not depend on timing (await_parts: those that leave, and who does their share).  A second kernel for these sums cost
 // 4-7 us per layer, and one CTA per tile adding them up to 13 us.
 //
-// Up to 64 tokens, or 256 where that is faster (best_plan), tiles are not cut: a tile has as many rows (8 to 128) as make all
+// Up to 256 tokens, where that is faster (best_plan), tiles are not cut: a tile has as many rows (8 to 128) as make all
 // tiles cost the same bytes, and belongs to one cluster of one, two or four CTAs that share its k.  A chunk is 256 k of any format then (one, two or four boxes).  The
 // CTAs of a cluster exchange FP32 sums through distributed shared memory (finish_in_cluster): each finishes a share of the tokens.
 // They run at the same time by construction, and no word in global memory is involved.
@@ -287,8 +287,7 @@ __device__ __forceinline__ void convert_fp8(const uint4 &a, const uint4 &b, uint
   cvt_e4m3x4(b.w, o[14], o[15]);
 }
 
-// row r of a segment's tile
-// (of `height` rows)
+// row r of a segment's tile of `height` rows
 __device__ __forceinline__ Row row_of(const StreamArgs &a, const Segment &g, int height, int r, bool wanted) {
   Row w;
   const int row = g.row_tile * height + r;  // row inside the format group
@@ -450,9 +449,9 @@ __device__ __forceinline__ void finish_in_cluster(StreamSmem &S, const StreamSch
   }
 }
 
-// NT: most tokens per tile (64 or 128).  WHOLE: every tile belongs to one CTA, a chunk has 256 k of any format (make_whole_plan).
+// NT: most tokens per tile (64 or 128).  WHOLE: every tile belongs to one cluster, a chunk has 256 k of any format (make_whole_plan).
 // MANY: of several token tiles; without it their arithmetic, which every role does ahead of its first chunk, is not there (decode
-// step of 32 rows 284 us with a division by their number, 277 with a loop, 269 without).
+// step of four blocks, 32 sequences at 600 tokens: 284 us with a division by their number, 277 with a loop, 269 without).
 template <int NT, bool BF16, bool WHOLE, bool MANY = false>
 __global__ void __launch_bounds__(kThreadBound<NT>, 1)
 gemm_stream_kernel(const __grid_constant__ CUtensorMap w4map, const __grid_constant__ CUtensorMap w8map,
@@ -1096,8 +1095,9 @@ bool make_whole_plan(int n4, int n8, int n16, int M, int K, int cluster, StreamP
 // What whole tiles of up to 64 tokens take more than cut ones, in microseconds.  Whole ones cost by their steps of 256 k and
 // by the exchange, cut ones by a CTA's share and by the parts of a tile.  Where a row of block scales is no
 // multiple of 16 bytes the warp that copies them 8 bytes at a time bounds both, whole tiles by their rows of NVFP4.
-// Fitted to the difference of both on 190 layers (1 to 150 MB, K 1024 to 16384, 50 to 90 % NVFP4) at 9 to 64 rows: of 890
-// points the choice is 0.04 % behind the faster on average, 5 % at worst; always whole was 0.8 % behind, 23 % at worst.
+// Fitted to the difference of both on 190 layers (1 to 150 MB, K 1024 to 16384, 50 to 90 % NVFP4) at 9 to 64 rows.  Of 1800
+// points, layers without FP16, with odd channels and K of 64 times an odd number among them, the choice is 0.15 % behind the faster on
+// average, 11 % at worst (3968 -> 4608 at 9 rows); always whole is 0.6 % behind, 23 % at worst.
 double whole_minus_cut(const StreamPlan &whole, const StreamPlan &cut, int n4, int K) {
   const StreamSched &s = whole.sc;
   const bool narrow = n4 > 0 && K % 256 != 0;
@@ -1111,8 +1111,10 @@ double whole_minus_cut(const StreamPlan &whole, const StreamPlan &cut, int n4, i
 // arrival, sums, each a round trip to L2 by code that is run once), a cluster 1700 and a CTA alone 1000.  32 rows, calls
 // one after another, us of cut tiles and of whole ones: 2560 -> 6144 10.6, 8.3; 4096 -> 2560 10.6, 7.7; 9728 -> 2560 12.5, 10.6;
 // 1024 -> 1024 8.0, 6.0; 8192 -> 8192 15.5, 13.7.  But a tile that no cluster of four has room for, of a long K, takes
-// longer than its shares: 13312 -> 4608 15.4, 17.6; 8192 -> 4224 13.2, 13.7; 12288 -> 4096 at 64 rows 16.0, 18.6.  From 150 MB on
-// tiles are cut: the tail is short beside the rest, and they use the MMA's 128 rows (8192 -> 57344, 292 MB, at 48 rows 73.6, 76.2).
+// longer than its shares: 13312 -> 4608 15.4, 17.6; 8192 -> 4224 at 9 rows 12.5, 13.7; 12288 -> 4096 at 64 rows 16.0, 18.6.  From 150 MB on
+// tiles are cut: the tail is short beside the rest, and they use the MMA's 128 rows (10496 -> 21760, 163 MB, at 9 and 32 rows 32.8,
+// 34.3 cut, 32.2, 33.9 at best whole; 8192 -> 57344, 292 MB, at 48 rows 73.6, 76.2).  Narrow copies of block scales are the
+// exception that is not made: 7552 -> 55424, 297 MB, at 32 rows 84.9, 68.9.
 //
 // More tokens come in tiles of 64, each work of its own: the weights are converted for each, where cut tiles convert them for 128
 // at a time, so that it pays where a CTA's share is small beside the tail.  The estimates decide; the margin covers theirs
