@@ -58,8 +58,9 @@ bool has_row_major(const rdq_layer &l) {
 // 12.1 / 13.1).  The streaming GEMM's narrow copies of block scales (8 bytes where K is no multiple of 256, 4 where it is
 // none of 128) keep few rows with the GEMV up to 40 MB, bf16 rows and K of no multiple of 128, unless K is below 2048: time of the GEMM over
 // the GEMV's at four rows, f16 and bf16, 26 MB (3659 x 9664) 1.06, 1.40; 40 MB (4677 x 11712) 1.14, 1.50; 26 MB (12227 x 2944) 0.95,
-// 1.21; but 30 MB (8613 x 4864) 0.75, 0.97 and 36 MB (33535 x 1472) 0.82, 0.96.  Of 56 layers the f16 rows of 4027 x 5504 (16 MB)
-// fare worst, 1.25 at nine.
+// 1.21; but 30 MB (8613 x 4864) 0.75, 0.97 and 36 MB (33535 x 1472) 0.82, 0.96.  Nor do 9 to 16 f16 rows gain by
+// it up to 18 MB where the GEMV's blocks are one wave of two to an SM (4027 x 5504 1.25 at nine, 2813 x 8768 1.06; but with fewer
+// or more of them 1671 x 12480 0.89, 5309 x 3520 0.88, 10415 x 2112 0.79).
 // Seven and eight rows that the GEMV does not keep in shared memory go to the streaming GEMM from 28 MB on where its
 // tiles are whole and its copies wide, or K is below 8000: 37 MB (3584 x 14336) 15.5 / 13.3 us, 38 MB (4096 x 12288) 16.5 / 12.1,
 // 30 MB (12672 x 3328) 0.83 of the time, 26 MB (5120 x 7168) 1.1; but 37 MB (3072 x 16000) 14.9 / 16.1, with bf16 rows
@@ -75,7 +76,9 @@ int stream_from(const rdq_layer &l, int x_type) {
     const bool bf16 = x_type == RDQ_BF16;
     const double few = wide || l.K < 2048 || (!bf16 && l.K % 128 == 0) ? (bf16 ? 24e6 : 22e6) : 40e6;
     if (bytes > few) return 1;
-    return bytes > (bf16 ? 18e6 : 12e6) ? 9 : RDQ_MAX_GEMV_M + 1;
+    const int N = l.n_fp4 + l.n_fp8 + l.n_fp16;
+    const bool one_wave = N > 16 * 148 && N <= 32 * 148;  // of the GEMV's blocks, two to an SM
+    return bytes > (bf16 || (!wide && one_wave) ? 18e6 : 12e6) ? 9 : RDQ_MAX_GEMV_M + 1;
   }
   if (bytes > 40e6) return bytes > 80e6 ? 1 : 3;
   if (bytes <= 28e6 || tiled_stages_x(8, l.K)) return 9;

@@ -90,6 +90,7 @@ def test_small_layers_without_tiles_stay_on_the_decode_kernel(n4, n8, k, decode_
 @pytest.mark.parametrize("n4,n8,k,tiled,x_type,first", [
     # row-major layers: f16 and bf16 rows between the lines, K of multiples of 256, 128 and 64, and a short K
     (5001, 2503, 2560, False, 0, 9), (5001, 2503, 2560, False, 1, 17),          # 14 MB
+    (2698, 1249, 5504, False, 0, 17), (3600, 1749, 3520, False, 0, 9),          # 15, 13 MB: a wave of the decode kernel, more than one
     (7001, 3503, 4096, False, 0, 1), (7001, 3503, 4096, False, 1, 1),           # 30 MB
     (6001, 3003, 4096, False, 0, 1), (6001, 3003, 3968, False, 1, 1 + 8),       # 26, 25 MB
     (8192, 4035, 2944, False, 0, 1), (8192, 4035, 2944, False, 1, 9),           # 25 MB
