@@ -1096,13 +1096,13 @@ bool make_whole_plan(int n4, int n8, int n16, int M, int K, int cluster, StreamP
 // by the exchange, cut ones by a CTA's share and by the parts of a tile.  Where a row of block scales is no
 // multiple of 16 bytes the warp that copies them 8 bytes at a time bounds both, whole tiles by their rows of NVFP4.
 // Fitted to the difference of both on 190 layers (1 to 150 MB, K 1024 to 16384, 50 to 90 % NVFP4) at 9 to 64 rows.  Of 1800
-// points, layers without FP16, with odd channels and K of 64 times an odd number among them, the choice is 0.15 % behind the faster on
-// average, 11 % at worst (3968 -> 4608 at 9 rows); always whole is 0.6 % behind, 23 % at worst.
+// points, layers without FP16, with odd channels and K of 64 times an odd number among them, the choice is 0.13 % behind the faster on
+// average, 10 % at worst (4096 -> 5120 at 9 rows); always whole is 0.6 % behind, 23 % at worst.
 double whole_minus_cut(const StreamPlan &whole, const StreamPlan &cut, int n4, int K) {
   const StreamSched &s = whole.sc;
   const bool narrow = n4 > 0 && K % 256 != 0;
   const int steps = whole.each * ((s.S[0] + s.cluster - 1) / s.cluster);
-  const double exchange = s.cluster == 1 ? 0.0 : (s.cluster == 2 ? 1.5 : 1.5 * whole.each);
+  const double exchange = s.cluster == 1 ? 0.0 : (s.cluster == 2 ? (narrow ? 1.2 : 1.5) : 1.5 * whole.each);
   return steps * (narrow ? 0.143 * ((s.R[0] + 31) / 32) : 0.32) + exchange -
          (1.2 + (narrow ? 0.74e-3 : 0.4e-3) * cut.share + 0.09 * cut.parts + 0.02 * s.nt);
 }
